@@ -20,8 +20,6 @@ namespace kfac {
 
 constexpr int DB = 128;        // diagonal block
 constexpr int PW = 512;        // Cholesky panel width (outer blocking)
-// floats of the diagonal kernel's shared memory: Lt, Pt, Xr, Tk
-constexpr int kDiagBaseFloats = DB * (DB + 4) + 24 * DB + 16 * 64;
 
 struct MatInfo {
   const float* F;
@@ -177,6 +175,9 @@ __global__ void damp_copy_kernel(const MatInfo* __restrict__ mats,
 
 // ------------------------------------------------ look-ahead of the Cholesky
 constexpr int DLD = DB + 4;   // shared-memory row pitch of a 128 x 128 block
+constexpr int SB = 32;        // sub-block of the diagonal kernel
+constexpr int SLP = SB + 4;   // row pitch of a 32 x 32 sub-block
+constexpr int DT = 512;       // threads of the diagonal kernel
 constexpr int kLookTile = DB * 32 * 4;          // one 128 x 32 fp32 operand tile
 constexpr int kLookStage = 4 * kLookTile;       // [A hi][A lo][B hi][B lo]
 constexpr int kLookCols = 2 * DB;               // tensor-memory columns
@@ -190,14 +191,15 @@ struct LookControl {
   volatile int abort_flag;
 };
 
-// Issue the three split-TF32 MMAs of one 32-k operand block: D(128 x 128) +=
+// Issue the three split-TF32 MMAs of one 32-k operand block: D(128 x n) +=
 // A B^T with A, B given as hi / lo tile addresses (K-major, 128-byte
 // swizzle).  hi*hi goes to columns [0, 128) of the tensor memory, the cross
 // terms to [128, 256).
 __device__ __forceinline__ void look_mma_block(unsigned tmem, unsigned a_hi,
                                                unsigned a_lo, unsigned b_hi,
-                                               unsigned b_lo, bool first) {
-  const unsigned idesc = tc_instr_desc(DB);
+                                               unsigned b_lo, int n,
+                                               bool first) {
+  const unsigned idesc = tc_instr_desc(n);
   const unsigned long long dah = tc_smem_desc(a_hi), dal = tc_smem_desc(a_lo);
   const unsigned long long dbh = tc_smem_desc(b_hi), dbl = tc_smem_desc(b_lo);
 #pragma unroll
@@ -210,6 +212,39 @@ __device__ __forceinline__ void look_mma_block(unsigned tmem, unsigned a_hi,
   }
 }
 
+// 16 bytes global -> shared without a register in between.
+__device__ __forceinline__ void cp_async16(unsigned dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src)
+               : "memory");
+}
+
+// W_kk (bs x bs) into S; beyond bs the identity, so that the sweeps below run
+// over whole sub-blocks.  Asynchronous where the rows are 16-byte aligned:
+// the caller waits (diag_load_wait) before its next barrier.
+__device__ __forceinline__ void diag_load(const float* Wd, long long ld, int bs,
+                                          bool vec, float* S) {
+  const int rows = (bs + SB - 1) / SB * SB;
+  for (int idx = threadIdx.x; idx < rows * (DB / 4); idx += DT) {
+    const int r = idx >> 5, c = (idx & 31) * 4;
+    float* dst = &S[r * DLD + c];
+    if (c > (r | (SB - 1))) continue;       // above the diagonal: never read
+    if (vec && r < bs && c + 3 < bs) {
+      cp_async16(smem_u32(dst), &Wd[r * ld + c]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float v = (r == c + e) ? 1.f : 0.f;
+        if (r < bs && c + e < bs) v = Wd[r * ld + c + e];
+        dst[e] = v;
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void diag_load_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // The diagonal block of step k has received the updates of all steps before
 // k - 1; the update of step k - 1,
 //   D = W_kk - L' L'^T,  L' = A' X_pp^T,
@@ -218,21 +253,38 @@ __device__ __forceinline__ void look_mma_block(unsigned tmem, unsigned a_hi,
 // output buffer) and X_pp (inverse of the previous diagonal block's factor),
 // so that this kernel does not have to wait for the panel solve and panel
 // update of step k - 1.  Both products run on the tensor cores (tcgen05,
-// split TF32, accumulators in tensor memory).  Result: D in Sa (rows and
-// columns below `bs` are meaningful).  256 threads.  Returns false if a
+// split TF32, accumulators in tensor memory).  All global loads are in flight
+// at once (16 x 16 bytes per thread); the blocks of X_pp above its diagonal
+// are neither loaded nor multiplied.  Result: D in S.  Returns false if a
 // bounded wait ran out (the status word is set; the caller stores nothing).
 __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
-                                               float* Sa, unsigned char* stage,
+                                               bool vec, float* S,
+                                               unsigned char* stage,
                                                LookControl* ctl) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long ld = mi.d;
   const float* Ap = mi.inv + (long long)o * ld + (o - DB);
   const float* Xp = mi.X + (long long)(o - DB) * ld + (o - DB);
-  const float* Wd = mi.W + (long long)o * ld + o;
-  const bool vec = (ld & 3) == 0 && (o & 3) == 0 &&
-                   ((reinterpret_cast<uintptr_t>(mi.inv) |
-                     reinterpret_cast<uintptr_t>(mi.X) |
-                     reinterpret_cast<uintptr_t>(mi.W)) & 15) == 0;
+  float4 va[4][2], vx[4][2];
+#pragma unroll
+  for (int kb = 0; kb < 4; ++kb) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int c = tid + DT * j, row = c >> 3, col = 32 * kb + 4 * (c & 7);
+      va[kb][j] = vx[kb][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float* pa = &Ap[row * ld + col];
+      const float* px = &Xp[row * ld + col];
+      if (vec) {
+        if (row < bs) va[kb][j] = *reinterpret_cast<const float4*>(pa);
+        if (row >= 32 * kb) vx[kb][j] = *reinterpret_cast<const float4*>(px);
+      } else {
+        if (row < bs) va[kb][j] = make_float4(pa[0], pa[1], pa[2], pa[3]);
+        if (row >= 32 * kb) vx[kb][j] = make_float4(px[0], px[1], px[2], px[3]);
+      }
+    }
+  }
+  // W_kk into S (the update is subtracted from it at the end)
+  diag_load(mi.W + (long long)o * ld + o, ld, bs, vec, S);
   if (tid == 0) {
     mbar_init(&ctl->bar[0], 1);
     mbar_init(&ctl->bar[1], 1);
@@ -248,22 +300,6 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
                  ::: "memory");
   }
-  // W_kk into Sa (the update is subtracted from it at the end)
-  for (int idx = tid; idx < DB * (DB / 4); idx += 256) {
-    const int r = idx >> 5, c = (idx & 31) * 4;
-    float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < bs) {
-      if (vec && c + 3 < bs) {
-        w = *reinterpret_cast<const float4*>(&Wd[r * ld + c]);
-      } else {
-        if (c < bs) w.x = Wd[r * ld + c];
-        if (c + 1 < bs) w.y = Wd[r * ld + c + 1];
-        if (c + 2 < bs) w.z = Wd[r * ld + c + 2];
-        if (c + 3 < bs) w.w = Wd[r * ld + c + 3];
-      }
-    }
-    *reinterpret_cast<float4*>(&Sa[r * DLD + c]) = w;
-  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -271,29 +307,7 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
   const unsigned sbase = smem_u32(stage);
   bool ok = true;
 
-  // ---- L' = A' X_pp^T: four operand blocks of 32 k through two stages; the
-  // global loads of block kb + 1 are in flight while block kb is split,
-  // stored and multiplied
-  float4 va[4], vx[4];
-  auto load_block = [&](int kb) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = tid + 256 * j, row = c >> 3, col = 32 * kb + 4 * (c & 7);
-      va[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (vec) {
-        if (row < bs) va[j] = *reinterpret_cast<const float4*>(&Ap[row * ld + col]);
-        vx[j] = *reinterpret_cast<const float4*>(&Xp[row * ld + col]);
-      } else {
-        if (row < bs) {
-          va[j].x = Ap[row * ld + col]; va[j].y = Ap[row * ld + col + 1];
-          va[j].z = Ap[row * ld + col + 2]; va[j].w = Ap[row * ld + col + 3];
-        }
-        vx[j].x = Xp[row * ld + col]; vx[j].y = Xp[row * ld + col + 1];
-        vx[j].z = Xp[row * ld + col + 2]; vx[j].w = Xp[row * ld + col + 3];
-      }
-    }
-  };
-  load_block(0);
+  // ---- L' = A' X_pp^T: four operand blocks of 32 k through two stages
 #pragma unroll
   for (int kb = 0; kb < 4; ++kb) {
     const int s = kb & 1;
@@ -301,19 +315,23 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
                                        &g_diag_status) && ok;
     const unsigned st = sbase + s * kLookStage;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = tid + 256 * j;
-      const unsigned off = (unsigned)sw128_chunk_off(c >> 3, c & 7);
-      store_split(st + off, st + kLookTile + off, va[j]);
-      store_split(st + 2 * kLookTile + off, st + 3 * kLookTile + off, vx[j]);
+    for (int j = 0; j < 2; ++j) {
+      const int c = tid + DT * j, row = c >> 3;
+      const unsigned off = (unsigned)sw128_chunk_off(row, c & 7);
+      store_split(st + off, st + kLookTile + off, va[kb][j]);
+      if (row >= 32 * kb)
+        store_split(st + 2 * kLookTile + off, st + 3 * kLookTile + off,
+                    vx[kb][j]);
     }
-    if (kb + 1 < 4) load_block(kb + 1);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (tid == 0 && !ctl->abort_flag) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      look_mma_block(tmem, st, st + kLookTile, st + 2 * kLookTile,
-                     st + 3 * kLookTile, kb == 0);
+      // columns below 32 kb of L' get nothing from this block of k
+      const unsigned skip = (unsigned)(32 * kb) * 128;
+      look_mma_block(tmem + 32 * kb, st, st + kLookTile,
+                     st + 2 * kLookTile + skip, st + 3 * kLookTile + skip,
+                     DB - 32 * kb, kb == 0);
       tc_commit(&ctl->bar[s]);
     }
   }
@@ -327,20 +345,19 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
   const int row = 32 * q + lane;
   ok = __all_sync(0xffffffffu, ok);     // the loads below are warp-wide
   if (ok) {
+    const unsigned blk = sbase + (unsigned)h * (2 * kLookTile);
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) {
-      const int c0 = 64 * h + 16 * cc;
+    for (int cc = 0; cc < 2; ++cc) {
+      const int c0 = 32 * h + 16 * cc;
       float v[16], w[16];
       tc_ld16(tmem + ((unsigned)(32 * q) << 16) + (unsigned)c0, v);
       tc_ld16(tmem + ((unsigned)(32 * q) << 16) + (unsigned)(DB + c0), w);
-      const unsigned blk = sbase + (unsigned)(c0 >> 5) * (2 * kLookTile);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float4 x = make_float4(v[4 * i] + w[4 * i], v[4 * i + 1] + w[4 * i + 1],
                                      v[4 * i + 2] + w[4 * i + 2],
                                      v[4 * i + 3] + w[4 * i + 3]);
-        const unsigned off =
-            (unsigned)sw128_chunk_off(row, ((c0 & 31) >> 2) + i);
+        const unsigned off = (unsigned)sw128_chunk_off(row, 4 * cc + i);
         store_split(blk + off, blk + kLookTile + off, x);
       }
     }
@@ -354,22 +371,33 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
 #pragma unroll
     for (int kb = 0; kb < 4; ++kb) {
       const unsigned blk = sbase + (unsigned)kb * (2 * kLookTile);
-      look_mma_block(tmem, blk, blk + kLookTile, blk, blk + kLookTile, kb == 0);
+      look_mma_block(tmem, blk, blk + kLookTile, blk, blk + kLookTile, DB,
+                     kb == 0);
     }
     tc_commit(&ctl->done);
   }
+  diag_load_wait();
   ok = mbar_wait_status(&ctl->done, 0, &ctl->abort_flag, &g_diag_status) && ok;
-  ok = __all_sync(0xffffffffu, ok);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (ok) {
+  __syncthreads();                      // every thread's part of W_kk is there
+  ok = __all_sync(0xffffffffu, ok);
+  if (ok && h <= q) {                   // sub-blocks on and below the diagonal
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) {
-      const int c0 = 64 * h + 16 * cc;
+    for (int cc = 0; cc < 2; ++cc) {
+      const int c0 = 32 * h + 16 * cc;
       float v[16], w[16];
       tc_ld16(tmem + ((unsigned)(32 * q) << 16) + (unsigned)c0, v);
       tc_ld16(tmem + ((unsigned)(32 * q) << 16) + (unsigned)(DB + c0), w);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) Sa[row * DLD + c0 + i] -= v[i] + w[i];
+      for (int i = 0; i < 4; ++i) {
+        float4* s4 = reinterpret_cast<float4*>(&S[row * DLD + c0 + 4 * i]);
+        float4 d = *s4;
+        d.x -= v[4 * i] + w[4 * i];
+        d.y -= v[4 * i + 1] + w[4 * i + 1];
+        d.z -= v[4 * i + 2] + w[4 * i + 2];
+        d.w -= v[4 * i + 3] + w[4 * i + 3];
+        *s4 = d;
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -382,280 +410,317 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
   return ctl->abort_flag == 0;
 }
 
+// ------------------------------------------------ one 128 x 128 diagonal block
+// Shared memory of the diagonal kernel, in floats.
+struct DiagSmem {
+  float S[DB * DLD];          // D / L in the sub-blocks on and below the
+                              // diagonal, X^T in those above it
+  float XDT[4][SB * SLP];     // inverse of sub-block p of the diagonal, transposed
+  float XD[4][SB * SLP];      // the same, row-major
+  float TT[3 * SB * SLP];     // T^T of the running block row
+  float LT[SB * SLP];         // L_pp, transposed
+  float rl[SB];               // 1 / l_cc
+  float4 Lp[2][SB];           // four columns of L_pp on their way to the warp
+};
+
+// r = 1 / sqrt(q) by the approximation and one Newton step: full fp32 accuracy
+// without the IEEE square root and division.  A pivot that is not positive
+// (or below the smallest normal number) counts as failed and becomes 1.
+__device__ __forceinline__ float pivot_rsqrt(float q, bool& bad) {
+  bad = !(q >= 1.17549435e-38f);
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q));
+  r = r * fmaf(-0.5f * q, r * r, 1.5f);
+  return bad ? 1.f : r;
+}
+
+// Cholesky factor of sub-block p of the diagonal by one warp, a row per lane in
+// registers, four columns per step: every lane factors the 4 x 4 pivot block
+// redundantly (ten shuffles fetch it), so the serial chain per column is one
+// reciprocal square root and two multiply-adds, and the rank-4 update reads
+// the other rows' four values as one broadcast 16-byte word each.
+__device__ __forceinline__ void diag_base(DiagSmem& sm, int p, int lane, int id,
+                                          int col0, int* info) {
+  float a[SB];
+#pragma unroll
+  for (int j = 0; j < SB / 4; ++j) {
+    const float4 v = *reinterpret_cast<const float4*>(
+        &sm.S[(SB * p + lane) * DLD + SB * p + 4 * j]);
+    a[4 * j] = v.x; a[4 * j + 1] = v.y; a[4 * j + 2] = v.z; a[4 * j + 3] = v.w;
+  }
+  int first = 0;
+#pragma unroll
+  for (int s = 0; s < SB / 4; ++s) {
+    const int j = 4 * s;
+    const unsigned all = 0xffffffffu;
+    const float p00 = __shfl_sync(all, a[j], j);
+    const float p10 = __shfl_sync(all, a[j], j + 1);
+    const float p11 = __shfl_sync(all, a[j + 1], j + 1);
+    const float p20 = __shfl_sync(all, a[j], j + 2);
+    const float p21 = __shfl_sync(all, a[j + 1], j + 2);
+    const float p22 = __shfl_sync(all, a[j + 2], j + 2);
+    const float p30 = __shfl_sync(all, a[j], j + 3);
+    const float p31 = __shfl_sync(all, a[j + 1], j + 3);
+    const float p32 = __shfl_sync(all, a[j + 2], j + 3);
+    const float p33 = __shfl_sync(all, a[j + 3], j + 3);
+    bool b0, b1, b2, b3;
+    const float r0 = pivot_rsqrt(p00, b0);
+    const float l10 = p10 * r0, l20 = p20 * r0, l30 = p30 * r0;
+    const float r1 = pivot_rsqrt(fmaf(-l10, l10, p11), b1);
+    const float l21 = fmaf(-l20, l10, p21) * r1;
+    const float l31 = fmaf(-l30, l10, p31) * r1;
+    const float r2 = pivot_rsqrt(fmaf(-l21, l21, fmaf(-l20, l20, p22)), b2);
+    const float l32 = fmaf(-l31, l21, fmaf(-l30, l20, p32)) * r2;
+    const float r3 = pivot_rsqrt(
+        fmaf(-l32, l32, fmaf(-l31, l31, fmaf(-l30, l30, p33))), b3);
+    if (first == 0) {
+      if (b0) first = j + 1;
+      else if (b1) first = j + 2;
+      else if (b2) first = j + 3;
+      else if (b3) first = j + 4;
+    }
+    // this lane's row of the four columns (rows above the pivot: unused)
+    const float x0 = a[j] * r0;
+    const float x1 = fmaf(-x0, l10, a[j + 1]) * r1;
+    const float x2 = fmaf(-x1, l21, fmaf(-x0, l20, a[j + 2])) * r2;
+    const float x3 =
+        fmaf(-x2, l32, fmaf(-x1, l31, fmaf(-x0, l30, a[j + 3]))) * r3;
+    if (s + 1 < SB / 4) {
+      sm.Lp[s & 1][lane] = make_float4(x0, x1, x2, x3);
+      __syncwarp();
+#pragma unroll
+      for (int c = j + 4; c < SB; ++c) {
+        const float4 v = sm.Lp[s & 1][c];
+        a[c] = fmaf(-x3, v.w, fmaf(-x2, v.z, fmaf(-x1, v.y, fmaf(-x0, v.x, a[c]))));
+      }
+    }
+    sm.LT[j * SLP + lane] = x0;
+    sm.LT[(j + 1) * SLP + lane] = x1;
+    sm.LT[(j + 2) * SLP + lane] = x2;
+    sm.LT[(j + 3) * SLP + lane] = x3;
+    if (lane == 0)
+      *reinterpret_cast<float4*>(&sm.rl[j]) = make_float4(r0, r1, r2, r3);
+  }
+  if (first != 0 && lane == 0)
+    atomicCAS(&info[id], 0, col0 + first);
+}
+
+// a <- a L_pp^-T for one row per thread (right-looking substitution): the rows
+// of L below sub-block p, or, started from a unit vector, a column of X_pp.
+__device__ __forceinline__ void diag_solve_row(const DiagSmem& sm, float a[SB]) {
+  float4 rl;
+#pragma unroll
+  for (int c = 0; c < SB; ++c) {
+    if ((c & 3) == 0) rl = *reinterpret_cast<const float4*>(&sm.rl[c]);
+    const float r = (c & 3) == 0 ? rl.x : (c & 3) == 1 ? rl.y
+                    : (c & 3) == 2 ? rl.z : rl.w;
+    const float x = a[c] * r;
+    a[c] = x;
+#pragma unroll
+    for (int g = (c + 1) >> 2; g < SB / 4; ++g) {
+      const float4 v = *reinterpret_cast<const float4*>(&sm.LT[c * SLP + 4 * g]);
+      if (4 * g > c) a[4 * g] = fmaf(-x, v.x, a[4 * g]);
+      if (4 * g + 1 > c) a[4 * g + 1] = fmaf(-x, v.y, a[4 * g + 1]);
+      if (4 * g + 2 > c) a[4 * g + 2] = fmaf(-x, v.z, a[4 * g + 2]);
+      a[4 * g + 3] = fmaf(-x, v.w, a[4 * g + 3]);
+    }
+  }
+}
+
+// acc(16 x 32) += A B^T over 32 k, one warp: A 16 rows, B 32 rows, both
+// contiguous along k with the given row pitches.  Lane (rg, cg) = (lane / 8,
+// lane % 8) holds rows rg + 4 i, columns cg + 8 j: the 16-byte loads of a
+// quarter warp fall into different banks.
+__device__ __forceinline__ void diag_mac(const float* A, int pa, const float* B,
+                                         int pb, int lane, float acc[4][4]) {
+  const float* ar = A + (lane >> 3) * pa;
+  const float* br = B + (lane & 7) * pb;
+#pragma unroll 4
+  for (int k = 0; k < SB; k += 4) {
+    float4 av[4], bv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      av[i] = *reinterpret_cast<const float4*>(&ar[4 * i * pa + k]);
+      bv[i] = *reinterpret_cast<const float4*>(&br[8 * i * pb + k]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        acc[i][j] = fmaf(av[i].w, bv[j].w, fmaf(av[i].z, bv[j].z,
+                    fmaf(av[i].y, bv[j].y, fmaf(av[i].x, bv[j].x, acc[i][j]))));
+  }
+}
+
+// Row block i of the inverse left of its diagonal sub-block, transposed:
+// X^T(j, i) = -T^T X_ii^T for sub-block j < i; `half`: its upper or lower 16
+// rows.  One warp.
+__device__ __forceinline__ void diag_x_block(DiagSmem& sm, int i, int j,
+                                             int half, int lane) {
+  float acc[4][4] = {};
+  diag_mac(&sm.TT[(SB * j + 16 * half) * SLP], SLP, sm.XD[i], SLP, lane, acc);
+  float* dst = &sm.S[(SB * j + 16 * half + (lane >> 3)) * DLD + SB * i +
+                     (lane & 7)];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) dst[4 * r * DLD + 8 * c] = -acc[r][c];
+}
+
 // Factor one diagonal block (<= 128 x 128) of W and invert the resulting
-// triangle: W_jj <- L_jj (lower), X_jj <- L_jj^-1 (lower, upper part zero).
-// One CTA of 256 threads per matrix that still has a block at `step`; thread
-// (br, bc) = (tid / 16, tid % 16) keeps the 8 x 8 block (br, bc) in registers
-// (consecutive lanes hold consecutive column blocks, so that rows of W and X
-// are read and written as contiguous 32-byte pieces).
-// Both sweeps advance by block columns of 8 with two barriers (Cholesky) or
-// one (inverse) per block column instead of one per column:
-//   Cholesky, block column kb: thread (kb, kb) factors its 8 x 8 block and
-//   inverts the small triangle, all in registers; the threads below multiply
-//   their blocks by that inverse (panel solve); every remaining block takes
-//   a rank-8 update from the panel, read from shared memory.
-//   Inverse, block row kb: the threads of block row kb apply the stored 8 x 8
-//   inverse to their blocks of the running right-hand side (rows kb of X are
-//   then final); the rows below take a rank-8 update.
+// triangle: X_kk <- L_kk^-1 (lower part; nothing reads L_kk itself).  One CTA
+// of 16 warps per matrix that still has a block at `step`.
+//
+// The block is swept in four sub-blocks of 32 columns.  Bound: the serial
+// chain of 128 pivots, so everything else is kept off it.  Per sub-block p,
+// one warp factors the 32 x 32 diagonal (diag_base); the rows below it (one
+// thread each) and, with unit vectors as input, the columns of its inverse
+// follow by substitution in other warps; the next diagonal sub-block is
+// updated by all warps, and while it is being factored the remaining warps
+// finish the update of the sub-blocks behind it and the off-diagonal part of
+// the inverse (row block p of X: T = L(p, <p) X(<p, <p) does not need X_pp).
+// 128 x 128 block, measured with the look-ahead: see the table at the plan.
 template <bool LOOK>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(DT, 1)
 chol_diag_kernel(const MatInfo* __restrict__ mats, const int* __restrict__ ids,
                  int step, int* __restrict__ info) {
   extern __shared__ __align__(16) float dsm[];
-  float (*Lt)[DB + 4] = reinterpret_cast<float (*)[DB + 4]>(dsm);  // L^T
-  float (*Pt)[DB] = reinterpret_cast<float (*)[DB]>(dsm + DB * (DB + 4));
-  float (*Xr)[8][DB] =
-      reinterpret_cast<float (*)[8][DB]>(dsm + DB * (DB + 4) + 8 * DB);
-  float (*Tk)[64] =
-      reinterpret_cast<float (*)[64]>(dsm + DB * (DB + 4) + 24 * DB);
+  DiagSmem& sm = *reinterpret_cast<DiagSmem*>(dsm);
   const int id = ids[blockIdx.x];
   const MatInfo mi = mats[id];
-  const int tid = threadIdx.x, br = tid >> 4, bc = tid & 15;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int o = step * DB;
   const int bs = min(DB, mi.d - o);
-  const int nkb = (bs + 7) >> 3;
+  const int np = (bs + SB - 1) / SB;      // sub-blocks in use
   const long long ld = mi.d;
-  float* Wd = mi.W + (long long)o * ld + o;
-  float* Xd = mi.X + (long long)o * ld + o;
-
-  // blocks strictly below the diagonal move as two 16-byte pieces per row
   const bool vec = (ld & 3) == 0 && (o & 3) == 0 &&
                    ((reinterpret_cast<uintptr_t>(mi.W) |
+                     reinterpret_cast<uintptr_t>(mi.inv) |
                      reinterpret_cast<uintptr_t>(mi.X)) & 15) == 0;
-  float a[8][8];
   if (LOOK) {
-    // the block with step - 1's update applied comes out of the look-ahead
-    // in shared memory (aliasing Lt, which is written only after the
-    // Cholesky sweep's barriers)
-    float* Sa = dsm;
+    // the operand stages alias everything behind S, which is written only
+    // after the look-ahead's last barrier
     unsigned char* stage = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(dsm + kDiagBaseFloats) + 1023) &
+        (reinterpret_cast<uintptr_t>(dsm + DB * DLD) + 1023) &
         ~(uintptr_t)1023);
     LookControl* ctl = reinterpret_cast<LookControl*>(stage + 2 * kLookStage);
-    if (!diag_lookahead(mi, o, bs, Sa, stage, ctl)) return;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int gi = 8 * br + i;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int gj = 8 * bc + j;
-        float v = (gi == gj) ? 1.f : 0.f;
-        if (gi < bs && gj <= gi) v = Sa[gi * DLD + gj];
-        a[i][j] = v;
-      }
-    }
+    if (!diag_lookahead(mi, o, bs, vec, sm.S, stage, ctl)) return;
+  } else {
+    diag_load(mi.W + (long long)o * ld + o, ld, bs, vec, sm.S);
+    diag_load_wait();
     __syncthreads();
-  } else
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gi = 8 * br + i;
-    if (vec && bc < br && gi < bs) {
-      const float4 v0 = *reinterpret_cast<const float4*>(&Wd[gi * ld + 8 * bc]);
-      const float4 v1 = *reinterpret_cast<const float4*>(&Wd[gi * ld + 8 * bc + 4]);
-      a[i][0] = v0.x; a[i][1] = v0.y; a[i][2] = v0.z; a[i][3] = v0.w;
-      a[i][4] = v1.x; a[i][5] = v1.y; a[i][6] = v1.z; a[i][7] = v1.w;
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int gj = 8 * bc + j;
-        float v = (gi == gj) ? 1.f : 0.f;        // identity beyond the block
-        if (gi < bs && gj <= gi) v = Wd[gi * ld + gj];
-        a[i][j] = v;
-      }
-    }
   }
 
-  // ---- Cholesky by block columns
-  for (int kb = 0; kb < nkb; ++kb) {
-    if (br == kb && bc == kb) {
-      // 8 x 8 Cholesky in registers; rl[c] = 1 / l_cc
-      float rl[8];
+  for (int p = 0; p < np; ++p) {
+    if (warp == p) {
+      diag_base(sm, p, lane, id, o + SB * p, info);
+    } else if (p > 0) {
+      const int hw = warp < p ? warp : warp - 1;    // 0 .. 14
+      // rest of the update by sub-block column p - 1, 16 x 32 per warp, and
+      // row block p - 1 of the inverse
+      const int nb = np - p;
+      const int rest = nb * (nb + 1) / 2 - 1;
+      if (hw < 2 * rest) {
+        int t = (hw >> 1) + 1, bi = 0;
+        while (t > bi) t -= ++bi;                   // lower sub-block (bi, t)
+        const int r0 = SB * (p + bi) + 16 * (hw & 1), c0 = SB * (p + t);
+        float acc[4][4] = {};
+        diag_mac(&sm.S[r0 * DLD + SB * (p - 1)], DLD,
+                 &sm.S[c0 * DLD + SB * (p - 1)], DLD, lane, acc);
+        float* dst = &sm.S[(r0 + (lane >> 3)) * DLD + c0 + (lane & 7)];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        float piv = a[c][c];
-        if (!(piv > 0.f)) {
-          atomicCAS(&info[id], 0, o + 8 * kb + c + 1);
-          piv = 1.f;
-        }
-        // rsqrt + one Newton step: full fp32 accuracy without the slow IEEE
-        // square root and division
-        float r = rsqrtf(piv);
-        r = r * (1.5f - 0.5f * piv * r * r);
-        rl[c] = r;
-        a[c][c] = piv * r;
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int i = c + 1; i < 8; ++i) a[i][c] *= r;
-#pragma unroll
-        for (int j = c + 1; j < 8; ++j)
-#pragma unroll
-          for (int i = j; i < 8; ++i) a[i][j] = fmaf(-a[i][c], a[j][c], a[i][j]);
+          for (int c = 0; c < 4; ++c) dst[4 * r * DLD + 8 * c] -= acc[r][c];
+      } else if (hw < 2 * rest + 2 * (p - 1)) {
+        const int u = hw - 2 * rest;
+        diag_x_block(sm, p - 1, u >> 1, u & 1, lane);
       }
-      // T = L_kk^-1 (lower), column by column: T[c][c] = rl[c],
-      // T[i][c] = -rl[i] * sum_{m=c}^{i-1} L[i][m] T[m][c]
-      float t[8][8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        t[c][c] = rl[c];
-#pragma unroll
-        for (int i = c + 1; i < 8; ++i) {
-          float acc = 0.f;
-#pragma unroll
-          for (int m = c; m < i; ++m) acc = fmaf(a[i][m], t[m][c], acc);
-          t[i][c] = -rl[i] * acc;
+      asm volatile("bar.sync 1, %0;" ::"n"(DT - 32) : "memory");
+      // T^T of row block p: T^T(j) = sum_k X^T(j, k) L(p, k)^T, j <= k < p
+      if (hw < 2 * p) {
+        const int j = hw >> 1, half = hw & 1;
+        float acc[4][4] = {};
+        for (int k = j; k < p; ++k) {
+          const float* A = k == j ? &sm.XDT[j][16 * half * SLP]
+                                  : &sm.S[(SB * j + 16 * half) * DLD + SB * k];
+          diag_mac(A, k == j ? SLP : DLD, &sm.S[SB * p * DLD + SB * k], DLD,
+                   lane, acc);
         }
-      }
+        float* dst = &sm.TT[(SB * j + 16 * half + (lane >> 3)) * SLP + (lane & 7)];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) Tk[kb][8 * i + j] = (j <= i) ? t[i][j] : 0.f;
-    }
-    __syncthreads();
-    if (bc == kb && br > kb) {
-      // panel solve: L_blk = A_blk T^T, L[i][c] = sum_{m<=c} A[i][m] T[c][m]
-      float t[8][8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 t0 = *reinterpret_cast<const float4*>(&Tk[kb][8 * i]);
-        const float4 t1 = *reinterpret_cast<const float4*>(&Tk[kb][8 * i + 4]);
-        t[i][0] = t0.x; t[i][1] = t0.y; t[i][2] = t0.z; t[i][3] = t0.w;
-        t[i][4] = t1.x; t[i][5] = t1.y; t[i][6] = t1.z; t[i][7] = t1.w;
-      }
-      float l[8][8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          float acc = 0.f;
-#pragma unroll
-          for (int m = 0; m <= c; ++m) acc = fmaf(a[i][m], t[c][m], acc);
-          l[i][c] = acc;
-        }
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        *reinterpret_cast<float4*>(&Pt[c][8 * br]) =
-            make_float4(l[0][c], l[1][c], l[2][c], l[3][c]);
-        *reinterpret_cast<float4*>(&Pt[c][8 * br + 4]) =
-            make_float4(l[4][c], l[5][c], l[6][c], l[7][c]);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) a[i][c] = l[i][c];
+          for (int c = 0; c < 4; ++c) dst[4 * r * SLP + 8 * c] = acc[r][c];
       }
     }
     __syncthreads();
-    if (bc > kb && bc <= br) {
+    if (warp >= p && warp < np) {
+      float a[SB];
+      float* row = &sm.S[(SB * warp + lane) * DLD + SB * p];
+      if (warp == p) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float4 r0 = *reinterpret_cast<const float4*>(&Pt[c][8 * br]);
-        const float4 r1 = *reinterpret_cast<const float4*>(&Pt[c][8 * br + 4]);
-        const float4 c0 = *reinterpret_cast<const float4*>(&Pt[c][8 * bc]);
-        const float4 c1 = *reinterpret_cast<const float4*>(&Pt[c][8 * bc + 4]);
-        const float pr[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-        const float pc[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        for (int j = 0; j < SB; ++j) a[j] = j == lane ? 1.f : 0.f;
+      } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) a[i][j] = fmaf(-pr[i], pc[j], a[i][j]);
+        for (int j = 0; j < SB; j += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(&row[j]);
+          a[j] = v.x; a[j + 1] = v.y; a[j + 2] = v.z; a[j + 3] = v.w;
+        }
       }
+      diag_solve_row(sm, a);
+      if (warp == p) {
+        row = &sm.XDT[p][lane * SLP];
+#pragma unroll
+        for (int j = 0; j < SB; ++j) sm.XD[p][j * SLP + lane] = a[j];
+      }
+#pragma unroll
+      for (int j = 0; j < SB; j += 4)
+        *reinterpret_cast<float4*>(&row[j]) =
+            make_float4(a[j], a[j + 1], a[j + 2], a[j + 3]);
     }
+    __syncthreads();
+    if (p + 1 < np) {
+      // next diagonal sub-block: row per lane, two columns per warp
+      const float* Lr = &sm.S[(SB * (p + 1)) * DLD + SB * p];
+      const int c = 2 * warp;
+      float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+      for (int k = 0; k < SB; k += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(&Lr[lane * DLD + k]);
+        const float4 u = *reinterpret_cast<const float4*>(&Lr[c * DLD + k]);
+        const float4 v = *reinterpret_cast<const float4*>(&Lr[(c + 1) * DLD + k]);
+        s0 = fmaf(x.w, u.w, fmaf(x.z, u.z, fmaf(x.y, u.y, fmaf(x.x, u.x, s0))));
+        s1 = fmaf(x.w, v.w, fmaf(x.z, v.z, fmaf(x.y, v.y, fmaf(x.x, v.x, s1))));
+      }
+      float* dst = &sm.S[(SB * (p + 1) + lane) * DLD + SB * (p + 1) + c];
+      dst[0] -= s0;
+      dst[1] -= s1;
+      __syncthreads();
+    }
+  }
+  if (np > 1) {
+    if (warp < 2 * (np - 1)) diag_x_block(sm, np - 1, warp >> 1, warp & 1, lane);
+    __syncthreads();
   }
 
-  // ---- L to global memory (lower part) and, transposed, to shared memory
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gi = 8 * br + i;
-    if (vec && bc < br && gi < bs) {
-      *reinterpret_cast<float4*>(&Wd[gi * ld + 8 * bc]) =
-          make_float4(a[i][0], a[i][1], a[i][2], a[i][3]);
-      *reinterpret_cast<float4*>(&Wd[gi * ld + 8 * bc + 4]) =
-          make_float4(a[i][4], a[i][5], a[i][6], a[i][7]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int gj = 8 * bc + j;
-        if (gi < bs && gj <= gi) Wd[gi * ld + gj] = a[i][j];
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int gj = 8 * bc + j;
-    float v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = (8 * br + i > gj) ? a[i][j] : 0.f;
-    *reinterpret_cast<float4*>(&Lt[gj][8 * br]) = make_float4(v[0], v[1], v[2], v[3]);
-    *reinterpret_cast<float4*>(&Lt[gj][8 * br + 4]) = make_float4(v[4], v[5], v[6], v[7]);
-  }
-  // ---- inverse of the triangle by block rows: R starts as I; the rows of
-  // block kb become X = T_kb R, every block row below subtracts L_blk X
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) a[i][j] = (8 * br + i == 8 * bc + j) ? 1.f : 0.f;
-  __syncthreads();
-  for (int kb = 0; kb < nkb; ++kb) {
-    const int buf = kb & 1;
-    if (br == kb && bc <= kb) {
-      float t[8][8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 t0 = *reinterpret_cast<const float4*>(&Tk[kb][8 * i]);
-        const float4 t1 = *reinterpret_cast<const float4*>(&Tk[kb][8 * i + 4]);
-        t[i][0] = t0.x; t[i][1] = t0.y; t[i][2] = t0.z; t[i][3] = t0.w;
-        t[i][4] = t1.x; t[i][5] = t1.y; t[i][6] = t1.z; t[i][7] = t1.w;
-      }
-      float x[8][8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float acc = 0.f;
-#pragma unroll
-          for (int m = 0; m <= i; ++m) acc = fmaf(t[i][m], a[m][j], acc);
-          x[i][j] = acc;
-        }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        *reinterpret_cast<float4*>(&Xr[buf][i][8 * bc]) =
-            make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
-        *reinterpret_cast<float4*>(&Xr[buf][i][8 * bc + 4]) =
-            make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) a[i][j] = x[i][j];
-      }
-    }
-    __syncthreads();
-    if (br > kb && bc <= kb) {
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float4 l0 = *reinterpret_cast<const float4*>(&Lt[8 * kb + c][8 * br]);
-        const float4 l1 = *reinterpret_cast<const float4*>(&Lt[8 * kb + c][8 * br + 4]);
-        const float4 x0 = *reinterpret_cast<const float4*>(&Xr[buf][c][8 * bc]);
-        const float4 x1 = *reinterpret_cast<const float4*>(&Xr[buf][c][8 * bc + 4]);
-        const float lc[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-        const float xr[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) a[i][j] = fmaf(-lc[i], xr[j], a[i][j]);
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gi = 8 * br + i;
-    if (vec && bc != br && gi < bs && 8 * bc + 7 < bs) {
-      const bool low = bc < br;
-      *reinterpret_cast<float4*>(&Xd[gi * ld + 8 * bc]) =
-          low ? make_float4(a[i][0], a[i][1], a[i][2], a[i][3])
-              : make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(&Xd[gi * ld + 8 * bc + 4]) =
-          low ? make_float4(a[i][4], a[i][5], a[i][6], a[i][7])
-              : make_float4(0.f, 0.f, 0.f, 0.f);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int gj = 8 * bc + j;
-        if (gi < bs && gj < bs) Xd[gi * ld + gj] = (gj <= gi) ? a[i][j] : 0.f;
-      }
+  // ---- X to global memory: a warp turns 32 columns x 4 rows of X^T (one
+  // 16-byte word per lane) into four contiguous row pieces.  The part above
+  // the diagonal sub-blocks was zeroed when the plan was made.
+  float* Xd = mi.X + (long long)o * ld + o;
+  for (int t = warp; t < np * (np + 1) / 2 * 8; t += DT / 32) {
+    int u = t >> 3, bi = 0;
+    while (u > bi) u -= ++bi;                       // sub-block (bi, u)
+    const int r0 = 4 * (t & 7);
+    const float* src = bi == u ? &sm.XDT[u][lane * SLP + r0]
+                               : &sm.S[(SB * u + lane) * DLD + SB * bi + r0];
+    const float4 v = *reinterpret_cast<const float4*>(src);
+    const int r = SB * bi + r0, c = SB * u + lane;
+    if (c < bs) {
+      if (r < bs) Xd[r * ld + c] = v.x;
+      if (r + 1 < bs) Xd[(r + 1) * ld + c] = v.y;
+      if (r + 2 < bs) Xd[(r + 2) * ld + c] = v.z;
+      if (r + 3 < bs) Xd[(r + 3) * ld + c] = v.w;
     }
   }
 }
@@ -851,11 +916,12 @@ refine_apply_kernel(const MatInfo* __restrict__ mats,
     inv[i] += it.Y[i];
 }
 
-constexpr size_t kDiagSmemBytes =
-    kDiagBaseFloats * sizeof(float);                        // Lt, Pt, Xr, Tk
+constexpr size_t kDiagSmemBytes = sizeof(DiagSmem);
 constexpr size_t kDiagLookSmemBytes =
-    kDiagBaseFloats * sizeof(float) + 1024 + 2 * kLookStage + 256;
-static_assert(kDiagLookSmemBytes <= 227 * 1024, "diagonal kernel shared memory");
+    DB * DLD * sizeof(float) + 1024 + 2 * kLookStage + 256;
+static_assert(kDiagLookSmemBytes >= kDiagSmemBytes &&
+                  kDiagLookSmemBytes <= 227 * 1024,
+              "diagonal kernel shared memory");
 
 struct Launch {
   int tails;     // grouped gemm: some contraction is not a multiple of 32
@@ -1406,10 +1472,10 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
       KFAC_CUDA(cudaStreamWaitEvent(st, p->events[l.wait_ev2], 0));
     if (l.kind == 0) {
       if (l.look)
-        chol_diag_kernel<true><<<l.n, 256, kDiagLookSmemBytes, st>>>(
+        chol_diag_kernel<true><<<l.n, DT, kDiagLookSmemBytes, st>>>(
             p->mats_dev, p->ids_dev + l.off, l.step, info);
       else
-        chol_diag_kernel<false><<<l.n, 256, kDiagSmemBytes, st>>>(
+        chol_diag_kernel<false><<<l.n, DT, kDiagSmemBytes, st>>>(
             p->mats_dev, p->ids_dev + l.off, l.step, info);
       KFAC_LAUNCH_CHECK("chol_diag_kernel");
     } else {
