@@ -32,6 +32,7 @@ struct MatInfo {
   float l2;
   float scale;
   float l2b;      // role 2: floor of the second half of the diagonal
+  int id;         // index of the matrix in the plan
 };
 
 // Per-run arguments, kept in device memory so that a captured CUDA graph of
@@ -245,6 +246,25 @@ __device__ __forceinline__ void diag_load_wait() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// Barriers and tensor memory of the look-ahead; needs nothing of the matrix.
+__device__ __forceinline__ void look_begin(LookControl* ctl) {
+  if (threadIdx.x == 32) {
+    mbar_init(&ctl->bar[0], 1);
+    mbar_init(&ctl->bar[1], 1);
+    mbar_init(&ctl->done, 1);
+    ctl->abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 32) {
+    asm volatile(
+        "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+        ::"r"(smem_u32(&ctl->tmem_base)), "r"(kLookCols)
+        : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
+                 ::: "memory");
+  }
+}
+
 // The diagonal block of step k has received the updates of all steps before
 // k - 1; the update of step k - 1,
 //   D = W_kk - L' L'^T,  L' = A' X_pp^T,
@@ -285,21 +305,6 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
   }
   // W_kk into S (the update is subtracted from it at the end)
   diag_load(mi.W + (long long)o * ld + o, ld, bs, vec, S);
-  if (tid == 0) {
-    mbar_init(&ctl->bar[0], 1);
-    mbar_init(&ctl->bar[1], 1);
-    mbar_init(&ctl->done, 1);
-    ctl->abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 0) {
-    asm volatile(
-        "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-        ::"r"(smem_u32(&ctl->tmem_base)), "r"(kLookCols)
-        : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
-                 ::: "memory");
-  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -412,295 +417,427 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
 
 // ------------------------------------------------ one 128 x 128 diagonal block
 // Shared memory of the diagonal kernel, in floats.
+constexpr int LSP = SB + 16;   // row pitch of Ls (reads run past the last column)
 struct DiagSmem {
   float S[DB * DLD];          // D / L in the sub-blocks on and below the
                               // diagonal, X^T in those above it
-  float XDT[4][SB * SLP];     // inverse of sub-block p of the diagonal, transposed
-  float XD[4][SB * SLP];      // the same, row-major
-  float TT[3 * SB * SLP];     // T^T of the running block row
-  float LT[SB * SLP];         // L_pp, transposed
+  float XD[4][SB * SLP];      // X_pp^T: inverse of sub-block p of the diagonal
+  float Ls[SB][LSP];          // L_pp by columns
   float rl[SB];               // 1 / l_cc
-  float4 Lp[2][SB];           // four columns of L_pp on their way to the warp
+  float pv[SB][8];            // the running step's eight columns
 };
 
-// r = 1 / sqrt(q) by the approximation and one Newton step: full fp32 accuracy
-// without the IEEE square root and division.  A pivot that is not positive
-// (or below the smallest normal number) counts as failed and becomes 1.
-__device__ __forceinline__ float pivot_rsqrt(float q, bool& bad) {
-  bad = !(q >= 1.17549435e-38f);
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Named barriers of the diagonal kernel.
+constexpr int kBarStep = 1;    // + step: eight columns of L_pp are in Ls
+constexpr int kRestWarps = 4; // warps of diag_base_rest
+constexpr int kBarNext = 4;    // + step (1, 2): the columns after the next are
+constexpr int kBarDiag = 7;    // the next diagonal sub-block is up to date
+constexpr int kBarRows = 8;    // so are the rows that follow it
+
+// Pivot k of an 8 x 8 block: r = 1 / sqrt(q) by the approximation and one
+// Newton step (full fp32 accuracy without the IEEE square root and division);
+// `next`, if given, becomes p / sqrt(q) without waiting for r.  CHECK: a pivot
+// that is not positive (or below the smallest normal number) counts as failed
+// and becomes 1.
+template <bool CHECK>
+__device__ __forceinline__ float diag_pivot(float q, float* next) {
+  if (CHECK && !(q >= 1.17549435e-38f)) return 1.f;
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q));
-  r = r * fmaf(-0.5f * q, r * r, 1.5f);
-  return bad ? 1.f : r;
+  const float e = fmaf(-(q * r), r, 1.f);
+  if (next != nullptr) {
+    const float g = *next * r;
+    *next = fmaf(0.5f * g, e, g);
+  }
+  return fmaf(0.5f * r, e, r);
 }
 
-// Cholesky factor of sub-block p of the diagonal by one warp, a row per lane in
-// registers, four columns per step: every lane factors the 4 x 4 pivot block
-// redundantly (ten shuffles fetch it), so the serial chain per column is one
-// reciprocal square root and two multiply-adds, and the rank-4 update reads
-// the other rows' four values as one broadcast 16-byte word each.
+// Cholesky factor of the 8 x 8 block p (lower part, in place), r = reciprocal
+// square roots of the pivots.
+template <bool CHECK>
+__device__ __forceinline__ void diag_chol8(float p[8][8], float r[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    float l = k < 7 ? p[k + 1][k] : 0.f;
+    r[k] = diag_pivot<CHECK>(p[k][k], k < 7 ? &l : nullptr);
+    if (k == 7) break;
+    p[k + 1][k] = CHECK ? p[k + 1][k] * r[k] : l;
+#pragma unroll
+    for (int i = k + 2; i < 8; ++i) p[i][k] *= r[k];
+#pragma unroll
+    for (int j = k + 1; j < 8; ++j)
+#pragma unroll
+      for (int i = j; i < 8; ++i) p[i][j] = fmaf(-p[i][k], p[j][k], p[i][j]);
+  }
+}
+
+// Row (a0 .. a7) of the step's eight columns through the 8 x 8 triangle:
+// l(i, k) gives L[i][k].
+template <typename F>
+__device__ __forceinline__ void diag_solve8(float x[8], const float r[8], F l) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    float v = x[k];
+#pragma unroll
+    for (int m = 0; m < k; ++m) v = fmaf(-x[m], l(k, m), v);
+    x[k] = v * r[k];
+  }
+}
+
+// The pivot block of the running step (lower part) into every lane.
+__device__ __forceinline__ void diag_load8(const DiagSmem& sm, int j,
+                                           float blk[8][8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int k = 0; k <= i; k += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(&sm.pv[j + i][k]);
+      blk[i][k] = v.x; blk[i][k + 1] = v.y;
+      blk[i][k + 2] = v.z; blk[i][k + 3] = v.w;
+    }
+}
+
+// Cholesky factor of sub-block p of the diagonal by one warp, a row per lane,
+// eight columns per step in registers.  Every lane factors the 8 x 8 pivot
+// block redundantly (fetched through shared memory: 36 shuffles measured 300
+// cycles more), so that the serial chain per column is one reciprocal square
+// root and a few multiply-adds, and the trip through shared memory that brings
+// the columns to the other rows comes once in eight columns.  Of a step's
+// rank-8 update this warp applies only the part on the next eight columns; the
+// columns after those are updated by other warps (diag_base_rest) meanwhile.
 __device__ __forceinline__ void diag_base(DiagSmem& sm, int p, int lane, int id,
-                                          int col0, int* info) {
-  float a[SB];
+                                          int col0, int followers, int* info) {
+  const float4* row = reinterpret_cast<const float4*>(
+      &sm.S[(SB * p + lane) * DLD + SB * p]);
+  float x[8];
+  float4 u = row[0], v = row[1];
+#pragma unroll 1
+  for (int s = 0; s < 4; ++s) {
+    const int j = 8 * s;
+    float blk[8][8], r[8];
+    float4* pv = reinterpret_cast<float4*>(sm.pv[lane]);
+    pv[0] = u;
+    pv[1] = v;
+    __syncwarp();
+    diag_load8(sm, j, blk);
+    diag_chol8<false>(blk, r);
+    if (!(r[7] == r[7])) {
+      // some pivot is not positive (every later one is NaN then): report the
+      // first, carry on with ones in their place
+      diag_load8(sm, j, blk);
+      diag_chol8<true>(blk, r);
+      int first = 0;
 #pragma unroll
-  for (int j = 0; j < SB / 4; ++j) {
-    const float4 v = *reinterpret_cast<const float4*>(
-        &sm.S[(SB * p + lane) * DLD + SB * p + 4 * j]);
-    a[4 * j] = v.x; a[4 * j + 1] = v.y; a[4 * j + 2] = v.z; a[4 * j + 3] = v.w;
-  }
-  int first = 0;
-#pragma unroll
-  for (int s = 0; s < SB / 4; ++s) {
-    const int j = 4 * s;
-    const unsigned all = 0xffffffffu;
-    const float p00 = __shfl_sync(all, a[j], j);
-    const float p10 = __shfl_sync(all, a[j], j + 1);
-    const float p11 = __shfl_sync(all, a[j + 1], j + 1);
-    const float p20 = __shfl_sync(all, a[j], j + 2);
-    const float p21 = __shfl_sync(all, a[j + 1], j + 2);
-    const float p22 = __shfl_sync(all, a[j + 2], j + 2);
-    const float p30 = __shfl_sync(all, a[j], j + 3);
-    const float p31 = __shfl_sync(all, a[j + 1], j + 3);
-    const float p32 = __shfl_sync(all, a[j + 2], j + 3);
-    const float p33 = __shfl_sync(all, a[j + 3], j + 3);
-    bool b0, b1, b2, b3;
-    const float r0 = pivot_rsqrt(p00, b0);
-    const float l10 = p10 * r0, l20 = p20 * r0, l30 = p30 * r0;
-    const float r1 = pivot_rsqrt(fmaf(-l10, l10, p11), b1);
-    const float l21 = fmaf(-l20, l10, p21) * r1;
-    const float l31 = fmaf(-l30, l10, p31) * r1;
-    const float r2 = pivot_rsqrt(fmaf(-l21, l21, fmaf(-l20, l20, p22)), b2);
-    const float l32 = fmaf(-l31, l21, fmaf(-l30, l20, p32)) * r2;
-    const float r3 = pivot_rsqrt(
-        fmaf(-l32, l32, fmaf(-l31, l31, fmaf(-l30, l30, p33))), b3);
-    if (first == 0) {
-      if (b0) first = j + 1;
-      else if (b1) first = j + 2;
-      else if (b2) first = j + 3;
-      else if (b3) first = j + 4;
+      for (int k = 7; k >= 0; --k)
+        if (!(blk[k][k] >= 1.17549435e-38f)) first = j + k + 1;
+      if (lane == 0 && first != 0) atomicCAS(&info[id], 0, col0 + first);
     }
-    // this lane's row of the four columns (rows above the pivot: unused)
-    const float x0 = a[j] * r0;
-    const float x1 = fmaf(-x0, l10, a[j + 1]) * r1;
-    const float x2 = fmaf(-x1, l21, fmaf(-x0, l20, a[j + 2])) * r2;
-    const float x3 =
-        fmaf(-x2, l32, fmaf(-x1, l31, fmaf(-x0, l30, a[j + 3]))) * r3;
-    if (s + 1 < SB / 4) {
-      sm.Lp[s & 1][lane] = make_float4(x0, x1, x2, x3);
-      __syncwarp();
+    // this lane's row (rows above the pivot: unused)
+    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+    x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+    diag_solve8(x, r, [&](int i, int k) { return blk[i][k]; });
+    float (*L)[LSP] = &sm.Ls[j];
 #pragma unroll
-      for (int c = j + 4; c < SB; ++c) {
-        const float4 v = sm.Lp[s & 1][c];
-        a[c] = fmaf(-x3, v.w, fmaf(-x2, v.z, fmaf(-x1, v.y, fmaf(-x0, v.x, a[c]))));
+    for (int k = 0; k < 8; ++k) L[k][lane] = x[k];
+    // (every lane stores the same)
+    *reinterpret_cast<float4*>(&sm.rl[j]) = make_float4(r[0], r[1], r[2], r[3]);
+    *reinterpret_cast<float4*>(&sm.rl[j + 4]) = make_float4(r[4], r[5], r[6], r[7]);
+    __syncwarp();
+    bar_arrive(kBarStep + s, followers + (s < 2 ? 32 * kRestWarps : 0));
+    if (s == 3) break;
+    if (s > 0) bar_sync(kBarNext + s, 32 + 32 * kRestWarps);
+    u = row[2 * s + 2];
+    v = row[2 * s + 3];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float4 l = *reinterpret_cast<const float4*>(&L[k][j + 8]);
+      const float4 m = *reinterpret_cast<const float4*>(&L[k][j + 12]);
+      u.x = fmaf(-x[k], l.x, u.x); u.y = fmaf(-x[k], l.y, u.y);
+      u.z = fmaf(-x[k], l.z, u.z); u.w = fmaf(-x[k], l.w, u.w);
+      v.x = fmaf(-x[k], m.x, v.x); v.y = fmaf(-x[k], m.y, v.y);
+      v.z = fmaf(-x[k], m.z, v.z); v.w = fmaf(-x[k], m.w, v.w);
+    }
+  }
+}
+
+// The part of diag_base's updates that its own warp leaves: step s on columns
+// 8 s + 16 .. 31 of the sub-block, in shared memory, four columns per warp.
+__device__ __forceinline__ void diag_base_rest(DiagSmem& sm, int p, int lane,
+                                               int h, int followers) {
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+    bar_sync(kBarStep + s, followers + 32 * kRestWarps);
+    const int c = 8 * s + 16 + 4 * h;
+    if (c < SB) {
+      const float (*L)[LSP] = &sm.Ls[8 * s];
+      float4* row = reinterpret_cast<float4*>(
+          &sm.S[(SB * p + lane) * DLD + SB * p + c]);
+      float4 u = *row;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float x = L[k][lane];
+        const float4 l = *reinterpret_cast<const float4*>(&L[k][c]);
+        u.x = fmaf(-x, l.x, u.x); u.y = fmaf(-x, l.y, u.y);
+        u.z = fmaf(-x, l.z, u.z); u.w = fmaf(-x, l.w, u.w);
       }
+      *row = u;
+      __syncwarp();
     }
-    sm.LT[j * SLP + lane] = x0;
-    sm.LT[(j + 1) * SLP + lane] = x1;
-    sm.LT[(j + 2) * SLP + lane] = x2;
-    sm.LT[(j + 3) * SLP + lane] = x3;
-    if (lane == 0)
-      *reinterpret_cast<float4*>(&sm.rl[j]) = make_float4(r0, r1, r2, r3);
-  }
-  if (first != 0 && lane == 0)
-    atomicCAS(&info[id], 0, col0 + first);
-}
-
-// a <- a L_pp^-T for one row per thread (right-looking substitution): the rows
-// of L below sub-block p, or, started from a unit vector, a column of X_pp.
-__device__ __forceinline__ void diag_solve_row(const DiagSmem& sm, float a[SB]) {
-  float4 rl;
-#pragma unroll
-  for (int c = 0; c < SB; ++c) {
-    if ((c & 3) == 0) rl = *reinterpret_cast<const float4*>(&sm.rl[c]);
-    const float r = (c & 3) == 0 ? rl.x : (c & 3) == 1 ? rl.y
-                    : (c & 3) == 2 ? rl.z : rl.w;
-    const float x = a[c] * r;
-    a[c] = x;
-#pragma unroll
-    for (int g = (c + 1) >> 2; g < SB / 4; ++g) {
-      const float4 v = *reinterpret_cast<const float4*>(&sm.LT[c * SLP + 4 * g]);
-      if (4 * g > c) a[4 * g] = fmaf(-x, v.x, a[4 * g]);
-      if (4 * g + 1 > c) a[4 * g + 1] = fmaf(-x, v.y, a[4 * g + 1]);
-      if (4 * g + 2 > c) a[4 * g + 2] = fmaf(-x, v.z, a[4 * g + 2]);
-      a[4 * g + 3] = fmaf(-x, v.w, a[4 * g + 3]);
-    }
+    bar_arrive(kBarNext + s + 1, 32 + 32 * kRestWarps);
   }
 }
 
-// acc(16 x 32) += A B^T over 32 k, one warp: A 16 rows, B 32 rows, both
-// contiguous along k with the given row pitches.  Lane (rg, cg) = (lane / 8,
-// lane % 8) holds rows rg + 4 i, columns cg + 8 j: the 16-byte loads of a
-// quarter warp fall into different banks.
-__device__ __forceinline__ void diag_mac(const float* A, int pa, const float* B,
-                                         int pb, int lane, float acc[4][4]) {
-  const float* ar = A + (lane >> 3) * pa;
-  const float* br = B + (lane & 7) * pb;
-#pragma unroll 4
+template <int NC>
+__device__ __forceinline__ void diag_follow_step(const DiagSmem& sm, int s,
+                                                 float a[2][SB], float* row0,
+                                                 float* row1) {
+  const int j = 8 * s;
+  const float (*L)[LSP] = &sm.Ls[j];
+  float r[8], l[8][8], x[2][8];
+#pragma unroll
+  for (int k = 0; k < 8; k += 4) {
+    const float4 v = *reinterpret_cast<const float4*>(&sm.rl[j + k]);
+    r[k] = v.x; r[k + 1] = v.y; r[k + 2] = v.z; r[k + 3] = v.w;
+  }
+#pragma unroll
+  for (int k = 0; k < 7; ++k)
+#pragma unroll
+    for (int i = 0; i < 8; i += 4) {
+      if (i + 3 <= k) continue;
+      const float4 v = *reinterpret_cast<const float4*>(&L[k][j + i]);
+      l[i][k] = v.x; l[i + 1][k] = v.y; l[i + 2][k] = v.z; l[i + 3][k] = v.w;
+    }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[q][k] = a[q][k];
+    diag_solve8(x[q], r, [&](int i, int k) { return l[i][k]; });
+    float4* row = reinterpret_cast<float4*>(&(q ? row1 : row0)[j]);
+    row[0] = make_float4(x[q][0], x[q][1], x[q][2], x[q][3]);
+    row[1] = make_float4(x[q][4], x[q][5], x[q][6], x[q][7]);
+  }
+  // the registers move down by eight columns
+#pragma unroll
+  for (int c = 0; c < NC; c += 4) {
+    float4 u = make_float4(a[0][c + 8], a[0][c + 9], a[0][c + 10], a[0][c + 11]);
+    float4 v = make_float4(a[1][c + 8], a[1][c + 9], a[1][c + 10], a[1][c + 11]);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float4 w = *reinterpret_cast<const float4*>(&L[k][j + 8 + c]);
+      u.x = fmaf(-x[0][k], w.x, u.x); v.x = fmaf(-x[1][k], w.x, v.x);
+      u.y = fmaf(-x[0][k], w.y, u.y); v.y = fmaf(-x[1][k], w.y, v.y);
+      u.z = fmaf(-x[0][k], w.z, u.z); v.z = fmaf(-x[1][k], w.z, v.z);
+      u.w = fmaf(-x[0][k], w.w, u.w); v.w = fmaf(-x[1][k], w.w, v.w);
+    }
+    a[0][c] = u.x; a[0][c + 1] = u.y; a[0][c + 2] = u.z; a[0][c + 3] = u.w;
+    a[1][c] = v.x; a[1][c + 1] = v.y; a[1][c + 2] = v.z; a[1][c + 3] = v.w;
+  }
+}
+
+// row <- row L_pp^-T for two rows per lane, step by step behind diag_base.
+// `unit0` / `unit1`: the row starts as the unit vector e_lane and ends as row
+// `lane` of X_pp^T.
+__device__ __forceinline__ void diag_follow(const DiagSmem& sm, int lane,
+                                            int followers, float* row0,
+                                            float* row1, bool unit0,
+                                            bool unit1) {
+  float a[2][SB];
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int j = 0; j < SB; j += 4) {
+      float4 v = make_float4(j == lane ? 1.f : 0.f, j + 1 == lane ? 1.f : 0.f,
+                             j + 2 == lane ? 1.f : 0.f, j + 3 == lane ? 1.f : 0.f);
+      if (!(q ? unit1 : unit0))
+        v = *reinterpret_cast<const float4*>(&(q ? row1 : row0)[j]);
+      a[q][j] = v.x; a[q][j + 1] = v.y; a[q][j + 2] = v.z; a[q][j + 3] = v.w;
+    }
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+    bar_sync(kBarStep + s, followers + 32 * kRestWarps);
+    diag_follow_step<24>(sm, s, a, row0, row1);
+  }
+#pragma unroll 1
+  for (int s = 2; s < 4; ++s) {
+    bar_sync(kBarStep + s, followers);
+    diag_follow_step<8>(sm, s, a, row0, row1);
+  }
+}
+
+// C(8 RI x ..) -= A B^T over 32 k by one warp: lane (rg, cg) holds rows
+// rg + RG i, columns cg + CG j (RG CG = 32); A and B are contiguous along k.
+// The 16-byte loads of a quarter warp fall into different banks.  `fresh`: C
+// starts from zero.
+template <int RG, int RI, int CJ>
+__device__ __forceinline__ void diag_mac(float* C, const float* A, int pa,
+                                         const float* B, int lane, bool fresh) {
+  constexpr int CG = 32 / RG;
+  const int rg = lane / CG, cg = lane % CG;
+  const float* ar = A + rg * pa;
+  const float* br = B + cg * DLD;
+  float acc[RI][CJ];
+#pragma unroll
+  for (int i = 0; i < RI; ++i)
+#pragma unroll
+    for (int j = 0; j < CJ; ++j) acc[i][j] = 0.f;
+#pragma unroll 2
   for (int k = 0; k < SB; k += 4) {
-    float4 av[4], bv[4];
+    float av[RI][4], bv[CJ][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      av[i] = *reinterpret_cast<const float4*>(&ar[4 * i * pa + k]);
-      bv[i] = *reinterpret_cast<const float4*>(&br[8 * i * pb + k]);
+    for (int i = 0; i < RI; ++i) {
+      const float4 v = *reinterpret_cast<const float4*>(&ar[RG * i * pa + k]);
+      av[i][0] = v.x; av[i][1] = v.y; av[i][2] = v.z; av[i][3] = v.w;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < CJ; ++j) {
+      const float4 v = *reinterpret_cast<const float4*>(&br[CG * j * DLD + k]);
+      bv[j][0] = v.x; bv[j][1] = v.y; bv[j][2] = v.z; bv[j][3] = v.w;
+    }
+    // (consecutive multiply-adds go to different accumulators)
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        acc[i][j] = fmaf(av[i].w, bv[j].w, fmaf(av[i].z, bv[j].z,
-                    fmaf(av[i].y, bv[j].y, fmaf(av[i].x, bv[j].x, acc[i][j]))));
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int j = 0; j < CJ; ++j)
+#pragma unroll
+        for (int i = 0; i < RI; ++i)
+          acc[i][j] = fmaf(av[i][e], bv[j][e], acc[i][j]);
   }
+  float* dst = C + rg * DLD + cg;
+#pragma unroll
+  for (int i = 0; i < RI; ++i)
+#pragma unroll
+    for (int j = 0; j < CJ; ++j) {
+      const float v = fresh ? 0.f : dst[RG * i * DLD + CG * j];
+      dst[RG * i * DLD + CG * j] = v - acc[i][j];
+    }
 }
 
-// Row block i of the inverse left of its diagonal sub-block, transposed:
-// X^T(j, i) = -T^T X_ii^T for sub-block j < i; `half`: its upper or lower 16
-// rows.  One warp.
-__device__ __forceinline__ void diag_x_block(DiagSmem& sm, int i, int j,
-                                             int half, int lane) {
-  float acc[4][4] = {};
-  diag_mac(&sm.TT[(SB * j + 16 * half) * SLP], SLP, sm.XD[i], SLP, lane, acc);
-  float* dst = &sm.S[(SB * j + 16 * half + (lane >> 3)) * DLD + SB * i +
-                     (lane & 7)];
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) dst[4 * r * DLD + 8 * c] = -acc[r][c];
+// Row-block r of column c of the working matrix loses its product with row c
+// of column p: r > c are rows of the block, r < c (r <= p) rows of X^T.
+// `half`: its upper or lower 16 rows.
+__device__ __forceinline__ void diag_update_block(DiagSmem& sm, int r, int half,
+                                                  int c, int p, int lane) {
+  const float* A = r == p ? &sm.XD[p][16 * half * SLP]
+                          : &sm.S[(SB * r + 16 * half) * DLD + SB * p];
+  diag_mac<8, 2, 8>(&sm.S[(SB * r + 16 * half) * DLD + SB * c], A,
+                    r == p ? SLP : DLD, &sm.S[SB * c * DLD + SB * p], lane,
+                    r == p);
 }
 
 // Factor one diagonal block (<= 128 x 128) of W and invert the resulting
 // triangle: X_kk <- L_kk^-1 (lower part; nothing reads L_kk itself).  One CTA
 // of 16 warps per matrix that still has a block at `step`.
 //
-// The block is swept in four sub-blocks of 32 columns.  Bound: the serial
-// chain of 128 pivots, so everything else is kept off it.  Per sub-block p,
-// one warp factors the 32 x 32 diagonal (diag_base); the rows below it (one
-// thread each) and, with unit vectors as input, the columns of its inverse
-// follow by substitution in other warps; the next diagonal sub-block is
-// updated by all warps, and while it is being factored the remaining warps
-// finish the update of the sub-blocks behind it and the off-diagonal part of
-// the inverse (row block p of X: T = L(p, <p) X(<p, <p) does not need X_pp).
-// 128 x 128 block, measured with the look-ahead: see the table at the plan.
+// Elimination of [D; I] by four sub-blocks of 32 columns: row-blocks in play at
+// sub-block p are p .. 3 of D and 0 .. p of X^T (which starts as I).  Bound:
+// the serial chain of 128 pivots.  So per sub-block one warp runs the pivot
+// chain alone (diag_base), two warps carry the other four row-blocks behind
+// it, two rows per lane (diag_follow), and the product of the finished column
+// with the next one is split: its diagonal sub-block first (six warps, then
+// the chain goes on), the rows that follow it (six warps, then the followers
+// go on), and the columns beyond next to the next chain.  Warps are placed so
+// that the chain has its scheduler to itself.
 template <bool LOOK>
 __global__ void __launch_bounds__(DT, 1)
-chol_diag_kernel(const MatInfo* __restrict__ mats, const int* __restrict__ ids,
-                 int step, int* __restrict__ info) {
+chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
+                 int* __restrict__ info) {
   extern __shared__ __align__(16) float dsm[];
   DiagSmem& sm = *reinterpret_cast<DiagSmem*>(dsm);
-  const int id = ids[blockIdx.x];
-  const MatInfo mi = mats[id];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // the operand stages of the look-ahead alias everything behind S, which is
+  // written only after its last barrier
+  unsigned char* stage = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(dsm + DB * DLD) + 1023) & ~(uintptr_t)1023);
+  LookControl* ctl = reinterpret_cast<LookControl*>(stage + 2 * kLookStage);
+  if (LOOK) look_begin(ctl);
+  const MatInfo mi = mats[blockIdx.x];
+  const int id = mi.id;
   const int o = step * DB;
   const int bs = min(DB, mi.d - o);
   const int np = (bs + SB - 1) / SB;      // sub-blocks in use
   const long long ld = mi.d;
-  const bool vec = (ld & 3) == 0 && (o & 3) == 0 &&
+  const bool vec = (ld & 3) == 0 &&
                    ((reinterpret_cast<uintptr_t>(mi.W) |
                      reinterpret_cast<uintptr_t>(mi.inv) |
                      reinterpret_cast<uintptr_t>(mi.X)) & 15) == 0;
   if (LOOK) {
-    // the operand stages alias everything behind S, which is written only
-    // after the look-ahead's last barrier
-    unsigned char* stage = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(dsm + DB * DLD) + 1023) &
-        ~(uintptr_t)1023);
-    LookControl* ctl = reinterpret_cast<LookControl*>(stage + 2 * kLookStage);
     if (!diag_lookahead(mi, o, bs, vec, sm.S, stage, ctl)) return;
   } else {
     diag_load(mi.W + (long long)o * ld + o, ld, bs, vec, sm.S);
     diag_load_wait();
-    __syncthreads();
   }
+  __syncthreads();
 
+  const int followers = 32 * (1 + (np + 1) / 2);   // threads of a step barrier
+  // roles: 0 chain; 3, 13 .. 15 the rest of its updates; 1, 2 followers;
+  // 5 6 7 9 10 11 rows and columns behind them; 3, 12 .. 15 the diagonal
+  // sub-block, with 0
+  const bool diag_warp = warp == 0 || warp == 3 || warp >= 12;
+  const bool work_warp = warp >= 5 && warp <= 11 && warp != 8;
+  const int worker = warp < 8 ? warp - 5 : warp - 6;            // 0 .. 5
   for (int p = 0; p < np; ++p) {
-    if (warp == p) {
-      diag_base(sm, p, lane, id, o + SB * p, info);
-    } else if (p > 0) {
-      const int hw = warp < p ? warp : warp - 1;    // 0 .. 14
-      // rest of the update by sub-block column p - 1, 16 x 32 per warp, and
-      // row block p - 1 of the inverse
-      const int nb = np - p;
-      const int rest = nb * (nb + 1) / 2 - 1;
-      if (hw < 2 * rest) {
-        int t = (hw >> 1) + 1, bi = 0;
-        while (t > bi) t -= ++bi;                   // lower sub-block (bi, t)
-        const int r0 = SB * (p + bi) + 16 * (hw & 1), c0 = SB * (p + t);
-        float acc[4][4] = {};
-        diag_mac(&sm.S[r0 * DLD + SB * (p - 1)], DLD,
-                 &sm.S[c0 * DLD + SB * (p - 1)], DLD, lane, acc);
-        float* dst = &sm.S[(r0 + (lane >> 3)) * DLD + c0 + (lane & 7)];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) dst[4 * r * DLD + 8 * c] -= acc[r][c];
-      } else if (hw < 2 * rest + 2 * (p - 1)) {
-        const int u = hw - 2 * rest;
-        diag_x_block(sm, p - 1, u >> 1, u & 1, lane);
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(DT - 32) : "memory");
-      // T^T of row block p: T^T(j) = sum_k X^T(j, k) L(p, k)^T, j <= k < p
-      if (hw < 2 * p) {
-        const int j = hw >> 1, half = hw & 1;
-        float acc[4][4] = {};
-        for (int k = j; k < p; ++k) {
-          const float* A = k == j ? &sm.XDT[j][16 * half * SLP]
-                                  : &sm.S[(SB * j + 16 * half) * DLD + SB * k];
-          diag_mac(A, k == j ? SLP : DLD, &sm.S[SB * p * DLD + SB * k], DLD,
-                   lane, acc);
+    if (p > 0) {
+      // product of sub-block column p - 1 with column p (this panel) ...
+      if (diag_warp) {
+        // lower 16 x 16 quadrants (0,0) (1,0) (1,1), 8 rows per warp
+        const int u = warp == 0 ? 0 : warp == 3 ? 1 : warp - 10;
+        const int r = (u < 2 ? 0 : 16) + 8 * (u & 1), c = u < 4 ? 0 : 16;
+        const int base = SB * p * DLD + SB * (p - 1);
+        diag_mac<4, 2, 2>(&sm.S[(SB * p + r) * DLD + SB * p + c],
+                          &sm.S[base + r * DLD], DLD, &sm.S[base + c * DLD],
+                          lane, false);
+        bar_sync(kBarDiag, 6 * 32);
+      } else if (work_warp || warp == 1 || warp == 2) {
+        if (work_warp && worker < 2 * (np - 1)) {
+          const int q = worker >> 1;         // rows below, then rows of X^T
+          const int r = q < np - 1 - p ? p + 1 + q : q - (np - 1 - p);
+          diag_update_block(sm, r, worker & 1, p, p - 1, lane);
         }
-        float* dst = &sm.TT[(SB * j + 16 * half + (lane >> 3)) * SLP + (lane & 7)];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) dst[4 * r * SLP + 8 * c] = acc[r][c];
+        bar_sync(kBarRows, 8 * 32);
       }
     }
-    __syncthreads();
-    if (warp >= p && warp < np) {
-      float a[SB];
-      float* row = &sm.S[(SB * warp + lane) * DLD + SB * p];
-      if (warp == p) {
+    if (warp == 0) {
+      diag_base(sm, p, lane, id, o + SB * p, followers, info);
+    } else if (warp == 3 || warp >= 13) {
+      diag_base_rest(sm, p, lane, warp == 3 ? 3 : warp - 13, followers);
+    } else if (warp <= 2) {
+      const int q = 2 * (warp - 1);
+      if (q < np) {
+        float* row[2];
+        bool unit[2];
 #pragma unroll
-        for (int j = 0; j < SB; ++j) a[j] = j == lane ? 1.f : 0.f;
-      } else {
-#pragma unroll
-        for (int j = 0; j < SB; j += 4) {
-          const float4 v = *reinterpret_cast<const float4*>(&row[j]);
-          a[j] = v.x; a[j + 1] = v.y; a[j + 2] = v.z; a[j + 3] = v.w;
+        for (int e = 0; e < 2; ++e) {
+          // rows below, then rows 0 .. p of X^T (an odd last one twice)
+          const int f = min(q + e, np - 1);
+          const int r = f < np - 1 - p ? p + 1 + f : f - (np - 1 - p);
+          unit[e] = r == p;
+          row[e] = unit[e] ? &sm.XD[p][lane * SLP]
+                           : &sm.S[(SB * r + lane) * DLD + SB * p];
         }
+        diag_follow(sm, lane, followers, row[0], row[1], unit[0], unit[1]);
       }
-      diag_solve_row(sm, a);
-      if (warp == p) {
-        row = &sm.XDT[p][lane * SLP];
-#pragma unroll
-        for (int j = 0; j < SB; ++j) sm.XD[p][j * SLP + lane] = a[j];
+    } else if (p > 0 && work_warp) {
+      // ... and with the columns beyond it, next to this panel's chain: rows
+      // c .. np - 1 of the block and rows 0 .. p - 1 of X^T
+      int first = 0;
+      for (int c = p + 1; c < np; ++c) {
+        const int n = 2 * (np - c + p);
+        for (int u = (worker + 12 - first) % 6; u < n; u += 6) {
+          const int q = u >> 1;
+          diag_update_block(sm, q < np - c ? c + q : q - (np - c), u & 1, c,
+                            p - 1, lane);
+        }
+        first = (first + n) % 6;
       }
-#pragma unroll
-      for (int j = 0; j < SB; j += 4)
-        *reinterpret_cast<float4*>(&row[j]) =
-            make_float4(a[j], a[j + 1], a[j + 2], a[j + 3]);
     }
-    __syncthreads();
-    if (p + 1 < np) {
-      // next diagonal sub-block: row per lane, two columns per warp
-      const float* Lr = &sm.S[(SB * (p + 1)) * DLD + SB * p];
-      const int c = 2 * warp;
-      float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-      for (int k = 0; k < SB; k += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(&Lr[lane * DLD + k]);
-        const float4 u = *reinterpret_cast<const float4*>(&Lr[c * DLD + k]);
-        const float4 v = *reinterpret_cast<const float4*>(&Lr[(c + 1) * DLD + k]);
-        s0 = fmaf(x.w, u.w, fmaf(x.z, u.z, fmaf(x.y, u.y, fmaf(x.x, u.x, s0))));
-        s1 = fmaf(x.w, v.w, fmaf(x.z, v.z, fmaf(x.y, v.y, fmaf(x.x, v.x, s1))));
-      }
-      float* dst = &sm.S[(SB * (p + 1) + lane) * DLD + SB * (p + 1) + c];
-      dst[0] -= s0;
-      dst[1] -= s1;
-      __syncthreads();
-    }
-  }
-  if (np > 1) {
-    if (warp < 2 * (np - 1)) diag_x_block(sm, np - 1, warp >> 1, warp & 1, lane);
     __syncthreads();
   }
 
@@ -708,23 +845,29 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, const int* __restrict__ ids,
   // 16-byte word per lane) into four contiguous row pieces.  The part above
   // the diagonal sub-blocks was zeroed when the plan was made.
   float* Xd = mi.X + (long long)o * ld + o;
-  for (int t = warp; t < np * (np + 1) / 2 * 8; t += DT / 32) {
-    int u = t >> 3, bi = 0;
-    while (u > bi) u -= ++bi;                       // sub-block (bi, u)
-    const int r0 = 4 * (t & 7);
-    const float* src = bi == u ? &sm.XDT[u][lane * SLP + r0]
-                               : &sm.S[(SB * u + lane) * DLD + SB * bi + r0];
-    const float4 v = *reinterpret_cast<const float4*>(src);
-    const int r = SB * bi + r0, c = SB * u + lane;
-    if (c < bs) {
-      if (r < bs) Xd[r * ld + c] = v.x;
-      if (r + 1 < bs) Xd[(r + 1) * ld + c] = v.y;
-      if (r + 2 < bs) Xd[(r + 2) * ld + c] = v.z;
-      if (r + 3 < bs) Xd[(r + 3) * ld + c] = v.w;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = 4 * warp + 64 * h, bi = r >> 5;
+    if (r >= bs) break;
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (u <= bi)
+        v[u] = *reinterpret_cast<const float4*>(
+            u == bi ? &sm.XD[u][lane * SLP + (r & (SB - 1))]
+                    : &sm.S[(SB * u + lane) * DLD + r]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int c = SB * u + lane;
+      if (u > bi || c >= bs) continue;
+      float* dst = Xd + r * ld + c;
+      dst[0] = v[u].x;
+      if (r + 1 < bs) dst[ld] = v[u].y;
+      if (r + 2 < bs) dst[2 * ld] = v[u].z;
+      if (r + 3 < bs) dst[3 * ld] = v[u].w;
     }
   }
 }
-
 
 // ---------------------------------------------------------------- refinement
 // One step of iterative refinement for factors whose fp32 inverse is visibly
@@ -926,8 +1069,8 @@ static_assert(kDiagLookSmemBytes >= kDiagSmemBytes &&
 struct Launch {
   int tails;     // grouped gemm: some contraction is not a multiple of 32
   int kind;      // 0 diag kernel, 1 grouped gemm, 2 join of the side stream
-  int off;       // offset into ids / descs
-  int n;         // number of ids / descs
+  int off;       // grouped gemm: offset into descs
+  int n;         // number of matrices / descs
   int tiles;     // grouped gemm: total tiles
   int step;      // diag kernel: panel index
   // A run uses two streams: the chain (0) and a side stream (1) for work
@@ -957,7 +1100,7 @@ struct kfac_inverse_plan {
   float* trace_dev;
   float* add_dev;
   int* info_dev;
-  int* ids_dev;
+  MatInfo* sorted_dev;     // mats_dev, largest first (diagonal kernels)
   GemmDesc* descs_dev;
   std::vector<Launch> launches;
   long long total_elems;
@@ -1054,6 +1197,7 @@ extern "C" int kfac_inverse_plan_create(
     m.l2 = l2_coef ? l2_coef[i] : 0.f;
     m.scale = scale ? scale[i] : 1.f;
     m.l2b = m.l2;
+    m.id = i;
     dmax = std::max(dmax, dims[i]);
     total_elems += (long long)dims[i] * dims[i];
   }
@@ -1064,7 +1208,6 @@ extern "C" int kfac_inverse_plan_create(
                    [&](int a, int b) { return dims[a] > dims[b]; });
 
   std::vector<GemmDesc> descs;
-  std::vector<int> ids;
   std::vector<Launch> launches;
   const bool use_tc = engine() == 1;
 
@@ -1118,9 +1261,10 @@ extern "C" int kfac_inverse_plan_create(
     int last_solve_ev = -1;
     for (int o = po; o < po + inner; o += DB) {
       const bool lk = look && o > po;
-      Launch dl = {0, 0, (int)ids.size(), 0, 0, o / DB, 0, -1, -1, -1, lk};
+      // the matrices that still have a block here are the first of `order`
+      Launch dl = {0, 0, 0, 0, 0, o / DB, 0, -1, -1, -1, lk};
       for (int i : order)
-        if (dims[i] > o) { ids.push_back(i); dl.n += 1; }
+        if (dims[i] > o) dl.n += 1;
       if (lk && o - 2 * DB >= po) dl.wait_ev = upd_ev[(o - 2 * DB) / DB];
       if (look) dl.rec_ev = diag_ev[o / DB] = n_events++;
       launches.push_back(dl);
@@ -1327,7 +1471,7 @@ extern "C" int kfac_inverse_plan_create(
   p->launches = launches;
   p->use_tc = use_tc;
   p->mats_dev = nullptr; p->trace_dev = nullptr; p->add_dev = nullptr;
-  p->info_dev = nullptr; p->ids_dev = nullptr; p->descs_dev = nullptr;
+  p->info_dev = nullptr; p->sorted_dev = nullptr; p->descs_dev = nullptr;
   p->add2_dev = nullptr; p->refine_items_dev = nullptr;
   p->refine_sums_dev = nullptr; p->refine_vec_dev = nullptr;
   p->refine_gate_dev = nullptr; p->refine_count_dev = nullptr;
@@ -1407,10 +1551,15 @@ extern "C" int kfac_inverse_plan_create(
   if (e == cudaSuccess) e = cudaMalloc(&p->trace_dev, sizeof(float) * count);
   if (e == cudaSuccess) e = cudaMalloc(&p->add_dev, sizeof(float) * count);
   if (e == cudaSuccess) e = cudaMalloc(&p->info_dev, sizeof(int) * count);
-  if (e == cudaSuccess) e = cudaMalloc(&p->ids_dev, sizeof(int) * std::max<size_t>(ids.size(), 1));
+  if (e == cudaSuccess) e = cudaMalloc(&p->sorted_dev, sizeof(MatInfo) * count);
   if (e == cudaSuccess) e = cudaMalloc(&p->descs_dev, sizeof(GemmDesc) * std::max<size_t>(descs.size(), 1));
   if (e == cudaSuccess) e = cudaMemcpy(p->mats_dev, mats.data(), sizeof(MatInfo) * count, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !ids.empty()) e = cudaMemcpy(p->ids_dev, ids.data(), sizeof(int) * ids.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    std::vector<MatInfo> sorted(count);
+    for (int i = 0; i < count; ++i) sorted[i] = mats[order[i]];
+    e = cudaMemcpy(p->sorted_dev, sorted.data(), sizeof(MatInfo) * count,
+                   cudaMemcpyHostToDevice);
+  }
   if (e == cudaSuccess && !descs.empty()) e = cudaMemcpy(p->descs_dev, descs.data(), sizeof(GemmDesc) * descs.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(chol_diag_kernel<false>,
@@ -1473,10 +1622,10 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
     if (l.kind == 0) {
       if (l.look)
         chol_diag_kernel<true><<<l.n, DT, kDiagLookSmemBytes, st>>>(
-            p->mats_dev, p->ids_dev + l.off, l.step, info);
+            p->sorted_dev, l.step, info);
       else
         chol_diag_kernel<false><<<l.n, DT, kDiagSmemBytes, st>>>(
-            p->mats_dev, p->ids_dev + l.off, l.step, info);
+            p->sorted_dev, l.step, info);
       KFAC_LAUNCH_CHECK("chol_diag_kernel");
     } else {
       int rc = p->use_tc
@@ -1665,7 +1814,7 @@ extern "C" int kfac_inverse_plan_destroy(kfac_inverse_plan* p) {
   cudaFree(p->trace_dev);
   cudaFree(p->add_dev);
   cudaFree(p->info_dev);
-  cudaFree(p->ids_dev);
+  cudaFree(p->sorted_dev);
   cudaFree(p->descs_dev);
   delete p;
   return KFAC_OK;
