@@ -67,7 +67,7 @@ gemm_grouped_kernel(const GemmDesc* __restrict__ descs, int ndesc, float lr,
   const int m0 = bi * TM, n0 = bj * TN;
   long long kbeg = 0, kend = sd.K;
   if (sd.flags & G_KBEG_N0) kbeg = n0;
-  if (sd.flags & G_KBEG_M0) kbeg = m0;
+  if (sd.flags & G_KBEG_M0) kbeg = max(0, m0 - sd.kbeg_off);
   if (sd.flags & G_KEND_M0) kend = min((long long)(m0 + TM), sd.K);
 
   float acc[8][8];
@@ -111,7 +111,9 @@ gemm_grouped_kernel(const GemmDesc* __restrict__ descs, int ndesc, float lr,
   }
 
   const bool mirror = (sd.flags & G_MIRROR) && (bi != bj);
-  const float alpha = sd.alpha, beta = sd.beta;
+  const float alpha = sd.alpha;
+  const float beta =
+      (sd.beta_until > 0 && m0 >= sd.beta_until) ? 0.f : sd.beta;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     int r = m0 + tile_row(ty, i);

@@ -235,7 +235,7 @@ enum GemmFlags {
   G_MIRROR = 2,    // also write C[n][m] for off-diagonal tiles
   G_KBEG_N0 = 4,   // B(k, n) is zero for k < n: start at the tile's n0
   G_KEND_M0 = 8,   // A(k, m) is zero for k > m: stop after the tile's rows
-  G_KBEG_M0 = 16,  // A(k, m) is zero for k < m: start at the tile's m0
+  G_KBEG_M0 = 16,  // A(k, m) is zero for k < m - kbeg_off: start there
   G_PRECOND = 32,  // epilogue splits into kf_W / kf_b and applies momentum
   G_SAME_AB = 64   // A and B are the same operand (X^T X): a tile on the
                    // diagonal may take its A rows from the staged B rows
@@ -260,6 +260,9 @@ struct GemmDesc {
   const int* gate;         // if set and *gate == 0 the problem is skipped
   float* C2;               // if set, C's new values are stored here as well
                            // (same row pitch; plain epilogue only)
+  int beta_until;          // > 0: rows from here on ignore beta (a multiple of
+                           // the tile rows)
+  int kbeg_off;            // G_KBEG_M0: A(k, m) is zero for k < m - kbeg_off
   // factor builds from staged operands: tensor maps (device memory) of the
   // hi and lo bf16 planes of X^T, see stage.cu
   const void* tmap_hi;

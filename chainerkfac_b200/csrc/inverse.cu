@@ -43,19 +43,6 @@ struct RunParams {
   int use_pi;
   int refine_max_dim;
   float refine_threshold;
-  // CUDA graph of one run (captured on first use)
-  RunParams* params_dev;
-  std::vector<cudaEvent_t> events;   // edges between the two streams
-  cudaEvent_t fork_ev, join_ev[2];
-  cudaStream_t side_stream[2];       // bulk / far stream of plain runs
-  cudaStream_t cap_side[2];          // the same during capture
-  bool look;
-  cudaStream_t cap_stream;
-  cudaGraphExec_t graph_exec;
-  int* graph_info;
-  float* graph_diag;
-  long long graph_launches;
-  bool graph_ok;
 };
 
 __global__ void set_run_params_kernel(RunParams* prm, float damping,
@@ -806,8 +793,8 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
     }
     if (warp == 0) {
       diag_base(sm, p, lane, id, o + SB * p, followers, info);
-    } else if (warp == 3 || warp >= 13) {
-      diag_base_rest(sm, p, lane, warp == 3 ? 3 : warp - 13, followers);
+    } else if (warp == 3 || (warp & 3) == 0) {
+      diag_base_rest(sm, p, lane, warp == 3 ? 3 : (warp >> 2) - 1, followers);
     } else if (warp <= 2) {
       const int q = 2 * (warp - 1);
       if (q < np) {
@@ -1066,21 +1053,30 @@ static_assert(kDiagLookSmemBytes >= kDiagSmemBytes &&
                   kDiagLookSmemBytes <= 227 * 1024,
               "diagonal kernel shared memory");
 
+// Streams of one run: the chain of diagonal kernels, panel solves and updates
+// behind it, trailing updates nothing waits for soon, rows of L^-1, and the
+// product of those rows.
+enum PlanStream { S_CHAIN, S_BULK, S_FAR, S_ROWS, S_PROD, S_COUNT };
+
 struct Launch {
   int tails;     // grouped gemm: some contraction is not a multiple of 32
-  int kind;      // 0 diag kernel, 1 grouped gemm, 2 join of the side stream
+  int kind;      // 0 diag kernel, 1 grouped gemm
   int off;       // grouped gemm: offset into descs
   int n;         // number of matrices / descs
   int tiles;     // grouped gemm: total tiles
   int step;      // diag kernel: panel index
-  // A run uses two streams: the chain (0) and a side stream (1) for work
-  // that is off the critical path.  A launch may wait for an event first and
-  // record one afterwards (indices into the plan's events, -1: none).
-  int stream;
-  int wait_ev;
+  int stream;    // PlanStream
+  // events (indices into the plan's events, -1: none) to wait for first and to
+  // record afterwards
+  int wait_ev[3];
   int rec_ev;
-  int wait_ev2;
   bool look;     // diag kernel: with the look-ahead prologue
+
+  void wait(int ev) {
+    if (ev < 0) return;
+    for (int& w : wait_ev)
+      if (w < 0) { w = ev; return; }
+  }
 };
 
 // Status word of the diagonal kernel's bounded waits (read by kfac_tc_status).
@@ -1120,10 +1116,10 @@ struct kfac_inverse_plan {
   float refine_threshold;
   // CUDA graph of one run (captured on first use)
   RunParams* params_dev;
-  std::vector<cudaEvent_t> events;   // edges between the two streams
-  cudaEvent_t fork_ev, join_ev[2];
-  cudaStream_t side_stream[2];       // bulk / far stream of plain runs
-  cudaStream_t cap_side[2];          // the same during capture
+  std::vector<cudaEvent_t> events;   // edges between the streams
+  cudaEvent_t fork_ev, join_ev[S_COUNT];
+  cudaStream_t side_stream[S_COUNT]; // streams of plain runs (from S_BULK on)
+  cudaStream_t cap_side[S_COUNT];    // the same during capture
   bool look;
   cudaStream_t cap_stream;
   cudaGraphExec_t graph_exec;
@@ -1216,10 +1212,18 @@ extern "C" int kfac_inverse_plan_create(
     const char* env = getenv("KFAC_INVERSE_LOOKAHEAD");
     return !(env && env[0] == '0');
   }();
+  // without the look-ahead everything but the far updates follows the chain
+  const int s_bulk = look ? S_BULK : S_CHAIN;
+  const int s_rows = look ? S_ROWS : S_CHAIN;
+  const int s_prod = look ? S_PROD : S_CHAIN;
   std::vector<int> diag_ev((dmax + DB - 1) / DB + 1, -1);
   std::vector<int> upd_ev((dmax + DB - 1) / DB + 1, -1);
-  auto begin_gemm = [&]() {
-    Launch l = {0, 1, (int)descs.size(), 0, 0, 0, 0, -1, -1, -1, false};
+  auto begin_gemm = [&](int stream) {
+    Launch l = {};
+    l.kind = 1;
+    l.off = (int)descs.size();
+    l.stream = stream;
+    l.wait_ev[0] = l.wait_ev[1] = l.wait_ev[2] = l.rec_ev = -1;
     return l;
   };
   auto push_desc = [&](Launch& l, GemmDesc g) {
@@ -1235,8 +1239,12 @@ extern "C" int kfac_inverse_plan_create(
     descs.push_back(g);
     l.n += 1;
   };
-  auto end_gemm = [&](Launch& l) {
-    if (l.n > 0) launches.push_back(l);
+  // append a launch (if it has work); its event, or -1
+  auto end_gemm = [&](Launch& l, bool record) {
+    if (l.n == 0) return -1;
+    if (record) l.rec_ev = n_events++;
+    launches.push_back(l);
+    return l.rec_ev;
   };
 
   int prev_far_ev = -1;
@@ -1245,31 +1253,43 @@ extern "C" int kfac_inverse_plan_create(
   // contractions, little work); the bulk of the flops is the update of the
   // trailing matrix with the whole panel (contraction length PW).
   //
-  // With look-ahead (default) a run uses three streams.  The chain (0)
-  // carries the diagonal kernels; inside a panel the diagonal kernel of step
-  // k applies step k-1's update to its own block itself (diag_lookahead), so
-  // it only waits for the panel update of step k-2.  The panel solves and
-  // panel updates of the steps run on the bulk stream (1) behind the chain,
-  // and the part of a panel's trailing update that the next panel does not
-  // need runs on the far stream (2).  Panel updates (and the near part of a
-  // trailing update, and the damped copy for the first block column) store
+  // The chain carries the diagonal kernels; inside a panel the diagonal
+  // kernel of step k applies step k-1's update to its own block itself
+  // (diag_lookahead), so it only waits for the panel update of step k-2.  The
+  // panel solves and panel updates of the steps run on the bulk stream behind
+  // the chain, and the part of a panel's trailing update that the next panel
+  // does not need runs on the far stream.  Panel updates (and the near part of
+  // a trailing update, and the damped copy for the first block column) store
   // their results a second time in the inverse's output buffer: that copy of
-  // block (k, k-1) is what diag_lookahead reads while the panel solve of
-  // step k-1 overwrites the original.
+  // block (k, k-1) is what diag_lookahead reads while the panel solve of step
+  // k-1 overwrites the original.
+  //
+  // The inverse grows with the factor, a row panel at a time: with X = L^-1,
+  //   T = L_p X_<p,  X_p = -X_pp T  (X_pp by doubling from the 128-blocks),
+  //   inv += X_p^T X_p,
+  // next to the chain of the following panels, which leaves most SMs idle.
+  // When the chain ends only the last panel's share is left (a 4608-row matrix:
+  // 0.15 ms instead of the 0.95 ms that the whole triangular inverse and
+  // product took behind the factorisation).  T^T waits in the unused upper
+  // triangle of W; rows and columns of inv before the running panel are no
+  // longer needed for the copies above.
   for (int po = 0; po < dmax; po += PW) {
     const int inner = std::min(PW, dmax - po);
+    int bulk_ev = -1;          // the bulk stream's last launch of this panel
     int last_solve_ev = -1;
     for (int o = po; o < po + inner; o += DB) {
       const bool lk = look && o > po;
       // the matrices that still have a block here are the first of `order`
-      Launch dl = {0, 0, 0, 0, 0, o / DB, 0, -1, -1, -1, lk};
+      Launch dl = begin_gemm(S_CHAIN);
+      dl.kind = 0;
+      dl.step = o / DB;
+      dl.look = lk;
       for (int i : order)
         if (dims[i] > o) dl.n += 1;
-      if (lk && o - 2 * DB >= po) dl.wait_ev = upd_ev[(o - 2 * DB) / DB];
-      if (look) dl.rec_ev = diag_ev[o / DB] = n_events++;
-      launches.push_back(dl);
+      if (lk && o - 2 * DB >= po) dl.wait(upd_ev[(o - 2 * DB) / DB]);
+      diag_ev[o / DB] = end_gemm(dl, look);
 
-      Launch trsm = begin_gemm();
+      Launch trsm = begin_gemm(s_bulk);
       for (int i : order) {
         const int d = dims[i];
         const int M = d - o - DB;
@@ -1283,18 +1303,15 @@ extern "C" int kfac_inverse_plan_create(
         g.alpha = 1.f; g.beta = 0.f; g.flags = 0;
         push_desc(trsm, g);
       }
-      if (look && trsm.n > 0) {
-        trsm.stream = 1;
-        trsm.wait_ev = diag_ev[o / DB];
-        trsm.rec_ev = last_solve_ev = n_events++;
-      }
-      end_gemm(trsm);
+      trsm.wait(diag_ev[o / DB]);
+      const int solve_ev = end_gemm(trsm, look);
+      if (solve_ev >= 0) bulk_ev = last_solve_ev = solve_ev;
 
       // update the rest of this panel's columns (full rectangle; entries
       // above the diagonal are written but never read).  With look-ahead the
       // next diagonal block is left to the next diagonal kernel.
       const int skip = (look && o + DB < po + inner) ? DB : 0;
-      Launch upd = begin_gemm();
+      Launch upd = begin_gemm(s_bulk);
       for (int i : order) {
         const int d = dims[i];
         const int M = d - o - DB - skip;
@@ -1312,11 +1329,8 @@ extern "C" int kfac_inverse_plan_create(
         if (look) g.C2 = m.inv + coff;
         push_desc(upd, g);
       }
-      if (look) {
-        upd.stream = 1;
-        if (upd.n > 0) upd.rec_ev = upd_ev[o / DB] = n_events++;
-      }
-      end_gemm(upd);
+      upd_ev[o / DB] = end_gemm(upd, look);
+      if (upd_ev[o / DB] >= 0) bulk_ev = upd_ev[o / DB];
     }
 
     // Update of the trailing matrix with the finished panel, in two parts:
@@ -1325,7 +1339,7 @@ extern "C" int kfac_inverse_plan_create(
     // the next panel's chain.  Both parts of one panel touch disjoint tiles;
     // parts of successive panels that touch the same tiles are ordered by
     // events (next-panel part p+1 after far part p) or by stream order.
-    Launch near = begin_gemm(), far = begin_gemm();
+    Launch near = begin_gemm(S_CHAIN);
     std::vector<GemmDesc> far_descs;
     for (int i : order) {
       const int d = dims[i];
@@ -1365,82 +1379,123 @@ extern "C" int kfac_inverse_plan_create(
         far_descs.push_back(h);
       }
     }
-    far.off = (int)descs.size();
-    for (auto& h : far_descs) push_desc(far, h);
-    int panel_ev = look ? last_solve_ev : -1;
-    if (!look && far.n > 0) {
+    int panel_ev = last_solve_ev;
+    if (!look && !far_descs.empty()) {
       // the far part needs the finished panel: an event recorded on the
       // chain right before the near part
       panel_ev = n_events++;
       launches.back().rec_ev = panel_ev;   // last launch of the panel's chain
     }
-    if (near.n > 0) {
-      near.wait_ev = prev_far_ev;          // far part of the previous panel
-      near.wait_ev2 = look ? panel_ev : -1;  // the bulk stream's last solve
-      prev_far_ev = -1;
-    }
-    if (far.n > 0) {
-      far.stream = 2;
-      far.wait_ev = panel_ev;
-      far.rec_ev = n_events++;
-      prev_far_ev = far.rec_ev;
-    }
-    end_gemm(near);
-    end_gemm(far);
-  }
-  {
-    // the triangular inverse reads all of L: join the side stream
-    Launch join = {0, 2, 0, 0, 0, 0, 0, -1, -1, -1, false};
-    launches.push_back(join);
-  }
+    near.wait(prev_far_ev);                // far part of the previous panel
+    if (look) near.wait(panel_ev);         // the bulk stream's last solve
+    if (near.n > 0) prev_far_ev = -1;
+    end_gemm(near, false);
+    Launch far = begin_gemm(S_FAR);
+    for (auto& h : far_descs) push_desc(far, h);
+    far.wait(panel_ev);
+    if (far.n > 0) prev_far_ev = end_gemm(far, true);
 
-  for (long long b = DB; b < dmax; b *= 2) {
-    Launch g1 = begin_gemm(), g2 = begin_gemm();
-    std::vector<GemmDesc> second;
-    for (int i : order) {
-      const int d = dims[i];
-      if (d <= b) continue;
-      const MatInfo& m = mats[i];
-      for (long long s = 0; s + b < d; s += 2 * b) {
-        const int r = (int)std::min<long long>(b, d - s - b);
+    // ---- row panel of the inverse
+    const int pend = std::min(po + PW, dmax);
+    bool first = true;
+    for (int b = DB; b < pend - po; b *= 2) {
+      // X_pp by doubling: T = L21 X11 (parked in the output matrix), then
+      // X21 = -X22 T
+      Launch g1 = begin_gemm(s_rows);
+      std::vector<GemmDesc> second;
+      for (int i : order) {
+        const int d = dims[i], end = std::min(po + PW, d);
+        const MatInfo& m = mats[i];
+        for (long long s = po; s + b < end; s += 2 * b) {
+          const int r = (int)std::min<long long>(b, end - s - b);
+          GemmDesc g = {};
+          g.A = strided_operand(m.W + (s + b) * d + s, 1, d, r);
+          g.B = strided_operand(m.X + s * d + s, d, 1, b);
+          g.C = m.inv + (s + b) * d + s;
+          g.ldc = d; g.M = r; g.N = b; g.K = b;
+          g.alpha = 1.f; g.beta = 0.f; g.flags = G_KBEG_N0;
+          push_desc(g1, g);
+          GemmDesc h = {};
+          h.A = strided_operand(m.X + (s + b) * d + s + b, 1, d, r);
+          h.B = strided_operand(m.inv + (s + b) * d + s, d, 1, b);
+          h.C = m.X + (s + b) * d + s;
+          h.ldc = d; h.M = r; h.N = b; h.K = r;
+          h.alpha = -1.f; h.beta = 0.f; h.flags = G_KEND_M0;
+          second.push_back(h);
+        }
+      }
+      if (first) {
+        g1.wait(bulk_ev);
+        g1.wait(diag_ev[(pend - 1) / DB]);
+        if (g1.n > 0) first = false;
+      }
+      end_gemm(g1, false);
+      Launch g2 = begin_gemm(s_rows);
+      for (auto& h : second) push_desc(g2, h);
+      end_gemm(g2, false);
+    }
+    Launch rows = begin_gemm(s_rows), next_t = begin_gemm(s_rows);
+    if (po > 0) {
+      for (int i : order) {
+        const int d = dims[i], w = std::min(PW, d - po);
+        if (w <= 0) continue;
+        const MatInfo& m = mats[i];
         GemmDesc g = {};
-        // T = L21 * X11, parked in the output matrix
-        g.A = strided_operand(m.W + (s + b) * d + s, 1, d, r);
-        g.B = strided_operand(m.X + s * d + s, d, 1, (int)b);
-        g.C = m.inv + (s + b) * d + s;
-        g.ldc = d; g.M = r; g.N = (int)b; g.K = b;
-        g.alpha = 1.f; g.beta = 0.f; g.flags = G_KBEG_N0;
-        push_desc(g1, g);
-        // X21 = -X22 * T
-        GemmDesc h = {};
-        h.A = strided_operand(m.X + (s + b) * d + s + b, 1, d, r);
-        h.B = strided_operand(m.inv + (s + b) * d + s, d, 1, (int)b);
-        h.C = m.X + (s + b) * d + s;
-        h.ldc = d; h.M = r; h.N = (int)b; h.K = r;
-        h.alpha = -1.f; h.beta = 0.f; h.flags = G_KEND_M0;
-        second.push_back(h);
+        g.A = strided_operand(m.X + (long long)po * d + po, 1, d, w);
+        g.B = strided_operand(m.W + po, 1, d, po);    // B(k, n) = T^T[n][k]
+        g.C = m.X + (long long)po * d;
+        g.ldc = d; g.M = w; g.N = po; g.K = w;
+        g.alpha = -1.f; g.beta = 0.f; g.flags = G_KEND_M0;
+        push_desc(rows, g);
       }
     }
-    end_gemm(g1);
-    g2.off = (int)descs.size();
-    for (auto& h : second) push_desc(g2, h);
-    end_gemm(g2);
-  }
-
-  {
-    Launch prod = begin_gemm();
+    if (first) {
+      rows.wait(bulk_ev);
+      rows.wait(diag_ev[(pend - 1) / DB]);
+      if (rows.n > 0) first = false;
+    }
+    int rows_ev = end_gemm(rows, look);
+    // the product, behind the rows (or, for a single panel, the doubling)
+    Launch prod = begin_gemm(s_prod);
     for (int i : order) {
-      const int d = dims[i];
+      const int d = dims[i], end = std::min(po + PW, d), w = end - po;
+      if (w <= 0) continue;
       const MatInfo& m = mats[i];
       GemmDesc g = {};
-      g.A = strided_operand(m.X, d, 1, d);
+      g.A = strided_operand(m.X + (long long)po * d, d, 1, end);
       g.B = g.A;
-      g.C = m.inv; g.ldc = d; g.M = d; g.N = d; g.K = d;
-      g.alpha = 1.f; g.beta = 0.f;
-      g.flags = G_LOWER | G_MIRROR | G_KBEG_M0 | G_SAME_AB;
+      g.C = m.inv; g.ldc = d; g.M = end; g.N = end; g.K = w;
+      g.alpha = 1.f; g.beta = po > 0 ? 1.f : 0.f;
+      g.beta_until = po; g.kbeg_off = po;
+      g.flags = G_LOWER | G_KBEG_M0 | G_SAME_AB | (end == d ? G_MIRROR : 0);
       push_desc(prod, g);
     }
-    end_gemm(prod);
+    if (look && rows_ev < 0 && !first) {
+      rows_ev = n_events++;
+      launches.back().rec_ev = rows_ev;      // the doubling's last launch
+    }
+    if (look && first) {
+      prod.wait(bulk_ev);
+      prod.wait(diag_ev[(pend - 1) / DB]);
+    }
+    prod.wait(rows_ev);
+    // T^T of the next panel
+    next_t.off = (int)descs.size();
+    for (int i : order) {
+      const int d = dims[i], w = std::min(PW, d - pend);
+      if (w <= 0) continue;
+      const MatInfo& m = mats[i];
+      GemmDesc g = {};
+      g.A = strided_operand(m.X, d, 1, pend);
+      g.B = strided_operand(m.W + (long long)pend * d, 1, d, w);
+      g.C = m.W + pend;
+      g.ldc = d; g.M = pend; g.N = w; g.K = pend;
+      g.alpha = 1.f; g.beta = 0.f; g.flags = G_KBEG_M0;
+      push_desc(next_t, g);
+    }
+    if (look && first) next_t.wait(bulk_ev);
+    end_gemm(next_t, false);
+    end_gemm(prod, false);
   }
 
   // refinement of the matrices of up to kRefineDimCap rows: Y = X R on the
@@ -1463,7 +1518,7 @@ extern "C" int kfac_inverse_plan_create(
     vec_elems += 2LL * dims[i];
     ritems.push_back(it);
   }
-  Launch refine_prod = begin_gemm();
+  Launch refine_prod = begin_gemm(S_CHAIN);
 
   kfac_inverse_plan* p = new kfac_inverse_plan();
   p->count = count;
@@ -1481,9 +1536,9 @@ extern "C" int kfac_inverse_plan_create(
   p->refine_max_dim = kRefineDimCap;
   p->refine_threshold = 3e-5f;
   p->params_dev = nullptr;
-  p->fork_ev = p->join_ev[0] = p->join_ev[1] = nullptr;
-  p->side_stream[0] = p->side_stream[1] = nullptr;
-  p->cap_side[0] = p->cap_side[1] = nullptr;
+  p->fork_ev = nullptr;
+  for (int k = 1; k < S_COUNT; ++k)
+    p->join_ev[k] = nullptr, p->side_stream[k] = p->cap_side[k] = nullptr;
   p->look = look;
   p->cap_stream = nullptr;
   p->graph_exec = nullptr;
@@ -1503,7 +1558,7 @@ extern "C" int kfac_inverse_plan_create(
   if (e == cudaSuccess)
     e = cudaStreamCreateWithPriority(&p->cap_stream, cudaStreamNonBlocking,
                                      prio_hi);
-  for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
+  for (int k = 1; k < S_COUNT && e == cudaSuccess; ++k) {
     e = cudaStreamCreateWithPriority(&p->cap_side[k], cudaStreamNonBlocking,
                                      prio_lo);
     if (e == cudaSuccess)
@@ -1512,7 +1567,7 @@ extern "C" int kfac_inverse_plan_create(
   }
   if (e == cudaSuccess)
     e = cudaEventCreateWithFlags(&p->fork_ev, cudaEventDisableTiming);
-  for (int k = 0; k < 2 && e == cudaSuccess; ++k)
+  for (int k = 1; k < S_COUNT && e == cudaSuccess; ++k)
     e = cudaEventCreateWithFlags(&p->join_ev[k], cudaEventDisableTiming);
   for (int k = 0; k < n_events + 1 && e == cudaSuccess; ++k) {
     cudaEvent_t ev = nullptr;
@@ -1589,11 +1644,13 @@ extern "C" int kfac_inverse_plan_create(
 static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
                         cudaStream_t main_st, cudaStream_t* side_st) {
   cudaStream_t st = main_st;
-  cudaStream_t sts[3] = {main_st, side_st[0], side_st[1]};
+  cudaStream_t sts[S_COUNT] = {main_st};
   // fork: the side streams start after what precedes this run
   KFAC_CUDA(cudaEventRecord(p->fork_ev, main_st));
-  KFAC_CUDA(cudaStreamWaitEvent(side_st[0], p->fork_ev, 0));
-  KFAC_CUDA(cudaStreamWaitEvent(side_st[1], p->fork_ev, 0));
+  for (int k = 1; k < S_COUNT; ++k) {
+    sts[k] = side_st[k];
+    KFAC_CUDA(cudaStreamWaitEvent(sts[k], p->fork_ev, 0));
+  }
   trace_kernel<<<p->count, 256, 0, st>>>(p->mats_dev, p->trace_dev, info);
   KFAC_LAUNCH_CHECK("trace_kernel");
   damping_kernel<<<ceil_div(p->count, 128), 128, 0, st>>>(
@@ -1607,18 +1664,9 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
     KFAC_LAUNCH_CHECK("damp_copy_kernel");
   }
   for (const Launch& l : p->launches) {
-    if (l.kind == 2) {
-      for (int k = 0; k < 2; ++k) {
-        KFAC_CUDA(cudaEventRecord(p->join_ev[k], side_st[k]));
-        KFAC_CUDA(cudaStreamWaitEvent(main_st, p->join_ev[k], 0));
-      }
-      continue;
-    }
     st = sts[l.stream];
-    if (l.wait_ev >= 0)
-      KFAC_CUDA(cudaStreamWaitEvent(st, p->events[l.wait_ev], 0));
-    if (l.wait_ev2 >= 0)
-      KFAC_CUDA(cudaStreamWaitEvent(st, p->events[l.wait_ev2], 0));
+    for (int ev : l.wait_ev)
+      if (ev >= 0) KFAC_CUDA(cudaStreamWaitEvent(st, p->events[ev], 0));
     if (l.kind == 0) {
       if (l.look)
         chol_diag_kernel<true><<<l.n, DT, kDiagLookSmemBytes, st>>>(
@@ -1638,6 +1686,10 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
     if (l.rec_ev >= 0) KFAC_CUDA(cudaEventRecord(p->events[l.rec_ev], st));
   }
   st = main_st;
+  for (int k = 1; k < S_COUNT; ++k) {
+    KFAC_CUDA(cudaEventRecord(p->join_ev[k], sts[k]));
+    KFAC_CUDA(cudaStreamWaitEvent(main_st, p->join_ev[k], 0));
+  }
   if (p->n_refine > 0) {
     const dim3 pgrid(ceil_div(p->refine_dmax, 8), p->n_refine);
     for (int stage = 0; stage < 3; ++stage) {
@@ -1796,7 +1848,7 @@ extern "C" int kfac_inverse_plan_destroy(kfac_inverse_plan* p) {
   if (p == nullptr) return KFAC_OK;
   plan_drop_graph(p);
   if (p->cap_stream != nullptr) cudaStreamDestroy(p->cap_stream);
-  for (int k = 0; k < 2; ++k) {
+  for (int k = 1; k < S_COUNT; ++k) {
     if (p->cap_side[k] != nullptr) cudaStreamDestroy(p->cap_side[k]);
     if (p->side_stream[k] != nullptr) cudaStreamDestroy(p->side_stream[k]);
     if (p->join_ev[k] != nullptr) cudaEventDestroy(p->join_ev[k]);

@@ -452,7 +452,7 @@ tc_gemm_kernel(const GemmDesc* __restrict__ descs, int ndesc,
     kend = min(g.K, kbeg + g.k_per_split);
   }
   if (g.flags & G_KBEG_N0) kbeg = max(kbeg, (long long)n0);
-  if (g.flags & G_KBEG_M0) kbeg = max(kbeg, (long long)m0);
+  if (g.flags & G_KBEG_M0) kbeg = max(kbeg, (long long)(m0 - g.kbeg_off));
   if (g.flags & G_KEND_M0) kend = min(kend, (long long)(m0 + TC_BM));
   // a gated-off problem runs no k-blocks and stores nothing
   const bool gated_off = g.gate != nullptr && *g.gate == 0;
@@ -655,7 +655,8 @@ tc_gemm_kernel(const GemmDesc* __restrict__ descs, int ndesc,
     }
     return;
   }
-  const float alpha = g.alpha, beta = g.beta;
+  const float alpha = g.alpha;
+  const float beta = (g.beta_until > 0 && m0 >= g.beta_until) ? 0.f : g.beta;
   const bool lower = (g.flags & G_LOWER) != 0;
   const bool mirror = (g.flags & G_MIRROR) != 0;
   // rows: C[gr][gc] = alpha * acc + beta * C[gr][gc]; the final value is kept
