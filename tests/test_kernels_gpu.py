@@ -505,6 +505,38 @@ def test_momentum_update_and_axpby(ops):
     assert rel(host(y), 0.25 * p + 0.75 * g) < 1e-6
 
 
+@pytest.mark.parametrize('shape', [
+    (4, 5), (33, 10), (7, 3, 1, 1), (3, 5, 7, 7), (8, 64, 8, 8),
+    (5, 33, 9, 11), (2, 129, 3, 2), (3, 8, 66, 63), (3, 20, 66, 63),
+    (2, 6, 112, 112), (1, 4, 64, 65)])
+@pytest.mark.parametrize('channels_last', [False, True])
+@pytest.mark.parametrize('mean', [0.0, 30.0])
+def test_bn_sample_grads_layouts(ops, shape, channels_last, mean):
+    """Planes read by a part of a warp, a warp or a block, channels-last rows
+    with and without 16-byte words, partial channel groups, against fp64; the
+    mean of x may be many times its spread."""
+    torch.manual_seed(1)
+    x = torch.randn(shape, device='cuda') + mean
+    gy = torch.randn(shape, device='cuda')
+    if channels_last and len(shape) == 4:
+        x = x.contiguous(memory_format=torch.channels_last)
+        gy = gy.contiguous(memory_format=torch.channels_last)
+    out = ops.bn_sample_grads(x, gy, 1e-5, 2.0)
+    xd, gd = x.double(), gy.double() * 2.0
+    batch = [0] + list(range(2, xd.dim()))
+    xh = (xd - xd.mean(batch, keepdim=True)) / torch.sqrt(
+        xd.var(batch, unbiased=False, keepdim=True) + 1e-5)
+    ref = torch.cat([(gd * xh).flatten(2).sum(2) if xd.dim() > 2 else gd * xh,
+                     gd.flatten(2).sum(2) if xd.dim() > 2 else gd], 1)
+    # fp32 sums of up to hw terms, each rounded: sqrt(hw) 2^-24 relative to
+    # the terms, of the order of the sums themselves for random signs, times
+    # the distance of the shift from the mean in units of the spread (< 5)
+    hw = 1
+    for v in shape[2:]:
+        hw *= v
+    assert rel(host(out), host(ref)) < 5 * 6e-8 * max(4.0, hw ** 0.5)
+
+
 def test_bn_kfgrad(ops, golden):
     g = golden('bn_4d')
     c = g['g_gamma'].shape[0]
