@@ -798,7 +798,9 @@ using namespace kfac;
 
 extern "C" size_t kfac_factor_workspace_bytes(int64_t rows, int d) {
   if (rows <= 0 || d <= 0) return 0;
-  if (engine() == 1) return tc_factor_workspace_bytes(rows, d);
+  // (a dense operand; tensor-core builds of any operand with these sides fit)
+  if (engine() == 1)
+    return tc_lone_workspace_bytes(strided_operand(nullptr, d, 1, d), rows, d);
   FactorSplit s = factor_split(rows, d);
   if (s.splits <= 1) return 0;
   return (size_t)s.splits * s.tiles * TM * TN * sizeof(float);
@@ -853,13 +855,11 @@ extern "C" size_t kfac_factor_conv_workspace_bytes(int n, int c, int h, int w,
   const int wo = (w + 2 * pad - ksize) / stride + 1;
   if (ho <= 0 || wo <= 0) return 0;
   const int d = c * ksize * ksize + (add_ones_col ? 1 : 0);
-  size_t bytes = kfac_factor_workspace_bytes((int64_t)n * ho * wo, d);
-  if (engine() == 1) {
-    Operand X = conv_input_operand(nullptr, c, h, w, ksize, stride, pad,
-                                   add_ones_col);
-    bytes += tc_pad_bytes(X, n);
-  }
-  return bytes;
+  if (engine() == 1)
+    return tc_lone_workspace_bytes(
+        conv_input_operand(nullptr, c, h, w, ksize, stride, pad, add_ones_col),
+        (long long)n * ho * wo, d);
+  return kfac_factor_workspace_bytes((int64_t)n * ho * wo, d);
 }
 
 extern "C" int kfac_factor_conv_input(const float* x, int n, int c, int h,

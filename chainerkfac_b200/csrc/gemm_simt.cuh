@@ -283,6 +283,7 @@ int launch_tc_grouped(const GemmDesc* descs_dev, int ndesc, int total_tiles,
                       cudaStream_t stream);
 bool tc_desc_has_tails(const GemmDesc& g);
 size_t tc_factor_workspace_bytes(long long rows, int d, bool staged = true);
+size_t tc_lone_workspace_bytes(const Operand& X, long long rows, int d);
 size_t tc_pad_bytes(const Operand& X, int n, int nhwc = 0);
 int run_factor_tc(const Operand& X, long long rows, int d, float alpha,
                   float beta, float* out, void* workspace,
@@ -304,6 +305,12 @@ size_t tc_factor_group_workspace_bytes(int count, const FactorJob* jobs,
 size_t tc_stage_bytes(long long rows, int d);
 int tc_stage_group(int count, const FactorJob* jobs, char* ws, void* tmaps,
                    cudaStream_t stream);
+// Factors from row-major staged planes (gram.cu).
+bool gram_grid_job(const FactorJob& job);   // shifted products
+size_t gram_workspace_bytes(int count, const FactorJob* jobs);
+int run_factor_group_gram(int count, const FactorJob* jobs, void* workspace,
+                          size_t workspace_bytes, cudaStream_t stream);
+int gram_status_read(int* out);
 int run_factor_group_tc(int count, const FactorJob* jobs, void* workspace,
                         size_t workspace_bytes, cudaStream_t stream,
                         bool staged = true);

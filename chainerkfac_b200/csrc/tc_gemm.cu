@@ -1599,8 +1599,8 @@ static long long tc_group_chunk(int count, const FactorJob* jobs) {
   return work / (waves * sm_count());
 }
 
-size_t tc_factor_group_workspace_bytes(int count, const FactorJob* jobs,
-                                       bool staged) {
+static size_t tc_pair_workspace_bytes(int count, const FactorJob* jobs,
+                                      bool staged) {
   const long long chunk = tc_group_chunk(count, jobs);
   staged = staged && tc_staged();
   size_t total = 0;
@@ -1613,6 +1613,39 @@ size_t tc_factor_group_workspace_bytes(int count, const FactorJob* jobs,
       total += (size_t)s.splits * s.tiles * TC_BM * TC_BN * sizeof(float);
   }
   return total;
+}
+
+// Factors that are built from staged planes (gram.cu), unless the caller chose
+// the staging pass of stage.cu or gives no workspace:
+//  * 3 x 3 convolutions as shifted products, at any size (32 images, us per
+//    factor before and now: 64 channels 56 x 56 228 -> 78, 256 channels 14 x 14
+//    171 -> 62; 8 images of 64 channels 14 x 14 68 -> 41);
+//  * wide factors, where the gather feeds every element to many tiles (1568 x
+//    2048: 57 -> 29; even at 1000 columns, slower below);
+//  * patches of strided convolutions with many channels (1x1, 512 channels
+//    28 x 28 channels-last: 84 -> 27; 3x3, 256 channels 28 x 28: 199 -> 155;
+//    the 3-channel 7x7 stem stays with the gather, 160 against 486).
+static bool tc_uses_gram(const FactorJob& job) {
+  if (tc_staged()) return false;
+  if (gram_grid_job(job)) return true;
+  if ((double)job.rows * job.d < 2e6) return false;
+  return job.d >= 1024 || (job.X.mode == 1 && job.X.C >= 128);
+}
+
+static void tc_by_feed(int count, const FactorJob* jobs, bool staged,
+                       std::vector<FactorJob>& gram,
+                       std::vector<FactorJob>& pair) {
+  for (int i = 0; i < count; ++i)
+    (staged && tc_uses_gram(jobs[i]) ? gram : pair).push_back(jobs[i]);
+}
+
+size_t tc_factor_group_workspace_bytes(int count, const FactorJob* jobs,
+                                       bool staged) {
+  std::vector<FactorJob> gram, pair;
+  tc_by_feed(count, jobs, staged, gram, pair);
+  return std::max(
+      gram_workspace_bytes((int)gram.size(), gram.data()),
+      tc_pair_workspace_bytes((int)pair.size(), pair.data(), staged));
 }
 
 // Per-device helper stream: the strided and the im2col launch of a grouped
@@ -1645,14 +1678,14 @@ struct alignas(64) TmapBlob {     // a CUtensorMap, opaque here
   unsigned char b[128];
 };
 
-int run_factor_group_tc(int count, const FactorJob* jobs, void* workspace,
-                        size_t workspace_bytes, cudaStream_t main_stream,
-                        bool staged) {
+static int run_factor_group_pair(int count, const FactorJob* jobs,
+                                 void* workspace, size_t workspace_bytes,
+                                 cudaStream_t main_stream, bool staged) {
   cudaStream_t stream = main_stream;
   int rc = tc_prepare();
   if (rc != KFAC_OK) return rc;
   staged = staged && tc_staged();
-  const size_t need = tc_factor_group_workspace_bytes(count, jobs, staged);
+  const size_t need = tc_pair_workspace_bytes(count, jobs, staged);
   if (need > 0 && (workspace == nullptr || workspace_bytes < need))
     return fail(KFAC_ERR_WORKSPACE,
                 "factor: workspace of %zu bytes needed, %zu given", need,
@@ -1664,14 +1697,6 @@ int run_factor_group_tc(int count, const FactorJob* jobs, void* workspace,
   std::vector<ReduceItem> reduces;
   std::vector<PadJob> pads;
   int pad_items = 0;
-  for (int i = 0; i < count; ++i) {
-    KFAC_REQUIRE(jobs[i].out != nullptr && jobs[i].X.base != nullptr,
-                 "factor: null pointer");
-    KFAC_REQUIRE(jobs[i].rows > 0 && jobs[i].d > 0 &&
-                     jobs[i].rows < (1LL << 31),
-                 "factor: rows=%lld d=%d out of range", jobs[i].rows,
-                 jobs[i].d);
-  }
   const TmapBlob* dev_maps = nullptr;
   if (staged) {
     // staging pass: X^T of every job as two bf16 planes, two tensor maps each
@@ -1864,9 +1889,31 @@ int run_factor_group_tc(int count, const FactorJob* jobs, void* workspace,
   return KFAC_OK;
 }
 
-int run_factor_tc(const Operand& X, long long rows, int d, float alpha,
-                  float beta, float* out, void* workspace,
-                  size_t workspace_bytes, cudaStream_t stream, bool staged) {
+int run_factor_group_tc(int count, const FactorJob* jobs, void* workspace,
+                        size_t workspace_bytes, cudaStream_t stream,
+                        bool staged) {
+  for (int i = 0; i < count; ++i) {
+    KFAC_REQUIRE(jobs[i].out != nullptr && jobs[i].X.base != nullptr,
+                 "factor: null pointer");
+    KFAC_REQUIRE(jobs[i].rows > 0 && jobs[i].d > 0 &&
+                     jobs[i].rows < (1LL << 31),
+                 "factor: rows=%lld d=%d out of range", jobs[i].rows,
+                 jobs[i].d);
+  }
+  std::vector<FactorJob> gram, pair;
+  tc_by_feed(count, jobs, staged, gram, pair);
+  if (!gram.empty()) {
+    const int rc = run_factor_group_gram((int)gram.size(), gram.data(),
+                                         workspace, workspace_bytes, stream);
+    if (rc != KFAC_OK) return rc;
+  }
+  if (pair.empty()) return KFAC_OK;
+  return run_factor_group_pair((int)pair.size(), pair.data(), workspace,
+                               workspace_bytes, stream, staged);
+}
+
+static FactorJob lone_job(const Operand& X, long long rows, int d, float alpha,
+                          float beta, float* out) {
   FactorJob job;
   job.X = X;
   job.rows = rows;
@@ -1876,6 +1923,21 @@ int run_factor_tc(const Operand& X, long long rows, int d, float alpha,
   job.alpha = alpha;
   job.beta = beta;
   job.out = out;
+  return job;
+}
+
+// Workspace of a factor built on its own from any operand of this geometry.
+size_t tc_lone_workspace_bytes(const Operand& X, long long rows, int d) {
+  const FactorJob job = lone_job(X, rows, d, 1.f, 0.f, nullptr);
+  return std::max(tc_factor_workspace_bytes(rows, d) +
+                      tc_pad_bytes(X, job.n),
+                  tc_factor_group_workspace_bytes(1, &job, true));
+}
+
+int run_factor_tc(const Operand& X, long long rows, int d, float alpha,
+                  float beta, float* out, void* workspace,
+                  size_t workspace_bytes, cudaStream_t stream, bool staged) {
+  const FactorJob job = lone_job(X, rows, d, alpha, beta, out);
   return run_factor_group_tc(1, &job, workspace, workspace_bytes, stream,
                              staged);
 }
@@ -1961,6 +2023,9 @@ extern "C" int kfac_tc_status(int* status_out) {
   int w = 0;
   int rc = kfac::diag_status_read(&w);
   if (rc != KFAC_OK) return rc;
-  *status_out = v | w;
+  int u = 0;
+  rc = kfac::gram_status_read(&u);
+  if (rc != KFAC_OK) return rc;
+  *status_out = v | w | u;
   return KFAC_OK;
 }

@@ -237,6 +237,51 @@ def test_scratch_buffers_are_per_stream(ops):
     assert rel(host(o2), w2.T @ w2 / 80000) < FACTOR_TOL
 
 
+@pytest.mark.parametrize('channels_last', [False, True])
+@pytest.mark.parametrize('n,c,h,w,stride', [
+    (2, 32, 8, 8, 1), (3, 33, 5, 9, 1), (1, 64, 1, 1, 1), (2, 64, 14, 1, 1),
+    (5, 70, 7, 7, 1), (4, 128, 9, 6, 1), (2, 257, 4, 4, 1), (33, 512, 7, 7, 1),
+    (2, 130, 41, 40, 2)])
+def test_factor_of_3x3_convolutions(ops, engine, n, c, h, w, stride,
+                                    channels_last):
+    """Patch factors as shifted products (stride 1: one granule of channels,
+    ragged granules, several tiles, images of one row or column) and from
+    staged patches, on top of an existing average, against fp64."""
+    if engine == 0 and channels_last:
+        pytest.skip('channels-last inputs belong to the tensor-core engine')
+    torch.manual_seed(2)
+    x = torch.randn(n, c, h, w, device='cuda').clamp_(min=0)
+    u = torch.nn.functional.unfold(x.double(), 3, padding=1, stride=stride)
+    u = u.transpose(1, 2).reshape(-1, 9 * c)
+    if channels_last:
+        x = x.contiguous(memory_format=torch.channels_last)
+    out = torch.full((9 * c, 9 * c), 3.0, device='cuda')
+    ops.factor_group([ops.conv_input_item(x, 3, stride, 1, False, 1.0 / n, 0.5,
+                                          out)], x.device)
+    ref = u.t() @ u / n + 1.5
+    assert rel(host(out), host(ref)) < FACTOR_TOL
+    check_symmetric(host(out))
+
+
+@pytest.mark.parametrize('rows,d,ones', [
+    (2000, 1024, False), (1999, 1025, False), (1500, 1411, True)])
+def test_wide_factor_from_staged_planes(ops, rows, d, ones):
+    """Tiles, strips and granules that the last column cuts."""
+    torch.manual_seed(3)
+    x = torch.randn(rows, d - int(ones), device='cuda')
+    out = torch.full((d, d), 3.0, device='cuda')
+    ops.factor_group([ops.dense_item(x, ones, 0.5, 0.5, out)], x.device)
+    xd = x.double()
+    if ones:
+        xd = torch.cat([xd, xd.new_ones(rows, 1)], 1)
+    assert rel(host(out), host(0.5 * (xd.t() @ xd) + 1.5)) < FACTOR_TOL
+    check_symmetric(host(out))
+    xt = x.t().contiguous()
+    if not ones:
+        ops.factor_group([ops.dense_t_item(xt, 1.0, 0.0, out)], x.device)
+        assert rel(host(out), host(xd.t() @ xd)) < FACTOR_TOL
+
+
 def test_factor_builds_from_staged_operands(ops, engine):
     """The optional operand feed of the factor builds (staging pass that
     writes X^T as two bf16 planes, TMA boxes into the tile kernel) against the
