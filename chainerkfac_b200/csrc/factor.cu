@@ -1255,6 +1255,7 @@ static int job_from_item(const kfac_factor_item& it, FactorJob& job) {
   job.out = it.out;
   job.n = it.n;
   job.nhwc = 0;
+  job.grouped = 1;
   KFAC_REQUIRE(it.layout == 0 ||
                    (it.layout == 1 && it.kind == KFAC_FACTOR_CONV_INPUT),
                "factor_group: layout %d of item kind %d unsupported", it.layout,

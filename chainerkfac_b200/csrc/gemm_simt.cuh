@@ -295,6 +295,7 @@ struct FactorJob {      // one factor of a grouped build
   int d;
   int n;                // batch size (im2col operands)
   int nhwc;             // im2col operand: the tensor is stored channels-last
+  int grouped;          // part of a grouped build (not a factor on its own)
   float alpha, beta;
   float* out;
 };
@@ -306,7 +307,8 @@ size_t tc_stage_bytes(long long rows, int d);
 int tc_stage_group(int count, const FactorJob* jobs, char* ws, void* tmaps,
                    cudaStream_t stream);
 // Factors from row-major staged planes (gram.cu).
-bool gram_grid_job(const FactorJob& job);   // shifted products
+bool gram_grid_job(const FactorJob& job);     // shifted products
+bool gram_direct_job(const FactorJob& job);   // no staged planes needed
 size_t gram_workspace_bytes(int count, const FactorJob* jobs);
 int run_factor_group_gram(int count, const FactorJob* jobs, void* workspace,
                           size_t workspace_bytes, cudaStream_t stream);

@@ -37,6 +37,23 @@
 
 namespace kfac {
 
+// Whether the products of an operand can be formed without staged planes
+// (direct_kernel): no appended column, 16-byte pitches and addresses; with the
+// rows contiguous one tile wide only, and images of 32 rows at least (a block
+// of 32 rows never spans two of them; a factor built on its own, whose
+// workspace is asked for without the image size, does not come here).
+bool gram_direct_job(const FactorJob& job) {
+  const Operand& X = job.X;
+  if (X.mode != 0 || X.extra_idx >= 0 || X.ncols != job.d) return false;
+  if (reinterpret_cast<uintptr_t>(X.base) & 15) return false;
+  if (X.s_col == 1 && X.period == 1) return X.s_outer % 4 == 0;
+  if (!job.grouped || job.d > 256 || X.s_col % 4 != 0) return false;
+  if (X.period == 1) return X.s_outer == 1;
+  return X.s_inner == 1 && X.period >= 32 && X.period % 4 == 0 &&
+         X.s_col == X.period && X.s_outer == X.s_col * X.ncols &&
+         job.rows % X.period == 0;
+}
+
 // Shifted products pay once the channels fill a good part of a granule; a
 // narrower convolution has few columns, and its patches are small too.
 bool gram_grid_job(const FactorJob& job) {
@@ -139,6 +156,25 @@ __host__ __device__ __forceinline__ void tri_of(int t, int& i, int& j) {
   j = t - i * (i + 1) / 2;
 }
 
+// Accumulator columns c0, c0 + 1, .. of a warp's 32 rows to its partial tile,
+// 32 columns at a time (columns up to the next multiple of 16 past `cend` may
+// be stored as well: they exist in the tile and nobody reads them).
+__device__ __forceinline__ void store_partial(unsigned taddr, float* p, int c0,
+                                              int cend, int step) {
+  for (; c0 < cend; c0 += step) {
+    float v[16], w[16];
+    tc_ld16_pair(taddr + c0, taddr + c0 + 16, v, w);
+    float* q = p + (long long)(c0 >> 2) * 1024;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      *reinterpret_cast<float4*>(q + i * 1024) =
+          make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+      *reinterpret_cast<float4*>(q + (4 + i) * 1024) =
+          make_float4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+    }
+  }
+}
+
 // One tile of up to 256 x 256 (two 128-row accumulators in tensor memory) over
 // one split of the contraction.  Bound by the tensor cores: 12 MMAs of 128 x
 // 256 x 16 (1536 cycles) per 64 KB stage.  Warp 0 issues the copies, warp 1
@@ -208,7 +244,7 @@ gram_kernel(const GramGroup* __restrict__ groups, int ngroups) {
   const int nvalid = sym ? min(64 * nb, ((g.d - 256 * tj) + 15) & ~15) : 64 * nb;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // the tensor maps were written by a copy that precedes this launch
       asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;"
                    ::"l"(g.tmap) : "memory");
@@ -248,7 +284,7 @@ gram_kernel(const GramGroup* __restrict__ groups, int ngroups) {
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // a diagonal tile needs columns 0..127 only for its first 128 rows
       const unsigned id0 = gr_idesc(share ? min(nvalid, 128) : nvalid);
       const unsigned id1 = gr_idesc(nvalid);
@@ -297,14 +333,8 @@ gram_kernel(const GramGroup* __restrict__ groups, int ngroups) {
     if (ok && 128 * h + 32 * q < rows) {
       float* p = g.partial +
                  ((long long)split * g.tiles + tile) * GR_TILE + row * 4;
-      for (int c0 = 0; c0 < cend; c0 += 16) {
-        float v[16];
-        tc_ld16(tmem + ((unsigned)(32 * q) << 16) + (unsigned)(256 * h + c0), v);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<float4*>(p + (long long)((c0 >> 2) + i) * 1024) =
-              make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-      }
+      store_partial(tmem + ((unsigned)(32 * q) << 16) + (unsigned)(256 * h), p,
+                    0, cend, 32);
     }
   }
   if (tid == 0 && ctl->abort_flag != 0) {
@@ -315,6 +345,326 @@ gram_kernel(const GramGroup* __restrict__ groups, int ngroups) {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+                 ::"r"(tmem), "r"(512)
+                 : "memory");
+}
+
+__device__ __forceinline__ void gr_split2(float x0, float x1, unsigned& hi,
+                                          unsigned& lo) {
+  // bf16 by adding half an ulp (ties away from zero), the remainder likewise
+  const unsigned r0 = __float_as_uint(x0) + 0x8000u;
+  const unsigned r1 = __float_as_uint(x1) + 0x8000u;
+  hi = __byte_perm(r0, r1, 0x7632);
+  const float l0 = x0 - __uint_as_float(r0 & 0xffff0000u);
+  const float l1 = x1 - __uint_as_float(r1 & 0xffff0000u);
+  lo = __byte_perm(__float_as_uint(l0) + 0x8000u,
+                   __float_as_uint(l1) + 0x8000u, 0x7632);
+}
+
+// ---------------------------------------------------- products without planes
+// Plain operands whose rows TMA can read as they are (16-byte pitches and
+// addresses).  32 KB of fp32 per stage arrive by TMA, sixteen warps split them
+// into the two bf16 planes of the MMA operands, so an element is read from
+// memory once per tile and never staged.  Up to 256 columns there is one tile
+// per split and the kernel is bound by HBM (96 KB in flight per SM); wider
+// factors are bound by the tensor cores and the shared-memory traffic of the
+// split.  us per factor, eight in a group (the gather kernel with one k-block
+// of loads in flight before): 100 352 x 64 36 -> 10, 100 352 x 256 52 -> 28,
+// 25 088 x 512 40 -> 30, 6272 x 1024 41 -> 30, 1568 x 2048 57 -> 28.
+//
+// Columns contiguous (rows x d): a granule is R rows of 64 columns, MN-major.
+// Rows contiguous (KM; n x d x hw, up to 256 columns): sub-blocks of `width`
+// columns x 32 rows, K-major with 64-byte swizzle.
+constexpr int DR_RAW = 32768;          // fp32 bytes of a stage = bytes of planes
+// Two sets of split warps take turns; every slot of either ring belongs to one
+// set for good, so that a set waits on each use of its barriers (a wait by
+// parity that skips a use may take an older phase for the one it wants).
+constexpr int DR_RAWS = 4;             // fp32 slots (2 and 4: 8 % slower)
+constexpr int DR_PLANES = 2;           // slots of split planes
+static_assert(DR_RAWS % 2 == 0 && DR_PLANES % 2 == 0, "two sets of warps");
+constexpr int DR_SPLIT = 16;           // split / epilogue warps
+constexpr int DR_THREADS = 32 * (DR_SPLIT + 2);   // and one each: TMA, MMA
+
+struct DirectGroup {
+  const void* tmap;
+  float* partial;
+  int nkb;             // k-blocks of 32 rows
+  int kb_split;        // per split: whole stages
+  int tiles;
+  int unit_begin;
+  int d;
+  int width;           // columns of a tile side: 64, 128, 256
+  int box_rows;        // rows of a TMA box
+  int per_image;       // KM: k-blocks of 32 rows per image
+};
+
+struct DrControl {
+  DirectGroup g;
+  unsigned long long raw_full[DR_RAWS], raw_empty[DR_RAWS];
+  unsigned long long full[DR_PLANES], empty[DR_PLANES];
+  unsigned long long accum;
+  unsigned tmem_base;
+  volatile int abort_flag;
+  int found;
+};
+
+// (planes first: a 128-row operand of a 64-column tile reads past its planes,
+// into rows of the accumulator that nobody uses)
+constexpr int DR_SMEM =
+    (DR_RAWS + DR_PLANES) * DR_RAW + ((int)sizeof(DrControl) + 1023) / 1024 * 1024 + 1024;
+static_assert(DR_SMEM <= 227 * 1024, "direct kernel shared memory");
+
+__device__ __forceinline__ unsigned long long dr_desc(unsigned addr, int lbo,
+                                                      int sbo, int swizzle) {
+  unsigned long long d = 0;
+  d |= (unsigned long long)((addr & 0x3FFFF) >> 4);
+  d |= (unsigned long long)(lbo >> 4) << 16;
+  d |= (unsigned long long)(sbo >> 4) << 32;
+  d |= (unsigned long long)1 << 46;
+  d |= (unsigned long long)swizzle << 61;
+  return d;
+}
+
+__device__ __forceinline__ void dr_load3(unsigned dst, const void* tmap, int x,
+                                         int y, int z, unsigned bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::"
+      "complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+
+template <bool KM>
+__global__ void __launch_bounds__(DR_THREADS, 1)
+direct_kernel(const DirectGroup* __restrict__ groups, int ngroups) {
+  extern __shared__ unsigned char gr_smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(gr_smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* raw = smem + DR_PLANES * DR_RAW;
+  DrControl* ctl =
+      reinterpret_cast<DrControl*>(raw + DR_RAWS * DR_RAW);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int unit = blockIdx.x;
+  for (int i = tid; i < ngroups; i += DR_THREADS) {
+    const int lo = groups[i].unit_begin;
+    const int hi = i + 1 < ngroups ? groups[i + 1].unit_begin : 0x7fffffff;
+    if (lo <= unit && unit < hi) ctl->found = i;
+  }
+  __syncthreads();
+  {
+    const int* s = reinterpret_cast<const int*>(groups + ctl->found);
+    int* d = reinterpret_cast<int*>(&ctl->g);
+    for (int i = tid; i < (int)(sizeof(DirectGroup) / sizeof(int));
+         i += DR_THREADS)
+      d[i] = s[i];
+  }
+  if (tid == 0) {
+    for (int s = 0; s < DR_RAWS; ++s) {
+      mbar_init(&ctl->raw_full[s], 1);
+      mbar_init(&ctl->raw_empty[s], 8);
+    }
+    for (int s = 0; s < DR_PLANES; ++s) {
+      mbar_init(&ctl->full[s], 8);
+      mbar_init(&ctl->empty[s], 1);
+    }
+    mbar_init(&ctl->accum, 1);
+    ctl->abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == DR_SPLIT + 1) {
+    asm volatile(
+        "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+        ::"r"(smem_u32(&ctl->tmem_base)), "r"(512)
+        : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
+                 ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+  const DirectGroup& g = ctl->g;
+  const unsigned tmem = ctl->tmem_base;
+  const int local = unit - g.unit_begin;
+  const int split = local / g.tiles, tile = local - split * g.tiles;
+  int ti, tj;
+  tri_of(tile, ti, tj);
+  const bool share = ti == tj;
+  const int width = g.width;
+  // rows of a stage: 32 KB of one side, or of both
+  const int R = share ? 8192 / width : 16;
+  const int row0 = split * g.kb_split * 32;
+  const int nst =
+      (min(g.kb_split, g.nkb - split * g.kb_split) * 32 + R - 1) / R;
+  const int nvalid = min(width, (g.d - 256 * tj + 15) & ~15);
+  const bool two = g.d - 256 * ti > 128;
+
+  if (warp == DR_SPLIT) {
+    if (elect_one()) {
+      asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;"
+                   ::"l"(g.tmap) : "memory");
+      for (int st = 0; st < nst; ++st) {
+        const int s = st % DR_RAWS;
+        if (st >= DR_RAWS &&
+            !mbar_wait_status(&ctl->raw_empty[s], ((st / DR_RAWS) - 1) & 1,
+                              &ctl->abort_flag, &g_gram_status))
+          break;
+        const unsigned bar = smem_u32(&ctl->raw_full[s]);
+        asm volatile(
+            "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+            ::"r"(bar), "r"(DR_RAW) : "memory");
+        unsigned dst = smem_u32(raw + s * DR_RAW);
+        if (KM) {
+          // sub-blocks of 32 rows (of one image each; past the end of an
+          // image or of the operand: zeros)
+          const int sub = 256 / width;
+          for (int q = 0; q < sub; ++q, dst += width * 128) {
+            const int b = (row0 >> 5) + st * sub + q;
+            const int img = b / g.per_image;
+            dr_load3(dst, g.tmap, 32 * (b - img * g.per_image), 0, img, bar);
+          }
+        } else if (share) {
+          const int r = row0 + st * R;
+          for (int c = 0; c < width; c += 64)
+            for (int q = 0; q < R; q += g.box_rows, dst += g.box_rows * 256)
+              dr_load3(dst, g.tmap, 256 * tj + c, r + q, 0, bar);
+        } else {
+          const int r = row0 + st * 16;
+          for (int c = 0; c < 512; c += 64, dst += 16 * 256)
+            dr_load3(dst, g.tmap, c < 256 ? 256 * ti + c : 256 * (tj - 1) + c,
+                     r, 0, bar);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == DR_SPLIT + 1) {
+    if (elect_one()) {
+      const unsigned major = KM ? 0u : (1u << 15) | (1u << 16);
+      const unsigned base = (1u << 4) | (1u << 7) | (1u << 10) | major |
+                            ((unsigned)(128 >> 4) << 24);
+      const unsigned id1 = base | ((unsigned)(nvalid >> 3) << 17);
+      const unsigned id0 =
+          base | ((unsigned)((share ? min(nvalid, 128) : nvalid) >> 3) << 17);
+      // bytes of a plane of one granule (or sub-block); the descriptors of a
+      // stage differ by their start address (16-byte units) alone
+      const int plane = KM ? width * 64 : R * 128;
+      const unsigned long long lo = plane >> 4;
+      const unsigned long long to_b = share ? 0 : 8 * plane >> 4;
+      const unsigned long long up = (KM ? 128 * 64 : 4 * plane) >> 4;
+      const unsigned long long first =
+          dr_desc(smem_u32(smem), KM ? 16 : (width == 64 ? 0 : 2 * plane),
+                  KM ? 512 : 1024, KM ? 4 : 2);
+      // k steps of 16 rows: KM: two per sub-block of 2 * plane bytes
+      const unsigned long long odd = (KM ? 32 : 2048) >> 4;
+      const unsigned long long even = (KM ? 2 * plane - 32 : 2048) >> 4;
+      const int steps = KM ? 2 * (256 / width) : R / 16;
+      for (int st = 0; st < nst; ++st) {
+        const int s = st % DR_PLANES;
+        if (!mbar_wait_status(&ctl->full[s], (st / DR_PLANES) & 1,
+                              &ctl->abort_flag, &g_gram_status))
+          break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        unsigned long long a = first + (s * DR_RAW >> 4);
+        unsigned acc = st != 0;
+#pragma unroll 1
+        for (int kk = 0; kk < steps; ++kk) {
+          const unsigned long long bb = a + to_b;
+          gr_mma(tmem, a + lo, bb, id0, acc);
+          gr_mma(tmem, a, bb + lo, id0, 1);
+          gr_mma(tmem, a, bb, id0, 1);
+          if (two) {
+            gr_mma(tmem + 256, a + up + lo, bb, id1, acc);
+            gr_mma(tmem + 256, a + up, bb + lo, id1, 1);
+            gr_mma(tmem + 256, a + up, bb, id1, 1);
+          }
+          acc = 1;
+          a += (kk & 1) ? even : odd;
+        }
+        tc_commit(&ctl->empty[s]);
+      }
+      tc_commit(&ctl->accum);
+    }
+    __syncwarp();
+  } else {
+    // split: eight warps share a stage and two sets of them take turns (one
+    // set needs 3000 cycles from the arrival of a stage to its hand-over).  A
+    // thread turns 8 consecutive values into 16 bytes of each plane, four
+    // times per stage.  The two halves are read in an order that keeps the
+    // lanes of a quarter warp on different banks.
+    const int tid = threadIdx.x & 255;
+    const int rows = KM ? width : R;       // rows of one plane
+    const int sub = KM ? 64 : 128;         // bytes of a plane row
+    const int chunk = KM ? tid & 3 : tid & 7;
+    unsigned src[4], dst[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int F = (KM ? tid >> 2 : tid >> 3) + (KM ? 64 : 32) * i;
+      const int blk = F / rows, r = F - blk * rows;
+      src[i] = F * (KM ? 128 : 256) + chunk * 32;
+      dst[i] = blk * 2 * rows * sub + r * sub +
+               ((KM ? chunk ^ ((r >> 1) & 3) : chunk ^ (r & 7)) << 4);
+    }
+    const int lo = rows * sub;
+    const int h = KM ? (tid >> 2) & 1 : chunk >> 2;
+    for (int st = warp >> 3; st < nst; st += 2) {
+      const int s = st % DR_RAWS, ps = st % DR_PLANES;
+      if (!mbar_wait_status(&ctl->raw_full[s], (st / DR_RAWS) & 1,
+                            &ctl->abort_flag, &g_gram_status))
+        break;
+      const unsigned char* p = raw + s * DR_RAW;
+      float4 a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[i] = *reinterpret_cast<const float4*>(p + src[i] + 16 * h);
+        b[i] = *reinterpret_cast<const float4*>(p + src[i] + 16 * (1 - h));
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->raw_empty[s]);
+      if (st >= DR_PLANES &&
+          !mbar_wait_status(&ctl->empty[ps], ((st / DR_PLANES) - 1) & 1,
+                            &ctl->abort_flag, &g_gram_status))
+        break;
+      unsigned char* q = smem + ps * DR_RAW;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        unsigned hi[4], l[4];
+        gr_split2(a[i].x, a[i].y, hi[0], l[0]);
+        gr_split2(a[i].z, a[i].w, hi[1], l[1]);
+        gr_split2(b[i].x, b[i].y, hi[2], l[2]);
+        gr_split2(b[i].z, b[i].w, hi[3], l[3]);
+        *reinterpret_cast<uint4*>(q + dst[i]) =
+            h ? make_uint4(hi[2], hi[3], hi[0], hi[1])
+              : make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(q + dst[i] + lo) =
+            h ? make_uint4(l[2], l[3], l[0], l[1])
+              : make_uint4(l[0], l[1], l[2], l[3]);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->full[ps]);
+    }
+    // epilogue, as in gram_kernel
+    bool ok =
+        mbar_wait_status(&ctl->accum, 0, &ctl->abort_flag, &g_gram_status);
+    ok = __all_sync(0xffffffffu, ok);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int hh = (warp >> 2) & 1, q = warp & 3;
+    const int row = 128 * hh + 32 * q + lane;
+    const int cend = share && hh == 0 ? min(nvalid, 128) : nvalid;
+    if (ok && 128 * hh + 32 * q < g.d - 256 * ti) {
+      float* p = g.partial +
+                 ((long long)split * g.tiles + tile) * GR_TILE + row * 4;
+      store_partial(tmem + ((unsigned)(32 * q) << 16) + (unsigned)(256 * hh), p,
+                    32 * (warp >> 3), cend, 64);
+    }
+  }
+  if (tid == 0 && ctl->abort_flag != 0) {
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == DR_SPLIT + 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
                  ::"r"(tmem), "r"(512)
                  : "memory");
@@ -344,18 +694,6 @@ struct StageJob {
 constexpr int kStageJobs = 512;
 constexpr int kStageRowsC = 128;   // rows per item, columns contiguous
 constexpr int kStageRowsK = 32;    // rows per item, rows contiguous
-
-__device__ __forceinline__ void gr_split2(float x0, float x1, unsigned& hi,
-                                          unsigned& lo) {
-  // bf16 by adding half an ulp (ties away from zero), the remainder likewise
-  const unsigned r0 = __float_as_uint(x0) + 0x8000u;
-  const unsigned r1 = __float_as_uint(x1) + 0x8000u;
-  hi = __byte_perm(r0, r1, 0x7632);
-  const float l0 = x0 - __uint_as_float(r0 & 0xffff0000u);
-  const float l1 = x1 - __uint_as_float(r1 & 0xffff0000u);
-  lo = __byte_perm(__float_as_uint(l0) + 0x8000u,
-                   __float_as_uint(l1) + 0x8000u, 0x7632);
-}
 
 __device__ __forceinline__ void gr_store8(const StageJob& j, int row, int col,
                                           const float v[8]) {
@@ -896,6 +1234,8 @@ inline int up32(long long v) { return (int)((v + 31) & ~31LL); }
 // Plan of one job: its plane and its groups of products.
 struct JobPlan {
   bool grid;               // shifted products of a 3 x 3 convolution
+  int direct;              // no planes: 1 columns, 2 rows contiguous
+  int width, per_image;    // direct only
   int cols, cp;            // columns of the plane
   int prows;               // its rows
   int line[8];
@@ -908,6 +1248,27 @@ struct JobPlan {
 void plan_job(const FactorJob& job, JobPlan& p) {
   const Operand& X = job.X;
   p.grid = gram_grid_job(job);
+  p.direct = gram_direct_job(job) ? (X.s_col == 1 && X.period == 1 ? 1 : 2)
+                                        : 0;
+  if (p.direct) {
+    p.cols = job.d;
+    p.prows = 0;
+    p.plane_bytes = 0;
+    p.width = job.d <= 64 ? 64 : (job.d <= 128 ? 128 : 256);
+    const int t = (job.d + 255) / 256;
+    p.ngroups = 1;
+    p.tiles[0] = t * (t + 1) / 2;
+    p.nga[0] = (job.d + GR_GRAN - 1) / GR_GRAN;
+    // k-blocks of 32 rows
+    if (p.direct == 2) {
+      const int hw = X.period == 1 ? (int)job.rows : X.period;
+      p.per_image = (hw + 31) / 32;
+      p.nkb[0] = (int)(job.rows / hw) * p.per_image;
+    } else {
+      p.nkb[0] = (int)((job.rows + 31) / 32);
+    }
+    return;
+  }
   if (!p.grid) {
     p.cols = job.d;
     p.prows = (int)job.rows;
@@ -946,8 +1307,13 @@ void plan_job(const FactorJob& job, JobPlan& p) {
   p.plane_bytes = ((size_t)p.prows * p.cp * 2 + 255) & ~(size_t)255;
 }
 
-// Duration of a k-block of one tile in units of a 128 x 256 product.
-inline int group_cost(const JobPlan& p, int k) { return p.nga[k] > 2 ? 2 : 1; }
+// Duration of a k-block of one tile in quarters of a 128 x 256 product (about
+// 200 cycles): products of staged planes by the tensor cores, without planes
+// by the memory traffic of one tile side.
+inline int group_cost(const JobPlan& p, int k) {
+  if (p.direct) return p.tiles[0] > 1 ? 8 : p.width / 32;
+  return p.nga[k] > 2 ? 8 : 4;
+}
 
 // A CTA keeps at least 16 k-blocks so that its prologue and epilogue stay
 // amortised, and never accumulates more than 128: the tensor core adds each
@@ -959,24 +1325,33 @@ void split_job(JobPlan& p, long long target) {
   p.partial_bytes = 0;
   for (int k = 0; k < p.ngroups; ++k) {
     long long chunk = target / group_cost(p, k);
-    chunk = std::max(16LL, std::min(128LL, chunk));
-    const long long sp = std::max(1LL, (p.nkb[k] + chunk / 2) / chunk);
+    // (one tile without planes: eight stages)
+    const long long least =
+        p.direct && p.tiles[0] == 1 ? 2048 / p.width : 16;
+    chunk = std::max(least, std::min(128LL, chunk));
+    const long long sp = std::max(1LL, p.nkb[k] / chunk);
     p.kb_split[k] = (int)((p.nkb[k] + sp - 1) / sp);
+    if (p.direct) {
+      // whole stages: 16 rows of two sides, or 256 / width k-blocks of one
+      // (tiles on the diagonal of a wide factor: 32 rows)
+      const int per = p.tiles[0] > 1 ? 1 : 256 / p.width;
+      p.kb_split[k] = (p.kb_split[k] + per - 1) / per * per;
+    }
     p.splits[k] = (p.nkb[k] + p.kb_split[k] - 1) / p.kb_split[k];
     p.partial_bytes +=
         (size_t)p.splits[k] * p.tiles[k] * GR_TILE * sizeof(float);
   }
 }
 
-// Work per CTA: about three waves over the SMs (2 to 4 measure the same, 6
-// waves 4 % slower).
+// Work per CTA: at most two waves over the SMs, so that the 10 us a CTA spends
+// before its first and behind its last product stay small.
 long long split_target(const std::vector<JobPlan>& plans, size_t b, size_t e) {
   long long work = 0;
   for (size_t i = b; i < e; ++i)
     for (int k = 0; k < plans[i].ngroups; ++k)
       work += (long long)plans[i].tiles[k] * plans[i].nkb[k] *
               group_cost(plans[i], k);
-  return work / (3LL * sm_count());
+  return work / (2LL * sm_count()) + 1;
 }
 
 // Jobs are worked off in batches whose planes stay below this many bytes, so
@@ -1024,6 +1399,12 @@ static int gram_prepare() {
   if (!done[dev]) {
     KFAC_CUDA(cudaFuncSetAttribute(
         gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM));
+    KFAC_CUDA(cudaFuncSetAttribute(direct_kernel<false>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   DR_SMEM));
+    KFAC_CUDA(cudaFuncSetAttribute(direct_kernel<true>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   DR_SMEM));
     KFAC_CUDA(cudaFuncSetAttribute(
         gram_expand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
         kXSmem));
@@ -1050,8 +1431,10 @@ static int gram_batch(const FactorJob* jobs, std::vector<JobPlan>& plans,
   std::vector<StageJob> stage[2];       // columns contiguous, rows contiguous
   int sitems[2] = {0, 0};
   std::vector<GramGroup> groups;
+  std::vector<DirectGroup> direct[2];   // columns contiguous, rows contiguous
   std::vector<GramOut> outs[2];         // plain, shifted
   int oitems[2] = {0, 0};
+  int direct_units[2] = {0, 0};
   void* dev_maps = nullptr;
   int rc = ring_alloc(n * sizeof(Map), &dev_maps);
   if (rc != KFAC_OK) return rc;
@@ -1060,6 +1443,53 @@ static int gram_batch(const FactorJob* jobs, std::vector<JobPlan>& plans,
     JobPlan& p = plans[i];
     split_job(p, target);
     const Operand& X = job.X;
+    if (p.direct) {
+      const bool km = p.direct == 2;
+      const long long hw = X.period == 1 ? job.rows : X.period;
+      DirectGroup g = {};
+      g.tmap = static_cast<const Map*>(dev_maps) + (i - b);
+      g.partial = reinterpret_cast<float*>(ws);
+      ws += p.partial_bytes;
+      g.nkb = p.nkb[0];
+      g.kb_split = p.kb_split[0];
+      g.tiles = p.tiles[0];
+      g.d = job.d;
+      g.width = p.width;
+      g.box_rows = p.tiles[0] > 1 ? 16 : 8192 / p.width;
+      g.per_image = p.per_image;
+      const cuuint64_t dims[3] = {(cuuint64_t)(km ? hw : job.d),
+                                  (cuuint64_t)(km ? job.d : job.rows),
+                                  (cuuint64_t)(km ? job.rows / hw : 1)};
+      const cuuint64_t pitch = (cuuint64_t)(km ? X.s_col : X.s_outer) * 4;
+      const cuuint64_t strides[2] = {pitch, pitch * dims[1]};
+      const cuuint32_t box[3] = {(cuuint32_t)(km ? 32 : GR_GRAN),
+                                 (cuuint32_t)(km ? p.width : g.box_rows), 1};
+      const cuuint32_t es[3] = {1, 1, 1};
+      const CUresult r = encode(
+          &maps[i - b].m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)X.base,
+          dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      if (r != CUDA_SUCCESS)
+        return fail(KFAC_ERR_CUDA,
+                    "factor: cuTensorMapEncodeTiled failed (%d) for a %lld x "
+                    "%d operand", (int)r, job.rows, job.d);
+      direct[km ? 1 : 0].push_back(g);
+      GramOut o = {};
+      o.out = job.out;
+      o.d = job.d;
+      o.alpha = job.alpha;
+      o.beta = job.beta;
+      o.partial[0] = g.partial;
+      o.splits[0] = p.splits[0];
+      o.tiles[0] = p.tiles[0];
+      const int rb = (job.d + 31) / 32;
+      o.strips = p.splits[0] <= 4;
+      o.item_begin = oitems[0];
+      oitems[0] += o.strips ? strips_before(rb) : rb * (rb + 1) / 2;
+      outs[0].push_back(o);
+      continue;
+    }
     StageJob s = {};
     s.base = X.base;
     s.extra = X.extra;
@@ -1157,6 +1587,24 @@ static int gram_batch(const FactorJob* jobs, std::vector<JobPlan>& plans,
                         : (o.strips ? strips_before(rb) : rb * (rb + 1) / 2);
     outs[w].push_back(o);
   }
+  for (int m = 0; m < 2; ++m) {
+    std::vector<DirectGroup>& v = direct[m];
+    if (v.empty()) continue;
+    // longest CTAs first
+    const auto cost = [](const DirectGroup& g) {
+      return g.kb_split * (g.tiles > 1 ? 8 : g.width / 32);
+    };
+    std::stable_sort(v.begin(), v.end(),
+                     [&](const DirectGroup& x, const DirectGroup& y) {
+                       return cost(x) > cost(y);
+                     });
+    int units = 0;
+    for (DirectGroup& g : v) {
+      g.unit_begin = units;
+      units += g.tiles * ((g.nkb + g.kb_split - 1) / g.kb_split);
+    }
+    direct_units[m] = units;
+  }
   // longest CTAs first
   std::stable_sort(groups.begin(), groups.end(),
                    [](const GramGroup& x, const GramGroup& y) {
@@ -1186,11 +1634,28 @@ static int gram_batch(const FactorJob* jobs, std::vector<JobPlan>& plans,
     KFAC_LAUNCH_CHECK(m == 0 ? "stage_cols_kernel" : "stage_rows_kernel");
   }
   void* dev = nullptr;
-  rc = upload(groups.data(), groups.size() * sizeof(GramGroup), stream, &dev);
-  if (rc != KFAC_OK) return rc;
-  gram_kernel<<<units, GR_THREADS, GR_SMEM, stream>>>(
-      static_cast<const GramGroup*>(dev), (int)groups.size());
-  KFAC_LAUNCH_CHECK("gram_kernel");
+  if (units > 0) {
+    rc = upload(groups.data(), groups.size() * sizeof(GramGroup), stream, &dev);
+    if (rc != KFAC_OK) return rc;
+    gram_kernel<<<units, GR_THREADS, GR_SMEM, stream>>>(
+        static_cast<const GramGroup*>(dev), (int)groups.size());
+    KFAC_LAUNCH_CHECK("gram_kernel");
+  }
+  for (int m = 0; m < 2; ++m) {
+    if (direct[m].empty()) continue;
+    rc = upload(direct[m].data(), direct[m].size() * sizeof(DirectGroup),
+                stream, &dev);
+    if (rc != KFAC_OK) return rc;
+    const DirectGroup* d_groups = static_cast<const DirectGroup*>(dev);
+    const int n_groups = (int)direct[m].size();
+    if (m == 0)
+      direct_kernel<false><<<direct_units[m], DR_THREADS, DR_SMEM, stream>>>(
+          d_groups, n_groups);
+    else
+      direct_kernel<true><<<direct_units[m], DR_THREADS, DR_SMEM, stream>>>(
+          d_groups, n_groups);
+    KFAC_LAUNCH_CHECK("direct_kernel");
+  }
   for (int w = 0; w < 2; ++w) {
     if (outs[w].empty()) continue;
     rc = upload(outs[w].data(), outs[w].size() * sizeof(GramOut), stream, &dev);

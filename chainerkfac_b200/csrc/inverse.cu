@@ -317,7 +317,7 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    if (tid == 0 && !ctl->abort_flag) {
+    if (warp == 0 && !ctl->abort_flag && elect_one()) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // columns below 32 kb of L' get nothing from this block of k
       const unsigned skip = (unsigned)(32 * kb) * 128;
@@ -358,7 +358,7 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   // ---- L' L'^T
-  if (tid == 0 && !ctl->abort_flag) {
+  if (warp == 0 && !ctl->abort_flag && elect_one()) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
     for (int kb = 0; kb < 4; ++kb) {

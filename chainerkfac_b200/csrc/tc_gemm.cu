@@ -532,7 +532,7 @@ tc_gemm_kernel(const GemmDesc* __restrict__ descs, int ndesc,
     }
   } else {
     // ===================== MMA issuer =====================
-    if (lane == 0) {
+    if (elect_one()) {
       const unsigned idesc = tc_instr_desc(n_inst);
       for (int kb = 0; kb < nkb; ++kb) {
         const int s = kb % TC_STAGES;
@@ -1144,7 +1144,7 @@ tc_pair_kernel(const GemmDesc* __restrict__ descs, int ndesc,
     }
   } else {
     // ===================== MMA issuer =====================
-    if (lane == 0) {
+    if (elect_one()) {
       const unsigned idesc = tc_instr_desc_bf16(n_inst);
       const unsigned a_off = share ? (unsigned)PK_TILE_BYTES : 0u;
       for (int kb = 0; kb < nkb; ++kb) {
@@ -1385,23 +1385,22 @@ tc_reduce_kernel(const ReduceItem* __restrict__ items,
        e < min(total, (int)(blockIdx.y + 1) * 1024); e += 64) {
     const int r = e / cols, c = e - r * cols;
     const float* p = it.partial + r * TC_BN + c;
-    float s0 = 0.f, s1 = 0.f;
-    int sp = q;
-    for (; sp + 4 < it.splits; sp += 8) {
-      s0 += p[sp * it.sstride];
-      s1 += p[(sp + 4) * it.sstride];
-    }
-    if (sp < it.splits) s0 += p[sp * it.sstride];
-    float s = s0 + s1;
+    // (eight loads in flight: a narrow factor has hundreds of splits)
+    float v[8] = {};
+    for (int sp = q; sp < it.splits; sp += 32)
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (sp + 4 * u < it.splits) v[u] += p[(sp + 4 * u) * it.sstride];
+    float s = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     const int gr = m0 + r, gc = n0 + c;
     if (q != 0 || gc > gr) continue;
     float* o = it.out + (long long)gr * d + gc;
-    float v = it.alpha * s;
-    if (it.beta != 0.f) v += it.beta * (*o);
-    *o = v;
-    if (gc < gr) it.out[(long long)gc * d + gr] = v;
+    float x = it.alpha * s;
+    if (it.beta != 0.f) x += it.beta * (*o);
+    *o = x;
+    if (gc < gr) it.out[(long long)gc * d + gr] = x;
   }
 }
 
@@ -1585,7 +1584,7 @@ size_t tc_pad_bytes(const Operand& X, int n, int nhwc) {
   return (e * sizeof(float) + 255) & ~(size_t)255;
 }
 
-// k-blocks per CTA for a group of factors: total work spread over ~4 waves.
+// k-blocks per CTA for a group of factors: total work spread over ~2 waves.
 static long long tc_group_chunk(int count, const FactorJob* jobs) {
   long long work = 0;
   for (int i = 0; i < count; ++i)
@@ -1593,8 +1592,8 @@ static long long tc_group_chunk(int count, const FactorJob* jobs) {
             ((jobs[i].rows + TC_BK - 1) / TC_BK) * tc_block_cost(jobs[i].d);
   static const long long waves = [] {
     const char* e = getenv("KFAC_TC_WAVES");
-    const long long w = e ? atoll(e) : 4;
-    return w > 0 ? w : 4;
+    const long long w = e ? atoll(e) : 2;
+    return w > 0 ? w : 2;
   }();
   return work / (waves * sm_count());
 }
@@ -1620,14 +1619,18 @@ static size_t tc_pair_workspace_bytes(int count, const FactorJob* jobs,
 //  * 3 x 3 convolutions as shifted products, at any size (32 images, us per
 //    factor before and now: 64 channels 56 x 56 228 -> 78, 256 channels 14 x 14
 //    171 -> 62; 8 images of 64 channels 14 x 14 68 -> 41);
-//  * wide factors, where the gather feeds every element to many tiles (1568 x
-//    2048: 57 -> 29; even at 1000 columns, slower below);
+//  * plain operands that TMA reads in place, from a million elements on (below
+//    that the launches count: all factors of a 1000-1000-10 network at 128
+//    rows 43 us with the gather, 72 us without);
+//  * other wide factors, where the gather feeds every element to many tiles
+//    (NCHW, 1568 x 2048: 68 -> 27; even at 1000 columns, slower below);
 //  * patches of strided convolutions with many channels (1x1, 512 channels
 //    28 x 28 channels-last: 84 -> 27; 3x3, 256 channels 28 x 28: 199 -> 155;
 //    the 3-channel 7x7 stem stays with the gather, 160 against 486).
 static bool tc_uses_gram(const FactorJob& job) {
   if (tc_staged()) return false;
   if (gram_grid_job(job)) return true;
+  if ((double)job.rows * job.d >= 1e6 && gram_direct_job(job)) return true;
   if ((double)job.rows * job.d < 2e6) return false;
   return job.d >= 1024 || (job.X.mode == 1 && job.X.C >= 128);
 }
@@ -1920,6 +1923,7 @@ static FactorJob lone_job(const Operand& X, long long rows, int d, float alpha,
   job.d = d;
   job.n = X.mode == 1 ? (int)(rows / ((long long)X.Ho * X.Wo)) : 0;
   job.nhwc = 0;
+  job.grouped = 0;
   job.alpha = alpha;
   job.beta = beta;
   job.out = out;
@@ -1928,10 +1932,16 @@ static FactorJob lone_job(const Operand& X, long long rows, int d, float alpha,
 
 // Workspace of a factor built on its own from any operand of this geometry.
 size_t tc_lone_workspace_bytes(const Operand& X, long long rows, int d) {
-  const FactorJob job = lone_job(X, rows, d, 1.f, 0.f, nullptr);
-  return std::max(tc_factor_workspace_bytes(rows, d) +
-                      tc_pad_bytes(X, job.n),
-                  tc_factor_group_workspace_bytes(1, &job, true));
+  FactorJob job = lone_job(X, rows, d, 1.f, 0.f, nullptr);
+  const size_t gather =
+      tc_factor_workspace_bytes(rows, d) + tc_pad_bytes(X, job.n);
+  // the address and the pitch decide between the feeds: the larger of both
+  job.X.s_outer = (X.s_outer + 3) & ~3LL;
+  const size_t aligned = tc_factor_group_workspace_bytes(1, &job, true);
+  job.X.base = reinterpret_cast<const float*>(sizeof(float));
+  return std::max(gather,
+                  std::max(aligned,
+                           tc_factor_group_workspace_bytes(1, &job, true)));
 }
 
 int run_factor_tc(const Operand& X, long long rows, int d, float alpha,

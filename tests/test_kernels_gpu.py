@@ -282,6 +282,25 @@ def test_wide_factor_from_staged_planes(ops, rows, d, ones):
         assert rel(host(out), host(xd.t() @ xd)) < FACTOR_TOL
 
 
+@pytest.mark.parametrize('n,c,h,w', [
+    (300, 60, 8, 8), (32, 64, 28, 28), (257, 100, 8, 5), (65, 128, 13, 12),
+    (1000, 256, 2, 2), (40, 200, 12, 12), (31, 260, 12, 12), (9, 1028, 11, 12)])
+@pytest.mark.parametrize('channels_last', [False, True])
+def test_factor_of_plain_operands_read_by_tma(ops, n, c, h, w, channels_last):
+    """Gradient factors of a million elements and more: one tile of 64, 128
+    and 256 columns and several, cut last rows and columns, images that are no
+    multiple of a k-block, on top of an existing average, against fp64."""
+    torch.manual_seed(4)
+    g = torch.randn(n, c, h, w, device='cuda')
+    m = g.permute(0, 2, 3, 1).reshape(-1, c).double()
+    if channels_last:
+        g = g.contiguous(memory_format=torch.channels_last)
+    out = torch.full((c, c), 3.0, device='cuda')
+    ops.factor_group([ops.conv_grad_item(g, 2.0, 0.5, out)], g.device)
+    assert rel(host(out), host(2.0 * (m.t() @ m) + 1.5)) < FACTOR_TOL
+    check_symmetric(host(out))
+
+
 def test_factor_builds_from_staged_operands(ops, engine):
     """The optional operand feed of the factor builds (staging pass that
     writes X^T as two bf16 planes, TMA boxes into the tile kernel) against the
