@@ -272,15 +272,23 @@ struct GemmDesc {
 int launch_grouped_gemm(const GemmDesc* descs_dev, int ndesc, int total_tiles,
                         float lr, float momentum, cudaStream_t stream);
 
-// Tensor-core engine (tc_gemm.cu): 128 x 256 tiles, tcgen05 split-TF32.
+// Tensor-core engine of the factor builds (tc_gemm.cu).
 int engine();   // 1: tensor cores (default), 0: fp32 FFMA tiles
 int tc_tiles(GemmDesc& g);
 // Opt the tile kernels into their shared-memory sizes on the current device
 // (once per device; the launch helpers call it, plans call it before capture).
 int tc_prepare();
-int launch_tc_grouped(const GemmDesc* descs_dev, int ndesc, int total_tiles,
-                      float lr, float momentum, bool tails,
-                      cudaStream_t stream);
+// Tile engine of the inverse and precondition products (tc_tile.cu).  Number
+// the tiles of a launch (fills tile_begin, tiles_m, tiles_n) and choose their
+// width; returns the launch's tile count.
+int tc_number_tiles(GemmDesc* descs, int n, int* tile_cols);
+int tc_prepare_tiles();
+// `descs_host`: the same descriptors on the host (small launches pass them as
+// kernel arguments), or NULL.
+int launch_tc_grouped(const GemmDesc* descs_dev, const GemmDesc* descs_host,
+                      int ndesc, int total_tiles, int tile_cols, bool precond,
+                      float lr, float momentum, cudaStream_t stream);
+int tile_status_read(int* out);
 bool tc_desc_has_tails(const GemmDesc& g);
 size_t tc_factor_workspace_bytes(long long rows, int d, bool staged = true);
 size_t tc_lone_workspace_bytes(const Operand& X, long long rows, int d);

@@ -24,9 +24,13 @@ constexpr int PW = 512;        // Cholesky panel width (outer blocking)
 struct MatInfo {
   const float* F;
   float* inv;
-  float* W;
-  float* X;
-  int d;
+  // working copies, rows `ld` floats apart (d rounded up to whole 128-byte
+  // lines, so that every row is read and written as 16-byte words)
+  float* W;       // damped factor, then L (and T^T above the diagonal)
+  float* X;       // L^-1
+  float* V;       // blocks of W before a panel solve overwrites them; T of the
+                  // doubling; X R of the refinement
+  int d, ld;
   int partner;
   int role;
   float l2;
@@ -116,7 +120,7 @@ __global__ void damping_kernel(const MatInfo* __restrict__ mats, int count,
 // the lower triangle and the rest of each diagonal 128-block (which the
 // trailing updates read-modify-write) is ever used, so only that is copied.
 // With `dual` the first block column below the first diagonal block is also
-// stored in the inverse's output buffer (see the look-ahead of the Cholesky).
+// stored in V (see the look-ahead of the Cholesky).
 __global__ void damp_copy_kernel(const MatInfo* __restrict__ mats,
                                  const float* __restrict__ add,
                                  const float* __restrict__ add2, int dual) {
@@ -126,12 +130,12 @@ __global__ void damp_copy_kernel(const MatInfo* __restrict__ mats,
   const bool vec = (d & 3) == 0 &&
                    ((reinterpret_cast<uintptr_t>(mi.F) |
                      reinterpret_cast<uintptr_t>(mi.W) |
-                     reinterpret_cast<uintptr_t>(mi.inv)) & 15) == 0;
+                     reinterpret_cast<uintptr_t>(mi.V)) & 15) == 0;
   for (int r = blockIdx.x; r < d; r += gridDim.x) {
     const float a = (mi.role == 2 && 2 * r >= d) ? a_second : a_first;
     const int cend = min(d, (r | (DB - 1)) + 1);
     const float* src = mi.F + (long long)r * d;
-    float* dst = mi.W + (long long)r * d;
+    float* dst = mi.W + (long long)r * mi.ld;
     if (vec) {
       // cend is a multiple of 128 or equals d, itself a multiple of 4 here
       const float4* s4 = reinterpret_cast<const float4*>(src);
@@ -147,14 +151,14 @@ __global__ void damp_copy_kernel(const MatInfo* __restrict__ mats,
         }
         d4[c4] = v;
         if (dual && r >= DB && c4 < DB / 4)
-          reinterpret_cast<float4*>(mi.inv + (long long)r * d)[c4] = v;
+          reinterpret_cast<float4*>(mi.V + (long long)r * mi.ld)[c4] = v;
       }
     } else {
       for (int c = threadIdx.x; c < cend; c += blockDim.x) {
         float v = src[c];
         if (r == c) v += a;
         dst[c] = v;
-        if (dual && r >= DB && c < DB) mi.inv[(long long)r * d + c] = v;
+        if (dual && r >= DB && c < DB) mi.V[(long long)r * mi.ld + c] = v;
       }
     }
   }
@@ -256,8 +260,7 @@ __device__ __forceinline__ void look_begin(LookControl* ctl) {
 // k - 1; the update of step k - 1,
 //   D = W_kk - L' L'^T,  L' = A' X_pp^T,
 // is computed here from A' (block (k, k-1) as it was before step k-1's panel
-// solve overwrote it; the updates keep a second copy of it in the inverse's
-// output buffer) and X_pp (inverse of the previous diagonal block's factor),
+// solve overwrote it; the updates keep a second copy of it in V) and X_pp (inverse of the previous diagonal block's factor),
 // so that this kernel does not have to wait for the panel solve and panel
 // update of step k - 1.  Both products run on the tensor cores (tcgen05,
 // split TF32, accumulators in tensor memory).  All global loads are in flight
@@ -269,8 +272,8 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
                                                unsigned char* stage,
                                                LookControl* ctl) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const long long ld = mi.d;
-  const float* Ap = mi.inv + (long long)o * ld + (o - DB);
+  const long long ld = mi.ld;
+  const float* Ap = mi.V + (long long)o * ld + (o - DB);
   const float* Xp = mi.X + (long long)(o - DB) * ld + (o - DB);
   float4 va[4][2], vx[4][2];
 #pragma unroll
@@ -750,10 +753,9 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
   const int o = step * DB;
   const int bs = min(DB, mi.d - o);
   const int np = (bs + SB - 1) / SB;      // sub-blocks in use
-  const long long ld = mi.d;
-  const bool vec = (ld & 3) == 0 &&
-                   ((reinterpret_cast<uintptr_t>(mi.W) |
-                     reinterpret_cast<uintptr_t>(mi.inv) |
+  const long long ld = mi.ld;
+  const bool vec = ((reinterpret_cast<uintptr_t>(mi.W) |
+                     reinterpret_cast<uintptr_t>(mi.V) |
                      reinterpret_cast<uintptr_t>(mi.X)) & 15) == 0;
   if (LOOK) {
     if (!diag_lookahead(mi, o, bs, vec, sm.S, stage, ctl)) return;
@@ -866,14 +868,13 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
 //   t = X v,  r = v - (F + add I) t,  e = X r   (fp64 accumulation)
 // e estimates (X - A^-1) v, so |e| / |t| estimates the relative error of X;
 // the step runs when that exceeds `threshold` and d <= `max_dim`.
-constexpr int kRefineDimCap = 1024;   // workspace is reserved up to this size
+constexpr int kRefineDimCap = 1024;   // larger factors are not refined
 
 struct RefineItem {
   int mat;          // index into the plan's matrices
   int d;
   int tile_begin;   // first 64 x 64 tile of this matrix in the residual grid
   int pad_;
-  float* Y;         // d x d scratch for X R
   double* vec;      // 2 d doubles: t, r
 };
 
@@ -1026,7 +1027,7 @@ refine_residual_kernel(const MatInfo* __restrict__ mats,
     for (int j = 0; j < 4; ++j) {
       const int gj = j0 + tx * 4 + j;
       if (gj < d)
-        mi.W[(long long)gi * d + gj] =
+        mi.W[(long long)gi * mi.ld + gj] =
             (float)((gi == gj ? 1.0 : 0.0) - acc[i][j]);
     }
   }
@@ -1039,11 +1040,10 @@ refine_apply_kernel(const MatInfo* __restrict__ mats,
                     const int* __restrict__ gate) {
   if (gate[blockIdx.y] == 0) return;
   const RefineItem it = items[blockIdx.y];
-  float* inv = mats[it.mat].inv;
-  const long long n = (long long)it.d * it.d;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    inv[i] += it.Y[i];
+  const MatInfo mi = mats[it.mat];
+  for (int r = blockIdx.x; r < it.d; r += gridDim.x)
+    for (int c = threadIdx.x; c < it.d; c += blockDim.x)
+      mi.inv[(long long)r * it.d + c] += mi.V[(long long)r * mi.ld + c];
 }
 
 constexpr size_t kDiagSmemBytes = sizeof(DiagSmem);
@@ -1059,7 +1059,7 @@ static_assert(kDiagLookSmemBytes >= kDiagSmemBytes &&
 enum PlanStream { S_CHAIN, S_BULK, S_FAR, S_ROWS, S_PROD, S_COUNT };
 
 struct Launch {
-  int tails;     // grouped gemm: some contraction is not a multiple of 32
+  int tile_cols; // grouped gemm: tile width
   int kind;      // 0 diag kernel, 1 grouped gemm
   int off;       // grouped gemm: offset into descs
   int n;         // number of matrices / descs
@@ -1098,6 +1098,7 @@ struct kfac_inverse_plan {
   int* info_dev;
   MatInfo* sorted_dev;     // mats_dev, largest first (diagonal kernels)
   GemmDesc* descs_dev;
+  std::vector<GemmDesc> descs;       // the same on the host
   std::vector<Launch> launches;
   long long total_elems;
   bool use_tc;
@@ -1129,15 +1130,18 @@ struct kfac_inverse_plan {
   bool graph_ok;
 };
 
-static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+static int matrix_pitch(int d) { return (d + 31) & ~31; }
+
+static size_t matrix_bytes(int d) {
+  const size_t bytes = (size_t)d * matrix_pitch(d) * sizeof(float);
+  return (bytes + 255) & ~(size_t)255;
+}
 
 extern "C" size_t kfac_inverse_workspace_bytes(int count, const int* dims) {
   size_t total = 0;
   for (int i = 0; i < count; ++i) {
     if (dims[i] <= 0) return 0;
-    const size_t bytes = align256((size_t)dims[i] * dims[i] * sizeof(float));
-    total += 2 * bytes;                              // W, X
-    if (dims[i] <= kRefineDimCap) total += bytes;    // Y of the refinement
+    total += 3 * matrix_bytes(dims[i]);              // W, X, V
   }
   return total;
 }
@@ -1173,21 +1177,19 @@ extern "C" int kfac_inverse_plan_create(
   // zeros by the wide tiles of the triangular-inverse products.
   KFAC_CUDA(cudaMemset(workspace, 0, need));
   std::vector<MatInfo> mats(count);
-  std::vector<float*> ybuf(count, nullptr);
   char* ws = static_cast<char*>(workspace);
   int dmax = 0;
   long long total_elems = 0;
   for (int i = 0; i < count; ++i) {
     MatInfo& m = mats[i];
-    size_t bytes = align256((size_t)dims[i] * dims[i] * sizeof(float));
+    const size_t bytes = matrix_bytes(dims[i]);
     m.F = factors[i];
     m.inv = inverses[i];
     m.W = reinterpret_cast<float*>(ws); ws += bytes;
     m.X = reinterpret_cast<float*>(ws); ws += bytes;
-    if (dims[i] <= kRefineDimCap) {
-      ybuf[i] = reinterpret_cast<float*>(ws); ws += bytes;
-    }
+    m.V = reinterpret_cast<float*>(ws); ws += bytes;
     m.d = dims[i];
+    m.ld = matrix_pitch(dims[i]);
     m.partner = partner ? partner[i] : -1;
     m.role = role[i];
     m.l2 = l2_coef ? l2_coef[i] : 0.f;
@@ -1228,8 +1230,7 @@ extern "C" int kfac_inverse_plan_create(
   };
   auto push_desc = [&](Launch& l, GemmDesc g) {
     g.tile_begin = l.tiles;
-    l.tiles += use_tc ? tc_tiles(g) : gemm_desc_tiles(g);
-    if (tc_desc_has_tails(g)) l.tails = 1;
+    if (!use_tc) l.tiles += gemm_desc_tiles(g);
     g.kfW = g.kfb = g.pW = g.pb = g.vW = g.vb = nullptr;
     g.dW = 0;
     g.splits = 1;
@@ -1242,6 +1243,8 @@ extern "C" int kfac_inverse_plan_create(
   // append a launch (if it has work); its event, or -1
   auto end_gemm = [&](Launch& l, bool record) {
     if (l.n == 0) return -1;
+    if (use_tc && l.kind == 1)
+      l.tiles = tc_number_tiles(&descs[l.off], l.n, &l.tile_cols);
     if (record) l.rec_ev = n_events++;
     launches.push_back(l);
     return l.rec_ev;
@@ -1260,9 +1263,9 @@ extern "C" int kfac_inverse_plan_create(
   // the chain, and the part of a panel's trailing update that the next panel
   // does not need runs on the far stream.  Panel updates (and the near part of
   // a trailing update, and the damped copy for the first block column) store
-  // their results a second time in the inverse's output buffer: that copy of
-  // block (k, k-1) is what diag_lookahead reads while the panel solve of step
-  // k-1 overwrites the original.
+  // their results a second time in V: that copy of block (k, k-1) is what
+  // diag_lookahead reads while the panel solve of step k-1 overwrites the
+  // original.
   //
   // The inverse grows with the factor, a row panel at a time: with X = L^-1,
   //   T = L_p X_<p,  X_p = -X_pp T  (X_pp by doubling from the 128-blocks),
@@ -1271,8 +1274,7 @@ extern "C" int kfac_inverse_plan_create(
   // When the chain ends only the last panel's share is left (a 4608-row matrix:
   // 0.15 ms instead of the 0.95 ms that the whole triangular inverse and
   // product took behind the factorisation).  T^T waits in the unused upper
-  // triangle of W; rows and columns of inv before the running panel are no
-  // longer needed for the copies above.
+  // triangle of W.
   for (int po = 0; po < dmax; po += PW) {
     const int inner = std::min(PW, dmax - po);
     int bulk_ev = -1;          // the bulk stream's last launch of this panel
@@ -1295,11 +1297,12 @@ extern "C" int kfac_inverse_plan_create(
         const int M = d - o - DB;
         if (M <= 0) continue;
         const MatInfo& m = mats[i];
+        const long long ld = m.ld;
         GemmDesc g = {};
-        float* panel = m.W + (long long)(o + DB) * d + o;
-        g.A = strided_operand(panel, 1, d, M);
-        g.B = strided_operand(m.X + (long long)o * d + o, 1, d, DB);
-        g.C = panel; g.ldc = d; g.M = M; g.N = DB; g.K = DB;
+        float* panel = m.W + (o + DB) * ld + o;
+        g.A = strided_operand(panel, 1, ld, M);
+        g.B = strided_operand(m.X + o * ld + o, 1, ld, DB);
+        g.C = panel; g.ldc = ld; g.M = M; g.N = DB; g.K = DB;
         g.alpha = 1.f; g.beta = 0.f; g.flags = 0;
         push_desc(trsm, g);
       }
@@ -1318,15 +1321,16 @@ extern "C" int kfac_inverse_plan_create(
         const int N = std::min(po + PW, d) - (o + DB);
         if (M <= 0 || N <= 0) continue;
         const MatInfo& m = mats[i];
+        const long long ld = m.ld;
         GemmDesc g = {};
-        float* panel = m.W + (long long)(o + DB + skip) * d + o;
-        const long long coff = (long long)(o + DB + skip) * d + (o + DB);
-        g.A = strided_operand(panel, 1, d, M);
-        g.B = strided_operand(m.W + (long long)(o + DB) * d + o, 1, d, N);
+        float* panel = m.W + (o + DB + skip) * ld + o;
+        const long long coff = (o + DB + skip) * ld + (o + DB);
+        g.A = strided_operand(panel, 1, ld, M);
+        g.B = strided_operand(m.W + (o + DB) * ld + o, 1, ld, N);
         g.C = m.W + coff;
-        g.ldc = d; g.M = M; g.N = N; g.K = DB;
+        g.ldc = ld; g.M = M; g.N = N; g.K = DB;
         g.alpha = -1.f; g.beta = 1.f; g.flags = 0;
-        if (look) g.C2 = m.inv + coff;
+        if (look) g.C2 = m.V + coff;
         push_desc(upd, g);
       }
       upd_ev[o / DB] = end_gemm(upd, look);
@@ -1347,34 +1351,35 @@ extern "C" int kfac_inverse_plan_create(
       if (M <= 0) continue;
       const int N1 = std::min(PW, M);
       const MatInfo& m = mats[i];
-      const float* panel = m.W + (long long)(po + PW) * d + po;
+      const long long ld = m.ld;
+      const float* panel = m.W + (po + PW) * ld + po;
       {
         GemmDesc g = {};     // square block on the diagonal: lower tiles
-        const long long coff = (long long)(po + PW) * d + (po + PW);
-        g.A = strided_operand(panel, 1, d, N1);
+        const long long coff = (po + PW) * ld + (po + PW);
+        g.A = strided_operand(panel, 1, ld, N1);
         g.B = g.A;
         g.C = m.W + coff;
-        g.ldc = d; g.M = N1; g.N = N1; g.K = PW;
+        g.ldc = ld; g.M = N1; g.N = N1; g.K = PW;
         g.alpha = -1.f; g.beta = 1.f; g.flags = G_LOWER | G_SAME_AB;
-        if (look) g.C2 = m.inv + coff;
+        if (look) g.C2 = m.V + coff;
         push_desc(near, g);
       }
       if (M > N1) {
-        const float* below = panel + (long long)N1 * d;
+        const float* below = panel + N1 * ld;
         GemmDesc g = {};     // rectangle below it
-        const long long coff = (long long)(po + PW + N1) * d + (po + PW);
-        g.A = strided_operand(below, 1, d, M - N1);
-        g.B = strided_operand(panel, 1, d, N1);
+        const long long coff = (po + PW + N1) * ld + (po + PW);
+        g.A = strided_operand(below, 1, ld, M - N1);
+        g.B = strided_operand(panel, 1, ld, N1);
         g.C = m.W + coff;
-        g.ldc = d; g.M = M - N1; g.N = N1; g.K = PW;
+        g.ldc = ld; g.M = M - N1; g.N = N1; g.K = PW;
         g.alpha = -1.f; g.beta = 1.f; g.flags = 0;
-        if (look) g.C2 = m.inv + coff;
+        if (look) g.C2 = m.V + coff;
         push_desc(near, g);
         GemmDesc h = {};     // everything beyond the next panel's columns
-        h.A = strided_operand(below, 1, d, M - N1);
+        h.A = strided_operand(below, 1, ld, M - N1);
         h.B = h.A;
-        h.C = m.W + (long long)(po + PW + N1) * d + (po + PW + N1);
-        h.ldc = d; h.M = M - N1; h.N = M - N1; h.K = PW;
+        h.C = m.W + (po + PW + N1) * ld + (po + PW + N1);
+        h.ldc = ld; h.M = M - N1; h.N = M - N1; h.K = PW;
         h.alpha = -1.f; h.beta = 1.f; h.flags = G_LOWER | G_SAME_AB;
         far_descs.push_back(h);
       }
@@ -1399,27 +1404,28 @@ extern "C" int kfac_inverse_plan_create(
     const int pend = std::min(po + PW, dmax);
     bool first = true;
     for (int b = DB; b < pend - po; b *= 2) {
-      // X_pp by doubling: T = L21 X11 (parked in the output matrix), then
+      // X_pp by doubling: T = L21 X11 (parked in V), then
       // X21 = -X22 T
       Launch g1 = begin_gemm(s_rows);
       std::vector<GemmDesc> second;
       for (int i : order) {
         const int d = dims[i], end = std::min(po + PW, d);
         const MatInfo& m = mats[i];
+        const long long ld = m.ld;
         for (long long s = po; s + b < end; s += 2 * b) {
           const int r = (int)std::min<long long>(b, end - s - b);
           GemmDesc g = {};
-          g.A = strided_operand(m.W + (s + b) * d + s, 1, d, r);
-          g.B = strided_operand(m.X + s * d + s, d, 1, b);
-          g.C = m.inv + (s + b) * d + s;
-          g.ldc = d; g.M = r; g.N = b; g.K = b;
+          g.A = strided_operand(m.W + (s + b) * ld + s, 1, ld, r);
+          g.B = strided_operand(m.X + s * ld + s, ld, 1, b);
+          g.C = m.V + (s + b) * ld + s;
+          g.ldc = ld; g.M = r; g.N = b; g.K = b;
           g.alpha = 1.f; g.beta = 0.f; g.flags = G_KBEG_N0;
           push_desc(g1, g);
           GemmDesc h = {};
-          h.A = strided_operand(m.X + (s + b) * d + s + b, 1, d, r);
-          h.B = strided_operand(m.inv + (s + b) * d + s, d, 1, b);
-          h.C = m.X + (s + b) * d + s;
-          h.ldc = d; h.M = r; h.N = b; h.K = r;
+          h.A = strided_operand(m.X + (s + b) * ld + s + b, 1, ld, r);
+          h.B = strided_operand(m.V + (s + b) * ld + s, ld, 1, b);
+          h.C = m.X + (s + b) * ld + s;
+          h.ldc = ld; h.M = r; h.N = b; h.K = r;
           h.alpha = -1.f; h.beta = 0.f; h.flags = G_KEND_M0;
           second.push_back(h);
         }
@@ -1440,11 +1446,12 @@ extern "C" int kfac_inverse_plan_create(
         const int d = dims[i], w = std::min(PW, d - po);
         if (w <= 0) continue;
         const MatInfo& m = mats[i];
+        const long long ld = m.ld;
         GemmDesc g = {};
-        g.A = strided_operand(m.X + (long long)po * d + po, 1, d, w);
-        g.B = strided_operand(m.W + po, 1, d, po);    // B(k, n) = T^T[n][k]
-        g.C = m.X + (long long)po * d;
-        g.ldc = d; g.M = w; g.N = po; g.K = w;
+        g.A = strided_operand(m.X + po * ld + po, 1, ld, w);
+        g.B = strided_operand(m.W + po, 1, ld, po);   // B(k, n) = T^T[n][k]
+        g.C = m.X + po * ld;
+        g.ldc = ld; g.M = w; g.N = po; g.K = w;
         g.alpha = -1.f; g.beta = 0.f; g.flags = G_KEND_M0;
         push_desc(rows, g);
       }
@@ -1462,7 +1469,7 @@ extern "C" int kfac_inverse_plan_create(
       if (w <= 0) continue;
       const MatInfo& m = mats[i];
       GemmDesc g = {};
-      g.A = strided_operand(m.X + (long long)po * d, d, 1, end);
+      g.A = strided_operand(m.X + (long long)po * m.ld, m.ld, 1, end);
       g.B = g.A;
       g.C = m.inv; g.ldc = d; g.M = end; g.N = end; g.K = w;
       g.alpha = 1.f; g.beta = po > 0 ? 1.f : 0.f;
@@ -1485,11 +1492,12 @@ extern "C" int kfac_inverse_plan_create(
       const int d = dims[i], w = std::min(PW, d - pend);
       if (w <= 0) continue;
       const MatInfo& m = mats[i];
+      const long long ld = m.ld;
       GemmDesc g = {};
-      g.A = strided_operand(m.X, d, 1, pend);
-      g.B = strided_operand(m.W + (long long)pend * d, 1, d, w);
+      g.A = strided_operand(m.X, ld, 1, pend);
+      g.B = strided_operand(m.W + pend * ld, 1, ld, w);
       g.C = m.W + pend;
-      g.ldc = d; g.M = pend; g.N = w; g.K = pend;
+      g.ldc = ld; g.M = pend; g.N = w; g.K = pend;
       g.alpha = 1.f; g.beta = 0.f; g.flags = G_KBEG_M0;
       push_desc(next_t, g);
     }
@@ -1510,7 +1518,6 @@ extern "C" int kfac_inverse_plan_create(
     it.d = dims[i];
     it.tile_begin = refine_tiles;
     it.pad_ = 0;
-    it.Y = ybuf[i];
     it.vec = reinterpret_cast<double*>(vec_elems);   // offset, fixed up below
     const int nt = (dims[i] + 63) / 64;
     refine_tiles += nt * nt;
@@ -1591,8 +1598,8 @@ extern "C" int kfac_inverse_plan_create(
         const MatInfo& m = mats[it.mat];
         GemmDesc g = {};
         g.A = strided_operand(m.inv, 1, d, d);     // A(k, m) = X[m][k]
-        g.B = strided_operand(m.W, d, 1, d);       // B(k, n) = R[k][n]
-        g.C = it.Y; g.ldc = d; g.M = d; g.N = d; g.K = d;
+        g.B = strided_operand(m.W, m.ld, 1, d);    // B(k, n) = R[k][n]
+        g.C = m.V; g.ldc = m.ld; g.M = d; g.N = d; g.K = d;
         g.alpha = 1.f; g.beta = 0.f; g.flags = G_LOWER | G_MIRROR;
         g.gate = p->refine_gate_dev + r;
         push_desc(refine_prod, g);
@@ -1601,7 +1608,11 @@ extern "C" int kfac_inverse_plan_create(
                      sizeof(RefineItem) * nr, cudaMemcpyHostToDevice);
     }
   }
+  if (use_tc && refine_prod.n > 0)
+    refine_prod.tiles = tc_number_tiles(&descs[refine_prod.off], refine_prod.n,
+                                        &refine_prod.tile_cols);
   p->refine_prod = refine_prod;
+  p->descs = descs;
   if (e == cudaSuccess) e = cudaMalloc(&p->mats_dev, sizeof(MatInfo) * count);
   if (e == cudaSuccess) e = cudaMalloc(&p->trace_dev, sizeof(float) * count);
   if (e == cudaSuccess) e = cudaMalloc(&p->add_dev, sizeof(float) * count);
@@ -1629,7 +1640,7 @@ extern "C" int kfac_inverse_plan_create(
     return fail(KFAC_ERR_CUDA, "inverse_plan_create: %s", cudaGetErrorString(e));
   }
   if (use_tc) {
-    const int rc = tc_prepare();
+    const int rc = tc_prepare_tiles();
     if (rc != KFAC_OK) {
       kfac_inverse_plan_destroy(p);
       return rc;
@@ -1677,8 +1688,9 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
       KFAC_LAUNCH_CHECK("chol_diag_kernel");
     } else {
       int rc = p->use_tc
-                   ? launch_tc_grouped(p->descs_dev + l.off, l.n, l.tiles, 0.f,
-                                       0.f, l.tails != 0, st)
+                   ? launch_tc_grouped(p->descs_dev + l.off, &p->descs[l.off],
+                                       l.n, l.tiles, l.tile_cols, false, 0.f,
+                                       0.f, st)
                    : launch_grouped_gemm(p->descs_dev + l.off, l.n, l.tiles,
                                          0.f, 0.f, st);
       if (rc != KFAC_OK) return rc;
@@ -1708,8 +1720,9 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
     KFAC_LAUNCH_CHECK("refine_residual_kernel");
     const Launch& l = p->refine_prod;
     int rc = p->use_tc
-                 ? launch_tc_grouped(p->descs_dev + l.off, l.n, l.tiles, 0.f,
-                                     0.f, l.tails != 0, st)
+                 ? launch_tc_grouped(p->descs_dev + l.off, &p->descs[l.off],
+                                     l.n, l.tiles, l.tile_cols, false, 0.f,
+                                       0.f, st)
                  : launch_grouped_gemm(p->descs_dev + l.off, l.n, l.tiles, 0.f,
                                        0.f, st);
     if (rc != KFAC_OK) return rc;

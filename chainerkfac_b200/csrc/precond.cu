@@ -76,7 +76,7 @@ extern "C" int kfac_precondition(
     g.alpha = 1.f; g.beta = 0.f; g.flags = 0;
     g.tile_begin = tiles1;
     g.splits = 1;
-    tiles1 += use_tc ? tc_tiles(g) : gemm_desc_tiles(g);
+    if (!use_tc) tiles1 += gemm_desc_tiles(g);
     // kf = T * A_inv, split and (optionally) applied
     GemmDesc& h = descs[count + i];
     h = GemmDesc();
@@ -94,21 +94,22 @@ extern "C" int kfac_precondition(
     h.dW = dw;
     h.tile_begin = tiles2;
     h.splits = 1;
-    tiles2 += use_tc ? tc_tiles(h) : gemm_desc_tiles(h);
+    if (!use_tc) tiles2 += gemm_desc_tiles(h);
+  }
+  int cols1 = 0, cols2 = 0;
+  if (use_tc) {
+    tiles1 = tc_number_tiles(descs.data(), count, &cols1);
+    tiles2 = tc_number_tiles(descs.data() + count, count, &cols2);
   }
   KFAC_CUDA(cudaMemcpyAsync(descs_dev, descs.data(),
                             descs.size() * sizeof(GemmDesc),
                             cudaMemcpyHostToDevice, st));
   if (use_tc) {
-    bool t1 = false, t2 = false;
-    for (int i = 0; i < count; ++i) {
-      t1 = t1 || tc_desc_has_tails(descs[i]);
-      t2 = t2 || tc_desc_has_tails(descs[count + i]);
-    }
-    int rc = launch_tc_grouped(descs_dev, count, tiles1, 0.f, 0.f, t1, st);
+    int rc = launch_tc_grouped(descs_dev, descs.data(), count, tiles1, cols1,
+                               false, 0.f, 0.f, st);
     if (rc != KFAC_OK) return rc;
-    return launch_tc_grouped(descs_dev + count, count, tiles2, lr, momentum,
-                             t2, st);
+    return launch_tc_grouped(descs_dev + count, descs.data() + count, count,
+                             tiles2, cols2, true, lr, momentum, st);
   }
   int rc = launch_grouped_gemm(descs_dev, count, tiles1, 0.f, 0.f, st);
   if (rc != KFAC_OK) return rc;

@@ -166,6 +166,10 @@ __device__ __forceinline__ void sts128(unsigned addr, float4 v) {
                : "memory");
 }
 
+__device__ __forceinline__ void sts32(unsigned addr, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+
 // hi = x rounded to TF32 (nearest, ties away from zero), lo = x - hi (exact in
 // fp32; the tensor core reads its top 11 bits).  The rounding is two integer
 // instructions (add half an ulp of TF32, clear the low 13 bits): cvt.rna

@@ -1,22 +1,9 @@
-// Tensor-core tile engine for sm_100a: tcgen05.mma (kind::tf32) with fp32
-// accumulators in tensor memory, fp32 operands split into two TF32 terms
-// (x = hi + lo with hi rounded to nearest, C += hi*hi + hi*lo + lo*hi) so that
-// results keep near-fp32 accuracy (a single TF32 pass misses the 1e-4 bound on
-// large factors).
-//
-// One CTA (16 producer/epilogue warps + 1 MMA warp) owns a 128 x N tile,
-// N <= 256.  Producer warps gather the operands from global memory (strided
-// views, transposing views or im2col patches of an NCHW tensor), split them
-// and write the K-major, 128-byte-swizzled shared-memory layout that the MMA
-// descriptors expect; two stages of 32 k each are kept in flight through
-// mbarriers.  The epilogue moves the accumulator tile TMEM -> registers ->
-// shared memory and writes rows (and, for symmetric outputs, mirrored columns)
-// with coalesced stores.  Every barrier wait is bounded; a wait that runs out
-// raises a status word instead of hanging.
-//
-// Factor builds (X^T X) have their own kernel further down, tc_pair_kernel:
-// 256 x 256 tiles, operands split into two bf16 terms (kind::f16 MMAs), the
-// im2col gather laid out with lanes along k.
+// Factor builds (C = alpha X^T X + beta C) on the tensor cores for sm_100a:
+// tc_pair_kernel, 256 x 256 tiles, operands gathered from global memory
+// (strided views or im2col patches of an NCHW tensor) and split into two bf16
+// terms (kind::f16 MMAs, fp32 accumulators in tensor memory), the im2col gather
+// laid out with lanes along k.  Every barrier wait is bounded; a wait that
+// runs out raises a status word instead of hanging.
 #include <algorithm>
 #include <mutex>
 #include <vector>
@@ -28,69 +15,10 @@ namespace kfac {
 
 constexpr int TC_BN = 256;
 constexpr int TC_BK = 32;
-// Producer warps per CTA (template parameter PW of the kernel, a multiple of
-// 8 that divides 96).  24 warps (72 registers per thread) gain 20 % on an
-// im2col gather with long image rows (128 pixels) but nothing at the 7..56
-// pixel rows of ResNet-50, where the per-thread offset bookkeeping that more
-// threads replicate costs as much as the extra warps hide; strided operands
-// need the 96 registers that only the 16-warp CTA leaves per thread.
-constexpr int TC_PW_STRIDED = 16;
-constexpr int TC_A_BYTES = TC_BM * TC_BK * 4;   // 16 KB
-constexpr int TC_B_BYTES = TC_BN * TC_BK * 4;   // 32 KB
-// one stage: [A hi][B hi][A lo][B lo]; a lo tile lies TC_LO_OFF after its hi
-constexpr int TC_LO_OFF = TC_A_BYTES + TC_B_BYTES;
-constexpr int TC_STAGE_BYTES = 2 * TC_LO_OFF;   // 96 KB
-// The A rows and then the B rows of a tile form one space of 384 rows; a
-// task index covers a band of 4 * PW of them (each warp 4 rows, or one
-// 16-byte column of 32 rows) and a thread has one task per band.
-template <int PW>
-struct TcMap {
-  static constexpr int kProducers = PW * 32;
-  static constexpr int kThreads = PW * 32 + 32;
-  static constexpr int kBand = PW * 4;
-  static constexpr int kTasks = (TC_BM + TC_BN) / kBand;
-  static_assert((TC_BM + TC_BN) % kBand == 0 && PW % 8 == 0 && TC_BM % 32 == 0,
-                "producer mapping");
-};
-constexpr int TC_STAGES = 2;
 constexpr int TC_EPI_PITCH = TC_BN + 1;         // floats
-constexpr int TC_SMEM_BYTES = TC_STAGES * TC_STAGE_BYTES + 8192 + 1024;
-// Two accumulators per tile: columns [0, 256) collect hi*hi, columns
-// [256, 512) the two cross terms, which are 2^-12 smaller; they are added in
-// the epilogue.  Keeping them apart means only one MMA in three adds into the
-// large sum.
-constexpr int TC_TMEM_COLS = 2 * TC_BN;
+constexpr int TC_TMEM_COLS = 2 * TC_BN;          // two 128-row accumulators
 
 static __device__ int g_tc_status = 0;
-
-#ifdef KFAC_TC_TRACE
-// Debug build only: CTA (0,0) records clock64() at fixed points of the
-// producer / MMA loops, 8 slots per k-block.
-__device__ long long* g_tc_trace = nullptr;
-__device__ int g_tc_trace_cap = 0;
-#define TC_TRACE(kb, slot)                                                   \
-  do {                                                                       \
-    if (g_tc_trace && blockIdx.x == 0 &&                  \
-        ((kb) * 8 + (slot)) < g_tc_trace_cap)                                \
-      g_tc_trace[(kb) * 8 + (slot)] = clock64();                             \
-  } while (0)
-#else
-#define TC_TRACE(kb, slot) do {} while (0)
-#endif
-
-struct TcControl {
-  unsigned long long full[TC_STAGES];
-  unsigned long long empty[TC_STAGES];
-  unsigned long long accum;
-  unsigned tmem_base;
-  volatile int abort_flag;
-  int found;
-  int coff_a[TC_BM];
-  int kykx_a[TC_BM];
-  int coff_b[TC_BN];
-  int kykx_b[TC_BN];
-  GemmDesc desc;
-};
 
 // Bounded wait on a phase parity; false if the limit ran out or the CTA is
 // already aborting (the status word behind kfac_tc_status is then set).
@@ -98,29 +26,6 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar,
                                           unsigned parity,
                                           volatile int* abort_flag) {
   return mbar_wait_status(bar, parity, abort_flag, &g_tc_status);
-}
-
-// im2col column tables for `rows` columns of a tile starting at column c0.
-__device__ __forceinline__ void tc_im2col_tables(const Operand& op, int c0,
-                                                 int rows, int* coff, int* kykx,
-                                                 int tid, int nthreads) {
-  for (int i = tid; i < rows; i += nthreads) {
-    int c = c0 + i;
-    int off = 0, info = -1;
-    if (c < op.ncols) {
-      int kk = op.ks * op.ks;
-      int ch = c / kk;
-      int r = c - ch * kk;
-      int ky = r / op.ks;
-      int kx = r - ky * op.ks;
-      off = ch * op.H * op.W + ky * op.W + kx;
-      info = (ky << 16) | kx;
-    } else if (c == op.extra_idx) {
-      info = -2;
-    }
-    coff[i] = off;
-    kykx[i] = info;
-  }
 }
 
 // Sources of constant columns: rows of the tile that lie beyond the operand
@@ -132,82 +37,15 @@ static __device__ __align__(256) float g_ones_page[64] = {
     1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1,
     1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
 
-// A producer thread moves TcMap<PW>::kTasks 16-byte chunks (4 consecutive k of one
-// tile row) per k-block, task t in band t of the 384 tile rows.  Within a
-// band the 8-warp group g = warp / 8 owns rows [32g, 32g + 32): operands
-// contiguous along k (and im2col operands) give a warp 4 rows x 8 chunks
-// (row = 4 * warp + lane / 8, chunk = lane % 8); operands contiguous along the
-// column index give it one chunk of 32 rows (row = 32g + lane, chunk =
-// warp % 8), so that a warp's loads of one k are 32 consecutive addresses.
-// Whether a task is an A row or a B row depends only on (t, g): uniform per
-// warp.  Per task everything that does not change with k is computed once:
-// the element address is
+// A producer task of a strided operand: everything that does not change with k
+// is computed once; the element address is
 //     p + (long long)o_j * m        (one multiply-add per element)
-// where o_j is the k-dependent offset shared by all tasks of the thread that
-// belong to the same operand.
+// where o_j is the k-dependent offset shared by all tasks of the thread.
 struct PTask {
   const char* p;    // column base (or the zero / ones page), as bytes
   int m;            // byte multiplier of the k-dependent offset (0 for pages)
   unsigned soff;    // swizzled byte offset inside the stage, ~0u: idle task
 };
-
-// 1: band t holds only A rows, 0: only B rows, -1: depends on the warp group
-template <int PW>
-__host__ __device__ constexpr int tc_band_side(int t) {
-  return 4 * PW * (t + 1) <= TC_BM ? 1 : (4 * PW * t >= TC_BM ? 0 : -1);
-}
-
-template <int PW>
-__device__ __forceinline__ bool tc_task_is_a(int t, int warp) {
-  return tc_band_side<PW>(t) >= 0 ? tc_band_side<PW>(t) == 1
-                                  : 4 * PW * t + 32 * (warp >> 3) < TC_BM;
-}
-
-template <bool IM2COL, int PW>
-__device__ __forceinline__ void tc_task_setup(const Operand& A,
-                                              const Operand& B, int m0, int n0,
-                                              int rows_b, bool skip_a,
-                                              const TcControl* ctl,
-                                              int warp, int lane,
-                                              PTask task[TcMap<PW>::kTasks]) {
-#pragma unroll
-  for (int t = 0; t < TcMap<PW>::kTasks; ++t) {
-    const bool is_a = tc_task_is_a<PW>(t, warp);
-    const Operand& op = is_a ? A : B;
-    const bool kf = IM2COL || op.kfast;
-    const int band_row = kf ? warp * 4 + (lane >> 3) : 32 * (warp >> 3) + lane;
-    const int row = TcMap<PW>::kBand * t + band_row - (is_a ? 0 : TC_BM);
-    const int rows = is_a ? (skip_a ? 0 : TC_BM) : rows_b;
-    const int chunk = kf ? (lane & 7) : (warp & 7);
-    PTask v;
-    v.soff = row < rows ? (unsigned)((is_a ? 0 : TC_A_BYTES) + row * 128 +
-                                     ((chunk ^ (row & 7)) << 4))
-                        : ~0u;
-    const float* p = g_zero_page;
-    int m = 0;
-    if (row < rows) {
-      const int c = (is_a ? m0 : n0) + row;
-      if (IM2COL) {
-        const int info = (is_a ? ctl->kykx_a : ctl->kykx_b)[row];
-        if (info >= 0) {
-          p = op.base + (is_a ? ctl->coff_a : ctl->coff_b)[row];
-          m = 1;
-        } else if (info == -2) {
-          p = g_ones_page;
-        }
-      } else if (c < op.ncols) {
-        p = op.base + (long long)c * op.s_col;
-        m = op.period == 1 ? (int)op.s_outer : 1;
-      } else if (c == op.extra_idx) {
-        if (op.extra) { p = op.extra; m = 1; }
-        else p = g_ones_page;
-      }
-    }
-    v.p = reinterpret_cast<const char*>(p);
-    v.m = m * 4;
-    task[t] = v;
-  }
-}
 
 // Position of a thread's chunk (4 consecutive k) in an operand's row space,
 // kept incrementally from k-block to k-block so that the hot loop has no
@@ -291,45 +129,6 @@ __device__ __forceinline__ void tc_koffsets(const Operand& op,
   }
 }
 
-// Gather the chunks of one operand (SIDE_A: the A rows, else the B rows) for
-// one k-block into registers.  The loads are issued back to back, each from
-// an address that is always legal; nothing between two loads depends on a
-// loaded value.  `vec` (uniform per tile): every chunk of this operand is
-// 16-byte aligned and contiguous.
-template <bool TAILS, int PW, bool SIDE_A>
-__device__ __forceinline__ void tc_load_side(
-    const PTask task[TcMap<PW>::kTasks], const int o[4], int k, int kend,
-    bool vec, int warp, float4 v[TcMap<PW>::kTasks]) {
-  constexpr int NT = TcMap<PW>::kTasks;
-  const bool tail = TAILS && (k + 3 >= kend);
-  if (vec && !tail) {
-#pragma unroll
-    for (int t = 0; t < NT; ++t)
-      if (tc_task_is_a<PW>(t, warp) == SIDE_A && task[t].soff != ~0u)
-        v[t] = *reinterpret_cast<const float4*>(
-            task[t].p + (long long)o[0] * task[t].m);
-  } else {
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      if (tc_task_is_a<PW>(t, warp) != SIDE_A || task[t].soff == ~0u) continue;
-      v[t].x = *reinterpret_cast<const float*>(task[t].p + (long long)o[0] * task[t].m);
-      v[t].y = *reinterpret_cast<const float*>(task[t].p + (long long)o[1] * task[t].m);
-      v[t].z = *reinterpret_cast<const float*>(task[t].p + (long long)o[2] * task[t].m);
-      v[t].w = *reinterpret_cast<const float*>(task[t].p + (long long)o[3] * task[t].m);
-    }
-  }
-  if (tail) {
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      if (tc_task_is_a<PW>(t, warp) != SIDE_A) continue;
-      if (k + 0 >= kend) v[t].x = 0.f;
-      if (k + 1 >= kend) v[t].y = 0.f;
-      if (k + 2 >= kend) v[t].z = 0.f;
-      if (k + 3 >= kend) v[t].w = 0.f;
-    }
-  }
-}
-
 // True when every 16-byte chunk of a k-contiguous strided operand is aligned
 // and contiguous for k-blocks that start at kbeg (uniform for the tile).
 __device__ __forceinline__ bool tc_operand_vec(const Operand& op,
@@ -340,16 +139,6 @@ __device__ __forceinline__ bool tc_operand_vec(const Operand& op,
   if (op.extra_idx >= 0 && op.extra != nullptr) return false;
   if (op.period == 1) return op.s_outer == 1;
   return (op.period & 3) == 0 && (op.s_outer & 3) == 0 && op.s_inner == 1;
-}
-
-template <int NT>
-__device__ __forceinline__ void tc_store_tile(const PTask task[NT],
-                                              unsigned stage,
-                                              const float4 v[NT]) {
-#pragma unroll
-  for (int t = 0; t < NT; ++t)
-    if (task[t].soff != ~0u)
-      store_split(stage + task[t].soff, stage + TC_LO_OFF + task[t].soff, v[t]);
 }
 
 // Lower-triangular enumeration with 128-row x 256-column tiles: tile (bi, bj)
@@ -365,336 +154,6 @@ __device__ __forceinline__ void tc_tri_tile(int t, int& bi, int& bj) {
   } else {
     bi = 2 * a;
     bj = t - a * (a + 1);
-  }
-}
-
-template <bool IM2COL, bool TAILS, int PW>
-__global__ void __launch_bounds__(TcMap<PW>::kThreads, 1)
-tc_gemm_kernel(const GemmDesc* __restrict__ descs, int ndesc,
-               const __grid_constant__ GemmDesc inline_desc, float lr,
-               float momentum) {
-  extern __shared__ unsigned char tc_smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-  TcControl* ctl =
-      reinterpret_cast<TcControl*>(smem + TC_STAGES * TC_STAGE_BYTES);
-  constexpr int TC_PRODUCERS = TcMap<PW>::kProducers;
-  constexpr int TC_PWARPS = PW;
-  constexpr int TC_THREADS = TcMap<PW>::kThreads;
-  constexpr int TC_NTASK = TcMap<PW>::kTasks;
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
-  const int tile = blockIdx.x;
-
-  // ---- locate the problem and copy its descriptor to shared memory.  The
-  // search is one parallel round: thread t tests descriptor t (tile_begin is
-  // ascending), instead of a chain of dependent global loads.
-  {
-    const GemmDesc* src = &inline_desc;
-    if (descs != nullptr) {
-      for (int i = tid; i < ndesc; i += TC_THREADS) {
-        const int lo = descs[i].tile_begin;
-        const int hi = (i + 1 < ndesc) ? descs[i + 1].tile_begin : 0x7fffffff;
-        if (lo <= tile && tile < hi) ctl->found = i;
-      }
-      __syncthreads();
-      src = descs + ctl->found;
-    }
-    const int* s = reinterpret_cast<const int*>(src);
-    int* d = reinterpret_cast<int*>(&ctl->desc);
-    for (int i = tid; i < (int)(sizeof(GemmDesc) / sizeof(int)); i += TC_THREADS)
-      d[i] = s[i];
-  }
-  if (tid == 0) {
-    for (int s = 0; s < TC_STAGES; ++s) {
-      mbar_init(&ctl->full[s], TC_PRODUCERS / 32);
-      mbar_init(&ctl->empty[s], 1);
-    }
-    mbar_init(&ctl->accum, 1);
-    ctl->abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == TC_PRODUCERS / 32) {
-    asm volatile(
-        "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-        ::"r"(smem_u32(&ctl->tmem_base)), "r"(TC_TMEM_COLS)
-        : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
-                 ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-  const GemmDesc& g = ctl->desc;
-  const unsigned tmem = ctl->tmem_base;
-  int lt = tile - g.tile_begin, split = 0;
-  if (g.splits > 1) {
-    split = lt / g.ntiles;
-    lt -= split * g.ntiles;
-  }
-  int bi, bj;
-  if (g.flags & G_LOWER) {
-    tc_tri_tile(lt, bi, bj);
-  } else {
-    bi = lt / g.tiles_n;
-    bj = lt - bi * g.tiles_n;
-  }
-  const int m0 = bi * TC_BM, n0 = bj * TC_BN;
-  int n_valid = min(TC_BN, g.N - n0);
-  if (g.flags & G_LOWER) n_valid = min(n_valid, m0 + TC_BM - n0);
-  const int n_inst = (n_valid + 15) & ~15;
-  const int m_valid = min(TC_BM, g.M - m0);
-
-  long long kbeg = 0, kend = g.K;
-  if (g.splits > 1) {
-    kbeg = (long long)split * g.k_per_split;
-    kend = min(g.K, kbeg + g.k_per_split);
-  }
-  if (g.flags & G_KBEG_N0) kbeg = max(kbeg, (long long)n0);
-  if (g.flags & G_KBEG_M0) kbeg = max(kbeg, (long long)(m0 - g.kbeg_off));
-  if (g.flags & G_KEND_M0) kend = min(kend, (long long)(m0 + TC_BM));
-  // a gated-off problem runs no k-blocks and stores nothing
-  const bool gated_off = g.gate != nullptr && *g.gate == 0;
-  const int nkb = (kend > kbeg && !gated_off)
-                      ? (int)((kend - kbeg + TC_BK - 1) / TC_BK) : 0;
-  // X^T X on a diagonal tile: the tile's A rows are rows [m0 - n0, m0 - n0 +
-  // 128) of its B rows (m0 - n0 is 0 or 128), so only B is staged and the A
-  // descriptors point into the B tiles.
-  const bool share_ab = (g.flags & G_SAME_AB) && (g.flags & G_LOWER) &&
-                        bj == (bi >> 1);
-
-  if (warp < TC_PRODUCERS / 32) {
-    // ===================== producers =====================
-    if (IM2COL) {
-      tc_im2col_tables(g.A, m0, TC_BM, ctl->coff_a, ctl->kykx_a, tid,
-                       TC_PRODUCERS);
-      tc_im2col_tables(g.B, n0, n_inst, ctl->coff_b, ctl->kykx_b, tid,
-                       TC_PRODUCERS);
-      asm volatile("bar.sync 1, %0;" ::"r"(TC_PRODUCERS) : "memory");
-    }
-    const Operand A = g.A, B = g.B;   // register copies: loop invariant
-    float4 v[TC_NTASK];
-    PTask task[TC_NTASK];
-    tc_task_setup<IM2COL, PW>(A, B, m0, n0, n_inst, share_ab, ctl, warp, lane,
-                              task);
-    const int kend_i = (int)kend;
-    KState ka, kb_state;
-    {
-      const bool a_kf = IM2COL || A.kfast;
-      const bool b_kf = IM2COL || B.kfast;
-      kstate_init<IM2COL>(A, kbeg + 4 * (a_kf ? (lane & 7) : (warp & 7)), ka);
-      kstate_init<IM2COL>(B, kbeg + 4 * (b_kf ? (lane & 7) : (warp & 7)),
-                          kb_state);
-    }
-    const unsigned smem_base = smem_u32(smem);
-    const bool vec_a = !IM2COL && tc_operand_vec(A, kbeg);
-    const bool vec_b = !IM2COL && tc_operand_vec(B, kbeg);
-    // iteration kb stores k-block kb-1 (loaded one iteration earlier) and
-    // issues the loads of k-block kb, which then fly while the tensor core
-    // works and while this warp waits for the stage to drain
-    for (int kb = 0; kb <= nkb; ++kb) {
-      if (kb > 0) {
-        const int pb = kb - 1;
-        const int s = pb % TC_STAGES;
-        if (tid == 0) TC_TRACE(pb, 0);
-        if (pb >= TC_STAGES) {
-          if (!mbar_wait(&ctl->empty[s], ((pb / TC_STAGES) - 1) & 1,
-                         &ctl->abort_flag))
-            break;
-        }
-        if (tid == 0) TC_TRACE(pb, 1);
-        tc_store_tile<TC_NTASK>(task, smem_base + s * TC_STAGE_BYTES, v);
-        if (tid == 0) TC_TRACE(pb, 2);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ctl->full[s]);
-        if (tid == 0) TC_TRACE(pb, 3);
-      }
-      if (kb < nkb) {
-        int oa[4], ob[4];
-        tc_koffsets<IM2COL, TAILS>(A, ka, kend_i, oa);
-        if (IM2COL) {
-          // both operands are the same patch matrix and use the same chunk
-          // mapping: one set of pixel offsets serves both
-#pragma unroll
-          for (int j = 0; j < 4; ++j) ob[j] = oa[j];
-        } else {
-          tc_koffsets<IM2COL, TAILS>(B, kb_state, kend_i, ob);
-        }
-        tc_load_side<TAILS, PW, true>(task, oa, ka.k, kend_i, vec_a, warp, v);
-        tc_load_side<TAILS, PW, false>(task, ob, IM2COL ? ka.k : kb_state.k,
-                                       kend_i, vec_b, warp, v);
-        kstate_advance<IM2COL>(A, ka);
-        if (!IM2COL) kstate_advance<IM2COL>(B, kb_state);
-        if (tid == 0) TC_TRACE(kb, 4);
-      }
-    }
-  } else {
-    // ===================== MMA issuer =====================
-    if (elect_one()) {
-      const unsigned idesc = tc_instr_desc(n_inst);
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % TC_STAGES;
-        TC_TRACE(kb, 5);
-        if (!mbar_wait(&ctl->full[s], (kb / TC_STAGES) & 1, &ctl->abort_flag))
-          break;
-        TC_TRACE(kb, 6);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned sa = smem_u32(smem + s * TC_STAGE_BYTES);
-        const unsigned a_off =
-            share_ab ? (unsigned)(TC_A_BYTES + (m0 - n0) * 128) : 0u;
-        const unsigned long long a_hi = tc_smem_desc(sa + a_off);
-        const unsigned long long b_hi = tc_smem_desc(sa + TC_A_BYTES);
-        const unsigned long long a_lo = tc_smem_desc(sa + TC_LO_OFF + a_off);
-        const unsigned long long b_lo =
-            tc_smem_desc(sa + TC_LO_OFF + TC_A_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < TC_BK / 8; ++kk) {
-          const unsigned long long adv = (unsigned long long)(kk * 32 >> 4);
-          tc_mma(tmem + TC_BN, a_lo + adv, b_hi + adv, idesc, (kb | kk) != 0);
-          tc_mma(tmem + TC_BN, a_hi + adv, b_lo + adv, idesc, 1);
-          tc_mma(tmem, a_hi + adv, b_hi + adv, idesc, (kb | kk) != 0);
-        }
-        tc_commit(&ctl->empty[s]);
-        TC_TRACE(kb, 7);
-      }
-      tc_commit(&ctl->accum);
-    }
-    __syncwarp();
-  }
-
-  // ===================== epilogue =====================
-  float* stage = reinterpret_cast<float*>(smem);
-  bool ok = true;
-  if (warp < TC_PRODUCERS / 32) {
-    if (nkb > 0) {
-      ok = mbar_wait(&ctl->accum, 0, &ctl->abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    }
-    // warp w reads the 32 accumulator rows of its TMEM quarter q = w % 4;
-    // the TC_PWARPS / 4 warps of a quarter take 16-column slices in turn
-    const int q = warp & 3, h = warp >> 2;
-    const int row = q * 32 + lane;
-    for (int c0 = h * 16; c0 < n_inst; c0 += 16 * (TC_PWARPS / 4)) {
-      float v[16];
-      if (nkb > 0 && ok) {
-        float w[16];
-        tc_ld16(tmem + ((unsigned)(q * 32) << 16) + (unsigned)c0, v);
-        tc_ld16(tmem + ((unsigned)(q * 32) << 16) + (unsigned)(TC_BN + c0), w);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] += w[i];
-      } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = 0.f;
-      }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) stage[row * TC_EPI_PITCH + c0 + i] = v[i];
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == TC_PRODUCERS / 32) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
-                 ::"r"(tmem), "r"(TC_TMEM_COLS)
-                 : "memory");
-  }
-  if (warp >= TC_PRODUCERS / 32 || ctl->abort_flag || gated_off) return;
-
-  if (g.splits > 1) {
-    float* p = g.partial + ((long long)split * g.ntiles + lt) * (TC_BM * TC_BN);
-    for (int r = warp; r < TC_BM; r += TC_PWARPS)
-      for (int c = lane; c < n_inst; c += 32)
-        p[r * TC_BN + c] = stage[r * TC_EPI_PITCH + c];
-    return;
-  }
-  if (g.flags & G_PRECOND) {
-    const int dW = g.dW;
-    for (int r = warp; r < m_valid; r += TC_PWARPS) {
-      const int gr = m0 + r;
-      float ov[TC_BN / 32], op[TC_BN / 32];
-      if (g.pW != nullptr) {
-#pragma unroll
-        for (int i = 0; i < TC_BN / 32; ++i) {
-          const int c = lane + 32 * i, gc = n0 + c;
-          ov[i] = op[i] = 0.f;
-          if (c < n_valid) {
-            if (gc < dW) {
-              ov[i] = g.vW[(long long)gr * dW + gc];
-              op[i] = g.pW[(long long)gr * dW + gc];
-            } else if (g.pb != nullptr) {
-              ov[i] = g.vb[gr];
-              op[i] = g.pb[gr];
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < TC_BN / 32; ++i) {
-        const int c = lane + 32 * i, gc = n0 + c;
-        if (c >= n_valid) continue;
-        const float kf = stage[r * TC_EPI_PITCH + c];
-        if (gc < dW) {
-          const long long idx = (long long)gr * dW + gc;
-          if (g.kfW) g.kfW[idx] = kf;
-          if (g.pW) {
-            const float nv = momentum * ov[i] - lr * kf;
-            g.vW[idx] = nv;
-            g.pW[idx] = op[i] + nv;
-          }
-        } else {
-          if (g.kfb) g.kfb[gr] = kf;
-          if (g.pb) {
-            const float nv = momentum * ov[i] - lr * kf;
-            g.vb[gr] = nv;
-            g.pb[gr] = op[i] + nv;
-          }
-        }
-      }
-    }
-    return;
-  }
-  const float alpha = g.alpha;
-  const float beta = (g.beta_until > 0 && m0 >= g.beta_until) ? 0.f : g.beta;
-  const bool lower = (g.flags & G_LOWER) != 0;
-  const bool mirror = (g.flags & G_MIRROR) != 0;
-  // rows: C[gr][gc] = alpha * acc + beta * C[gr][gc]; the final value is kept
-  // in the staging tile for the mirrored pass.  A lane owns columns lane,
-  // lane + 32, ...; all of a row's reads of C are issued before any is used.
-  for (int r = warp; r < m_valid; r += TC_PWARPS) {
-    const int gr = m0 + r;
-    float* crow = g.C + (long long)gr * g.ldc + n0;
-    const int cend = lower ? min(n_valid, gr - n0 + 1) : n_valid;
-    float old[TC_BN / 32];
-    if (beta != 0.f) {
-#pragma unroll
-      for (int i = 0; i < TC_BN / 32; ++i) {
-        const int c = lane + 32 * i;
-        old[i] = c < cend ? crow[c] : 0.f;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < TC_BN / 32; ++i) {
-      const int c = lane + 32 * i;
-      if (c < cend) {
-        float v = alpha * stage[r * TC_EPI_PITCH + c];
-        if (beta != 0.f) v += beta * old[i];
-        crow[c] = v;
-        if (g.C2 != nullptr) g.C2[(long long)gr * g.ldc + n0 + c] = v;
-        if (mirror) stage[r * TC_EPI_PITCH + c] = v;
-      }
-    }
-  }
-  if (mirror) {
-    asm volatile("bar.sync 1, %0;" ::"r"(TC_PRODUCERS) : "memory");
-    for (int c = warp; c < n_valid; c += TC_PWARPS) {
-      const int gc = n0 + c;
-      for (int r = lane; r < m_valid; r += 32) {
-        const int gr = m0 + r;
-        if (gc < gr) g.C[(long long)gc * g.ldc + gr] = stage[r * TC_EPI_PITCH + c];
-      }
-    }
   }
 }
 
@@ -1425,12 +884,6 @@ int tc_prepare() {
   KFAC_REQUIRE(dev >= 0 && dev < 64, "device index %d unsupported", dev);
   std::lock_guard<std::mutex> lock(mu);
   if (!done[dev]) {
-    KFAC_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<false, false, TC_PW_STRIDED>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   TC_SMEM_BYTES));
-    KFAC_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<false, true, TC_PW_STRIDED>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   TC_SMEM_BYTES));
     KFAC_CUDA(cudaFuncSetAttribute(tc_pair_kernel<false, false, true>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    PK_SMEM_BYTES));
@@ -1448,25 +901,6 @@ int tc_prepare() {
                                    PK_SMEM_BYTES));
     done[dev] = true;
   }
-  return KFAC_OK;
-}
-
-int launch_tc_grouped(const GemmDesc* descs_dev, int ndesc, int total_tiles,
-                      float lr, float momentum, bool tails,
-                      cudaStream_t stream) {
-  if (ndesc <= 0 || total_tiles <= 0) return KFAC_OK;
-  int rc = tc_prepare();
-  if (rc != KFAC_OK) return rc;
-  GemmDesc dummy = {};
-  if (tails)
-    tc_gemm_kernel<false, true, TC_PW_STRIDED><<<total_tiles, TcMap<TC_PW_STRIDED>::kThreads, TC_SMEM_BYTES,
-                                  stream>>>(descs_dev, ndesc, dummy, lr,
-                                            momentum);
-  else
-    tc_gemm_kernel<false, false, TC_PW_STRIDED><<<total_tiles, TcMap<TC_PW_STRIDED>::kThreads, TC_SMEM_BYTES,
-                                   stream>>>(descs_dev, ndesc, dummy, lr,
-                                             momentum);
-  KFAC_LAUNCH_CHECK("tc_gemm_kernel");
   return KFAC_OK;
 }
 
@@ -1974,14 +1408,6 @@ extern "C" int kfac_get_factor_staging(void) {
   return kfac::tc_staged() ? 1 : 0;
 }
 
-#ifdef KFAC_TC_TRACE
-extern "C" int kfac_tc_trace(long long* buf_dev, int capacity) {
-  KFAC_CUDA(cudaMemcpyToSymbol(kfac::g_tc_trace, &buf_dev, sizeof(buf_dev)));
-  KFAC_CUDA(cudaMemcpyToSymbol(kfac::g_tc_trace_cap, &capacity, sizeof(int)));
-  return KFAC_OK;
-}
-#endif
-
 namespace kfac {
 // Self-test of the bounded barrier wait every tile kernel relies on: one warp
 // waits on a barrier that nothing will ever arrive at, with a short limit.
@@ -2030,12 +1456,11 @@ extern "C" int kfac_tc_status(int* status_out) {
   KFAC_CUDA(cudaDeviceSynchronize());
   int v = 0;
   KFAC_CUDA(cudaMemcpyFromSymbol(&v, kfac::g_tc_status, sizeof(int)));
-  int w = 0;
+  int w = 0, t = 0, u = 0;
   int rc = kfac::diag_status_read(&w);
+  if (rc == KFAC_OK) rc = kfac::tile_status_read(&t);
+  if (rc == KFAC_OK) rc = kfac::gram_status_read(&u);
   if (rc != KFAC_OK) return rc;
-  int u = 0;
-  rc = kfac::gram_status_read(&u);
-  if (rc != KFAC_OK) return rc;
-  *status_out = v | w | u;
+  *status_out = v | w | t | u;
   return KFAC_OK;
 }

@@ -1,0 +1,782 @@
+// Tensor-core tile engine of the inverse and precondition products for
+// sm_100a: C = alpha A B + beta C over many problems in one launch (GemmDesc),
+// tcgen05.mma (kind::tf32) with fp32 accumulators in tensor memory, fp32
+// operands split into two TF32 terms (x = hi + lo with hi rounded to nearest,
+// C += hi*hi + hi*lo + lo*hi) so that results keep near-fp32 accuracy (a
+// single TF32 pass misses the 1e-4 bound on large factors).
+//
+// One CTA owns a 128 x TN tile.  Producer warps load the operands from global
+// memory with 16-byte loads, one or two 32-k blocks ahead in registers, split them
+// and write the K-major, 128-byte-swizzled shared-memory layout that the MMA
+// descriptors expect; one more warp issues the MMAs.  The epilogue moves
+// 32 x 32 pieces of the accumulator TMEM -> registers -> shared memory ->
+// global rows (and, for symmetric outputs, mirrored rows straight from the
+// registers, where a column of a piece is contiguous).
+//
+// Bound: the long products by the MMAs (three per product) and, next to them,
+// the shared-memory traffic of their operands; the many short ones (K = 128
+// inside a Cholesky panel) by latency: descriptor fetch, one trip to L2 per
+// register block, the epilogue's trip for C.  Hence the descriptors of small
+// launches travel as kernel arguments, C is prefetched before the accumulator
+// is waited for, and TN = 128 (half the work per CTA, twice the CTAs) is used
+// while 128 x 256 tiles would leave SMs idle.  One tile with K = 128: 20 us with
+// an update of C and 12.4 us without before, 13.5 and 11 us now; a 2304-row
+// inverse 888 -> 791 us, 14 pairs of odd sides 541 -> 447 us.
+//
+// Every barrier wait is bounded; a wait that runs out raises a status word
+// instead of hanging.
+#include <algorithm>
+#include <mutex>
+
+#include "gemm_simt.cuh"
+#include "tc_common.cuh"
+
+namespace kfac {
+
+constexpr int TT_BK = 32;
+constexpr int TT_EP = 36;         // row pitch of an epilogue piece (floats)
+constexpr int TT_INLINE = 8;      // descriptors that fit the kernel arguments
+
+static __device__ int g_tile_status = 0;
+
+template <int TN>
+struct TileMap {
+  static constexpr int kProducers = TN == 256 ? 384 : 256;
+  static constexpr int kWarps = kProducers / 32;
+  static constexpr int kThreads = kProducers + 32;
+  static constexpr int kStages = TN == 256 ? 2 : 3;
+  static constexpr int kABytes = TC_BM * TT_BK * 4;       // 16 KB
+  static constexpr int kBBytes = TN * TT_BK * 4;
+  static constexpr int kLo = kABytes + kBBytes;   // a lo tile after its hi tile
+  static constexpr int kStage = 2 * kLo;
+  static constexpr int kTmem = 2 * TN;            // hi*hi, then cross terms
+  static constexpr int kSmem = kStages * kStage + 1024 + 1024;
+};
+
+struct TileControl {
+  unsigned long long full[3];
+  unsigned long long empty[3];
+  unsigned long long accum;
+  unsigned tmem_base;
+  volatile int abort_flag;
+  GemmDesc desc;
+};
+static_assert(sizeof(TileControl) <= 1024, "tile control block");
+
+struct TileInline {
+  int n;                       // 0: descriptors in device memory
+  GemmDesc d[TT_INLINE];
+};
+static_assert(sizeof(TileInline) <= 3800, "kernel argument space");
+
+// One producer unit: four 16-byte chunks (4 consecutive k of one tile row) per
+// 32-k block.  Operands contiguous along k: a warp covers 16 rows, one load
+// instruction 4 rows x 128 bytes.  Operands contiguous along the tile rows: a
+// warp covers 16 k x 32 rows, a thread a 4 x 4 block that it transposes by
+// naming its registers; lanes are laid out so that loads cover 128-byte pieces
+// of four k and the stores of a quarter warp fall into different banks.
+// Operands whose rows are not 16-byte aligned (the caller's matrices of odd
+// sides) are read a float per lane along the contiguous index instead: a load
+// instruction still covers one 128-byte piece, of one row (k along the lanes,
+// 16 rows of a thread's k) or of one k (rows along the lanes, 16 k of a
+// thread's row).
+//
+// Rows past the operand's last one repeat it: their accumulator rows (columns)
+// are never stored.  Only the appended column of a gradient and the end of the
+// contraction need values of their own.
+struct TileUnit {
+  const float* p;        // first element of the unit in the current block
+  int o[3];              // 16-byte words: offsets of chunks 1 .. 3
+  int step;              // else: elements from one row (kfast) or k to the next
+  int adv;               // elements from one block to the next
+  int k;                 // first k of the unit in the current block
+  int row;               // first row (not kfast: of four consecutive ones)
+  int last;              // kfast: rows from there to the operand's last one
+  unsigned soff;         // store offset of chunk 0 inside a stage
+  int flags;
+};
+enum { U_KFAST = 1, U_LIVE = 2, U_EXTRA = 4 };
+
+// Rows of an operand can be read as 16-byte words.
+__host__ __device__ __forceinline__ bool tile_operand_vec(const Operand& op) {
+  const long long ld = op.kfast ? op.s_col : op.s_outer;
+  return (reinterpret_cast<uintptr_t>(op.base) & 15) == 0 && (ld & 3) == 0;
+}
+
+// `wu`: index of the 32-thread unit among those of its side; `rows`: valid rows
+// of the side (units past them stay idle: their rows are never stored).
+template <bool VEC>
+__device__ __forceinline__ void tile_unit_setup(const Operand& op, int r0,
+                                                int wu, int lane, int kbeg,
+                                                int rows, unsigned side_off,
+                                                TileUnit& u) {
+  const bool kf = op.kfast != 0;
+  const int ld = kf ? (int)op.s_col : (int)op.s_outer;
+  u.flags = kf ? U_KFAST : 0;
+  // the unit holds the appended column
+  const int first = kf ? 16 * wu : 32 * (wu >> 1), span = kf ? 16 : 32;
+  if (first < rows) u.flags |= U_LIVE;
+  if (op.extra_idx >= r0 + first && op.extra_idx < r0 + first + span)
+    u.flags |= U_EXTRA;
+  if (!VEC) {
+    const int row = kf ? first : first + lane;
+    u.k = kbeg + (kf ? lane : 16 * (wu & 1));
+    u.row = r0 + row;
+    const int r = min(u.row, op.ncols - 1);
+    u.last = op.ncols - 1 - r;
+    u.p = op.base + (kf ? (long long)r * ld + u.k : (long long)u.k * ld + r);
+    u.step = ld;
+    u.adv = kf ? TT_BK : TT_BK * ld;
+    u.soff = side_off + (kf ? (unsigned)(row * 128 + 4 * (lane & 3))
+                            : (unsigned)(row * 128));
+    return;
+  }
+  if (kf) {
+    const int chunk = lane & 7, row = first + (lane >> 3);
+    u.k = kbeg + 4 * chunk;
+    u.row = r0 + row;
+    const int r = min(u.row, op.ncols - 1);
+    u.last = op.ncols - 1 - r;
+    u.p = op.base + (long long)r * ld + u.k;
+#pragma unroll
+    for (int i = 1; i < 4; ++i) u.o[i - 1] = min(4 * i, u.last) * ld;
+    u.adv = TT_BK;
+    u.soff = side_off + sw128_chunk_off(row, chunk);
+  } else {
+    const int kq = 4 * (wu & 1) + (lane & 3);
+    const int row = first + 4 * (lane >> 2);
+    u.k = kbeg + 4 * kq;
+    u.row = r0 + row;
+    u.last = 0;
+    // (whole words: the pitch covers the last one)
+    u.p = op.base + (long long)u.k * ld + min(u.row, (op.ncols - 1) & ~3);
+#pragma unroll
+    for (int i = 1; i < 4; ++i) u.o[i - 1] = i * ld;
+    u.adv = TT_BK * ld;
+    u.soff = side_off + sw128_chunk_off(row, kq);
+  }
+}
+
+template <bool VEC>
+__device__ __forceinline__ void tile_unit_load(const Operand& op, TileUnit& u,
+                                               int kend, float4 v[4]) {
+  if (!(u.flags & U_LIVE)) return;
+  const bool kf = (u.flags & U_KFAST) != 0;
+  const float* p = u.p;
+  if (!VEC) {
+    float x[16];
+    if (kf) {
+      const bool in = u.k < kend;
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        x[i] = in ? p[(long long)min(i, u.last) * u.step] : 0.f;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i, p += u.step)
+        x[i] = u.k + i < kend ? *p : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      v[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+  } else if (u.k + 3 < kend) {
+    v[0] = *reinterpret_cast<const float4*>(p);
+#pragma unroll
+    for (int i = 1; i < 4; ++i)
+      v[i] = *reinterpret_cast<const float4*>(p + u.o[i - 1]);
+  } else {
+    // the end of the contraction: of every row, or whole k
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float* q = i == 0 ? p : p + u.o[i - 1];
+      const int left = kf ? kend - u.k : (u.k + i < kend ? 4 : 0);
+      v[i].x = left > 0 ? q[0] : 0.f;
+      v[i].y = left > 1 ? q[1] : 0.f;
+      v[i].z = left > 2 ? q[2] : 0.f;
+      v[i].w = left > 3 ? q[3] : 0.f;
+    }
+  }
+  if (u.flags & U_EXTRA) {
+    // the appended column (row extra_idx of the tile) of a gradient
+    float* x = reinterpret_cast<float*>(v);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int a = i >> 2, b = i & 3;
+      const int k = VEC ? (kf ? u.k + b : u.k + a) : (kf ? u.k : u.k + i);
+      const int c = VEC ? (kf ? u.row + 4 * a : u.row + b)
+                        : (kf ? u.row + i : u.row);
+      if (c == op.extra_idx)
+        x[i] = k >= kend ? 0.f : (op.extra != nullptr ? op.extra[k] : 1.f);
+    }
+  }
+  u.k += TT_BK;
+  u.p += u.adv;
+}
+
+template <bool VEC>
+__device__ __forceinline__ void tile_unit_store(const TileUnit& u, unsigned st,
+                                                unsigned lo, const float4 v[4]) {
+  if (!(u.flags & U_LIVE)) return;
+  const unsigned at = st + u.soff;
+  const int lane = threadIdx.x & 31;
+  if (!VEC) {
+    if (u.flags & U_KFAST) {
+      // k = lane of rows 0 .. 15 (a multiple of 16 rows from the tile's start)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float4 q = v[i >> 2];
+        const float x = (i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y
+                        : (i & 3) == 2 ? q.z : q.w;
+        const float h = tf32_round(x);
+        const unsigned d = at + 128 * i + (((lane >> 2) ^ (i & 7)) << 4);
+        sts32(d, h);
+        sts32(d + lo, x - h);
+      }
+    } else {
+      // chunks of row `lane`, from the 16 k of this unit on
+      const int half = ((threadIdx.x >> 5) & 1) * 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const unsigned d = at + (((half + i) ^ (lane & 7)) << 4);
+        store_split(d, d + lo, v[i]);
+      }
+    }
+  } else if (u.flags & U_KFAST) {
+    // chunk i is 4 i rows down: the swizzle flips with every second step
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const unsigned d = (at ^ ((i & 1) ? 0x40u : 0u)) + 512 * i;
+      store_split(d, d + lo, v[i]);
+    }
+  } else {
+    store_split(at, at + lo, make_float4(v[0].x, v[1].x, v[2].x, v[3].x));
+    const unsigned d1 = (at ^ 0x10u) + 128;
+    store_split(d1, d1 + lo, make_float4(v[0].y, v[1].y, v[2].y, v[3].y));
+    const unsigned d2 = (at ^ 0x20u) + 256;
+    store_split(d2, d2 + lo, make_float4(v[0].z, v[1].z, v[2].z, v[3].z));
+    const unsigned d3 = (at ^ 0x30u) + 384;
+    store_split(d3, d3 + lo, make_float4(v[0].w, v[1].w, v[2].w, v[3].w));
+  }
+}
+
+// 32 accumulator columns of this warp's 32 rows (both accumulators added, times
+// alpha) into its shared-memory piece, a row per lane.
+template <int TN>
+__device__ __forceinline__ void tile_acc_piece(unsigned tmem, int q, int c0,
+                                               float alpha, bool zero,
+                                               float* piece, int lane) {
+  const unsigned row = (unsigned)(q * 32) << 16;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float v[16], w[16];
+    if (!zero) {
+      tc_ld16(tmem + row + (unsigned)(c0 + 16 * h), v);
+      tc_ld16(tmem + row + (unsigned)(TN + c0 + 16 * h), w);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = w[i] = 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; i += 4)
+      *reinterpret_cast<float4*>(&piece[lane * TT_EP + 16 * h + i]) =
+          make_float4(alpha * (v[i] + w[i]), alpha * (v[i + 1] + w[i + 1]),
+                      alpha * (v[i + 2] + w[i + 2]),
+                      alpha * (v[i + 3] + w[i + 3]));
+  }
+}
+
+// Tile (bi, bj) of lower-triangular problem tile t; 128 x 256 tiles exist iff
+// 2 bj <= bi, 128 x 128 tiles iff bj <= bi.
+template <int TN>
+__device__ __forceinline__ void tile_lower(int t, int& bi, int& bj) {
+  if (TN == 128) {
+    tri_tile(t, bi, bj);
+    return;
+  }
+  int a = (int)sqrtf((float)t);
+  while ((a + 1) * (a + 1) <= t) ++a;
+  while (a * a > t) --a;
+  if (t < a * (a + 1)) {
+    bi = 2 * a - 1;
+    bj = t - a * a;
+  } else {
+    bi = 2 * a;
+    bj = t - a * (a + 1);
+  }
+}
+
+// Preconditioning epilogue of one 32 x 32 piece: kf to the weight and bias
+// parts, and the momentum update where the layer has it fused.
+__device__ __forceinline__ void tile_precond(const GemmDesc& g,
+                                             const float* piece, int gr0,
+                                             int rows, int gc0, int cols,
+                                             int lane, float lr,
+                                             float momentum) {
+  const int dW = g.dW;
+  const bool fused = g.pW != nullptr;
+  if ((dW & 3) == 0 && gc0 + 31 < dW && cols >= 32 &&
+      ((reinterpret_cast<uintptr_t>(g.kfW) | reinterpret_cast<uintptr_t>(g.pW) |
+        reinterpret_cast<uintptr_t>(g.vW)) & 15) == 0) {
+    const int sub = lane >> 3, wc = 4 * (lane & 7);
+    const float* pp = piece + sub * TT_EP + wc;
+    long long idx = (long long)(gr0 + sub) * dW + gc0 + wc;
+#pragma unroll 1
+    for (int i0 = 0; i0 < 8; i0 += 4, idx += 16LL * dW, pp += 16 * TT_EP) {
+      float4 ov[4], op[4];
+      long long at = idx;
+#pragma unroll
+      for (int i = 0; i < 4; ++i, at += 4LL * dW) {
+        if (!fused || 4 * (i0 + i) + sub >= rows) continue;
+        ov[i] = *reinterpret_cast<const float4*>(g.vW + at);
+        op[i] = *reinterpret_cast<const float4*>(g.pW + at);
+      }
+      at = idx;
+#pragma unroll
+      for (int i = 0; i < 4; ++i, at += 4LL * dW) {
+        if (4 * (i0 + i) + sub >= rows) continue;
+        const float4 kf = *reinterpret_cast<const float4*>(&pp[4 * i * TT_EP]);
+        if (g.kfW) *reinterpret_cast<float4*>(g.kfW + at) = kf;
+        if (!fused) continue;
+        float4 nv;
+        nv.x = momentum * ov[i].x - lr * kf.x;
+        nv.y = momentum * ov[i].y - lr * kf.y;
+        nv.z = momentum * ov[i].z - lr * kf.z;
+        nv.w = momentum * ov[i].w - lr * kf.w;
+        *reinterpret_cast<float4*>(g.vW + at) = nv;
+        *reinterpret_cast<float4*>(g.pW + at) =
+            make_float4(op[i].x + nv.x, op[i].y + nv.y, op[i].z + nv.z,
+                        op[i].w + nv.w);
+      }
+    }
+    return;
+  }
+  // a column per lane, eight rows at a time
+  if (lane >= cols) return;
+  const bool w = gc0 + lane < dW;
+  float* okf = w ? g.kfW : g.kfb;
+  float* opar = w ? g.pW : g.pb;
+  float* ovel = w ? g.vW : g.vb;
+  const long long step = w ? dW : 1;
+  long long idx = gr0 * step + (w ? gc0 + lane : 0);
+  for (int r0 = 0; r0 < rows; r0 += 8, idx += 8 * step) {
+    float ov[8], op[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (opar != nullptr && r0 + i < rows) {
+        ov[i] = ovel[idx + i * step];
+        op[i] = opar[idx + i * step];
+      }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (r0 + i >= rows) continue;
+      const float kf = piece[(r0 + i) * TT_EP + lane];
+      if (okf != nullptr) okf[idx + i * step] = kf;
+      if (opar == nullptr) continue;
+      const float nv = momentum * ov[i] - lr * kf;
+      ovel[idx + i * step] = nv;
+      opar[idx + i * step] = op[i] + nv;
+    }
+  }
+}
+
+// PRE: the preconditioning epilogue (every problem of the launch has it).  VEC:
+// all operands of the launch have rows of 16-byte words (one kernel with both
+// ways of loading spills).
+template <int TN, bool PRE, bool VEC>
+__global__ void __launch_bounds__(TileMap<TN>::kThreads, 1)
+tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
+               const __grid_constant__ TileInline inl, float lr,
+               float momentum) {
+  using Map = TileMap<TN>;
+  extern __shared__ unsigned char tt_smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(tt_smem_raw) + 1023) & ~(uintptr_t)1023);
+  TileControl* ctl =
+      reinterpret_cast<TileControl*>(smem + Map::kStages * Map::kStage);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tile = tile0 + blockIdx.x;
+
+  if (warp == Map::kWarps) {
+    if (lane == 0) {
+#pragma unroll
+      for (int s = 0; s < Map::kStages; ++s) {
+        mbar_init(&ctl->full[s], Map::kWarps);
+        mbar_init(&ctl->empty[s], 1);
+      }
+      mbar_init(&ctl->accum, 1);
+      ctl->abort_flag = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    asm volatile(
+        "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+        ::"r"(smem_u32(&ctl->tmem_base)), "r"(Map::kTmem)
+        : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
+                 ::: "memory");
+  } else {
+    // the problem this tile belongs to (tile_begin is ascending): bisection
+    // by every warp, then a copy of the descriptor
+    constexpr int kWords = (int)(sizeof(GemmDesc) / sizeof(int));
+    int* dst = reinterpret_cast<int*>(&ctl->desc);
+    if (inl.n > 0) {
+      int f = 0;
+#pragma unroll
+      for (int i = 1; i < TT_INLINE; ++i)
+        if (i < inl.n && inl.d[i].tile_begin <= tile) f = i;
+      const int* src = reinterpret_cast<const int*>(&inl.d[f]);
+      for (int i = tid; i < kWords; i += Map::kProducers) dst[i] = src[i];
+    } else {
+      // one round of parallel loads instead of a chain of dependent ones
+      int f = 0;
+      for (int i = lane; i < ndesc; i += 32)
+        if (descs[i].tile_begin <= tile) f = i;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        f = max(f, __shfl_xor_sync(0xffffffffu, f, o));
+      const int* src = reinterpret_cast<const int*>(descs + f);
+      for (int i = tid; i < kWords; i += Map::kProducers) dst[i] = src[i];
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+  const GemmDesc& g = ctl->desc;
+  const unsigned tmem = ctl->tmem_base;
+  const int flags = g.flags;
+  const int lt = tile - g.tile_begin;
+  int bi, bj;
+  if (flags & G_LOWER) {
+    tile_lower<TN>(lt, bi, bj);
+  } else {
+    bi = lt / g.tiles_n;
+    bj = lt - bi * g.tiles_n;
+  }
+  const int m0 = bi * TC_BM, n0 = bj * TN;
+  int n_valid = min(TN, g.N - n0);
+  if (flags & G_LOWER) n_valid = min(n_valid, m0 + TC_BM - n0);
+  const int n_inst = (n_valid + 15) & ~15;
+  const int m_valid = min(TC_BM, g.M - m0);
+  int kbeg = 0, kend = (int)g.K;
+  if (flags & G_KBEG_N0) kbeg = max(kbeg, n0);
+  if (flags & G_KBEG_M0) kbeg = max(kbeg, m0 - g.kbeg_off);
+  if (flags & G_KEND_M0) kend = min(kend, m0 + TC_BM);
+  // a gated-off problem runs no k-blocks and stores nothing
+  const bool gated_off = g.gate != nullptr && *g.gate == 0;
+  const int nkb =
+      (kend > kbeg && !gated_off) ? (kend - kbeg + TT_BK - 1) / TT_BK : 0;
+  // X^T X on a diagonal tile: the tile's A rows are rows [m0 - n0, + 128) of
+  // its B rows, so only B is staged and the A descriptors point into it
+  const bool share_ab = (flags & G_SAME_AB) && (flags & G_LOWER) &&
+                        m0 >= n0 && m0 - n0 + TC_BM <= TN;
+
+  if (warp < Map::kWarps) {
+    // ===================== producers =====================
+    // units 0 .. 7 of 32 threads: A rows, then the B rows; two per thread
+    const bool a0 = warp < 8;
+    const Operand& op0 = a0 ? g.A : g.B;
+    const Operand& op1 = g.B;
+    TileUnit u0, u1;
+    tile_unit_setup<VEC>(op0, a0 ? m0 : n0, a0 ? warp : warp - 8, lane, kbeg,
+                    a0 ? (share_ab ? 0 : m_valid) : n_valid,
+                    a0 ? 0 : Map::kABytes, u0);
+    tile_unit_setup<VEC>(op1, n0, warp + Map::kWarps - 8, lane, kbeg, n_valid,
+                    Map::kABytes, u1);
+    const unsigned base = smem_u32(smem);
+    auto load = [&](float4* v) {
+      tile_unit_load<VEC>(op0, u0, kend, v);
+      tile_unit_load<VEC>(op1, u1, kend, v + 4);
+    };
+    auto store = [&](int kb, const float4* v) {
+      const int s = kb % Map::kStages;
+      if (kb >= Map::kStages &&
+          !mbar_wait_status(&ctl->empty[s], ((kb / Map::kStages) - 1) & 1,
+                            &ctl->abort_flag, &g_tile_status))
+        return false;
+      const unsigned st = base + s * Map::kStage;
+      tile_unit_store<VEC>(u0, st, Map::kLo, v);
+      tile_unit_store<VEC>(u1, st, Map::kLo, v + 4);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->full[s]);
+      return true;
+    };
+    float4 va[8];
+    if (nkb > 0) load(va);
+    if (TN == 256 || !VEC) {
+      // one block ahead: the MMAs of a block take longer than a trip to L2
+#pragma unroll 1
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!store(kb, va)) break;
+        if (kb + 1 < nkb) load(va);
+      }
+    } else {
+      float4 vb[8];
+      if (nkb > 1) load(vb);
+#pragma unroll 1
+      for (int kb = 0; kb < nkb; kb += 2) {
+        if (!store(kb, va)) break;
+        if (kb + 2 < nkb) load(va);
+        if (kb + 1 < nkb) {
+          if (!store(kb + 1, vb)) break;
+          if (kb + 3 < nkb) load(vb);
+        }
+      }
+    }
+  } else if (elect_one()) {
+    // ===================== MMA issuer =====================
+    const unsigned idesc = tc_instr_desc(n_inst);
+    const unsigned a_off =
+        share_ab ? (unsigned)(Map::kABytes + (m0 - n0) * 128) : 0u;
+    for (int kb = 0; kb < nkb; ++kb) {
+      const int s = kb % Map::kStages;
+      if (!mbar_wait_status(&ctl->full[s], (kb / Map::kStages) & 1,
+                            &ctl->abort_flag, &g_tile_status))
+        break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned sa = smem_u32(smem + s * Map::kStage);
+      const unsigned long long a_hi = tc_smem_desc(sa + a_off);
+      const unsigned long long b_hi = tc_smem_desc(sa + Map::kABytes);
+      const unsigned long long a_lo = tc_smem_desc(sa + Map::kLo + a_off);
+      const unsigned long long b_lo =
+          tc_smem_desc(sa + Map::kLo + Map::kABytes);
+#pragma unroll
+      for (int kk = 0; kk < TT_BK / 8; ++kk) {
+        const unsigned long long adv = (unsigned long long)(kk * 32 >> 4);
+        tc_mma(tmem + TN, a_lo + adv, b_hi + adv, idesc, (kb | kk) != 0);
+        tc_mma(tmem + TN, a_hi + adv, b_lo + adv, idesc, 1);
+        tc_mma(tmem, a_hi + adv, b_hi + adv, idesc, (kb | kk) != 0);
+      }
+      tc_commit(&ctl->empty[s]);
+    }
+    tc_commit(&ctl->accum);
+  }
+
+  // ===================== epilogue =====================
+  // warp w: accumulator rows of quarter q, 32-column pieces h, h + G, ...
+  constexpr int G = Map::kWarps / 4;
+  const int q = warp & 3, h = warp >> 2;
+  if (warp < Map::kWarps && !gated_off) {
+    const int row0 = q * 32, rows = min(32, m_valid - row0);
+    const bool lower = (flags & G_LOWER) != 0;
+    const float alpha = g.alpha;
+    const float beta =
+        (g.beta_until > 0 && m0 >= g.beta_until) ? 0.f : g.beta;
+    float* C = g.C;
+    float* C2 = g.C2;
+    const long long ldc = g.ldc;
+    // rows of a piece as 16-byte words: lane -> row 4 i + lane / 8, word lane % 8
+    const bool vec = (ldc & 3) == 0 &&
+                     (reinterpret_cast<uintptr_t>(C) & 15) == 0 &&
+                     (reinterpret_cast<uintptr_t>(C2) & 15) == 0;
+    const int sub = lane >> 3, wc = 4 * (lane & 7);
+    float4 old[8];
+    auto prefetch = [&](int c0) {
+      if constexpr (PRE) return;
+      if (beta == 0.f || c0 >= n_valid) return;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = row0 + 4 * i + sub, c = c0 + wc;
+        old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r >= m_valid || c >= n_valid) continue;
+        const float* p = C + (long long)(m0 + r) * ldc + n0 + c;
+        if (vec && c + 3 < n_valid) {
+          old[i] = *reinterpret_cast<const float4*>(p);
+        } else {
+          old[i].x = p[0];
+          if (c + 1 < n_valid) old[i].y = p[1];
+          if (c + 2 < n_valid) old[i].z = p[2];
+          if (c + 3 < n_valid) old[i].w = p[3];
+        }
+      }
+    };
+    prefetch(32 * h);
+    bool ok = true;
+    if (nkb > 0) {
+      ok = mbar_wait_status(&ctl->accum, 0, &ctl->abort_flag, &g_tile_status);
+      ok = __all_sync(0xffffffffu, ok);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    // every warp has its own piece of the (drained) first stage
+    float* piece = reinterpret_cast<float*>(smem) + warp * 32 * TT_EP;
+    for (int c0 = 32 * h; c0 < n_valid && ok; c0 += 32 * G) {
+      tile_acc_piece<TN>(tmem, q, c0, alpha, nkb == 0, piece, lane);
+      __syncwarp();
+      if (PRE) {
+        if (rows > 0)
+          tile_precond(g, piece, m0 + row0, rows, n0 + c0, n_valid - c0, lane,
+                       lr, momentum);
+      } else if (rows > 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = row0 + 4 * i + sub, c = c0 + wc;
+          const int gr = m0 + r;
+          const int cend = lower ? min(n_valid, gr - n0 + 1) : n_valid;
+          float4 x =
+              *reinterpret_cast<const float4*>(&piece[(4 * i + sub) * TT_EP + wc]);
+          if (beta != 0.f) {
+            x.x += beta * old[i].x; x.y += beta * old[i].y;
+            x.z += beta * old[i].z; x.w += beta * old[i].w;
+            if (flags & G_MIRROR)
+              *reinterpret_cast<float4*>(&piece[(4 * i + sub) * TT_EP + wc]) = x;
+          }
+          if (r >= m_valid || c >= cend) continue;
+          const long long idx = (long long)gr * ldc + n0 + c;
+          if (vec && c + 3 < cend) {
+            *reinterpret_cast<float4*>(C + idx) = x;
+            if (C2 != nullptr) *reinterpret_cast<float4*>(C2 + idx) = x;
+          } else {
+            const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (c + e < cend) {
+                C[idx + e] = xs[e];
+                if (C2 != nullptr) C2[idx + e] = xs[e];
+              }
+          }
+        }
+        // C of the next piece while this one is mirrored
+        prefetch(c0 + 32 * G);
+        if (flags & G_MIRROR) {
+          // the final values are in the piece; a row per lane, so that a
+          // column of the piece is a contiguous store
+          __syncwarp();
+          const int gr = m0 + row0 + lane;
+          if (lane < rows) {
+            float* dst = C + (long long)(n0 + c0) * ldc + gr;
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const float4 x =
+                  *reinterpret_cast<const float4*>(&piece[lane * TT_EP + i]);
+              const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e, dst += ldc)
+                if (c0 + i + e < n_valid && n0 + c0 + i + e < gr) *dst = xs[e];
+            }
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == Map::kWarps) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+                 ::"r"(tmem), "r"(Map::kTmem)
+                 : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ host side
+typedef void (*TileKernel)(const GemmDesc*, int, int, const TileInline, float,
+                           float);
+
+struct TileVariant {
+  TileKernel kernel;
+  int threads, smem;
+};
+
+template <int TN, bool PRE, bool VEC>
+static TileVariant tile_variant() {
+  return {tc_tile_kernel<TN, PRE, VEC>, TileMap<TN>::kThreads,
+          TileMap<TN>::kSmem};
+}
+
+// [128 columns][precondition][16-byte rows]
+static const TileVariant kTileVariants[2][2][2] = {
+    {{tile_variant<256, false, false>(), tile_variant<256, false, true>()},
+     {tile_variant<256, true, false>(), tile_variant<256, true, true>()}},
+    {{tile_variant<128, false, false>(), tile_variant<128, false, true>()},
+     {tile_variant<128, true, false>(), tile_variant<128, true, true>()}}};
+
+int tc_prepare_tiles() {
+  static std::mutex mu;
+  static bool done[64] = {false};
+  int dev = 0;
+  KFAC_CUDA(cudaGetDevice(&dev));
+  KFAC_REQUIRE(dev >= 0 && dev < 64, "device index %d unsupported", dev);
+  std::lock_guard<std::mutex> lock(mu);
+  if (!done[dev]) {
+    for (int k = 0; k < 8; ++k) {
+      const TileVariant& v = kTileVariants[k >> 2][(k >> 1) & 1][k & 1];
+      KFAC_CUDA(cudaFuncSetAttribute(
+          v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+    }
+    done[dev] = true;
+  }
+  return KFAC_OK;
+}
+
+static int tile_count(const GemmDesc& g, int tn) {
+  const int tm = (g.M + TC_BM - 1) / TC_BM, nn = (g.N + tn - 1) / tn;
+  if (!(g.flags & G_LOWER)) return tm * nn;
+  if (tn == TC_BM) return tm * (tm + 1) / 2;
+  const int a = tm / 2;
+  return (tm & 1) ? (a + 1) * (a + 1) : a * (a + 1);
+}
+
+static bool tile_desc_vec(const GemmDesc& g) {
+  return tile_operand_vec(g.A) && tile_operand_vec(g.B);
+}
+
+int tc_number_tiles(GemmDesc* descs, int n, int* tile_cols) {
+  std::stable_partition(descs, descs + n, tile_desc_vec);
+  // Narrow tiles (half the work per CTA, but the A rows are loaded, split and
+  // read by the MMAs twice as often) where they leave a quarter of the SMs to
+  // the launches of other streams.  Measured with the line at 20, 74, 111 and
+  // 148 of 148 SMs: a 2304-row inverse 835, 791, 791, 791 us; a 4608-row one
+  // 1954, 1934, 1915, 1902; 108 factors of ResNet-50 in three concurrent plans
+  // 6.10, 6.22, 6.27, 6.33 ms.
+  long long narrow = 0;
+  for (int i = 0; i < n; ++i) narrow += tile_count(descs[i], 128);
+  const int tn = 4 * narrow <= 3LL * sm_count() ? 128 : 256;
+  int total = 0;
+  for (int i = 0; i < n; ++i) {
+    descs[i].tile_begin = total;
+    descs[i].tiles_m = (descs[i].M + TC_BM - 1) / TC_BM;
+    descs[i].tiles_n = (descs[i].N + tn - 1) / tn;
+    total += tile_count(descs[i], tn);
+  }
+  *tile_cols = tn;
+  return total;
+}
+
+int launch_tc_grouped(const GemmDesc* descs_dev, const GemmDesc* descs_host,
+                      int ndesc, int total_tiles, int tile_cols, bool precond,
+                      float lr, float momentum, cudaStream_t stream) {
+  if (ndesc <= 0 || total_tiles <= 0) return KFAC_OK;
+  const int rc = tc_prepare_tiles();
+  if (rc != KFAC_OK) return rc;
+  // the problems with 16-byte rows come first (tc_number_tiles); where all
+  // tiles fit the chip at once one launch of the general kernel ends sooner
+  // than two in a row
+  int n_vec = 0;
+  while (n_vec < ndesc && tile_desc_vec(descs_host[n_vec])) ++n_vec;
+  if (n_vec < ndesc && total_tiles <= sm_count()) n_vec = 0;
+  for (int k = 0; k < 2; ++k) {
+    const int first = k == 0 ? 0 : n_vec, n = k == 0 ? n_vec : ndesc - n_vec;
+    if (n == 0) continue;
+    const int tile0 = descs_host[first].tile_begin;
+    const int end =
+        first + n < ndesc ? descs_host[first + n].tile_begin : total_tiles;
+    TileInline inl;
+    inl.n = 0;
+    if (n <= TT_INLINE) {
+      inl.n = n;
+      std::copy(descs_host + first, descs_host + first + n, inl.d);
+    }
+    const TileVariant& v = kTileVariants[tile_cols == 128][precond][k == 0];
+    v.kernel<<<end - tile0, v.threads, v.smem, stream>>>(
+        descs_dev + first, n, tile0, inl, lr, momentum);
+    KFAC_LAUNCH_CHECK("tc_tile_kernel");
+  }
+  return KFAC_OK;
+}
+
+int tile_status_read(int* out) {
+  KFAC_CUDA(cudaMemcpyFromSymbol(out, g_tile_status, sizeof(int)));
+  return KFAC_OK;
+}
+
+}  // namespace kfac

@@ -514,6 +514,38 @@ def precond_case(rng, dG, dW, bias):
     return Gi, Ai, gW, gb
 
 
+@pytest.mark.parametrize('shapes', [
+    [(128, 256, False), (64, 60, False)],            # 16-byte rows, few tiles
+    [(33, 31, True), (129, 257, False), (5, 3, True)],   # none of them
+    [(1024, 1152, False), (512, 1000, True), (260, 2048, False),
+     (301, 785, True)],          # both, more tiles than SMs: two launches
+])
+def test_precondition_tile_variants(ops, shapes):
+    """Narrow and wide tiles, operands read as 16-byte words and float by
+    float, cut rows, columns and contractions, the appended bias column."""
+    rng = np.random.default_rng(31)
+    cases = [precond_case(rng, *s) for s in shapes]
+    Gi, Ai, gW = ([dev(c[k]) for c in cases] for k in range(3))
+    gb = [None if c[3] is None else dev(c[3]) for c in cases]
+    kW = [torch.empty_like(t) for t in gW]
+    kb = [None if t is None else torch.empty_like(t) for t in gb]
+    ops.precondition(Gi, Ai, gW, gb, kW, kb)
+    for c, w, b in zip(cases, kW, kb):
+        g = c[2].astype(np.float64)
+        if c[3] is not None:
+            g = np.concatenate([g, c[3].astype(np.float64)[:, None]], 1)
+        ref = c[0].astype(np.float64) @ g @ c[1].astype(np.float64)
+        got = host(w) if b is None else np.concatenate(
+            [host(w), host(b)[:, None]], 1)
+        assert rel(got, ref) < 2e-5     # TF32 pairs and fp32 sums: < 1e-5
+
+
+@pytest.mark.parametrize('d', [1, 31, 127, 129, 257, 385, 513, 770, 1025])
+def test_inverse_around_block_sizes(ops, d):
+    """Sides around the diagonal block, the panel and the row pitch."""
+    run_pairs(ops, [d], [max(1, d // 3)], 1e-3, seed=d)
+
+
 def test_precondition_matches_oracle(ops):
     rng = np.random.default_rng(11)
     shapes = [(10, 1000, True), (64, 147, True), (300, 129, False),
