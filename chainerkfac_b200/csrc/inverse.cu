@@ -12,6 +12,7 @@
 // all matrices that are still active.
 #include <vector>
 #include <algorithm>
+#include <mutex>
 
 #include "gemm_simt.cuh"
 #include "tc_common.cuh"
@@ -1119,10 +1120,9 @@ struct kfac_inverse_plan {
   RunParams* params_dev;
   std::vector<cudaEvent_t> events;   // edges between the streams
   cudaEvent_t fork_ev, join_ev[S_COUNT];
-  cudaStream_t side_stream[S_COUNT]; // streams of plain runs (from S_BULK on)
-  cudaStream_t cap_side[S_COUNT];    // the same during capture
+  cudaStream_t side_stream[S_COUNT]; // streams of plain runs (from S_BULK on),
+                                     // made by the first of them
   bool look;
-  cudaStream_t cap_stream;
   cudaGraphExec_t graph_exec;
   int* graph_info;
   float* graph_diag;
@@ -1545,9 +1545,8 @@ extern "C" int kfac_inverse_plan_create(
   p->params_dev = nullptr;
   p->fork_ev = nullptr;
   for (int k = 1; k < S_COUNT; ++k)
-    p->join_ev[k] = nullptr, p->side_stream[k] = p->cap_side[k] = nullptr;
+    p->join_ev[k] = nullptr, p->side_stream[k] = nullptr;
   p->look = look;
-  p->cap_stream = nullptr;
   p->graph_exec = nullptr;
   p->graph_info = nullptr;
   p->graph_diag = nullptr;
@@ -1558,20 +1557,6 @@ extern "C" int kfac_inverse_plan_create(
   }
   cudaError_t e = cudaGetDevice(&p->device);
   if (e == cudaSuccess) e = cudaMalloc(&p->params_dev, sizeof(RunParams));
-  // the chain is latency-bound and uses few SMs: it gets the higher
-  // priority, the side stream's tiles fill the rest
-  int prio_lo = 0, prio_hi = 0;
-  if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
-  if (e == cudaSuccess)
-    e = cudaStreamCreateWithPriority(&p->cap_stream, cudaStreamNonBlocking,
-                                     prio_hi);
-  for (int k = 1; k < S_COUNT && e == cudaSuccess; ++k) {
-    e = cudaStreamCreateWithPriority(&p->cap_side[k], cudaStreamNonBlocking,
-                                     prio_lo);
-    if (e == cudaSuccess)
-      e = cudaStreamCreateWithPriority(&p->side_stream[k],
-                                       cudaStreamNonBlocking, prio_lo);
-  }
   if (e == cudaSuccess)
     e = cudaEventCreateWithFlags(&p->fork_ev, cudaEventDisableTiming);
   for (int k = 1; k < S_COUNT && e == cudaSuccess; ++k)
@@ -1739,20 +1724,49 @@ static void plan_drop_graph(kfac_inverse_plan* p) {
   p->graph_exec = nullptr;
 }
 
-// Capture one run into a graph (on the plan's own stream: nothing executes
-// during capture).  On any failure the plan falls back to plain launches.
+// Side streams of a run, behind its chain.
+static cudaError_t make_side_streams(cudaStream_t* side) {
+  int lo = 0, hi = 0;
+  cudaError_t e = cudaDeviceGetStreamPriorityRange(&lo, &hi);
+  for (int k = 1; k < S_COUNT && e == cudaSuccess; ++k)
+    if (side[k] == nullptr)
+      e = cudaStreamCreateWithPriority(&side[k], cudaStreamNonBlocking, lo);
+  return e;
+}
+
+// Streams that plans are captured on, one set per device: nothing executes
+// during a capture, the graph only keeps their priorities.
+struct CaptureStreams {
+  std::mutex mu;                     // held from the first launch to the last
+  cudaStream_t chain = nullptr;
+  cudaStream_t side[S_COUNT] = {};
+};
+
+// Capture one run into a graph.  On any failure the plan falls back to plain
+// launches.
 static void plan_capture(kfac_inverse_plan* p, int* info, float* diag_dev) {
+  static CaptureStreams sets[64];
   plan_drop_graph(p);
+  CaptureStreams& c = sets[p->device & 63];
+  std::lock_guard<std::mutex> lock(c.mu);
+  // the chain is latency-bound and uses few SMs: it gets the higher
+  // priority, the side streams' tiles fill the rest
+  int lo = 0, hi = 0;
+  cudaError_t made = cudaDeviceGetStreamPriorityRange(&lo, &hi);
+  if (made == cudaSuccess && c.chain == nullptr)
+    made = cudaStreamCreateWithPriority(&c.chain, cudaStreamNonBlocking, hi);
+  if (made == cudaSuccess) made = make_side_streams(c.side);
   const long long before = launch_count_now();
-  if (cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeRelaxed) !=
-      cudaSuccess) {
+  if (made != cudaSuccess ||
+      cudaStreamBeginCapture(c.chain, cudaStreamCaptureModeRelaxed) !=
+          cudaSuccess) {
     cudaGetLastError();
     p->graph_ok = false;
     return;
   }
-  const int rc = plan_enqueue(p, info, diag_dev, p->cap_stream, p->cap_side);
+  const int rc = plan_enqueue(p, info, diag_dev, c.chain, c.side);
   cudaGraph_t graph = nullptr;
-  cudaError_t e = cudaStreamEndCapture(p->cap_stream, &graph);
+  cudaError_t e = cudaStreamEndCapture(c.chain, &graph);
   const long long captured = launch_count_now() - before;
   count_launches(-captured);          // nothing ran yet
   if (rc == KFAC_OK && e == cudaSuccess && graph != nullptr)
@@ -1797,6 +1811,7 @@ extern "C" int kfac_inverse_plan_run(kfac_inverse_plan* p, float damping,
       }
     }
   }
+  KFAC_CUDA(make_side_streams(p->side_stream));
   return plan_enqueue(p, info, diag_dev, st, p->side_stream);
 }
 
@@ -1860,9 +1875,7 @@ extern "C" int kfac_inverse_plan_set_second_floor(kfac_inverse_plan* p,
 extern "C" int kfac_inverse_plan_destroy(kfac_inverse_plan* p) {
   if (p == nullptr) return KFAC_OK;
   plan_drop_graph(p);
-  if (p->cap_stream != nullptr) cudaStreamDestroy(p->cap_stream);
   for (int k = 1; k < S_COUNT; ++k) {
-    if (p->cap_side[k] != nullptr) cudaStreamDestroy(p->cap_side[k]);
     if (p->side_stream[k] != nullptr) cudaStreamDestroy(p->side_stream[k]);
     if (p->join_ev[k] != nullptr) cudaEventDestroy(p->join_ev[k]);
   }
