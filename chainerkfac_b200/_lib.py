@@ -74,6 +74,8 @@ SIGNATURES = {
     'kfac_factor_conv_grad': (I, [VP, I, I, I, I, F, F, VP, VP, SZ, VP]),
     'kfac_factor_group_workspace_bytes': (SZ, [I, ctypes.POINTER(FactorItem)]),
     'kfac_factor_group': (I, [I, ctypes.POINTER(FactorItem), VP, SZ, VP]),
+    'kfac_factor_group_second': (I, [I, ctypes.POINTER(FactorItem), c_void_pp,
+                                     F, F, VP, SZ, VP]),
     'kfac_bn_sample_grads': (I, [VP, VP, I, I, I, F, F, VP, VP, VP]),
     'kfac_bn_sample_grads_group': (I, [I, ctypes.POINTER(BnItem), VP]),
     'kfac_bn_precondition_group': (I, [I, c_int_p] + [c_void_pp] * 10 +
@@ -112,6 +114,8 @@ SIGNATURES = {
     'kfac_wire_unpack_sum_as': (I, [I, I, c_void_pp, c_i64_p, c_int_p,
                                     c_int_p, F, F, c_void_pp, I, VP]),
 }
+
+ERR_WORKSPACE = 3        # KFAC_ERR_WORKSPACE
 
 _lib = None
 

@@ -1256,6 +1256,8 @@ static int job_from_item(const kfac_factor_item& it, FactorJob& job) {
   job.n = it.n;
   job.nhwc = 0;
   job.grouped = 1;
+  job.out2 = nullptr;
+  job.a2 = job.b2 = 0.f;
   KFAC_REQUIRE(it.layout == 0 ||
                    (it.layout == 1 && it.kind == KFAC_FACTOR_CONV_INPUT),
                "factor_group: layout %d of item kind %d unsupported", it.layout,
@@ -1335,20 +1337,41 @@ extern "C" size_t kfac_factor_group_workspace_bytes(
 extern "C" int kfac_factor_group(int count, const kfac_factor_item* items,
                                  void* workspace, size_t workspace_bytes,
                                  void* stream) {
+  return kfac_factor_group_second(count, items, nullptr, 0.f, 0.f, workspace,
+                                  workspace_bytes, stream);
+}
+
+extern "C" int kfac_factor_group_second(int count,
+                                        const kfac_factor_item* items,
+                                        float* const* second, float a2,
+                                        float b2, void* workspace,
+                                        size_t workspace_bytes, void* stream) {
   KFAC_REQUIRE(count > 0 && items != nullptr, "factor_group: no items");
   std::vector<FactorJob> jobs(count);
   for (int i = 0; i < count; ++i) {
     int rc = job_from_item(items[i], jobs[i]);
     if (rc != KFAC_OK) return rc;
+    if (second != nullptr) {
+      jobs[i].out2 = second[i];
+      jobs[i].a2 = a2;
+      jobs[i].b2 = b2;
+    }
   }
   if (engine() == 1)
     return run_factor_group_tc(count, jobs.data(), workspace, workspace_bytes,
                                (cudaStream_t)stream);
+  size_t need = 0;
+  for (int i = 0; i < count; ++i)
+    need = std::max(need, simt_item_bytes(jobs[i]));
+  if (need > 0 && (workspace == nullptr || workspace_bytes < need))
+    return fail(KFAC_ERR_WORKSPACE,
+                "factor: workspace of %zu bytes needed, %zu given", need,
+                workspace_bytes);
   for (int i = 0; i < count; ++i) {   // fp32 engine: one factor after another
     int rc = run_factor(jobs[i].X, jobs[i].rows, jobs[i].d, jobs[i].alpha,
                         jobs[i].beta, jobs[i].out, workspace, workspace_bytes,
                         (cudaStream_t)stream);
     if (rc != KFAC_OK) return rc;
   }
-  return KFAC_OK;
+  return run_second_outputs(count, jobs.data(), (cudaStream_t)stream);
 }

@@ -306,6 +306,8 @@ struct FactorJob {      // one factor of a grouped build
   int grouped;          // part of a grouped build (not a factor on its own)
   float alpha, beta;
   float* out;
+  float* out2;          // if set: out2 = a2 * (new out) + b2 * out2
+  float a2, b2;
 };
 size_t tc_factor_group_workspace_bytes(int count, const FactorJob* jobs,
                                        bool staged = true);
@@ -321,6 +323,7 @@ size_t gram_workspace_bytes(int count, const FactorJob* jobs);
 int run_factor_group_gram(int count, const FactorJob* jobs, void* workspace,
                           size_t workspace_bytes, cudaStream_t stream);
 int gram_status_read(int* out);
+int run_second_outputs(int count, const FactorJob* jobs, cudaStream_t stream);
 int run_factor_group_tc(int count, const FactorJob* jobs, void* workspace,
                         size_t workspace_bytes, cudaStream_t stream,
                         bool staged = true);

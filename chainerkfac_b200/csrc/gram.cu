@@ -923,6 +923,8 @@ stage_rows_kernel(const StageJob* __restrict__ jobs, int njobs, int items) {
 // -------------------------------------------------------------------- output
 struct GramOut {
   float* out;
+  float* out2;                 // if set: out2 = a2 * (new out) + b2 * out2
+  float a2, b2;
   int d;                       // side of the factor
   int C;                       // channels (shifted products), 0: plain
   int strips;                  // plain: 32 x 128 pieces, else 32 x 32
@@ -970,7 +972,8 @@ __device__ __forceinline__ void reduce_piece(const GramOut& o, int m0, int n0,
                                              float (*t)[132]) {
   const int d = o.d, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ti = m0 >> 8, tj = n0 >> 8;
-  const float alpha = o.alpha, beta = o.beta;
+  const float alpha = o.alpha, beta = o.beta, a2 = o.a2, b2 = o.b2;
+  float* out2 = o.out2;
   float old[4][W];
   if (beta != 0.f) {
 #pragma unroll
@@ -1026,6 +1029,34 @@ __device__ __forceinline__ void reduce_piece(const GramOut& o, int m0, int n0,
   for (int i = 0; i < 4 * W; ++i) {
     const int r = m0 + lane, c = n0 + warp + 8 * i;
     if (r < d && c < r) o.out[(long long)c * d + r] = t[lane][warp + 8 * i];
+  }
+  if (out2 == nullptr) return;
+  // the second output, through the same tile
+  float next[4][W];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const int r = m0 + warp + 8 * i, c = n0 + lane + 32 * k;
+      if (r < d && c <= r) {
+        float* p = out2 + (long long)r * d + c;
+        float v = a2 * t[warp + 8 * i][lane + 32 * k];
+        if (b2 != 0.f) v += b2 * *p;
+        *p = v;
+        next[i][k] = v;
+      }
+    }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+      t[warp + 8 * i][lane + 32 * k] = next[i][k];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4 * W; ++i) {
+    const int r = m0 + lane, c = n0 + warp + 8 * i;
+    if (r < d && c < r) out2[(long long)c * d + r] = t[lane][warp + 8 * i];
   }
 }
 
@@ -1094,7 +1125,7 @@ __device__ __forceinline__ long long gram_at(int ga, int gb, int tb, int row,
 
 constexpr int kXThreads = 4 * 9 * kXc;    // 9 kXc columns, 4 sets of row taps
 
-__global__ void __launch_bounds__(kXThreads, 5)
+__global__ void __launch_bounds__(kXThreads, 4)
 gram_expand_kernel(const GramOut* __restrict__ outs, int nouts) {
   extern __shared__ float xs[];        // [block][kXc][kXc + 1]
   __shared__ int s_begin[kStageJobs];
@@ -1160,7 +1191,8 @@ gram_expand_kernel(const GramOut* __restrict__ outs, int nouts) {
   __syncthreads();
   // A thread owns one column (channel, tap) and walks the row taps: the blocks
   // a pair of taps needs are looked up once for all row channels.
-  const float alpha = o.alpha, beta = o.beta;
+  const float alpha = o.alpha, beta = o.beta, a2 = o.a2, b2 = o.b2;
+  const bool two = o.out2 != nullptr;
   const int col = threadIdx.x % (9 * kXc), set = threadIdx.x / (9 * kXc);
   const int cc = col / 9, ct = col - 9 * cc;
   for (int pass = 0; pass < (bi == bj ? 1 : 2); ++pass) {
@@ -1186,10 +1218,16 @@ gram_expand_kernel(const GramOut* __restrict__ outs, int nouts) {
       const int at0 = rows_first ? cc : cc * (kXc + 1);
       float* p = o.out + (long long)(9 * ra + rt) * d + 9 * ca + col;
       const long long step = 9LL * d;
-      float old[kXc];
+      float* second = o.out2 + (p - o.out);
+      float old[kXc], old2[kXc];
 #pragma unroll
       for (int rc = 0; rc < kXc; ++rc)
         old[rc] = beta != 0.f && rc < nr ? __ldcg(p + rc * step) : 0.f;
+      if (two) {
+#pragma unroll
+        for (int rc = 0; rc < kXc; ++rc)
+          old2[rc] = b2 != 0.f && rc < nr ? __ldcg(second + rc * step) : 0.f;
+      }
 #pragma unroll
       for (int rc = 0; rc < kXc; ++rc) {
         int at = at0 + rc * sr;
@@ -1199,7 +1237,9 @@ gram_expand_kernel(const GramOut* __restrict__ outs, int nouts) {
         if (e2) v -= p2[at];
         if (e3) v += p3[at];
         v = fmaf(beta, old[rc], alpha * v);
-        if (rc < nr) p[rc * step] = v;
+        if (rc >= nr) continue;
+        p[rc * step] = v;
+        if (two) second[rc * step] = fmaf(b2, old2[rc], a2 * v);
       }
     }
   }
@@ -1372,9 +1412,7 @@ size_t batch_end(const std::vector<JobPlan>& plans, size_t b) {
 
 }  // namespace
 
-size_t gram_workspace_bytes(int count, const FactorJob* jobs) {
-  std::vector<JobPlan> plans(count);
-  for (int i = 0; i < count; ++i) plan_job(jobs[i], plans[i]);
+static size_t plans_bytes(std::vector<JobPlan>& plans) {
   size_t most = 0;
   for (size_t b = 0, e; b < plans.size(); b = e) {
     e = batch_end(plans, b);
@@ -1387,6 +1425,12 @@ size_t gram_workspace_bytes(int count, const FactorJob* jobs) {
     most = std::max(most, bytes);
   }
   return most;
+}
+
+size_t gram_workspace_bytes(int count, const FactorJob* jobs) {
+  std::vector<JobPlan> plans(count);
+  for (int i = 0; i < count; ++i) plan_job(jobs[i], plans[i]);
+  return plans_bytes(plans);
 }
 
 static int gram_prepare() {
@@ -1477,6 +1521,9 @@ static int gram_batch(const FactorJob* jobs, std::vector<JobPlan>& plans,
       direct[km ? 1 : 0].push_back(g);
       GramOut o = {};
       o.out = job.out;
+      o.out2 = job.out2;
+      o.a2 = job.a2;
+      o.b2 = job.b2;
       o.d = job.d;
       o.alpha = job.alpha;
       o.beta = job.beta;
@@ -1541,6 +1588,9 @@ static int gram_batch(const FactorJob* jobs, std::vector<JobPlan>& plans,
 
     GramOut o = {};
     o.out = job.out;
+    o.out2 = job.out2;
+    o.a2 = job.a2;
+    o.b2 = job.b2;
     o.d = job.d;
     o.C = p.grid ? X.C : 0;
     o.alpha = job.alpha;
@@ -1682,7 +1732,7 @@ int run_factor_group_gram(int count, const FactorJob* jobs, void* workspace,
   if (rc != KFAC_OK) return rc;
   std::vector<JobPlan> plans(count);
   for (int i = 0; i < count; ++i) plan_job(jobs[i], plans[i]);
-  const size_t need = gram_workspace_bytes(count, jobs);
+  const size_t need = plans_bytes(plans);
   if (workspace == nullptr || workspace_bytes < need)
     return fail(KFAC_ERR_WORKSPACE,
                 "factor: workspace of %zu bytes needed, %zu given", need,

@@ -1339,14 +1339,46 @@ int run_factor_group_tc(int count, const FactorJob* jobs, void* workspace,
   }
   std::vector<FactorJob> gram, pair;
   tc_by_feed(count, jobs, staged, gram, pair);
+  // (nothing is queued by a call that fails for want of workspace)
+  const size_t need =
+      tc_pair_workspace_bytes((int)pair.size(), pair.data(), staged);
+  if (need > 0 && (workspace == nullptr || workspace_bytes < need))
+    return fail(KFAC_ERR_WORKSPACE,
+                "factor: workspace of %zu bytes needed, %zu given", need,
+                workspace_bytes);
   if (!gram.empty()) {
     const int rc = run_factor_group_gram((int)gram.size(), gram.data(),
                                          workspace, workspace_bytes, stream);
     if (rc != KFAC_OK) return rc;
   }
   if (pair.empty()) return KFAC_OK;
-  return run_factor_group_pair((int)pair.size(), pair.data(), workspace,
-                               workspace_bytes, stream, staged);
+  const int rc = run_factor_group_pair((int)pair.size(), pair.data(), workspace,
+                                       workspace_bytes, stream, staged);
+  if (rc != KFAC_OK) return rc;
+  return run_second_outputs((int)pair.size(), pair.data(), stream);
+}
+
+// Second outputs of factors whose kernels do not write them.
+int run_second_outputs(int count, const FactorJob* jobs, cudaStream_t stream) {
+  std::vector<const float*> x;
+  std::vector<float*> out;
+  std::vector<int64_t> n;
+  float a2 = 0.f, b2 = 0.f;
+  for (int i = 0; i < count; ++i) {
+    if (jobs[i].out2 == nullptr) continue;
+    x.push_back(jobs[i].out);
+    out.push_back(jobs[i].out2);
+    n.push_back((int64_t)jobs[i].d * jobs[i].d);
+    a2 = jobs[i].a2;
+    b2 = jobs[i].b2;
+  }
+  for (size_t k = 0; k < x.size(); k += 1024) {
+    const int part = (int)std::min<size_t>(1024, x.size() - k);
+    const int rc = kfac_axpby_group(part, &n[k], a2, &x[k], b2, &out[k],
+                                    &out[k], (void*)stream);
+    if (rc != KFAC_OK) return rc;
+  }
+  return KFAC_OK;
 }
 
 static FactorJob lone_job(const Operand& X, long long rows, int d, float alpha,
@@ -1358,6 +1390,8 @@ static FactorJob lone_job(const Operand& X, long long rows, int d, float alpha,
   job.n = X.mode == 1 ? (int)(rows / ((long long)X.Ho * X.Wo)) : 0;
   job.nhwc = 0;
   job.grouped = 0;
+  job.out2 = nullptr;
+  job.a2 = job.b2 = 0.f;
   job.alpha = alpha;
   job.beta = beta;
   job.out = out;

@@ -215,14 +215,29 @@ def conv_grad_item(gy, alpha, beta, out):
 _group_ws = Workspace()
 
 
-def factor_group(items, device):
-    """Build all given factors (see *_item) in one grouped call."""
+def factor_group(items, device, second=None, a2=0.0, b2=0.0):
+    """Build all given factors (see *_item) in one grouped call.  With
+    ``second`` (a list of tensors or None, one per item) the call also leaves
+    second[i] = a2 * factor + b2 * second[i]."""
     lib = _lib.load()
     arr = (_lib.FactorItem * len(items))(*items)
-    nbytes = lib.kfac_factor_group_workspace_bytes(len(items), arr)
-    ws = _group_ws.get(nbytes, device)
-    _lib.check(lib.kfac_factor_group(len(items), arr, _p(ws), ws.numel(),
-                                     _stream()), 'kfac_factor_group')
+    ptrs = None
+    if second is not None:
+        for t in second:
+            _chk(t, 'second')
+        ptrs = _lib.ptr_array([None if t is None else t.data_ptr()
+                               for t in second])
+
+    def build(ws):
+        return lib.kfac_factor_group_second(
+            len(items), arr, ptrs, a2, b2, _p(ws), ws.numel(), _stream())
+    # with the workspace that is there; the bytes are only asked for when the
+    # call finds it too small (it checks before it queues anything)
+    rc = build(_group_ws.get(0, device))
+    if rc == _lib.ERR_WORKSPACE:
+        rc = build(_group_ws.get(
+            lib.kfac_factor_group_workspace_bytes(len(items), arr), device))
+    _lib.check(rc, 'kfac_factor_group')
 
 
 def bn_item(x, gy, eps, scale, out=None, stats=None):
@@ -469,6 +484,15 @@ def class_bounds():
         'KFAC_CLASS_BOUNDS', '1024,3000').split(','))
 
 
+class _PlanDiag(object):
+    def __init__(self, plans):
+        self._plans, self._where = plans.plans, plans.where
+
+    def __getitem__(self, i):
+        plan, j = self._where[i]
+        return self._plans[plan].diag[j]
+
+
 class InversePlanSet(object):
     """Several InversePlans over disjoint subsets of (factor, inverse) pairs,
     run on separate CUDA streams.  The long serial chain of diagonal-block
@@ -493,10 +517,12 @@ class InversePlanSet(object):
         for i in range(n):
             groups.setdefault(size_class(i), []).append(i)
         self.plans, self.index, self.class_keys = [], [], []
+        self.where = {}          # factor -> (plan, position in it)
         self.bounds = tuple(bounds)
         for key, idx in sorted(groups.items(), reverse=True):
             self.class_keys.append(key)
             pos = {g: j for j, g in enumerate(idx)}
+            self.where.update((g, (len(self.plans), j)) for g, j in pos.items())
             self.plans.append(InversePlan(
                 [factors[i] for i in idx], [inverses[i] for i in idx],
                 [pos[partner[i]] if partner[i] >= 0 else -1 for i in idx],
@@ -542,10 +568,15 @@ class InversePlanSet(object):
         ``join=False`` the current stream does not wait for the classes on
         side streams: the call returns {class: event} for them and the
         caller orders later work after those events itself."""
+        rest = [c for c in range(len(self.plans)) if c not in self._early]
+        if len(self.plans) == 1 and rest:     # nothing runs beside it
+            self.plans[0].run(damping, use_pi)
+            if after_class is not None:
+                after_class(0)
+            return {}
         cur = torch.cuda.current_stream()
         start = torch.cuda.Event()
         start.record(cur)
-        rest = [c for c in range(len(self.plans)) if c not in self._early]
         for c, st in zip(rest[1:], self.streams):
             st.wait_event(start)
             with torch.cuda.stream(st):
@@ -594,6 +625,11 @@ class InversePlanSet(object):
         for plan, idx in zip(self.plans, self.index):
             out[self._perm[self.plans.index(plan)]] = getattr(plan, attr)
         return out
+
+    @property
+    def diag_items(self):
+        """The values of ``diag`` one by one, gathered when they are read."""
+        return _PlanDiag(self)
 
     @property
     def info(self):

@@ -128,8 +128,16 @@ class FisherBlock(object):
         self._plan.run(self.damping, self._pi_type == PI_TYPE_TRACENORM)
         self.set_diag_vals(self._plan.diag)
 
-    def set_diag_vals(self, diag):
-        raise NotImplementedError
+    # The values added to the diagonals by the last damped inverse are read
+    # when somebody asks for them: ``diag[start + j]`` for factor j.
+    _diag_src = None
+
+    def set_diag_vals(self, diag, start=0):
+        self._diag_src = (diag, start)
+
+    def diag_val(self, j):
+        diag, start = self._diag_src
+        return diag[start + j]
 
     def update_kfgrads(self):
         raise NotImplementedError

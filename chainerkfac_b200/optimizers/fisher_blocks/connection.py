@@ -81,6 +81,7 @@ class FisherBlockConnection(FisherBlock):
                 self._keep_gy = tensor
             return hit[1]
         it = build()
+        it.block, it.which = self, which
         if it.x == tensor.data_ptr():     # read in place, not from a copy
             it._keep = it._keep[-1:]      # the factor buffer only
             memo[which] = (key, it)
@@ -131,9 +132,8 @@ class FisherBlockConnection(FisherBlock):
         l2 = getattr(self.link.W, 'l2_coef', 0.0) or 0.0
         return [(0, l2, 1.0), (1, l2, 1.0)]
 
-    def set_diag_vals(self, diag):
-        self.diag_val_forward = diag[0]
-        self.diag_val_backward = diag[1]
+    diag_val_forward = property(lambda self: self.diag_val(0))
+    diag_val_backward = property(lambda self: self.diag_val(1))
 
     def get_diagvals(self):
         """Vectors added to the diagonals (connection.py:66-77), as views of

@@ -320,7 +320,9 @@ class FisherBlockBatchNormalization(FisherBlock):
         n, c2 = grads.shape
         self._F = self.factor_buffer(c2 // 2, grads.device)
         self.covs = [self._F]
-        return ops.dense_item(grads, False, 1.0 / n, 0.0, self._F)
+        it = ops.dense_item(grads, False, 1.0 / n, 0.0, self._F)
+        it.block, it.which = self, 0
+        return it
 
     def compute_F(self, in_data, out_grad_data):
         # batch_normalization.py:78-131: per-sample gradients of (gamma, beta)
@@ -343,8 +345,7 @@ class FisherBlockBatchNormalization(FisherBlock):
         l2_beta = getattr(self.link.beta, 'l2_coef', 0.0) or 0.0
         return [(2, l2_gamma, float(self.stab_coeff), l2_beta)]
 
-    def set_diag_vals(self, diag):
-        self.diag_val_backward = diag[0]
+    diag_val_backward = property(lambda self: self.diag_val(0))
 
     def get_diagvals(self):
         if self._lr is not None:

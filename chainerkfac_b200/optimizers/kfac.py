@@ -11,6 +11,8 @@ preconditioning launch pair, optionally with the momentum update fused in),
 and hook dispatch is a dictionary lookup instead of a scan.
 """
 
+import weakref
+
 import numpy as np
 import torch
 from torch import nn
@@ -62,7 +64,8 @@ class KFACHook(object):
 
     def __init__(self, fblocks):
         self.fblocks = fblocks
-        self._handles = []
+        self._handles = []       # (block, handle of its module hook)
+        self._active = False
         self._by_array = None
         # optional observers fb -> None, called after the block's own hook
         self.on_forward = None
@@ -98,36 +101,73 @@ class KFACHook(object):
 
     def _make_forward_hook(self, fblock):
         link = fblock.link
+        is_bn = isinstance(link, L.BatchNormalization)
+        ref = weakref.ref(self)    # the modules must not keep an optimizer alive
 
         def hook(module, inputs, output):
-            if not (torch.is_grad_enabled() and output.requires_grad):
+            me = ref()
+            if me is None or not me._active or not output.requires_grad or \
+                    not torch.is_grad_enabled():
                 return
-            if isinstance(link, L.BatchNormalization):
+            x = inputs[0]
+            if x.requires_grad:
+                x = x.detach()
+            if is_bn:
                 if not module.training:
                     return
-                in_data = (inputs[0].detach(), link.gamma.data, link.beta.data)
+                in_data = (x, link.gamma.data, link.beta.data)
+            elif link.b is None:
+                in_data = (x, link.W.data)
             else:
-                in_data = (inputs[0].detach(), link.W.data) + (
-                    () if link.b is None else (link.b.data,))
+                in_data = (x, link.W.data, link.b.data)
             func = fblock.funcclass()
-            self.forward_postprocess(func, in_data)
-            output.register_hook(
-                lambda g: self.backward_preprocess(func, in_data,
-                                                   (g.detach(),)))
+            # the block this hook was made for; an overridden protocol method
+            # is called by its name
+            direct = type(me) is KFACHook
+            if direct:
+                fblock.forward_postprocess(func, in_data)
+                if me.on_forward is not None:
+                    me.on_forward(fblock)
+            else:
+                me.forward_postprocess(func, in_data)
+
+            def backward(g):
+                if g.requires_grad:
+                    g = g.detach()
+                if direct:
+                    fblock.backward_preprocess(func, in_data, (g,))
+                    if me.on_backward is not None:
+                        me.on_backward(fblock)
+                else:
+                    me.backward_preprocess(func, in_data, (g,))
+            output.register_hook(backward)
         return hook
 
+    # The module hooks stay registered between ``with`` blocks (registering
+    # and removing them cost 7 us per layer and step) and do nothing outside.
     def __enter__(self):
-        for fb in self.fblocks:
-            self._handles.append(
-                fb.link.module.register_forward_hook(
-                    self._make_forward_hook(fb)))
+        if [fb for fb, _ in self._handles] != list(self.fblocks):
+            self._remove()
+            self._handles = [
+                (fb, fb.link.module.register_forward_hook(
+                    self._make_forward_hook(fb))) for fb in self.fblocks]
+        self._active = True
         return self
 
     def __exit__(self, *exc):
-        for h in self._handles:
+        self._active = False
+        return False
+
+    def _remove(self):
+        for _, h in self._handles:
             h.remove()
         self._handles = []
-        return False
+
+    def __del__(self):
+        try:
+            self._remove()
+        except Exception:       # interpreter shutdown
+            pass
 
 
 class KFACUpdateRule(_base.UpdateRule):
@@ -176,6 +216,35 @@ class KFACUpdateRule(_base.UpdateRule):
                             self.hyperparam.lr, self.effective_momentum())
 
     update_core_gpu = update_core
+
+
+def build_factors(blocks, device):
+    """Factors of ``blocks`` from their pending hook arguments, and their
+    running averages, which the build itself keeps up to date where a block
+    has one and all its factors are built here."""
+    items = pending_factor_items(blocks)
+    done, r = set(), None
+    if items:
+        built = {}
+        for it in items:
+            built.setdefault(id(it.block), []).append(it)
+        for fb in blocks:
+            mine = built.get(id(fb))
+            if mine is None or fb.low_rank_active or fb.cov_emas is None or \
+                    len(mine) != len(fb.cov_emas):
+                continue
+            decay = fb.cov_ema_decay
+            if decay != 1.0 and (r is None or decay == r):
+                r = decay
+                done.add(id(fb))
+        if done:
+            ops.factor_group(
+                items, device,
+                [it.block.cov_emas[it.which] if id(it.block) in done else None
+                 for it in items], r, 1.0 - r)
+        else:
+            ops.factor_group(items, device)
+    update_cov_emas_grouped([fb for fb in blocks if id(fb) not in done])
 
 
 def update_cov_emas_grouped(blocks):
@@ -295,11 +364,13 @@ class KFAC(_base.GradientMethod):
         # streams (the serial chains of the largest factors outlast
         # everything else): the next forward pass then overlaps them, and
         # every layer waits for its own class right before it is called
-        # (forward pre-hooks installed by setup()).  Off by default: code that
+        # (forward pre-hooks, installed when it is switched on).  Off by
+        # default: code that
         # reads weights other than by calling the layers (checkpoints,
         # parameter statistics) must call join() first.  Single process, one
         # damping group, every update fused into the preconditioning.
-        self.defer_join = False
+        self._pre_hooked = False
+        self._defer_join = False
         self._pending_classes = {}      # class index -> event
         self._block_class = {}          # id(fblock) -> class index
         self._deferred_refs = None      # gradients the side streams still read
@@ -323,12 +394,24 @@ class KFAC(_base.GradientMethod):
             self.fblocks.append(fblock)
         self._set_low_rank(1, 0, None)
         self.kfhook = KFACHook(self.fblocks)
-        for fb in self.fblocks:
-            module = getattr(fb.link, 'module', None)
-            if module is not None:
-                module.register_forward_pre_hook(
-                    lambda m, inp, fb=fb: self._wait_for_block(fb))
+        self._pre_hooked = False
+        self.defer_join = self._defer_join
         return self
+
+    @property
+    def defer_join(self):
+        return self._defer_join
+
+    @defer_join.setter
+    def defer_join(self, on):
+        self._defer_join = on
+        if on and self.fblocks and not self._pre_hooked:
+            self._pre_hooked = True
+            for fb in self.fblocks:
+                module = getattr(fb.link, 'module', None)
+                if module is not None:
+                    module.register_forward_pre_hook(
+                        lambda m, inp, fb=fb: self._wait_for_block(fb))
 
     def _wait_for_block(self, fb):
         """Forward pre-hook of a layer: its weights may still be being
@@ -359,7 +442,7 @@ class KFAC(_base.GradientMethod):
 
     def reallocate_cleared_grads(self):
         for param in self.target.params(include_uninit=False):
-            if hasattr(param, 'kfgrad') and param.kfgrad is None:
+            if getattr(param, 'kfgrad', self) is None:
                 param.kfgrad = torch.zeros_like(param.data)
         super(KFAC, self).reallocate_cleared_grads()
 
@@ -372,7 +455,10 @@ class KFAC(_base.GradientMethod):
         items = pending_factor_items(self.fblocks, forward_only)
         if items:
             dev = next(self.target.params()).data.device
-            ops.factor_group(items, dev)
+            if self.acc_iters > 1 and type(self) is KFAC and not forward_only:
+                self._build_and_accumulate(items, dev)
+            else:
+                ops.factor_group(items, dev)
         if not forward_only:
             for fb in self.fblocks:
                 fb._keep_x = fb._keep_gy = None
@@ -469,15 +555,11 @@ class KFAC(_base.GradientMethod):
         side = self._eager_stream
         side.wait_event(ready)
         with torch.cuda.stream(side):
-            items = pending_factor_items(blocks)
-            # the activations and gradients behind the items stay referenced
-            # until the main stream has waited for this build
-            e['keep'].append(items)
-            if items:
-                ops.factor_group(items, first.link.W.data.device
-                                 if hasattr(first.link, 'W')
-                                 else first.link.gamma.data.device)
-            update_cov_emas_grouped(blocks)
+            # (the blocks keep the activations and gradients referenced until
+            # the main stream has waited for this build)
+            build_factors(blocks, first.link.W.data.device
+                          if hasattr(first.link, 'W')
+                          else first.link.gamma.data.device)
             e['plan'].start_class(c, first.damping,
                                   first._pi_type == PI_TYPE_TRACENORM)
             built = torch.cuda.Event()
@@ -533,6 +615,31 @@ class KFAC(_base.GradientMethod):
             'acc_count {} should not be larger than acc_iters {}'.format(
                 self.acc_count, self.acc_iters))
 
+    def _build_and_accumulate(self, items, device):
+        """The factors of this micro-step with their share of the sum
+        (``accumulate_covs``) added in the same pass, for the blocks that are
+        built as a whole."""
+        built = {}
+        for it in items:
+            built.setdefault(id(it.block), []).append(it)
+        first = self.acc_count == 0
+        second = []
+        for it in items:
+            fb = it.block
+            whole = len(built[id(fb)]) == len(fb.covs)
+            if first and whole and it is built[id(fb)][0]:
+                acc = fb.__dict__.get('_acc_bufs')
+                if acc is None or [a.shape for a in acc] != \
+                        [c.shape for c in fb.covs]:
+                    acc = [torch.empty_like(c) for c in fb.covs]
+                fb._acc_bufs = acc
+            old = fb._acc_bufs if first and whole else \
+                getattr(fb, 'acc_covs', None)
+            fb._acc_done = bool(whole and old is not None)
+            second.append(old[it.which] if fb._acc_done else None)
+        ops.factor_group(items, device, second, 1.0 / self.acc_iters,
+                         0.0 if first else 1.0)
+
     def _accumulate_group(self, pairs):
         """acc += x / acc_iters for (x, acc) pairs, acc = x / acc_iters for
         (x, None); one grouped launch each for the new and for the existing
@@ -565,15 +672,20 @@ class KFAC(_base.GradientMethod):
 
     def accumulate_covs(self):
         """``kfac.py:295-304``."""
-        pairs = []
+        pairs, rest = [], []
         for fblock in self.fblocks:
             fblock.check_attr('covs')
             old = getattr(fblock, 'acc_covs', None)
+            if fblock.__dict__.pop('_acc_done', False):
+                if old is None:
+                    fblock.acc_covs = list(fblock._acc_bufs)
+                continue
+            rest.append(fblock)
             for j, c in enumerate(fblock.covs):
                 pairs.append((c, None if old is None else old[j]))
         accs = self._accumulate_group(pairs)
         k = 0
-        for fblock in self.fblocks:
+        for fblock in rest:
             n = len(fblock.covs)
             fblock.acc_covs = accs[k:k + n]
             k += n
@@ -685,10 +797,7 @@ class KFAC(_base.GradientMethod):
                     seen.add(id(owner[i]))
                     if id(owner[i]) not in ema_done:
                         blocks.append(owner[i])
-            items = pending_factor_items(blocks)
-            if items:
-                ops.factor_group(items, dev)
-            update_cov_emas_grouped(blocks)
+            build_factors(blocks, dev)
             if c + 1 < len(classes):
                 plan.start_class(c, first.damping,
                                  first._pi_type == PI_TYPE_TRACENORM)
@@ -768,12 +877,12 @@ class KFAC(_base.GradientMethod):
                         self._block_class[id(fb)] = owner_cls[k]
                     k += n
                 continue
-            diag = plan.diag
+            diag = plan.diag_items
             k = 0
             for fb in group:
                 n = len(fb.plan_factors())
                 if n:
-                    fb.set_diag_vals(diag[k:k + n])
+                    fb.set_diag_vals(diag, k)
                 k += n
         conn = [fb for fb in fblocks
                 if isinstance(fb, FB.FisherBlockConnection) and

@@ -181,6 +181,16 @@ size_t kfac_factor_group_workspace_bytes(int count,
 int kfac_factor_group(int count, const kfac_factor_item* items,
                       void* workspace, size_t workspace_bytes, void* stream);
 
+/* kfac_factor_group that keeps a second array per factor up to date in the
+ * same pass: second[i] = a2 * items[i].out + b2 * second[i] (d x d, symmetric;
+ * NULL entries: none; b2 == 0: second[i] is not read).  The running averages of
+ * FisherBlock.update_cov_emas (optimizers/fisher_block.py:155-163) and the sums
+ * of KFAC.accumulate_covs (optimizers/kfac.py:295-304). */
+int kfac_factor_group_second(int count, const kfac_factor_item* items,
+                             float* const* second, float a2, float b2,
+                             void* workspace, size_t workspace_bytes,
+                             void* stream);
+
 /* Per-sample BatchNormalization gradients: out is (n x 2c),
  * out[s, j] = scale * sum_hw gy[s,j,:] * xhat[s,j,:] and
  * out[s, c+j] = scale * sum_hw gy[s,j,:], xhat = x normalised with the batch

@@ -263,6 +263,30 @@ def test_factor_of_3x3_convolutions(ops, engine, n, c, h, w, stride,
     check_symmetric(host(out))
 
 
+@pytest.mark.parametrize('b2', [0.0, 0.75])
+def test_factor_group_second_output(ops, engine, b2):
+    """Running averages kept up to date by the build: factors that are
+    assembled from shifted products, reduced from wide and narrow pieces,
+    built by the gather kernel, and one without a second array."""
+    torch.manual_seed(5)
+    xc = torch.randn(3, 40, 9, 8, device='cuda')
+    xs = [torch.randn(r, d, device='cuda')
+          for r, d in ((2100, 1028), (40000, 60), (70, 33), (50, 20))]
+    u = torch.nn.functional.unfold(xc.double(), 3, padding=1)
+    mats = [u.transpose(1, 2).reshape(-1, 360)] + [x.double() for x in xs]
+    outs = [torch.empty(m.shape[1], m.shape[1], device='cuda') for m in mats]
+    second = [torch.full_like(o, 3.0) for o in outs[:4]] + [None]
+    items = [ops.conv_input_item(xc, 3, 1, 1, False, 0.5, 0.0, outs[0])] + [
+        ops.dense_item(x, False, 0.5, 0.0, o) for x, o in zip(xs, outs[1:])]
+    ops.factor_group(items, xc.device, second, 0.25, b2)
+    for m, o, s in zip(mats, outs, second):
+        ref = 0.5 * (m.t() @ m)
+        assert rel(host(o), host(ref)) < FACTOR_TOL
+        if s is not None:
+            assert rel(host(s), host(0.25 * ref + b2 * 3.0)) < FACTOR_TOL
+            check_symmetric(host(s))
+
+
 @pytest.mark.parametrize('rows,d,ones', [
     (2000, 1024, False), (1999, 1025, False), (1500, 1411, True)])
 def test_wide_factor_from_staged_planes(ops, rows, d, ones):
