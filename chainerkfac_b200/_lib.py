@@ -161,5 +161,4 @@ def float_array(values):
 
 
 def ptr_array(values):
-    return (ctypes.c_void_p * len(values))(*[
-        (None if v is None else int(v)) for v in values])
+    return (ctypes.c_void_p * len(values))(*values)

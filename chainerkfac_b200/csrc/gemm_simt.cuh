@@ -279,9 +279,11 @@ int tc_tiles(GemmDesc& g);
 // (once per device; the launch helpers call it, plans call it before capture).
 int tc_prepare();
 // Tile engine of the inverse and precondition products (tc_tile.cu).  Number
-// the tiles of a launch (fills tile_begin, tiles_m, tiles_n) and choose their
-// width; returns the launch's tile count.
-int tc_number_tiles(GemmDesc* descs, int n, int* tile_cols);
+// the tiles of a launch (fills tile_begin, tiles_m, tiles_n; may reorder the
+// problems) and choose their width, narrow up to `narrow_max` narrow tiles;
+// returns the launch's tile count.
+constexpr int kTileInline = 8;   // descriptors that fit the kernel arguments
+int tc_number_tiles(GemmDesc* descs, int n, int narrow_max, int* tile_cols);
 int tc_prepare_tiles();
 // `descs_host`: the same descriptors on the host (small launches pass them as
 // kernel arguments), or NULL.

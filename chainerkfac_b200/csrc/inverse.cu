@@ -908,27 +908,51 @@ refine_probe_kernel(const MatInfo* __restrict__ mats,
     sums[2 * blockIdx.y] = 0.0;
     sums[2 * blockIdx.y + 1] = 0.0;
   }
-  if (row >= d) return;
+  if (8 * blockIdx.x >= d) return;
   double* t = it.vec;
   double* r = it.vec + d;
-  const float* mrow = (stage == 1 ? mi.F : mi.inv) + (long long)row * d;
   double s = 0.0;
-  if (stage == 0) {
-    for (int c = lane; c < d; c += 32) s += (double)mrow[c] * probe_sign(c);
-  } else {
+  if (row < d) {
+    const float* mrow = (stage == 1 ? mi.F : mi.inv) + (long long)row * d;
     const double* x = stage == 1 ? t : r;
-    for (int c = lane; c < d; c += 32) s += (double)mrow[c] * x[c];
+    // eight loads of the row in flight per lane
+    for (int c0 = lane; c0 < d; c0 += 256) {
+      float m[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        m[i] = c0 + 32 * i < d ? mrow[c0 + 32 * i] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int c = c0 + 32 * i;
+        if (c < d) s += (double)m[i] * (stage == 0 ? (double)probe_sign(c) : x[c]);
+      }
+    }
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if (lane != 0) return;
-  if (stage == 0) {
-    t[row] = s;
-  } else if (stage == 1) {
-    const float a = damp_of_row(mi, add[it.mat], add2[it.mat], row);
-    r[row] = (double)probe_sign(row) - (s + (double)a * t[row]);
-  } else {
-    atomicAdd(&sums[2 * blockIdx.y], s * s);
-    atomicAdd(&sums[2 * blockIdx.y + 1], t[row] * t[row]);
+  __shared__ double part[2][8];
+  if (lane == 0) {
+    double e2 = 0.0, t2 = 0.0;
+    if (row < d) {
+      if (stage == 0) {
+        t[row] = s;
+      } else if (stage == 1) {
+        const float a = damp_of_row(mi, add[it.mat], add2[it.mat], row);
+        r[row] = (double)probe_sign(row) - (s + (double)a * t[row]);
+      } else {
+        e2 = s * s;
+        t2 = t[row] * t[row];
+      }
+    }
+    part[0][threadIdx.x >> 5] = e2;
+    part[1][threadIdx.x >> 5] = t2;
+  }
+  if (stage != 2) return;
+  // (one addition per block: the rows of a matrix share two words)
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double v = 0.0;
+    for (int w = 0; w < 8; ++w) v += part[threadIdx.x][w];
+    atomicAdd(&sums[2 * blockIdx.y + threadIdx.x], v);
   }
 }
 
@@ -1107,6 +1131,7 @@ struct kfac_inverse_plan {
   float* add2_dev;
   int n_refine;
   int refine_dmax;
+  int dmax;                // largest side
   int refine_tiles;
   Launch refine_prod;
   RefineItem* refine_items_dev;
@@ -1244,7 +1269,8 @@ extern "C" int kfac_inverse_plan_create(
   auto end_gemm = [&](Launch& l, bool record) {
     if (l.n == 0) return -1;
     if (use_tc && l.kind == 1)
-      l.tiles = tc_number_tiles(&descs[l.off], l.n, &l.tile_cols);
+      l.tiles = tc_number_tiles(&descs[l.off], l.n, 3 * sm_count() / 4,
+                                &l.tile_cols);
     if (record) l.rec_ev = n_events++;
     launches.push_back(l);
     return l.rec_ev;
@@ -1539,6 +1565,7 @@ extern "C" int kfac_inverse_plan_create(
   p->refine_gate_dev = nullptr; p->refine_count_dev = nullptr;
   p->n_refine = (int)ritems.size();
   p->refine_dmax = refine_dmax;
+  p->dmax = dmax;
   p->refine_tiles = refine_tiles;
   p->refine_max_dim = kRefineDimCap;
   p->refine_threshold = 3e-5f;
@@ -1595,6 +1622,7 @@ extern "C" int kfac_inverse_plan_create(
   }
   if (use_tc && refine_prod.n > 0)
     refine_prod.tiles = tc_number_tiles(&descs[refine_prod.off], refine_prod.n,
+                                        sm_count(),
                                         &refine_prod.tile_cols);
   p->refine_prod = refine_prod;
   p->descs = descs;
@@ -1654,7 +1682,8 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
       p->add2_dev, diag_dev);
   KFAC_LAUNCH_CHECK("damping_kernel");
   {
-    dim3 grid(512, p->count);
+    // a block copies about four rows of the largest matrix
+    dim3 grid(std::max(1, std::min(512, p->dmax / 4)), p->count);
     damp_copy_kernel<<<grid, 256, 0, st>>>(p->mats_dev, p->add_dev,
                                            p->add2_dev, p->look ? 1 : 0);
     KFAC_LAUNCH_CHECK("damp_copy_kernel");

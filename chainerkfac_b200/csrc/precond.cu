@@ -98,12 +98,14 @@ extern "C" int kfac_precondition(
   }
   int cols1 = 0, cols2 = 0;
   if (use_tc) {
-    tiles1 = tc_number_tiles(descs.data(), count, &cols1);
-    tiles2 = tc_number_tiles(descs.data() + count, count, &cols2);
+    tiles1 = tc_number_tiles(descs.data(), count, sm_count(), &cols1);
+    tiles2 = tc_number_tiles(descs.data() + count, count, sm_count(), &cols2);
   }
-  KFAC_CUDA(cudaMemcpyAsync(descs_dev, descs.data(),
-                            descs.size() * sizeof(GemmDesc),
-                            cudaMemcpyHostToDevice, st));
+  // (the tile kernel takes the descriptors of a few layers as an argument)
+  if (!use_tc || count > kTileInline)
+    KFAC_CUDA(cudaMemcpyAsync(descs_dev, descs.data(),
+                              descs.size() * sizeof(GemmDesc),
+                              cudaMemcpyHostToDevice, st));
   if (use_tc) {
     int rc = launch_tc_grouped(descs_dev, descs.data(), count, tiles1, cols1,
                                false, 0.f, 0.f, st);

@@ -35,7 +35,7 @@ namespace kfac {
 
 constexpr int TT_BK = 32;
 constexpr int TT_EP = 36;         // row pitch of an epilogue piece (floats)
-constexpr int TT_INLINE = 8;      // descriptors that fit the kernel arguments
+constexpr int TT_INLINE = kTileInline;
 
 static __device__ int g_tile_status = 0;
 
@@ -720,17 +720,19 @@ static bool tile_desc_vec(const GemmDesc& g) {
   return tile_operand_vec(g.A) && tile_operand_vec(g.B);
 }
 
-int tc_number_tiles(GemmDesc* descs, int n, int* tile_cols) {
+int tc_number_tiles(GemmDesc* descs, int n, int narrow_max, int* tile_cols) {
   std::stable_partition(descs, descs + n, tile_desc_vec);
   // Narrow tiles (half the work per CTA, but the A rows are loaded, split and
-  // read by the MMAs twice as often) where they leave a quarter of the SMs to
-  // the launches of other streams.  Measured with the line at 20, 74, 111 and
+  // read by the MMAs twice as often) up to `narrow_max` of them: as many as
+  // there are SMs for a launch that runs alone (512 x 4608 x 4608: 144 narrow
+  // tiles 125 us, 72 wide ones 190 us), three quarters where launches of other
+  // streams run beside it.  Measured with the line at 20, 74, 111 and
   // 148 of 148 SMs: a 2304-row inverse 835, 791, 791, 791 us; a 4608-row one
   // 1954, 1934, 1915, 1902; 108 factors of ResNet-50 in three concurrent plans
   // 6.10, 6.22, 6.27, 6.33 ms.
   long long narrow = 0;
   for (int i = 0; i < n; ++i) narrow += tile_count(descs[i], 128);
-  const int tn = 4 * narrow <= 3LL * sm_count() ? 128 : 256;
+  const int tn = narrow <= narrow_max ? 128 : 256;
   int total = 0;
   for (int i = 0; i < n; ++i) {
     descs[i].tile_begin = total;

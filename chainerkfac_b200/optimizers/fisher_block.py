@@ -96,11 +96,11 @@ class FisherBlock(object):
         first = self.cov_emas is None
         if first:
             self.cov_emas = [torch.empty_like(c) for c in self.covs]
-        for cov, ema in zip(self.covs, self.cov_emas):
-            if r == 1.0 or first:
-                ops.axpby(1.0, cov, 0.0, ema, ema)
-            else:
-                ops.axpby(r, cov, 1.0 - r, ema, ema)
+        if r == 1.0 or first:
+            ops.axpby_group(1.0, self.covs, 0.0, self.cov_emas, self.cov_emas)
+        else:
+            ops.axpby_group(r, self.covs, 1.0 - r, self.cov_emas,
+                            self.cov_emas)
 
     # -- damped inverse (fisher_block.py:165-179) -------------------------
     def plan_entries(self):
