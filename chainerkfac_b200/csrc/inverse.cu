@@ -1276,11 +1276,23 @@ extern "C" int kfac_inverse_plan_create(
     return l.rec_ev;
   };
 
+  // Width of the chain's panels.  Between two panels the chain waits for the
+  // last solve and the near part of the trailing update, so matrices of up to
+  // two panels are one where the longer panel updates of a step still fit the
+  // SMs (1024 rows 380 -> 360 us; 68 such matrices at once, or 4608 rows, whose
+  // panel updates are what the chain waits for, gain nothing from it).
+  long long step_tiles = 0;
+  for (int i = 0; i < count; ++i)
+    if (dims[i] > PW)
+      step_tiles += (long long)((dims[i] - 1) / DB) * ((dims[i] - DB + 255) / 256);
+  const int CW =
+      look && dmax <= 2 * PW && step_tiles <= sm_count() ? 2 * PW : PW;
+
   int prev_far_ev = -1;
   // Two-level right-looking Cholesky: panels of PW columns are factored by
   // 128-wide inner steps whose updates stay inside the panel (short
   // contractions, little work); the bulk of the flops is the update of the
-  // trailing matrix with the whole panel (contraction length PW).
+  // trailing matrix with the whole panel (contraction length CW).
   //
   // The chain carries the diagonal kernels; inside a panel the diagonal
   // kernel of step k applies step k-1's update to its own block itself
@@ -1301,132 +1313,9 @@ extern "C" int kfac_inverse_plan_create(
   // 0.15 ms instead of the 0.95 ms that the whole triangular inverse and
   // product took behind the factorisation).  T^T waits in the unused upper
   // triangle of W.
-  for (int po = 0; po < dmax; po += PW) {
-    const int inner = std::min(PW, dmax - po);
-    int bulk_ev = -1;          // the bulk stream's last launch of this panel
-    int last_solve_ev = -1;
-    for (int o = po; o < po + inner; o += DB) {
-      const bool lk = look && o > po;
-      // the matrices that still have a block here are the first of `order`
-      Launch dl = begin_gemm(S_CHAIN);
-      dl.kind = 0;
-      dl.step = o / DB;
-      dl.look = lk;
-      for (int i : order)
-        if (dims[i] > o) dl.n += 1;
-      if (lk && o - 2 * DB >= po) dl.wait(upd_ev[(o - 2 * DB) / DB]);
-      diag_ev[o / DB] = end_gemm(dl, look);
-
-      Launch trsm = begin_gemm(s_bulk);
-      for (int i : order) {
-        const int d = dims[i];
-        const int M = d - o - DB;
-        if (M <= 0) continue;
-        const MatInfo& m = mats[i];
-        const long long ld = m.ld;
-        GemmDesc g = {};
-        float* panel = m.W + (o + DB) * ld + o;
-        g.A = strided_operand(panel, 1, ld, M);
-        g.B = strided_operand(m.X + o * ld + o, 1, ld, DB);
-        g.C = panel; g.ldc = ld; g.M = M; g.N = DB; g.K = DB;
-        g.alpha = 1.f; g.beta = 0.f; g.flags = 0;
-        push_desc(trsm, g);
-      }
-      trsm.wait(diag_ev[o / DB]);
-      const int solve_ev = end_gemm(trsm, look);
-      if (solve_ev >= 0) bulk_ev = last_solve_ev = solve_ev;
-
-      // update the rest of this panel's columns (full rectangle; entries
-      // above the diagonal are written but never read).  With look-ahead the
-      // next diagonal block is left to the next diagonal kernel.
-      const int skip = (look && o + DB < po + inner) ? DB : 0;
-      Launch upd = begin_gemm(s_bulk);
-      for (int i : order) {
-        const int d = dims[i];
-        const int M = d - o - DB - skip;
-        const int N = std::min(po + PW, d) - (o + DB);
-        if (M <= 0 || N <= 0) continue;
-        const MatInfo& m = mats[i];
-        const long long ld = m.ld;
-        GemmDesc g = {};
-        float* panel = m.W + (o + DB + skip) * ld + o;
-        const long long coff = (o + DB + skip) * ld + (o + DB);
-        g.A = strided_operand(panel, 1, ld, M);
-        g.B = strided_operand(m.W + (o + DB) * ld + o, 1, ld, N);
-        g.C = m.W + coff;
-        g.ldc = ld; g.M = M; g.N = N; g.K = DB;
-        g.alpha = -1.f; g.beta = 1.f; g.flags = 0;
-        if (look) g.C2 = m.V + coff;
-        push_desc(upd, g);
-      }
-      upd_ev[o / DB] = end_gemm(upd, look);
-      if (upd_ev[o / DB] >= 0) bulk_ev = upd_ev[o / DB];
-    }
-
-    // Update of the trailing matrix with the finished panel, in two parts:
-    // the columns of the next panel (needed before the chain can go on) on
-    // the chain's stream, the columns beyond them on the far stream, next to
-    // the next panel's chain.  Both parts of one panel touch disjoint tiles;
-    // parts of successive panels that touch the same tiles are ordered by
-    // events (next-panel part p+1 after far part p) or by stream order.
-    Launch near = begin_gemm(S_CHAIN);
-    std::vector<GemmDesc> far_descs;
-    for (int i : order) {
-      const int d = dims[i];
-      const int M = d - po - PW;
-      if (M <= 0) continue;
-      const int N1 = std::min(PW, M);
-      const MatInfo& m = mats[i];
-      const long long ld = m.ld;
-      const float* panel = m.W + (po + PW) * ld + po;
-      {
-        GemmDesc g = {};     // square block on the diagonal: lower tiles
-        const long long coff = (po + PW) * ld + (po + PW);
-        g.A = strided_operand(panel, 1, ld, N1);
-        g.B = g.A;
-        g.C = m.W + coff;
-        g.ldc = ld; g.M = N1; g.N = N1; g.K = PW;
-        g.alpha = -1.f; g.beta = 1.f; g.flags = G_LOWER | G_SAME_AB;
-        if (look) g.C2 = m.V + coff;
-        push_desc(near, g);
-      }
-      if (M > N1) {
-        const float* below = panel + N1 * ld;
-        GemmDesc g = {};     // rectangle below it
-        const long long coff = (po + PW + N1) * ld + (po + PW);
-        g.A = strided_operand(below, 1, ld, M - N1);
-        g.B = strided_operand(panel, 1, ld, N1);
-        g.C = m.W + coff;
-        g.ldc = ld; g.M = M - N1; g.N = N1; g.K = PW;
-        g.alpha = -1.f; g.beta = 1.f; g.flags = 0;
-        if (look) g.C2 = m.V + coff;
-        push_desc(near, g);
-        GemmDesc h = {};     // everything beyond the next panel's columns
-        h.A = strided_operand(below, 1, ld, M - N1);
-        h.B = h.A;
-        h.C = m.W + (po + PW + N1) * ld + (po + PW + N1);
-        h.ldc = ld; h.M = M - N1; h.N = M - N1; h.K = PW;
-        h.alpha = -1.f; h.beta = 1.f; h.flags = G_LOWER | G_SAME_AB;
-        far_descs.push_back(h);
-      }
-    }
-    int panel_ev = last_solve_ev;
-    if (!look && !far_descs.empty()) {
-      // the far part needs the finished panel: an event recorded on the
-      // chain right before the near part
-      panel_ev = n_events++;
-      launches.back().rec_ev = panel_ev;   // last launch of the panel's chain
-    }
-    near.wait(prev_far_ev);                // far part of the previous panel
-    if (look) near.wait(panel_ev);         // the bulk stream's last solve
-    if (near.n > 0) prev_far_ev = -1;
-    end_gemm(near, false);
-    Launch far = begin_gemm(S_FAR);
-    for (auto& h : far_descs) push_desc(far, h);
-    far.wait(panel_ev);
-    if (far.n > 0) prev_far_ev = end_gemm(far, true);
-
-    // ---- row panel of the inverse
+  int bulk_ev = -1;            // the bulk stream's last launch of this panel
+  // Row panel po of the inverse, once the chain is through with it.
+  auto row_panel = [&](int po) {
     const int pend = std::min(po + PW, dmax);
     bool first = true;
     for (int b = DB; b < pend - po; b *= 2) {
@@ -1530,6 +1419,134 @@ extern "C" int kfac_inverse_plan_create(
     if (look && first) next_t.wait(bulk_ev);
     end_gemm(next_t, false);
     end_gemm(prod, false);
+  };
+  for (int co = 0; co < dmax; co += CW) {
+    const int inner = std::min(CW, dmax - co);
+    bulk_ev = -1;
+    int last_solve_ev = -1;
+    for (int o = co; o < co + inner; o += DB) {
+      const bool lk = look && o > co;
+      // the matrices that still have a block here are the first of `order`
+      Launch dl = begin_gemm(S_CHAIN);
+      dl.kind = 0;
+      dl.step = o / DB;
+      dl.look = lk;
+      for (int i : order)
+        if (dims[i] > o) dl.n += 1;
+      if (lk && o - 2 * DB >= co) dl.wait(upd_ev[(o - 2 * DB) / DB]);
+      diag_ev[o / DB] = end_gemm(dl, look);
+
+      Launch trsm = begin_gemm(s_bulk);
+      for (int i : order) {
+        const int d = dims[i];
+        const int M = d - o - DB;
+        if (M <= 0) continue;
+        const MatInfo& m = mats[i];
+        const long long ld = m.ld;
+        GemmDesc g = {};
+        float* panel = m.W + (o + DB) * ld + o;
+        g.A = strided_operand(panel, 1, ld, M);
+        g.B = strided_operand(m.X + o * ld + o, 1, ld, DB);
+        g.C = panel; g.ldc = ld; g.M = M; g.N = DB; g.K = DB;
+        g.alpha = 1.f; g.beta = 0.f; g.flags = 0;
+        push_desc(trsm, g);
+      }
+      trsm.wait(diag_ev[o / DB]);
+      const int solve_ev = end_gemm(trsm, look);
+      if (solve_ev >= 0) bulk_ev = last_solve_ev = solve_ev;
+
+      // update the rest of this panel's columns (full rectangle; entries
+      // above the diagonal are written but never read).  With look-ahead the
+      // next diagonal block is left to the next diagonal kernel.
+      const int skip = (look && o + DB < co + inner) ? DB : 0;
+      Launch upd = begin_gemm(s_bulk);
+      for (int i : order) {
+        const int d = dims[i];
+        const int M = d - o - DB - skip;
+        const int N = std::min(co + CW, d) - (o + DB);
+        if (M <= 0 || N <= 0) continue;
+        const MatInfo& m = mats[i];
+        const long long ld = m.ld;
+        GemmDesc g = {};
+        float* panel = m.W + (o + DB + skip) * ld + o;
+        const long long coff = (o + DB + skip) * ld + (o + DB);
+        g.A = strided_operand(panel, 1, ld, M);
+        g.B = strided_operand(m.W + (o + DB) * ld + o, 1, ld, N);
+        g.C = m.W + coff;
+        g.ldc = ld; g.M = M; g.N = N; g.K = DB;
+        g.alpha = -1.f; g.beta = 1.f; g.flags = 0;
+        if (look) g.C2 = m.V + coff;
+        push_desc(upd, g);
+      }
+      upd_ev[o / DB] = end_gemm(upd, look);
+      if (upd_ev[o / DB] >= 0) bulk_ev = upd_ev[o / DB];
+      // (the last rows of a chain panel come behind its trailing update)
+      if ((o + DB) % PW == 0 && o + DB < co + inner) row_panel(o + DB - PW);
+    }
+
+    // Update of the trailing matrix with the finished panel, in two parts:
+    // the columns of the next panel (needed before the chain can go on) on
+    // the chain's stream, the columns beyond them on the far stream, next to
+    // the next panel's chain.  Both parts of one panel touch disjoint tiles;
+    // parts of successive panels that touch the same tiles are ordered by
+    // events (next-panel part p+1 after far part p) or by stream order.
+    Launch near = begin_gemm(S_CHAIN);
+    std::vector<GemmDesc> far_descs;
+    for (int i : order) {
+      const int d = dims[i];
+      const int M = d - co - CW;
+      if (M <= 0) continue;
+      const int N1 = std::min(CW, M);
+      const MatInfo& m = mats[i];
+      const long long ld = m.ld;
+      const float* panel = m.W + (co + CW) * ld + co;
+      {
+        GemmDesc g = {};     // square block on the diagonal: lower tiles
+        const long long coff = (co + CW) * ld + (co + CW);
+        g.A = strided_operand(panel, 1, ld, N1);
+        g.B = g.A;
+        g.C = m.W + coff;
+        g.ldc = ld; g.M = N1; g.N = N1; g.K = CW;
+        g.alpha = -1.f; g.beta = 1.f; g.flags = G_LOWER | G_SAME_AB;
+        if (look) g.C2 = m.V + coff;
+        push_desc(near, g);
+      }
+      if (M > N1) {
+        const float* below = panel + N1 * ld;
+        GemmDesc g = {};     // rectangle below it
+        const long long coff = (co + CW + N1) * ld + (co + CW);
+        g.A = strided_operand(below, 1, ld, M - N1);
+        g.B = strided_operand(panel, 1, ld, N1);
+        g.C = m.W + coff;
+        g.ldc = ld; g.M = M - N1; g.N = N1; g.K = CW;
+        g.alpha = -1.f; g.beta = 1.f; g.flags = 0;
+        if (look) g.C2 = m.V + coff;
+        push_desc(near, g);
+        GemmDesc h = {};     // everything beyond the next panel's columns
+        h.A = strided_operand(below, 1, ld, M - N1);
+        h.B = h.A;
+        h.C = m.W + (co + CW + N1) * ld + (co + CW + N1);
+        h.ldc = ld; h.M = M - N1; h.N = M - N1; h.K = CW;
+        h.alpha = -1.f; h.beta = 1.f; h.flags = G_LOWER | G_SAME_AB;
+        far_descs.push_back(h);
+      }
+    }
+    int panel_ev = last_solve_ev;
+    if (!look && !far_descs.empty()) {
+      // the far part needs the finished panel: an event recorded on the
+      // chain right before the near part
+      panel_ev = n_events++;
+      launches.back().rec_ev = panel_ev;   // last launch of the panel's chain
+    }
+    near.wait(prev_far_ev);                // far part of the previous panel
+    if (look) near.wait(panel_ev);         // the bulk stream's last solve
+    if (near.n > 0) prev_far_ev = -1;
+    end_gemm(near, false);
+    Launch far = begin_gemm(S_FAR);
+    for (auto& h : far_descs) push_desc(far, h);
+    far.wait(panel_ev);
+    if (far.n > 0) prev_far_ev = end_gemm(far, true);
+    row_panel((std::min(co + inner, dmax) - 1) / PW * PW);
   }
 
   // refinement of the matrices of up to kRefineDimCap rows: Y = X R on the
