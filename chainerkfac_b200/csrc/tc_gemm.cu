@@ -1058,15 +1058,16 @@ static size_t tc_pair_workspace_bytes(int count, const FactorJob* jobs,
 //    rows 43 us with the gather, 72 us without);
 //  * other wide factors, where the gather feeds every element to many tiles
 //    (NCHW, 1568 x 2048: 68 -> 27; even at 1000 columns, slower below);
-//  * patches of strided convolutions with many channels (1x1, 512 channels
-//    28 x 28 channels-last: 84 -> 27; 3x3, 256 channels 28 x 28: 199 -> 155;
-//    the 3-channel 7x7 stem stays with the gather, 160 against 486).
+//  * patches of other convolutions unless they have few channels (1x1 / 2, 512
+//    channels 28 x 28 channels-last: 84 -> 27; 3x3 / 2, 256 channels 28 x 28:
+//    199 -> 155; 3x3 with bias, 37 channels 15 x 15: 75 -> 52; even at 16
+//    channels; the 3-channel 7x7 stem 160 against 486).
 static bool tc_uses_gram(const FactorJob& job) {
   if (tc_staged()) return false;
   if (gram_grid_job(job)) return true;
   if ((double)job.rows * job.d >= 1e6 && gram_direct_job(job)) return true;
-  if ((double)job.rows * job.d < 2e6) return false;
-  return job.d >= 1024 || (job.X.mode == 1 && job.X.C >= 128);
+  if (job.X.mode == 1 && job.X.C >= 20) return true;
+  return job.d >= 1024 && (double)job.rows * job.d >= 2e6;
 }
 
 static void tc_by_feed(int count, const FactorJob* jobs, bool staged,

@@ -751,11 +751,16 @@ int launch_tc_grouped(const GemmDesc* descs_dev, const GemmDesc* descs_host,
   const int rc = tc_prepare_tiles();
   if (rc != KFAC_OK) return rc;
   // the problems with 16-byte rows come first (tc_number_tiles); where all
-  // tiles fit the chip at once one launch of the general kernel ends sooner
-  // than two in a row
+  // tiles fit the chip at once, one launch of the general kernel (2 us per
+  // k-block) may end sooner than two in a row (1 us, and 10 us more)
   int n_vec = 0;
   while (n_vec < ndesc && tile_desc_vec(descs_host[n_vec])) ++n_vec;
-  if (n_vec < ndesc && total_tiles <= sm_count()) n_vec = 0;
+  if (n_vec < ndesc && total_tiles <= sm_count()) {
+    long long k[2] = {0, 0};
+    for (int i = 0; i < ndesc; ++i)
+      k[i >= n_vec] = std::max(k[i >= n_vec], descs_host[i].K / TT_BK);
+    if (2 * std::max(k[0], k[1]) <= k[0] + 2 * k[1] + 10) n_vec = 0;
+  }
   for (int k = 0; k < 2; ++k) {
     const int first = k == 0 ? 0 : n_vec, n = k == 0 ? n_vec : ndesc - n_vec;
     if (n == 0) continue;
