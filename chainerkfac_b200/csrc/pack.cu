@@ -70,11 +70,11 @@ int ring_alloc(size_t bytes, void** out) {
   return KFAC_OK;
 }
 
-// Work is cut into items that one 256-thread block handles: a 64x64 tile of a
-// packed triangle (tile column <= tile row), or a run of kChunk elements of a
-// plain array.  item_begin is the running count of items over the arrays of
-// the call, so a block finds its array by bisection and its tile by inverting
-// t = tr(tr+1)/2 + tc.
+// Work is cut into items that one 256-thread block handles: a run of kChunk
+// elements of a plain array or, packing, of the wire; unpacking, also a 64x64
+// tile of a triangle (tile column <= tile row).  item_begin is the running
+// count of items over the arrays of the call, so a block finds its array by
+// bisection and its tile by inverting t = tr(tr+1)/2 + tc.
 static const int kTile = 64;
 static const int kChunk = 8192;
 static const int kMaxWires = 16;
@@ -118,47 +118,99 @@ __device__ __forceinline__ int find_array(const int* s_begin, int n_arrays,
   return lo;
 }
 
+// Packing walks the wire: a work item is a run of kChunk wire elements of one
+// array, from one 16-byte boundary to another, and a thread writes whole words
+// (whose elements may lie in two rows of a triangle).  Bound by HBM.  With
+// 64 x 64 tiles of the triangle, whose rows start anywhere in the wire, every
+// 256-byte store began and ended inside a sector: ResNet-50 in fp32 221 us, now
+// 151 us, 6.1 TB/s.  Eight elements in flight in eight blocks per SM; sixteen
+// in four blocks take 187 us, the thread's own latency is then the bound.
 template <typename W>
 __global__ void __launch_bounds__(256, kBlocksPerSm)
 wire_pack_kernel(const WireArray* __restrict__ arrs, int n_arrays,
                  int total_items, W* __restrict__ wire) {
+  constexpr int V = 16 / sizeof(W);
+  constexpr int U = 8 / V;             // words in flight
   __shared__ int s_begin[kTabCap];
   load_item_table(arrs, n_arrays, s_begin);
-  const int tx = threadIdx.x & (kTile - 1), ty = threadIdx.x >> 6;
+  // elements from the last 16-byte boundary to the wire's start
+  const int skew = (int)((reinterpret_cast<uintptr_t>(wire) / sizeof(W)) % V);
   for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
     const WireArray a = arrs[find_array(s_begin, n_arrays, item)];
-    const int t = item - (int)a.item_begin;
-    W* __restrict__ dst = wire + a.wire_off;
-    if (a.tri > 0 && a.select) {
-      int tr, tc;
-      tri_index(t, tr, tc);
-      const int d = a.tri;
-      const int c = tc * kTile + tx;
-      const float* __restrict__ src = a.ptr;
-#pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        const int rb = tr * kTile + half * 32 + ty;
-        float v[8];
+    // runs begin at a word; the array's own first and last word may be shared
+    // with its neighbours
+    const long long w0 = (long long)(item - (int)a.item_begin) * kChunk -
+                         (a.wire_off + skew) % V;
+    const int lo = (int)max(0ll, -w0);
+    const int n = (int)min((long long)kChunk, a.wire_n - w0);
+    const float* __restrict__ src = a.ptr;
+    const int d = a.tri;
+    W* __restrict__ dst = wire + a.wire_off + w0;
+    for (int k0 = V * (int)threadIdx.x; k0 < n; k0 += 256 * V * U) {
+      float v[U][V];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int r = rb + 4 * i;
-          if (r < d && c <= r) v[i] = src[(long long)r * d + c];
+      for (int u = 0; u < U; ++u) {
+        const int k = k0 + 256 * V * u;
+        if (k < lo || k + V > n) continue;     // see below
+        if (!a.select) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) v[u][e] = 0.f;
+          continue;
+        }
+        const float* p;
+        if (d > 0) {
+          const long long w = w0 + k;
+          int r = (int)((sqrtf(8.f * (float)w + 1.f) - 1.f) * 0.5f);
+          while ((long long)(r + 1) * (r + 2) / 2 <= w) ++r;
+          while ((long long)r * (r + 1) / 2 > w) --r;
+          const int c = (int)(w - (long long)r * (r + 1) / 2);
+          p = src + (long long)r * d + c;
+          if (r + 1 - c < V) {
+            // two or more rows
+            const float* q = p;
+            int m = r + 1 - c, row = r;
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+              v[u][e] = *q++;
+              if (--m == 0) {
+                ++row;
+                q = src + (long long)row * d;
+                m = row + 1;
+              }
+            }
+            continue;
+          }
+        } else {
+          p = src + w0 + k;
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int r = rb + 4 * i;
-          if (r < d && c <= r)
-            dst[(long long)r * (r + 1) / 2 + c] = to_wire<W>(v[i]);
-        }
+        for (int e = 0; e < V; ++e) v[u][e] = p[e];
       }
-    } else {
-      // plain array, or the slot of a skipped array that is to be cleared
-      const long long base = (long long)t * kChunk;
-      const float* __restrict__ src = a.ptr;
-#pragma unroll 8
-      for (int k = threadIdx.x; k < kChunk; k += 256) {
-        const long long w = base + k;
-        if (w < a.wire_n) dst[w] = to_wire<W>(a.select ? src[w] : 0.f);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = k0 + 256 * V * u;
+        if (k >= n) break;
+        if (k >= lo && k + V <= n) {
+          union { W w[V]; uint4 q; } out;
+#pragma unroll
+          for (int e = 0; e < V; ++e) out.w[e] = to_wire<W>(v[u][e]);
+          *reinterpret_cast<uint4*>(dst + k) = out.q;
+          continue;
+        }
+        for (int e = max(0, lo - k); e < V && k + e < n; ++e) {
+          float x = 0.f;
+          if (a.select) {
+            const long long w = w0 + k + e;
+            if (d > 0) {
+              int r, c;
+              tri_index(w, r, c);
+              x = src[(long long)r * d + c];
+            } else {
+              x = src[w];
+            }
+          }
+          dst[k + e] = to_wire<W>(x);
+        }
       }
     }
   }
@@ -259,7 +311,7 @@ wire_unpack_kernel(const WireArray* __restrict__ arrs, int n_arrays,
 
 static int build_table(int n_arrays, float* const* arrays,
                        const int64_t* nelems, const int* tri_dim,
-                       const int* select, bool skipped_get_items,
+                       const int* select, bool pack, bool skipped_get_items,
                        std::vector<WireArray>& tab, long long& total,
                        long long& items) {
   KFAC_REQUIRE(n_arrays > 0 && arrays && nelems && tri_dim,
@@ -287,10 +339,12 @@ static int build_table(int n_arrays, float* const* arrays,
     a.wire_off = total;
     total += a.wire_n;
     a.item_begin = items;
-    if (a.select && a.tri > 0) {
+    if (pack) {
+      if (a.select || skipped_get_items) items += (a.wire_n + 7 + kChunk - 1) / kChunk;
+    } else if (a.select && a.tri > 0) {
       long long t = (a.tri + kTile - 1) / kTile;
       items += t * (t + 1) / 2;
-    } else if (a.select || skipped_get_items) {
+    } else if (a.select) {
       items += (a.wire_n + kChunk - 1) / kChunk;
     }
   }
@@ -334,7 +388,8 @@ extern "C" int kfac_wire_pack_as(int wire_dtype, int n_arrays,
   std::vector<WireArray> tab;
   long long total = 0, items = 0;
   int rc = build_table(n_arrays, const_cast<float* const*>(arrays), nelems,
-                       tri_dim, select, zero_skipped != 0, tab, total, items);
+                       tri_dim, select, true, zero_skipped != 0, tab, total,
+                       items);
   if (rc != KFAC_OK) return rc;
   KFAC_REQUIRE(wire != nullptr || total == 0, "wire_pack: null wire buffer");
   if (items == 0) return KFAC_OK;
@@ -379,8 +434,8 @@ extern "C" int kfac_wire_unpack_sum_as(int wire_dtype, int n_arrays,
                kMaxWires);
   std::vector<WireArray> tab;
   long long total = 0, items = 0;
-  int rc = build_table(n_arrays, arrays, nelems, tri_dim, select, false, tab,
-                       total, items);
+  int rc = build_table(n_arrays, arrays, nelems, tri_dim, select, false, false,
+                       tab, total, items);
   if (rc != KFAC_OK) return rc;
   WireSources srcs;
   srcs.n = n_wires;

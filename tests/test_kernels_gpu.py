@@ -819,6 +819,34 @@ def test_wire_pack_unpack_bit_exact(ops):
         assert rel(host(o), 0.5 * a + 0.5) < 1e-6
 
 
+@pytest.mark.parametrize('skew', [0, 1, 3])
+@pytest.mark.parametrize('wdt', [torch.float32, torch.float16,
+                                 torch.bfloat16])
+def test_wire_pack_runs(ops, wdt, skew):
+    """Runs of 8192 wire elements written in 16-byte words: triangles and
+    plain arrays shorter than a word, one run long give or take an element,
+    and several runs long, from wires that start inside a word.  Exact."""
+    sizes = [(127, True), (1, True), (128, True), (2, True), (3, True),
+             (130, True), (8191, False), (8192, False), (8193, False),
+             (5, False), (257, True), (20001, False)]
+    g = torch.Generator(device='cuda').manual_seed(3)
+    arrs = [torch.randn((n, n) if t else (n,), generator=g, device='cuda')
+            for n, t in sizes]
+    tri = [t for _, t in sizes]
+    select = [i % 5 != 4 for i in range(len(sizes))]
+    n = ops.wire_nelems(arrs, tri)
+    parts = []
+    for a, t, s in zip(arrs, tri, select):
+        m = a.shape[0]
+        w = a[tuple(torch.tril_indices(m, m, device='cuda'))] if t else a
+        parts.append(w if s else torch.zeros_like(w))
+    buf = torch.full((n + skew + 1,), 7.0, device='cuda', dtype=wdt)
+    ops.wire_pack(arrs, tri, buf[skew:skew + n], select=select,
+                  zero_skipped=True)
+    assert torch.equal(buf[skew:skew + n], torch.cat(parts).to(wdt))
+    assert (buf[:skew] == 7).all() and (buf[skew + n:] == 7).all()
+
+
 @pytest.mark.parametrize('wdt', [torch.float16, torch.bfloat16])
 def test_wire_reduced_precision(ops, wdt):
     """A 16-bit wire buffer holds each value rounded to the wire type (the
