@@ -823,10 +823,12 @@ struct ReduceItem {     // one output tile whose split partials are summed
 // device memory, so the call neither allocates nor copies one).
 __global__ void __launch_bounds__(256)
 tc_reduce_kernel(const ReduceItem* __restrict__ items,
-                 const __grid_constant__ ReduceItem single) {
+                 const __grid_constant__ ReduceItem single, int chunk) {
   // Four lanes share one output element: lane q sums the splits
   // q, q+4, q+8, ... (always in that order), then the four sums are added in
-  // a fixed tree, so the result does not depend on scheduling.
+  // a fixed tree, so the result does not depend on scheduling.  Bound by the
+  // latency of its loads: a block takes `chunk` elements of its tile, 64 while
+  // that leaves SMs idle (100 352 x 64, 196 splits: 248 us with 1024).
   ReduceItem it = items != nullptr ? items[blockIdx.x] : single;
   if (items == nullptr) {
     it.tile = (int)blockIdx.x;
@@ -840,8 +842,8 @@ tc_reduce_kernel(const ReduceItem* __restrict__ items,
   const int cols = min(min(TC_BN, d - n0), m0 + TC_BM - n0);
   const int q = threadIdx.x & 3;
   const int total = rows * cols;
-  for (int e = blockIdx.y * 1024 + (threadIdx.x >> 2);
-       e < min(total, (int)(blockIdx.y + 1) * 1024); e += 64) {
+  for (int e = blockIdx.y * chunk + (threadIdx.x >> 2);
+       e < min(total, (int)(blockIdx.y + 1) * chunk); e += 64) {
     const int r = e / cols, c = e - r * cols;
     const float* p = it.partial + r * TC_BN + c;
     // (eight loads in flight: a narrow factor has hundreds of splits)
@@ -1314,14 +1316,22 @@ static int run_factor_group_pair(int count, const FactorJob* jobs,
                                 cudaMemcpyHostToDevice, stream));
     }
     int dmax = 0;
-    for (const ReduceItem& it : reduces) dmax = it.d > dmax ? it.d : dmax;
+    long long elems = 0;
+    for (const ReduceItem& it : reduces) {
+      dmax = it.d > dmax ? it.d : dmax;
+      elems += (long long)std::min(it.d, TC_BM) * std::min(it.d, TC_BN);
+    }
+    // eight blocks of 256 threads on every SM, in multiples of 64 elements
+    const long long per = elems / (8ll * sm_count());
+    const int chunk =
+        (int)std::min(1024ll, std::max(64ll, (per + 63) / 64 * 64));
     const int rmax = dmax < TC_BM ? dmax : TC_BM;
     const int cmax = dmax < TC_BN ? dmax : TC_BN;
-    dim3 rgrid((unsigned)reduces.size(), (rmax * cmax + 1023) / 1024);
+    dim3 rgrid((unsigned)reduces.size(), (rmax * cmax + chunk - 1) / chunk);
     // a lone factor: its items are consecutive tiles of one output, passed
     // by value (reduces[0] is tile 0)
     tc_reduce_kernel<<<rgrid, 256, 0, stream>>>(
-        static_cast<const ReduceItem*>(dev), reduces[0]);
+        static_cast<const ReduceItem*>(dev), reduces[0], chunk);
     KFAC_LAUNCH_CHECK("tc_reduce_kernel");
   }
   return KFAC_OK;
