@@ -119,98 +119,66 @@ __device__ __forceinline__ int find_array(const int* s_begin, int n_arrays,
 }
 
 // Packing walks the wire: a work item is a run of kChunk wire elements of one
-// array, from one 16-byte boundary to another, and a thread writes whole words
-// (whose elements may lie in two rows of a triangle).  Bound by HBM.  With
-// 64 x 64 tiles of the triangle, whose rows start anywhere in the wire, every
-// 256-byte store began and ended inside a sector: ResNet-50 in fp32 221 us, now
-// 151 us, 6.1 TB/s.  Eight elements in flight in eight blocks per SM; sixteen
-// in four blocks take 187 us, the thread's own latency is then the bound.
+// array, from one 128-byte line to another; a warp writes 32 of them at a time
+// and a thread has kPackU loads in flight, stepping through the triangle from
+// one to the next.  Bound by HBM.  With 64 x 64 tiles of the triangle, whose
+// rows start anywhere in the wire, every 256-byte store began and ended inside a
+// sector.  ResNet-50 in fp32: 221 us in tiles, 149 us now (4.1 TB/s of bytes
+// read and written; dirty lines of the kernel before are written back beside).
+// 16 loads in flight take 158 us, 16-byte words per thread the same 151 us.
+static const int kPackU = 8;
+
 template <typename W>
 __global__ void __launch_bounds__(256, kBlocksPerSm)
 wire_pack_kernel(const WireArray* __restrict__ arrs, int n_arrays,
                  int total_items, W* __restrict__ wire) {
-  constexpr int V = 16 / sizeof(W);
-  constexpr int U = 8 / V;             // words in flight
+  constexpr int kLine = 128 / sizeof(W);
   __shared__ int s_begin[kTabCap];
   load_item_table(arrs, n_arrays, s_begin);
-  // elements from the last 16-byte boundary to the wire's start
-  const int skew = (int)((reinterpret_cast<uintptr_t>(wire) / sizeof(W)) % V);
+  // elements from the last line boundary to the wire's start
+  const int skew =
+      (int)((reinterpret_cast<uintptr_t>(wire) / sizeof(W)) % kLine);
   for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
     const WireArray a = arrs[find_array(s_begin, n_arrays, item)];
-    // runs begin at a word; the array's own first and last word may be shared
-    // with its neighbours
+    // (the first run of an array begins in its predecessor's last line)
     const long long w0 = (long long)(item - (int)a.item_begin) * kChunk -
-                         (a.wire_off + skew) % V;
+                         (a.wire_off + skew) % kLine;
     const int lo = (int)max(0ll, -w0);
     const int n = (int)min((long long)kChunk, a.wire_n - w0);
-    const float* __restrict__ src = a.ptr;
+    const float* __restrict__ src = a.select ? a.ptr : nullptr;
     const int d = a.tri;
     W* __restrict__ dst = wire + a.wire_off + w0;
-    for (int k0 = V * (int)threadIdx.x; k0 < n; k0 += 256 * V * U) {
-      float v[U][V];
+    int k = threadIdx.x;
+    // element w0 + k of the triangle: row r, column c (r = 0, c < 0 before it)
+    int r = 0, c = 0;
+    if (d > 0) {
+      const long long w = w0 + k;
+      if (w > 0) {
+        r = (int)((sqrtf(8.f * (float)w + 1.f) - 1.f) * 0.5f);
+        while ((long long)(r + 1) * (r + 2) / 2 <= w) ++r;
+        while ((long long)r * (r + 1) / 2 > w) --r;
+      }
+      c = (int)(w - (long long)r * (r + 1) / 2);
+    }
+    for (; k < n; k += 256 * kPackU) {
+      float v[kPackU];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int k = k0 + 256 * V * u;
-        if (k < lo || k + V > n) continue;     // see below
-        if (!a.select) {
-#pragma unroll
-          for (int e = 0; e < V; ++e) v[u][e] = 0.f;
-          continue;
-        }
-        const float* p;
-        if (d > 0) {
-          const long long w = w0 + k;
-          int r = (int)((sqrtf(8.f * (float)w + 1.f) - 1.f) * 0.5f);
-          while ((long long)(r + 1) * (r + 2) / 2 <= w) ++r;
-          while ((long long)r * (r + 1) / 2 > w) --r;
-          const int c = (int)(w - (long long)r * (r + 1) / 2);
-          p = src + (long long)r * d + c;
-          if (r + 1 - c < V) {
-            // two or more rows
-            const float* q = p;
-            int m = r + 1 - c, row = r;
-#pragma unroll
-            for (int e = 0; e < V; ++e) {
-              v[u][e] = *q++;
-              if (--m == 0) {
-                ++row;
-                q = src + (long long)row * d;
-                m = row + 1;
-              }
-            }
-            continue;
+      for (int u = 0; u < kPackU; ++u) {
+        const int at = k + 256 * u;
+        v[u] = 0.f;
+        if (src != nullptr && at >= lo && at < n)
+          v[u] = d > 0 ? src[(long long)r * d + c] : src[w0 + at];
+        c += 256;
+        if (d > 0)
+          while (c > r) {
+            c -= r + 1;
+            ++r;
           }
-        } else {
-          p = src + w0 + k;
-        }
-#pragma unroll
-        for (int e = 0; e < V; ++e) v[u][e] = p[e];
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int k = k0 + 256 * V * u;
-        if (k >= n) break;
-        if (k >= lo && k + V <= n) {
-          union { W w[V]; uint4 q; } out;
-#pragma unroll
-          for (int e = 0; e < V; ++e) out.w[e] = to_wire<W>(v[u][e]);
-          *reinterpret_cast<uint4*>(dst + k) = out.q;
-          continue;
-        }
-        for (int e = max(0, lo - k); e < V && k + e < n; ++e) {
-          float x = 0.f;
-          if (a.select) {
-            const long long w = w0 + k + e;
-            if (d > 0) {
-              int r, c;
-              tri_index(w, r, c);
-              x = src[(long long)r * d + c];
-            } else {
-              x = src[w];
-            }
-          }
-          dst[k + e] = to_wire<W>(x);
-        }
+      for (int u = 0; u < kPackU; ++u) {
+        const int at = k + 256 * u;
+        if (at >= lo && at < n) dst[at] = to_wire<W>(v[u]);
       }
     }
   }
@@ -340,7 +308,9 @@ static int build_table(int n_arrays, float* const* arrays,
     total += a.wire_n;
     a.item_begin = items;
     if (pack) {
-      if (a.select || skipped_get_items) items += (a.wire_n + 7 + kChunk - 1) / kChunk;
+      // (runs begin at a 128-byte line: up to 63 elements before the array)
+      if (a.select || skipped_get_items)
+        items += (a.wire_n + 63 + kChunk - 1) / kChunk;
     } else if (a.select && a.tri > 0) {
       long long t = (a.tri + kTile - 1) / kTile;
       items += t * (t + 1) / 2;

@@ -823,9 +823,9 @@ def test_wire_pack_unpack_bit_exact(ops):
 @pytest.mark.parametrize('wdt', [torch.float32, torch.float16,
                                  torch.bfloat16])
 def test_wire_pack_runs(ops, wdt, skew):
-    """Runs of 8192 wire elements written in 16-byte words: triangles and
-    plain arrays shorter than a word, one run long give or take an element,
-    and several runs long, from wires that start inside a word.  Exact."""
+    """Runs of 8192 wire elements written by whole lines: triangles and
+    plain arrays shorter than a line, one run long give or take an element,
+    and several runs long, from wires that start inside a line.  Exact."""
     sizes = [(127, True), (1, True), (128, True), (2, True), (3, True),
              (130, True), (8191, False), (8192, False), (8193, False),
              (5, False), (257, True), (20001, False)]
