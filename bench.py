@@ -72,7 +72,8 @@ WORKLOADS = {
 # bench scales them by the algorithmic work of its own launches.
 # stage: (case, measured bytes, algorithmic bytes, algorithmic flops)
 TRAFFIC_CASES = {
-    'factor': ('conv3x3_c256_hw14 (tc_pair_kernel)', 33.9e6, 29.4e6,
+    'factor': ('conv3x3_c256_hw14 (staging, gram_kernel, expansion)',
+               76.5e6, 29.4e6,
                32 * 14 * 14 * 2304 * 2305.0),
     'inverse': None,
     'precondition': None,
@@ -897,12 +898,12 @@ def time_alone(torch, fn, reps):
 
 
 STAGE_KERNELS = {
-    'factor': 'tc_pair_kernel (grouped strided and im2col launches over all '
-              'factors, plus staging copies and the split reduce)',
-    'inverse': 'tc_gemm_kernel + chol_diag_kernel (batched blocked Cholesky, '
+    'factor': 'gram_kernel + direct_kernel + tc_pair_kernel (grouped launches '
+              'over all factors, plus staging and the split reductions)',
+    'inverse': 'tc_tile_kernel + chol_diag_kernel (batched blocked Cholesky, '
                'triangular inverse and symmetric product of every factor, '
                'three size classes on three streams)',
-    'precondition': 'tc_gemm_kernel (two grouped launches over all layers, '
+    'precondition': 'tc_tile_kernel (two grouped launches over all layers, '
                     'update fused)'}
 
 
