@@ -6,7 +6,7 @@
 // single TF32 pass misses the 1e-4 bound on large factors).
 //
 // One CTA owns a 128 x TN tile.  Producer warps load the operands from global
-// memory with 16-byte loads, one or two 32-k blocks ahead in registers, split them
+// memory with 16-byte loads, one to three 32-k blocks ahead in registers, split them
 // and write the K-major, 128-byte-swizzled shared-memory layout that the MMA
 // descriptors expect; one more warp issues the MMAs.  The epilogue moves
 // 32 x 32 pieces of the accumulator TMEM -> registers -> shared memory ->
@@ -21,7 +21,10 @@
 // is waited for, and TN = 128 (half the work per CTA, twice the CTAs) is used
 // while 128 x 256 tiles would leave SMs idle.  One tile with K = 128: 20 us with
 // an update of C and 12.4 us without before, 13.5 and 11 us now; a 2304-row
-// inverse 888 -> 791 us, 14 pairs of odd sides 541 -> 447 us.
+// inverse 888 -> 791 us, 14 pairs of odd sides 541 -> 447 us.  The 128-wide tile
+// has 16 producer warps of one unit and three blocks in flight: with eight warps
+// of two units and two blocks a k-block took the 1.3 us of a 256-wide one (144
+// tiles with K = 4608 190 -> 125 us; 2304-row inverse 796 -> 759 us).
 //
 // Every barrier wait is bounded; a wait that runs out raises a status word
 // instead of hanging.
@@ -41,7 +44,8 @@ static __device__ int g_tile_status = 0;
 
 template <int TN>
 struct TileMap {
-  static constexpr int kProducers = TN == 256 ? 384 : 256;
+  static constexpr int kProducers = TN == 256 ? 384 : 512;
+  static constexpr bool kTwo = TN == 256;         // units per producer thread
   static constexpr int kWarps = kProducers / 32;
   static constexpr int kThreads = kProducers + 32;
   static constexpr int kStages = TN == 256 ? 2 : 3;
@@ -472,7 +476,7 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
 
   if (warp < Map::kWarps) {
     // ===================== producers =====================
-    // units 0 .. 7 of 32 threads: A rows, then the B rows; two per thread
+    // units 0 .. 7 of 32 threads: A rows, then the B rows
     const bool a0 = warp < 8;
     const Operand& op0 = a0 ? g.A : g.B;
     const Operand& op1 = g.B;
@@ -480,12 +484,13 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
     tile_unit_setup<VEC>(op0, a0 ? m0 : n0, a0 ? warp : warp - 8, lane, kbeg,
                     a0 ? (share_ab ? 0 : m_valid) : n_valid,
                     a0 ? 0 : Map::kABytes, u0);
-    tile_unit_setup<VEC>(op1, n0, warp + Map::kWarps - 8, lane, kbeg, n_valid,
-                    Map::kABytes, u1);
+    if (Map::kTwo)
+      tile_unit_setup<VEC>(op1, n0, warp + Map::kWarps - 8, lane, kbeg, n_valid,
+                      Map::kABytes, u1);
     const unsigned base = smem_u32(smem);
     auto load = [&](float4* v) {
       tile_unit_load<VEC>(op0, u0, kend, v);
-      tile_unit_load<VEC>(op1, u1, kend, v + 4);
+      if (Map::kTwo) tile_unit_load<VEC>(op1, u1, kend, v + 4);
     };
     auto store = [&](int kb, const float4* v) {
       const int s = kb % Map::kStages;
@@ -495,23 +500,24 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
         return false;
       const unsigned st = base + s * Map::kStage;
       tile_unit_store<VEC>(u0, st, Map::kLo, v);
-      tile_unit_store<VEC>(u1, st, Map::kLo, v + 4);
+      if (Map::kTwo) tile_unit_store<VEC>(u1, st, Map::kLo, v + 4);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl->full[s]);
       return true;
     };
-    float4 va[8];
+    constexpr int kVals = Map::kTwo ? 8 : 4;
+    float4 va[kVals];
     if (nkb > 0) load(va);
-    if (TN == 256 || !VEC) {
+    if (TN == 256) {
       // one block ahead: the MMAs of a block take longer than a trip to L2
 #pragma unroll 1
       for (int kb = 0; kb < nkb; ++kb) {
         if (!store(kb, va)) break;
         if (kb + 1 < nkb) load(va);
       }
-    } else {
-      float4 vb[8];
+    } else if (!VEC) {
+      float4 vb[kVals];
       if (nkb > 1) load(vb);
 #pragma unroll 1
       for (int kb = 0; kb < nkb; kb += 2) {
@@ -520,6 +526,23 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
         if (kb + 1 < nkb) {
           if (!store(kb + 1, vb)) break;
           if (kb + 3 < nkb) load(vb);
+        }
+      }
+    } else {
+      float4 vb[kVals], vc[kVals];
+      if (nkb > 1) load(vb);
+      if (nkb > 2) load(vc);
+#pragma unroll 1
+      for (int kb = 0; kb < nkb; kb += 3) {
+        if (!store(kb, va)) break;
+        if (kb + 3 < nkb) load(va);
+        if (kb + 1 < nkb) {
+          if (!store(kb + 1, vb)) break;
+          if (kb + 4 < nkb) load(vb);
+        }
+        if (kb + 2 < nkb) {
+          if (!store(kb + 2, vc)) break;
+          if (kb + 5 < nkb) load(vc);
         }
       }
     }
