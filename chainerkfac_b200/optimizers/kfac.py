@@ -109,6 +109,8 @@ class KFACHook(object):
             if me is None or not me._active or not output.requires_grad or \
                     not torch.is_grad_enabled():
                 return
+            if module is not link.module:
+                return      # a deep copy of the layer, which took the hook along
             x = inputs[0]
             if x.requires_grad:
                 x = x.detach()

@@ -53,6 +53,36 @@ def test_public_interface_and_defaults():
         ck.KFAC(use_cholesky=False).setup(small_model())
 
 
+def run_hooked(opt, call):
+    """Forward and backward of ``call`` inside the optimizer's hooks, with
+    the blocks only remembering their arguments."""
+    for fb in opt.fblocks:
+        fb.deferred = True
+    with opt.kfhook:
+        call().sum().backward()
+
+
+def test_hooks_do_not_follow_copies_of_the_model():
+    """A copy of the model made after the first step (a teacher, an average)
+    that runs inside the loss leaves the blocks of the original alone."""
+    import copy
+    import chainerkfac_b200 as ck
+    model = nn.Sequential(nn.Linear(3, 4), nn.Linear(4, 2))
+    opt = ck.KFAC().setup(model)
+    x = torch.randn(5, 3)
+    run_hooked(opt, lambda: model(x))
+    other = copy.deepcopy(model)
+    run_hooked(opt, lambda: model(x) + 2 * other(x + 1))
+    fb = opt.fblocks[0]
+    assert fb._pending_A[0].data_ptr() == x.data_ptr()
+    assert torch.equal(opt.fblocks[1]._pending_G[1][0], torch.ones(5, 2))
+    for fb in opt.fblocks:
+        fb._pending_A = fb._pending_G = None
+    run_hooked(opt, lambda: other(x))
+    assert all(fb._pending_A is None and fb._pending_G is None
+               for fb in opt.fblocks)
+
+
 def test_bn_low_rank_history_weights_follow_the_running_average():
     """Host logic of the low-rank form of a BatchNormalization block: which
     blocks take it, how the history ring rotates, and that the slot weights
