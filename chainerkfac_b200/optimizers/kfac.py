@@ -147,8 +147,16 @@ class KFACHook(object):
 
     # The module hooks stay registered between ``with`` blocks (registering
     # and removing them cost 7 us per layer and step) and do nothing outside.
+    # They are made anew when one is no longer the last hook of its module: the
+    # blocks see what the layer hands on behind a program's own hooks.
+    def _registered(self):
+        return len(self._handles) == len(self.fblocks) and all(
+            mine is fb and next(reversed(fb.link.module._forward_hooks),
+                                None) == handle.id
+            for (mine, handle), fb in zip(self._handles, self.fblocks))
+
     def __enter__(self):
-        if [fb for fb, _ in self._handles] != list(self.fblocks):
+        if not self._registered():
             self._remove()
             self._handles = [
                 (fb, fb.link.module.register_forward_hook(

@@ -83,6 +83,25 @@ def test_hooks_do_not_follow_copies_of_the_model():
                for fb in opt.fblocks)
 
 
+def test_hooks_run_behind_the_hooks_a_program_registers_meanwhile():
+    """A block sees the layer's output and its gradient behind hooks that were
+    registered after the first step, and outlives a program that clears the
+    layer's hooks."""
+    import chainerkfac_b200 as ck
+    layer = nn.Linear(3, 4)
+    opt = ck.KFAC().setup(nn.Sequential(layer))
+    fb, x = opt.fblocks[0], torch.randn(5, 3)
+    run_hooked(opt, lambda: layer(x))
+    layer.register_forward_hook(lambda module, inputs, output: output * 3)
+    fb._pending_G = None
+    run_hooked(opt, lambda: 2 * layer(x))
+    assert torch.equal(fb._pending_G[1][0], torch.full((5, 4), 2.0))
+    layer._forward_hooks.clear()
+    fb._pending_A = fb._pending_G = None
+    run_hooked(opt, lambda: layer(x))
+    assert fb._pending_A is not None and fb._pending_G is not None
+
+
 def test_bn_low_rank_history_weights_follow_the_running_average():
     """Host logic of the low-rank form of a BatchNormalization block: which
     blocks take it, how the history ring rotates, and that the slot weights
