@@ -99,6 +99,11 @@ class KFACHook(object):
             if self.on_backward is not None:
                 self.on_backward(fblock)
 
+    def _direct(self):
+        return type(self) is KFACHook and \
+            'forward_postprocess' not in self.__dict__ and \
+            'backward_preprocess' not in self.__dict__
+
     def _make_forward_hook(self, fblock):
         link = fblock.link
         is_bn = isinstance(link, L.BatchNormalization)
@@ -124,24 +129,23 @@ class KFACHook(object):
                 in_data = (x, link.W.data, link.b.data)
             func = fblock.funcclass()
             # the block this hook was made for; an overridden protocol method
-            # is called by its name
-            direct = type(me) is KFACHook
-            if direct:
+            # (of a subclass, or put on the hook object) is called by its name
+            if not me._direct():
+                me.forward_postprocess(func, in_data)
+            elif fblock.is_mine(func, in_data):
                 fblock.forward_postprocess(func, in_data)
                 if me.on_forward is not None:
                     me.on_forward(fblock)
-            else:
-                me.forward_postprocess(func, in_data)
 
             def backward(g):
                 if g.requires_grad:
                     g = g.detach()
-                if direct:
+                if not me._direct():
+                    me.backward_preprocess(func, in_data, (g,))
+                elif fblock.is_mine(func, in_data, (g,)):
                     fblock.backward_preprocess(func, in_data, (g,))
                     if me.on_backward is not None:
                         me.on_backward(fblock)
-                else:
-                    me.backward_preprocess(func, in_data, (g,))
             output.register_hook(backward)
         return hook
 

@@ -102,6 +102,27 @@ def test_hooks_run_behind_the_hooks_a_program_registers_meanwhile():
     assert fb._pending_A is not None and fb._pending_G is not None
 
 
+def test_hooks_call_overridden_protocol_methods():
+    """Protocol methods replaced on the hook object and a block's own
+    ``is_mine`` are asked, as by a subclass of the hook."""
+    import chainerkfac_b200 as ck
+    model = nn.Sequential(nn.Linear(3, 4), nn.Linear(4, 2))
+    opt = ck.KFAC().setup(model)
+    x = torch.randn(5, 3)
+    opt.fblocks[1].is_mine = lambda func, in_data, out_grad_data=None: False
+    run_hooked(opt, lambda: model(x))
+    assert opt.fblocks[0]._pending_A is not None
+    assert getattr(opt.fblocks[1], '_pending_A', None) is None
+    seen = []
+    opt.kfhook.forward_postprocess = \
+        lambda func, in_data: seen.append(in_data[0].shape)
+    opt.kfhook.backward_preprocess = \
+        lambda func, in_data, out_grad_data: seen.append(
+            out_grad_data[0].shape)
+    run_hooked(opt, lambda: model(x))
+    assert [tuple(s) for s in seen] == [(5, 3), (5, 4), (5, 2), (5, 4)]
+
+
 def test_bn_low_rank_history_weights_follow_the_running_average():
     """Host logic of the low-rank form of a BatchNormalization block: which
     blocks take it, how the history ring rotates, and that the slot weights
