@@ -498,12 +498,17 @@ def class_bounds():
 
 
 class _PlanDiag(object):
-    def __init__(self, plans):
-        self._plans, self._where = plans.plans, plans.where
+    """The values of an InversePlanSet's ``diag``, each read from its plan when
+    it is asked for; a slice is a view that starts at another factor."""
+
+    def __init__(self, plans, start=0):
+        self._plans, self._start = plans, start
 
     def __getitem__(self, i):
-        plan, j = self._where[i]
-        return self._plans[plan].diag[j]
+        if isinstance(i, slice):
+            return _PlanDiag(self._plans, self._start + (i.start or 0))
+        plan, j = self._plans.where[self._start + i]
+        return self._plans.plans[plan].diag[j]
 
 
 class InversePlanSet(object):

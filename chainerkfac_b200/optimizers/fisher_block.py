@@ -128,16 +128,18 @@ class FisherBlock(object):
         self._plan.run(self.damping, self._pi_type == PI_TYPE_TRACENORM)
         self.set_diag_vals(self._plan.diag)
 
-    # The values added to the diagonals by the last damped inverse are read
-    # when somebody asks for them: ``diag[start + j]`` for factor j.
+    # The values added to the diagonals by the last damped inverse are read when
+    # somebody asks for them, into tensors of their own: the plan writes the
+    # next step's over its copy.
     _diag_src = None
 
-    def set_diag_vals(self, diag, start=0):
-        self._diag_src = (diag, start)
+    def set_diag_vals(self, diag):
+        self._diag_src = diag
 
     def diag_val(self, j):
-        diag, start = self._diag_src
-        return diag[start + j]
+        if self._diag_src is None:
+            raise AttributeError('no damped inverse of %s yet' % self._linkname)
+        return self._diag_src[j].clone()
 
     def update_kfgrads(self):
         raise NotImplementedError

@@ -896,7 +896,7 @@ class KFAC(_base.GradientMethod):
             for fb in group:
                 n = len(fb.plan_factors())
                 if n:
-                    fb.set_diag_vals(diag, k)
+                    fb.set_diag_vals(diag[k:k + n])
                 k += n
         conn = [fb for fb in fblocks
                 if isinstance(fb, FB.FisherBlockConnection) and

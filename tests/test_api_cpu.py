@@ -123,6 +123,34 @@ def test_hooks_call_overridden_protocol_methods():
     assert [tuple(s) for s in seen] == [(5, 3), (5, 4), (5, 2), (5, 4)]
 
 
+def test_damping_values_are_those_of_their_step():
+    """Values added to the diagonals: none before the first inverse; read later,
+    they are the block's own in the order of the plans; a value read in one step
+    does not change with the next.  Blocks that override ``set_diag_vals`` get
+    one sequence of their values."""
+    import types
+    import chainerkfac_b200 as ck
+    from chainerkfac_b200 import ops
+    opt = ck.KFAC().setup(small_model())
+    conv, bn, fc = opt.fblocks
+    assert not hasattr(conv, 'diag_val_forward')
+    assert not hasattr(bn, 'diag_val_backward')
+    # factors 0, 1 (conv), 2 (bn), 3, 4 (fc) in two plans
+    plans = [types.SimpleNamespace(diag=torch.tensor([3.0, 4.0])),
+             types.SimpleNamespace(diag=torch.tensor([0.0, 1.0, 2.0]))]
+    where = {0: (1, 0), 1: (1, 1), 2: (1, 2), 3: (0, 0), 4: (0, 1)}
+    diag = ops._PlanDiag(types.SimpleNamespace(plans=plans, where=where))
+    got = []
+    fc.set_diag_vals = lambda diag: got.extend([diag[0], diag[1]])
+    for fb, k, n in ((conv, 0, 2), (bn, 2, 1), (fc, 3, 2)):
+        fb.set_diag_vals(diag[k:k + n])
+    assert (float(got[0]), float(got[1])) == (3.0, 4.0)
+    first = conv.diag_val_forward, conv.diag_val_backward, bn.diag_val_backward
+    plans[1].diag += 10.0             # the next step's inverses
+    assert [float(v) for v in first] == [0.0, 1.0, 2.0]
+    assert float(conv.diag_val_backward) == 11.0
+
+
 def test_bn_low_rank_history_weights_follow_the_running_average():
     """Host logic of the low-rank form of a BatchNormalization block: which
     blocks take it, how the history ring rotates, and that the slot weights
