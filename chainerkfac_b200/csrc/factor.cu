@@ -185,14 +185,17 @@ static int run_factor(const Operand& X, long long rows, int d, float alpha,
 // ------------------------------------------------------------ BN sample grads
 // Per-sample gradients of all BatchNormalization layers of a step.  The work
 // is HBM-bound (x and gy read once, 8 bytes per activation), so both tensors
-// are read in ONE pass: sums of x and x^2 in double precision for the batch
-// statistics, and sums of g and g (x - k) per (sample, channel), k the
-// channel's first element.  The finishing launch adds up the statistics and
-// turns the second sum into sum g xhat = istd (sum g (x - k) - (mean - k)
-// sum g); k lies within the spread of x, so nothing cancels.  (A pass for the
-// statistics and a second one for the gradients, with one 4-byte load in
-// flight per thread, took 1002 us for the 53 layers of ResNet-50 at 32 images
-// in NCHW and 3400 us channels-last; now 634 us and 557 us, 5.1 TB/s.)
+// are read in ONE pass: sums of x, x^2, g and g x per (sample, channel), all
+// in double precision.  They leave as sums around the sample's own mean m,
+// a = sum g x - m sum g; the finishing launch adds up the statistics and forms
+// sum g xhat = istd (a + (m - mean) sum g).  a is a difference of doubles, and
+// m lies within sqrt(n) spreads of the mean however uneven the image is, so
+// that the two fp32 terms cancel by no more than that.  (Shifting by one element
+// instead lost sqrt(n hw) spreads of accuracy where that element was the odd
+// one out.)  For the 53 layers of ResNet-50 at 32 images, us: shifted by one
+// element, fp32 products 648 (NCHW) and 572 (channels-last); double products of
+// every element 687 and 618; products around the first of four elements
+// (bn_take4) 541 and 581 (5.3 and 4.9 TB/s).
 struct BnItem {
   const float* x;
   const float* gy;
@@ -224,15 +227,32 @@ __device__ __forceinline__ int bn_find_item(const int* begins, int n, int b) {
 
 struct BnSum {
   double s, ss;      // of x, x^2
-  float a, g;        // of g (x - k), g
+  double a, g;       // of g x, g
 };
 
-__device__ __forceinline__ void bn_take(BnSum& t, float x, float g, float k) {
-  const double v = x;
+__device__ __forceinline__ void bn_take(BnSum& t, float x, float g) {
+  const double v = x, w = g;
   t.s += v;
   t.ss = fma(v, v, t.ss);
-  t.a += g * (x - k);
-  t.g += g;
+  t.a = fma(w, v, t.a);
+  t.g += w;
+}
+
+// Four elements: g x around the first of them in fp32 (its roundings are of the
+// spread within the four, not of the mean), four conversions less.
+__device__ __forceinline__ void bn_take4(BnSum& t, const float x[4],
+                                         const float g[4]) {
+  const float k = x[0];
+  const float a = fmaf(g[1], x[1] - k, fmaf(g[2], x[2] - k, g[3] * (x[3] - k)));
+  const double w = (g[0] + g[1]) + (g[2] + g[3]);
+  t.a = fma(w, (double)k, t.a + (double)a);
+  t.g += w;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double v = x[i];
+    t.s += v;
+    t.ss = fma(v, v, t.ss);
+  }
 }
 
 __device__ __forceinline__ void bn_add(BnSum& t, const BnSum& u) {
@@ -258,8 +278,8 @@ __device__ __forceinline__ void bn_leave(const BnItem& it, int smp, int ch,
   part[0] = t.s;
   part[it.c] = t.ss;
   float* o = it.out + (long long)smp * 2 * it.c + ch;
-  o[0] = t.a;
-  o[it.c] = t.g;
+  o[0] = (float)(t.a - t.s / it.hw * t.g);
+  o[it.c] = (float)t.g;
 }
 
 // (sample, channel) plane: `lanes` threads each (a power of two, or all 256).
@@ -271,9 +291,8 @@ __device__ __forceinline__ void bn_sum_planes(const BnItem& it, int b,
   const long long plane = (long long)b * (256 / lanes) + tid / lanes;
   const bool on = plane < planes;
   const int smp = (int)(plane / it.c), ch = (int)(plane - (long long)smp * it.c);
-  BnSum t = {0.0, 0.0, 0.f, 0.f};
+  BnSum t = {0.0, 0.0, 0.0, 0.0};
   if (on) {
-    const float k = __ldg(it.x + (long long)ch * it.hw);
     const float* px = it.x + plane * it.hw;
     const float* pg = it.gy + plane * it.hw;
     const int first = tid & (lanes - 1);
@@ -284,15 +303,14 @@ __device__ __forceinline__ void bn_sum_planes(const BnItem& it, int b,
 #pragma unroll 2
       for (int i = first; i < n4; i += lanes) {
         const float4 x = __ldcs(x4 + i), g = __ldcs(g4 + i);
-        bn_take(t, x.x, g.x, k);
-        bn_take(t, x.y, g.y, k);
-        bn_take(t, x.z, g.z, k);
-        bn_take(t, x.w, g.w, k);
+        const float xs[4] = {x.x, x.y, x.z, x.w};
+        const float gs[4] = {g.x, g.y, g.z, g.w};
+        bn_take4(t, xs, gs);
       }
     } else {
 #pragma unroll 4
       for (int i = first; i < it.hw; i += lanes)
-        bn_take(t, __ldcs(px + i), __ldcs(pg + i), k);
+        bn_take(t, __ldcs(px + i), __ldcs(pg + i));
     }
   }
   for (int o = min(lanes, 32) >> 1; o > 0; o >>= 1) bn_shuffle_add(t, o);
@@ -318,23 +336,35 @@ __device__ __forceinline__ void bn_sum_last4(const BnItem& it, int b,
   const int ch = c0 + 4 * sub;
   BnSum t[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) t[i] = {0.0, 0.0, 0.f, 0.f};
+  for (int i = 0; i < 4; ++i) t[i] = {0.0, 0.0, 0.0, 0.0};
   if (ch < it.c) {
-    const float4 k = __ldg(reinterpret_cast<const float4*>(it.x + ch));
     const long long o = (long long)smp * it.hw * it.c + ch;
     const float* px = it.x + o;
     const float* pg = it.gy + o;
     const int step = 256 / lanes;
-#pragma unroll 4
-    for (int q = tid / lanes; q < it.hw; q += step) {
+    int q = tid / lanes;
+    for (; q + 3 * step < it.hw; q += 4 * step) {
+      float x[4][4], g[4][4];          // [channel][pixel]
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const long long at = (long long)(q + k * step) * it.c;
+        const float4 u = __ldcs(reinterpret_cast<const float4*>(px + at));
+        const float4 v = __ldcs(reinterpret_cast<const float4*>(pg + at));
+        x[0][k] = u.x; x[1][k] = u.y; x[2][k] = u.z; x[3][k] = u.w;
+        g[0][k] = v.x; g[1][k] = v.y; g[2][k] = v.z; g[3][k] = v.w;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) bn_take4(t[i], x[i], g[i]);
+    }
+    for (; q < it.hw; q += step) {
       const float4 x =
           __ldcs(reinterpret_cast<const float4*>(px + (long long)q * it.c));
       const float4 g =
           __ldcs(reinterpret_cast<const float4*>(pg + (long long)q * it.c));
-      bn_take(t[0], x.x, g.x, k.x);
-      bn_take(t[1], x.y, g.y, k.y);
-      bn_take(t[2], x.z, g.z, k.z);
-      bn_take(t[3], x.w, g.w, k.w);
+      bn_take(t[0], x.x, g.x);
+      bn_take(t[1], x.y, g.y);
+      bn_take(t[2], x.z, g.z);
+      bn_take(t[3], x.w, g.w);
     }
   }
   for (int o = 16; o >= lanes; o >>= 1)
@@ -359,16 +389,25 @@ __device__ __forceinline__ void bn_sum_last(const BnItem& it, int b,
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int groups = (it.c + 31) >> 5;
   const int smp = b / groups, ch = 32 * (b - smp * groups) + lane;
-  BnSum t = {0.0, 0.0, 0.f, 0.f};
+  BnSum t = {0.0, 0.0, 0.0, 0.0};
   if (ch < it.c) {
-    const float k = __ldg(it.x + ch);
     const long long o = (long long)smp * it.hw * it.c + ch;
     const float* px = it.x + o;
     const float* pg = it.gy + o;
-#pragma unroll 8
-    for (int q = warp; q < it.hw; q += 8)
+    int q = warp;
+    for (; q + 56 < it.hw; q += 64) {
+      float x[8], g[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        x[k] = __ldcs(px + (long long)(q + 8 * k) * it.c);
+        g[k] = __ldcs(pg + (long long)(q + 8 * k) * it.c);
+      }
+      bn_take4(t, x, g);
+      bn_take4(t, x + 4, g + 4);
+    }
+    for (; q < it.hw; q += 8)
       bn_take(t, __ldcs(px + (long long)q * it.c),
-              __ldcs(pg + (long long)q * it.c), k);
+              __ldcs(pg + (long long)q * it.c));
   }
   sh[tid] = t;
   __syncthreads();
@@ -378,7 +417,11 @@ __device__ __forceinline__ void bn_sum_last(const BnItem& it, int b,
   }
 }
 
-__global__ void __launch_bounds__(256, 4)
+// Planes run best at full occupancy (8, 6, 4 blocks per SM: 541, 571, 605 us for
+// the layers above), the four channels of a channels-last thread at 80 registers
+// (4, 3, 2 blocks: 646, 581, 658 us).
+template <bool LAST>
+__global__ void __launch_bounds__(256, LAST ? 3 : 8)
 bn_sums_group_kernel(const BnItem* __restrict__ items, int nitems) {
   __shared__ int s_begin[kBnItemsMax];
   __shared__ BnSum sh[256];
@@ -387,9 +430,9 @@ bn_sums_group_kernel(const BnItem* __restrict__ items, int nitems) {
   __syncthreads();
   const BnItem it = items[bn_find_item(s_begin, nitems, blockIdx.x)];
   const int b = blockIdx.x - it.sum_begin;
-  if (it.mode == kBnPlanes4) bn_sum_planes<true>(it, b, sh);
+  if (!LAST && it.mode == kBnPlanes4) bn_sum_planes<true>(it, b, sh);
+  else if (!LAST) bn_sum_planes<false>(it, b, sh);
   else if (it.mode == kBnLast4) bn_sum_last4(it, b, sh);
-  else if (it.mode == kBnPlanes) bn_sum_planes<false>(it, b, sh);
   else bn_sum_last(it, b, sh);
 }
 
@@ -431,15 +474,13 @@ bn_finish_grads_kernel(const BnItem* __restrict__ items, int nitems) {
   double var = ss / per - mean * mean;
   if (var < 0.0) var = 0.0;
   const float istd = (float)(1.0 / sqrt(var + (double)it.eps));
-  const bool last = it.mode == kBnLast || it.mode == kBnLast4;
-  const float k0 = __ldg(it.x + (last ? ch : (long long)ch * it.hw));
-  const float off = (float)(mean - (double)k0);
   float* o = it.out + ch;
 #pragma unroll 4
   for (int k = warp; k < it.n; k += 8) {
     float* p = o + (long long)k * 2 * it.c;
     const float a = p[0], g = p[it.c];
-    p[0] = it.scale * (istd * (a - off * g));
+    const float off = (float)(part[(long long)k * 2 * it.c] / it.hw - mean);
+    p[0] = it.scale * (istd * (a + off * g));
     p[it.c] = it.scale * g;
   }
   if (warp == 0) {
@@ -916,47 +957,54 @@ extern "C" int kfac_bn_sample_grads_group(int count,
   KFAC_REQUIRE(count <= kBnItemsMax,
                "bn_sample_grads_group: %d layers in one call, at most %d",
                count, kBnItemsMax);
-  std::vector<BnItem> tab(count);
-  long long sb = 0, fb = 0;
-  for (int i = 0; i < count; ++i) {
-    const kfac_bn_item& k = items[i];
-    KFAC_REQUIRE(k.x && k.gy && k.out && k.stats,
-                 "bn_sample_grads_group: null pointer at %d", i);
-    KFAC_REQUIRE(k.n > 0 && k.c > 0 && k.hw > 0 &&
-                     (k.layout == 0 || k.layout == 1),
-                 "bn_sample_grads_group: bad shape or layout at %d", i);
-    BnItem& t = tab[i];
-    t.x = k.x; t.gy = k.gy; t.out = k.out; t.stats = k.stats;
-    t.n = k.n; t.c = k.c; t.hw = k.hw;
-    t.eps = k.eps; t.scale = k.scale;
-    t.sum_begin = (int)sb;
-    t.fin_begin = (int)fb;
-    const bool aligned =
-        ((reinterpret_cast<uintptr_t>(k.x) | reinterpret_cast<uintptr_t>(k.gy)) &
-         15) == 0;
-    if (k.layout == 1 && k.hw > 1) {
-      // 128 bytes of channels per pixel and block; 64 for large images, so
-      // that a batch of few samples still gives blocks enough
-      const bool vec = aligned && k.c % 4 == 0;
-      t.mode = vec ? kBnLast4 : kBnLast;
-      t.lanes = k.hw > 4096 ? 4 : 8;
-      const int width = vec ? 4 * t.lanes : 32;
-      sb += (long long)k.n * ((k.c + width - 1) / width);
-    } else {
-      // about four loads per thread and plane; a whole block only for planes
-      // that keep 256 threads busy as well
-      const bool vec = aligned && k.hw % 4 == 0;
-      t.mode = vec ? kBnPlanes4 : kBnPlanes;
-      const int words = vec ? k.hw / 4 : k.hw;
-      int lanes = 1;
-      while (lanes < 32 && lanes * 4 <= words) lanes *= 2;
-      t.lanes = words >= 1024 ? 256 : lanes;
-      const int planes = 256 / t.lanes;
-      sb += ((long long)k.n * k.c + planes - 1) / planes;
+  // planes first, channels-last behind them: a launch each sums them (their
+  // best occupancies differ), one launch finishes all
+  std::vector<BnItem> tab;
+  long long sb[2] = {0, 0}, fb = 0;
+  int first[3] = {0, 0, count};
+  for (int m = 0; m < 2; ++m) {
+    first[m] = (int)tab.size();
+    for (int i = 0; i < count; ++i) {
+      const kfac_bn_item& k = items[i];
+      KFAC_REQUIRE(k.x && k.gy && k.out && k.stats,
+                   "bn_sample_grads_group: null pointer at %d", i);
+      KFAC_REQUIRE(k.n > 0 && k.c > 0 && k.hw > 0 &&
+                       (k.layout == 0 || k.layout == 1),
+                   "bn_sample_grads_group: bad shape or layout at %d", i);
+      if ((k.layout == 1 && k.hw > 1) != (m == 1)) continue;
+      BnItem t;
+      t.x = k.x; t.gy = k.gy; t.out = k.out; t.stats = k.stats;
+      t.n = k.n; t.c = k.c; t.hw = k.hw;
+      t.eps = k.eps; t.scale = k.scale;
+      t.sum_begin = (int)sb[m];
+      t.fin_begin = (int)fb;
+      const bool aligned = ((reinterpret_cast<uintptr_t>(k.x) |
+                             reinterpret_cast<uintptr_t>(k.gy)) & 15) == 0;
+      if (m == 1) {
+        // 128 bytes of channels per pixel and block; 64 for large images, so
+        // that a batch of few samples still gives blocks enough
+        const bool vec = aligned && k.c % 4 == 0;
+        t.mode = vec ? kBnLast4 : kBnLast;
+        t.lanes = k.hw > 4096 ? 4 : 8;
+        const int width = vec ? 4 * t.lanes : 32;
+        sb[m] += (long long)k.n * ((k.c + width - 1) / width);
+      } else {
+        // about four loads per thread and plane; a whole block only for planes
+        // that keep 256 threads busy as well
+        const bool vec = aligned && k.hw % 4 == 0;
+        t.mode = vec ? kBnPlanes4 : kBnPlanes;
+        const int words = vec ? k.hw / 4 : k.hw;
+        int lanes = 1;
+        while (lanes < 32 && lanes * 4 <= words) lanes *= 2;
+        t.lanes = words >= 1024 ? 256 : lanes;
+        const int planes = 256 / t.lanes;
+        sb[m] += ((long long)k.n * k.c + planes - 1) / planes;
+      }
+      fb += (k.c + 31) / 32;
+      KFAC_REQUIRE(sb[m] < (1ll << 31) && fb < (1ll << 31),
+                   "bn_sample_grads_group: too many blocks");
+      tab.push_back(t);
     }
-    fb += (k.c + 31) / 32;
-    KFAC_REQUIRE(sb < (1ll << 31) && fb < (1ll << 31),
-                 "bn_sample_grads_group: too many blocks");
   }
   void* dev = nullptr;
   int rc = ring_alloc(tab.size() * sizeof(BnItem), &dev);
@@ -964,11 +1012,18 @@ extern "C" int kfac_bn_sample_grads_group(int count,
   cudaStream_t st = (cudaStream_t)stream;
   KFAC_CUDA(cudaMemcpyAsync(dev, tab.data(), tab.size() * sizeof(BnItem),
                             cudaMemcpyHostToDevice, st));
-  bn_sums_group_kernel<<<(int)sb, 256, 0, st>>>(static_cast<BnItem*>(dev),
-                                                count);
-  KFAC_LAUNCH_CHECK("bn_sums_group_kernel");
-  bn_finish_grads_kernel<<<(int)fb, 256, 0, st>>>(static_cast<BnItem*>(dev),
-                                                  count);
+  const BnItem* d_items = static_cast<const BnItem*>(dev);
+  for (int m = 0; m < 2; ++m) {
+    const int n = first[m + 1] - first[m];
+    if (n == 0) continue;
+    if (m == 0)
+      bn_sums_group_kernel<false><<<(int)sb[m], 256, 0, st>>>(d_items, n);
+    else
+      bn_sums_group_kernel<true><<<(int)sb[m], 256, 0, st>>>(
+          d_items + first[m], n);
+    KFAC_LAUNCH_CHECK("bn_sums_group_kernel");
+  }
+  bn_finish_grads_kernel<<<(int)fb, 256, 0, st>>>(d_items, count);
   KFAC_LAUNCH_CHECK("bn_finish_grads_kernel");
   return KFAC_OK;
 }

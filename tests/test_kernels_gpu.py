@@ -657,6 +657,41 @@ def test_bn_sample_grads_layouts(ops, shape, channels_last, mean):
     assert rel(host(out), host(ref)) < 5 * 6e-8 * max(4.0, hw ** 0.5)
 
 
+@pytest.mark.parametrize('shape', [
+    (33, 10), (8, 64, 8, 8), (5, 33, 9, 11), (32, 8, 56, 56)])
+@pytest.mark.parametrize('channels_last', [False, True])
+@pytest.mark.parametrize('where', ['first', 'corners', 'sample'])
+def test_bn_sample_grads_with_outliers(ops, shape, channels_last, where):
+    """The first value of every channel, the corner of every image or a whole
+    sample far outside the rest: no digits are lost to it."""
+    torch.manual_seed(6)
+    x = 3.0 + 1e-3 * torch.randn(shape, device='cuda')
+    gy = torch.randn(shape, device='cuda')
+    at = {'first': (slice(0, 1), slice(None), 0, 0),
+          'corners': (slice(None), slice(None), 0, 0),
+          'sample': (slice(0, 1),)}[where]
+    x[at[:x.dim()]] += 5.0
+    if channels_last and len(shape) == 4:
+        x = x.contiguous(memory_format=torch.channels_last)
+        gy = gy.contiguous(memory_format=torch.channels_last)
+    out = ops.bn_sample_grads(x, gy, 1e-5, 2.0)
+    xd, gd = x.double(), gy.double() * 2.0
+    batch = [0] + list(range(2, xd.dim()))
+    xh = (xd - xd.mean(batch, keepdim=True)) / torch.sqrt(
+        xd.var(batch, unbiased=False, keepdim=True) + 1e-5)
+    ref = torch.cat([(gd * xh).flatten(2).sum(2) if xd.dim() > 2 else gd * xh,
+                     gd.flatten(2).sum(2) if xd.dim() > 2 else gd], 1)
+    # every rounding is 2^-24 of a term: of the two terms of sum g xhat (the
+    # sample's own part and its mean's distance from the batch's, at most
+    # sqrt(n) spreads, times sum g), of their sum and of the factors
+    n, c = shape[0], shape[1]
+    assert rel(host(out[:, c:]), host(ref[:, c:])) < 4 * 2.0 ** -24
+    off = (xh.flatten(2).mean(2) if xd.dim() > 2 else xh) * ref[:, c:]
+    size = (off.norm() + (ref[:, :c] - off).norm() + ref[:, :c].norm()).item()
+    err = (out[:, :c].double() - ref[:, :c]).norm().item()
+    assert err < 4 * 2.0 ** -24 * size
+
+
 def test_bn_kfgrad(ops, golden):
     g = golden('bn_4d')
     c = g['g_gamma'].shape[0]
