@@ -318,6 +318,11 @@ size_t tc_factor_group_workspace_bytes(int count, const FactorJob* jobs,
 size_t tc_stage_bytes(long long rows, int d);
 int tc_stage_group(int count, const FactorJob* jobs, char* ws, void* tmaps,
                    cudaStream_t stream);
+// Rules of all factor builds (tc_gemm.cu): most 32-row k-blocks that a CTA
+// accumulates (KFAC_TC_MAX_KBLOCKS, else `fallback`), waves of CTAs that a
+// grouped build is cut into (KFAC_TC_WAVES, else 2).
+long long factor_max_kblocks(long long fallback);
+long long factor_waves();
 // Factors from row-major staged planes (gram.cu).
 bool gram_grid_job(const FactorJob& job);     // shifted products
 bool gram_direct_job(const FactorJob& job);   // no staged planes needed

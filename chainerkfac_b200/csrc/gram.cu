@@ -1356,20 +1356,23 @@ inline int group_cost(const JobPlan& p, int k) {
 }
 
 // A CTA keeps at least 16 k-blocks so that its prologue and epilogue stay
-// amortised, and never accumulates more than 128: the tensor core adds each
-// product into the fp32 accumulator with truncation, so that a long sum
-// drifts (relative error of a 100 352-row factor of non-negative values:
-// 2e-4 when one CTA accumulates 1500 k-blocks, 4.7e-5 at 256, 2e-5 at 128);
-// the partial tiles are added with rounding to nearest.
+// amortised, and never accumulates more than 128 (KFAC_TC_MAX_KBLOCKS): the
+// tensor core adds each product into the fp32 accumulator with truncation, so
+// that a long sum drifts (relative error of a 100 352-row factor of non-negative
+// values: 2e-4 when one CTA accumulates 1500 k-blocks, 4.7e-5 at 256, 2e-5 at
+// 128); the partial tiles are added with rounding to nearest.
 void split_job(JobPlan& p, long long target) {
+  // (whole stages: a multiple of four)
+  const long long most = factor_max_kblocks(128) & ~3LL;
   p.partial_bytes = 0;
   for (int k = 0; k < p.ngroups; ++k) {
     long long chunk = target / group_cost(p, k);
     // (one tile without planes: eight stages)
     const long long least =
         p.direct && p.tiles[0] == 1 ? 2048 / p.width : 16;
-    chunk = std::max(least, std::min(128LL, chunk));
-    const long long sp = std::max(1LL, p.nkb[k] / chunk);
+    chunk = std::max(least, std::min(most, chunk));
+    const long long sp =
+        std::max(std::max(1LL, p.nkb[k] / chunk), (p.nkb[k] + most - 1) / most);
     p.kb_split[k] = (int)((p.nkb[k] + sp - 1) / sp);
     if (p.direct) {
       // whole stages: 16 rows of two sides, or 256 / width k-blocks of one
@@ -1383,7 +1386,7 @@ void split_job(JobPlan& p, long long target) {
   }
 }
 
-// Work per CTA: at most two waves over the SMs, so that the 10 us a CTA spends
+// Work per CTA: at most two waves over the SMs (KFAC_TC_WAVES), so that the 10 us a CTA spends
 // before its first and behind its last product stay small.
 long long split_target(const std::vector<JobPlan>& plans, size_t b, size_t e) {
   long long work = 0;
@@ -1391,7 +1394,7 @@ long long split_target(const std::vector<JobPlan>& plans, size_t b, size_t e) {
     for (int k = 0; k < plans[i].ngroups; ++k)
       work += (long long)plans[i].tiles[k] * plans[i].nkb[k] *
               group_cost(plans[i], k);
-  return work / (2LL * sm_count()) + 1;
+  return work / (factor_waves() * sm_count()) + 1;
 }
 
 // Jobs are worked off in batches whose planes stay below this many bytes, so

@@ -955,14 +955,24 @@ static long long tc_block_cost(int d) {
 // never accumulates more than this many k-blocks (of 32 rows); the partial
 // tiles of longer contractions are summed in fp32 by the reduce kernel, with
 // rounding to nearest.  256 keeps the drift at half the 1e-4 bound and costs
-// nothing measurable; 128 costs 15 % of the factor stage.
-static long long tc_max_kblocks() {
+// nothing measurable here; 128 costs 15 % of the factor stage with this kernel,
+// nothing with those of gram.cu.
+long long factor_max_kblocks(long long fallback) {
   static const long long v = [] {
     const char* e = getenv("KFAC_TC_MAX_KBLOCKS");
-    const long long k = e ? atoll(e) : 256;
-    return k >= 16 ? k : 256;
+    return e ? atoll(e) : 0LL;
   }();
-  return v;
+  return v >= 16 ? v : fallback;
+}
+
+static long long tc_max_kblocks() { return factor_max_kblocks(256); }
+
+long long factor_waves() {
+  static const long long v = [] {
+    const char* e = getenv("KFAC_TC_WAVES");
+    return e ? atoll(e) : 0LL;
+  }();
+  return v > 0 ? v : 2;
 }
 
 static TcFactorSplit tc_split_for(long long rows, int d, long long chunk) {
@@ -972,7 +982,9 @@ static TcFactorSplit tc_split_for(long long rows, int d, long long chunk) {
   if (chunk < 16) chunk = 16;
   if (chunk > tc_max_kblocks()) chunk = tc_max_kblocks();
   const long long kblocks = (rows + TC_BK - 1) / TC_BK;
-  long long sp = (kblocks + chunk / 2) / chunk;
+  // (the nearest number of splits, none longer than the limit)
+  long long sp = std::max((kblocks + chunk / 2) / chunk,
+                          (kblocks + tc_max_kblocks() - 1) / tc_max_kblocks());
   if (sp < 1) sp = 1;
   long long kps = (kblocks + sp - 1) / sp * TC_BK;
   s.splits = (int)((rows + kps - 1) / kps);
@@ -1026,12 +1038,7 @@ static long long tc_group_chunk(int count, const FactorJob* jobs) {
   for (int i = 0; i < count; ++i)
     work += (long long)tc_factor_ctas(jobs[i].d) *
             ((jobs[i].rows + TC_BK - 1) / TC_BK) * tc_block_cost(jobs[i].d);
-  static const long long waves = [] {
-    const char* e = getenv("KFAC_TC_WAVES");
-    const long long w = e ? atoll(e) : 2;
-    return w > 0 ? w : 2;
-  }();
-  return work / (waves * sm_count());
+  return work / (factor_waves() * sm_count());
 }
 
 static size_t tc_pair_workspace_bytes(int count, const FactorJob* jobs,

@@ -325,6 +325,37 @@ def test_factor_of_plain_operands_read_by_tma(ops, n, c, h, w, channels_last):
     check_symmetric(host(out))
 
 
+@pytest.mark.parametrize('kblocks,d,ones', [
+    (129, 64, False), (196, 256, False), (255, 512, False), (230, 1028, False),
+    (255, 130, True), (380, 250, True)])
+def test_long_contractions_are_cut_in_groups(ops, engine, kblocks, d, ones):
+    """Beside work that fills the chip many times over, a contraction a little
+    longer than one CTA may accumulate is cut all the same.  Non-negative values:
+    the truncating accumulator drifts by up to 2^-25 per MMA, six per 32 rows, of
+    at most 128 (gather kernel, for appended columns: 256) 32-row blocks; what the
+    two-term split leaves out (2^-17 of a value, of either sign) averages out."""
+    if engine == 0:
+        pytest.skip('the limit belongs to the tensor-core engine')
+    torch.manual_seed(8)
+    big = torch.rand(65536, 1024, device='cuda')
+    x = torch.rand(32 * kblocks, d - int(ones), device='cuda')
+    out = torch.empty(d, d, device='cuda')
+    outs = [torch.empty(1024, 1024, device='cuda') for _ in range(6)]
+    bigs = [torch.empty(250, 250, device='cuda') for _ in range(12)]
+    ops.factor_group(
+        [ops.dense_item(x, ones, 1.0, 0.0, out)] +
+        [ops.dense_item(big, False, 1.0, 0.0, o) for o in outs] +
+        [ops.dense_item(big.view(-1, 256)[:, :249].contiguous(), True, 1.0,
+                        0.0, o) for o in bigs], x.device)
+    xd = x.double()
+    if ones:
+        xd = torch.cat([xd, xd.new_ones(32 * kblocks, 1)], 1)
+    limit = 256 if ones else 128
+    assert rel(host(out), host(xd.t() @ xd)) < 6 * limit * 2.0 ** -25
+    bd = big.double()
+    assert rel(host(outs[3]), host(bd.t() @ bd)) < 6 * 128 * 2.0 ** -25
+
+
 def test_factor_builds_from_staged_operands(ops, engine):
     """The optional operand feed of the factor builds (staging pass that
     writes X^T as two bf16 planes, TMA boxes into the tile kernel) against the
