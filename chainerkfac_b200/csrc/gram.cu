@@ -1397,17 +1397,28 @@ long long split_target(const std::vector<JobPlan>& plans, size_t b, size_t e) {
   return work / (factor_waves() * sm_count()) + 1;
 }
 
-// Jobs are worked off in batches whose planes stay below this many bytes, so
-// that the workspace does not grow with the network.  (Staging a batch beside
-// the products of the one before, in two workspaces, gained nothing: both
+// Jobs are worked off in batches whose planes and partial tiles stay below this
+// many bytes, so that the workspace does not grow with the network.  A batch's
+// partial tiles are counted with the fewest splits its jobs can have; cutting
+// them further into two waves of CTAs adds at most a tile each (0.1 GB).  (All
+// factors of ResNet-50 at 32 images take 1.4 GB and one batch.  Staging a batch
+// beside the products of the one before, in two workspaces, gained nothing: both
 // halves are bound by the same memory traffic.)
-constexpr size_t kPlaneBytesMax = (size_t)1 << 30;
+constexpr size_t kBatchBytesMax = (size_t)2 << 30;
+
+size_t least_bytes(const JobPlan& p) {
+  const long long most = factor_max_kblocks(128) & ~3LL;
+  long long tiles = 0;
+  for (int k = 0; k < p.ngroups; ++k)
+    tiles += p.tiles[k] * ((p.nkb[k] + most - 1) / most);
+  return 2 * p.plane_bytes + (size_t)tiles * GR_TILE * sizeof(float);
+}
 
 size_t batch_end(const std::vector<JobPlan>& plans, size_t b) {
   size_t e = b, bytes = 0;
   while (e < plans.size() && e - b < (size_t)kStageJobs) {
-    bytes += 2 * plans[e].plane_bytes;
-    if (e > b && bytes > kPlaneBytesMax) break;
+    bytes += least_bytes(plans[e]);
+    if (e > b && bytes > kBatchBytesMax) break;
     ++e;
   }
   return e;

@@ -57,6 +57,28 @@ def test_pure_host_entry_points(lib):
         lib.kfac_set_factor_staging(0)
 
 
+def test_workspace_of_grouped_factors_is_bounded(lib):
+    """However many factors a grouped build has, wide ones with many partial
+    tiles each or narrow ones with long contractions: one batch's planes and
+    partial tiles (2 GB, and a tile per CTA of two waves)."""
+    from chainerkfac_b200 import _lib
+
+    def need(rows, d, count):
+        items = []
+        for _ in range(count):
+            it = _lib.FactorItem()
+            it.kind, it.x, it.out, it.alpha = 0, 256, 256, 1.0
+            it.rows, it.d_in, it.ld = rows, d, d
+            items.append(it)
+        return lib.kfac_factor_group_workspace_bytes(
+            count, (_lib.FactorItem * count)(*items))
+    limit = (2 << 30) + (400 << 18)
+    for rows, d in ((1024, 4096), (32768, 4096), (100352, 64), (4000, 1025)):
+        assert need(rows, d, 10) < limit
+        assert need(rows, d, 400) < limit
+        assert need(rows, d, 400) >= need(rows, d, 1)
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from chainerkfac_b200 import _lib
     monkeypatch.setattr(_lib, '_lib', None)

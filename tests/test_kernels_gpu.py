@@ -356,6 +356,35 @@ def test_long_contractions_are_cut_in_groups(ops, engine, kblocks, d, ones):
     assert rel(host(outs[3]), host(bd.t() @ bd)) < 6 * 128 * 2.0 ** -25
 
 
+def test_group_of_several_batches(ops, engine):
+    """Factors whose partial tiles do not fit the workspace of one batch
+    (285 MB each), and kinds that come behind them, against fp64."""
+    if engine == 0:
+        pytest.skip('batches belong to the tensor-core engine')
+    torch.manual_seed(9)
+    x = torch.randn(32768, 4096, device='cuda')
+    xc = torch.randn(3, 40, 9, 8, device='cuda')
+    xs = torch.randn(1999, 1025, device='cuda')
+    out = [torch.empty(4096, 4096, device='cuda') for _ in range(9)]
+    oc = [torch.empty(360, 360, device='cuda') for _ in range(2)]
+    os = torch.empty(1025, 1025, device='cuda')
+    items = [ops.conv_input_item(xc, 3, 1, 1, False, 1.0, 0.0, oc[0])] + [
+        ops.dense_item(x, False, 2.0 ** -i, 0.0, o)
+        for i, o in enumerate(out)] + [
+        ops.conv_input_item(xc, 3, 1, 1, False, 1.0, 0.0, oc[1]),
+        ops.dense_item(xs, False, 1.0, 0.0, os)]
+    ops.factor_group(items, x.device)
+    ref = x.double().t() @ x.double()
+    for i, o in enumerate(out):
+        assert float((o.double() * 2.0 ** i - ref).norm() / ref.norm()) < \
+            FACTOR_TOL
+    u = torch.nn.functional.unfold(xc.double(), 3, padding=1)
+    u = u.transpose(1, 2).reshape(-1, 360)
+    assert all(rel(host(o), host(u.t() @ u)) < FACTOR_TOL for o in oc)
+    xd = xs.double()
+    assert rel(host(os), host(xd.t() @ xd)) < FACTOR_TOL
+
+
 def test_factor_builds_from_staged_operands(ops, engine):
     """The optional operand feed of the factor builds (staging pass that
     writes X^T as two bf16 planes, TMA boxes into the tile kernel) against the
