@@ -55,11 +55,20 @@ bool gram_direct_job(const FactorJob& job) {
 }
 
 // Shifted products pay once the channels fill a good part of a granule; a
-// narrower convolution has few columns, and its patches are small too.
+// narrower convolution has few columns, and its patches are small too.  Images
+// of two rows or columns are mostly border: the zeros around them are more rows
+// than they have pixels, and a block of the factor is the small difference of
+// large sums (exact zeros came out as 2e-5 of the diagonal).  Below 384 pixels in
+// all, the nine groups of products cost more than they save.  us for four factors
+// alike, shifted and from patches, 64 and 512 channels:
+//   128 images 1x1 55 45, 344 234; 2x2 59 60, 394 323; 3x3 60 68, 460 464;
+//   32 images 3x3 58 52, 318 273; 4x4 55 59, 332 325; 7x7 58 71, 417 558;
+//   8 images 5x5 52 50, 292 259; 7x7 56 56, 307 303; 14x14 56 71, 384 559.
 bool gram_grid_job(const FactorJob& job) {
   const Operand& X = job.X;
   return X.mode == 1 && X.ks == 3 && X.st == 1 && X.pd == 1 &&
-         X.extra_idx < 0 && X.C >= 32;
+         X.extra_idx < 0 && X.C >= 32 && job.rows >= 384 &&
+         (long long)(X.H + 2) * (X.W + 2) <= 3LL * X.H * X.W;
 }
 
 namespace {

@@ -1059,7 +1059,7 @@ static size_t tc_pair_workspace_bytes(int count, const FactorJob* jobs,
 
 // Factors that are built from staged planes (gram.cu), unless the caller chose
 // the staging pass of stage.cu or gives no workspace:
-//  * 3 x 3 convolutions as shifted products, at any size (32 images, us per
+//  * 3 x 3 convolutions as shifted products (gram_grid_job; 32 images, us per
 //    factor before and now: 64 channels 56 x 56 228 -> 78, 256 channels 14 x 14
 //    171 -> 62; 8 images of 64 channels 14 x 14 68 -> 41);
 //  * plain operands that TMA reads in place, from a million elements on (below

@@ -241,7 +241,9 @@ def test_scratch_buffers_are_per_stream(ops):
 @pytest.mark.parametrize('n,c,h,w,stride', [
     (2, 32, 8, 8, 1), (3, 33, 5, 9, 1), (1, 64, 1, 1, 1), (2, 64, 14, 1, 1),
     (5, 70, 7, 7, 1), (4, 128, 9, 6, 1), (2, 257, 4, 4, 1), (33, 512, 7, 7, 1),
-    (2, 130, 41, 40, 2)])
+    (2, 130, 41, 40, 2), (6, 32, 8, 8, 1), (43, 33, 3, 3, 1),
+    (32, 70, 7, 2, 1), (28, 129, 2, 7, 1), (8, 128, 9, 6, 1),
+    (28, 257, 4, 4, 1), (200, 64, 2, 2, 1)])
 def test_factor_of_3x3_convolutions(ops, engine, n, c, h, w, stride,
                                     channels_last):
     """Patch factors as shifted products (stride 1: one granule of channels,
@@ -261,6 +263,24 @@ def test_factor_of_3x3_convolutions(ops, engine, n, c, h, w, stride,
     ref = u.t() @ u / n + 1.5
     assert rel(host(out), host(ref)) < FACTOR_TOL
     check_symmetric(host(out))
+
+
+@pytest.mark.parametrize('n,c,h,w', [
+    (32, 64, 1, 1), (128, 70, 1, 1), (32, 256, 2, 2), (40, 32, 1, 9)])
+def test_taps_outside_small_images_stay_zero(ops, n, c, h, w):
+    """Entries between taps that never see the image at the same position are
+    sums of zeros; nothing is left there by larger sums."""
+    torch.manual_seed(7)
+    x = torch.rand(n, c, h, w, device='cuda') + 1.0
+    out = torch.full((9 * c, 9 * c), 3.0, device='cuda')
+    ops.factor_group([ops.conv_input_item(x, 3, 1, 1, False, 1.0 / n, 0.0,
+                                          out)], x.device)
+    u = torch.nn.functional.unfold(x.double(), 3, padding=1)
+    u = u.transpose(1, 2).reshape(-1, 9 * c)
+    ref = u.t() @ u / n
+    assert rel(host(out), host(ref)) < FACTOR_TOL
+    assert bool((ref == 0).any())
+    assert float(out[ref == 0].abs().max()) == 0.0
 
 
 @pytest.mark.parametrize('b2', [0.0, 0.75])
