@@ -64,6 +64,7 @@ SIGNATURES = {
     'kfac_get_factor_staging': (I, []),
     'kfac_tc_status': (I, [c_int_p]),
     'kfac_selftest_wait_expiry': (I, [c_int_p, c_int_p]),
+    'kfac_selftest_pivots': (I, [I, VP, VP, VP, VP, VP, VP]),
     'kfac_factor_workspace_bytes': (SZ, [I64, I]),
     'kfac_factor_dense': (I, [VP, I64, I, I64, I, F, F, VP, VP, SZ, VP]),
     'kfac_factor_noalloc_max_bytes': (SZ, []),

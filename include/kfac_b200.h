@@ -85,6 +85,14 @@ int kfac_tc_status(int* status_out);
  * behind kfac_tc_status is not touched.  Synchronises the device. */
 int kfac_selftest_wait_expiry(int* status_out, int* returned_out);
 
+/* Self-test of the pivots of the diagonal kernel: for `count` values q and p
+ * (device memory) rsqrt[i] = 1 / sqrt(q[i]) and quot[i] = p[i] / sqrt(q[i]) as a
+ * factorisation computes them, checked[i] = 1 / sqrt(q[i]) with 1 in place of a
+ * pivot that failed (not positive, below the smallest normal number, NaN). */
+int kfac_selftest_pivots(int count, const float* q, const float* p,
+                         float* rsqrt, float* quot, float* checked,
+                         void* stream);
+
 /* ------------------------------------------------------------------ factors
  * out(d x d) = alpha * X^T X + beta * out, X a (rows x d) matrix that is never
  * materialised.  Only one triangle of tiles is computed; both triangles of

@@ -596,6 +596,41 @@ def test_inverse_bn_block_floors_each_half_separately(ops):
     plan.close()
 
 
+def test_pivots_over_the_exponent_range(ops):
+    """1 / sqrt(q) and p / sqrt(q) of the diagonal kernel against fp64, four
+    values in every binade of the normal numbers and their neighbours: 2^-24 for
+    the last rounding, half of that for q r, which enters the correction by half
+    (and 2^-24 for p r), and 2^-45 of the approximation's squared 2^-22.9."""
+    from chainerkfac_b200 import _lib
+    rng = np.random.default_rng(21)
+    e = np.repeat(np.arange(-126, 128), 64)
+    q = np.ldexp(1.0 + rng.random(e.size), e).astype(np.float32)
+    q = q[(q >= np.float32(2.0 ** -126)) & np.isfinite(q)]
+    edge = np.float32([2.0 ** -126, 1.0, 2.0, 4.0,
+                       np.finfo(np.float32).max])
+    q = np.concatenate([q, edge, np.nextafter(edge[1:], np.float32(0))])
+    p = (np.sqrt(q) * rng.uniform(-1.0, 1.0, q.size)).astype(np.float32)
+    bad = np.float32([0.0, -0.0, -1.0, -np.inf, np.nan, 1e-39, -1e-39])
+    n = q.size
+    args = [dev(np.concatenate([q, bad])),
+            dev(np.concatenate([p, np.ones_like(bad)]))]
+    outs = [torch.empty_like(args[0]) for _ in range(3)]
+    lib = _lib.load()
+    _lib.check(lib.kfac_selftest_pivots(
+        n + bad.size, *[t.data_ptr() for t in args + outs], ops._stream()),
+        'kfac_selftest_pivots')
+    r, quot, checked = [host(t).astype(np.float64) for t in outs]
+    want = 1.0 / np.sqrt(q.astype(np.float64))
+    ulp = 2.0 ** -24
+    assert np.max(np.abs(r[:n] / want - 1.0)) < 1.5 * ulp + 2.0 ** -44
+    assert np.array_equal(checked[:n], r[:n])
+    tail = np.abs(quot[:n] - p * want) / np.abs(p * want)
+    assert np.max(tail) < 2.5 * ulp + 2.0 ** -44
+    # a failed pivot: NaN from then on, or one where the caller asks for it
+    assert np.all(~np.isfinite(r[n:])) and np.array_equal(
+        checked[n:], np.ones(bad.size))
+
+
 def test_inverse_reports_non_spd(ops):
     a = np.eye(40, dtype=np.float32)
     a[17, 17] = -1.0
