@@ -546,33 +546,37 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
         }
       }
     }
-  } else if (elect_one()) {
-    // ===================== MMA issuer =====================
-    const unsigned idesc = tc_instr_desc(n_inst);
-    const unsigned a_off =
-        share_ab ? (unsigned)(Map::kABytes + (m0 - n0) * 128) : 0u;
-    for (int kb = 0; kb < nkb; ++kb) {
-      const int s = kb % Map::kStages;
-      if (!mbar_wait_status(&ctl->full[s], (kb / Map::kStages) & 1,
-                            &ctl->abort_flag, &g_tile_status))
-        break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const unsigned sa = smem_u32(smem + s * Map::kStage);
-      const unsigned long long a_hi = tc_smem_desc(sa + a_off);
-      const unsigned long long b_hi = tc_smem_desc(sa + Map::kABytes);
-      const unsigned long long a_lo = tc_smem_desc(sa + Map::kLo + a_off);
-      const unsigned long long b_lo =
-          tc_smem_desc(sa + Map::kLo + Map::kABytes);
+  } else {
+    if (elect_one()) {
+      // ===================== MMA issuer =====================
+      const unsigned idesc = tc_instr_desc(n_inst);
+      const unsigned a_off =
+          share_ab ? (unsigned)(Map::kABytes + (m0 - n0) * 128) : 0u;
+      for (int kb = 0; kb < nkb; ++kb) {
+        const int s = kb % Map::kStages;
+        if (!mbar_wait_status(&ctl->full[s], (kb / Map::kStages) & 1,
+                              &ctl->abort_flag, &g_tile_status))
+          break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const unsigned sa = smem_u32(smem + s * Map::kStage);
+        const unsigned long long a_hi = tc_smem_desc(sa + a_off);
+        const unsigned long long b_hi = tc_smem_desc(sa + Map::kABytes);
+        const unsigned long long a_lo = tc_smem_desc(sa + Map::kLo + a_off);
+        const unsigned long long b_lo =
+            tc_smem_desc(sa + Map::kLo + Map::kABytes);
 #pragma unroll
-      for (int kk = 0; kk < TT_BK / 8; ++kk) {
-        const unsigned long long adv = (unsigned long long)(kk * 32 >> 4);
-        tc_mma(tmem + TN, a_lo + adv, b_hi + adv, idesc, (kb | kk) != 0);
-        tc_mma(tmem + TN, a_hi + adv, b_lo + adv, idesc, 1);
-        tc_mma(tmem, a_hi + adv, b_hi + adv, idesc, (kb | kk) != 0);
+        for (int kk = 0; kk < TT_BK / 8; ++kk) {
+          const unsigned long long adv = (unsigned long long)(kk * 32 >> 4);
+          tc_mma(tmem + TN, a_lo + adv, b_hi + adv, idesc, (kb | kk) != 0);
+          tc_mma(tmem + TN, a_hi + adv, b_lo + adv, idesc, 1);
+          tc_mma(tmem, a_hi + adv, b_hi + adv, idesc, (kb | kk) != 0);
+        }
+        tc_commit(&ctl->empty[s]);
       }
-      tc_commit(&ctl->empty[s]);
+      tc_commit(&ctl->accum);
     }
-    tc_commit(&ctl->accum);
+    // (the block barrier and the release of the tensor memory are warp-wide)
+    __syncwarp();
   }
 
   // ===================== epilogue =====================
