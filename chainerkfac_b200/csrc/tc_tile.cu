@@ -753,10 +753,12 @@ int tc_number_tiles(GemmDesc* descs, int n, int narrow_max, int* tile_cols) {
   // read by the MMAs twice as often) up to `narrow_max` of them: as many as
   // there are SMs for a launch that runs alone (512 x 4608 x 4608: 144 narrow
   // tiles 125 us, 72 wide ones 190 us), three quarters where launches of other
-  // streams run beside it.  Measured with the line at 20, 74, 111 and
-  // 148 of 148 SMs: a 2304-row inverse 835, 791, 791, 791 us; a 4608-row one
-  // 1954, 1934, 1915, 1902; 108 factors of ResNet-50 in three concurrent plans
-  // 6.10, 6.22, 6.27, 6.33 ms.
+  // streams run beside it.  Measured with the line at 0, 20, 74, 111, 148 and
+  // 222 of 148 SMs: a 2304-row inverse 841, 819, 765, 763, 766, 769 us; a
+  // 4608-row one 2010, 1921, 1905, 1868, 1864, 1885; 14 pairs of odd sides 439,
+  // 425, 402, 390, 390, 390; the pair 4608 / 512 with its preconditioning 2225,
+  // 2138, 2119, 2081, 2048, 2072; 108 factors of ResNet-50 in three concurrent
+  // plans 6.10, 6.15, 6.17, 6.18, 6.19, 6.26 ms.
   long long narrow = 0;
   for (int i = 0; i < n; ++i) narrow += tile_count(descs[i], 128);
   const int tn = narrow <= narrow_max ? 128 : 256;
@@ -778,15 +780,17 @@ int launch_tc_grouped(const GemmDesc* descs_dev, const GemmDesc* descs_host,
   const int rc = tc_prepare_tiles();
   if (rc != KFAC_OK) return rc;
   // the problems with 16-byte rows come first (tc_number_tiles); where all
-  // tiles fit the chip at once, one launch of the general kernel (2 us per
-  // k-block) may end sooner than two in a row (1 us, and 10 us more)
+  // tiles fit the chip at once, one launch of the general kernel (1.3 us per
+  // k-block of a 128-wide tile) may end sooner than two in a row (0.75 us, and
+  // 10 us more).  Both products of 256 x 1024 beside 10 x 301: 92 us in two
+  // launches each, 83 us in one; 128 x 2048 beside 127 x 1023: 153 and 120.
   int n_vec = 0;
   while (n_vec < ndesc && tile_desc_vec(descs_host[n_vec])) ++n_vec;
   if (n_vec < ndesc && total_tiles <= sm_count()) {
     long long k[2] = {0, 0};
     for (int i = 0; i < ndesc; ++i)
       k[i >= n_vec] = std::max(k[i >= n_vec], descs_host[i].K / TT_BK);
-    if (2 * std::max(k[0], k[1]) <= k[0] + 2 * k[1] + 10) n_vec = 0;
+    if (26 * std::max(k[0], k[1]) <= 15 * k[0] + 26 * k[1] + 200) n_vec = 0;
   }
   for (int k = 0; k < 2; ++k) {
     const int first = k == 0 ? 0 : n_vec, n = k == 0 ? n_vec : ndesc - n_vec;
