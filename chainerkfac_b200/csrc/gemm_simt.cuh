@@ -286,7 +286,7 @@ constexpr int kTileInline = 8;   // descriptors that fit the kernel arguments
 int tc_number_tiles(GemmDesc* descs, int n, int narrow_max, int* tile_cols);
 int tc_prepare_tiles();
 // `descs_host`: the same descriptors on the host (small launches pass them as
-// kernel arguments), or NULL.
+// kernel arguments; `descs_dev` is not read then).
 int launch_tc_grouped(const GemmDesc* descs_dev, const GemmDesc* descs_host,
                       int ndesc, int total_tiles, int tile_cols, bool precond,
                       float lr, float momentum, cudaStream_t stream);

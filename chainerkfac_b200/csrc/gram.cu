@@ -2,8 +2,8 @@
 //
 // Every operand X (rows x columns, in whatever layout the caller holds it) is
 // first written once as two bf16 planes, hi and lo with x = hi + lo, rows
-// contiguous along the columns (stage_planes kernels, HBM-bound).  The
-// products then need no producer warps: TMA copies 32 rows x 64 columns of
+// contiguous along the columns (stage_cols_kernel, stage_rows_kernel; HBM-bound).
+// The products then need no producer warps: TMA copies 32 rows x 64 columns of
 // both planes (8 KB) per instruction straight into the 128-byte-swizzled,
 // MN-major operand layout of tcgen05.mma, with zeros past the last column.
 // The in-kernel gather that this replaces spent four issue slots per clock on
@@ -84,8 +84,6 @@ constexpr int GR_THREADS = 256;
 constexpr int GR_TILE = 256 * 256;                 // floats of a partial tile
 constexpr int GR_SHIFTS = 13;
 
-struct GrControl;
-
 // Products of one contraction range of one operand: A granules (64 columns)
 // against B granules.
 struct GramGroup {
@@ -150,11 +148,11 @@ __device__ __forceinline__ void gr_mma(unsigned tmem_d, unsigned long long da,
 }
 
 __device__ __forceinline__ void gr_load(unsigned dst, const void* tmap, int x,
-                                        int y, unsigned bar) {
+                                        int y, int z, unsigned bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::"
       "complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(0), "r"(bar)
+      ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar)
       : "memory");
 }
 
@@ -284,11 +282,12 @@ gram_kernel(const GramGroup* __restrict__ groups, int ngroups) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           if (i < nb)
-            gr_load(st + GR_SIDE + i * GR_GBYTES, g.tmap, bx[i], r + by[i], bar);
+            gr_load(st + GR_SIDE + i * GR_GBYTES, g.tmap, bx[i], r + by[i], 0,
+                    bar);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           if (i < la)
-            gr_load(st + i * GR_GBYTES, g.tmap, ax[i], r + ay[i], bar);
+            gr_load(st + i * GR_GBYTES, g.tmap, ax[i], r + ay[i], 0, bar);
       }
     }
     __syncwarp();
@@ -359,18 +358,6 @@ gram_kernel(const GramGroup* __restrict__ groups, int ngroups) {
                  : "memory");
 }
 
-__device__ __forceinline__ void gr_split2(float x0, float x1, unsigned& hi,
-                                          unsigned& lo) {
-  // bf16 by adding half an ulp (ties away from zero), the remainder likewise
-  const unsigned r0 = __float_as_uint(x0) + 0x8000u;
-  const unsigned r1 = __float_as_uint(x1) + 0x8000u;
-  hi = __byte_perm(r0, r1, 0x7632);
-  const float l0 = x0 - __uint_as_float(r0 & 0xffff0000u);
-  const float l1 = x1 - __uint_as_float(r1 & 0xffff0000u);
-  lo = __byte_perm(__float_as_uint(l0) + 0x8000u,
-                   __float_as_uint(l1) + 0x8000u, 0x7632);
-}
-
 // ---------------------------------------------------- products without planes
 // Plain operands whose rows TMA can read as they are (16-byte pitches and
 // addresses).  32 KB of fp32 per stage arrive by TMA, sixteen warps split them
@@ -433,15 +420,6 @@ __device__ __forceinline__ unsigned long long dr_desc(unsigned addr, int lbo,
   d |= (unsigned long long)1 << 46;
   d |= (unsigned long long)swizzle << 61;
   return d;
-}
-
-__device__ __forceinline__ void dr_load3(unsigned dst, const void* tmap, int x,
-                                         int y, int z, unsigned bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::"
-      "complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar)
-      : "memory");
 }
 
 template <bool KM>
@@ -531,17 +509,17 @@ direct_kernel(const DirectGroup* __restrict__ groups, int ngroups) {
           for (int q = 0; q < sub; ++q, dst += width * 128) {
             const int b = (row0 >> 5) + st * sub + q;
             const int img = b / g.per_image;
-            dr_load3(dst, g.tmap, 32 * (b - img * g.per_image), 0, img, bar);
+            gr_load(dst, g.tmap, 32 * (b - img * g.per_image), 0, img, bar);
           }
         } else if (share) {
           const int r = row0 + st * R;
           for (int c = 0; c < width; c += 64)
             for (int q = 0; q < R; q += g.box_rows, dst += g.box_rows * 256)
-              dr_load3(dst, g.tmap, 256 * tj + c, r + q, 0, bar);
+              gr_load(dst, g.tmap, 256 * tj + c, r + q, 0, bar);
         } else {
           const int r = row0 + st * 16;
           for (int c = 0; c < 512; c += 64, dst += 16 * 256)
-            dr_load3(dst, g.tmap, c < 256 ? 256 * ti + c : 256 * (tj - 1) + c,
+            gr_load(dst, g.tmap, c < 256 ? 256 * ti + c : 256 * (tj - 1) + c,
                      r, 0, bar);
         }
       }
@@ -638,10 +616,10 @@ direct_kernel(const DirectGroup* __restrict__ groups, int ngroups) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         unsigned hi[4], l[4];
-        gr_split2(a[i].x, a[i].y, hi[0], l[0]);
-        gr_split2(a[i].z, a[i].w, hi[1], l[1]);
-        gr_split2(b[i].x, b[i].y, hi[2], l[2]);
-        gr_split2(b[i].z, b[i].w, hi[3], l[3]);
+        split_bf16x2(a[i].x, a[i].y, hi[0], l[0]);
+        split_bf16x2(a[i].z, a[i].w, hi[1], l[1]);
+        split_bf16x2(b[i].x, b[i].y, hi[2], l[2]);
+        split_bf16x2(b[i].z, b[i].w, hi[3], l[3]);
         *reinterpret_cast<uint4*>(q + dst[i]) =
             h ? make_uint4(hi[2], hi[3], hi[0], hi[1])
               : make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -708,7 +686,7 @@ __device__ __forceinline__ void gr_store8(const StageJob& j, int row, int col,
                                           const float v[8]) {
   unsigned h[4], l[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) gr_split2(v[2 * i], v[2 * i + 1], h[i], l[i]);
+  for (int i = 0; i < 4; ++i) split_bf16x2(v[2 * i], v[2 * i + 1], h[i], l[i]);
   unsigned short* p = j.hi + (long long)row * j.cp + col;
   *reinterpret_cast<uint4*>(p) = make_uint4(h[0], h[1], h[2], h[3]);
   *reinterpret_cast<uint4*>(p + j.plane) = make_uint4(l[0], l[1], l[2], l[3]);
@@ -1395,8 +1373,8 @@ void split_job(JobPlan& p, long long target) {
   }
 }
 
-// Work per CTA: at most two waves over the SMs (KFAC_TC_WAVES), so that the 10 us a CTA spends
-// before its first and behind its last product stay small.
+// Work per CTA: at most two waves over the SMs (KFAC_TC_WAVES), so that the 10 us
+// a CTA spends before its first and behind its last product stay small.
 long long split_target(const std::vector<JobPlan>& plans, size_t b, size_t e) {
   long long work = 0;
   for (size_t i = b; i < e; ++i)

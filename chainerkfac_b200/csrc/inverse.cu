@@ -436,9 +436,9 @@ constexpr int kBarRows = 8;    // so are the rows that follow it
 // Pivot k of an 8 x 8 block: r = 1 / sqrt(q) by the approximation and one
 // Newton step; `next`, if given, becomes p / sqrt(q) without waiting for r.  The
 // step's own error is far below fp32, the roundings of q r, of the last sum and
-// (for `next`) of p r leave 1.5 and 2.5 units of 2^-24 (kfac_selftest_pivots).  CHECK: a pivot
-// that is not positive (or below the smallest normal number) counts as failed
-// and becomes 1.
+// (for `next`) of p r leave 1.5 and 2.5 units of 2^-24 (kfac_selftest_pivots).
+// CHECK: a pivot that is not positive (or below the smallest normal number)
+// counts as failed and becomes 1.
 template <bool CHECK>
 __device__ __forceinline__ float diag_pivot(float q, float* next) {
   if (CHECK && !(q >= 1.17549435e-38f)) return 1.f;
@@ -746,9 +746,8 @@ __device__ __forceinline__ void diag_update_block(DiagSmem& sm, int r, int half,
 // it, two rows per lane (diag_follow), and the product of the finished column
 // with the next one is split: its diagonal sub-block first (six warps, then
 // the chain goes on), the rows that follow it (six warps, then the followers
-// go on), and the columns beyond next to the next chain.  Warps are placed so
-// that the chain has its scheduler to itself.  128 rows: 61 us with 8 x 8
-// register blocks per thread and a barrier per block column, 20 us now with
+// go on), and the columns beyond next to the next chain.  128 rows: 61 us with
+// 8 x 8 register blocks per thread and a barrier per block column, 20 us now with
 // the launch, 31 us with the look-ahead's two products in front.
 template <bool LOOK>
 __global__ void __launch_bounds__(DT, 1)
@@ -781,9 +780,10 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
   __syncthreads();
 
   const int followers = 32 * (1 + (np + 1) / 2);   // threads of a step barrier
-  // roles: 0 chain; 3, 13 .. 15 the rest of its updates; 1, 2 followers;
-  // 5 6 7 9 10 11 rows and columns behind them; 3, 12 .. 15 the diagonal
-  // sub-block, with 0
+  // roles: 0 chain; 3, 4, 8, 12 the rest of its updates (on 3, 13 .. 15, which
+  // keeps them from the chain's scheduler: 0.4 % slower at 2304 and 4608 rows);
+  // 1, 2 followers; 5 6 7 9 10 11 rows and columns behind them; 3, 12 .. 15 the
+  // diagonal sub-block, with 0
   const bool diag_warp = warp == 0 || warp == 3 || warp >= 12;
   const bool work_warp = warp >= 5 && warp <= 11 && warp != 8;
   const int worker = warp < 8 ? warp - 5 : warp - 6;            // 0 .. 5
@@ -1139,7 +1139,6 @@ struct kfac_inverse_plan {
   GemmDesc* descs_dev;
   std::vector<GemmDesc> descs;       // the same on the host
   std::vector<Launch> launches;
-  long long total_elems;
   bool use_tc;
   // refinement (see refine_* kernels)
   float* add2_dev;
@@ -1218,7 +1217,6 @@ extern "C" int kfac_inverse_plan_create(
   std::vector<MatInfo> mats(count);
   char* ws = static_cast<char*>(workspace);
   int dmax = 0;
-  long long total_elems = 0;
   for (int i = 0; i < count; ++i) {
     MatInfo& m = mats[i];
     const size_t bytes = matrix_bytes(dims[i]);
@@ -1236,7 +1234,6 @@ extern "C" int kfac_inverse_plan_create(
     m.l2b = m.l2;
     m.id = i;
     dmax = std::max(dmax, dims[i]);
-    total_elems += (long long)dims[i] * dims[i];
   }
   // large matrices first: their tiles are scheduled first
   std::vector<int> order(count);
@@ -1586,7 +1583,6 @@ extern "C" int kfac_inverse_plan_create(
 
   kfac_inverse_plan* p = new kfac_inverse_plan();
   p->count = count;
-  p->total_elems = total_elems;
   p->launches = launches;
   p->use_tc = use_tc;
   p->mats_dev = nullptr; p->trace_dev = nullptr; p->add_dev = nullptr;

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "gemm_simt.cuh"
+#include "tc_common.cuh"
 
 namespace kfac {
 
@@ -39,24 +40,11 @@ struct StageJob {
   long long item_begin;
 };
 
-__device__ __forceinline__ void split2(float x0, float x1, unsigned& hi,
-                                       unsigned& lo) {
-  // same rounding as the in-kernel split of the gather path: bf16 by adding
-  // half an ulp (ties away from zero), the remainder rounded the same way
-  const unsigned r0 = __float_as_uint(x0) + 0x8000u;
-  const unsigned r1 = __float_as_uint(x1) + 0x8000u;
-  hi = __byte_perm(r0, r1, 0x7632);
-  const float l0 = x0 - __uint_as_float(r0 & 0xffff0000u);
-  const float l1 = x1 - __uint_as_float(r1 & 0xffff0000u);
-  lo = __byte_perm(__float_as_uint(l0) + 0x8000u,
-                   __float_as_uint(l1) + 0x8000u, 0x7632);
-}
-
 __device__ __forceinline__ void store8(const StageJob& j, long long row,
                                        long long k0, const float v[8]) {
   unsigned h[4], l[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) split2(v[2 * i], v[2 * i + 1], h[i], l[i]);
+  for (int i = 0; i < 4; ++i) split_bf16x2(v[2 * i], v[2 * i + 1], h[i], l[i]);
   const long long off = row * j.kp + k0;
   *reinterpret_cast<uint4*>(j.hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
   *reinterpret_cast<uint4*>(j.lo + off) = make_uint4(l[0], l[1], l[2], l[3]);

@@ -2,7 +2,7 @@
 // and the diagonal kernel of the inverse (inverse.cu): shared-memory and
 // instruction descriptors for K-major, 128-byte-swizzled fp32 (TF32) operand
 // tiles, MMA issue / commit, accumulator loads from tensor memory, bounded
-// barrier waits, and the split of fp32 values into two TF32 terms.
+// barrier waits, and the splits of fp32 values into two TF32 or bf16 terms.
 #pragma once
 
 #include "common.cuh"
@@ -187,6 +187,22 @@ __device__ __forceinline__ void store_split(unsigned hi_addr, unsigned lo_addr,
   l.x = x.x - h.x; l.y = x.y - h.y; l.z = x.z - h.z; l.w = x.w - h.w;
   sts128(hi_addr, h);
   sts128(lo_addr, l);
+}
+
+// Two values as bf16 terms x = hi + lo: one word of each (the first value in the
+// low half).  Rounding to bf16 is an integer add of half an ulp (ties away from
+// zero); the byte permute then takes the upper halves.  No cvt: conversions issue
+// on the quarter-rate XU pipe (measured at 130 % of its sustained peak with
+// cvt.rn.bf16x2 in the gather kernel).
+__device__ __forceinline__ void split_bf16x2(float x0, float x1, unsigned& hi,
+                                             unsigned& lo) {
+  const unsigned r0 = __float_as_uint(x0) + 0x8000u;
+  const unsigned r1 = __float_as_uint(x1) + 0x8000u;
+  hi = __byte_perm(r0, r1, 0x7632);
+  const float l0 = x0 - __uint_as_float(r0 & 0xffff0000u);
+  const float l1 = x1 - __uint_as_float(r1 & 0xffff0000u);
+  lo = __byte_perm(__float_as_uint(l0) + 0x8000u,
+                   __float_as_uint(l1) + 0x8000u, 0x7632);
 }
 
 }  // namespace kfac

@@ -181,22 +181,6 @@ __device__ __forceinline__ void tc_mma_bf16(unsigned tmem_d,
       : "memory");
 }
 
-// Two consecutive k -> one word of the hi tile and one of the lo tile (the
-// first k in the low half).  Rounding to bf16 is an integer add of half an ulp
-// (ties away from zero); the byte permute then takes the upper halves.  No
-// cvt: conversions issue on the quarter-rate XU pipe (measured at 130 % of its
-// sustained peak with cvt.rn.bf16x2 here).
-__device__ __forceinline__ void split_bf16x2(float x0, float x1, unsigned& hi,
-                                             unsigned& lo) {
-  const unsigned r0 = __float_as_uint(x0) + 0x8000u;
-  const unsigned r1 = __float_as_uint(x1) + 0x8000u;
-  hi = __byte_perm(r0, r1, 0x7632);
-  const float l0 = x0 - __uint_as_float(r0 & 0xffff0000u);
-  const float l1 = x1 - __uint_as_float(r1 & 0xffff0000u);
-  lo = __byte_perm(__float_as_uint(l0) + 0x8000u,
-                   __float_as_uint(l1) + 0x8000u, 0x7632);
-}
-
 __device__ __forceinline__ void store_split_bf16(unsigned hi_addr,
                                                  unsigned lo_addr, float4 a,
                                                  float4 b) {
