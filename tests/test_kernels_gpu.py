@@ -246,9 +246,10 @@ def test_scratch_buffers_are_per_stream(ops):
     (28, 257, 4, 4, 1), (200, 64, 2, 2, 1)])
 def test_factor_of_3x3_convolutions(ops, engine, n, c, h, w, stride,
                                     channels_last):
-    """Patch factors as shifted products (stride 1: one granule of channels,
-    ragged granules, several tiles, images of one row or column) and from
-    staged patches, on top of an existing average, against fp64."""
+    """Patch factors as shifted products (one granule of channels, ragged
+    granules, several tiles, the smallest images and pixel counts that go there)
+    and from staged patches (images of one or two rows or columns, few pixels,
+    stride 2), on top of an existing average, against fp64."""
     if engine == 0 and channels_last:
         pytest.skip('channels-last inputs belong to the tensor-core engine')
     torch.manual_seed(2)
@@ -286,10 +287,10 @@ def test_taps_outside_small_images_stay_zero(ops, n, c, h, w):
 @pytest.mark.parametrize('b2', [0.0, 0.75])
 def test_factor_group_second_output(ops, engine, b2):
     """Running averages kept up to date by the build: factors that are
-    assembled from shifted products, reduced from wide and narrow pieces,
-    built by the gather kernel, and one without a second array."""
+    assembled from shifted products (432 pixels), reduced from wide and narrow
+    pieces, built by the gather kernel, and one without a second array."""
     torch.manual_seed(5)
-    xc = torch.randn(3, 40, 9, 8, device='cuda')
+    xc = torch.randn(6, 40, 9, 8, device='cuda')
     xs = [torch.randn(r, d, device='cuda')
           for r, d in ((2100, 1028), (40000, 60), (70, 33), (50, 20))]
     u = torch.nn.functional.unfold(xc.double(), 3, padding=1)
@@ -763,9 +764,10 @@ def test_bn_sample_grads_layouts(ops, shape, channels_last, mean):
         xd.var(batch, unbiased=False, keepdim=True) + 1e-5)
     ref = torch.cat([(gd * xh).flatten(2).sum(2) if xd.dim() > 2 else gd * xh,
                      gd.flatten(2).sum(2) if xd.dim() > 2 else gd], 1)
-    # fp32 sums of up to hw terms, each rounded: sqrt(hw) 2^-24 relative to
-    # the terms, of the order of the sums themselves for random signs, times
-    # the distance of the shift from the mean in units of the spread (< 5)
+    # as for fp32 sums of up to hw terms, each rounded: sqrt(hw) 2^-24 relative
+    # to the terms, of the order of the sums themselves for random signs, times
+    # the distance of a shift from the mean in units of the spread (< 5); what
+    # the double sums leave is bounded in test_bn_sample_grads_with_outliers
     hw = 1
     for v in shape[2:]:
         hw *= v
