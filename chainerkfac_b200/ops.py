@@ -290,7 +290,8 @@ def bn_item(x, gy, eps, scale, out=None, stats=None):
 
 
 def bn_sample_grads_group(items):
-    """Per-sample gradients of all given layers (see bn_item), two launches."""
+    """Per-sample gradients of all given layers (see bn_item): a launch per
+    layout that occurs and one that finishes."""
     if not items:
         return
     lib = _lib.load()

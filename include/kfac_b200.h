@@ -212,7 +212,7 @@ int kfac_bn_sample_grads(const float* x, const float* gy, int n, int c, int hw,
                          void* stream);
 
 /* kfac_bn_sample_grads for all BatchNormalization layers of a step in two
- * launches (the reference computes them layer by layer inside its backward
+ * launches, three when both layouts occur (the reference computes them layer by layer inside its backward
  * hook, normalizations/batch_normalization.py:78-124).  `layout` 1: x and gy
  * are stored channels-last, (n, hw, c); 0: (n, c, hw) as in the reference.
  * `items` is a host array (<= 256 entries) read during the call. */

@@ -774,6 +774,27 @@ def test_bn_sample_grads_layouts(ops, shape, channels_last, mean):
     assert rel(host(out), host(ref)) < 5 * 6e-8 * max(4.0, hw ** 0.5)
 
 
+def test_bn_sample_grads_of_mixed_layouts_in_one_group(ops):
+    """Layers of both layouts, in any order, in one grouped call give what each
+    gives alone, bit for bit."""
+    torch.manual_seed(11)
+    pairs = []
+    for k, shape in enumerate([(4, 16, 9, 9), (4, 5), (3, 7, 5, 6), (4, 32, 8, 8),
+                               (2, 70, 66, 63), (4, 64, 1, 1), (6, 12, 7, 7)]):
+        x, gy = torch.randn(shape, device='cuda'), torch.randn(shape,
+                                                               device='cuda')
+        if len(shape) == 4 and k % 3 == 0:
+            x = x.contiguous(memory_format=torch.channels_last)
+            gy = gy.contiguous(memory_format=torch.channels_last)
+        pairs.append((x, gy))
+    alone = [ops.bn_sample_grads(x, gy, 1e-5, 2.0) for x, gy in pairs]
+    for order in (range(7), range(6, -1, -1), (0, 3, 6), (1, 2)):
+        items = [ops.bn_item(*pairs[i], 1e-5, 2.0) for i in order]
+        ops.bn_sample_grads_group(items)
+        for i, it in zip(order, items):
+            assert torch.equal(it.result, alone[i])
+
+
 @pytest.mark.parametrize('shape', [
     (33, 10), (8, 64, 8, 8), (5, 33, 9, 11), (32, 8, 56, 56)])
 @pytest.mark.parametrize('channels_last', [False, True])
