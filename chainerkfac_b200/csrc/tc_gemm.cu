@@ -1074,9 +1074,21 @@ size_t tc_factor_group_workspace_bytes(int count, const FactorJob* jobs,
                                        bool staged) {
   std::vector<FactorJob> gram, pair;
   tc_by_feed(count, jobs, staged, gram, pair);
+  // (a lone factor may have to be gathered, see run_factor_group_tc)
+  if (count == 1) pair.assign(jobs, jobs + 1);
   return std::max(
       gram_workspace_bytes((int)gram.size(), gram.data()),
       tc_pair_workspace_bytes((int)pair.size(), pair.data(), staged));
+}
+
+// Whether calls on this stream are being recorded into a graph.
+static bool stream_captures(cudaStream_t stream) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return cs != cudaStreamCaptureStatusNone;
 }
 
 // Per-device helper stream: the strided and the im2col launch of a grouped
@@ -1340,7 +1352,13 @@ int run_factor_group_tc(int count, const FactorJob* jobs, void* workspace,
                  jobs[i].d);
   }
   std::vector<FactorJob> gram, pair;
-  tc_by_feed(count, jobs, staged, gram, pair);
+  // The feeds of gram.cu copy tables from this call's host memory, which a graph
+  // would read again when it is replayed; the gather kernel takes a lone factor's
+  // descriptors as arguments.
+  if (count == 1 && stream_captures(stream))
+    pair.assign(jobs, jobs + 1);
+  else
+    tc_by_feed(count, jobs, staged, gram, pair);
   // (nothing is queued by a call that fails for want of workspace)
   const size_t need =
       tc_pair_workspace_bytes((int)pair.size(), pair.data(), staged);

@@ -377,6 +377,50 @@ def test_long_contractions_are_cut_in_groups(ops, engine, kblocks, d, ones):
     assert rel(host(outs[3]), host(bd.t() @ bd)) < 6 * 128 * 2.0 ** -25
 
 
+@pytest.mark.parametrize('build', ['dense', 'ones', 'conv_grad', 'conv_1x1',
+                                   'group_of_one'])
+def test_lone_factor_in_a_captured_graph(ops, engine, build):
+    """A factor built on its own can be recorded into a graph: replayed after
+    other builds, it reads its operand anew and nothing else that is gone."""
+    torch.manual_seed(12)
+    shape = (64, 256, 12, 12) if build.startswith('conv') else (9000, 256)
+    x = torch.randn(shape, device='cuda')
+    d = 257 if build == 'ones' else 256
+    out = torch.empty(d, d, device='cuda')
+
+    def call():
+        if build in ('dense', 'ones'):
+            ops.factor_dense(x, build == 'ones', alpha=0.5, out=out)
+        elif build == 'conv_grad':
+            ops.factor_conv_grad(x, alpha=0.5, out=out)
+        elif build == 'conv_1x1':
+            ops.factor_conv_input(x, 1, 1, 0, alpha=0.5, out=out)
+        else:
+            ops.factor_group([ops.dense_item(x, False, 0.5, 0.0, out)],
+                             x.device)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        call()
+    x.normal_()
+    other = torch.randn(20000, 256, device='cuda')
+    for _ in range(20):
+        ops.factor_dense(other, False)
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    m = x.double()
+    m = m.permute(0, 2, 3, 1).reshape(-1, 256) if m.dim() == 4 else m
+    if build == 'ones':
+        m = torch.cat([m, m.new_ones(m.shape[0], 1)], 1)
+    assert rel(host(out), host(0.5 * (m.t() @ m))) < FACTOR_TOL
+    check_symmetric(host(out))
+
+
 def test_group_of_several_batches(ops, engine):
     """Factors whose partial tiles do not fit the workspace of one batch
     (285 MB each), and kinds that come behind them, against fp64."""
