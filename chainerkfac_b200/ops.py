@@ -500,14 +500,17 @@ def class_bounds():
 
 class _PlanDiag(object):
     """The values of an InversePlanSet's ``diag``, each read from its plan when
-    it is asked for; a slice is a view that starts at another factor."""
+    it is asked for; ``at(k)`` counts from factor k on."""
+
+    __slots__ = ('_plans', '_start')
 
     def __init__(self, plans, start=0):
         self._plans, self._start = plans, start
 
+    def at(self, k):
+        return _PlanDiag(self._plans, self._start + k)
+
     def __getitem__(self, i):
-        if isinstance(i, slice):
-            return _PlanDiag(self._plans, self._start + (i.start or 0))
         plan, j = self._plans.where[self._start + i]
         return self._plans.plans[plan].diag[j]
 

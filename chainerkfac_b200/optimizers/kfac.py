@@ -64,7 +64,9 @@ class KFACHook(object):
 
     def __init__(self, fblocks):
         self.fblocks = fblocks
-        self._handles = []       # (block, handle of its module hook)
+        self._handles = []       # handles of the module hooks
+        self._hooked = []        # their blocks, and (hooks of the module, key)
+        self._places = []
         self._active = False
         self._by_array = None
         # optional observers fb -> None, called after the block's own hook
@@ -99,22 +101,27 @@ class KFACHook(object):
             if self.on_backward is not None:
                 self.on_backward(fblock)
 
-    def _direct(self):
-        return type(self) is KFACHook and \
-            'forward_postprocess' not in self.__dict__ and \
-            'backward_preprocess' not in self.__dict__
-
     def _make_forward_hook(self, fblock):
         link = fblock.link
+        mine = link.module
         is_bn = isinstance(link, L.BatchNormalization)
         ref = weakref.ref(self)    # the modules must not keep an optimizer alive
+        # The block this hook was made for gets the call at once; protocol methods
+        # that are overridden (in a subclass, or put on the hook object) are
+        # called by their names, and a block's own is_mine is asked (the stock
+        # one says yes to a call of the block's own module).
+        stock_hook = type(self) is KFACHook
+        stock_block = type(fblock).is_mine in (
+            FB.FisherBlockConnection.is_mine,
+            FB.FisherBlockBatchNormalization.is_mine)
+        block = fblock.__dict__
 
         def hook(module, inputs, output):
             me = ref()
             if me is None or not me._active or not output.requires_grad or \
                     not torch.is_grad_enabled():
                 return
-            if module is not link.module:
+            if module is not mine:
                 return      # a deep copy of the layer, which took the hook along
             x = inputs[0]
             if x.requires_grad:
@@ -128,11 +135,10 @@ class KFACHook(object):
             else:
                 in_data = (x, link.W.data, link.b.data)
             func = fblock.funcclass()
-            # the block this hook was made for; an overridden protocol method
-            # (of a subclass, or put on the hook object) is called by its name
-            if not me._direct():
+            if not stock_hook or 'forward_postprocess' in me.__dict__:
                 me.forward_postprocess(func, in_data)
-            elif fblock.is_mine(func, in_data):
+            elif (stock_block and 'is_mine' not in block) or \
+                    fblock.is_mine(func, in_data):
                 fblock.forward_postprocess(func, in_data)
                 if me.on_forward is not None:
                     me.on_forward(fblock)
@@ -140,9 +146,10 @@ class KFACHook(object):
             def backward(g):
                 if g.requires_grad:
                     g = g.detach()
-                if not me._direct():
+                if not stock_hook or 'backward_preprocess' in me.__dict__:
                     me.backward_preprocess(func, in_data, (g,))
-                elif fblock.is_mine(func, in_data, (g,)):
+                elif (stock_block and 'is_mine' not in block) or \
+                        fblock.is_mine(func, in_data, (g,)):
                     fblock.backward_preprocess(func, in_data, (g,))
                     if me.on_backward is not None:
                         me.on_backward(fblock)
@@ -154,17 +161,22 @@ class KFACHook(object):
     # They are made anew when one is no longer the last hook of its module: the
     # blocks see what the layer hands on behind a program's own hooks.
     def _registered(self):
-        return len(self._handles) == len(self.fblocks) and all(
-            mine is fb and next(reversed(fb.link.module._forward_hooks),
-                                None) == handle.id
-            for (mine, handle), fb in zip(self._handles, self.fblocks))
+        if self._hooked != list(self.fblocks):
+            return False
+        for hooks, key in self._places:
+            if next(reversed(hooks), None) != key:
+                return False
+        return True
 
     def __enter__(self):
         if not self._registered():
             self._remove()
-            self._handles = [
-                (fb, fb.link.module.register_forward_hook(
-                    self._make_forward_hook(fb))) for fb in self.fblocks]
+            self._hooked = list(self.fblocks)
+            for fb in self._hooked:
+                handle = fb.link.module.register_forward_hook(
+                    self._make_forward_hook(fb))
+                self._handles.append(handle)
+                self._places.append((fb.link.module._forward_hooks, handle.id))
         self._active = True
         return self
 
@@ -173,9 +185,9 @@ class KFACHook(object):
         return False
 
     def _remove(self):
-        for _, h in self._handles:
+        for h in self._handles:
             h.remove()
-        self._handles = []
+        self._handles, self._hooked, self._places = [], [], []
 
     def __del__(self):
         try:
@@ -896,7 +908,7 @@ class KFAC(_base.GradientMethod):
             for fb in group:
                 n = len(fb.plan_factors())
                 if n:
-                    fb.set_diag_vals(diag[k:k + n])
+                    fb.set_diag_vals(diag.at(k))
                 k += n
         conn = [fb for fb in fblocks
                 if isinstance(fb, FB.FisherBlockConnection) and

@@ -142,8 +142,8 @@ def test_damping_values_are_those_of_their_step():
     diag = ops._PlanDiag(types.SimpleNamespace(plans=plans, where=where))
     got = []
     fc.set_diag_vals = lambda diag: got.extend([diag[0], diag[1]])
-    for fb, k, n in ((conv, 0, 2), (bn, 2, 1), (fc, 3, 2)):
-        fb.set_diag_vals(diag[k:k + n])
+    for fb, k in ((conv, 0), (bn, 2), (fc, 3)):
+        fb.set_diag_vals(diag.at(k))
     assert (float(got[0]), float(got[1])) == (3.0, 4.0)
     first = conv.diag_val_forward, conv.diag_val_backward, bn.diag_val_backward
     plans[1].diag += 10.0             # the next step's inverses
