@@ -127,7 +127,6 @@ gemm_grouped_kernel(const GemmDesc* __restrict__ descs, int ndesc, float lr,
       if (beta != 0.f) v += beta * (*p);
       *p = v;
       if (mirror) sd.C[(long long)c * sd.ldc + r] = v;
-      if (sd.C2 != nullptr) sd.C2[(long long)r * sd.ldc + c] = v;
     }
   }
 }

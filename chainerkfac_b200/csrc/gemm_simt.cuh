@@ -237,9 +237,19 @@ enum GemmFlags {
   G_KEND_M0 = 8,   // A(k, m) is zero for k > m: stop after the tile's rows
   G_KBEG_M0 = 16,  // A(k, m) is zero for k < m - kbeg_off: start there
   G_PRECOND = 32,  // epilogue splits into kf_W / kf_b and applies momentum
-  G_SAME_AB = 64   // A and B are the same operand (X^T X): a tile on the
+  G_SAME_AB = 64,  // A and B are the same operand (X^T X): a tile on the
                    // diagonal may take its A rows from the staged B rows
+  G_HALF = 128,    // operands are split into two fp16 terms (scales sa, sb)
+  G_PACKED = 256   // operands lie in memory as fp16 terms (ca, cb)
 };
+
+// Operands in fp16 terms lie in chunks of 128 rows (of A^T or B^T) x 32 k, 16 KB
+// each and laid out as the MMAs read them from shared memory: K-major (128-byte
+// rows, hi terms of 32 k, then lo terms) or MN-major (two groups of 64 rows:
+// hi terms of 32 k, 128 bytes each, then lo terms), both 128-byte swizzled.
+// Consecutive k-blocks of a 128-row tile follow each other.
+constexpr int kChunk = 16384;
+enum PackKind { PACK_NONE, PACK_K, PACK_MN };
 
 struct GemmDesc {
   Operand A, B;
@@ -258,8 +268,6 @@ struct GemmDesc {
   long long k_per_split;
   float* partial;          // partial tiles when splits > 1
   const int* gate;         // if set and *gate == 0 the problem is skipped
-  float* C2;               // if set, C's new values are stored here as well
-                           // (same row pitch; plain epilogue only)
   int beta_until;          // > 0: rows from here on ignore beta (a multiple of
                            // the tile rows)
   int kbeg_off;            // G_KBEG_M0: A(k, m) is zero for k < m - kbeg_off
@@ -267,6 +275,17 @@ struct GemmDesc {
   // hi and lo bf16 planes of X^T, see stage.cu
   const void* tmap_hi;
   const void* tmap_lo;
+  // products of operands in two fp16 terms
+  float sa, sb;            // G_HALF: powers of two that scale the operands
+  const unsigned char *ca, *cb;  // G_PACKED: chunk of the first tile and k
+  long long ca_tile, cb_tile;    // bytes from one 128-row tile to the next
+  // the result is also stored in chunks, as an operand of later products: rows
+  // of C are the chunks' rows (PACK_K) or their k (PACK_MN)
+  unsigned char* pack;     // chunk of C's first row and column
+  long long pack_tile;
+  float pack_scale;
+  int pack_kind;
+  const float* unscale;    // if set, C(m, n) = .. + unscale[m] unscale[n] A B
 };
 
 int launch_grouped_gemm(const GemmDesc* descs_dev, int ndesc, int total_tiles,
@@ -283,6 +302,12 @@ int tc_prepare();
 // problems) and choose their width, narrow up to `narrow_max` narrow tiles;
 // returns the launch's tile count.
 constexpr int kTileInline = 8;   // descriptors that fit the kernel arguments
+constexpr int TT_INLINE = kTileInline;
+struct TileInline {
+  int n;                       // 0: descriptors in device memory
+  GemmDesc d[TT_INLINE];
+};
+static_assert(sizeof(TileInline) <= 3800, "kernel argument space");
 int tc_number_tiles(GemmDesc* descs, int n, int narrow_max, int* tile_cols);
 int tc_prepare_tiles();
 // `descs_host`: the same descriptors on the host (small launches pass them as
@@ -291,6 +316,12 @@ int launch_tc_grouped(const GemmDesc* descs_dev, const GemmDesc* descs_host,
                       int ndesc, int total_tiles, int tile_cols, bool precond,
                       float lr, float momentum, cudaStream_t stream);
 int tile_status_read(int* out);
+// The same for operands in fp16 chunks (tc_packed.cu), always in 128 x 128 tiles.
+int packed_number_tiles(GemmDesc* descs, int n);
+int packed_prepare();
+int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
+                  int ndesc, int total_tiles, cudaStream_t stream);
+int packed_status_read(int* out);
 bool tc_desc_has_tails(const GemmDesc& g);
 size_t tc_factor_workspace_bytes(long long rows, int d, bool staged = true);
 size_t tc_lone_workspace_bytes(const Operand& X, long long rows, int d);

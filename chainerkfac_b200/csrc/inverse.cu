@@ -1,10 +1,20 @@
 // Batched damped inverse of symmetric positive definite factors.
 //
-//   W = F + add * I                     (copy; the running average F is kept)
+//   W = S (F + add * I) S               (copy; the running average F is kept)
 //   W = L L^T                           blocked right-looking Cholesky, NB = 128
 //   X = L^-1                            diagonal blocks in the diagonal kernel,
 //                                       then row panels as their columns finish
-//   inv = X^T X                         a panel's contribution at a time
+//   inv = S X^T X S                     a panel's contribution at a time
+//
+// S is diagonal, powers of two that bring the diagonal of W into [1, 4).  That is
+// exact, and bounds what the products below work on, so that they can take it as
+// two fp16 terms (22 significant bits) of one scale per kind:
+//   |W|, |L| < 4, scaled by 2^13;
+//   |X|, scaled by 2^4: a column of X has norm sqrt((W^-1)_jj), and an entry of
+//   4096 means a condition number above 1.6e7, where a Cholesky factorisation
+//   in fp32 has no correct digit left (such entries saturate); small entries
+//   are held to 2^-29, the diagonal of X is 1/2 or more;
+//   T = L X, of at most twice the norm of a column of X, scaled by 2^3.
 //
 // A plan precomputes, for a fixed set of matrices, the descriptor lists of
 // every grouped-GEMM launch; running it replays them, each launch covering all
@@ -29,8 +39,7 @@ struct MatInfo {
   // lines, so that every row is read and written as 16-byte words)
   float* W;       // damped factor, then L (and T^T above the diagonal)
   float* X;       // L^-1
-  float* V;       // blocks of W before a panel solve overwrites them; T of the
-                  // doubling; X R of the refinement
+  float* V;       // T of the doubling; X R of the refinement
   int d, ld;
   int partner;
   int role;
@@ -38,7 +47,22 @@ struct MatInfo {
   float scale;
   float l2b;      // role 2: floor of the second half of the diagonal
   int id;         // index of the matrix in the plan
+  float* diag;    // diagonal of F, `ld` floats (zeros past d)
+  float* S;       // the scales, likewise
+  // L and X in fp16 chunks (see GemmDesc; NULL: not used), L by 128-row tile,
+  // X by 128-column tile, `tile` bytes apart
+  unsigned char *PL, *PX;
+  long long tile;
 };
+constexpr float kScaleL = 8192.f, kScaleX = 16.f, kScaleT = 8.f;
+
+
+__host__ __device__ static int matrix_pitch(int d) { return (d + 31) & ~31; }
+
+__host__ __device__ static size_t matrix_bytes(int d) {
+  const size_t bytes = (size_t)d * matrix_pitch(d) * sizeof(float);
+  return (bytes + 255) & ~(size_t)255;
+}
 
 // Per-run arguments, kept in device memory so that a captured CUDA graph of
 // the plan's launches can be replayed with new values: a one-thread kernel
@@ -59,12 +83,16 @@ __global__ void set_run_params_kernel(RunParams* prm, float damping,
   prm->refine_threshold = refine_threshold;
 }
 
+// Also keeps the diagonal (the scales are made of it).
 __global__ void trace_kernel(const MatInfo* __restrict__ mats,
                              float* __restrict__ trace, int* __restrict__ info) {
   const MatInfo mi = mats[blockIdx.x];
   float s = 0.f;
-  for (int i = threadIdx.x; i < mi.d; i += blockDim.x)
-    s += mi.F[(long long)i * mi.d + i];
+  for (int i = threadIdx.x; i < mi.d; i += blockDim.x) {
+    const float v = mi.F[(long long)i * mi.d + i];
+    mi.diag[i] = v;
+    s += v;
+  }
   __shared__ float sh[32];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
@@ -79,87 +107,100 @@ __global__ void trace_kernel(const MatInfo* __restrict__ mats,
   }
 }
 
-__global__ void damping_kernel(const MatInfo* __restrict__ mats, int count,
-                               const float* __restrict__ trace,
-                               const RunParams* __restrict__ prm,
-                               float* __restrict__ add,
-                               float* __restrict__ add2,
-                               float* __restrict__ add_out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
+// What is added to the diagonal of matrix i (role 2: to its first and second
+// half, scale and shift parameters with floors of their own).
+__device__ __forceinline__ float2 damping_of(const MatInfo* mats, int i,
+                                             const MatInfo& mi,
+                                             const float* trace,
+                                             const RunParams* prm) {
   const float damping = prm->damping;
-  const int use_pi = prm->use_pi;
-  const MatInfo mi = mats[i];
-  float g = fmaxf(mi.l2, damping);
-  float v, v2;
-  if (mi.role == 2) {
-    // first half of the diagonal (scale parameters) and second half (shift
-    // parameters) have their own floors
-    v = g * mi.scale;
-    v2 = fmaxf(mi.l2b, damping) * mi.scale;
-  } else {
-    float r = sqrtf(g);
-    float pi = 1.f;
-    if (use_pi && mi.partner >= 0) {
-      const MatInfo mp = mats[mi.partner];
-      // pi = sqrt(tr(A) dim(G) / (tr(G) dim(A))) with A the forward factor
-      float tA = mi.role == 0 ? trace[i] : trace[mi.partner];
-      float tG = mi.role == 0 ? trace[mi.partner] : trace[i];
-      float dA = (float)(mi.role == 0 ? mi.d : mp.d);
-      float dG = (float)(mi.role == 0 ? mp.d : mi.d);
-      pi = sqrtf((tA * dG) / (tG * dA));
-    }
-    v = mi.role == 0 ? pi * r : (1.f / pi) * r;
-    v2 = v;
+  const float g = fmaxf(mi.l2, damping);
+  if (mi.role == 2)
+    return make_float2(g * mi.scale, fmaxf(mi.l2b, damping) * mi.scale);
+  const float r = sqrtf(g);
+  float pi = 1.f;
+  if (prm->use_pi && mi.partner >= 0) {
+    const MatInfo& mp = mats[mi.partner];
+    // pi = sqrt(tr(A) dim(G) / (tr(G) dim(A))) with A the forward factor
+    float tA = mi.role == 0 ? trace[i] : trace[mi.partner];
+    float tG = mi.role == 0 ? trace[mi.partner] : trace[i];
+    float dA = (float)(mi.role == 0 ? mi.d : mp.d);
+    float dG = (float)(mi.role == 0 ? mp.d : mi.d);
+    pi = sqrtf((tA * dG) / (tG * dA));
   }
-  add[i] = v;
-  add2[i] = v2;
-  if (add_out) add_out[i] = v;
+  const float v = mi.role == 0 ? pi * r : (1.f / pi) * r;
+  return make_float2(v, v);
 }
 
-// W = F + add * I, blockIdx.y = matrix, blockIdx.x strides over rows.  Only
-// the lower triangle and the rest of each diagonal 128-block (which the
+// Power of two s with s^2 x in [1, 4).  An x that is no positive normal number
+// fails as a pivot and stays as it is.
+__device__ __forceinline__ float equil_scale(float x) {
+  if (!(x >= 1.17549435e-38f)) return 1.f;
+  const int e = (int)(__float_as_uint(x) >> 23) - 127;
+  return __uint_as_float((unsigned)(127 - (e >> 1)) << 23);
+}
+
+// W = S (F + add * I) S, blockIdx.y = matrix, blockIdx.x strides over rows.
+// Only the lower triangle and the rest of each diagonal 128-block (which the
 // trailing updates read-modify-write) is ever used, so only that is copied.
-// With `dual` the first block column below the first diagonal block is also
-// stored in V (see the look-ahead of the Cholesky).
+// `equil` off: S = I.
 __global__ void damp_copy_kernel(const MatInfo* __restrict__ mats,
-                                 const float* __restrict__ add,
-                                 const float* __restrict__ add2, int dual) {
+                                 const float* __restrict__ trace,
+                                 const RunParams* __restrict__ prm,
+                                 float* __restrict__ add,
+                                 float* __restrict__ add2,
+                                 float* __restrict__ add_out, int equil) {
   const MatInfo mi = mats[blockIdx.y];
-  const float a_first = add[blockIdx.y], a_second = add2[blockIdx.y];
+  const float2 ad = damping_of(mats, blockIdx.y, mi, trace, prm);
+  const float a_first = ad.x, a_second = ad.y;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    add[blockIdx.y] = a_first;
+    add2[blockIdx.y] = a_second;
+    if (add_out) add_out[blockIdx.y] = a_first;
+  }
   const int d = mi.d;
+  auto damp = [&](int r) {
+    return (mi.role == 2 && 2 * r >= d) ? a_second : a_first;
+  };
+  auto scale = [&](int r, float f) {
+    return equil ? equil_scale(f + damp(r)) : 1.f;
+  };
   const bool vec = (d & 3) == 0 &&
                    ((reinterpret_cast<uintptr_t>(mi.F) |
-                     reinterpret_cast<uintptr_t>(mi.W) |
-                     reinterpret_cast<uintptr_t>(mi.V)) & 15) == 0;
+                     reinterpret_cast<uintptr_t>(mi.W)) & 15) == 0;
   for (int r = blockIdx.x; r < d; r += gridDim.x) {
-    const float a = (mi.role == 2 && 2 * r >= d) ? a_second : a_first;
+    const float a = damp(r), sr = scale(r, mi.diag[r]);
+    if (threadIdx.x == 0) mi.S[r] = sr;
     const int cend = min(d, (r | (DB - 1)) + 1);
     const float* src = mi.F + (long long)r * d;
     float* dst = mi.W + (long long)r * mi.ld;
     if (vec) {
       // cend is a multiple of 128 or equals d, itself a multiple of 4 here
       const float4* s4 = reinterpret_cast<const float4*>(src);
+      const float4* g4 = reinterpret_cast<const float4*>(mi.diag);
       float4* d4 = reinterpret_cast<float4*>(dst);
 #pragma unroll 4
       for (int c4 = threadIdx.x; c4 < (cend >> 2); c4 += blockDim.x) {
         float4 v = s4[c4];
+        const float4 g = g4[c4];
         if ((r >> 2) == c4) {
           if ((r & 3) == 0) v.x += a;
           else if ((r & 3) == 1) v.y += a;
           else if ((r & 3) == 2) v.z += a;
           else v.w += a;
         }
+        v.x = v.x * sr * scale(4 * c4, g.x);
+        v.y = v.y * sr * scale(4 * c4 + 1, g.y);
+        v.z = v.z * sr * scale(4 * c4 + 2, g.z);
+        v.w = v.w * sr * scale(4 * c4 + 3, g.w);
         d4[c4] = v;
-        if (dual && r >= DB && c4 < DB / 4)
-          reinterpret_cast<float4*>(mi.V + (long long)r * mi.ld)[c4] = v;
       }
     } else {
       for (int c = threadIdx.x; c < cend; c += blockDim.x) {
         float v = src[c];
         if (r == c) v += a;
+        v = v * sr * scale(c, mi.diag[c]);
         dst[c] = v;
-        if (dual && r >= DB && c < DB) mi.V[(long long)r * mi.ld + c] = v;
       }
     }
   }
@@ -260,8 +301,8 @@ __device__ __forceinline__ void look_begin(LookControl* ctl) {
 // The diagonal block of step k has received the updates of all steps before
 // k - 1; the update of step k - 1,
 //   D = W_kk - L' L'^T,  L' = A' X_pp^T,
-// is computed here from A' (block (k, k-1) as it was before step k-1's panel
-// solve overwrote it; the updates keep a second copy of it in V) and X_pp (inverse of the previous diagonal block's factor),
+// is computed here from A' (block (k, k-1), which the panel solve of step k-1
+// leaves as it was) and X_pp (inverse of the previous diagonal block's factor),
 // so that this kernel does not have to wait for the panel solve and panel
 // update of step k - 1.  Both products run on the tensor cores (tcgen05,
 // split TF32, accumulators in tensor memory).  All global loads are in flight
@@ -274,7 +315,7 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
                                                LookControl* ctl) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long ld = mi.ld;
-  const float* Ap = mi.V + (long long)o * ld + (o - DB);
+  const float* Ap = mi.W + (long long)o * ld + (o - DB);
   const float* Xp = mi.X + (long long)(o - DB) * ld + (o - DB);
   float4 va[4][2], vx[4][2];
 #pragma unroll
@@ -752,7 +793,7 @@ __device__ __forceinline__ void diag_update_block(DiagSmem& sm, int r, int half,
 template <bool LOOK>
 __global__ void __launch_bounds__(DT, 1)
 chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
-                 int* __restrict__ info) {
+                 int* __restrict__ info, int pack) {
   extern __shared__ __align__(16) float dsm[];
   DiagSmem& sm = *reinterpret_cast<DiagSmem*>(dsm);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -849,6 +890,12 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
   // 16-byte word per lane) into four contiguous row pieces.  The part above
   // the diagonal sub-blocks was zeroed when the plan was made.
   float* Xd = mi.X + (long long)o * ld + o;
+  // (from X and d: two more pointers across the chain cost registers that it
+  // does not have)
+  const long long ptile =
+      (long long)((mi.d + DB - 1) / DB) * (DB / 32) * kChunk;
+  unsigned char* const px = reinterpret_cast<unsigned char*>(mi.X) +
+                            matrix_bytes(mi.d);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int r = 4 * warp + 64 * h, bi = r >> 5;
@@ -863,12 +910,37 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int c = SB * u + lane;
-      if (u > bi || c >= bs) continue;
-      float* dst = Xd + r * ld + c;
-      dst[0] = v[u].x;
-      if (r + 1 < bs) dst[ld] = v[u].y;
-      if (r + 2 < bs) dst[2 * ld] = v[u].z;
-      if (r + 3 < bs) dst[3 * ld] = v[u].w;
+      if (u > bi) continue;
+      if (c < bs) {
+        float* dst = Xd + r * ld + c;
+        dst[0] = v[u].x;
+        if (r + 1 < bs) dst[ld] = v[u].y;
+        if (r + 2 < bs) dst[2 * ld] = v[u].z;
+        if (r + 3 < bs) dst[3 * ld] = v[u].w;
+      }
+      if (pack) {
+        // the same as fp16 terms: an even lane takes rows r, r + 1 of its and
+        // the next column, an odd one rows r + 2, r + 3 (columns past bs are
+        // zero above the diagonal; their chunks exist)
+        const bool odd = lane & 1;
+        const float p0 = __shfl_xor_sync(0xffffffffu, odd ? v[u].x : v[u].z, 1);
+        const float p1 = __shfl_xor_sync(0xffffffffu, odd ? v[u].y : v[u].w, 1);
+        const int k = r + (odd ? 2 : 0);
+        unsigned char* q = px + step * ptile +
+                           (long long)((o + k) >> 5) * kChunk +
+                           (u >> 1) * 8192 + 4 * ((c & 7) >> 1);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          if (k + e >= bs) continue;
+          unsigned hi, lo;
+          const float x0 = e == 0 ? (odd ? p0 : v[u].x) : (odd ? p1 : v[u].y);
+          const float x1 = e == 0 ? (odd ? v[u].z : p0) : (odd ? v[u].w : p1);
+          split_half2(kScaleX * x0, kScaleX * x1, hi, lo);
+          unsigned char* w = q + sw128_chunk_off((k + e) & 31, (c & 63) >> 3);
+          *reinterpret_cast<unsigned*>(w) = hi;
+          *reinterpret_cast<unsigned*>(w + 4096) = lo;
+        }
+      }
     }
   }
 }
@@ -1110,6 +1182,7 @@ struct Launch {
   int wait_ev[3];
   int rec_ev;
   bool look;     // diag kernel: with the look-ahead prologue
+  bool packed;   // grouped gemm: operands in fp16 chunks
 
   void wait(int ev) {
     if (ev < 0) return;
@@ -1134,12 +1207,13 @@ struct kfac_inverse_plan {
   MatInfo* mats_dev;
   float* trace_dev;
   float* add_dev;
+  float* scale_dev;        // diag and S of every matrix
   int* info_dev;
   MatInfo* sorted_dev;     // mats_dev, largest first (diagonal kernels)
   GemmDesc* descs_dev;
   std::vector<GemmDesc> descs;       // the same on the host
   std::vector<Launch> launches;
-  bool use_tc;
+  bool use_tc, packed;
   // refinement (see refine_* kernels)
   float* add2_dev;
   int n_refine;
@@ -1168,18 +1242,20 @@ struct kfac_inverse_plan {
   bool graph_ok;
 };
 
-static int matrix_pitch(int d) { return (d + 31) & ~31; }
-
-static size_t matrix_bytes(int d) {
-  const size_t bytes = (size_t)d * matrix_pitch(d) * sizeof(float);
-  return (bytes + 255) & ~(size_t)255;
+// fp16 chunks of a matrix: tiles of 128 rows, 32 k a chunk.
+static size_t chunk_tile_bytes(int d) {
+  return (size_t)((d + DB - 1) / DB) * (DB / 32) * kChunk;
+}
+static size_t chunk_bytes(int d) {
+  return (size_t)((d + DB - 1) / DB) * chunk_tile_bytes(d);
 }
 
 extern "C" size_t kfac_inverse_workspace_bytes(int count, const int* dims) {
   size_t total = 0;
   for (int i = 0; i < count; ++i) {
     if (dims[i] <= 0) return 0;
-    total += 3 * matrix_bytes(dims[i]);              // W, X, V
+    total += 3 * matrix_bytes(dims[i]) +             // W, X, V
+             2 * chunk_bytes(dims[i]);               // L and X in chunks
   }
   return total;
 }
@@ -1214,6 +1290,11 @@ extern "C" int kfac_inverse_plan_create(
   // Blocks of X above the diagonal blocks are never written and are read as
   // zeros by the wide tiles of the triangular-inverse products.
   KFAC_CUDA(cudaMemset(workspace, 0, need));
+  const bool use_tc = engine() == 1;
+  // fp16 terms: every operand of the products has rows of 16-byte words
+  const int half =
+      use_tc && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 ? G_HALF : 0;
+  const int packed = half ? G_PACKED : 0;
   std::vector<MatInfo> mats(count);
   char* ws = static_cast<char*>(workspace);
   int dmax = 0;
@@ -1223,8 +1304,8 @@ extern "C" int kfac_inverse_plan_create(
     m.F = factors[i];
     m.inv = inverses[i];
     m.W = reinterpret_cast<float*>(ws); ws += bytes;
-    m.X = reinterpret_cast<float*>(ws); ws += bytes;
     m.V = reinterpret_cast<float*>(ws); ws += bytes;
+    m.X = reinterpret_cast<float*>(ws); ws += bytes;
     m.d = dims[i];
     m.ld = matrix_pitch(dims[i]);
     m.partner = partner ? partner[i] : -1;
@@ -1233,7 +1314,33 @@ extern "C" int kfac_inverse_plan_create(
     m.scale = scale ? scale[i] : 1.f;
     m.l2b = m.l2;
     m.id = i;
+    if (half) {
+      m.tile = chunk_tile_bytes(dims[i]);
+      // (the diagonal kernel takes PX to lie right behind X)
+      m.PX = reinterpret_cast<unsigned char*>(ws); ws += chunk_bytes(dims[i]);
+      m.PL = reinterpret_cast<unsigned char*>(ws); ws += chunk_bytes(dims[i]);
+    } else {
+      m.tile = 0;
+      m.PL = m.PX = nullptr;
+    }
     dmax = std::max(dmax, dims[i]);
+  }
+  // diagonals and scales
+  size_t n_scale = 0;
+  for (const MatInfo& m : mats) n_scale += 2 * (size_t)m.ld;
+  float* scale_dev = nullptr;
+  cudaError_t e = cudaMalloc(&scale_dev, n_scale * sizeof(float));
+  if (e == cudaSuccess) e = cudaMemset(scale_dev, 0, n_scale * sizeof(float));
+  if (e != cudaSuccess) {
+    cudaFree(scale_dev);
+    return fail(KFAC_ERR_CUDA, "inverse_plan_create: %s", cudaGetErrorString(e));
+  }
+  {
+    float* sc = scale_dev;
+    for (MatInfo& m : mats) {
+      m.diag = sc; sc += m.ld;
+      m.S = sc; sc += m.ld;
+    }
   }
   // large matrices first: their tiles are scheduled first
   std::vector<int> order(count);
@@ -1243,10 +1350,25 @@ extern "C" int kfac_inverse_plan_create(
 
   std::vector<GemmDesc> descs;
   std::vector<Launch> launches;
-  const bool use_tc = engine() == 1;
+  // operands in chunks: L from row r and column k on, X from row k and column m
+  auto chunk_l = [](const MatInfo& m, long long r, long long k) {
+    return m.PL + (r / DB) * m.tile + k / 32 * kChunk;
+  };
+  auto chunk_x = [](const MatInfo& m, long long k, long long c) {
+    return m.PX + (c / DB) * m.tile + k / 32 * kChunk;
+  };
+  // products of rows ra and rb of L, from column k on
+  auto set_l = [&](GemmDesc& g, const MatInfo& m, long long ra, long long rb,
+                   long long k) {
+    g.sa = g.sb = kScaleL;
+    if (!packed) return;
+    g.ca = chunk_l(m, ra, k);
+    g.cb = chunk_l(m, rb, k);
+    g.ca_tile = g.cb_tile = m.tile;
+  };
 
   int n_events = 0;
-  const bool look = use_tc && [] {
+  const bool look = packed && [] {
     const char* env = getenv("KFAC_INVERSE_LOOKAHEAD");
     return !(env && env[0] == '0');
   }();
@@ -1273,6 +1395,9 @@ extern "C" int kfac_inverse_plan_create(
     g.ntiles = 0;
     g.k_per_split = 0;
     g.partial = nullptr;
+    // (the scales of the fp16 terms come out again with alpha)
+    if (g.flags & (G_HALF | G_PACKED)) g.alpha /= g.sa * g.sb;
+    l.packed = (g.flags & G_PACKED) != 0;
     descs.push_back(g);
     l.n += 1;
   };
@@ -1280,8 +1405,10 @@ extern "C" int kfac_inverse_plan_create(
   auto end_gemm = [&](Launch& l, bool record) {
     if (l.n == 0) return -1;
     if (use_tc && l.kind == 1)
-      l.tiles = tc_number_tiles(&descs[l.off], l.n, 3 * sm_count() / 4,
-                                &l.tile_cols);
+      l.tiles = l.packed
+                    ? packed_number_tiles(&descs[l.off], l.n)
+                    : tc_number_tiles(&descs[l.off], l.n, 3 * sm_count() / 4,
+                                      &l.tile_cols);
     if (record) l.rec_ev = n_events++;
     launches.push_back(l);
     return l.rec_ev;
@@ -1300,21 +1427,19 @@ extern "C" int kfac_inverse_plan_create(
       look && dmax <= 2 * PW && step_tiles <= sm_count() ? 2 * PW : PW;
 
   int prev_far_ev = -1;
-  // Two-level right-looking Cholesky: panels of PW columns are factored by
-  // 128-wide inner steps whose updates stay inside the panel (short
-  // contractions, little work); the bulk of the flops is the update of the
-  // trailing matrix with the whole panel (contraction length CW).
+  // Two-level Cholesky: panels of CW columns are factored by 128-wide inner steps
+  // whose updates stay inside the panel (short contractions, little work).  A
+  // panel's columns get the rest in two parts: everything but the panel right
+  // before them while that one's chain runs (far stream; a contraction over all
+  // panels so far, so that C is passed over once and not once per panel), and
+  // that panel's share when its chain ends (near).
   //
   // The chain carries the diagonal kernels; inside a panel the diagonal
   // kernel of step k applies step k-1's update to its own block itself
   // (diag_lookahead), so it only waits for the panel update of step k-2.  The
   // panel solves and panel updates of the steps run on the bulk stream behind
-  // the chain, and the part of a panel's trailing update that the next panel
-  // does not need runs on the far stream.  Panel updates (and the near part of
-  // a trailing update, and the damped copy for the first block column) store
-  // their results a second time in V: that copy of block (k, k-1) is what
-  // diag_lookahead reads while the panel solve of step k-1 overwrites the
-  // original.
+  // the chain.  A panel solve leaves W as it is (the look-ahead reads it) and
+  // stores L as fp16 chunks, which is how every product reads it.
   //
   // The inverse grows with the factor, a row panel at a time: with X = L^-1,
   //   T = L_p X_<p,  X_p = -X_pp T  (X_pp by doubling from the 128-blocks),
@@ -1345,14 +1470,25 @@ extern "C" int kfac_inverse_plan_create(
           g.B = strided_operand(m.X + s * ld + s, ld, 1, b);
           g.C = m.V + (s + b) * ld + s;
           g.ldc = ld; g.M = r; g.N = b; g.K = b;
-          g.alpha = 1.f; g.beta = 0.f; g.flags = G_KBEG_N0;
+          g.alpha = 1.f; g.beta = 0.f; g.flags = G_KBEG_N0 | packed;
+          g.sa = kScaleL; g.sb = kScaleX;
+          if (packed) {
+            g.ca = chunk_l(m, s + b, s);
+            g.cb = chunk_x(m, s, s);
+            g.ca_tile = g.cb_tile = m.tile;
+          }
           push_desc(g1, g);
           GemmDesc h = {};
           h.A = strided_operand(m.X + (s + b) * ld + s + b, 1, ld, r);
           h.B = strided_operand(m.V + (s + b) * ld + s, ld, 1, b);
           h.C = m.X + (s + b) * ld + s;
           h.ldc = ld; h.M = r; h.N = b; h.K = r;
-          h.alpha = -1.f; h.beta = 0.f; h.flags = G_KEND_M0;
+          h.alpha = -1.f; h.beta = 0.f; h.flags = G_KEND_M0 | half;
+          h.sa = kScaleX; h.sb = kScaleT;
+          if (packed) {
+            h.pack = chunk_x(m, s + b, s); h.pack_tile = m.tile;
+            h.pack_scale = kScaleX; h.pack_kind = PACK_MN;
+          }
           second.push_back(h);
         }
       }
@@ -1378,7 +1514,13 @@ extern "C" int kfac_inverse_plan_create(
         g.B = strided_operand(m.W + po, 1, ld, po);   // B(k, n) = T^T[n][k]
         g.C = m.X + po * ld;
         g.ldc = ld; g.M = w; g.N = po; g.K = w;
-        g.alpha = -1.f; g.beta = 0.f; g.flags = G_KEND_M0;
+        g.alpha = -1.f; g.beta = 0.f; g.flags = G_KEND_M0 | half;
+        g.sa = kScaleX; g.sb = kScaleT;
+        if (packed) {              // nothing reads these rows but as chunks
+          g.C = nullptr;
+          g.pack = chunk_x(m, po, 0); g.pack_tile = m.tile;
+          g.pack_scale = kScaleX; g.pack_kind = PACK_MN;
+        }
         push_desc(rows, g);
       }
     }
@@ -1391,16 +1533,27 @@ extern "C" int kfac_inverse_plan_create(
     // the product, behind the rows (or, for a single panel, the doubling)
     Launch prod = begin_gemm(s_prod);
     for (int i : order) {
-      const int d = dims[i], end = std::min(po + PW, d), w = end - po;
-      if (w <= 0) continue;
+      const int d = dims[i], end = std::min(po + PW, d);
+      if (end <= po) continue;
+      // two panels at a time (half as many passes over inv), but for the last
+      // one, which the end of the run waits for
+      const bool odd = (po / PW) & 1, last = end == d;
+      if (!odd && !last && po + 2 * PW < d) continue;
+      const int ks = odd && !last ? po - PW : po;
       const MatInfo& m = mats[i];
       GemmDesc g = {};
-      g.A = strided_operand(m.X + (long long)po * m.ld, m.ld, 1, end);
+      g.A = strided_operand(m.X + (long long)ks * m.ld, m.ld, 1, end);
       g.B = g.A;
-      g.C = m.inv; g.ldc = d; g.M = end; g.N = end; g.K = w;
-      g.alpha = 1.f; g.beta = po > 0 ? 1.f : 0.f;
-      g.beta_until = po; g.kbeg_off = po;
-      g.flags = G_LOWER | G_KBEG_M0 | G_SAME_AB | (end == d ? G_MIRROR : 0);
+      g.C = m.inv; g.ldc = d; g.M = end; g.N = end; g.K = end - ks;
+      g.alpha = 1.f; g.beta = ks > 0 ? 1.f : 0.f;
+      g.beta_until = ks; g.kbeg_off = ks;
+      g.flags = G_LOWER | G_KBEG_M0 | G_SAME_AB | (last ? G_MIRROR : 0) | packed;
+      g.sa = g.sb = kScaleX;
+      if (packed) {
+        g.ca = g.cb = chunk_x(m, ks, 0);
+        g.ca_tile = g.cb_tile = m.tile;
+      }
+      g.unscale = m.S;
       push_desc(prod, g);
     }
     if (look && rows_ev < 0 && !first) {
@@ -1424,7 +1577,13 @@ extern "C" int kfac_inverse_plan_create(
       g.B = strided_operand(m.W + pend * ld, 1, ld, w);
       g.C = m.W + pend;
       g.ldc = ld; g.M = pend; g.N = w; g.K = pend;
-      g.alpha = 1.f; g.beta = 0.f; g.flags = G_KBEG_M0;
+      g.alpha = 1.f; g.beta = 0.f; g.flags = G_KBEG_M0 | packed;
+      g.sa = kScaleX; g.sb = kScaleL;
+      if (packed) {
+        g.ca = chunk_x(m, 0, 0);
+        g.cb = chunk_l(m, pend, 0);
+        g.ca_tile = g.cb_tile = m.tile;
+      }
       push_desc(next_t, g);
     }
     if (look && first) next_t.wait(bulk_ev);
@@ -1459,7 +1618,13 @@ extern "C" int kfac_inverse_plan_create(
         g.A = strided_operand(panel, 1, ld, M);
         g.B = strided_operand(m.X + o * ld + o, 1, ld, DB);
         g.C = panel; g.ldc = ld; g.M = M; g.N = DB; g.K = DB;
-        g.alpha = 1.f; g.beta = 0.f; g.flags = 0;
+        g.alpha = 1.f; g.beta = 0.f; g.flags = half;
+        g.sa = kScaleL; g.sb = kScaleX;
+        if (packed) {              // L is read as chunks only
+          g.C = nullptr;
+          g.pack = chunk_l(m, o + DB, o); g.pack_tile = m.tile;
+          g.pack_scale = kScaleL; g.pack_kind = PACK_K;
+        }
         push_desc(trsm, g);
       }
       trsm.wait(diag_ev[o / DB]);
@@ -1485,8 +1650,8 @@ extern "C" int kfac_inverse_plan_create(
         g.B = strided_operand(m.W + (o + DB) * ld + o, 1, ld, N);
         g.C = m.W + coff;
         g.ldc = ld; g.M = M; g.N = N; g.K = DB;
-        g.alpha = -1.f; g.beta = 1.f; g.flags = 0;
-        if (look) g.C2 = m.V + coff;
+        g.alpha = -1.f; g.beta = 1.f; g.flags = packed;
+        set_l(g, m, o + DB + skip, o + DB, o);
         push_desc(upd, g);
       }
       upd_ev[o / DB] = end_gemm(upd, look);
@@ -1495,12 +1660,11 @@ extern "C" int kfac_inverse_plan_create(
       if ((o + DB) % PW == 0 && o + DB < co + inner) row_panel(o + DB - PW);
     }
 
-    // Update of the trailing matrix with the finished panel, in two parts:
-    // the columns of the next panel (needed before the chain can go on) on
-    // the chain's stream, the columns beyond them on the far stream, next to
-    // the next panel's chain.  Both parts of one panel touch disjoint tiles;
-    // parts of successive panels that touch the same tiles are ordered by
-    // events (next-panel part p+1 after far part p) or by stream order.
+    // Updates behind the finished panel: the columns of the next panel with this
+    // one (needed before the chain can go on) on the chain's stream, those of
+    // the panel after it with all panels so far on the far stream, next to the
+    // next panel's chain.  What touches the same tiles is ordered by events
+    // (near of a panel after far of the one before).
     Launch near = begin_gemm(S_CHAIN);
     std::vector<GemmDesc> far_descs;
     for (int i : order) {
@@ -1518,8 +1682,8 @@ extern "C" int kfac_inverse_plan_create(
         g.B = g.A;
         g.C = m.W + coff;
         g.ldc = ld; g.M = N1; g.N = N1; g.K = CW;
-        g.alpha = -1.f; g.beta = 1.f; g.flags = G_LOWER | G_SAME_AB;
-        if (look) g.C2 = m.V + coff;
+        g.alpha = -1.f; g.beta = 1.f; g.flags = G_LOWER | G_SAME_AB | packed;
+        set_l(g, m, co + CW, co + CW, co);
         push_desc(near, g);
       }
       if (M > N1) {
@@ -1530,16 +1694,32 @@ extern "C" int kfac_inverse_plan_create(
         g.B = strided_operand(panel, 1, ld, N1);
         g.C = m.W + coff;
         g.ldc = ld; g.M = M - N1; g.N = N1; g.K = CW;
-        g.alpha = -1.f; g.beta = 1.f; g.flags = 0;
-        if (look) g.C2 = m.V + coff;
+        g.alpha = -1.f; g.beta = 1.f; g.flags = packed;
+        set_l(g, m, co + CW + N1, co + CW, co);
         push_desc(near, g);
-        GemmDesc h = {};     // everything beyond the next panel's columns
-        h.A = strided_operand(below, 1, ld, M - N1);
+      }
+      // the columns of the panel after the next: all panels so far
+      const int f = co + 2 * CW, F = d - f;
+      if (F > 0) {
+        const int N2 = std::min(CW, F);
+        GemmDesc h = {};     // square block on the diagonal
+        h.A = strided_operand(m.W + (long long)f * ld, 1, ld, N2);
         h.B = h.A;
-        h.C = m.W + (co + CW + N1) * ld + (co + CW + N1);
-        h.ldc = ld; h.M = M - N1; h.N = M - N1; h.K = CW;
-        h.alpha = -1.f; h.beta = 1.f; h.flags = G_LOWER | G_SAME_AB;
+        h.C = m.W + (long long)f * ld + f;
+        h.ldc = ld; h.M = N2; h.N = N2; h.K = co + CW;
+        h.alpha = -1.f; h.beta = 1.f; h.flags = G_LOWER | G_SAME_AB | packed;
+        set_l(h, m, f, f, 0);
         far_descs.push_back(h);
+        if (F > N2) {
+          GemmDesc r = {};   // rectangle below it
+          r.A = strided_operand(m.W + (long long)(f + N2) * ld, 1, ld, F - N2);
+          r.B = strided_operand(m.W + (long long)f * ld, 1, ld, N2);
+          r.C = m.W + (long long)(f + N2) * ld + f;
+          r.ldc = ld; r.M = F - N2; r.N = N2; r.K = co + CW;
+          r.alpha = -1.f; r.beta = 1.f; r.flags = packed;
+          set_l(r, m, f + N2, f, 0);
+          far_descs.push_back(r);
+        }
       }
     }
     int panel_ev = last_solve_ev;
@@ -1585,6 +1765,7 @@ extern "C" int kfac_inverse_plan_create(
   p->count = count;
   p->launches = launches;
   p->use_tc = use_tc;
+  p->packed = packed != 0;
   p->mats_dev = nullptr; p->trace_dev = nullptr; p->add_dev = nullptr;
   p->info_dev = nullptr; p->sorted_dev = nullptr; p->descs_dev = nullptr;
   p->add2_dev = nullptr; p->refine_items_dev = nullptr;
@@ -1609,7 +1790,8 @@ extern "C" int kfac_inverse_plan_create(
     const char* env = getenv("KFAC_INVERSE_GRAPH");
     p->graph_ok = !(env && env[0] == '0');
   }
-  cudaError_t e = cudaGetDevice(&p->device);
+  p->scale_dev = scale_dev;
+  e = cudaGetDevice(&p->device);
   if (e == cudaSuccess) e = cudaMalloc(&p->params_dev, sizeof(RunParams));
   if (e == cudaSuccess)
     e = cudaEventCreateWithFlags(&p->fork_ev, cudaEventDisableTiming);
@@ -1680,7 +1862,8 @@ extern "C" int kfac_inverse_plan_create(
     return fail(KFAC_ERR_CUDA, "inverse_plan_create: %s", cudaGetErrorString(e));
   }
   if (use_tc) {
-    const int rc = tc_prepare_tiles();
+    int rc = tc_prepare_tiles();
+    if (rc == KFAC_OK) rc = packed_prepare();
     if (rc != KFAC_OK) {
       kfac_inverse_plan_destroy(p);
       return rc;
@@ -1704,15 +1887,12 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
   }
   trace_kernel<<<p->count, 256, 0, st>>>(p->mats_dev, p->trace_dev, info);
   KFAC_LAUNCH_CHECK("trace_kernel");
-  damping_kernel<<<ceil_div(p->count, 128), 128, 0, st>>>(
-      p->mats_dev, p->count, p->trace_dev, p->params_dev, p->add_dev,
-      p->add2_dev, diag_dev);
-  KFAC_LAUNCH_CHECK("damping_kernel");
   {
     // a block copies about four rows of the largest matrix
     dim3 grid(std::max(1, std::min(512, p->dmax / 4)), p->count);
-    damp_copy_kernel<<<grid, 256, 0, st>>>(p->mats_dev, p->add_dev,
-                                           p->add2_dev, p->look ? 1 : 0);
+    damp_copy_kernel<<<grid, 256, 0, st>>>(
+        p->mats_dev, p->trace_dev, p->params_dev, p->add_dev, p->add2_dev,
+        diag_dev, p->use_tc ? 1 : 0);
     KFAC_LAUNCH_CHECK("damp_copy_kernel");
   }
   for (const Launch& l : p->launches) {
@@ -1722,13 +1902,16 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
     if (l.kind == 0) {
       if (l.look)
         chol_diag_kernel<true><<<l.n, DT, kDiagLookSmemBytes, st>>>(
-            p->sorted_dev, l.step, info);
+            p->sorted_dev, l.step, info, p->packed);
       else
         chol_diag_kernel<false><<<l.n, DT, kDiagSmemBytes, st>>>(
-            p->sorted_dev, l.step, info);
+            p->sorted_dev, l.step, info, p->packed);
       KFAC_LAUNCH_CHECK("chol_diag_kernel");
     } else {
-      int rc = p->use_tc
+      int rc = l.packed
+                   ? launch_packed(p->descs_dev + l.off, &p->descs[l.off], l.n,
+                                   l.tiles, st)
+               : p->use_tc
                    ? launch_tc_grouped(p->descs_dev + l.off, &p->descs[l.off],
                                        l.n, l.tiles, l.tile_cols, false, 0.f,
                                        0.f, st)
@@ -1950,6 +2133,7 @@ extern "C" int kfac_inverse_plan_destroy(kfac_inverse_plan* p) {
   if (p->fork_ev != nullptr) cudaEventDestroy(p->fork_ev);
   for (cudaEvent_t ev : p->events) cudaEventDestroy(ev);
   cudaFree(p->params_dev);
+  cudaFree(p->scale_dev);
   cudaFree(p->add2_dev);
   cudaFree(p->refine_items_dev);
   cudaFree(p->refine_sums_dev);

@@ -5,6 +5,8 @@
 // barrier waits, and the splits of fp32 values into two TF32 or bf16 terms.
 #pragma once
 
+#include <cuda_fp16.h>
+
 #include "common.cuh"
 
 namespace kfac {
@@ -105,6 +107,40 @@ __device__ __forceinline__ void tc_mma(unsigned tmem_d, unsigned long long da,
       : "memory");
 }
 
+// K-major tiles of 16-bit values have the descriptor above.  MN-major: 64 columns
+// per 128-byte row of one k, groups of 8 k 1024 bytes apart, the next 64 columns
+// `step` bytes further.
+__device__ __forceinline__ unsigned long long tc_smem_desc_mn(unsigned addr,
+                                                              unsigned step) {
+  unsigned long long d = 0;
+  d |= (unsigned long long)((addr & 0x3FFFF) >> 4);
+  d |= (unsigned long long)(step >> 4) << 16;
+  d |= (unsigned long long)(1024 >> 4) << 32;
+  d |= (unsigned long long)1 << 46;
+  d |= (unsigned long long)2 << 61;
+  return d;
+}
+
+// D = f32, A = B = f16, M = m (256: a pair of CTAs), N = n
+__device__ __forceinline__ unsigned tc_half_desc(int n, bool a_mn, bool b_mn,
+                                                 int m = TC_BM) {
+  return (1u << 4) | ((unsigned)a_mn << 15) | ((unsigned)b_mn << 16) |
+         ((unsigned)(n >> 3) << 17) | ((unsigned)(m >> 4) << 24);
+}
+
+__device__ __forceinline__ void tc_mma_half(unsigned tmem_d,
+                                            unsigned long long da,
+                                            unsigned long long db,
+                                            unsigned idesc,
+                                            unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 __device__ __forceinline__ void tc_commit(unsigned long long* bar) {
   asm volatile(
       "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
@@ -187,6 +223,29 @@ __device__ __forceinline__ void store_split(unsigned hi_addr, unsigned lo_addr,
   l.x = x.x - h.x; l.y = x.y - h.y; l.z = x.z - h.z; l.w = x.w - h.w;
   sts128(hi_addr, h);
   sts128(lo_addr, l);
+}
+
+__device__ __forceinline__ void sts64(unsigned addr, unsigned a, unsigned b) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b)
+               : "memory");
+}
+
+// Two values, already scaled into the range of fp16, as fp16 terms y = hi + lo:
+// both rounded to nearest, so hi + lo carries 22 significant bits down to 2^-3
+// and an absolute error of at most 2^-25 below (fp16 denormals; the tensor core
+// takes them as they are).  Finite values beyond the range saturate; what is not
+// finite leaves a NaN in lo (y * 0).
+__device__ __forceinline__ unsigned half2_sat(float y0, float y1) {
+  unsigned r;
+  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y1), "f"(y0));
+  return r;
+}
+
+__device__ __forceinline__ void split_half2(float y0, float y1, unsigned& hi,
+                                            unsigned& lo) {
+  hi = half2_sat(y0, y1);
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  lo = half2_sat(fmaf(y0, 0.f, y0 - f.x), fmaf(y1, 0.f, y1 - f.y));
 }
 
 // Two values as bf16 terms x = hi + lo: one word of each (the first value in the

@@ -1510,11 +1510,12 @@ extern "C" int kfac_tc_status(int* status_out) {
   KFAC_CUDA(cudaDeviceSynchronize());
   int v = 0;
   KFAC_CUDA(cudaMemcpyFromSymbol(&v, kfac::g_tc_status, sizeof(int)));
-  int w = 0, t = 0, u = 0;
+  int w = 0, t = 0, u = 0, p = 0;
   int rc = kfac::diag_status_read(&w);
   if (rc == KFAC_OK) rc = kfac::tile_status_read(&t);
   if (rc == KFAC_OK) rc = kfac::gram_status_read(&u);
+  if (rc == KFAC_OK) rc = kfac::packed_status_read(&p);
   if (rc != KFAC_OK) return rc;
-  *status_out = v | w | t | u;
+  *status_out = v | w | t | u | p;
   return KFAC_OK;
 }

@@ -1,0 +1,411 @@
+// Products of operands that lie in memory as fp16 terms (chunks of 128 rows x
+// 32 k, GemmDesc::ca / cb): the long products of the inverse, C = alpha A B +
+// beta C over many problems in one launch, three tcgen05.mma (kind::f16) per
+// product, C += hi*hi + hi*lo + lo*hi, the cross terms in accumulators of their
+// own.
+//
+// A k-block of an operand tile is one bulk copy of 16 KB, already in the layout
+// the MMAs read: no value is loaded, split and stored again by every tile that
+// uses it.  That is what the tile kernel (tc_tile.cu) spends its time on: a
+// 128 x 256 x 32 block takes 1600 ns there with TF32 terms, its MMAs 810, its
+// loads alone 630.  1332 tiles with K = 4608 run here at 1335 TFLOP/s of bf16-rate
+// MMAs (97 % of what a long cuBLAS loop sustains), the tile kernel reached 580 of
+// half that rate.  Bound: long products by the MMAs and the feed from L2 (32 KB
+// per SM and 384 cycles of MMAs); the K = 512 ones by their passes over C, so two
+// CTAs share an SM, one in its epilogue beside the other's MMAs (three stages of
+// 32 KB and half of the tensor memory each).  256 x 256 tiles of two CTAs
+// (cta_group::2), which halve the feed, took 690 ns per k-block against 4 x 240 /
+// 2 here: not kept.
+//
+// Warp 0 issues the copies, warp 1 the MMAs, eight warps the epilogue.
+//
+// Every barrier wait is bounded; a wait that runs out raises a status word
+// instead of hanging.
+#include <algorithm>
+#include <mutex>
+
+#include "gemm_simt.cuh"
+#include "tc_common.cuh"
+
+namespace kfac {
+
+constexpr int KP_STAGES = 3;
+constexpr int KP_STAGE = 2 * kChunk;
+constexpr int KP_EPI_WARPS = 8;
+constexpr int KP_THREADS = 32 * (2 + KP_EPI_WARPS);
+constexpr int KP_SMEM = KP_STAGES * KP_STAGE + 2048;
+// Longest contraction of one accumulator, in k-blocks of 32.  The tensor core
+// adds with truncation, so a sum drifts with the number of MMAs behind it; past
+// this many the accumulators are added to C (round to nearest) and start anew.
+// Errors of inverses of 27 to 4608 rows against fp64 (Wishart, low-rank, badly
+// scaled and non-negative factors, damping 1e-6 to 1e-2), relative to those with
+// TF32 terms and a pass over C per 512 k: up to 3.8 without a cut, 1.7 with one
+// per 1024 k, 0.43 to 1.02 with 512, counted from the product's first k so that
+// a long sum's large leading part does not carry the next panel's.
+constexpr int KP_SEGMENT = 16;
+
+static __device__ int g_packed_status = 0;
+
+struct PackedControl {
+  unsigned long long full[KP_STAGES];    // the copies have arrived
+  unsigned long long empty[KP_STAGES];   // the MMAs have read the stage
+  unsigned long long accum;              // a segment's accumulators are final
+  unsigned long long drained;            // and have been read
+  unsigned tmem_base;
+  volatile int abort_flag;
+  GemmDesc desc;
+};
+static_assert(sizeof(PackedControl) <= 1024, "packed control block");
+
+__device__ __forceinline__ void bulk_load(unsigned dst, const void* src,
+                                          unsigned long long* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1], %2, [%3];"
+      ::"r"(dst), "l"(src), "r"(kChunk), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// 32 columns of 16 accumulator rows of a warp's quarter: v[4 j + 2 h + e] is row
+// lane / 4 + 8 h, column 8 j + 2 (lane % 4) + e.
+__device__ __forceinline__ void tc_ld_16x32(unsigned taddr, float v[16]) {
+  unsigned r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+        "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Elements of a 16 x 32 piece of C in that order, this lane's first at row r,
+// column c: f(i, row offset, column offset) for those stored, which are all
+// (WHOLE), or the ones in front of `rows` and `cols` and (lower) not above the
+// diagonal.
+template <bool WHOLE, typename F>
+__device__ __forceinline__ void piece_each(int r, int c, int rows, int cols,
+                                           bool lower, F f) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int dr = 8 * ((i >> 1) & 1), dc = 8 * (i >> 2) + (i & 1);
+    if (WHOLE || (r + dr < rows && c + dc < cols &&
+                  (!lower || c + dc <= r + dr)))
+      f(i, dr, dc);
+  }
+}
+
+__global__ void __launch_bounds__(KP_THREADS, 2)
+packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
+                   const __grid_constant__ TileInline inl) {
+  constexpr int TN = 128;
+  extern __shared__ unsigned char kp_smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(kp_smem_raw) + 1023) & ~(uintptr_t)1023);
+  PackedControl* ctl =
+      reinterpret_cast<PackedControl*>(smem + KP_STAGES * KP_STAGE);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tile = blockIdx.x;
+
+  if (warp == 0) {
+    if (lane == 0) {
+#pragma unroll
+      for (int s = 0; s < KP_STAGES; ++s) {
+        mbar_init(&ctl->full[s], 1);
+        mbar_init(&ctl->empty[s], 1);
+      }
+      mbar_init(&ctl->accum, 1);
+      mbar_init(&ctl->drained, KP_EPI_WARPS);
+      ctl->abort_flag = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    asm volatile(
+        "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+        ::"r"(smem_u32(&ctl->tmem_base)), "r"(2 * TN)
+        : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
+                 ::: "memory");
+  } else {
+    // the problem this tile belongs to (tile_begin is ascending)
+    constexpr int kWords = (int)(sizeof(GemmDesc) / sizeof(int));
+    const GemmDesc* src;
+    int f = 0;
+    if (inl.n > 0) {
+#pragma unroll
+      for (int i = 1; i < TT_INLINE; ++i)
+        if (i < inl.n && inl.d[i].tile_begin <= tile) f = i;
+      src = &inl.d[f];
+    } else {
+      for (int i = lane; i < ndesc; i += 32)
+        if (descs[i].tile_begin <= tile) f = i;
+      f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
+      src = descs + f;
+    }
+    int* dst = reinterpret_cast<int*>(&ctl->desc);
+    for (int i = tid - 64; i < kWords; i += 32 * KP_EPI_WARPS)
+      dst[i] = reinterpret_cast<const int*>(src)[i];
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+  const GemmDesc& g = ctl->desc;
+  const unsigned tmem = ctl->tmem_base;
+  const int flags = g.flags;
+  const int lt = tile - g.tile_begin;
+  int bi, bj;
+  if (flags & G_LOWER) {
+    tri_tile(lt, bi, bj);
+  } else {
+    bi = lt / g.tiles_n;
+    bj = lt - bi * g.tiles_n;
+  }
+  const int m0 = bi * TN, n0 = bj * TN;
+  const bool share_ab = (flags & G_SAME_AB) && bi == bj;
+  int kbeg = 0;
+  if (flags & G_KBEG_M0) kbeg = max(0, m0 - g.kbeg_off);
+  if (flags & G_KBEG_N0) kbeg = max(kbeg, n0);
+  const int nkb = max(0, (int)((g.K - kbeg + 31) >> 5));
+  const int kb0 = kbeg >> 5, seg0 = kb0 / KP_SEGMENT;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      const long long k0 = (long long)kb0 * kChunk;
+      const unsigned char* a = g.ca + bi * g.ca_tile + k0;
+      const unsigned char* b = g.cb + bj * g.cb_tile + k0;
+      const unsigned bytes = share_ab ? kChunk : 2 * kChunk;
+      for (int kb = 0; kb < nkb; ++kb, a += kChunk, b += kChunk) {
+        const int s = kb % KP_STAGES;
+        if (kb >= KP_STAGES &&
+            !mbar_wait_status(&ctl->empty[s], ((kb / KP_STAGES) - 1) & 1,
+                              &ctl->abort_flag, &g_packed_status))
+          break;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                     ::"r"(smem_u32(&ctl->full[s])), "r"(bytes)
+                     : "memory");
+        const unsigned st = smem_u32(smem + s * KP_STAGE);
+        if (!share_ab) bulk_load(st, a, &ctl->full[s]);
+        bulk_load(st + kChunk, b, &ctl->full[s]);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const bool ka = g.A.kfast != 0, kb_ = g.B.kfast != 0;
+      const unsigned idesc = tc_half_desc(TN, !ka, !kb_);
+      // from the hi to the lo terms, and from 16 k to the next (16-byte units)
+      const unsigned long long lo_a = (ka ? 64 : 4096) >> 4;
+      const unsigned long long lo_b = (kb_ ? 64 : 4096) >> 4;
+      const unsigned long long adv_a = (ka ? 32 : 2048) >> 4;
+      const unsigned long long adv_b = (kb_ ? 32 : 2048) >> 4;
+      for (int kb = 0; kb < nkb; ++kb) {
+        const int s = kb % KP_STAGES;
+        const int seg = (kb0 + kb) / KP_SEGMENT - seg0;
+        const bool fresh = kb == 0 || (kb0 + kb) % KP_SEGMENT == 0;
+        if (fresh && seg > 0 &&
+            !mbar_wait_status(&ctl->drained, (seg - 1) & 1, &ctl->abort_flag,
+                              &g_packed_status))
+          break;
+        if (!mbar_wait_status(&ctl->full[s], (kb / KP_STAGES) & 1,
+                              &ctl->abort_flag, &g_packed_status))
+          break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const unsigned sb = smem_u32(smem + s * KP_STAGE) + kChunk;
+        const unsigned sa = share_ab ? sb : sb - kChunk;
+        unsigned long long a = ka ? tc_smem_desc(sa) : tc_smem_desc_mn(sa, 8192);
+        unsigned long long b = kb_ ? tc_smem_desc(sb) : tc_smem_desc_mn(sb, 8192);
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk, a += adv_a, b += adv_b) {
+          const unsigned acc = !fresh || kk != 0;
+          tc_mma_half(tmem + TN, a + lo_a, b, idesc, acc);
+          tc_mma_half(tmem + TN, a, b + lo_b, idesc, 1);
+          tc_mma_half(tmem, a, b, idesc, acc);
+        }
+        tc_commit(&ctl->empty[s]);
+        if (kb + 1 == nkb || (kb0 + kb + 1) % KP_SEGMENT == 0)
+          tc_commit(&ctl->accum);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ===================== epilogue =====================
+    // warp: accumulator rows of quarter q, 32-column pieces h and h + 2, 16 rows
+    // at a time straight from the registers (8-byte words of eight rows an
+    // instruction: whole 32-byte sectors)
+    const int q = warp & 3, h = (warp - 2) >> 2;
+    const int rows = g.M, cols = g.N;
+    const bool lower = (flags & G_LOWER) != 0;
+    const float alpha = g.alpha;
+    float beta = (g.beta_until > 0 && m0 >= g.beta_until) ? 0.f : g.beta;
+    const float* un = g.unscale;
+    const long long ldc = g.ldc;
+    const bool vec = (ldc & 1) == 0 &&
+                     (reinterpret_cast<uintptr_t>(g.C) & 7) == 0;
+    const int lr = lane >> 2, lc = 2 * (lane & 3);
+    bool ok = true;
+    const int nseg = nkb > 0 ? (kb0 + nkb - 1) / KP_SEGMENT - seg0 + 1 : 1;
+#pragma unroll 1
+    for (int it = 0; it < 4 * nseg; ++it) {
+      const int u = it & 3, seg = it >> 2;
+      if (it == 4) beta = 1.f;             // onto the segments before
+      const int r0 = m0 + 32 * q + 16 * (u & 1);
+      const int c0 = n0 + 32 * h + 64 * (u >> 1);
+      const bool live = r0 < rows && c0 < cols && !(lower && c0 > r0 + 15);
+      const bool whole =
+          r0 + 16 <= rows && c0 + 32 <= cols && (!lower || c0 + 31 <= r0);
+      const int r = r0 + lr, c = c0 + lc;
+      float* p = g.C + (long long)r * ldc + c;
+      float old[16];
+      if (beta != 0.f && live) {
+        if (whole && vec) {
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            const float2 x = *reinterpret_cast<const float2*>(
+                p + 8 * ((i >> 1) & 1) * ldc + 8 * (i >> 2));
+            old[i] = x.x;
+            old[i + 1] = x.y;
+          }
+        } else {
+          piece_each<false>(r, c, rows, cols, lower, [&](int i, int dr, int dc) {
+            old[i] = p[dr * ldc + dc];
+          });
+        }
+      }
+      if (u == 0 && nkb > 0) {
+        ok = mbar_wait_status(&ctl->accum, seg & 1, &ctl->abort_flag,
+                              &g_packed_status);
+        ok = __all_sync(0xffffffffu, ok);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      if (!ok) break;
+      float v[16];
+      if (nkb > 0 && live) {
+        float w[16];
+        const unsigned at = tmem + ((unsigned)(32 * q + 16 * (u & 1)) << 16) +
+                            (unsigned)(c0 - n0);
+        tc_ld_16x32(at, v);
+        tc_ld_16x32(at + TN, w);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = alpha * (v[i] + w[i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+      }
+      if (u == 3 && seg + 1 < nseg) {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl->drained);
+      }
+      if (!live) continue;
+      if (un != nullptr) {
+        // (rows and columns past the matrix: inside the vector's padding)
+        const float s0 = un[r], s1 = un[r + 8];
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+          const float2 sc = *reinterpret_cast<const float2*>(&un[c + 2 * j]);
+          v[j] = v[j] * s0 * sc.x;
+          v[j + 1] = v[j + 1] * s0 * sc.y;
+          v[j + 2] = v[j + 2] * s1 * sc.x;
+          v[j + 3] = v[j + 3] * s1 * sc.y;
+        }
+      }
+      if (beta != 0.f) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] += beta * old[i];
+      }
+      if (whole && vec) {
+#pragma unroll
+        for (int i = 0; i < 16; i += 2)
+          *reinterpret_cast<float2*>(p + 8 * ((i >> 1) & 1) * ldc +
+                                     8 * (i >> 2)) =
+              make_float2(v[i], v[i + 1]);
+      } else {
+        piece_each<false>(r, c, rows, cols, lower, [&](int i, int dr, int dc) {
+          p[dr * ldc + dc] = v[i];
+        });
+      }
+      if (flags & G_MIRROR) {
+        float* t = g.C + (long long)c * ldc + r;
+        if (whole)
+          piece_each<true>(r, c, rows, cols, lower, [&](int i, int dr, int dc) {
+            t[dc * ldc + dr] = v[i];
+          });
+        else
+          piece_each<false>(r, c, rows, cols, lower, [&](int i, int dr, int dc) {
+            t[dc * ldc + dr] = v[i];
+          });
+      }
+    }
+  }
+  if (tid == 0 && ctl->abort_flag != 0) {
+    // a wait ran out: give the copies already issued time to land before
+    // the shared memory is handed back (bounded: 64 us)
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+                 ::"r"(tmem), "r"(2 * TN)
+                 : "memory");
+}
+
+// ------------------------------------------------------------------ host side
+int packed_prepare() {
+  static std::mutex mu;
+  static bool done[64] = {false};
+  int dev = 0;
+  KFAC_CUDA(cudaGetDevice(&dev));
+  KFAC_REQUIRE(dev >= 0 && dev < 64, "device index %d unsupported", dev);
+  std::lock_guard<std::mutex> lock(mu);
+  if (!done[dev]) {
+    KFAC_CUDA(cudaFuncSetAttribute(packed_tile_kernel,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   KP_SMEM));
+    done[dev] = true;
+  }
+  return KFAC_OK;
+}
+
+int packed_number_tiles(GemmDesc* descs, int n) {
+  int total = 0;
+  for (int i = 0; i < n; ++i) {
+    GemmDesc& g = descs[i];
+    const int tm = (g.M + TC_BM - 1) / TC_BM, tn = (g.N + TC_BM - 1) / TC_BM;
+    g.tile_begin = total;
+    g.tiles_m = tm;
+    g.tiles_n = tn;
+    total += (g.flags & G_LOWER) ? tm * (tm + 1) / 2 : tm * tn;
+  }
+  return total;
+}
+
+int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
+                  int ndesc, int total_tiles, cudaStream_t stream) {
+  if (ndesc <= 0 || total_tiles <= 0) return KFAC_OK;
+  const int rc = packed_prepare();
+  if (rc != KFAC_OK) return rc;
+  TileInline inl;
+  inl.n = 0;
+  if (ndesc <= TT_INLINE) {
+    inl.n = ndesc;
+    std::copy(descs_host, descs_host + ndesc, inl.d);
+  }
+  packed_tile_kernel<<<total_tiles, KP_THREADS, KP_SMEM, stream>>>(
+      descs_dev, ndesc, inl);
+  KFAC_LAUNCH_CHECK("packed_tile_kernel");
+  return KFAC_OK;
+}
+
+int packed_status_read(int* out) {
+  KFAC_CUDA(cudaMemcpyFromSymbol(out, g_packed_status, sizeof(int)));
+  return KFAC_OK;
+}
+
+}  // namespace kfac

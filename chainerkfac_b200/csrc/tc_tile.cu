@@ -30,48 +30,43 @@
 // instead of hanging.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "gemm_simt.cuh"
 #include "tc_common.cuh"
+#include "tc_epilogue.cuh"
 
 namespace kfac {
 
 constexpr int TT_BK = 32;
-constexpr int TT_EP = 36;         // row pitch of an epilogue piece (floats)
-constexpr int TT_INLINE = kTileInline;
-
 static __device__ int g_tile_status = 0;
 
-template <int TN>
+template <int TN, bool HALF>
 struct TileMap {
   static constexpr int kProducers = TN == 256 ? 384 : 512;
   static constexpr bool kTwo = TN == 256;         // units per producer thread
   static constexpr int kWarps = kProducers / 32;
   static constexpr int kThreads = kProducers + 32;
-  static constexpr int kStages = TN == 256 ? 2 : 3;
-  static constexpr int kABytes = TC_BM * TT_BK * 4;       // 16 KB
-  static constexpr int kBBytes = TN * TT_BK * 4;
-  static constexpr int kLo = kABytes + kBBytes;   // a lo tile after its hi tile
-  static constexpr int kStage = 2 * kLo;
+  static constexpr int kStages = (TN == 256 ? 2 : 3) * (HALF ? 2 : 1);
+  // operand rows of 128 bytes: 32 TF32 values, or both fp16 terms of 32
+  static constexpr int kABytes = TC_BM * 128;             // 16 KB
+  static constexpr int kBBytes = TN * 128;
+  static constexpr int kLo = kABytes + kBBytes;   // TF32: lo tiles, hi before
+  static constexpr int kStage = HALF ? kLo : 2 * kLo;
   static constexpr int kTmem = 2 * TN;            // hi*hi, then cross terms
   static constexpr int kSmem = kStages * kStage + 1024 + 1024;
 };
+constexpr int TT_MAX_STAGES = 6;
 
 struct TileControl {
-  unsigned long long full[3];
-  unsigned long long empty[3];
+  unsigned long long full[TT_MAX_STAGES];
+  unsigned long long empty[TT_MAX_STAGES];
   unsigned long long accum;
   unsigned tmem_base;
   volatile int abort_flag;
   GemmDesc desc;
 };
 static_assert(sizeof(TileControl) <= 1024, "tile control block");
-
-struct TileInline {
-  int n;                       // 0: descriptors in device memory
-  GemmDesc d[TT_INLINE];
-};
-static_assert(sizeof(TileInline) <= 3800, "kernel argument space");
 
 // One producer unit: four 16-byte chunks (4 consecutive k of one tile row) per
 // 32-k block.  Operands contiguous along k: a warp covers 16 rows, one load
@@ -262,135 +257,110 @@ __device__ __forceinline__ void tile_unit_store(const TileUnit& u, unsigned st,
   }
 }
 
-// 32 accumulator columns of this warp's 32 rows (both accumulators added, times
-// alpha) into its shared-memory piece, a row per lane.
-template <int TN>
-__device__ __forceinline__ void tile_acc_piece(unsigned tmem, int q, int c0,
-                                               float alpha, bool zero,
-                                               float* piece, int lane) {
-  const unsigned row = (unsigned)(q * 32) << 16;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    float v[16], w[16];
-    if (!zero) {
-      tc_ld16(tmem + row + (unsigned)(c0 + 16 * h), v);
-      tc_ld16(tmem + row + (unsigned)(TN + c0 + 16 * h), w);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = w[i] = 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < 16; i += 4)
-      *reinterpret_cast<float4*>(&piece[lane * TT_EP + 16 * h + i]) =
-          make_float4(alpha * (v[i] + w[i]), alpha * (v[i + 1] + w[i + 1]),
-                      alpha * (v[i + 2] + w[i + 2]),
-                      alpha * (v[i + 3] + w[i + 3]));
-  }
-}
+// One producer unit of a product in fp16 terms (all operands have rows of
+// 16-byte words).  Operands contiguous along k are stored K-major, 16 rows a
+// unit: a 128-byte row holds the hi terms of 32 k, then the lo terms.  A thread
+// takes four k of rows 4 (lane / 8) .. + 3, so that the two rows of a half warp's
+// 8-byte stores differ in the bit that moves the swizzle across the halves of
+// a row.  Operands contiguous along the tile rows are stored MN-major, as they
+// are: a unit is 64 rows x 8 k, one swizzle atom (1 KB) per term; 64 rows take
+// four atoms of hi and four of lo terms.
+struct HalfUnit {
+  const float* p;
+  int o[3];              // offsets of words 1 .. 3
+  int adv;
+  int k;
+  unsigned soff;
+  bool kf, live;
+};
 
-// Tile (bi, bj) of lower-triangular problem tile t; 128 x 256 tiles exist iff
-// 2 bj <= bi, 128 x 128 tiles iff bj <= bi.
-template <int TN>
-__device__ __forceinline__ void tile_lower(int t, int& bi, int& bj) {
-  if (TN == 128) {
-    tri_tile(t, bi, bj);
-    return;
-  }
-  int a = (int)sqrtf((float)t);
-  while ((a + 1) * (a + 1) <= t) ++a;
-  while (a * a > t) --a;
-  if (t < a * (a + 1)) {
-    bi = 2 * a - 1;
-    bj = t - a * a;
+// (a unit past the operand's last row reads that one again)
+__device__ __forceinline__ void half_unit_setup(const Operand& op, int r0,
+                                                int wu, int lane, int kbeg,
+                                                int rows, unsigned side_off,
+                                                HalfUnit& u) {
+  u.kf = op.kfast != 0;
+  const int ld = u.kf ? (int)op.s_col : (int)op.s_outer;
+  if (u.kf) {
+    const int row = 16 * wu + 4 * (lane >> 3), chunk = lane & 7;
+    u.live = 16 * wu < rows;
+    u.k = kbeg + 4 * chunk;
+    const int r = min(r0 + row, op.ncols - 1);
+    u.p = op.base + (long long)r * ld + u.k;
+#pragma unroll
+    for (int i = 1; i < 4; ++i) u.o[i - 1] = min(i, op.ncols - 1 - r) * ld;
+    u.adv = TT_BK;
+    u.soff = side_off + sw128_chunk_off(row, chunk >> 1) + 8 * (chunk & 1);
   } else {
-    bi = 2 * a;
-    bj = t - a * (a + 1);
+    const int group = wu >> 2, octet = wu & 3, kk = lane >> 4;
+    const int row = 64 * group + 4 * (lane & 15);
+    u.live = 64 * group < rows;
+    u.k = kbeg + 8 * octet + kk;
+    // (whole words: the pitch covers the last one)
+    u.p = op.base + (long long)u.k * ld + min(r0 + row, (op.ncols - 1) & ~3);
+#pragma unroll
+    for (int i = 1; i < 4; ++i) u.o[i - 1] = 2 * i * ld;
+    u.adv = TT_BK * ld;
+    u.soff = side_off + 8192 * group + 1024 * octet +
+             sw128_chunk_off(kk, (lane & 15) >> 1) + 8 * (lane & 1);
   }
 }
 
-// Preconditioning epilogue of one 32 x 32 piece: kf to the weight and bias
-// parts, and the momentum update where the layer has it fused.
-__device__ __forceinline__ void tile_precond(const GemmDesc& g,
-                                             const float* piece, int gr0,
-                                             int rows, int gc0, int cols,
-                                             int lane, float lr,
-                                             float momentum) {
-  const int dW = g.dW;
-  const bool fused = g.pW != nullptr;
-  if ((dW & 3) == 0 && gc0 + 31 < dW && cols >= 32 &&
-      ((reinterpret_cast<uintptr_t>(g.kfW) | reinterpret_cast<uintptr_t>(g.pW) |
-        reinterpret_cast<uintptr_t>(g.vW)) & 15) == 0) {
-    const int sub = lane >> 3, wc = 4 * (lane & 7);
-    const float* pp = piece + sub * TT_EP + wc;
-    long long idx = (long long)(gr0 + sub) * dW + gc0 + wc;
-#pragma unroll 1
-    for (int i0 = 0; i0 < 8; i0 += 4, idx += 16LL * dW, pp += 16 * TT_EP) {
-      float4 ov[4], op[4];
-      long long at = idx;
+// FULL: the block ends before kend.  No branch around a thread's loads then, so
+// that those of several blocks stay in flight across the stores of one (a
+// 256-wide k-block took 1600 ns with such a branch, 1150 without).
+template <bool FULL>
+__device__ __forceinline__ void half_unit_load(HalfUnit& u, int kend,
+                                               float4 v[4]) {
+  const float* p = u.p;
+  if (FULL) {
+    v[0] = *reinterpret_cast<const float4*>(p);
 #pragma unroll
-      for (int i = 0; i < 4; ++i, at += 4LL * dW) {
-        if (!fused || 4 * (i0 + i) + sub >= rows) continue;
-        ov[i] = *reinterpret_cast<const float4*>(g.vW + at);
-        op[i] = *reinterpret_cast<const float4*>(g.pW + at);
-      }
-      at = idx;
+    for (int i = 1; i < 4; ++i)
+      v[i] = *reinterpret_cast<const float4*>(p + u.o[i - 1]);
+  } else {
+    // the end of the contraction: of every row, or whole k
 #pragma unroll
-      for (int i = 0; i < 4; ++i, at += 4LL * dW) {
-        if (4 * (i0 + i) + sub >= rows) continue;
-        const float4 kf = *reinterpret_cast<const float4*>(&pp[4 * i * TT_EP]);
-        if (g.kfW) *reinterpret_cast<float4*>(g.kfW + at) = kf;
-        if (!fused) continue;
-        float4 nv;
-        nv.x = momentum * ov[i].x - lr * kf.x;
-        nv.y = momentum * ov[i].y - lr * kf.y;
-        nv.z = momentum * ov[i].z - lr * kf.z;
-        nv.w = momentum * ov[i].w - lr * kf.w;
-        *reinterpret_cast<float4*>(g.vW + at) = nv;
-        *reinterpret_cast<float4*>(g.pW + at) =
-            make_float4(op[i].x + nv.x, op[i].y + nv.y, op[i].z + nv.z,
-                        op[i].w + nv.w);
-      }
+    for (int i = 0; i < 4; ++i) {
+      const float* q = i == 0 ? p : p + u.o[i - 1];
+      const int left = u.kf ? kend - u.k : (u.k + 2 * i < kend ? 4 : 0);
+      v[i].x = left > 0 ? q[0] : 0.f;
+      v[i].y = left > 1 ? q[1] : 0.f;
+      v[i].z = left > 2 ? q[2] : 0.f;
+      v[i].w = left > 3 ? q[3] : 0.f;
     }
-    return;
   }
-  // a column per lane, eight rows at a time
-  if (lane >= cols) return;
-  const bool w = gc0 + lane < dW;
-  float* okf = w ? g.kfW : g.kfb;
-  float* opar = w ? g.pW : g.pb;
-  float* ovel = w ? g.vW : g.vb;
-  const long long step = w ? dW : 1;
-  long long idx = gr0 * step + (w ? gc0 + lane : 0);
-  for (int r0 = 0; r0 < rows; r0 += 8, idx += 8 * step) {
-    float ov[8], op[8];
+  u.k += TT_BK;
+  u.p += u.adv;
+}
+
+__device__ __forceinline__ void half_unit_store(const HalfUnit& u, unsigned st,
+                                                const float4 v[4],
+                                                float scale) {
+  const unsigned at = st + u.soff;
+  // a step of one row (two k) down also flips the swizzle by 16 (32) bytes
+  const unsigned flip = u.kf ? 0x10u : 0x20u, step = u.kf ? 128u : 256u;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (opar != nullptr && r0 + i < rows) {
-        ov[i] = ovel[idx + i * step];
-        op[i] = opar[idx + i * step];
-      }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (r0 + i >= rows) continue;
-      const float kf = piece[(r0 + i) * TT_EP + lane];
-      if (okf != nullptr) okf[idx + i * step] = kf;
-      if (opar == nullptr) continue;
-      const float nv = momentum * ov[i] - lr * kf;
-      ovel[idx + i * step] = nv;
-      opar[idx + i * step] = op[i] + nv;
-    }
+  for (int i = 0; i < 4; ++i) {
+    const unsigned d = (at ^ (flip * i)) + step * i;
+    unsigned h0, h1, l0, l1;
+    split_half2(scale * v[i].x, scale * v[i].y, h0, l0);
+    split_half2(scale * v[i].z, scale * v[i].w, h1, l1);
+    sts64(d, h0, h1);
+    sts64(u.kf ? d ^ 0x40u : d + 4096, l0, l1);
   }
 }
 
 // PRE: the preconditioning epilogue (every problem of the launch has it).  VEC:
 // all operands of the launch have rows of 16-byte words (one kernel with both
-// ways of loading spills).
-template <int TN, bool PRE, bool VEC>
-__global__ void __launch_bounds__(TileMap<TN>::kThreads, 1)
+// ways of loading spills).  HALF: operands in two fp16 terms (VEC only).
+template <int TN, bool PRE, bool VEC, bool HALF>
+__global__ void __launch_bounds__(TileMap<TN, HALF>::kThreads, 1)
 tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
                const __grid_constant__ TileInline inl, float lr,
                float momentum) {
-  using Map = TileMap<TN>;
+  static_assert(!HALF || VEC, "fp16 terms need rows of 16-byte words");
+  using Map = TileMap<TN, HALF>;
   extern __shared__ unsigned char tt_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(tt_smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -480,17 +450,42 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
     const bool a0 = warp < 8;
     const Operand& op0 = a0 ? g.A : g.B;
     const Operand& op1 = g.B;
-    TileUnit u0, u1;
-    tile_unit_setup<VEC>(op0, a0 ? m0 : n0, a0 ? warp : warp - 8, lane, kbeg,
-                    a0 ? (share_ab ? 0 : m_valid) : n_valid,
-                    a0 ? 0 : Map::kABytes, u0);
-    if (Map::kTwo)
-      tile_unit_setup<VEC>(op1, n0, warp + Map::kWarps - 8, lane, kbeg, n_valid,
-                      Map::kABytes, u1);
+    using Unit = typename std::conditional<HALF, HalfUnit, TileUnit>::type;
+    Unit u0, u1;
+    const float scale0 = HALF ? (a0 ? g.sa : g.sb) : 1.f;
+    const float scale1 = HALF ? g.sb : 1.f;
+    {
+      const int r0 = a0 ? m0 : n0, wu = a0 ? warp : warp - 8;
+      const int rows = a0 ? (share_ab ? 0 : m_valid) : n_valid;
+      const unsigned side = a0 ? 0 : Map::kABytes;
+      if constexpr (HALF) {
+        half_unit_setup(op0, r0, wu, lane, kbeg, rows, side, u0);
+        if (Map::kTwo)
+          half_unit_setup(op1, n0, warp + Map::kWarps - 8, lane, kbeg, n_valid,
+                          Map::kABytes, u1);
+      } else {
+        tile_unit_setup<VEC>(op0, r0, wu, lane, kbeg, rows, side, u0);
+        if (Map::kTwo)
+          tile_unit_setup<VEC>(op1, n0, warp + Map::kWarps - 8, lane, kbeg,
+                               n_valid, Map::kABytes, u1);
+      }
+    }
     const unsigned base = smem_u32(smem);
-    auto load = [&](float4* v) {
-      tile_unit_load<VEC>(op0, u0, kend, v);
-      if (Map::kTwo) tile_unit_load<VEC>(op1, u1, kend, v + 4);
+    // blocks that end before kend (fp16 terms)
+    const int nfull = (kend - kbeg) / TT_BK;
+    auto load = [&](int kb, float4* v) {
+      if constexpr (HALF) {
+        if (kb < nfull) {
+          half_unit_load<true>(u0, kend, v);
+          if (Map::kTwo) half_unit_load<true>(u1, kend, v + 4);
+        } else {
+          half_unit_load<false>(u0, kend, v);
+          if (Map::kTwo) half_unit_load<false>(u1, kend, v + 4);
+        }
+      } else {
+        tile_unit_load<VEC>(op0, u0, kend, v);
+        if (Map::kTwo) tile_unit_load<VEC>(op1, u1, kend, v + 4);
+      }
     };
     auto store = [&](int kb, const float4* v) {
       const int s = kb % Map::kStages;
@@ -499,8 +494,13 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
                             &ctl->abort_flag, &g_tile_status))
         return false;
       const unsigned st = base + s * Map::kStage;
-      tile_unit_store<VEC>(u0, st, Map::kLo, v);
-      if (Map::kTwo) tile_unit_store<VEC>(u1, st, Map::kLo, v + 4);
+      if constexpr (HALF) {
+        half_unit_store(u0, st, v, scale0);
+        if (Map::kTwo) half_unit_store(u1, st, v + 4, scale1);
+      } else {
+        tile_unit_store<VEC>(u0, st, Map::kLo, v);
+        if (Map::kTwo) tile_unit_store<VEC>(u1, st, Map::kLo, v + 4);
+      }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl->full[s]);
@@ -508,46 +508,91 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
     };
     constexpr int kVals = Map::kTwo ? 8 : 4;
     float4 va[kVals];
-    if (nkb > 0) load(va);
-    if (TN == 256) {
+    bool idle = false;
+    if constexpr (HALF) idle = !u0.live && !(Map::kTwo && u1.live);
+    if (idle) {
+      // none of this warp's rows is used: it only keeps the barriers going
+      for (int kb = 0; kb < nkb; ++kb) {
+        const int s = kb % Map::kStages;
+        if (kb >= Map::kStages &&
+            !mbar_wait_status(&ctl->empty[s], ((kb / Map::kStages) - 1) & 1,
+                              &ctl->abort_flag, &g_tile_status))
+          break;
+        if (lane == 0) mbar_arrive(&ctl->full[s]);
+      }
+    } else if (TN == 256 && !HALF) {
       // one block ahead: the MMAs of a block take longer than a trip to L2
+      if (nkb > 0) load(0, va);
 #pragma unroll 1
       for (int kb = 0; kb < nkb; ++kb) {
         if (!store(kb, va)) break;
-        if (kb + 1 < nkb) load(va);
+        if (kb + 1 < nkb) load(kb + 1, va);
       }
-    } else if (!VEC) {
+    } else if (!VEC || TN == 256) {
       float4 vb[kVals];
-      if (nkb > 1) load(vb);
+      if (nkb > 0) load(0, va);
+      if (nkb > 1) load(1, vb);
 #pragma unroll 1
       for (int kb = 0; kb < nkb; kb += 2) {
         if (!store(kb, va)) break;
-        if (kb + 2 < nkb) load(va);
+        if (kb + 2 < nkb) load(kb + 2, va);
         if (kb + 1 < nkb) {
           if (!store(kb + 1, vb)) break;
-          if (kb + 3 < nkb) load(vb);
+          if (kb + 3 < nkb) load(kb + 3, vb);
         }
       }
     } else {
       float4 vb[kVals], vc[kVals];
-      if (nkb > 1) load(vb);
-      if (nkb > 2) load(vc);
+      if (nkb > 0) load(0, va);
+      if (nkb > 1) load(1, vb);
+      if (nkb > 2) load(2, vc);
 #pragma unroll 1
       for (int kb = 0; kb < nkb; kb += 3) {
         if (!store(kb, va)) break;
-        if (kb + 3 < nkb) load(va);
+        if (kb + 3 < nkb) load(kb + 3, va);
         if (kb + 1 < nkb) {
           if (!store(kb + 1, vb)) break;
-          if (kb + 4 < nkb) load(vb);
+          if (kb + 4 < nkb) load(kb + 4, vb);
         }
         if (kb + 2 < nkb) {
           if (!store(kb + 2, vc)) break;
-          if (kb + 5 < nkb) load(vc);
+          if (kb + 5 < nkb) load(kb + 5, vc);
         }
       }
     }
   } else {
-    if (elect_one()) {
+    if (HALF && elect_one()) {
+      // ===================== MMA issuer, fp16 terms =====================
+      const bool ka = g.A.kfast != 0, kb_ = g.B.kfast != 0;
+      const unsigned idesc = tc_half_desc(n_inst, !ka, !kb_);
+      const unsigned a_off =
+          share_ab ? (unsigned)(Map::kABytes + (m0 - n0) * 128) : 0u;
+      // from the hi to the lo terms, and from 16 k to the next (16-byte units)
+      const unsigned long long lo_a = (ka ? 64 : 4096) >> 4;
+      const unsigned long long lo_b = (kb_ ? 64 : 4096) >> 4;
+      const unsigned long long adv_a = (ka ? 32 : 2048) >> 4;
+      const unsigned long long adv_b = (kb_ ? 32 : 2048) >> 4;
+      for (int kb = 0; kb < nkb; ++kb) {
+        const int s = kb % Map::kStages;
+        if (!mbar_wait_status(&ctl->full[s], (kb / Map::kStages) & 1,
+                              &ctl->abort_flag, &g_tile_status))
+          break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const unsigned sa = smem_u32(smem + s * Map::kStage) + a_off;
+        const unsigned sb = smem_u32(smem + s * Map::kStage) + Map::kABytes;
+        unsigned long long a = ka ? tc_smem_desc(sa) : tc_smem_desc_mn(sa, 8192);
+        unsigned long long b = kb_ ? tc_smem_desc(sb) : tc_smem_desc_mn(sb, 8192);
+#pragma unroll
+        for (int kk = 0; kk < TT_BK / 16; ++kk, a += adv_a, b += adv_b) {
+          tc_mma_half(tmem + TN, a + lo_a, b, idesc, (kb | kk) != 0);
+          tc_mma_half(tmem + TN, a, b + lo_b, idesc, 1);
+          tc_mma_half(tmem, a, b, idesc, (kb | kk) != 0);
+        }
+        tc_commit(&ctl->empty[s]);
+      }
+      tc_commit(&ctl->accum);
+    }
+    if (!HALF && elect_one()) {
       // ===================== MMA issuer =====================
       const unsigned idesc = tc_instr_desc(n_inst);
       const unsigned a_off =
@@ -580,111 +625,18 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
   }
 
   // ===================== epilogue =====================
-  // warp w: accumulator rows of quarter q, 32-column pieces h, h + G, ...
-  constexpr int G = Map::kWarps / 4;
-  const int q = warp & 3, h = warp >> 2;
+  // warp w: accumulator rows of quarter q, 32-column pieces h, h + G, ...; its
+  // own piece of the (drained) first stages
   if (warp < Map::kWarps && !gated_off) {
-    const int row0 = q * 32, rows = min(32, m_valid - row0);
-    const bool lower = (flags & G_LOWER) != 0;
-    const float alpha = g.alpha;
-    const float beta =
-        (g.beta_until > 0 && m0 >= g.beta_until) ? 0.f : g.beta;
-    float* C = g.C;
-    float* C2 = g.C2;
-    const long long ldc = g.ldc;
-    // rows of a piece as 16-byte words: lane -> row 4 i + lane / 8, word lane % 8
-    const bool vec = (ldc & 3) == 0 &&
-                     (reinterpret_cast<uintptr_t>(C) & 15) == 0 &&
-                     (reinterpret_cast<uintptr_t>(C2) & 15) == 0;
-    const int sub = lane >> 3, wc = 4 * (lane & 7);
-    float4 old[8];
-    auto prefetch = [&](int c0) {
-      if constexpr (PRE) return;
-      if (beta == 0.f || c0 >= n_valid) return;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int r = row0 + 4 * i + sub, c = c0 + wc;
-        old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r >= m_valid || c >= n_valid) continue;
-        const float* p = C + (long long)(m0 + r) * ldc + n0 + c;
-        if (vec && c + 3 < n_valid) {
-          old[i] = *reinterpret_cast<const float4*>(p);
-        } else {
-          old[i].x = p[0];
-          if (c + 1 < n_valid) old[i].y = p[1];
-          if (c + 2 < n_valid) old[i].z = p[2];
-          if (c + 3 < n_valid) old[i].w = p[3];
-        }
-      }
-    };
-    prefetch(32 * h);
-    bool ok = true;
-    if (nkb > 0) {
-      ok = mbar_wait_status(&ctl->accum, 0, &ctl->abort_flag, &g_tile_status);
-      ok = __all_sync(0xffffffffu, ok);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    }
-    // every warp has its own piece of the (drained) first stage
-    float* piece = reinterpret_cast<float*>(smem) + warp * 32 * TT_EP;
-    for (int c0 = 32 * h; c0 < n_valid && ok; c0 += 32 * G) {
-      tile_acc_piece<TN>(tmem, q, c0, alpha, nkb == 0, piece, lane);
-      __syncwarp();
-      if (PRE) {
-        if (rows > 0)
-          tile_precond(g, piece, m0 + row0, rows, n0 + c0, n_valid - c0, lane,
-                       lr, momentum);
-      } else if (rows > 0) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int r = row0 + 4 * i + sub, c = c0 + wc;
-          const int gr = m0 + r;
-          const int cend = lower ? min(n_valid, gr - n0 + 1) : n_valid;
-          float4 x =
-              *reinterpret_cast<const float4*>(&piece[(4 * i + sub) * TT_EP + wc]);
-          if (beta != 0.f) {
-            x.x += beta * old[i].x; x.y += beta * old[i].y;
-            x.z += beta * old[i].z; x.w += beta * old[i].w;
-            if (flags & G_MIRROR)
-              *reinterpret_cast<float4*>(&piece[(4 * i + sub) * TT_EP + wc]) = x;
-          }
-          if (r >= m_valid || c >= cend) continue;
-          const long long idx = (long long)gr * ldc + n0 + c;
-          if (vec && c + 3 < cend) {
-            *reinterpret_cast<float4*>(C + idx) = x;
-            if (C2 != nullptr) *reinterpret_cast<float4*>(C2 + idx) = x;
-          } else {
-            const float xs[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (c + e < cend) {
-                C[idx + e] = xs[e];
-                if (C2 != nullptr) C2[idx + e] = xs[e];
-              }
-          }
-        }
-        // C of the next piece while this one is mirrored
-        prefetch(c0 + 32 * G);
-        if (flags & G_MIRROR) {
-          // the final values are in the piece; a row per lane, so that a
-          // column of the piece is a contiguous store
-          __syncwarp();
-          const int gr = m0 + row0 + lane;
-          if (lane < rows) {
-            float* dst = C + (long long)(n0 + c0) * ldc + gr;
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 x =
-                  *reinterpret_cast<const float4*>(&piece[lane * TT_EP + i]);
-              const float xs[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e, dst += ldc)
-                if (c0 + i + e < n_valid && n0 + c0 + i + e < gr) *dst = xs[e];
-            }
-          }
-        }
-      }
-      __syncwarp();
-    }
+    TileOut o;
+    o.m0 = m0; o.n0 = n0; o.m_valid = m_valid; o.n_valid = n_valid;
+    o.lr = lr; o.momentum = momentum;
+    tile_epilogue<TN, Map::kWarps / 4, PRE>(
+        g, o, tmem, nkb == 0, warp & 3, warp >> 2, lane,
+        reinterpret_cast<float*>(smem) + warp * 32 * TT_EP, [&] {
+          return mbar_wait_status(&ctl->accum, 0, &ctl->abort_flag,
+                                  &g_tile_status);
+        });
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -704,10 +656,10 @@ struct TileVariant {
   int threads, smem;
 };
 
-template <int TN, bool PRE, bool VEC>
+template <int TN, bool PRE, bool VEC, bool HALF = false>
 static TileVariant tile_variant() {
-  return {tc_tile_kernel<TN, PRE, VEC>, TileMap<TN>::kThreads,
-          TileMap<TN>::kSmem};
+  return {tc_tile_kernel<TN, PRE, VEC, HALF>, TileMap<TN, HALF>::kThreads,
+          TileMap<TN, HALF>::kSmem};
 }
 
 // [128 columns][precondition][16-byte rows]
@@ -716,6 +668,10 @@ static const TileVariant kTileVariants[2][2][2] = {
      {tile_variant<256, true, false>(), tile_variant<256, true, true>()}},
     {{tile_variant<128, false, false>(), tile_variant<128, false, true>()},
      {tile_variant<128, true, false>(), tile_variant<128, true, true>()}}};
+// [128 columns]: fp16 terms
+static const TileVariant kHalfVariants[2] = {
+    tile_variant<256, false, true, true>(),
+    tile_variant<128, false, true, true>()};
 
 int tc_prepare_tiles() {
   static std::mutex mu;
@@ -725,8 +681,10 @@ int tc_prepare_tiles() {
   KFAC_REQUIRE(dev >= 0 && dev < 64, "device index %d unsupported", dev);
   std::lock_guard<std::mutex> lock(mu);
   if (!done[dev]) {
-    for (int k = 0; k < 8; ++k) {
-      const TileVariant& v = kTileVariants[k >> 2][(k >> 1) & 1][k & 1];
+    for (int k = 0; k < 10; ++k) {
+      const TileVariant& v = k < 8
+                                 ? kTileVariants[k >> 2][(k >> 1) & 1][k & 1]
+                                 : kHalfVariants[k - 8];
       KFAC_CUDA(cudaFuncSetAttribute(
           v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
     }
@@ -804,7 +762,12 @@ int launch_tc_grouped(const GemmDesc* descs_dev, const GemmDesc* descs_host,
       inl.n = n;
       std::copy(descs_host + first, descs_host + first + n, inl.d);
     }
-    const TileVariant& v = kTileVariants[tile_cols == 128][precond][k == 0];
+    bool half = k == 0 && !precond;
+    for (int i = 0; half && i < n; ++i)
+      half = (descs_host[first + i].flags & G_HALF) != 0;
+    const TileVariant& v =
+        half ? kHalfVariants[tile_cols == 128]
+             : kTileVariants[tile_cols == 128][precond][k == 0];
     v.kernel<<<end - tile0, v.threads, v.smem, stream>>>(
         descs_dev + first, n, tile0, inl, lr, momentum);
     KFAC_LAUNCH_CHECK("tc_tile_kernel");

@@ -688,6 +688,60 @@ def test_inverse_reports_non_spd(ops):
     plan.close()
 
 
+@pytest.mark.parametrize('d', [97, 130, 640, 1100, 2200])
+def test_inverse_of_badly_scaled_factors(ops, d):
+    """Columns whose scales span six orders of magnitude: the error of entry
+    (i, j) against sqrt(inv_ii inv_jj), the bound a Cholesky factorisation has
+    whatever the scales (condition of the scaled factor about 30, fp32 sums of
+    at most d terms: d 2^-24 30 at worst, 4e-3 at 2200; 1e-4 as everywhere)."""
+    rng = np.random.default_rng(d)
+    x = rng.standard_normal((2 * d, d))
+    x *= np.logspace(-3, 3, d)[rng.permutation(d)]
+    f = (x.T @ x / (2 * d)).astype(np.float32)
+    f = (f + f.T) / 2
+    F = [dev(f)]
+    inv = [torch.empty_like(F[0])]
+    plan = ops.InversePlan(F, inv, [-1], [2], scale=[1.0])
+    plan.run(1e-6)
+    torch.cuda.synchronize()
+    assert host(plan.info).tolist() == [0]
+    truth = np.linalg.inv(f.astype(np.float64) + 1e-6 * np.eye(d))
+    s = np.sqrt(np.diag(truth))
+    got = host(inv[0])
+    assert np.array_equal(got, got.T)
+    assert (np.abs(got - truth) / s[:, None] / s[None, :]).max() < 1e-4
+    plan.close()
+
+
+@pytest.mark.parametrize('d,row,col', [(40, 30, 5), (400, 390, 5),
+                                       (700, 600, 130), (1300, 1290, 700)])
+def test_inverse_reports_the_first_failing_pivot(ops, d, row, col):
+    """A large entry left of row `row` makes that pivot negative, wherever the
+    entry takes part in a product, and no pivot before it."""
+    a = np.eye(d, dtype=np.float32)
+    a[row, col] = a[col, row] = 1e6
+    F = [dev(a)]
+    inv = [torch.empty_like(F[0])]
+    plan = ops.InversePlan(F, inv, [-1], [2], scale=[0.0])
+    plan.run(0.0)
+    assert host(plan.info).tolist() == [row + 1]
+    plan.close()
+
+
+@pytest.mark.parametrize('value', [float('inf'), float('nan')])
+@pytest.mark.parametrize('d,row,col', [(300, 200, 5), (1100, 1000, 20)])
+def test_inverse_of_a_non_finite_factor_is_not_finite(ops, value, d, row, col):
+    a = np.eye(d, dtype=np.float32)
+    a[row, col] = a[col, row] = value
+    F = [dev(a)]
+    inv = [torch.empty_like(F[0])]
+    plan = ops.InversePlan(F, inv, [-1], [2], scale=[0.0])
+    plan.run(0.0)
+    assert host(plan.info).tolist() == [row + 1]
+    assert not np.isfinite(host(inv[0])).all()
+    plan.close()
+
+
 # ------------------------------------------------------------- precondition
 def precond_case(rng, dG, dW, bias):
     dA = dW + int(bias)
