@@ -1428,17 +1428,17 @@ extern "C" int kfac_inverse_plan_create(
 
   int prev_far_ev = -1;
   // Two-level Cholesky: panels of CW columns are factored by 128-wide inner steps
-  // whose updates stay inside the panel (short contractions, little work).  A
-  // panel's columns get the rest in two parts: everything but the panel right
-  // before them while that one's chain runs (far stream; a contraction over all
-  // panels so far, so that C is passed over once and not once per panel), and
-  // that panel's share when its chain ends (near).
+  // whose updates stay inside the panel (or one block column more, see `ahead`;
+  // short contractions, little work).  The other columns get a panel's share in two
+  // parts: everything but the panel right before them while that one's chain
+  // runs (far stream; a contraction over all panels so far, so that C is passed
+  // over once and not once per panel), and that panel's share when its chain
+  // ends (near).
   //
-  // The chain carries the diagonal kernels; inside a panel the diagonal
-  // kernel of step k applies step k-1's update to its own block itself
-  // (diag_lookahead), so it only waits for the panel update of step k-2.  The
-  // panel solves and panel updates of the steps run on the bulk stream behind
-  // the chain.  A panel solve leaves W as it is (the look-ahead reads it) and
+  // The chain carries the diagonal kernels; the diagonal kernel of step k applies
+  // step k-1's update to its own block itself (diag_lookahead), so it only waits
+  // for the panel update of step k-2.  The panel solves, panel updates and near
+  // updates run on the bulk stream behind the chain.  A panel solve leaves W as it is (the look-ahead reads it) and
   // stores L as fp16 chunks, which is how every product reads it.
   //
   // The inverse grows with the factor, a row panel at a time: with X = L^-1,
@@ -1590,12 +1590,23 @@ extern "C" int kfac_inverse_plan_create(
     end_gemm(next_t, false);
     end_gemm(prod, false);
   };
+  // Whether a panel's steps also update the next one's first block column.  The
+  // chain then goes on there without waiting for the near update, which only
+  // the second block needs (4608 rows beside 512: 1766 -> 1684 us); where the
+  // tiles fill the SMs anyway, the passes over that column only cost (108
+  // factors of ResNet-50, plans of 120, 309 and 225 row tiles: 4605 us without,
+  // 4650 in the first plan, 4690 in all).
+  long long row_tiles = 0;
+  for (int i = 0; i < count; ++i) row_tiles += (dims[i] + DB - 1) / DB;
+  const bool ahead = look && 2 * row_tiles <= sm_count();
+  const int E = ahead ? DB : 0;
+  int near_ev = -1;            // near updates of the panel before
   for (int co = 0; co < dmax; co += CW) {
     const int inner = std::min(CW, dmax - co);
     bulk_ev = -1;
     int last_solve_ev = -1;
     for (int o = co; o < co + inner; o += DB) {
-      const bool lk = look && o > co;
+      const bool lk = look && (ahead ? o > 0 : o > co);
       // the matrices that still have a block here are the first of `order`
       Launch dl = begin_gemm(S_CHAIN);
       dl.kind = 0;
@@ -1603,7 +1614,10 @@ extern "C" int kfac_inverse_plan_create(
       dl.look = lk;
       for (int i : order)
         if (dims[i] > o) dl.n += 1;
-      if (lk && o - 2 * DB >= co) dl.wait(upd_ev[(o - 2 * DB) / DB]);
+      if (lk && o >= 2 * DB && (ahead || o - 2 * DB >= co))
+        dl.wait(upd_ev[o / DB - 2]);
+      // (without look-ahead all of this is one stream)
+      if (look && o == (ahead ? co + DB : co)) dl.wait(near_ev);
       diag_ev[o / DB] = end_gemm(dl, look);
 
       Launch trsm = begin_gemm(s_bulk);
@@ -1631,15 +1645,16 @@ extern "C" int kfac_inverse_plan_create(
       const int solve_ev = end_gemm(trsm, look);
       if (solve_ev >= 0) bulk_ev = last_solve_ev = solve_ev;
 
-      // update the rest of this panel's columns (full rectangle; entries
-      // above the diagonal are written but never read).  With look-ahead the
-      // next diagonal block is left to the next diagonal kernel.
-      const int skip = (look && o + DB < co + inner) ? DB : 0;
+      // update the rest of this panel's columns, with `ahead` the block column
+      // after them too (full rectangle; entries above the diagonal are written
+      // but never read).  With look-ahead the next diagonal block is left to the next
+      // diagonal kernel.
+      const int skip = look && (ahead || o + DB < co + inner) ? DB : 0;
       Launch upd = begin_gemm(s_bulk);
       for (int i : order) {
         const int d = dims[i];
         const int M = d - o - DB - skip;
-        const int N = std::min(co + CW, d) - (o + DB);
+        const int N = std::min(co + CW + E, d) - (o + DB);
         if (M <= 0 || N <= 0) continue;
         const MatInfo& m = mats[i];
         const long long ld = m.ld;
@@ -1660,68 +1675,42 @@ extern "C" int kfac_inverse_plan_create(
       if ((o + DB) % PW == 0 && o + DB < co + inner) row_panel(o + DB - PW);
     }
 
-    // Updates behind the finished panel: the columns of the next panel with this
-    // one (needed before the chain can go on) on the chain's stream, those of
-    // the panel after it with all panels so far on the far stream, next to the
-    // next panel's chain.  What touches the same tiles is ordered by events
-    // (near of a panel after far of the one before).
-    Launch near = begin_gemm(S_CHAIN);
+    // Updates behind the finished panel, for windows of columns that begin with a
+    // panel (`ahead`: one block later): the next window with this panel, the window after it with all panels so
+    // far, next to the next panel's chain.  What touches the same tiles is
+    // ordered by events (near of a panel after far of the one before).
+    Launch near = begin_gemm(s_bulk);
     std::vector<GemmDesc> far_descs;
-    for (int i : order) {
-      const int d = dims[i];
-      const int M = d - co - CW;
-      if (M <= 0) continue;
-      const int N1 = std::min(CW, M);
-      const MatInfo& m = mats[i];
+    auto window = [&](const MatInfo& m, int d, int s, int k, int K,
+                      std::vector<GemmDesc>& out) {
+      const int M = d - s, N = std::min(CW, M);
+      if (M <= 0) return;
       const long long ld = m.ld;
-      const float* panel = m.W + (co + CW) * ld + co;
-      {
-        GemmDesc g = {};     // square block on the diagonal: lower tiles
-        const long long coff = (co + CW) * ld + (co + CW);
-        g.A = strided_operand(panel, 1, ld, N1);
-        g.B = g.A;
-        g.C = m.W + coff;
-        g.ldc = ld; g.M = N1; g.N = N1; g.K = CW;
-        g.alpha = -1.f; g.beta = 1.f; g.flags = G_LOWER | G_SAME_AB | packed;
-        set_l(g, m, co + CW, co + CW, co);
-        push_desc(near, g);
-      }
-      if (M > N1) {
-        const float* below = panel + N1 * ld;
-        GemmDesc g = {};     // rectangle below it
-        const long long coff = (co + CW + N1) * ld + (co + CW);
-        g.A = strided_operand(below, 1, ld, M - N1);
-        g.B = strided_operand(panel, 1, ld, N1);
-        g.C = m.W + coff;
-        g.ldc = ld; g.M = M - N1; g.N = N1; g.K = CW;
-        g.alpha = -1.f; g.beta = 1.f; g.flags = packed;
-        set_l(g, m, co + CW + N1, co + CW, co);
-        push_desc(near, g);
-      }
-      // the columns of the panel after the next: all panels so far
-      const int f = co + 2 * CW, F = d - f;
-      if (F > 0) {
-        const int N2 = std::min(CW, F);
-        GemmDesc h = {};     // square block on the diagonal
-        h.A = strided_operand(m.W + (long long)f * ld, 1, ld, N2);
-        h.B = h.A;
-        h.C = m.W + (long long)f * ld + f;
-        h.ldc = ld; h.M = N2; h.N = N2; h.K = co + CW;
-        h.alpha = -1.f; h.beta = 1.f; h.flags = G_LOWER | G_SAME_AB | packed;
-        set_l(h, m, f, f, 0);
-        far_descs.push_back(h);
-        if (F > N2) {
-          GemmDesc r = {};   // rectangle below it
-          r.A = strided_operand(m.W + (long long)(f + N2) * ld, 1, ld, F - N2);
-          r.B = strided_operand(m.W + (long long)f * ld, 1, ld, N2);
-          r.C = m.W + (long long)(f + N2) * ld + f;
-          r.ldc = ld; r.M = F - N2; r.N = N2; r.K = co + CW;
-          r.alpha = -1.f; r.beta = 1.f; r.flags = packed;
-          set_l(r, m, f + N2, f, 0);
-          far_descs.push_back(r);
-        }
-      }
+      const float* rows = m.W + s * ld + k;
+      GemmDesc g = {};     // square block on the diagonal: lower tiles
+      g.A = strided_operand(rows, 1, ld, N);
+      g.B = g.A;
+      g.C = m.W + s * ld + s;
+      g.ldc = ld; g.M = N; g.N = N; g.K = K;
+      g.alpha = -1.f; g.beta = 1.f; g.flags = G_LOWER | G_SAME_AB | packed;
+      set_l(g, m, s, s, k);
+      out.push_back(g);
+      if (M == N) return;
+      GemmDesc h = {};     // rectangle below it
+      h.A = strided_operand(rows + N * ld, 1, ld, M - N);
+      h.B = strided_operand(rows, 1, ld, N);
+      h.C = m.W + (long long)(s + N) * ld + s;
+      h.ldc = ld; h.M = M - N; h.N = N; h.K = K;
+      h.alpha = -1.f; h.beta = 1.f; h.flags = packed;
+      set_l(h, m, s + N, s, k);
+      out.push_back(h);
+    };
+    std::vector<GemmDesc> near_descs;
+    for (int i : order) {
+      window(mats[i], dims[i], co + CW + E, co, CW, near_descs);
+      window(mats[i], dims[i], co + 2 * CW + E, 0, co + CW, far_descs);
     }
+    for (auto& g : near_descs) push_desc(near, g);
     int panel_ev = last_solve_ev;
     if (!look && !far_descs.empty()) {
       // the far part needs the finished panel: an event recorded on the
@@ -1730,9 +1719,8 @@ extern "C" int kfac_inverse_plan_create(
       launches.back().rec_ev = panel_ev;   // last launch of the panel's chain
     }
     near.wait(prev_far_ev);                // far part of the previous panel
-    if (look) near.wait(panel_ev);         // the bulk stream's last solve
     if (near.n > 0) prev_far_ev = -1;
-    end_gemm(near, false);
+    near_ev = end_gemm(near, look);
     Launch far = begin_gemm(S_FAR);
     for (auto& h : far_descs) push_desc(far, h);
     far.wait(panel_ev);
