@@ -212,38 +212,46 @@ constexpr int DLD = DB + 4;   // shared-memory row pitch of a 128 x 128 block
 constexpr int SB = 32;        // sub-block of the diagonal kernel
 constexpr int SLP = SB + 4;   // row pitch of a 32 x 32 sub-block
 constexpr int DT = 512;       // threads of the diagonal kernel
-constexpr int kLookTile = DB * 32 * 4;          // one 128 x 32 fp32 operand tile
-constexpr int kLookStage = 4 * kLookTile;       // [A hi][A lo][B hi][B lo]
+constexpr int kLookTile = DB * 128;    // both fp16 terms of 128 rows x 32 k
+constexpr int kLookBytes = 8 * kLookTile;       // four k-blocks of A' and of X
 constexpr int kLookCols = 2 * DB;               // tensor-memory columns
 
 static __device__ int g_diag_status = 0;
 
 struct LookControl {
-  unsigned long long bar[2];   // a stage's MMAs have finished reading it
-  unsigned long long done;     // all MMAs of the second product have finished
+  unsigned long long done[2];  // all MMAs of the first, second product
   unsigned tmem_base;
   volatile int abort_flag;
 };
 
-// Issue the three split-TF32 MMAs of one 32-k operand block: D(128 x n) +=
-// A B^T with A, B given as hi / lo tile addresses (K-major, 128-byte
-// swizzle).  hi*hi goes to columns [0, 128) of the tensor memory, the cross
-// terms to [128, 256).
-__device__ __forceinline__ void look_mma_block(unsigned tmem, unsigned a_hi,
-                                               unsigned a_lo, unsigned b_hi,
-                                               unsigned b_lo, int n,
-                                               bool first) {
-  const unsigned idesc = tc_instr_desc(n);
-  const unsigned long long dah = tc_smem_desc(a_hi), dal = tc_smem_desc(a_lo);
-  const unsigned long long dbh = tc_smem_desc(b_hi), dbl = tc_smem_desc(b_lo);
+// Issue the three MMAs per product of one 32-k operand block: D(128 x n) += A B^T
+// with A, B given as tiles of 128-byte rows, hi terms then lo terms.  hi*hi goes
+// to columns [0, 128) of the tensor memory, the cross terms to [128, 256).
+__device__ __forceinline__ void look_mma_block(unsigned tmem, unsigned a,
+                                               unsigned b, int n, bool first) {
+  const unsigned idesc = tc_half_desc(n, false, false);
+  const unsigned long long da = tc_smem_desc(a), db = tc_smem_desc(b);
+  constexpr unsigned long long lo = 64 >> 4;
 #pragma unroll
-  for (int kk = 0; kk < 4; ++kk) {
+  for (int kk = 0; kk < 2; ++kk) {
     const unsigned long long adv = (unsigned long long)(kk * 32 >> 4);
     const unsigned acc = (first && kk == 0) ? 0u : 1u;
-    tc_mma(tmem + DB, dal + adv, dbh + adv, idesc, acc);
-    tc_mma(tmem + DB, dah + adv, dbl + adv, idesc, 1u);
-    tc_mma(tmem, dah + adv, dbh + adv, idesc, acc);
+    tc_mma_half(tmem + DB, da + lo + adv, db + adv, idesc, acc);
+    tc_mma_half(tmem + DB, da + adv, db + lo + adv, idesc, 1u);
+    tc_mma_half(tmem, da + adv, db + adv, idesc, acc);
   }
+}
+
+// Four scaled values of a row as fp16 terms into a tile (8-byte word `word` of
+// the row's hi and lo terms).
+__device__ __forceinline__ void look_store4(unsigned tile, int row, int word,
+                                            float4 x, float scale) {
+  const unsigned d = tile + sw128_chunk_off(row, word >> 1) + 8 * (word & 1);
+  unsigned h0, h1, l0, l1;
+  split_half2(scale * x.x, scale * x.y, h0, l0);
+  split_half2(scale * x.z, scale * x.w, h1, l1);
+  sts64(d, h0, h1);
+  sts64(d ^ 0x40u, l0, l1);
 }
 
 // 16 bytes global -> shared without a register in between.
@@ -282,9 +290,8 @@ __device__ __forceinline__ void diag_load_wait() {
 // Barriers and tensor memory of the look-ahead; needs nothing of the matrix.
 __device__ __forceinline__ void look_begin(LookControl* ctl) {
   if (threadIdx.x == 32) {
-    mbar_init(&ctl->bar[0], 1);
-    mbar_init(&ctl->bar[1], 1);
-    mbar_init(&ctl->done, 1);
+    mbar_init(&ctl->done[0], 1);
+    mbar_init(&ctl->done[1], 1);
     ctl->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -305,10 +312,12 @@ __device__ __forceinline__ void look_begin(LookControl* ctl) {
 // leaves as it was) and X_pp (inverse of the previous diagonal block's factor),
 // so that this kernel does not have to wait for the panel solve and panel
 // update of step k - 1.  Both products run on the tensor cores (tcgen05,
-// split TF32, accumulators in tensor memory).  All global loads are in flight
-// at once (16 x 16 bytes per thread); the blocks of X_pp above its diagonal
-// are neither loaded nor multiplied.  Result: D in S.  Returns false if a
-// bounded wait ran out (the status word is set; the caller stores nothing).
+// operands in two fp16 terms, accumulators in tensor memory).  All global loads
+// are in flight at once (16 x 16 bytes per thread); the blocks of X_pp above its
+// diagonal are neither loaded nor multiplied.  Result: D in S.  Returns false if
+// a bounded wait ran out (the status word is set; the caller stores nothing).
+// With TF32 terms, twice the MMA time and shared memory for two k-blocks at a
+// time, the whole kernel took 31.7 us on average of a plan of 856 rows, now 29.6.
 __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
                                                bool vec, float* S,
                                                unsigned char* stage,
@@ -317,12 +326,16 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
   const long long ld = mi.ld;
   const float* Ap = mi.W + (long long)o * ld + (o - DB);
   const float* Xp = mi.X + (long long)(o - DB) * ld + (o - DB);
+  // rows of a warp: eight; those of a half warp differ in the bit that moves the
+  // swizzle across the halves of a 128-byte row (8-byte stores)
+  const int row0 = 8 * warp + 4 * ((lane >> 3) & 1) + (lane >> 4);
+  const int word = lane & 7;
   float4 va[4][2], vx[4][2];
 #pragma unroll
   for (int kb = 0; kb < 4; ++kb) {
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const int c = tid + DT * j, row = c >> 3, col = 32 * kb + 4 * (c & 7);
+      const int row = row0 + 2 * j, col = 32 * kb + 4 * word;
       va[kb][j] = vx[kb][j] = make_float4(0.f, 0.f, 0.f, 0.f);
       const float* pa = &Ap[row * ld + col];
       const float* px = &Xp[row * ld + col];
@@ -344,58 +357,60 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
   const unsigned sbase = smem_u32(stage);
   bool ok = true;
 
-  // ---- L' = A' X_pp^T: four operand blocks of 32 k through two stages
+  // ---- L' = A' X_pp^T, a block of 32 k at a time behind its MMAs
 #pragma unroll
   for (int kb = 0; kb < 4; ++kb) {
-    const int s = kb & 1;
-    if (kb >= 2) ok = mbar_wait_status(&ctl->bar[s], 0, &ctl->abort_flag,
-                                       &g_diag_status) && ok;
-    const unsigned st = sbase + s * kLookStage;
+    const unsigned ta = sbase + 2 * kb * kLookTile, tx = ta + kLookTile;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const int c = tid + DT * j, row = c >> 3;
-      const unsigned off = (unsigned)sw128_chunk_off(row, c & 7);
-      store_split(st + off, st + kLookTile + off, va[kb][j]);
-      if (row >= 32 * kb)
-        store_split(st + 2 * kLookTile + off, st + 3 * kLookTile + off,
-                    vx[kb][j]);
+      const int row = row0 + 2 * j;
+      look_store4(ta, row, word, va[kb][j], kScaleL);
+      if (row >= 32 * kb) look_store4(tx, row, word, vx[kb][j], kScaleX);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    if (warp == 0 && !ctl->abort_flag && elect_one()) {
+    if (warp == 0 && elect_one()) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // columns below 32 kb of L' get nothing from this block of k
-      const unsigned skip = (unsigned)(32 * kb) * 128;
-      look_mma_block(tmem + 32 * kb, st, st + kLookTile,
-                     st + 2 * kLookTile + skip, st + 3 * kLookTile + skip,
+      look_mma_block(tmem + 32 * kb, ta, tx + (unsigned)(32 * kb) * 128,
                      DB - 32 * kb, kb == 0);
-      tc_commit(&ctl->bar[s]);
+      if (kb == 3) tc_commit(&ctl->done[0]);
     }
   }
-  ok = mbar_wait_status(&ctl->bar[0], 1, &ctl->abort_flag, &g_diag_status) && ok;
-  ok = mbar_wait_status(&ctl->bar[1], 1, &ctl->abort_flag, &g_diag_status) && ok;
+  ok = mbar_wait_status(&ctl->done[0], 0, &ctl->abort_flag, &g_diag_status);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
   // ---- L' out of tensor memory, split, into the operand blocks of the second
-  // product (A and B are the same matrix: [hi][lo] per 32 k, four blocks)
+  // product (A and B are the same matrix: four blocks of 32 k)
   const int q = warp & 3, h = warp >> 2;
   const int row = 32 * q + lane;
   ok = __all_sync(0xffffffffu, ok);     // the loads below are warp-wide
   if (ok) {
-    const unsigned blk = sbase + (unsigned)h * (2 * kLookTile);
+    const unsigned blk = sbase + (unsigned)h * kLookTile;
+    // (the scale of A' X_pp^T is kScaleL kScaleX; L' keeps kScaleL of it)
+    constexpr float s = 1.f / kScaleX;
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc) {
       const int c0 = 32 * h + 16 * cc;
       float v[16], w[16];
-      tc_ld16(tmem + ((unsigned)(32 * q) << 16) + (unsigned)c0, v);
-      tc_ld16(tmem + ((unsigned)(32 * q) << 16) + (unsigned)(DB + c0), w);
+      tc_ld16_pair(tmem + ((unsigned)(32 * q) << 16) + (unsigned)c0,
+                   tmem + ((unsigned)(32 * q) << 16) + (unsigned)(DB + c0), v,
+                   w);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 x = make_float4(v[4 * i] + w[4 * i], v[4 * i + 1] + w[4 * i + 1],
-                                     v[4 * i + 2] + w[4 * i + 2],
-                                     v[4 * i + 3] + w[4 * i + 3]);
-        const unsigned off = (unsigned)sw128_chunk_off(row, 4 * cc + i);
-        store_split(blk + off, blk + kLookTile + off, x);
+      for (int i = 0; i < 2; ++i) {
+        unsigned hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = 8 * i + 2 * e;
+          split_half2(s * (v[c] + w[c]), s * (v[c + 1] + w[c + 1]), hi[e],
+                      lo[e]);
+        }
+        const unsigned d = blk + sw128_chunk_off(row, 2 * cc + i);
+        sts128(d, make_float4(__uint_as_float(hi[0]), __uint_as_float(hi[1]),
+                              __uint_as_float(hi[2]), __uint_as_float(hi[3])));
+        sts128(d ^ 0x40u,
+               make_float4(__uint_as_float(lo[0]), __uint_as_float(lo[1]),
+                           __uint_as_float(lo[2]), __uint_as_float(lo[3])));
       }
     }
   }
@@ -407,32 +422,33 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
     for (int kb = 0; kb < 4; ++kb) {
-      const unsigned blk = sbase + (unsigned)kb * (2 * kLookTile);
-      look_mma_block(tmem, blk, blk + kLookTile, blk, blk + kLookTile, DB,
-                     kb == 0);
+      const unsigned blk = sbase + (unsigned)kb * kLookTile;
+      look_mma_block(tmem, blk, blk, DB, kb == 0);
     }
-    tc_commit(&ctl->done);
+    tc_commit(&ctl->done[1]);
   }
   diag_load_wait();
-  ok = mbar_wait_status(&ctl->done, 0, &ctl->abort_flag, &g_diag_status) && ok;
+  ok = mbar_wait_status(&ctl->done[1], 0, &ctl->abort_flag, &g_diag_status) && ok;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   __syncthreads();                      // every thread's part of W_kk is there
   ok = __all_sync(0xffffffffu, ok);
   if (ok && h <= q) {                   // sub-blocks on and below the diagonal
+    constexpr float s = -1.f / (kScaleL * kScaleL);
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc) {
       const int c0 = 32 * h + 16 * cc;
       float v[16], w[16];
-      tc_ld16(tmem + ((unsigned)(32 * q) << 16) + (unsigned)c0, v);
-      tc_ld16(tmem + ((unsigned)(32 * q) << 16) + (unsigned)(DB + c0), w);
+      tc_ld16_pair(tmem + ((unsigned)(32 * q) << 16) + (unsigned)c0,
+                   tmem + ((unsigned)(32 * q) << 16) + (unsigned)(DB + c0), v,
+                   w);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float4* s4 = reinterpret_cast<float4*>(&S[row * DLD + c0 + 4 * i]);
         float4 d = *s4;
-        d.x -= v[4 * i] + w[4 * i];
-        d.y -= v[4 * i + 1] + w[4 * i + 1];
-        d.z -= v[4 * i + 2] + w[4 * i + 2];
-        d.w -= v[4 * i + 3] + w[4 * i + 3];
+        d.x += s * (v[4 * i] + w[4 * i]);
+        d.y += s * (v[4 * i + 1] + w[4 * i + 1]);
+        d.z += s * (v[4 * i + 2] + w[4 * i + 2]);
+        d.w += s * (v[4 * i + 3] + w[4 * i + 3]);
         *s4 = d;
       }
     }
@@ -789,7 +805,7 @@ __device__ __forceinline__ void diag_update_block(DiagSmem& sm, int r, int half,
 // the chain goes on), the rows that follow it (six warps, then the followers
 // go on), and the columns beyond next to the next chain.  128 rows: 61 us with
 // 8 x 8 register blocks per thread and a barrier per block column, 20 us now with
-// the launch, 31 us with the look-ahead's two products in front.
+// the launch, 29 us with the look-ahead's two products in front.
 template <bool LOOK>
 __global__ void __launch_bounds__(DT, 1)
 chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
@@ -801,7 +817,7 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
   // written only after its last barrier
   unsigned char* stage = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(dsm + DB * DLD) + 1023) & ~(uintptr_t)1023);
-  LookControl* ctl = reinterpret_cast<LookControl*>(stage + 2 * kLookStage);
+  LookControl* ctl = reinterpret_cast<LookControl*>(stage + kLookBytes);
   if (LOOK) look_begin(ctl);
   const MatInfo mi = mats[blockIdx.x];
   const int id = mi.id;
@@ -1159,7 +1175,7 @@ refine_apply_kernel(const MatInfo* __restrict__ mats,
 
 constexpr size_t kDiagSmemBytes = sizeof(DiagSmem);
 constexpr size_t kDiagLookSmemBytes =
-    DB * DLD * sizeof(float) + 1024 + 2 * kLookStage + 256;
+    DB * DLD * sizeof(float) + 1024 + kLookBytes + 256;
 static_assert(kDiagLookSmemBytes >= kDiagSmemBytes &&
                   kDiagLookSmemBytes <= 227 * 1024,
               "diagonal kernel shared memory");
