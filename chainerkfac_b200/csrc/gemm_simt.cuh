@@ -286,6 +286,26 @@ struct GemmDesc {
   float pack_scale;
   int pack_kind;
   const float* unscale;    // if set, C(m, n) = .. + unscale[m] unscale[n] A B
+  // preconditioning in chunks: reciprocals of the scales of A^T's rows and B's
+  // columns; norms of A_inv's rows and the largest norm of a gradient row (float
+  // bits), which bound the first product
+  const float *rs, *cs;
+  const float* norm;
+  const unsigned* peak;
+};
+
+// Rows of a matrix (and an appended column) as K-major chunks, each scaled by a
+// power of two of its own.
+struct PackRows {
+  const float* src;
+  const float* extra;      // appended column, NULL: none
+  unsigned char* dst;
+  float* inv;              // reciprocal of a row's scale
+  float* norm;             // 2-norm of a row, NULL: not wanted
+  unsigned* peak;          // largest of the norms (atomic maximum of the bits)
+  int rows, cols;
+  int row_begin;           // first row in the launch
+  int pad_;
 };
 
 int launch_grouped_gemm(const GemmDesc* descs_dev, int ndesc, int total_tiles,
@@ -322,6 +342,13 @@ int packed_prepare();
 int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
                   int ndesc, int total_tiles, cudaStream_t stream);
 int packed_status_read(int* out);
+// Preconditioning on chunks: rows into chunks, then the product whose result is
+// chunks again (`last` false) or the preconditioned gradient.
+int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,
+                     int njobs, int rows, cudaStream_t stream);
+int launch_packed_precond(const GemmDesc* descs_dev, const GemmDesc* descs_host,
+                          int ndesc, int total_tiles, bool last, float lr,
+                          float momentum, cudaStream_t stream);
 bool tc_desc_has_tails(const GemmDesc& g);
 size_t tc_factor_workspace_bytes(long long rows, int d, bool staged = true);
 size_t tc_lone_workspace_bytes(const Operand& X, long long rows, int d);

@@ -1,6 +1,8 @@
 // Preconditioning kf = G_inv * [grad_W, grad_b] * A_inv for all layers in two
 // grouped launches; the second launch's epilogue splits the result into the
-// weight and bias parts and can apply the momentum update in place.
+// weight and bias parts and can apply the momentum update in place.  Larger
+// calls go through fp16 chunks (tc_packed.cu): a launch that writes the three
+// operands' rows as chunks, U = grad * A_inv^T, kf = G_inv * U.
 #include <vector>
 
 #include "gemm_simt.cuh"
@@ -9,16 +11,162 @@ using namespace kfac;
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// One layer's operands in chunks and their rows' scales, offsets in bytes.
+struct ChunkLayout {
+  size_t G, A, g, U;             // G_inv, A_inv, gradient, grad * A_inv^T
+  size_t inv_G, inv_A, inv_g, norm_A;
+  size_t total;
+};
+
+static ChunkLayout chunk_layout(int dG, int dA) {
+  auto chunks = [](int rows, int k) {
+    return (size_t)((rows + 127) / 128) * ((k + 31) / 32) * kChunk;
+  };
+  ChunkLayout c;
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t here = at;
+    at += align256(bytes);
+    return here;
+  };
+  c.G = take(chunks(dG, dG));
+  c.A = take(chunks(dA, dA));
+  c.g = take(chunks(dG, dA));
+  c.U = take(chunks(dA, dG));
+  c.inv_G = take(dG * sizeof(float));
+  c.inv_A = take(dA * sizeof(float));
+  c.inv_g = take(dG * sizeof(float));
+  c.norm_A = take(dA * sizeof(float));
+  c.total = at;
+  return c;
+}
+
+// Whether a call goes through chunks: it costs a launch and a half more (27 us
+// against 17 at the smallest sizes), a k-block 0.4 us instead of 0.75, or of 1.05
+// where the tile kernel cannot load 16-byte words.  The longest layer decides, by
+// its k-blocks in both products.  us by one launch kind and the other: 256 x 256
+// (16 k-blocks) 27 33, 128 x 512 (20) 30 35, 512 x 512 (32) 41 39, 512 x 2048 (80)
+// 78 61, 512 x 4608 165 138; with odd sides 53 x 334 (13) 30 33, 211 x 130 (12)
+// 33 33, 301 x 785 (35) 64 51, 1000 x 10 (33) 49 32, 1000 x 1001 102 62.
+static bool chunks_pay(int count, const int* dG, const int* dW,
+                       const std::vector<int>& hb) {
+  for (int i = 0; i < count; ++i) {
+    const int dA = dW[i] + hb[i];
+    const int blocks = (dA + 31) / 32 + (dG[i] + 31) / 32;
+    const bool words = ((dG[i] | dW[i] | hb[i]) & 3) == 0;
+    if (blocks >= (words ? 32 : 20)) return true;
+  }
+  return false;
+}
+
+// kfac_precondition through chunks.
+static int precondition_chunks(
+    int count, const int* dG, const int* dW, const std::vector<int>& hb,
+    const float* const* G_inv, const float* const* A_inv,
+    const float* const* grad_W, const float* const* grad_b, float* const* kf_W,
+    float* const* kf_b, float* const* param_W, float* const* param_b,
+    float* const* mom_W, float* const* mom_b, float lr, float momentum, char* ws,
+    cudaStream_t st) {
+  // tables and peaks, in front of the layers' chunks
+  const size_t jobs_at = align256(2 * (size_t)count * sizeof(GemmDesc));
+  const size_t peaks_at =
+      jobs_at + align256(3 * (size_t)count * sizeof(PackRows));
+  const size_t tables = peaks_at + align256((size_t)count * sizeof(unsigned));
+  std::vector<char> host(tables, 0);
+  GemmDesc* descs = reinterpret_cast<GemmDesc*>(host.data());
+  PackRows* jobs = reinterpret_cast<PackRows*>(host.data() + jobs_at);
+  char* const base = ws;
+  const GemmDesc* descs_dev = reinterpret_cast<GemmDesc*>(base);
+  unsigned* peaks = reinterpret_cast<unsigned*>(base + peaks_at);
+  ws += tables;
+  int njobs = 0;
+  int rows = 0;
+  auto at = [](char* base, size_t off) {
+    return reinterpret_cast<unsigned char*>(base + off);
+  };
+  auto vec = [](char* base, size_t off) {
+    return reinterpret_cast<float*>(base + off);
+  };
+  for (int i = 0; i < count; ++i) {
+    const int dg = dG[i], dw = dW[i], da = dw + hb[i];
+    const ChunkLayout c = chunk_layout(dg, da);
+    const long long nkA = (da + 31) / 32, nkG = (dg + 31) / 32;
+    auto job = [&](const float* src, const float* extra, size_t dst, size_t inv,
+                   float* norm, unsigned* peak, int nrows, int cols) {
+      PackRows j = {};
+      j.src = src; j.extra = extra; j.dst = at(ws, dst); j.inv = vec(ws, inv);
+      j.norm = norm; j.peak = peak; j.rows = nrows; j.cols = cols;
+      j.row_begin = rows;
+      rows += nrows;
+      jobs[njobs++] = j;
+    };
+    job(A_inv[i], nullptr, c.A, c.inv_A, vec(ws, c.norm_A), nullptr, da, da);
+    job(G_inv[i], nullptr, c.G, c.inv_G, nullptr, nullptr, dg, dg);
+    job(grad_W[i], hb[i] ? grad_b[i] : nullptr, c.g, c.inv_g, nullptr,
+        peaks + i, dg, dw);
+    // U = grad * A_inv^T
+    GemmDesc& u = descs[i];
+    u = GemmDesc();
+    u.A.kfast = u.B.kfast = 1;
+    u.M = dg; u.N = da; u.K = da;
+    u.alpha = 1.f;
+    u.ca = at(ws, c.g); u.ca_tile = nkA * kChunk;
+    u.cb = at(ws, c.A); u.cb_tile = nkA * kChunk;
+    u.pack = at(ws, c.U); u.pack_tile = nkG * kChunk;
+    u.rs = vec(ws, c.inv_g); u.cs = vec(ws, c.inv_A);
+    u.norm = vec(ws, c.norm_A); u.peak = peaks + i;
+    // kf = G_inv * U, split and (optionally) applied
+    GemmDesc& h = descs[count + i];
+    h = GemmDesc();
+    h.A.kfast = 1;
+    h.M = dg; h.N = da; h.K = dg;
+    h.alpha = 1.f;
+    h.ca = at(ws, c.G); h.ca_tile = nkG * kChunk;
+    h.cb = u.pack; h.cb_tile = u.pack_tile;
+    h.rs = vec(ws, c.inv_G);
+    h.norm = u.norm; h.peak = u.peak;
+    const bool fused = param_W && param_W[i];
+    h.kfW = kf_W ? kf_W[i] : nullptr;
+    h.kfb = (hb[i] && kf_b) ? kf_b[i] : nullptr;
+    h.pW = fused ? param_W[i] : nullptr;
+    h.vW = fused ? mom_W[i] : nullptr;
+    h.pb = (fused && hb[i]) ? param_b[i] : nullptr;
+    h.vb = (fused && hb[i]) ? mom_b[i] : nullptr;
+    h.dW = dw;
+    ws += c.total;
+  }
+  const int tiles = packed_number_tiles(descs, count);
+  packed_number_tiles(descs + count, count);             // the same tiles
+  // (the tables of a few layers travel as kernel arguments)
+  if (count > kTileInline)
+    KFAC_CUDA(cudaMemcpyAsync(base, host.data(), tables,
+                              cudaMemcpyHostToDevice, st));
+  else
+    KFAC_CUDA(cudaMemsetAsync(peaks, 0, count * sizeof(unsigned), st));
+  int rc = launch_pack_rows(reinterpret_cast<PackRows*>(base + jobs_at), jobs,
+                            njobs, rows, st);
+  if (rc == KFAC_OK)
+    rc = launch_packed_precond(descs_dev, descs, count, tiles, false, lr,
+                               momentum, st);
+  if (rc == KFAC_OK)
+    rc = launch_packed_precond(descs_dev + count, descs + count, count, tiles,
+                               true, lr, momentum, st);
+  return rc;
+}
+
 extern "C" size_t kfac_precond_workspace_bytes(int count, const int* dG,
                                                const int* dW,
                                                const int* has_bias) {
   if (count <= 0 || !dG || !dW) return 0;
   size_t total = align256(2 * (size_t)count * sizeof(GemmDesc));
+  size_t chunks = total + align256(3 * (size_t)count * sizeof(PackRows)) +
+                  align256((size_t)count * sizeof(unsigned));
   for (int i = 0; i < count; ++i) {
     size_t dA = (size_t)dW[i] + ((has_bias && has_bias[i]) ? 1 : 0);
     total += align256((size_t)dG[i] * dA * sizeof(float));
+    chunks += chunk_layout(dG[i], (int)dA).total;
   }
-  return total;
+  return total > chunks ? total : chunks;
 }
 
 extern "C" int kfac_precondition(
@@ -56,6 +204,11 @@ extern "C" int kfac_precondition(
                 workspace_bytes);
   cudaStream_t st = (cudaStream_t)stream;
   char* ws = static_cast<char*>(workspace);
+  if (engine() == 1 && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 &&
+      chunks_pay(count, dG, dW, hb))
+    return precondition_chunks(count, dG, dW, hb, G_inv, A_inv, grad_W, grad_b,
+                               kf_W, kf_b, param_W, param_b, mom_W, mom_b, lr,
+                               momentum, ws, st);
   GemmDesc* descs_dev = reinterpret_cast<GemmDesc*>(ws);
   ws += align256(2 * (size_t)count * sizeof(GemmDesc));
 

@@ -248,6 +248,14 @@ __device__ __forceinline__ void split_half2(float y0, float y1, unsigned& hi,
   lo = half2_sat(fmaf(y0, 0.f, y0 - f.x), fmaf(y1, 0.f, y1 - f.y));
 }
 
+// Power of two that brings values of up to `amax` (bits of a non-negative float)
+// to at most 2^15, and its reciprocal; both are normal numbers for every `amax`.
+__device__ __forceinline__ float half_scale(unsigned amax, float* inverse) {
+  const int e = max((int)(amax >> 23), 27) - 127;        // floor(log2)
+  *inverse = __uint_as_float((unsigned)(127 - 14 + e) << 23);
+  return __uint_as_float((unsigned)(127 + 14 - e) << 23);
+}
+
 // Two values as bf16 terms x = hi + lo: one word of each (the first value in the
 // low half).  Rounding to bf16 is an integer add of half an ulp (ties away from
 // zero); the byte permute then takes the upper halves.  No cvt: conversions issue

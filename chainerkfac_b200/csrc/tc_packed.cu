@@ -29,11 +29,16 @@
 
 namespace kfac {
 
-constexpr int KP_STAGES = 3;
+// Stages: three for two CTAs an SM.  Six in preconditioning launches without a
+// second tile for an SM (148 tiles with K = 4608: 66 us with three, 50 with six);
+// the inverse's launches run beside each other and keep room for two (108
+// factors of ResNet-50 with their preconditioning: 4384 us, 4500 with six stages
+// in its small launches).
+constexpr int KP_STAGES_MAX = 6;
 constexpr int KP_STAGE = 2 * kChunk;
 constexpr int KP_EPI_WARPS = 8;
 constexpr int KP_THREADS = 32 * (2 + KP_EPI_WARPS);
-constexpr int KP_SMEM = KP_STAGES * KP_STAGE + 2048;
+constexpr int packed_smem(int stages) { return stages * KP_STAGE + 2048; }
 // Longest contraction of one accumulator, in k-blocks of 32.  The tensor core
 // adds with truncation, so a sum drifts with the number of MMAs behind it; past
 // this many the accumulators are added to C (round to nearest) and start anew.
@@ -46,9 +51,15 @@ constexpr int KP_SEGMENT = 16;
 
 static __device__ int g_packed_status = 0;
 
+struct PackInline {
+  int n;                       // 0: jobs in device memory
+  PackRows j[3 * TT_INLINE];   // three operands a layer
+};
+static_assert(sizeof(PackInline) <= 3800, "kernel argument space");
+
 struct PackedControl {
-  unsigned long long full[KP_STAGES];    // the copies have arrived
-  unsigned long long empty[KP_STAGES];   // the MMAs have read the stage
+  unsigned long long full[KP_STAGES_MAX];    // the copies have arrived
+  unsigned long long empty[KP_STAGES_MAX];   // the MMAs have read the stage
   unsigned long long accum;              // a segment's accumulators are final
   unsigned long long drained;            // and have been read
   unsigned tmem_base;
@@ -98,22 +109,205 @@ __device__ __forceinline__ void piece_each(int r, int c, int rows, int cols,
   }
 }
 
-__global__ void __launch_bounds__(KP_THREADS, 2)
+// Scale of a column of U = grad A_inv^T as an operand of the second product:
+// its entries are at most the largest norm of a gradient row times the norm of
+// the column's row of A_inv.
+__device__ __forceinline__ float u_scale(const unsigned* peak, float norm,
+                                         float* inverse) {
+  return half_scale(__float_as_uint(__uint_as_float(*peak) * norm), inverse);
+}
+
+// First product of the preconditioning: a 16 x 32 piece of U into chunks, rows as
+// k (zeros up to the end of the last k-block).
+__device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
+                                        int r, int c) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int gr = r + 8 * h;
+    const bool in = gr < g.M;
+    const float s0 = g.rs[min(gr, g.M - 1)];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      // (columns past the last one: any values, nobody stores their results)
+      const int gc = c + 8 * j, k0 = min(gc, g.N - 1), k1 = min(gc + 1, g.N - 1);
+      float inverse;
+      const float x0 = in ? v[4 * j + 2 * h] * s0 * g.cs[k0] : 0.f;
+      const float x1 = in ? v[4 * j + 2 * h + 1] * s0 * g.cs[k1] : 0.f;
+      unsigned hi, lo;
+      split_half2(x0 * u_scale(g.peak, g.norm[k0], &inverse),
+                  x1 * u_scale(g.peak, g.norm[k1], &inverse), hi, lo);
+      unsigned char* p = g.pack + (long long)(gc >> 7) * g.pack_tile +
+                         (long long)(gr >> 5) * kChunk +
+                         ((gc >> 6) & 1) * 8192 +
+                         sw128_chunk_off(gr & 31, (gc & 63) >> 3) + 2 * (gc & 7);
+      *reinterpret_cast<unsigned*>(p) = hi;
+      *reinterpret_cast<unsigned*>(p + 4096) = lo;
+    }
+  }
+}
+
+// Second product: a 16 x 32 piece of kf to the weight and bias parts, and the
+// momentum update where the layer has it fused.
+__device__ __forceinline__ void store_kf(const GemmDesc& g, float v[16], int r,
+                                         int c, bool whole, float lr,
+                                         float momentum) {
+  const float s0 = g.rs[min(r, g.M - 1)], s1 = g.rs[min(r + 8, g.M - 1)];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float inverse;
+    u_scale(g.peak, g.norm[min(c + 8 * (j >> 1) + (j & 1), g.N - 1)], &inverse);
+    const int i = 4 * (j >> 1) + (j & 1);
+    v[i] = v[i] * s0 * inverse;
+    v[i + 2] = v[i + 2] * s1 * inverse;
+  }
+  const int dW = g.dW;
+  const bool fused = g.pW != nullptr;
+  if (whole && (dW & 1) == 0 &&
+      ((reinterpret_cast<uintptr_t>(g.kfW) | reinterpret_cast<uintptr_t>(g.pW) |
+        reinterpret_cast<uintptr_t>(g.vW)) & 7) == 0) {
+    const long long at = (long long)r * dW + c;
+    if (g.kfW != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<float2*>(g.kfW + at + 8 * (i >> 1) +
+                                   8LL * (i & 1) * dW) =
+            make_float2(v[2 * i], v[2 * i + 1]);
+    }
+    if (!fused) return;
+    float2 ov[8], op[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const long long d = at + 8 * (i >> 1) + 8LL * (i & 1) * dW;
+      ov[i] = *reinterpret_cast<const float2*>(g.vW + d);
+      op[i] = *reinterpret_cast<const float2*>(g.pW + d);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const long long d = at + 8 * (i >> 1) + 8LL * (i & 1) * dW;
+      const float n0 = momentum * ov[i].x - lr * v[2 * i];
+      const float n1 = momentum * ov[i].y - lr * v[2 * i + 1];
+      *reinterpret_cast<float2*>(g.vW + d) = make_float2(n0, n1);
+      *reinterpret_cast<float2*>(g.pW + d) =
+          make_float2(op[i].x + n0, op[i].y + n1);
+    }
+    return;
+  }
+  float ov[16], op[16];
+  auto part = [&](int dr, int dc, float* w, float* b) {
+    return c + dc < dW ? w + (long long)(r + dr) * dW + c + dc : b + r + dr;
+  };
+  if (fused)
+    // (past the edges the last row or column: no branch, all in flight)
+    piece_each<true>(r, c, g.M, g.N, false, [&](int i, int dr, int dc) {
+      const int y = min(r + dr, g.M - 1), x = min(c + dc, g.N - 1);
+      const long long at = x < dW ? (long long)y * dW + x : y;
+      ov[i] = (x < dW ? g.vW : g.vb)[at];
+      op[i] = (x < dW ? g.pW : g.pb)[at];
+    });
+  piece_each<false>(r, c, g.M, g.N, false, [&](int i, int dr, int dc) {
+    if ((c + dc < dW ? g.kfW : g.kfb) != nullptr)
+      *part(dr, dc, g.kfW, g.kfb) = v[i];
+    if (!fused) return;
+    const float n = momentum * ov[i] - lr * v[i];
+    *part(dr, dc, g.vW, g.vb) = n;
+    *part(dr, dc, g.pW, g.pb) = op[i] + n;
+  });
+}
+
+// One row per warp: its largest value, then (the row is in the L1 cache) the
+// scaled terms.  Bound by HBM: 4 bytes read and 4 written per element.
+__global__ void __launch_bounds__(256)
+pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
+                 const __grid_constant__ PackInline inl) {
+  const int lane = threadIdx.x & 31;
+  const int row_all = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row_all >= rows) return;
+  int f = 0;
+  if (inl.n > 0) {
+    for (int i = lane; i < inl.n; i += 32)
+      if (inl.j[i].row_begin <= row_all) f = i;
+  } else {
+    for (int i = lane; i < njobs; i += 32)
+      if (jobs[i].row_begin <= row_all) f = i;
+  }
+  f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
+  const PackRows job = inl.n > 0 ? inl.j[f] : jobs[f];
+  const int row = row_all - job.row_begin, cols = job.cols;
+  const int total = cols + (job.extra != nullptr ? 1 : 0);
+  const float* src = job.src + (long long)row * cols;
+  const bool vec =
+      (cols & 3) == 0 && (reinterpret_cast<uintptr_t>(job.src) & 15) == 0;
+  auto load = [&](int k) {
+    if (vec && k + 3 < cols) return *reinterpret_cast<const float4*>(src + k);
+    float x[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      x[e] = k + e < cols ? src[k + e]
+             : k + e < total ? job.extra[row] : 0.f;
+    return make_float4(x[0], x[1], x[2], x[3]);
+  };
+  unsigned top = 0;
+#pragma unroll 4
+  for (int k = 4 * lane; k < total; k += 128) {
+    const float4 x = load(k);
+    top = max(max(top, max(__float_as_uint(x.x) & 0x7fffffffu,
+                           __float_as_uint(x.y) & 0x7fffffffu)),
+              max(__float_as_uint(x.z) & 0x7fffffffu,
+                  __float_as_uint(x.w) & 0x7fffffffu));
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  float inverse;
+  const float s = half_scale(top, &inverse);
+  const int nkb = (total + 31) >> 5;
+  unsigned char* dst = job.dst + (long long)(row >> 7) * nkb * kChunk;
+  float sum = 0.f;
+#pragma unroll 4
+  for (int k = 4 * lane; k < 32 * nkb; k += 128) {
+    const float4 x = load(k);
+    const float y0 = s * x.x, y1 = s * x.y, y2 = s * x.z, y3 = s * x.w;
+    sum += y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3;
+    unsigned h0, h1, l0, l1;
+    split_half2(y0, y1, h0, l0);
+    split_half2(y2, y3, h1, l1);
+    unsigned char* p = dst + (long long)(k >> 5) * kChunk +
+                       sw128_chunk_off(row & 127, (k & 31) >> 3) +
+                       8 * ((k >> 2) & 1);
+    *reinterpret_cast<uint2*>(p) = make_uint2(h0, h1);
+    p = reinterpret_cast<unsigned char*>(reinterpret_cast<uintptr_t>(p) ^ 0x40);
+    *reinterpret_cast<uint2*>(p) = make_uint2(l0, l1);
+  }
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if (lane == 0) {
+    job.inv[row] = inverse;
+    // (a little up: the sum is rounded)
+    const float norm = 1.0001f * sqrtf(sum) * inverse;
+    if (job.norm != nullptr) job.norm[row] = norm;
+    if (job.peak != nullptr)
+      atomicMax(job.peak, __float_as_uint(norm) & 0x7fffffffu);
+  }
+}
+
+// MODE 0: the products of the inverse; 1, 2: first and second product of the
+// preconditioning, uncut as a sum of TF32 terms was, with half its MMAs.
+template <int MODE, int STAGES>
+__global__ void __launch_bounds__(KP_THREADS, STAGES == 3 ? 2 : 1)
 packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
-                   const __grid_constant__ TileInline inl) {
+                   const __grid_constant__ TileInline inl, float plr,
+                   float momentum) {
+  constexpr int kSegment = MODE == 0 ? KP_SEGMENT : 1 << 20;
   constexpr int TN = 128;
   extern __shared__ unsigned char kp_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(kp_smem_raw) + 1023) & ~(uintptr_t)1023);
   PackedControl* ctl =
-      reinterpret_cast<PackedControl*>(smem + KP_STAGES * KP_STAGE);
+      reinterpret_cast<PackedControl*>(smem + STAGES * KP_STAGE);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tile = blockIdx.x;
 
   if (warp == 0) {
     if (lane == 0) {
 #pragma unroll
-      for (int s = 0; s < KP_STAGES; ++s) {
+      for (int s = 0; s < STAGES; ++s) {
         mbar_init(&ctl->full[s], 1);
         mbar_init(&ctl->empty[s], 1);
       }
@@ -171,7 +365,7 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
   if (flags & G_KBEG_M0) kbeg = max(0, m0 - g.kbeg_off);
   if (flags & G_KBEG_N0) kbeg = max(kbeg, n0);
   const int nkb = max(0, (int)((g.K - kbeg + 31) >> 5));
-  const int kb0 = kbeg >> 5, seg0 = kb0 / KP_SEGMENT;
+  const int kb0 = kbeg >> 5, seg0 = kb0 / kSegment;
 
   if (warp == 0) {
     if (elect_one()) {
@@ -180,9 +374,9 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
       const unsigned char* b = g.cb + bj * g.cb_tile + k0;
       const unsigned bytes = share_ab ? kChunk : 2 * kChunk;
       for (int kb = 0; kb < nkb; ++kb, a += kChunk, b += kChunk) {
-        const int s = kb % KP_STAGES;
-        if (kb >= KP_STAGES &&
-            !mbar_wait_status(&ctl->empty[s], ((kb / KP_STAGES) - 1) & 1,
+        const int s = kb % STAGES;
+        if (kb >= STAGES &&
+            !mbar_wait_status(&ctl->empty[s], ((kb / STAGES) - 1) & 1,
                               &ctl->abort_flag, &g_packed_status))
           break;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
@@ -204,14 +398,14 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
       const unsigned long long adv_a = (ka ? 32 : 2048) >> 4;
       const unsigned long long adv_b = (kb_ ? 32 : 2048) >> 4;
       for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % KP_STAGES;
-        const int seg = (kb0 + kb) / KP_SEGMENT - seg0;
-        const bool fresh = kb == 0 || (kb0 + kb) % KP_SEGMENT == 0;
+        const int s = kb % STAGES;
+        const int seg = (kb0 + kb) / kSegment - seg0;
+        const bool fresh = kb == 0 || (kb0 + kb) % kSegment == 0;
         if (fresh && seg > 0 &&
             !mbar_wait_status(&ctl->drained, (seg - 1) & 1, &ctl->abort_flag,
                               &g_packed_status))
           break;
-        if (!mbar_wait_status(&ctl->full[s], (kb / KP_STAGES) & 1,
+        if (!mbar_wait_status(&ctl->full[s], (kb / STAGES) & 1,
                               &ctl->abort_flag, &g_packed_status))
           break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -227,7 +421,7 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
           tc_mma_half(tmem, a, b, idesc, acc);
         }
         tc_commit(&ctl->empty[s]);
-        if (kb + 1 == nkb || (kb0 + kb + 1) % KP_SEGMENT == 0)
+        if (kb + 1 == nkb || (kb0 + kb + 1) % kSegment == 0)
           tc_commit(&ctl->accum);
       }
     }
@@ -248,20 +442,22 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
                      (reinterpret_cast<uintptr_t>(g.C) & 7) == 0;
     const int lr = lane >> 2, lc = 2 * (lane & 3);
     bool ok = true;
-    const int nseg = nkb > 0 ? (kb0 + nkb - 1) / KP_SEGMENT - seg0 + 1 : 1;
+    const int nseg = nkb > 0 ? (kb0 + nkb - 1) / kSegment - seg0 + 1 : 1;
 #pragma unroll 1
     for (int it = 0; it < 4 * nseg; ++it) {
       const int u = it & 3, seg = it >> 2;
       if (it == 4) beta = 1.f;             // onto the segments before
       const int r0 = m0 + 32 * q + 16 * (u & 1);
       const int c0 = n0 + 32 * h + 64 * (u >> 1);
-      const bool live = r0 < rows && c0 < cols && !(lower && c0 > r0 + 15);
+      // (U has zeros behind its last row up to the end of the k-block)
+      const bool live = r0 < (MODE == 1 ? (rows + 31) & ~31 : rows) &&
+                        c0 < cols && !(lower && c0 > r0 + 15);
       const bool whole =
           r0 + 16 <= rows && c0 + 32 <= cols && (!lower || c0 + 31 <= r0);
       const int r = r0 + lr, c = c0 + lc;
       float* p = g.C + (long long)r * ldc + c;
       float old[16];
-      if (beta != 0.f && live) {
+      if (MODE == 0 && beta != 0.f && live) {
         if (whole && vec) {
 #pragma unroll
           for (int i = 0; i < 16; i += 2) {
@@ -271,8 +467,10 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
             old[i + 1] = x.y;
           }
         } else {
-          piece_each<false>(r, c, rows, cols, lower, [&](int i, int dr, int dc) {
-            old[i] = p[dr * ldc + dc];
+          // (past the edges the last row or column: no branch, all in flight)
+          piece_each<true>(r, c, rows, cols, lower, [&](int i, int dr, int dc) {
+            old[i] = g.C[(long long)min(r + dr, rows - 1) * ldc +
+                         min(c + dc, cols - 1)];
           });
         }
       }
@@ -303,6 +501,14 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
         if (lane == 0) mbar_arrive(&ctl->drained);
       }
       if (!live) continue;
+      if constexpr (MODE == 1) {
+        store_u(g, v, r, c);
+        continue;
+      }
+      if constexpr (MODE == 2) {
+        store_kf(g, v, r, c, whole && c0 + 32 <= g.dW, plr, momentum);
+        continue;
+      }
       if (un != nullptr) {
         // (rows and columns past the matrix: inside the vector's padding)
         const float s0 = un[r], s1 = un[r + 8];
@@ -357,6 +563,17 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
 }
 
 // ------------------------------------------------------------------ host side
+struct PackedVariant {
+  void (*kernel)(const GemmDesc*, int, const TileInline, float, float);
+  int stages;
+};
+// by mode; the preconditioning also with one CTA an SM
+static const PackedVariant kPackedVariants[] = {{packed_tile_kernel<0, 3>, 3},
+                                                {packed_tile_kernel<1, 3>, 3},
+                                                {packed_tile_kernel<2, 3>, 3},
+                                                {packed_tile_kernel<1, 6>, 6},
+                                                {packed_tile_kernel<2, 6>, 6}};
+
 int packed_prepare() {
   static std::mutex mu;
   static bool done[64] = {false};
@@ -365,9 +582,10 @@ int packed_prepare() {
   KFAC_REQUIRE(dev >= 0 && dev < 64, "device index %d unsupported", dev);
   std::lock_guard<std::mutex> lock(mu);
   if (!done[dev]) {
-    KFAC_CUDA(cudaFuncSetAttribute(packed_tile_kernel,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   KP_SMEM));
+    for (const PackedVariant& v : kPackedVariants)
+      KFAC_CUDA(cudaFuncSetAttribute(
+          v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+          packed_smem(v.stages)));
     done[dev] = true;
   }
   return KFAC_OK;
@@ -386,8 +604,9 @@ int packed_number_tiles(GemmDesc* descs, int n) {
   return total;
 }
 
-int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
-                  int ndesc, int total_tiles, cudaStream_t stream) {
+static int launch_mode(int mode, const GemmDesc* descs_dev,
+                       const GemmDesc* descs_host, int ndesc, int total_tiles,
+                       float lr, float momentum, cudaStream_t stream) {
   if (ndesc <= 0 || total_tiles <= 0) return KFAC_OK;
   const int rc = packed_prepare();
   if (rc != KFAC_OK) return rc;
@@ -397,9 +616,39 @@ int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
     inl.n = ndesc;
     std::copy(descs_host, descs_host + ndesc, inl.d);
   }
-  packed_tile_kernel<<<total_tiles, KP_THREADS, KP_SMEM, stream>>>(
-      descs_dev, ndesc, inl);
+  const bool one = mode > 0 && total_tiles <= sm_count();
+  const PackedVariant& v = kPackedVariants[one ? mode + 2 : mode];
+  v.kernel<<<total_tiles, KP_THREADS, packed_smem(v.stages), stream>>>(
+      descs_dev, ndesc, inl, lr, momentum);
   KFAC_LAUNCH_CHECK("packed_tile_kernel");
+  return KFAC_OK;
+}
+
+int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
+                  int ndesc, int total_tiles, cudaStream_t stream) {
+  return launch_mode(0, descs_dev, descs_host, ndesc, total_tiles, 0.f, 0.f,
+                     stream);
+}
+
+int launch_packed_precond(const GemmDesc* descs_dev, const GemmDesc* descs_host,
+                          int ndesc, int total_tiles, bool last, float lr,
+                          float momentum, cudaStream_t stream) {
+  return launch_mode(last ? 2 : 1, descs_dev, descs_host, ndesc, total_tiles, lr,
+                     momentum, stream);
+}
+
+int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,
+                     int njobs, int rows, cudaStream_t stream) {
+  if (njobs <= 0 || rows <= 0) return KFAC_OK;
+  PackInline inl;
+  inl.n = 0;
+  if (njobs <= 3 * TT_INLINE) {
+    inl.n = njobs;
+    std::copy(jobs_host, jobs_host + njobs, inl.j);
+  }
+  pack_rows_kernel<<<ceil_div(rows, 8), 256, 0, stream>>>(jobs_dev, njobs, rows,
+                                                          inl);
+  KFAC_LAUNCH_CHECK("pack_rows_kernel");
   return KFAC_OK;
 }
 

@@ -50,7 +50,8 @@ int64_t kfac_launch_count(void);
  * 1 (default, the product): tcgen05 tensor cores with fp32 operands split into
  * two terms, three MMAs per product, fp32 accumulation: two bf16 terms (16
  * significant bits) for the factor builds, two fp16 terms of scaled values (22
- * bits) for the inverse, two TF32 terms (22 bits) for the precondition products.  Relative Frobenius error of a factor
+ * bits) for the inverse and long precondition products, two TF32 terms (22 bits)
+ * for short ones.  Relative Frobenius error of a factor
  * stays below 1e-5 (bound of the reference comparison: 1e-4).
  * 0: fp32 FFMA tiles on the CUDA cores.  Not a supported product path: it is
  * the accuracy yardstick the parity tests run beside the tensor-core engine

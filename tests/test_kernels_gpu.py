@@ -778,6 +778,66 @@ def test_precondition_tile_variants(ops, shapes):
         assert rel(got, ref) < 2e-5     # TF32 pairs and fp32 sums: < 1e-5
 
 
+@pytest.mark.parametrize('dG,dW,bias,offset,magnitude', [
+    (512, 512, False, 0, 1.0), (33, 640, True, 0, 1e-18),
+    (1, 1024, False, 0, 1e12), (640, 5, True, 1, 1.0),
+    (300, 1023, True, 0, 1e12), (129, 897, False, 1, 1e-18),
+    (257, 1000, False, 2, 1.0), (1025, 255, True, 3, 1e-18)])
+def test_precondition_of_long_layers(ops, dG, dW, bias, offset, magnitude):
+    """Long enough for operands in chunks: cut tiles and k-blocks, the bias as an
+    appended column, parameters at odd addresses, gradient rows of different
+    sizes (dead units), with and without a copy of kf.  22-bit terms: 2^-21 per
+    operand and sums of up to 1025 + 256 terms, 1e-5 in all."""
+    rng = np.random.default_rng(dG * 7 + dW)
+    Gi, Ai, gW, gb = precond_case(rng, dG, dW, bias)
+    rows = (magnitude * 10.0 ** rng.integers(-4, 1, dG)).astype(np.float32)
+    gW = gW * rows[:, None]
+    gW[dG // 2] *= dG == 1
+    gb = None if gb is None else gb * rows
+
+    def place(a):      # `offset` floats behind a 16-byte boundary
+        buf = torch.zeros(a.size + 4, device='cuda')
+        t = buf[offset:offset + a.size].view(a.shape)
+        t.copy_(dev(a))
+        return t
+    pW = rng.standard_normal(gW.shape).astype(np.float32)
+    vW = (magnitude * rng.standard_normal(gW.shape)).astype(np.float32)
+    bias_t = [None] * 3 if gb is None else [
+        place(a) for a in (gb, np.ones_like(gb), np.zeros_like(gb))]
+    g = gW.astype(np.float64)
+    if gb is not None:
+        g = np.concatenate([g, gb.astype(np.float64)[:, None]], 1)
+    ref = Gi.astype(np.float64) @ g @ Ai.astype(np.float64)
+    for kf in (place(np.zeros_like(gW)), None):
+        kb = None if gb is None or kf is None else torch.empty_like(bias_t[0])
+        w2, v2 = place(pW), place(vW)
+        b2 = None if gb is None else bias_t[1].clone()
+        vb2 = None if gb is None else bias_t[2].clone()
+        ops.precondition([dev(Gi)], [dev(Ai)], [place(gW)], [bias_t[0]],
+                         [kf], [kb], [w2], [b2], [v2], [vb2], lr=0.5,
+                         momentum=0.9)
+        if kf is not None:
+            got = host(kf) if kb is None else np.concatenate(
+                [host(kf), host(kb)[:, None]], 1)
+            assert rel(got, ref) < 1e-5
+        want = 0.9 * vW.astype(np.float64) - 0.5 * ref[:, :dW]
+        assert rel(host(v2), want) < 1e-5
+        assert rel(host(w2), pW + want) < 1e-5
+        if gb is not None:
+            assert rel(host(vb2), -0.5 * ref[:, dW]) < 1e-5
+            assert rel(host(b2), 1.0 - 0.5 * ref[:, dW]) < 1e-5
+
+
+@pytest.mark.parametrize('value', [float('inf'), float('nan')])
+def test_precondition_of_a_non_finite_gradient_is_not_finite(ops, value):
+    rng = np.random.default_rng(3)
+    Gi, Ai, gW, _ = precond_case(rng, 130, 1030, False)
+    gW[17, 1000] = value
+    kf = torch.zeros(gW.shape, device='cuda')
+    ops.precondition([dev(Gi)], [dev(Ai)], [dev(gW)], [None], [kf], [None])
+    assert not np.isfinite(host(kf)).any()
+
+
 @pytest.mark.parametrize('d', [1, 31, 127, 129, 257, 385, 513, 770, 1025])
 def test_inverse_around_block_sizes(ops, d):
     """Sides around the diagonal block, the panel and the row pitch."""
