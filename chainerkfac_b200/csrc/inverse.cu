@@ -219,6 +219,7 @@ constexpr int kLookCols = 2 * DB;               // tensor-memory columns
 static __device__ int g_diag_status = 0;
 
 struct LookControl {
+  unsigned long long full[4];  // a k-block of the first product is stored
   unsigned long long done[2];  // all MMAs of the first, second product
   unsigned tmem_base;
   volatile int abort_flag;
@@ -290,6 +291,8 @@ __device__ __forceinline__ void diag_load_wait() {
 // Barriers and tensor memory of the look-ahead; needs nothing of the matrix.
 __device__ __forceinline__ void look_begin(LookControl* ctl) {
   if (threadIdx.x == 32) {
+#pragma unroll
+    for (int kb = 0; kb < 4; ++kb) mbar_init(&ctl->full[kb], DT / 32);
     mbar_init(&ctl->done[0], 1);
     mbar_init(&ctl->done[1], 1);
     ctl->abort_flag = 0;
@@ -348,6 +351,7 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
       }
     }
   }
+  look_begin(ctl);
   // W_kk into S (the update is subtracted from it at the end)
   diag_load(mi.W + (long long)o * ld + o, ld, bs, vec, S);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -357,7 +361,22 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
   const unsigned sbase = smem_u32(stage);
   bool ok = true;
 
-  // ---- L' = A' X_pp^T, a block of 32 k at a time behind its MMAs
+  // ---- L' = A' X_pp^T: the MMAs of a block of 32 k as soon as all warps have
+  // stored it, issued between the first warp's own stores
+  auto issue = [&](int kb) {
+    const bool go = mbar_wait_status(&ctl->full[kb], 0, &ctl->abort_flag,
+                                     &g_diag_status);
+    if (__all_sync(0xffffffffu, go) && elect_one()) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned ta = sbase + 2 * kb * kLookTile;
+      // columns below 32 kb of L' get nothing from this block of k
+      look_mma_block(tmem + 32 * kb, ta,
+                     ta + kLookTile + (unsigned)(32 * kb) * 128, DB - 32 * kb,
+                     kb == 0);
+      if (kb == 3) tc_commit(&ctl->done[0]);
+    }
+    __syncwarp();
+  };
 #pragma unroll
   for (int kb = 0; kb < 4; ++kb) {
     const unsigned ta = sbase + 2 * kb * kLookTile, tx = ta + kLookTile;
@@ -368,15 +387,11 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
       if (row >= 32 * kb) look_store4(tx, row, word, vx[kb][j], kScaleX);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (warp == 0 && elect_one()) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // columns below 32 kb of L' get nothing from this block of k
-      look_mma_block(tmem + 32 * kb, ta, tx + (unsigned)(32 * kb) * 128,
-                     DB - 32 * kb, kb == 0);
-      if (kb == 3) tc_commit(&ctl->done[0]);
-    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&ctl->full[kb]);
+    if (warp == 0 && kb > 0) issue(kb - 1);
   }
+  if (warp == 0) issue(3);
   ok = mbar_wait_status(&ctl->done[0], 0, &ctl->abort_flag, &g_diag_status);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
@@ -818,7 +833,6 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
   unsigned char* stage = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(dsm + DB * DLD) + 1023) & ~(uintptr_t)1023);
   LookControl* ctl = reinterpret_cast<LookControl*>(stage + kLookBytes);
-  if (LOOK) look_begin(ctl);
   const MatInfo mi = mats[blockIdx.x];
   const int id = mi.id;
   const int o = step * DB;
@@ -906,57 +920,68 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
   // 16-byte word per lane) into four contiguous row pieces.  The part above
   // the diagonal sub-blocks was zeroed when the plan was made.
   float* Xd = mi.X + (long long)o * ld + o;
+  if (!vec) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = 4 * warp + 64 * h, bi = r >> 5;
+      if (r >= bs) break;
+      for (int u = 0; u <= bi; ++u) {
+        const float4 v = *reinterpret_cast<const float4*>(
+            u == bi ? &sm.XD[u][lane * SLP + (r & (SB - 1))]
+                    : &sm.S[(SB * u + lane) * DLD + r]);
+        const int c = SB * u + lane;
+        if (c >= bs) continue;
+        float* dst = Xd + r * ld + c;
+        dst[0] = v.x;
+        if (r + 1 < bs) dst[ld] = v.y;
+        if (r + 2 < bs) dst[2 * ld] = v.z;
+        if (r + 3 < bs) dst[3 * ld] = v.w;
+      }
+    }
+    return;
+  }
   // (from X and d: two more pointers across the chain cost registers that it
   // does not have)
   const long long ptile =
       (long long)((mi.d + DB - 1) / DB) * (DB / 32) * kChunk;
   unsigned char* const px = reinterpret_cast<unsigned char*>(mi.X) +
-                            matrix_bytes(mi.d);
+                            matrix_bytes(mi.d) + step * ptile;
+  // a warp takes 16 rows x 32 columns, a lane a 4 x 4 block: four words along the
+  // rows of X^T, turned by naming registers, so that X and its fp16 terms are
+  // stored in words of four columns.  Lanes are laid out so that a quarter
+  // warp's loads fall into different banks.  (2.2 us with a column of four rows
+  // a lane, 2.0 us now; the rest is what one SM can store.)
+  const int nb = (bs + SB - 1) / SB;
+  for (int item = warp; item < nb * (nb + 1); item += DT / 32) {
+    int bi = 0, u = item >> 1;
+    while (u > bi) u -= ++bi;
+    const int c = 4 * (lane >> 2), r = 16 * (item & 1) + 4 * (lane & 3);
+    float x[4][4];              // [column][row]
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int r = 4 * warp + 64 * h, bi = r >> 5;
-    if (r >= bs) break;
-    float4 v[4];
+    for (int e = 0; e < 4; ++e) {
+      const float4 v = *reinterpret_cast<const float4*>(
+          u == bi ? &sm.XD[u][(c + e) * SLP + r]
+                  : &sm.S[(SB * u + c + e) * DLD + SB * bi + r]);
+      x[e][0] = v.x; x[e][1] = v.y; x[e][2] = v.z; x[e][3] = v.w;
+    }
+    const int gc = SB * u + c;
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (u <= bi)
-        v[u] = *reinterpret_cast<const float4*>(
-            u == bi ? &sm.XD[u][lane * SLP + (r & (SB - 1))]
-                    : &sm.S[(SB * u + lane) * DLD + r]);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int c = SB * u + lane;
-      if (u > bi) continue;
-      if (c < bs) {
-        float* dst = Xd + r * ld + c;
-        dst[0] = v[u].x;
-        if (r + 1 < bs) dst[ld] = v[u].y;
-        if (r + 2 < bs) dst[2 * ld] = v[u].z;
-        if (r + 3 < bs) dst[3 * ld] = v[u].w;
-      }
-      if (pack) {
-        // the same as fp16 terms: an even lane takes rows r, r + 1 of its and
-        // the next column, an odd one rows r + 2, r + 3 (columns past bs are
-        // zero above the diagonal; their chunks exist)
-        const bool odd = lane & 1;
-        const float p0 = __shfl_xor_sync(0xffffffffu, odd ? v[u].x : v[u].z, 1);
-        const float p1 = __shfl_xor_sync(0xffffffffu, odd ? v[u].y : v[u].w, 1);
-        const int k = r + (odd ? 2 : 0);
-        unsigned char* q = px + step * ptile +
-                           (long long)((o + k) >> 5) * kChunk +
-                           (u >> 1) * 8192 + 4 * ((c & 7) >> 1);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          if (k + e >= bs) continue;
-          unsigned hi, lo;
-          const float x0 = e == 0 ? (odd ? p0 : v[u].x) : (odd ? p1 : v[u].y);
-          const float x1 = e == 0 ? (odd ? v[u].z : p0) : (odd ? v[u].w : p1);
-          split_half2(kScaleX * x0, kScaleX * x1, hi, lo);
-          unsigned char* w = q + sw128_chunk_off((k + e) & 31, (c & 63) >> 3);
-          *reinterpret_cast<unsigned*>(w) = hi;
-          *reinterpret_cast<unsigned*>(w + 4096) = lo;
-        }
-      }
+    for (int e = 0; e < 4; ++e) {
+      const int gr = SB * bi + r + e;
+      if (gr >= bs) continue;
+      // (columns past bs are zeros above the diagonal, inside the row pitch)
+      *reinterpret_cast<float4*>(Xd + gr * ld + gc) =
+          make_float4(x[0][e], x[1][e], x[2][e], x[3][e]);
+      if (!pack) continue;
+      unsigned h0, h1, l0, l1;
+      split_half2(kScaleX * x[0][e], kScaleX * x[1][e], h0, l0);
+      split_half2(kScaleX * x[2][e], kScaleX * x[3][e], h1, l1);
+      unsigned char* q = px + (long long)((o + gr) >> 5) * kChunk +
+                         (gc >> 6) * 8192 +
+                         sw128_chunk_off(gr & 31, (gc & 63) >> 3) +
+                         8 * ((gc >> 2) & 1);
+      *reinterpret_cast<uint2*>(q) = make_uint2(h0, h1);
+      *reinterpret_cast<uint2*>(q + 4096) = make_uint2(l0, l1);
     }
   }
 }
