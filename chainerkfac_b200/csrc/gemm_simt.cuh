@@ -287,11 +287,10 @@ struct GemmDesc {
   int pack_kind;
   const float* unscale;    // if set, C(m, n) = .. + unscale[m] unscale[n] A B
   // preconditioning in chunks: reciprocals of the scales of A^T's rows and B's
-  // columns; norms of A_inv's rows and the largest norm of a gradient row (float
-  // bits), which bound the first product
+  // columns; norms of A_inv's rows and of the gradient's M rows, which bound the
+  // first product
   const float *rs, *cs;
-  const float* norm;
-  const unsigned* peak;
+  const float *norm, *norm_g;
 };
 
 // Rows of a matrix (and an appended column) as K-major chunks, each scaled by a
@@ -302,7 +301,6 @@ struct PackRows {
   unsigned char* dst;
   float* inv;              // reciprocal of a row's scale
   float* norm;             // 2-norm of a row, NULL: not wanted
-  unsigned* peak;          // largest of the norms (atomic maximum of the bits)
   int rows, cols;
   int row_begin;           // first row in the launch
   int pad_;

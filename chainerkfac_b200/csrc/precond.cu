@@ -14,7 +14,7 @@ static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // One layer's operands in chunks and their rows' scales, offsets in bytes.
 struct ChunkLayout {
   size_t G, A, g, U;             // G_inv, A_inv, gradient, grad * A_inv^T
-  size_t inv_G, inv_A, inv_g, norm_A;
+  size_t inv_G, inv_A, inv_g, norm_A, norm_g;
   size_t total;
 };
 
@@ -37,17 +37,18 @@ static ChunkLayout chunk_layout(int dG, int dA) {
   c.inv_A = take(dA * sizeof(float));
   c.inv_g = take(dG * sizeof(float));
   c.norm_A = take(dA * sizeof(float));
+  c.norm_g = take(dG * sizeof(float));
   c.total = at;
   return c;
 }
 
-// Whether a call goes through chunks: it costs a launch and a half more (27 us
-// against 17 at the smallest sizes), a k-block 0.4 us instead of 0.75, or of 1.05
-// where the tile kernel cannot load 16-byte words.  The longest layer decides, by
-// its k-blocks in both products.  us by one launch kind and the other: 256 x 256
-// (16 k-blocks) 27 33, 128 x 512 (20) 30 35, 512 x 512 (32) 41 39, 512 x 2048 (80)
-// 78 61, 512 x 4608 165 138; with odd sides 53 x 334 (13) 30 33, 211 x 130 (12)
-// 33 33, 301 x 785 (35) 64 51, 1000 x 10 (33) 49 32, 1000 x 1001 102 62.
+// Whether a call goes through chunks: it costs a launch more, a k-block 0.4 us
+// instead of 0.75, or of 1.05 where the tile kernel cannot load 16-byte words.
+// The longest layer decides, by its k-blocks in both products.  us in tiles and
+// in chunks: 512 x 512 (32 k-blocks) 41 33, 512 x 4608 165 132; with odd sides 301
+// x 785 (35) 64 47, 1000 x 10 (33) 49 30, 1000 x 1001 102 58; and below the line,
+// 4 us for a memset included that the chunks no longer need, 256 x 256 (16) 27 33,
+// 128 x 512 (20) 30 35, 53 x 334 (13) 30 33, 211 x 130 (12) 33 33.
 static bool chunks_pay(int count, const int* dG, const int* dW,
                        const std::vector<int>& hb) {
   for (int i = 0; i < count; ++i) {
@@ -67,17 +68,15 @@ static int precondition_chunks(
     float* const* kf_b, float* const* param_W, float* const* param_b,
     float* const* mom_W, float* const* mom_b, float lr, float momentum, char* ws,
     cudaStream_t st) {
-  // tables and peaks, in front of the layers' chunks
+  // tables, in front of the layers' chunks
   const size_t jobs_at = align256(2 * (size_t)count * sizeof(GemmDesc));
-  const size_t peaks_at =
+  const size_t tables =
       jobs_at + align256(3 * (size_t)count * sizeof(PackRows));
-  const size_t tables = peaks_at + align256((size_t)count * sizeof(unsigned));
   std::vector<char> host(tables, 0);
   GemmDesc* descs = reinterpret_cast<GemmDesc*>(host.data());
   PackRows* jobs = reinterpret_cast<PackRows*>(host.data() + jobs_at);
   char* const base = ws;
   const GemmDesc* descs_dev = reinterpret_cast<GemmDesc*>(base);
-  unsigned* peaks = reinterpret_cast<unsigned*>(base + peaks_at);
   ws += tables;
   int njobs = 0;
   int rows = 0;
@@ -92,18 +91,18 @@ static int precondition_chunks(
     const ChunkLayout c = chunk_layout(dg, da);
     const long long nkA = (da + 31) / 32, nkG = (dg + 31) / 32;
     auto job = [&](const float* src, const float* extra, size_t dst, size_t inv,
-                   float* norm, unsigned* peak, int nrows, int cols) {
+                   float* norm, int nrows, int cols) {
       PackRows j = {};
       j.src = src; j.extra = extra; j.dst = at(ws, dst); j.inv = vec(ws, inv);
-      j.norm = norm; j.peak = peak; j.rows = nrows; j.cols = cols;
+      j.norm = norm; j.rows = nrows; j.cols = cols;
       j.row_begin = rows;
       rows += nrows;
       jobs[njobs++] = j;
     };
-    job(A_inv[i], nullptr, c.A, c.inv_A, vec(ws, c.norm_A), nullptr, da, da);
-    job(G_inv[i], nullptr, c.G, c.inv_G, nullptr, nullptr, dg, dg);
-    job(grad_W[i], hb[i] ? grad_b[i] : nullptr, c.g, c.inv_g, nullptr,
-        peaks + i, dg, dw);
+    job(A_inv[i], nullptr, c.A, c.inv_A, vec(ws, c.norm_A), da, da);
+    job(G_inv[i], nullptr, c.G, c.inv_G, nullptr, dg, dg);
+    job(grad_W[i], hb[i] ? grad_b[i] : nullptr, c.g, c.inv_g,
+        vec(ws, c.norm_g), dg, dw);
     // U = grad * A_inv^T
     GemmDesc& u = descs[i];
     u = GemmDesc();
@@ -114,7 +113,7 @@ static int precondition_chunks(
     u.cb = at(ws, c.A); u.cb_tile = nkA * kChunk;
     u.pack = at(ws, c.U); u.pack_tile = nkG * kChunk;
     u.rs = vec(ws, c.inv_g); u.cs = vec(ws, c.inv_A);
-    u.norm = vec(ws, c.norm_A); u.peak = peaks + i;
+    u.norm = vec(ws, c.norm_A); u.norm_g = vec(ws, c.norm_g);
     // kf = G_inv * U, split and (optionally) applied
     GemmDesc& h = descs[count + i];
     h = GemmDesc();
@@ -124,7 +123,7 @@ static int precondition_chunks(
     h.ca = at(ws, c.G); h.ca_tile = nkG * kChunk;
     h.cb = u.pack; h.cb_tile = u.pack_tile;
     h.rs = vec(ws, c.inv_G);
-    h.norm = u.norm; h.peak = u.peak;
+    h.norm = u.norm; h.norm_g = u.norm_g;
     const bool fused = param_W && param_W[i];
     h.kfW = kf_W ? kf_W[i] : nullptr;
     h.kfb = (hb[i] && kf_b) ? kf_b[i] : nullptr;
@@ -141,8 +140,6 @@ static int precondition_chunks(
   if (count > kTileInline)
     KFAC_CUDA(cudaMemcpyAsync(base, host.data(), tables,
                               cudaMemcpyHostToDevice, st));
-  else
-    KFAC_CUDA(cudaMemsetAsync(peaks, 0, count * sizeof(unsigned), st));
   int rc = launch_pack_rows(reinterpret_cast<PackRows*>(base + jobs_at), jobs,
                             njobs, rows, st);
   if (rc == KFAC_OK)
@@ -159,8 +156,7 @@ extern "C" size_t kfac_precond_workspace_bytes(int count, const int* dG,
                                                const int* has_bias) {
   if (count <= 0 || !dG || !dW) return 0;
   size_t total = align256(2 * (size_t)count * sizeof(GemmDesc));
-  size_t chunks = total + align256(3 * (size_t)count * sizeof(PackRows)) +
-                  align256((size_t)count * sizeof(unsigned));
+  size_t chunks = total + align256(3 * (size_t)count * sizeof(PackRows));
   for (int i = 0; i < count; ++i) {
     size_t dA = (size_t)dW[i] + ((has_bias && has_bias[i]) ? 1 : 0);
     total += align256((size_t)dG[i] * dA * sizeof(float));

@@ -112,15 +112,24 @@ __device__ __forceinline__ void piece_each(int r, int c, int rows, int cols,
 // Scale of a column of U = grad A_inv^T as an operand of the second product:
 // its entries are at most the largest norm of a gradient row times the norm of
 // the column's row of A_inv.
-__device__ __forceinline__ float u_scale(const unsigned* peak, float norm,
+__device__ __forceinline__ float u_scale(float peak, float norm,
                                          float* inverse) {
-  return half_scale(__float_as_uint(__uint_as_float(*peak) * norm), inverse);
+  return half_scale(__float_as_uint(peak * norm) & 0x7fffffffu, inverse);
+}
+
+// Largest norm of a gradient row, by a warp (as bits: NaN stays the largest).
+__device__ __forceinline__ float peak_norm(const GemmDesc& g, int lane) {
+  unsigned m = 0;
+#pragma unroll 4
+  for (int i = lane; i < g.M; i += 32)
+    m = max(m, __float_as_uint(g.norm_g[i]) & 0x7fffffffu);
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, m));
 }
 
 // First product of the preconditioning: a 16 x 32 piece of U into chunks, rows as
 // k (zeros up to the end of the last k-block).
 __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
-                                        int r, int c) {
+                                        int r, int c, float peak) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int gr = r + 8 * h;
@@ -134,8 +143,8 @@ __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
       const float x0 = in ? v[4 * j + 2 * h] * s0 * g.cs[k0] : 0.f;
       const float x1 = in ? v[4 * j + 2 * h + 1] * s0 * g.cs[k1] : 0.f;
       unsigned hi, lo;
-      split_half2(x0 * u_scale(g.peak, g.norm[k0], &inverse),
-                  x1 * u_scale(g.peak, g.norm[k1], &inverse), hi, lo);
+      split_half2(x0 * u_scale(peak, g.norm[k0], &inverse),
+                  x1 * u_scale(peak, g.norm[k1], &inverse), hi, lo);
       unsigned char* p = g.pack + (long long)(gc >> 7) * g.pack_tile +
                          (long long)(gr >> 5) * kChunk +
                          ((gc >> 6) & 1) * 8192 +
@@ -149,13 +158,13 @@ __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
 // Second product: a 16 x 32 piece of kf to the weight and bias parts, and the
 // momentum update where the layer has it fused.
 __device__ __forceinline__ void store_kf(const GemmDesc& g, float v[16], int r,
-                                         int c, bool whole, float lr,
-                                         float momentum) {
+                                         int c, bool whole, float peak,
+                                         float lr, float momentum) {
   const float s0 = g.rs[min(r, g.M - 1)], s1 = g.rs[min(r + 8, g.M - 1)];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     float inverse;
-    u_scale(g.peak, g.norm[min(c + 8 * (j >> 1) + (j & 1), g.N - 1)], &inverse);
+    u_scale(peak, g.norm[min(c + 8 * (j >> 1) + (j & 1), g.N - 1)], &inverse);
     const int i = 4 * (j >> 1) + (j & 1);
     v[i] = v[i] * s0 * inverse;
     v[i + 2] = v[i + 2] * s1 * inverse;
@@ -282,8 +291,6 @@ pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
     // (a little up: the sum is rounded)
     const float norm = 1.0001f * sqrtf(sum) * inverse;
     if (job.norm != nullptr) job.norm[row] = norm;
-    if (job.peak != nullptr)
-      atomicMax(job.peak, __float_as_uint(norm) & 0x7fffffffu);
   }
 }
 
@@ -441,6 +448,7 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
     const bool vec = (ldc & 1) == 0 &&
                      (reinterpret_cast<uintptr_t>(g.C) & 7) == 0;
     const int lr = lane >> 2, lc = 2 * (lane & 3);
+    const float peak = MODE == 0 ? 0.f : peak_norm(g, lane);
     bool ok = true;
     const int nseg = nkb > 0 ? (kb0 + nkb - 1) / kSegment - seg0 + 1 : 1;
 #pragma unroll 1
@@ -502,11 +510,11 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
       }
       if (!live) continue;
       if constexpr (MODE == 1) {
-        store_u(g, v, r, c);
+        store_u(g, v, r, c, peak);
         continue;
       }
       if constexpr (MODE == 2) {
-        store_kf(g, v, r, c, whole && c0 + 32 <= g.dW, plr, momentum);
+        store_kf(g, v, r, c, whole && c0 + 32 <= g.dW, peak, plr, momentum);
         continue;
       }
       if (un != nullptr) {
