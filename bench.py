@@ -146,8 +146,8 @@ def algorithmic_bytes(layers, prebuilt=False, lowrank=None):
 
 def measure_tf32_peak(device):
     """Dense TF32 matmul throughput (8192^3, best of 10), measured the way the
-    bf16 figure of MEASURED_PEAKS.json was: the fp32 data of this path can at
-    best run at this rate (a third of it with the split-TF32 scheme)."""
+    bf16 figure of MEASURED_PEAKS.json was: what fp32 data runs at without a
+    split (for comparison)."""
     import torch
     old = torch.backends.cuda.matmul.allow_tf32
     torch.backends.cuda.matmul.allow_tf32 = True
@@ -900,11 +900,12 @@ def time_alone(torch, fn, reps):
 STAGE_KERNELS = {
     'factor': 'gram_kernel + direct_kernel + tc_pair_kernel (grouped launches '
               'over all factors, plus staging and the split reductions)',
-    'inverse': 'tc_tile_kernel + chol_diag_kernel (batched blocked Cholesky, '
+    'inverse': 'packed_tile_kernel + tc_tile_kernel + chol_diag_kernel '
+               '(batched blocked Cholesky, '
                'triangular inverse and symmetric product of every factor, '
                'three size classes on three streams)',
-    'precondition': 'tc_tile_kernel (two grouped launches over all layers, '
-                    'update fused)'}
+    'precondition': 'pack_rows_kernel + packed_tile_kernel (three grouped '
+                    'launches over all layers, update fused)'}
 
 
 def run_ours(args):
@@ -1125,10 +1126,11 @@ def run_ours(args):
                                'MEASURED_PEAKS.json (stage timed alone)'
                                % peaks['source'],
                 # fp32 operands are split into two terms and every product
-                # costs three MMAs: bf16 terms for the factors, TF32 terms
-                # for the inverse and precondition products
+                # costs three MMAs at the 16-bit rate: bf16 terms for the
+                # factors, fp16 terms for the inverse and the preconditioning
+                # of long layers
                 'frac_of_split_ceiling': achieved / (
-                    (peaks['tflops_burst'] if dom == 'factor' else tf32) / 3.0),
+                    peaks['tflops_burst'] / 3.0),
                 'tf32_tflops_measured_here': tf32,
                 'step_tflops': (float(sum(flops.values()) * acc /
                                       (ms_per_step * 1e-3) / 1e12)

@@ -1,9 +1,13 @@
-// Tensor-core tile engine of the inverse and precondition products for
-// sm_100a: C = alpha A B + beta C over many problems in one launch (GemmDesc),
-// tcgen05.mma (kind::tf32) with fp32 accumulators in tensor memory, fp32
-// operands split into two TF32 terms (x = hi + lo with hi rounded to nearest,
-// C += hi*hi + hi*lo + lo*hi) so that results keep near-fp32 accuracy (a
-// single TF32 pass misses the 1e-4 bound on large factors).
+// Tensor-core tile engine for sm_100a: C = alpha A B + beta C over many problems
+// in one launch (GemmDesc), operands fp32 in memory, split by every tile into two
+// terms, x = hi + lo, C += hi*hi + hi*lo + lo*hi in fp32 accumulators in tensor
+// memory (a single TF32 pass misses the 1e-4 bound on large factors).
+//
+// Two kinds of terms: fp16 (tcgen05.mma kind::f16), where the values' range is
+// known - the short products of the inverse that make L and X, see inverse.cu -
+// and TF32 (kind::tf32) for the preconditioning of short layers and for the
+// refinement.  The long products read operands that were split once
+// (tc_packed.cu).
 //
 // One CTA owns a 128 x TN tile.  Producer warps load the operands from global
 // memory with 16-byte loads, one to three 32-k blocks ahead in registers, split them
@@ -13,9 +17,9 @@
 // global rows (and, for symmetric outputs, mirrored rows straight from the
 // registers, where a column of a piece is contiguous).
 //
-// Bound: the long products by the MMAs (three per product) and, next to them,
-// the shared-memory traffic of their operands; the many short ones (K = 128
-// inside a Cholesky panel) by latency: descriptor fetch, one trip to L2 per
+// Bound: long products by the loads and stores of their operands, not by the
+// MMAs (a 128 x 256 x 32 block 1600 ns with TF32 terms, the MMAs of it 810); the
+// many short ones (K = 128 inside a Cholesky panel) by latency: descriptor fetch, one trip to L2 per
 // register block, the epilogue's trip for C.  Hence the descriptors of small
 // launches travel as kernel arguments, C is prefetched before the accumulator
 // is waited for, and TN = 128 (half the work per CTA, twice the CTAs) is used
