@@ -286,22 +286,26 @@ struct GemmDesc {
   float pack_scale;
   int pack_kind;
   const float* unscale;    // if set, C(m, n) = .. + unscale[m] unscale[n] A B
-  // preconditioning in chunks: reciprocals of the scales of A^T's rows and B's
-  // columns; norms of A_inv's rows and of the gradient's M rows, which bound the
-  // first product
+  // preconditioning in chunks, see PackRows: factors of the first product's rows
+  // and columns, exponents of the second's
   const float *rs, *cs;
-  const float *norm, *norm_g;
+  const short *re, *ce;
 };
 
 // Rows of a matrix (and an appended column) as K-major chunks, each scaled by a
-// power of two of its own.
+// power of two of its own, the columns before that by others.  A row of scale 2^s
+// whose values then have the 2-norm 2^n or less (n as small as a whole number
+// can be) leaves n - s, and 2^-n times `gain` as the factor that brings its
+// products with rows treated alike to at most `gain`; without `fit` it leaves -s.
 struct PackRows {
   const float* src;
   const float* extra;      // appended column, NULL: none
+  const short* col;        // exponents of the columns' factors, NULL: none
   unsigned char* dst;
-  float* inv;              // reciprocal of a row's scale
-  float* norm;             // 2-norm of a row, NULL: not wanted
-  int rows, cols;
+  short* exp;
+  float* fit;
+  float gain;
+  int cols;
   int row_begin;           // first row in the launch
   int pad_;
 };
@@ -342,6 +346,7 @@ int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
 int packed_status_read(int* out);
 // Preconditioning on chunks: rows into chunks, then the product whose result is
 // chunks again (`last` false) or the preconditioned gradient.
+constexpr int kChunkExp = 14;    // scaled values of a row are below 2^15
 int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,
                      int njobs, int rows, cudaStream_t stream);
 int launch_packed_precond(const GemmDesc* descs_dev, const GemmDesc* descs_host,

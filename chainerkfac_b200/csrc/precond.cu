@@ -14,7 +14,8 @@ static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // One layer's operands in chunks and their rows' scales, offsets in bytes.
 struct ChunkLayout {
   size_t G, A, g, U;             // G_inv, A_inv, gradient, grad * A_inv^T
-  size_t inv_G, inv_A, inv_g, norm_A, norm_g;
+  size_t exp_G, exp_A, exp_g;    // exponents of rows
+  size_t fit_A, fit_g;           // factors of U's columns and rows
   size_t total;
 };
 
@@ -33,11 +34,12 @@ static ChunkLayout chunk_layout(int dG, int dA) {
   c.A = take(chunks(dA, dA));
   c.g = take(chunks(dG, dA));
   c.U = take(chunks(dA, dG));
-  c.inv_G = take(dG * sizeof(float));
-  c.inv_A = take(dA * sizeof(float));
-  c.inv_g = take(dG * sizeof(float));
-  c.norm_A = take(dA * sizeof(float));
-  c.norm_g = take(dG * sizeof(float));
+  // (read in fours up to the end of a k-block)
+  c.exp_G = take((dG + 31) * sizeof(short));
+  c.exp_A = take((dA + 31) * sizeof(short));
+  c.exp_g = take((dG + 31) * sizeof(short));
+  c.fit_A = take(dA * sizeof(float));
+  c.fit_g = take(dG * sizeof(float));
   c.total = at;
   return c;
 }
@@ -60,6 +62,8 @@ static bool chunks_pay(int count, const int* dG, const int* dW,
   return false;
 }
 
+constexpr float kGainU = 32768.f;
+
 // kfac_precondition through chunks.
 static int precondition_chunks(
     int count, const int* dG, const int* dW, const std::vector<int>& hb,
@@ -78,31 +82,41 @@ static int precondition_chunks(
   char* const base = ws;
   const GemmDesc* descs_dev = reinterpret_cast<GemmDesc*>(base);
   ws += tables;
-  int njobs = 0;
-  int rows = 0;
+  int rows = 0, rows_G = 0;
   auto at = [](char* base, size_t off) {
     return reinterpret_cast<unsigned char*>(base + off);
   };
   auto vec = [](char* base, size_t off) {
     return reinterpret_cast<float*>(base + off);
   };
+  auto exps = [](char* base, size_t off) {
+    return reinterpret_cast<short*>(base + off);
+  };
   for (int i = 0; i < count; ++i) {
     const int dg = dG[i], dw = dW[i], da = dw + hb[i];
     const ChunkLayout c = chunk_layout(dg, da);
     const long long nkA = (da + 31) / 32, nkG = (dg + 31) / 32;
-    auto job = [&](const float* src, const float* extra, size_t dst, size_t inv,
-                   float* norm, int nrows, int cols) {
-      PackRows j = {};
-      j.src = src; j.extra = extra; j.dst = at(ws, dst); j.inv = vec(ws, inv);
-      j.norm = norm; j.rows = nrows; j.cols = cols;
-      j.row_begin = rows;
-      rows += nrows;
-      jobs[njobs++] = j;
+    // Rows of the gradient and of A_inv, then (in a launch of its own) those of
+    // G_inv, whose columns take what U's rows are divided by: rows of the
+    // gradient of any scale, nearly dead units among them, are held alike.
+    // U's terms stay below 2^15 and take that out of kf again.
+    auto job = [&](PackRows& j, const float* src, const float* extra,
+                   size_t dst, int cols, int nrows, int& begin) {
+      j = PackRows();
+      j.src = src; j.extra = extra; j.dst = at(ws, dst);
+      j.cols = cols;
+      j.row_begin = begin;
+      begin += nrows;
     };
-    job(A_inv[i], nullptr, c.A, c.inv_A, vec(ws, c.norm_A), da, da);
-    job(G_inv[i], nullptr, c.G, c.inv_G, nullptr, dg, dg);
-    job(grad_W[i], hb[i] ? grad_b[i] : nullptr, c.g, c.inv_g,
-        vec(ws, c.norm_g), dg, dw);
+    PackRows& ja = jobs[2 * i];
+    job(ja, A_inv[i], nullptr, c.A, da, da, rows);
+    ja.exp = exps(ws, c.exp_A); ja.fit = vec(ws, c.fit_A); ja.gain = kGainU;
+    PackRows& jg = jobs[2 * i + 1];
+    job(jg, grad_W[i], hb[i] ? grad_b[i] : nullptr, c.g, dw, dg, rows);
+    jg.exp = exps(ws, c.exp_g); jg.fit = vec(ws, c.fit_g); jg.gain = 1.f;
+    PackRows& jG = jobs[2 * count + i];
+    job(jG, G_inv[i], nullptr, c.G, dg, dg, rows_G);
+    jG.exp = exps(ws, c.exp_G); jG.col = jg.exp;
     // U = grad * A_inv^T
     GemmDesc& u = descs[i];
     u = GemmDesc();
@@ -112,18 +126,16 @@ static int precondition_chunks(
     u.ca = at(ws, c.g); u.ca_tile = nkA * kChunk;
     u.cb = at(ws, c.A); u.cb_tile = nkA * kChunk;
     u.pack = at(ws, c.U); u.pack_tile = nkG * kChunk;
-    u.rs = vec(ws, c.inv_g); u.cs = vec(ws, c.inv_A);
-    u.norm = vec(ws, c.norm_A); u.norm_g = vec(ws, c.norm_g);
+    u.rs = jg.fit; u.cs = ja.fit;
     // kf = G_inv * U, split and (optionally) applied
     GemmDesc& h = descs[count + i];
     h = GemmDesc();
     h.A.kfast = 1;
     h.M = dg; h.N = da; h.K = dg;
-    h.alpha = 1.f;
     h.ca = at(ws, c.G); h.ca_tile = nkG * kChunk;
     h.cb = u.pack; h.cb_tile = u.pack_tile;
-    h.rs = vec(ws, c.inv_G);
-    h.norm = u.norm; h.norm_g = u.norm_g;
+    h.alpha = 1.f / kGainU;
+    h.re = jG.exp; h.ce = ja.exp;
     const bool fused = param_W && param_W[i];
     h.kfW = kf_W ? kf_W[i] : nullptr;
     h.kfb = (hb[i] && kf_b) ? kf_b[i] : nullptr;
@@ -140,8 +152,11 @@ static int precondition_chunks(
   if (count > kTileInline)
     KFAC_CUDA(cudaMemcpyAsync(base, host.data(), tables,
                               cudaMemcpyHostToDevice, st));
-  int rc = launch_pack_rows(reinterpret_cast<PackRows*>(base + jobs_at), jobs,
-                            njobs, rows, st);
+  const PackRows* jobs_dev = reinterpret_cast<PackRows*>(base + jobs_at);
+  int rc = launch_pack_rows(jobs_dev, jobs, 2 * count, rows, st);
+  if (rc == KFAC_OK)
+    rc = launch_pack_rows(jobs_dev + 2 * count, jobs + 2 * count, count, rows_G,
+                          st);
   if (rc == KFAC_OK)
     rc = launch_packed_precond(descs_dev, descs, count, tiles, false, lr,
                                momentum, st);

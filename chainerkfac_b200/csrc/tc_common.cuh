@@ -248,12 +248,21 @@ __device__ __forceinline__ void split_half2(float y0, float y1, unsigned& hi,
   lo = half2_sat(fmaf(y0, 0.f, y0 - f.x), fmaf(y1, 0.f, y1 - f.y));
 }
 
-// Power of two that brings values of up to `amax` (bits of a non-negative float)
-// to at most 2^15, and its reciprocal; both are normal numbers for every `amax`.
-__device__ __forceinline__ float half_scale(unsigned amax, float* inverse) {
-  const int e = max((int)(amax >> 23), 27) - 127;        // floor(log2)
-  *inverse = __uint_as_float((unsigned)(127 - 14 + e) << 23);
-  return __uint_as_float((unsigned)(127 + 14 - e) << 23);
+// Floor of the binary logarithm of |x|; kNoExp for zero, 128 for what is not
+// finite.  Below the normal numbers -127, which is an upper bound.
+constexpr int kNoExp = -4096;
+__device__ __forceinline__ int exp_of(float x) {
+  const unsigned u = __float_as_uint(x) & 0x7fffffffu;
+  return u != 0 ? (int)(u >> 23) - 127 : kNoExp;
+}
+
+// x 2^n in two exact steps; n beyond +-252 counts as that, which takes every
+// finite x out of the range of fp32 or leaves a zero.
+__device__ __forceinline__ float scale_exp(float x, int n) {
+  n = max(min(n, 252), -252);
+  const int h = n >> 1;
+  return x * __uint_as_float((unsigned)(127 + h) << 23) *
+         __uint_as_float((unsigned)(127 + n - h) << 23);
 }
 
 // Two values as bf16 terms x = hi + lo: one word of each (the first value in the

@@ -109,27 +109,13 @@ __device__ __forceinline__ void piece_each(int r, int c, int rows, int cols,
   }
 }
 
-// Scale of a column of U = grad A_inv^T as an operand of the second product:
-// its entries are at most the largest norm of a gradient row times the norm of
-// the column's row of A_inv.
-__device__ __forceinline__ float u_scale(float peak, float norm,
-                                         float* inverse) {
-  return half_scale(__float_as_uint(peak * norm) & 0x7fffffffu, inverse);
-}
-
-// Largest norm of a gradient row, by a warp (as bits: NaN stays the largest).
-__device__ __forceinline__ float peak_norm(const GemmDesc& g, int lane) {
-  unsigned m = 0;
-#pragma unroll 4
-  for (int i = lane; i < g.M; i += 32)
-    m = max(m, __float_as_uint(g.norm_g[i]) & 0x7fffffffu);
-  return __uint_as_float(__reduce_max_sync(0xffffffffu, m));
-}
-
-// First product of the preconditioning: a 16 x 32 piece of U into chunks, rows as
-// k (zeros up to the end of the last k-block).
+// First product of the preconditioning: a 16 x 32 piece of U = grad A_inv^T into
+// chunks, rows as k (zeros up to the end of the last k-block).  Rows and columns
+// are divided by bounds of the norms of what they are products of, so that an
+// entry is held relative to the most that its row and column could make it; the
+// rows' part is in G_inv's columns, the columns' comes out of kf.
 __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
-                                        int r, int c, float peak) {
+                                        int r, int c) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int gr = r + 8 * h;
@@ -139,12 +125,9 @@ __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
     for (int j = 0; j < 4; ++j) {
       // (columns past the last one: any values, nobody stores their results)
       const int gc = c + 8 * j, k0 = min(gc, g.N - 1), k1 = min(gc + 1, g.N - 1);
-      float inverse;
-      const float x0 = in ? v[4 * j + 2 * h] * s0 * g.cs[k0] : 0.f;
-      const float x1 = in ? v[4 * j + 2 * h + 1] * s0 * g.cs[k1] : 0.f;
       unsigned hi, lo;
-      split_half2(x0 * u_scale(peak, g.norm[k0], &inverse),
-                  x1 * u_scale(peak, g.norm[k1], &inverse), hi, lo);
+      split_half2(in ? v[4 * j + 2 * h] * s0 * g.cs[k0] : 0.f,
+                  in ? v[4 * j + 2 * h + 1] * s0 * g.cs[k1] : 0.f, hi, lo);
       unsigned char* p = g.pack + (long long)(gc >> 7) * g.pack_tile +
                          (long long)(gr >> 5) * kChunk +
                          ((gc >> 6) & 1) * 8192 +
@@ -158,16 +141,15 @@ __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
 // Second product: a 16 x 32 piece of kf to the weight and bias parts, and the
 // momentum update where the layer has it fused.
 __device__ __forceinline__ void store_kf(const GemmDesc& g, float v[16], int r,
-                                         int c, bool whole, float peak,
-                                         float lr, float momentum) {
-  const float s0 = g.rs[min(r, g.M - 1)], s1 = g.rs[min(r + 8, g.M - 1)];
+                                         int c, bool whole, float lr,
+                                         float momentum) {
+  const int e0 = g.re[min(r, g.M - 1)], e1 = g.re[min(r + 8, g.M - 1)];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    float inverse;
-    u_scale(peak, g.norm[min(c + 8 * (j >> 1) + (j & 1), g.N - 1)], &inverse);
+    const int e = g.ce[min(c + 8 * (j >> 1) + (j & 1), g.N - 1)];
     const int i = 4 * (j >> 1) + (j & 1);
-    v[i] = v[i] * s0 * inverse;
-    v[i + 2] = v[i + 2] * s1 * inverse;
+    v[i] = scale_exp(v[i], e0 + e);
+    v[i + 2] = scale_exp(v[i + 2], e1 + e);
   }
   const int dW = g.dW;
   const bool fused = g.pW != nullptr;
@@ -255,25 +237,34 @@ pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
              : k + e < total ? job.extra[row] : 0.f;
     return make_float4(x[0], x[1], x[2], x[3]);
   };
-  unsigned top = 0;
+  // (the exponents' array is padded to whole k-blocks)
+  auto load_exp = [&](int k) {
+    return job.col != nullptr ? *reinterpret_cast<const short4*>(job.col + k)
+                              : make_short4(0, 0, 0, 0);
+  };
+  int top = 2 * kNoExp;
 #pragma unroll 4
   for (int k = 4 * lane; k < total; k += 128) {
     const float4 x = load(k);
-    top = max(max(top, max(__float_as_uint(x.x) & 0x7fffffffu,
-                           __float_as_uint(x.y) & 0x7fffffffu)),
-              max(__float_as_uint(x.z) & 0x7fffffffu,
-                  __float_as_uint(x.w) & 0x7fffffffu));
+    const short4 e = load_exp(k);
+    // (a zero, in front of and behind the end of the row, counts for nothing)
+    top = max(max(top, max(x.x != 0.f ? exp_of(x.x) + e.x : top,
+                           x.y != 0.f ? exp_of(x.y) + e.y : top)),
+              max(x.z != 0.f ? exp_of(x.z) + e.z : top,
+                  x.w != 0.f ? exp_of(x.w) + e.w : top));
   }
   top = __reduce_max_sync(0xffffffffu, top);
-  float inverse;
-  const float s = half_scale(top, &inverse);
+  if (top == 2 * kNoExp) top = 0;            // a row of zeros
+  const int s = kChunkExp - top;
   const int nkb = (total + 31) >> 5;
   unsigned char* dst = job.dst + (long long)(row >> 7) * nkb * kChunk;
   float sum = 0.f;
 #pragma unroll 4
   for (int k = 4 * lane; k < 32 * nkb; k += 128) {
     const float4 x = load(k);
-    const float y0 = s * x.x, y1 = s * x.y, y2 = s * x.z, y3 = s * x.w;
+    const short4 e = load_exp(k);
+    const float y0 = scale_exp(x.x, s + e.x), y1 = scale_exp(x.y, s + e.y);
+    const float y2 = scale_exp(x.z, s + e.z), y3 = scale_exp(x.w, s + e.w);
     sum += y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3;
     unsigned h0, h1, l0, l1;
     split_half2(y0, y1, h0, l0);
@@ -287,10 +278,13 @@ pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   if (lane == 0) {
-    job.inv[row] = inverse;
-    // (a little up: the sum is rounded)
-    const float norm = 1.0001f * sqrtf(sum) * inverse;
-    if (job.norm != nullptr) job.norm[row] = norm;
+    // sum < 2^(f + 1), its root at most 2^n (rounding of the sum: far inside
+    // the factor of two that fp16 has left above 2^15)
+    const int n = sum == 0.f ? 0 : (exp_of(sum) + 2) >> 1;
+    job.exp[row] = (short)(job.fit == nullptr ? -s
+                           : sum == 0.f      ? kNoExp
+                                             : n - s);
+    if (job.fit != nullptr) job.fit[row] = scale_exp(job.gain, -n);
   }
 }
 
@@ -448,7 +442,6 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
     const bool vec = (ldc & 1) == 0 &&
                      (reinterpret_cast<uintptr_t>(g.C) & 7) == 0;
     const int lr = lane >> 2, lc = 2 * (lane & 3);
-    const float peak = MODE == 0 ? 0.f : peak_norm(g, lane);
     bool ok = true;
     const int nseg = nkb > 0 ? (kb0 + nkb - 1) / kSegment - seg0 + 1 : 1;
 #pragma unroll 1
@@ -510,11 +503,11 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
       }
       if (!live) continue;
       if constexpr (MODE == 1) {
-        store_u(g, v, r, c, peak);
+        store_u(g, v, r, c);
         continue;
       }
       if constexpr (MODE == 2) {
-        store_kf(g, v, r, c, whole && c0 + 32 <= g.dW, peak, plr, momentum);
+        store_kf(g, v, r, c, whole && c0 + 32 <= g.dW, plr, momentum);
         continue;
       }
       if (un != nullptr) {

@@ -828,6 +828,62 @@ def test_precondition_of_long_layers(ops, dG, dW, bias, offset, magnitude):
             assert rel(host(b2), 1.0 - 0.5 * ref[:, dW]) < 1e-5
 
 
+def _precondition(ops, Gi, Ai, g, bias=False):
+    """kf of one layer, and what fp64 gives for the same fp32 inputs; with
+    `bias` the last column of `g` is the bias gradient."""
+    Gi, Ai, g = (a.astype(np.float32) for a in (Gi, Ai, g))
+    cols = g.shape[1] - int(bias)
+    kW = torch.empty((g.shape[0], cols), device='cuda')
+    kb = torch.empty(g.shape[0], device='cuda') if bias else None
+    ops.precondition([dev(Gi)], [dev(Ai)], [dev(np.ascontiguousarray(
+        g[:, :cols]))], [dev(np.ascontiguousarray(g[:, cols])) if bias else None],
+        [kW], [kb])
+    got = host(kW)
+    if bias:
+        got = np.concatenate([got, host(kb)[:, None]], 1)
+    return got, Gi.astype(np.float64) @ g.astype(np.float64) @ \
+        Ai.astype(np.float64).T
+
+
+def _worst(got, ref, axis):
+    """Largest error of a row (axis 1) or column (axis 0), relative to it."""
+    norm = np.linalg.norm(ref, axis=axis)
+    err = np.linalg.norm(got - ref, axis=axis)
+    assert not err[norm == 0].any()
+    return (err[norm > 0] / norm[norm > 0]).max()
+
+
+def _inverse_of(rng, d, scale, damping):
+    x = rng.standard_normal((2 * d, d)) * scale
+    return np.linalg.inv(x.T @ x / (2 * d) + damping * np.eye(d))
+
+
+@pytest.mark.parametrize('dG,dW,bias', [(64, 1024, False), (300, 785, True),
+                                        (513, 511, False)])
+@pytest.mark.parametrize('small', [1e-4, 1e-8, 1e-12, 1e-30])
+def test_precondition_of_rows_of_any_scale(ops, dG, dW, bias, small):
+    """Every row of kf to 1e-5 of itself, however small its gradient is beside
+    the other rows': half of the rows, all but one, rows spread evenly; G_inv
+    nearly diagonal, so that a row of kf is as small as its gradient, and as the
+    damped factor of such rows.  22-bit terms (2^-21 per operand) and sums of up
+    to 1024 + 513 terms, cut off towards zero: 1e-5."""
+    rng = np.random.default_rng(dG + dW)
+    dA = dW + int(bias)
+    Ai = _inverse_of(rng, dA, 1.0, 1e-2)
+    near = np.diag(rng.random(dG) + 0.5) + \
+        small * 0.1 * rng.standard_normal((dG, dG))
+    base = rng.standard_normal((dG, dA))
+    half = np.where(np.arange(dG) % 2, small, 1.0)
+    for rows in (half, np.where(np.arange(dG) == 7, 1.0, small),
+                 small ** rng.random(dG)):
+        got, ref = _precondition(ops, near, Ai, base * rows[:, None], bias)
+        assert _worst(got, ref, 1) < 1e-5
+    got, ref = _precondition(ops, _inverse_of(rng, dG, half, small ** 2), Ai,
+                             base * half[:, None], bias) \
+        if small > 1e-10 else (ref, ref)
+    assert _worst(got, ref, 1) < 1e-5
+
+
 @pytest.mark.parametrize('value', [float('inf'), float('nan')])
 def test_precondition_of_a_non_finite_gradient_is_not_finite(ops, value):
     rng = np.random.default_rng(3)
