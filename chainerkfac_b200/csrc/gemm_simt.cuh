@@ -261,7 +261,20 @@ struct GemmDesc {
   int flags;
   int tile_begin;
   int tiles_m, tiles_n;
-  float *kfW, *kfb, *pW, *pb, *vW, *vb;
+  union {
+    struct {               // preconditioning, the product that gives kf
+      float *kfW, *kfb, *pW, *pb, *vW, *vb;
+    };
+    // the one before it, in chunks: rows of G_inv (M x M) packed beside it, from
+    // row inv_begin of the launch on
+    struct {
+      const float* inv;
+      unsigned char* inv_pack;
+      const short* inv_col;
+      short* inv_exp;
+      long long inv_begin;
+    };
+  };
   int dW;
   int splits;              // tensor-core engine: CTAs along the contraction
   int ntiles;              // tiles of one split (virtual tile = split * ntiles + tile)
@@ -297,17 +310,31 @@ struct GemmDesc {
 // whose values then have the 2-norm 2^n or less (n as small as a whole number
 // can be) leaves n - s, and 2^-n times `gain` as the factor that brings its
 // products with rows treated alike to at most `gain`; without `fit` it leaves -s.
-struct PackRows {
+struct PackRow {
   const float* src;
   const float* extra;      // appended column, NULL: none
-  const short* col;        // exponents of the columns' factors, NULL: none
+  const short* col;        // exponents of the columns' factors
+  int col_sign;            // 1, or -1 where the columns are divided by them
   unsigned char* dst;
   short* exp;
   float* fit;
   float gain;
   int cols;
+};
+struct PackRows : PackRow {
   int row_begin;           // first row in the launch
-  int pad_;
+};
+
+// Sizes of the columns of a gradient (and its bias column): exponents of the
+// largest value of each row, then of each column with the rows brought to one
+// size.
+struct GradSizes {
+  const float* src;
+  const float* extra;
+  short* row;
+  short* col;
+  int rows, cols;
+  int row_begin, col_begin;      // first row and group of columns
 };
 
 int launch_grouped_gemm(const GemmDesc* descs_dev, int ndesc, int total_tiles,
@@ -344,13 +371,17 @@ int packed_prepare();
 int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
                   int ndesc, int total_tiles, cudaStream_t stream);
 int packed_status_read(int* out);
-// Preconditioning on chunks: rows into chunks, then the product whose result is
-// chunks again (`last` false) or the preconditioned gradient.
+// Preconditioning on chunks: sizes of the gradients, rows into chunks, then the
+// product whose result is chunks again (beside it `inv_rows` rows of G_inv are
+// packed) and the one that gives the preconditioned gradient (inv_rows = 0).
 constexpr int kChunkExp = 14;    // scaled values of a row are below 2^15
+int launch_grad_sizes(const GradSizes* jobs_dev, const GradSizes* jobs_host,
+                      int njobs, int rows, int groups, bool wide,
+                      cudaStream_t stream);
 int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,
                      int njobs, int rows, cudaStream_t stream);
 int launch_packed_precond(const GemmDesc* descs_dev, const GemmDesc* descs_host,
-                          int ndesc, int total_tiles, bool last, float lr,
+                          int ndesc, int total_tiles, int inv_rows, float lr,
                           float momentum, cudaStream_t stream);
 bool tc_desc_has_tails(const GemmDesc& g);
 size_t tc_factor_workspace_bytes(long long rows, int d, bool staged = true);

@@ -15,6 +15,7 @@ static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 struct ChunkLayout {
   size_t G, A, g, U;             // G_inv, A_inv, gradient, grad * A_inv^T
   size_t exp_G, exp_A, exp_g;    // exponents of rows
+  size_t row, col;               // sizes of the gradient's rows and columns
   size_t fit_A, fit_g;           // factors of U's columns and rows
   size_t total;
 };
@@ -38,6 +39,8 @@ static ChunkLayout chunk_layout(int dG, int dA) {
   c.exp_G = take((dG + 31) * sizeof(short));
   c.exp_A = take((dA + 31) * sizeof(short));
   c.exp_g = take((dG + 31) * sizeof(short));
+  c.row = take(dG * sizeof(short));
+  c.col = take((dA + 31) * sizeof(short));
   c.fit_A = take(dA * sizeof(float));
   c.fit_g = take(dG * sizeof(float));
   c.total = at;
@@ -74,15 +77,20 @@ static int precondition_chunks(
     cudaStream_t st) {
   // tables, in front of the layers' chunks
   const size_t jobs_at = align256(2 * (size_t)count * sizeof(GemmDesc));
+  const size_t sizes_at =
+      jobs_at + align256(2 * (size_t)count * sizeof(PackRows));
   const size_t tables =
-      jobs_at + align256(3 * (size_t)count * sizeof(PackRows));
+      sizes_at + align256((size_t)count * sizeof(GradSizes));
   std::vector<char> host(tables, 0);
   GemmDesc* descs = reinterpret_cast<GemmDesc*>(host.data());
   PackRows* jobs = reinterpret_cast<PackRows*>(host.data() + jobs_at);
+  GradSizes* sizes = reinterpret_cast<GradSizes*>(host.data() + sizes_at);
   char* const base = ws;
   const GemmDesc* descs_dev = reinterpret_cast<GemmDesc*>(base);
   ws += tables;
-  int rows = 0, rows_G = 0;
+  int rows = 0, rows_G = 0, groups = 0, wide_groups = 0;
+  for (int i = 0; i < count; ++i) wide_groups += (dW[i] + hb[i] + 31) / 32;
+  const bool wide = wide_groups >= sm_count() / 2;
   auto at = [](char* base, size_t off) {
     return reinterpret_cast<unsigned char*>(base + off);
   };
@@ -96,27 +104,35 @@ static int precondition_chunks(
     const int dg = dG[i], dw = dW[i], da = dw + hb[i];
     const ChunkLayout c = chunk_layout(dg, da);
     const long long nkA = (da + 31) / 32, nkG = (dg + 31) / 32;
-    // Rows of the gradient and of A_inv, then (in a launch of its own) those of
-    // G_inv, whose columns take what U's rows are divided by: rows of the
-    // gradient of any scale, nearly dead units among them, are held alike.
-    // U's terms stay below 2^15 and take that out of kf again.
+    // Sums run over the gradient's columns, then over its rows.  The columns are
+    // divided by their size and those of A_inv multiplied by it, so that features
+    // of any scale are held alike; likewise the rows (what U's are divided by)
+    // and G_inv's columns, which is why G_inv is packed beside the first product.
+    // Errors without: see the tests of rows and features of any scale.
+    const float* const bias = hb[i] ? grad_b[i] : nullptr;
+    GradSizes& z = sizes[i];
+    z = GradSizes();
+    z.src = grad_W[i]; z.extra = bias;
+    z.row = exps(ws, c.row); z.col = exps(ws, c.col);
+    z.rows = dg; z.cols = dw;
+    z.row_begin = rows_G; z.col_begin = groups;
+    groups += wide ? (da + 31) / 32 : (da + 7) / 8;
     auto job = [&](PackRows& j, const float* src, const float* extra,
-                   size_t dst, int cols, int nrows, int& begin) {
+                   size_t dst, const short* col, int sign, int cols, int nrows,
+                   int& begin) {
       j = PackRows();
       j.src = src; j.extra = extra; j.dst = at(ws, dst);
+      j.col = col; j.col_sign = sign;
       j.cols = cols;
       j.row_begin = begin;
       begin += nrows;
     };
     PackRows& ja = jobs[2 * i];
-    job(ja, A_inv[i], nullptr, c.A, da, da, rows);
+    job(ja, A_inv[i], nullptr, c.A, z.col, 1, da, da, rows);
     ja.exp = exps(ws, c.exp_A); ja.fit = vec(ws, c.fit_A); ja.gain = kGainU;
     PackRows& jg = jobs[2 * i + 1];
-    job(jg, grad_W[i], hb[i] ? grad_b[i] : nullptr, c.g, dw, dg, rows);
+    job(jg, grad_W[i], bias, c.g, z.col, -1, dw, dg, rows);
     jg.exp = exps(ws, c.exp_g); jg.fit = vec(ws, c.fit_g); jg.gain = 1.f;
-    PackRows& jG = jobs[2 * count + i];
-    job(jG, G_inv[i], nullptr, c.G, dg, dg, rows_G);
-    jG.exp = exps(ws, c.exp_G); jG.col = jg.exp;
     // U = grad * A_inv^T
     GemmDesc& u = descs[i];
     u = GemmDesc();
@@ -127,6 +143,10 @@ static int precondition_chunks(
     u.cb = at(ws, c.A); u.cb_tile = nkA * kChunk;
     u.pack = at(ws, c.U); u.pack_tile = nkG * kChunk;
     u.rs = jg.fit; u.cs = ja.fit;
+    u.inv = G_inv[i]; u.inv_pack = at(ws, c.G);
+    u.inv_col = jg.exp; u.inv_exp = exps(ws, c.exp_G);
+    u.inv_begin = rows_G;
+    rows_G += dg;
     // kf = G_inv * U, split and (optionally) applied
     GemmDesc& h = descs[count + i];
     h = GemmDesc();
@@ -135,7 +155,7 @@ static int precondition_chunks(
     h.ca = at(ws, c.G); h.ca_tile = nkG * kChunk;
     h.cb = u.pack; h.cb_tile = u.pack_tile;
     h.alpha = 1.f / kGainU;
-    h.re = jG.exp; h.ce = ja.exp;
+    h.re = u.inv_exp; h.ce = ja.exp;
     const bool fused = param_W && param_W[i];
     h.kfW = kf_W ? kf_W[i] : nullptr;
     h.kfb = (hb[i] && kf_b) ? kf_b[i] : nullptr;
@@ -153,16 +173,15 @@ static int precondition_chunks(
     KFAC_CUDA(cudaMemcpyAsync(base, host.data(), tables,
                               cudaMemcpyHostToDevice, st));
   const PackRows* jobs_dev = reinterpret_cast<PackRows*>(base + jobs_at);
-  int rc = launch_pack_rows(jobs_dev, jobs, 2 * count, rows, st);
+  int rc = launch_grad_sizes(reinterpret_cast<GradSizes*>(base + sizes_at),
+                             sizes, count, rows_G, groups, wide, st);
+  if (rc == KFAC_OK) rc = launch_pack_rows(jobs_dev, jobs, 2 * count, rows, st);
   if (rc == KFAC_OK)
-    rc = launch_pack_rows(jobs_dev + 2 * count, jobs + 2 * count, count, rows_G,
-                          st);
-  if (rc == KFAC_OK)
-    rc = launch_packed_precond(descs_dev, descs, count, tiles, false, lr,
+    rc = launch_packed_precond(descs_dev, descs, count, tiles, rows_G, lr,
                                momentum, st);
   if (rc == KFAC_OK)
     rc = launch_packed_precond(descs_dev + count, descs + count, count, tiles,
-                               true, lr, momentum, st);
+                               0, lr, momentum, st);
   return rc;
 }
 
@@ -171,7 +190,8 @@ extern "C" size_t kfac_precond_workspace_bytes(int count, const int* dG,
                                                const int* has_bias) {
   if (count <= 0 || !dG || !dW) return 0;
   size_t total = align256(2 * (size_t)count * sizeof(GemmDesc));
-  size_t chunks = total + align256(3 * (size_t)count * sizeof(PackRows));
+  size_t chunks = total + align256(2 * (size_t)count * sizeof(PackRows)) +
+                  align256((size_t)count * sizeof(GradSizes));
   for (int i = 0; i < count; ++i) {
     size_t dA = (size_t)dW[i] + ((has_bias && has_bias[i]) ? 1 : 0);
     total += align256((size_t)dG[i] * dA * sizeof(float));

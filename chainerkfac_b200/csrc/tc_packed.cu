@@ -53,9 +53,14 @@ static __device__ int g_packed_status = 0;
 
 struct PackInline {
   int n;                       // 0: jobs in device memory
-  PackRows j[3 * TT_INLINE];   // three operands a layer
+  PackRows j[2 * TT_INLINE];   // two operands a layer
 };
 static_assert(sizeof(PackInline) <= 3800, "kernel argument space");
+
+struct GradInline {
+  int n;
+  GradSizes j[TT_INLINE];
+};
 
 struct PackedControl {
   unsigned long long full[KP_STAGES_MAX];    // the copies have arrived
@@ -205,25 +210,107 @@ __device__ __forceinline__ void store_kf(const GemmDesc& g, float v[16], int r,
   });
 }
 
-// One row per warp: its largest value, then (the row is in the L1 cache) the
-// scaled terms.  Bound by HBM: 4 bytes read and 4 written per element.
+// The launches of a preconditioning may begin while the one before still runs
+// (programmatic dependent launch); they read nothing that it writes, and write
+// nothing, before wait_for_launch_before, which returns when it is complete.
+__device__ __forceinline__ void let_next_launch_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_launch_before() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Sizes of the rows of gradients (see GradSizes), a block per row.
 __global__ void __launch_bounds__(256)
-pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
-                 const __grid_constant__ PackInline inl) {
-  const int lane = threadIdx.x & 31;
-  const int row_all = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (row_all >= rows) return;
+grad_rows_kernel(const GradSizes* __restrict__ jobs, int njobs,
+                 const __grid_constant__ GradInline inl) {
+  __shared__ int part[8];
+  let_next_launch_begin();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const GradSizes* all = inl.n > 0 ? inl.j : jobs;
   int f = 0;
-  if (inl.n > 0) {
-    for (int i = lane; i < inl.n; i += 32)
-      if (inl.j[i].row_begin <= row_all) f = i;
-  } else {
-    for (int i = lane; i < njobs; i += 32)
-      if (jobs[i].row_begin <= row_all) f = i;
-  }
+  for (int i = lane; i < njobs; i += 32)
+    if (all[i].row_begin <= (int)blockIdx.x) f = i;
   f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
-  const PackRows job = inl.n > 0 ? inl.j[f] : jobs[f];
-  const int row = row_all - job.row_begin, cols = job.cols;
+  const GradSizes& job = all[f];
+  const int row = blockIdx.x - job.row_begin, cols = job.cols;
+  const float* src = job.src + (long long)row * cols;
+  int top = kNoExp;
+  if (job.extra != nullptr && threadIdx.x == 0) top = exp_of(job.extra[row]);
+  // (eight loads in flight; past the end the last one again)
+  for (int k0 = threadIdx.x; k0 < cols; k0 += 8 * 256) {
+    float x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = src[min(k0 + 256 * u, cols - 1)];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) top = max(top, exp_of(x[u]));
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) part[warp] = top;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) top = max(top, part[i]);
+    job.row[row] = (short)top;
+  }
+}
+
+// Sizes of the columns behind it, W columns per block and 1024 / W rows at a time.
+// Narrow groups where wide ones would leave SMs idle (1000 x 1000: 5 us less), wide
+// ones elsewhere (512 x 4608: 6.5 us, 16 with narrow ones).
+template <int W>
+__global__ void __launch_bounds__(1024)
+grad_cols_kernel(const GradSizes* __restrict__ jobs, int njobs,
+                 const __grid_constant__ GradInline inl) {
+  __shared__ int part[32][W + 1];
+  let_next_launch_begin();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const GradSizes* all = inl.n > 0 ? inl.j : jobs;
+  int f = 0;
+  for (int i = lane; i < njobs; i += 32)
+    if (all[i].col_begin <= (int)blockIdx.x) f = i;
+  f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
+  const GradSizes job = all[f];
+  const int c0 = W * (blockIdx.x - job.col_begin), c = c0 + lane % W;
+  const bool tail = c >= job.cols;       // the appended column, or none
+  const float* src = tail ? job.extra : job.src + c;
+  const long long step = tail ? 1 : job.cols;
+  const int total = job.cols + (job.extra != nullptr ? 1 : 0);
+  int top = kNoExp;
+  wait_for_launch_before();
+  if (c < total) {
+    constexpr int S = 1024 / W;
+    for (int r0 = (32 / W) * warp + lane / W; r0 < job.rows; r0 += 8 * S) {
+      float x[8];
+      int e[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int r = min(r0 + S * u, job.rows - 1);
+        x[u] = src[r * step];
+        e[u] = job.row[r];
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (x[u] != 0.f) top = max(top, exp_of(x[u]) - e[u]);
+    }
+  }
+#pragma unroll
+  for (int o = W; o < 32; o *= 2)
+    top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+  if (lane < W) part[warp][lane] = top;
+  __syncthreads();
+  if (warp >= W) return;
+  top = __reduce_max_sync(0xffffffffu, part[lane][warp]);
+  // (not below -126, so that the factor is a normal number; a column of zeros
+  // gets that as well)
+  if (lane == 0 && c0 + warp < total) job.col[c0 + warp] = (short)max(top, -126);
+}
+
+// A row by a warp: its largest value, then (the row is in the L1 cache) the
+// scaled terms.  Bound by HBM: 4 bytes read and 4 written per element.
+__device__ __forceinline__ void pack_row(const PackRow& job, int row,
+                                         int lane) {
+  const int cols = job.cols;
   const int total = cols + (job.extra != nullptr ? 1 : 0);
   const float* src = job.src + (long long)row * cols;
   const bool vec =
@@ -237,35 +324,17 @@ pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
              : k + e < total ? job.extra[row] : 0.f;
     return make_float4(x[0], x[1], x[2], x[3]);
   };
-  // (the exponents' array is padded to whole k-blocks)
+  const int sign = job.col_sign;
+  // (what stands behind the row's end is not read as an exponent)
   auto load_exp = [&](int k) {
-    return job.col != nullptr ? *reinterpret_cast<const short4*>(job.col + k)
-                              : make_short4(0, 0, 0, 0);
+    if (k + 3 < total) return *reinterpret_cast<const short4*>(job.col + k);
+    return make_short4(k < total ? job.col[k] : 0,
+                       k + 1 < total ? job.col[k + 1] : 0,
+                       k + 2 < total ? job.col[k + 2] : 0, 0);
   };
-  int top = 2 * kNoExp;
-#pragma unroll 4
-  for (int k = 4 * lane; k < total; k += 128) {
-    const float4 x = load(k);
-    const short4 e = load_exp(k);
-    // (a zero, in front of and behind the end of the row, counts for nothing)
-    top = max(max(top, max(x.x != 0.f ? exp_of(x.x) + e.x : top,
-                           x.y != 0.f ? exp_of(x.y) + e.y : top)),
-              max(x.z != 0.f ? exp_of(x.z) + e.z : top,
-                  x.w != 0.f ? exp_of(x.w) + e.w : top));
-  }
-  top = __reduce_max_sync(0xffffffffu, top);
-  if (top == 2 * kNoExp) top = 0;            // a row of zeros
-  const int s = kChunkExp - top;
   const int nkb = (total + 31) >> 5;
   unsigned char* dst = job.dst + (long long)(row >> 7) * nkb * kChunk;
-  float sum = 0.f;
-#pragma unroll 4
-  for (int k = 4 * lane; k < 32 * nkb; k += 128) {
-    const float4 x = load(k);
-    const short4 e = load_exp(k);
-    const float y0 = scale_exp(x.x, s + e.x), y1 = scale_exp(x.y, s + e.y);
-    const float y2 = scale_exp(x.z, s + e.z), y3 = scale_exp(x.w, s + e.w);
-    sum += y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3;
+  auto store = [&](int k, float y0, float y1, float y2, float y3) {
     unsigned h0, h1, l0, l1;
     split_half2(y0, y1, h0, l0);
     split_half2(y2, y3, h1, l1);
@@ -275,6 +344,74 @@ pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
     *reinterpret_cast<uint2*>(p) = make_uint2(h0, h1);
     p = reinterpret_cast<unsigned char*>(reinterpret_cast<uintptr_t>(p) ^ 0x40);
     *reinterpret_cast<uint2*>(p) = make_uint2(l0, l1);
+  };
+  // Factors and the scaled row inside the range of fp32 with 2^60 to spare below
+  // (what is left of a value under that is less than its terms hold): one
+  // multiplication for the column and one for the row.  With the exponents
+  // added up for every element a call on 1024 x 2048 took 87 us, now 7x.
+  auto factor = [&](int e) {
+    return __uint_as_float(0x3f800000u + (unsigned)((sign * e) << 23));
+  };
+  unsigned widest = 0;
+  float peak = 0.f;
+  // (four loads in flight; zeros behind the end)
+#pragma unroll 1
+  for (int k0 = 4 * lane; k0 < total; k0 += 512)
+#pragma unroll
+  for (int k = k0; k < k0 + 512; k += 128) {
+    const float4 x = load(k);
+    const short4 e = load_exp(k);
+    widest = max(max(max(widest, (unsigned)abs(e.x)), (unsigned)abs(e.y)),
+                 max((unsigned)abs(e.z), (unsigned)abs(e.w)));
+    peak = fmaxf(fmaxf(peak, fmaxf(fabsf(x.x * factor(e.x)),
+                                   fabsf(x.y * factor(e.y)))),
+                 fmaxf(fabsf(x.z * factor(e.z)), fabsf(x.w * factor(e.w))));
+  }
+  widest = __reduce_max_sync(0xffffffffu, widest);
+  const unsigned bits =
+      __reduce_max_sync(0xffffffffu, __float_as_uint(peak));
+  int top = (int)(bits >> 23) - 127, s;
+  float sum = 0.f;
+  if (widest <= 126 && top >= -60 && top <= 100) {
+    s = kChunkExp - top;
+    const float f = __uint_as_float((unsigned)(127 + s) << 23);
+#pragma unroll 1
+    for (int k0 = 4 * lane; k0 < 32 * nkb; k0 += 512)
+#pragma unroll
+    for (int k = k0; k < k0 + 512; k += 128) {
+      const float4 x = load(k);
+      const short4 e = load_exp(k);
+      const float y0 = x.x * factor(e.x) * f, y1 = x.y * factor(e.y) * f;
+      const float y2 = x.z * factor(e.z) * f, y3 = x.w * factor(e.w) * f;
+      sum += y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3;
+      if (k < 32 * nkb) store(k, y0, y1, y2, y3);
+    }
+  } else {
+    top = 2 * kNoExp;
+#pragma unroll 1
+    for (int k = 4 * lane; k < total; k += 128) {
+      const float4 x = load(k);
+      const short4 e = load_exp(k);
+      // (a zero, in the row or behind its end, counts for nothing)
+      if (x.x != 0.f) top = max(top, exp_of(x.x) + sign * e.x);
+      if (x.y != 0.f) top = max(top, exp_of(x.y) + sign * e.y);
+      if (x.z != 0.f) top = max(top, exp_of(x.z) + sign * e.z);
+      if (x.w != 0.f) top = max(top, exp_of(x.w) + sign * e.w);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (top == 2 * kNoExp) top = 0;            // a row of zeros
+    s = kChunkExp - top;
+#pragma unroll 1
+    for (int k = 4 * lane; k < 32 * nkb; k += 128) {
+      const float4 x = load(k);
+      const short4 e = load_exp(k);
+      const float y0 = scale_exp(x.x, s + sign * e.x);
+      const float y1 = scale_exp(x.y, s + sign * e.y);
+      const float y2 = scale_exp(x.z, s + sign * e.z);
+      const float y3 = scale_exp(x.w, s + sign * e.w);
+      sum += y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3;
+      store(k, y0, y1, y2, y3);
+    }
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   if (lane == 0) {
@@ -288,13 +425,47 @@ pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
   }
 }
 
+__global__ void __launch_bounds__(256)
+pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
+                 const __grid_constant__ PackInline inl) {
+  const int lane = threadIdx.x & 31;
+  const int row_all = blockIdx.x * 8 + (threadIdx.x >> 5);
+  let_next_launch_begin();
+  if (row_all >= rows) return;
+  const PackRows* all = inl.n > 0 ? inl.j : jobs;
+  int f = 0;
+  for (int i = lane; i < njobs; i += 32)
+    if (all[i].row_begin <= row_all) f = i;
+  f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
+  const PackRows job = all[f];
+  wait_for_launch_before();
+  pack_row(job, row_all - job.row_begin, lane);
+}
+
+// A row of G_inv, of all layers' in a launch of the first product.
+__device__ __noinline__ void pack_inverse(const GemmDesc* all, int n,
+                                             int row_all, int lane) {
+  int f = 0;
+  for (int i = lane; i < n; i += 32)
+    if (all[i].inv_begin <= row_all) f = i;
+  f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
+  const GemmDesc& g = all[f];
+  PackRow job;
+  job.src = g.inv; job.extra = nullptr;
+  job.col = g.inv_col; job.col_sign = 1;
+  job.dst = g.inv_pack;
+  job.exp = g.inv_exp; job.fit = nullptr; job.gain = 0.f;
+  job.cols = g.M;
+  pack_row(job, row_all - (int)g.inv_begin, lane);
+}
+
 // MODE 0: the products of the inverse; 1, 2: first and second product of the
 // preconditioning, uncut as a sum of TF32 terms was, with half its MMAs.
 template <int MODE, int STAGES>
 __global__ void __launch_bounds__(KP_THREADS, STAGES == 3 ? 2 : 1)
 packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
                    const __grid_constant__ TileInline inl, float plr,
-                   float momentum) {
+                   float momentum, int inv_rows, int inv_ctas) {
   constexpr int kSegment = MODE == 0 ? KP_SEGMENT : 1 << 20;
   constexpr int TN = 128;
   extern __shared__ unsigned char kp_smem_raw[];
@@ -303,7 +474,25 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
   PackedControl* ctl =
       reinterpret_cast<PackedControl*>(smem + STAGES * KP_STAGE);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tile = blockIdx.x;
+  // First product: the rows of G_inv, which the next launch needs, are packed by
+  // `inv_ctas` CTAs in front of the tiles (on SMs without one) and by the
+  // epilogue's warps while the MMAs run.  us in a launch of its own, in CTAs
+  // only, by the epilogues only: 512 x 512 +3.5, 40, 46; 1024 x 2048 +4, 87, 79.
+  const int tile = (int)blockIdx.x - inv_ctas;
+  auto pack_inverses = [&](int worker) {
+    const int workers = inv_ctas * (KP_THREADS / 32) +
+                        ((int)gridDim.x - inv_ctas) * KP_EPI_WARPS;
+    for (int i = worker; i < inv_rows; i += workers)
+      pack_inverse(inl.n > 0 ? inl.d : descs, ndesc, i, lane);
+  };
+  if constexpr (MODE == 1) {
+    if (tile < 0) {
+      let_next_launch_begin();
+      wait_for_launch_before();
+      pack_inverses(blockIdx.x * (KP_THREADS / 32) + warp);
+      return;
+    }
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -348,6 +537,10 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if constexpr (MODE > 0) {
+    let_next_launch_begin();     // (its CTAs cannot take this one's tensor memory)
+    wait_for_launch_before();
+  }
 
   const GemmDesc& g = ctl->desc;
   const unsigned tmem = ctl->tmem_base;
@@ -442,6 +635,9 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
     const bool vec = (ldc & 1) == 0 &&
                      (reinterpret_cast<uintptr_t>(g.C) & 7) == 0;
     const int lr = lane >> 2, lc = 2 * (lane & 3);
+    if constexpr (MODE == 1)
+      pack_inverses(inv_ctas * (KP_THREADS / 32) + tile * KP_EPI_WARPS + warp -
+                    2);
     bool ok = true;
     const int nseg = nkb > 0 ? (kb0 + nkb - 1) / kSegment - seg0 + 1 : 1;
 #pragma unroll 1
@@ -564,8 +760,29 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
 }
 
 // ------------------------------------------------------------------ host side
+// `early`: the launch may begin before the one in front of it has ended.
+template <typename... P, typename... A>
+static int launch_behind(const char* name, bool early, void (*kernel)(P...),
+                         int blocks, int threads, int smem, cudaStream_t stream,
+                         A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
+  KFAC_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  KFAC_LAUNCH_CHECK(name);
+  return KFAC_OK;
+}
+
 struct PackedVariant {
-  void (*kernel)(const GemmDesc*, int, const TileInline, float, float);
+  void (*kernel)(const GemmDesc*, int, const TileInline, float, float, int,
+                 int);
   int stages;
 };
 // by mode; the preconditioning also with one CTA an SM
@@ -607,7 +824,8 @@ int packed_number_tiles(GemmDesc* descs, int n) {
 
 static int launch_mode(int mode, const GemmDesc* descs_dev,
                        const GemmDesc* descs_host, int ndesc, int total_tiles,
-                       float lr, float momentum, cudaStream_t stream) {
+                       int inv_rows, float lr, float momentum,
+                       cudaStream_t stream) {
   if (ndesc <= 0 || total_tiles <= 0) return KFAC_OK;
   const int rc = packed_prepare();
   if (rc != KFAC_OK) return rc;
@@ -619,23 +837,44 @@ static int launch_mode(int mode, const GemmDesc* descs_dev,
   }
   const bool one = mode > 0 && total_tiles <= sm_count();
   const PackedVariant& v = kPackedVariants[one ? mode + 2 : mode];
-  v.kernel<<<total_tiles, KP_THREADS, packed_smem(v.stages), stream>>>(
-      descs_dev, ndesc, inl, lr, momentum);
-  KFAC_LAUNCH_CHECK("packed_tile_kernel");
-  return KFAC_OK;
+  const int inv_ctas =
+      one ? std::min(sm_count() - total_tiles, (int)ceil_div(inv_rows, KP_THREADS / 32))
+          : 0;
+  return launch_behind("packed_tile_kernel", mode > 0, v.kernel,
+                       total_tiles + inv_ctas, KP_THREADS,
+                       packed_smem(v.stages), stream, descs_dev, ndesc, inl, lr,
+                       momentum, inv_rows, inv_ctas);
 }
 
 int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
                   int ndesc, int total_tiles, cudaStream_t stream) {
-  return launch_mode(0, descs_dev, descs_host, ndesc, total_tiles, 0.f, 0.f,
+  return launch_mode(0, descs_dev, descs_host, ndesc, total_tiles, 0, 0.f, 0.f,
                      stream);
 }
 
 int launch_packed_precond(const GemmDesc* descs_dev, const GemmDesc* descs_host,
-                          int ndesc, int total_tiles, bool last, float lr,
+                          int ndesc, int total_tiles, int inv_rows, float lr,
                           float momentum, cudaStream_t stream) {
-  return launch_mode(last ? 2 : 1, descs_dev, descs_host, ndesc, total_tiles, lr,
-                     momentum, stream);
+  return launch_mode(inv_rows > 0 ? 1 : 2, descs_dev, descs_host, ndesc,
+                     total_tiles, inv_rows, lr, momentum, stream);
+}
+
+int launch_grad_sizes(const GradSizes* jobs_dev, const GradSizes* jobs_host,
+                      int njobs, int rows, int groups, bool wide,
+                      cudaStream_t stream) {
+  if (njobs <= 0 || rows <= 0) return KFAC_OK;
+  GradInline inl;
+  inl.n = 0;
+  if (njobs <= TT_INLINE) {
+    inl.n = njobs;
+    std::copy(jobs_host, jobs_host + njobs, inl.j);
+  }
+  const int rc = launch_behind("grad_rows_kernel", false, grad_rows_kernel, rows,
+                               256, 0, stream, jobs_dev, njobs, inl);
+  if (rc != KFAC_OK) return rc;
+  return launch_behind("grad_cols_kernel", true,
+                       wide ? grad_cols_kernel<32> : grad_cols_kernel<8>, groups,
+                       1024, 0, stream, jobs_dev, njobs, inl);
 }
 
 int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,
@@ -643,14 +882,13 @@ int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,
   if (njobs <= 0 || rows <= 0) return KFAC_OK;
   PackInline inl;
   inl.n = 0;
-  if (njobs <= 3 * TT_INLINE) {
+  if (njobs <= 2 * TT_INLINE) {
     inl.n = njobs;
     std::copy(jobs_host, jobs_host + njobs, inl.j);
   }
-  pack_rows_kernel<<<ceil_div(rows, 8), 256, 0, stream>>>(jobs_dev, njobs, rows,
-                                                          inl);
-  KFAC_LAUNCH_CHECK("pack_rows_kernel");
-  return KFAC_OK;
+  return launch_behind("pack_rows_kernel", true, pack_rows_kernel,
+                       (int)ceil_div(rows, 8), 256, 0, stream, jobs_dev, njobs,
+                       rows, inl);
 }
 
 int packed_status_read(int* out) {

@@ -845,9 +845,11 @@ def _precondition(ops, Gi, Ai, g, bias=False):
         Ai.astype(np.float64).T
 
 
-def _worst(got, ref, axis):
-    """Largest error of a row (axis 1) or column (axis 0), relative to it."""
-    norm = np.linalg.norm(ref, axis=axis)
+def _worst(got, ref, axis, terms=0.0):
+    """Largest error of a row (axis 1) or column (axis 0), relative to it;
+    with `terms`, the sums of the products' sizes, to a sixteenth of those at
+    least (what cancels in a sum is not lost by its error)."""
+    norm = np.linalg.norm(np.maximum(np.abs(ref), terms / 16), axis=axis)
     err = np.linalg.norm(got - ref, axis=axis)
     assert not err[norm == 0].any()
     return (err[norm > 0] / norm[norm > 0]).max()
@@ -881,6 +883,38 @@ def test_precondition_of_rows_of_any_scale(ops, dG, dW, bias, small):
     got, ref = _precondition(ops, _inverse_of(rng, dG, half, small ** 2), Ai,
                              base * half[:, None], bias) \
         if small > 1e-10 else (ref, ref)
+    assert _worst(got, ref, 1) < 1e-5
+
+
+@pytest.mark.parametrize('dG,dW,bias', [(64, 1024, False), (300, 785, True),
+                                        (513, 511, False)])
+@pytest.mark.parametrize('small', [1e-4, 1e-8, 1e-12])
+def test_precondition_of_features_of_any_scale(ops, dG, dW, bias, small):
+    """Every row and column of kf to 1e-5 of itself with input features of
+    different scales, A_inv that of such features with a damping below the
+    smallest or between the two kinds (features that are nearly always zero), some
+    features exactly zero, and with rows of different scales besides.  A single
+    large entry takes nothing from the other rows.  Bound: as for rows."""
+    rng = np.random.default_rng(dG + dW + 1)
+    dA = dW + int(bias)
+    Gi = _inverse_of(rng, dG, 1.0, 1e-2)
+    base = rng.standard_normal((dG, dA))
+    half = np.where(np.arange(dA) % 2, small, 1.0)
+    half[dA // 3] = 0.0
+    spread = small ** rng.random(dA)
+    rows = small ** rng.random(dG)
+    near = np.diag(rng.random(dG) + 0.5) + \
+        small * 0.1 * rng.standard_normal((dG, dG))
+    for f, damping in ((half, 1e-3), (spread, 1e-3), (spread, small ** 2)):
+        Ai = _inverse_of(rng, dA, f, damping)
+        for G, g in ((Gi, base * f), (near, base * f * rows[:, None])):
+            got, ref = _precondition(ops, G, Ai, g, bias)
+            terms = np.abs(G) @ np.abs(g) @ np.abs(Ai)
+            assert _worst(got, ref, 1, terms) < 1e-5
+            assert _worst(got, ref, 0, terms) < 1e-5
+    g = base.copy()
+    g[5, 3] = 1 / small
+    got, ref = _precondition(ops, near, _inverse_of(rng, dA, 1.0, 1e-2), g, bias)
     assert _worst(got, ref, 1) < 1e-5
 
 
