@@ -372,8 +372,9 @@ int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
                   int ndesc, int total_tiles, cudaStream_t stream);
 int packed_status_read(int* out);
 // Preconditioning on chunks: sizes of the gradients, rows into chunks, then the
-// product whose result is chunks again (beside it `inv_rows` rows of G_inv are
-// packed) and the one that gives the preconditioned gradient (inv_rows = 0).
+// product whose result is chunks again and the one that gives the preconditioned
+// gradient.  Beside the first, `inv_rows` rows of G_inv are packed, where
+// packed_takes_rows says that this pays.
 constexpr int kChunkExp = 14;    // scaled values of a row are below 2^15
 int launch_grad_sizes(const GradSizes* jobs_dev, const GradSizes* jobs_host,
                       int njobs, int rows, int groups, bool wide,
@@ -381,8 +382,9 @@ int launch_grad_sizes(const GradSizes* jobs_dev, const GradSizes* jobs_host,
 int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,
                      int njobs, int rows, cudaStream_t stream);
 int launch_packed_precond(const GemmDesc* descs_dev, const GemmDesc* descs_host,
-                          int ndesc, int total_tiles, int inv_rows, float lr,
-                          float momentum, cudaStream_t stream);
+                          int ndesc, int total_tiles, bool last, int inv_rows,
+                          float lr, float momentum, cudaStream_t stream);
+bool packed_takes_rows(int total_tiles, int rows);
 bool tc_desc_has_tails(const GemmDesc& g);
 size_t tc_factor_workspace_bytes(long long rows, int d, bool staged = true);
 size_t tc_lone_workspace_bytes(const Operand& X, long long rows, int d);

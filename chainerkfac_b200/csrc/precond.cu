@@ -78,7 +78,7 @@ static int precondition_chunks(
   // tables, in front of the layers' chunks
   const size_t jobs_at = align256(2 * (size_t)count * sizeof(GemmDesc));
   const size_t sizes_at =
-      jobs_at + align256(2 * (size_t)count * sizeof(PackRows));
+      jobs_at + align256(3 * (size_t)count * sizeof(PackRows));
   const size_t tables =
       sizes_at + align256((size_t)count * sizeof(GradSizes));
   std::vector<char> host(tables, 0);
@@ -107,7 +107,7 @@ static int precondition_chunks(
     // Sums run over the gradient's columns, then over its rows.  The columns are
     // divided by their size and those of A_inv multiplied by it, so that features
     // of any scale are held alike; likewise the rows (what U's are divided by)
-    // and G_inv's columns, which is why G_inv is packed beside the first product.
+    // and G_inv's columns, which is why G_inv is packed later.
     // Errors without: see the tests of rows and features of any scale.
     const float* const bias = hb[i] ? grad_b[i] : nullptr;
     GradSizes& z = sizes[i];
@@ -133,6 +133,10 @@ static int precondition_chunks(
     PackRows& jg = jobs[2 * i + 1];
     job(jg, grad_W[i], bias, c.g, z.col, -1, dw, dg, rows);
     jg.exp = exps(ws, c.exp_g); jg.fit = vec(ws, c.fit_g); jg.gain = 1.f;
+    PackRows& jG = jobs[2 * count + i];
+    int inv_begin = rows_G;
+    job(jG, G_inv[i], nullptr, c.G, jg.exp, 1, dg, dg, rows_G);
+    jG.exp = exps(ws, c.exp_G);
     // U = grad * A_inv^T
     GemmDesc& u = descs[i];
     u = GemmDesc();
@@ -143,10 +147,9 @@ static int precondition_chunks(
     u.cb = at(ws, c.A); u.cb_tile = nkA * kChunk;
     u.pack = at(ws, c.U); u.pack_tile = nkG * kChunk;
     u.rs = jg.fit; u.cs = ja.fit;
-    u.inv = G_inv[i]; u.inv_pack = at(ws, c.G);
-    u.inv_col = jg.exp; u.inv_exp = exps(ws, c.exp_G);
-    u.inv_begin = rows_G;
-    rows_G += dg;
+    u.inv = jG.src; u.inv_pack = jG.dst;
+    u.inv_col = jG.col; u.inv_exp = jG.exp;
+    u.inv_begin = inv_begin;
     // kf = G_inv * U, split and (optionally) applied
     GemmDesc& h = descs[count + i];
     h = GemmDesc();
@@ -155,7 +158,7 @@ static int precondition_chunks(
     h.ca = at(ws, c.G); h.ca_tile = nkG * kChunk;
     h.cb = u.pack; h.cb_tile = u.pack_tile;
     h.alpha = 1.f / kGainU;
-    h.re = u.inv_exp; h.ce = ja.exp;
+    h.re = jG.exp; h.ce = ja.exp;
     const bool fused = param_W && param_W[i];
     h.kfW = kf_W ? kf_W[i] : nullptr;
     h.kfb = (hb[i] && kf_b) ? kf_b[i] : nullptr;
@@ -176,12 +179,16 @@ static int precondition_chunks(
   int rc = launch_grad_sizes(reinterpret_cast<GradSizes*>(base + sizes_at),
                              sizes, count, rows_G, groups, wide, st);
   if (rc == KFAC_OK) rc = launch_pack_rows(jobs_dev, jobs, 2 * count, rows, st);
+  const bool beside = packed_takes_rows(tiles, rows_G);
+  if (rc == KFAC_OK && !beside)
+    rc = launch_pack_rows(jobs_dev + 2 * count, jobs + 2 * count, count, rows_G,
+                          st);
   if (rc == KFAC_OK)
-    rc = launch_packed_precond(descs_dev, descs, count, tiles, rows_G, lr,
-                               momentum, st);
+    rc = launch_packed_precond(descs_dev, descs, count, tiles, false,
+                               beside ? rows_G : 0, lr, momentum, st);
   if (rc == KFAC_OK)
     rc = launch_packed_precond(descs_dev + count, descs + count, count, tiles,
-                               0, lr, momentum, st);
+                               true, 0, lr, momentum, st);
   return rc;
 }
 
@@ -190,7 +197,7 @@ extern "C" size_t kfac_precond_workspace_bytes(int count, const int* dG,
                                                const int* has_bias) {
   if (count <= 0 || !dG || !dW) return 0;
   size_t total = align256(2 * (size_t)count * sizeof(GemmDesc));
-  size_t chunks = total + align256(2 * (size_t)count * sizeof(PackRows)) +
+  size_t chunks = total + align256(3 * (size_t)count * sizeof(PackRows)) +
                   align256((size_t)count * sizeof(GradSizes));
   for (int i = 0; i < count; ++i) {
     size_t dA = (size_t)dW[i] + ((has_bias && has_bias[i]) ? 1 : 0);

@@ -220,39 +220,61 @@ __device__ __forceinline__ void wait_for_launch_before() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Sizes of the rows of gradients (see GradSizes), a block per row.
+// Sizes of the rows of gradients (see GradSizes), WARPS warps per row.  A block per
+// row where there are few (the latency of a row counts), a warp per row elsewhere
+// (54 layers of ResNet-50: 60 us with blocks, 23 with warps).
+template <int WARPS>
 __global__ void __launch_bounds__(256)
-grad_rows_kernel(const GradSizes* __restrict__ jobs, int njobs,
+grad_rows_kernel(const GradSizes* __restrict__ jobs, int njobs, int rows,
                  const __grid_constant__ GradInline inl) {
   __shared__ int part[8];
   let_next_launch_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row_all = (8 / WARPS) * blockIdx.x + warp / WARPS;
+  if (row_all >= rows) return;           // (whole blocks where WARPS is 8)
   const GradSizes* all = inl.n > 0 ? inl.j : jobs;
   int f = 0;
   for (int i = lane; i < njobs; i += 32)
-    if (all[i].row_begin <= (int)blockIdx.x) f = i;
+    if (all[i].row_begin <= row_all) f = i;
   f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
   const GradSizes& job = all[f];
-  const int row = blockIdx.x - job.row_begin, cols = job.cols;
+  const int row = row_all - job.row_begin, cols = job.cols;
   const float* src = job.src + (long long)row * cols;
+  const int at = 32 * (warp % WARPS) + lane;
+  constexpr int S = 32 * WARPS;
   int top = kNoExp;
-  if (job.extra != nullptr && threadIdx.x == 0) top = exp_of(job.extra[row]);
+  if (job.extra != nullptr && at == 0) top = exp_of(job.extra[row]);
   // (eight loads in flight; past the end the last one again)
-  for (int k0 = threadIdx.x; k0 < cols; k0 += 8 * 256) {
-    float x[8];
+  if (WARPS == 1 && (cols & 3) == 0 &&
+      (reinterpret_cast<uintptr_t>(job.src) & 15) == 0) {
+    const float4* s4 = reinterpret_cast<const float4*>(src);
+    const int n = cols >> 2;
+    for (int k0 = at; k0 < n; k0 += 8 * S) {
+      float4 x[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) x[u] = src[min(k0 + 256 * u, cols - 1)];
+      for (int u = 0; u < 8; ++u) x[u] = s4[min(k0 + S * u, n - 1)];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) top = max(top, exp_of(x[u]));
+      for (int u = 0; u < 8; ++u)
+        top = max(max(max(top, exp_of(x[u].x)), exp_of(x[u].y)),
+                  max(exp_of(x[u].z), exp_of(x[u].w)));
+    }
+  } else {
+    for (int k0 = at; k0 < cols; k0 += 8 * S) {
+      float x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = src[min(k0 + S * u, cols - 1)];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) top = max(top, exp_of(x[u]));
+    }
   }
   top = __reduce_max_sync(0xffffffffu, top);
-  if (lane == 0) part[warp] = top;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  if (WARPS > 1) {
+    if (lane == 0) part[warp] = top;
+    __syncthreads();
 #pragma unroll
     for (int i = 0; i < 8; ++i) top = max(top, part[i]);
-    job.row[row] = (short)top;
   }
+  if (at == 0) job.row[row] = (short)top;
 }
 
 // Sizes of the columns behind it, W columns per block and 1024 / W rows at a time.
@@ -308,6 +330,8 @@ grad_cols_kernel(const GradSizes* __restrict__ jobs, int njobs,
 
 // A row by a warp: its largest value, then (the row is in the L1 cache) the
 // scaled terms.  Bound by HBM: 4 bytes read and 4 written per element.
+// INV: exponents of any size (those of the gradient's columns are 126 at most).
+template <bool INV>
 __device__ __forceinline__ void pack_row(const PackRow& job, int row,
                                          int lane) {
   const int cols = job.cols;
@@ -347,10 +371,11 @@ __device__ __forceinline__ void pack_row(const PackRow& job, int row,
   };
   // Factors and the scaled row inside the range of fp32 with 2^60 to spare below
   // (what is left of a value under that is less than its terms hold): one
-  // multiplication for the column and one for the row.  With the exponents
-  // added up for every element a call on 1024 x 2048 took 87 us, now 7x.
+  // multiplication for the column and one for the row, and not the exponents
+  // added up for every element.
+  const unsigned unit = (unsigned)sign << 23;
   auto factor = [&](int e) {
-    return __uint_as_float(0x3f800000u + (unsigned)((sign * e) << 23));
+    return __uint_as_float(0x3f800000u + (unsigned)e * unit);
   };
   unsigned widest = 0;
   float peak = 0.f;
@@ -361,13 +386,14 @@ __device__ __forceinline__ void pack_row(const PackRow& job, int row,
   for (int k = k0; k < k0 + 512; k += 128) {
     const float4 x = load(k);
     const short4 e = load_exp(k);
-    widest = max(max(max(widest, (unsigned)abs(e.x)), (unsigned)abs(e.y)),
-                 max((unsigned)abs(e.z), (unsigned)abs(e.w)));
+    if (INV)
+      widest = max(max(max(widest, (unsigned)abs(e.x)), (unsigned)abs(e.y)),
+                   max((unsigned)abs(e.z), (unsigned)abs(e.w)));
     peak = fmaxf(fmaxf(peak, fmaxf(fabsf(x.x * factor(e.x)),
                                    fabsf(x.y * factor(e.y)))),
                  fmaxf(fabsf(x.z * factor(e.z)), fabsf(x.w * factor(e.w))));
   }
-  widest = __reduce_max_sync(0xffffffffu, widest);
+  if (INV) widest = __reduce_max_sync(0xffffffffu, widest);
   const unsigned bits =
       __reduce_max_sync(0xffffffffu, __float_as_uint(peak));
   int top = (int)(bits >> 23) - 127, s;
@@ -383,7 +409,7 @@ __device__ __forceinline__ void pack_row(const PackRow& job, int row,
       const short4 e = load_exp(k);
       const float y0 = x.x * factor(e.x) * f, y1 = x.y * factor(e.y) * f;
       const float y2 = x.z * factor(e.z) * f, y3 = x.w * factor(e.w) * f;
-      sum += y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3;
+      if (!INV) sum += y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3;
       if (k < 32 * nkb) store(k, y0, y1, y2, y3);
     }
   } else {
@@ -409,19 +435,21 @@ __device__ __forceinline__ void pack_row(const PackRow& job, int row,
       const float y1 = scale_exp(x.y, s + sign * e.y);
       const float y2 = scale_exp(x.z, s + sign * e.z);
       const float y3 = scale_exp(x.w, s + sign * e.w);
-      sum += y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3;
+      if (!INV) sum += y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3;
       store(k, y0, y1, y2, y3);
     }
+  }
+  if (INV) {
+    if (lane == 0) job.exp[row] = (short)-s;
+    return;
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   if (lane == 0) {
     // sum < 2^(f + 1), its root at most 2^n (rounding of the sum: far inside
     // the factor of two that fp16 has left above 2^15)
     const int n = sum == 0.f ? 0 : (exp_of(sum) + 2) >> 1;
-    job.exp[row] = (short)(job.fit == nullptr ? -s
-                           : sum == 0.f      ? kNoExp
-                                             : n - s);
-    if (job.fit != nullptr) job.fit[row] = scale_exp(job.gain, -n);
+    job.exp[row] = (short)(sum == 0.f ? kNoExp : n - s);
+    job.fit[row] = scale_exp(job.gain, -n);
   }
 }
 
@@ -439,7 +467,10 @@ pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
   f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
   const PackRows job = all[f];
   wait_for_launch_before();
-  pack_row(job, row_all - job.row_begin, lane);
+  if (job.fit != nullptr)
+    pack_row<false>(job, row_all - job.row_begin, lane);
+  else
+    pack_row<true>(job, row_all - job.row_begin, lane);
 }
 
 // A row of G_inv, of all layers' in a launch of the first product.
@@ -456,7 +487,7 @@ __device__ __noinline__ void pack_inverse(const GemmDesc* all, int n,
   job.dst = g.inv_pack;
   job.exp = g.inv_exp; job.fit = nullptr; job.gain = 0.f;
   job.cols = g.M;
-  pack_row(job, row_all - (int)g.inv_begin, lane);
+  pack_row<true>(job, row_all - (int)g.inv_begin, lane);
 }
 
 // MODE 0: the products of the inverse; 1, 2: first and second product of the
@@ -474,7 +505,7 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
   PackedControl* ctl =
       reinterpret_cast<PackedControl*>(smem + STAGES * KP_STAGE);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // First product: the rows of G_inv, which the next launch needs, are packed by
+  // First product: the rows of G_inv, which the next launch needs, may be packed by
   // `inv_ctas` CTAs in front of the tiles (on SMs without one) and by the
   // epilogue's warps while the MMAs run.  us in a launch of its own, in CTAs
   // only, by the epilogues only: 512 x 512 +3.5, 40, 46; 1024 x 2048 +4, 87, 79.
@@ -853,10 +884,18 @@ int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
 }
 
 int launch_packed_precond(const GemmDesc* descs_dev, const GemmDesc* descs_host,
-                          int ndesc, int total_tiles, int inv_rows, float lr,
-                          float momentum, cudaStream_t stream) {
-  return launch_mode(inv_rows > 0 ? 1 : 2, descs_dev, descs_host, ndesc,
-                     total_tiles, inv_rows, lr, momentum, stream);
+                          int ndesc, int total_tiles, bool last, int inv_rows,
+                          float lr, float momentum, cudaStream_t stream) {
+  return launch_mode(last ? 2 : 1, descs_dev, descs_host, ndesc, total_tiles,
+                     inv_rows, lr, momentum, stream);
+}
+
+// One wave of tiles, and no warp with more than one row: else the rows hold up the
+// tiles (54 pairs of ResNet-50: 4413 us with a launch of their own, 4565 without).
+bool packed_takes_rows(int total_tiles, int rows) {
+  const int free = sm_count() - total_tiles;
+  return free >= 0 &&
+         rows <= free * (KP_THREADS / 32) + total_tiles * KP_EPI_WARPS;
 }
 
 int launch_grad_sizes(const GradSizes* jobs_dev, const GradSizes* jobs_host,
@@ -869,8 +908,11 @@ int launch_grad_sizes(const GradSizes* jobs_dev, const GradSizes* jobs_host,
     inl.n = njobs;
     std::copy(jobs_host, jobs_host + njobs, inl.j);
   }
-  const int rc = launch_behind("grad_rows_kernel", false, grad_rows_kernel, rows,
-                               256, 0, stream, jobs_dev, njobs, inl);
+  const bool many = rows > 8 * sm_count();
+  const int rc = launch_behind(
+      "grad_rows_kernel", false, many ? grad_rows_kernel<1> : grad_rows_kernel<8>,
+      many ? (int)ceil_div(rows, 8) : rows, 256, 0, stream, jobs_dev, njobs, rows,
+      inl);
   if (rc != KFAC_OK) return rc;
   return launch_behind("grad_cols_kernel", true,
                        wide ? grad_cols_kernel<32> : grad_cols_kernel<8>, groups,
