@@ -47,20 +47,25 @@ static ChunkLayout chunk_layout(int dG, int dA) {
   return c;
 }
 
-// Whether a call goes through chunks: it costs a launch more, a k-block 0.4 us
-// instead of 0.75, or of 1.05 where the tile kernel cannot load 16-byte words.
-// The longest layer decides, by its k-blocks in both products.  us in tiles and
-// in chunks: 512 x 512 (32 k-blocks) 41 33, 512 x 4608 165 132; with odd sides 301
-// x 785 (35) 64 47, 1000 x 10 (33) 49 30, 1000 x 1001 102 58; and below the line,
-// 4 us for a memset included that the chunks no longer need, 256 x 256 (16) 27 33,
-// 128 x 512 (20) 30 35, 53 x 334 (13) 30 33, 211 x 130 (12) 33 33.
+// Whether a call goes through chunks, by its longest layer: three launches more than
+// in tiles, but a k-block costs 0.4 us instead of 0.6 - 0.9, or of up to 1.5 where
+// the tile kernel cannot load 16-byte words of A_inv and has to append a bias
+// column.  k-blocks of the sum over rows count twice: the tile kernel has more
+// tiles there, and chunks of a long A_inv cost more to make.  us in tiles and in
+// chunks, by 2 kb(dG) + kb(dA):
+//   words: 256 x 256 (24) 26 31, 256 x 768 (40) 38 39, 448 x 448 (42) 36 38, 128 x
+//     1152 (44) 43 45, 512 x 512 (48) 40 38, 256 x 1024 (48) 45 43, 64 x 2304 (76)
+//     62 62, 512 x 4608 (176) 163 138;
+//   odd: 189 x 189 (18) 33 40, 253 x 253 (24) 39 41, 317 x 317 (30) 43 43, 64 x 801
+//     (30) 47 46, 95 x 855 (33) 54 47, 509 x 509 (48) 59 47;
+//   with a bias: 64 x 147 (9) 21 36, 53 x 333 (15) 31 37, 64 x 400 (17) 30 30, 200 x
+//     100 (18) 33 31, 10 x 500 (18) 31 30, 200 x 200 (21) 34 31, 400 x 64 (29) 36 30.
 static bool chunks_pay(int count, const int* dG, const int* dW,
                        const std::vector<int>& hb) {
   for (int i = 0; i < count; ++i) {
     const int dA = dW[i] + hb[i];
-    const int blocks = (dA + 31) / 32 + (dG[i] + 31) / 32;
-    const bool words = ((dG[i] | dW[i] | hb[i]) & 3) == 0;
-    if (blocks >= (words ? 32 : 20)) return true;
+    const int line = hb[i] ? 18 : (dA & 3) != 0 ? 30 : 45;
+    if (2 * ((dG[i] + 31) / 32) + (dA + 31) / 32 >= line) return true;
   }
   return false;
 }

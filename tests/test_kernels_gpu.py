@@ -782,7 +782,8 @@ def test_precondition_tile_variants(ops, shapes):
     (512, 512, False, 0, 1.0), (33, 640, True, 0, 1e-18),
     (1, 1024, False, 0, 1e12), (640, 5, True, 1, 1.0),
     (300, 1023, True, 0, 1e12), (129, 897, False, 1, 1e-18),
-    (257, 1000, False, 2, 1.0), (1025, 255, True, 3, 1e-18)])
+    (257, 1000, False, 2, 1.0), (1025, 255, True, 3, 1e-18),
+    (1, 2048, False, 0, 1e12)])
 def test_precondition_of_long_layers(ops, dG, dW, bias, offset, magnitude):
     """Long enough for operands in chunks: cut tiles and k-blocks, the bias as an
     appended column, parameters at odd addresses, gradient rows of different
@@ -860,7 +861,7 @@ def _inverse_of(rng, d, scale, damping):
     return np.linalg.inv(x.T @ x / (2 * d) + damping * np.eye(d))
 
 
-@pytest.mark.parametrize('dG,dW,bias', [(64, 1024, False), (300, 785, True),
+@pytest.mark.parametrize('dG,dW,bias', [(64, 1600, False), (300, 785, True),
                                         (513, 511, False)])
 @pytest.mark.parametrize('small', [1e-4, 1e-8, 1e-12, 1e-30])
 def test_precondition_of_rows_of_any_scale(ops, dG, dW, bias, small):
@@ -868,7 +869,7 @@ def test_precondition_of_rows_of_any_scale(ops, dG, dW, bias, small):
     the other rows': half of the rows, all but one, rows spread evenly; G_inv
     nearly diagonal, so that a row of kf is as small as its gradient, and as the
     damped factor of such rows.  22-bit terms (2^-21 per operand) and sums of up
-    to 1024 + 513 terms, cut off towards zero: 1e-5."""
+    to 1600 + 64 terms, cut off towards zero: 1e-5."""
     rng = np.random.default_rng(dG + dW)
     dA = dW + int(bias)
     Ai = _inverse_of(rng, dA, 1.0, 1e-2)
@@ -886,7 +887,7 @@ def test_precondition_of_rows_of_any_scale(ops, dG, dW, bias, small):
     assert _worst(got, ref, 1) < 1e-5
 
 
-@pytest.mark.parametrize('dG,dW,bias', [(64, 1024, False), (300, 785, True),
+@pytest.mark.parametrize('dG,dW,bias', [(64, 1600, False), (300, 785, True),
                                         (513, 511, False)])
 @pytest.mark.parametrize('small', [1e-4, 1e-8, 1e-12])
 def test_precondition_of_features_of_any_scale(ops, dG, dW, bias, small):
