@@ -3,6 +3,7 @@
 // weight and bias parts and can apply the momentum update in place.  Larger
 // calls go through fp16 chunks (tc_packed.cu): a launch that writes the three
 // operands' rows as chunks, U = grad * A_inv^T, kf = G_inv * U.
+#include <algorithm>
 #include <vector>
 
 #include "gemm_simt.cuh"
@@ -47,6 +48,19 @@ static ChunkLayout chunk_layout(int dG, int dA) {
   return c;
 }
 
+// Tables in front of the layers' chunks: two products a layer, then these.
+struct ChunkTables {
+  size_t jobs, sizes, total;
+};
+
+static ChunkTables chunk_tables(int count) {
+  ChunkTables t;
+  t.jobs = align256(2 * (size_t)count * sizeof(GemmDesc));
+  t.sizes = t.jobs + align256(3 * (size_t)count * sizeof(PackRows));
+  t.total = t.sizes + align256((size_t)count * sizeof(GradSizes));
+  return t;
+}
+
 // Whether a call goes through chunks, by its longest layer: three launches more than
 // in tiles, but a k-block costs 0.4 us instead of 0.6 - 0.9, or of up to 1.5 where
 // the tile kernel cannot load 16-byte words of A_inv and has to append a bias
@@ -80,12 +94,9 @@ static int precondition_chunks(
     float* const* kf_b, float* const* param_W, float* const* param_b,
     float* const* mom_W, float* const* mom_b, float lr, float momentum, char* ws,
     cudaStream_t st) {
-  // tables, in front of the layers' chunks
-  const size_t jobs_at = align256(2 * (size_t)count * sizeof(GemmDesc));
-  const size_t sizes_at =
-      jobs_at + align256(3 * (size_t)count * sizeof(PackRows));
-  const size_t tables =
-      sizes_at + align256((size_t)count * sizeof(GradSizes));
+  const ChunkTables at_table = chunk_tables(count);
+  const size_t jobs_at = at_table.jobs, sizes_at = at_table.sizes;
+  const size_t tables = at_table.total;
   std::vector<char> host(tables, 0);
   GemmDesc* descs = reinterpret_cast<GemmDesc*>(host.data());
   PackRows* jobs = reinterpret_cast<PackRows*>(host.data() + jobs_at);
@@ -197,19 +208,28 @@ static int precondition_chunks(
   return rc;
 }
 
+static size_t tile_workspace(int count, const int* dG, const int* dW,
+                             const std::vector<int>& hb) {
+  size_t total = align256(2 * (size_t)count * sizeof(GemmDesc));
+  for (int i = 0; i < count; ++i)
+    total += align256((size_t)dG[i] * (dW[i] + hb[i]) * sizeof(float));
+  return total;
+}
+
+// The chunks, or T of the tile kernel where the call goes that way (and for a
+// workspace at an odd address and the FFMA engine, which take nothing else).
 extern "C" size_t kfac_precond_workspace_bytes(int count, const int* dG,
                                                const int* dW,
                                                const int* has_bias) {
   if (count <= 0 || !dG || !dW) return 0;
-  size_t total = align256(2 * (size_t)count * sizeof(GemmDesc));
-  size_t chunks = total + align256(3 * (size_t)count * sizeof(PackRows)) +
-                  align256((size_t)count * sizeof(GradSizes));
-  for (int i = 0; i < count; ++i) {
-    size_t dA = (size_t)dW[i] + ((has_bias && has_bias[i]) ? 1 : 0);
-    total += align256((size_t)dG[i] * dA * sizeof(float));
-    chunks += chunk_layout(dG[i], (int)dA).total;
-  }
-  return total > chunks ? total : chunks;
+  std::vector<int> hb(count, 0);
+  for (int i = 0; i < count; ++i) hb[i] = has_bias && has_bias[i] ? 1 : 0;
+  const size_t tiles = tile_workspace(count, dG, dW, hb);
+  if (!chunks_pay(count, dG, dW, hb)) return tiles;
+  size_t chunks = chunk_tables(count).total;
+  for (int i = 0; i < count; ++i)
+    chunks += chunk_layout(dG[i], dW[i] + hb[i]).total;
+  return std::max(chunks, tiles);
 }
 
 extern "C" int kfac_precondition(

@@ -57,6 +57,24 @@ def test_pure_host_entry_points(lib):
         lib.kfac_set_factor_staging(0)
 
 
+def test_workspace_of_a_preconditioning_is_what_its_route_takes(lib):
+    """Short layers need one product in fp32 and the tables, not the chunks of
+    longer calls (8 bytes per element and more)."""
+    from chainerkfac_b200 import _lib
+
+    def need(*layers):
+        return lib.kfac_precond_workspace_bytes(
+            len(layers), *(_lib.int_array([l[k] for l in layers])
+                           for k in range(3)))
+    short = [(64, 256, 0), (100, 40, 1), (256, 64, 0)]
+    product = sum(-(-4 * g * (w + b) // 256) * 256 for g, w, b in short)
+    assert product <= need(*short) <= product + 4096
+    for g, w, b in ((512, 4608, 0), (300, 785, 1)):
+        d = w + b
+        assert need((g, w, b)) >= 4 * (d * d + g * g + 2 * g * d)
+    assert need((512, 4608, 0), *short) > need((512, 4608, 0)) + product
+
+
 def test_workspace_of_grouped_factors_is_bounded(lib):
     """However many factors a grouped build has, wide ones with many partial
     tiles each or narrow ones with long contractions: one batch's planes and
