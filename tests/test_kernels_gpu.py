@@ -756,10 +756,10 @@ def precond_case(rng, dG, dW, bias):
     [(128, 256, False), (64, 60, False)],            # 16-byte rows, few tiles
     [(33, 31, True), (129, 257, False), (5, 3, True)],   # none of them
     [(1024, 1152, False), (512, 1000, True), (260, 2048, False),
-     (301, 785, True)],          # both, more tiles than SMs: two launches
+     (301, 785, True)],          # both: long layers, in chunks
 ])
 def test_precondition_tile_variants(ops, shapes):
-    """Narrow and wide tiles, operands read as 16-byte words and float by
+    """Narrow tiles and chunks, operands read as 16-byte words and float by
     float, cut rows, columns and contractions, the appended bias column."""
     rng = np.random.default_rng(31)
     cases = [precond_case(rng, *s) for s in shapes]
@@ -776,6 +776,47 @@ def test_precondition_tile_variants(ops, shapes):
         got = host(w) if b is None else np.concatenate(
             [host(w), host(b)[:, None]], 1)
         assert rel(got, ref) < 2e-5     # TF32 pairs and fp32 sums: < 1e-5
+
+
+@pytest.mark.parametrize('fused', [False, True])
+def test_precondition_of_many_short_layers(ops, fused):
+    """Layers that are all short, of whole 16-byte words and not, with more tiles
+    than SMs: 256 columns a tile and a launch for each kind; kf alone and with the
+    momentum update (to the roundings of its three operations)."""
+    rng = np.random.default_rng(37)
+    shapes = [(384, 384, False), (384, 380, False), (256, 512, False)] * 6 + \
+        [(255, 255, False), (129, 96, True), (253, 257, False)] * 6
+    cases = [precond_case(rng, *s) for s in shapes]
+    Gi, Ai, gW = ([dev(c[k]) for c in cases] for k in range(3))
+    gb = [None if c[3] is None else dev(c[3]) for c in cases]
+    kW = [torch.empty_like(t) for t in gW]
+    kb = [None if t is None else torch.empty_like(t) for t in gb]
+    update = []
+    if fused:
+        pW, vW = ([dev(rng.standard_normal(c[2].shape).astype(np.float32))
+                   for c in cases] for _ in range(2))
+        pb, vb = ([None if t is None else torch.full_like(t, x) for t in gb]
+                  for x in (1.0, 2.0))
+        old = [(host(p), host(v)) for p, v in zip(pW, vW)]
+        update = [pW, pb, vW, vb, 0.5, 0.9]
+    ops.precondition(Gi, Ai, gW, gb, kW, kb, *update)
+    for i, (c, w, b) in enumerate(zip(cases, kW, kb)):
+        g, got = c[2].astype(np.float64), host(w)
+        if b is not None:
+            g = np.concatenate([g, c[3].astype(np.float64)[:, None]], 1)
+            got = np.concatenate([got, host(b)[:, None]], 1)
+        ref = c[0].astype(np.float64) @ g @ c[1].astype(np.float64)
+        assert rel(got, ref) < 2e-5     # as above
+        if not fused:
+            continue
+        parts = [(got[:, :c[2].shape[1]], *old[i], pW[i], vW[i])]
+        if b is not None:
+            parts.append((got[:, -1], 1.0, 2.0, pb[i], vb[i]))
+        for kf, p, v, p_new, v_new in parts:
+            v = 0.9 * v - 0.5 * kf.astype(np.float64)
+            scale = np.abs(v).max()
+            assert np.abs(host(v_new) - v).max() < 2.0 ** -22 * (scale + 4.0)
+            assert np.abs(host(p_new) - p - v).max() < 2.0 ** -22 * (scale + 8.0)
 
 
 @pytest.mark.parametrize('dG,dW,bias,offset,magnitude', [
