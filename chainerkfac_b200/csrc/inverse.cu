@@ -262,16 +262,16 @@ __device__ __forceinline__ void cp_async16(unsigned dst, const float* src) {
 }
 
 // W_kk (bs x bs) into S; beyond bs the identity, so that the sweeps below run
-// over whole sub-blocks.  Asynchronous where the rows are 16-byte aligned:
-// the caller waits (diag_load_wait) before its next barrier.
+// over whole sub-blocks.  Asynchronous: the caller waits (diag_load_wait) before
+// its next barrier.
 __device__ __forceinline__ void diag_load(const float* Wd, long long ld, int bs,
-                                          bool vec, float* S) {
+                                          float* S) {
   const int rows = (bs + SB - 1) / SB * SB;
   for (int idx = threadIdx.x; idx < rows * (DB / 4); idx += DT) {
     const int r = idx >> 5, c = (idx & 31) * 4;
     float* dst = &S[r * DLD + c];
     if (c > (r | (SB - 1))) continue;       // above the diagonal: never read
-    if (vec && r < bs && c + 3 < bs) {
+    if (r < bs && c + 3 < bs) {
       cp_async16(smem_u32(dst), &Wd[r * ld + c]);
     } else {
 #pragma unroll
@@ -322,7 +322,7 @@ __device__ __forceinline__ void look_begin(LookControl* ctl) {
 // With TF32 terms, twice the MMA time and shared memory for two k-blocks at a
 // time, the whole kernel took 31.7 us on average of a plan of 856 rows, now 29.6.
 __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
-                                               bool vec, float* S,
+                                               float* S,
                                                unsigned char* stage,
                                                LookControl* ctl) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -342,18 +342,13 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
       va[kb][j] = vx[kb][j] = make_float4(0.f, 0.f, 0.f, 0.f);
       const float* pa = &Ap[row * ld + col];
       const float* px = &Xp[row * ld + col];
-      if (vec) {
-        if (row < bs) va[kb][j] = *reinterpret_cast<const float4*>(pa);
-        if (row >= 32 * kb) vx[kb][j] = *reinterpret_cast<const float4*>(px);
-      } else {
-        if (row < bs) va[kb][j] = make_float4(pa[0], pa[1], pa[2], pa[3]);
-        if (row >= 32 * kb) vx[kb][j] = make_float4(px[0], px[1], px[2], px[3]);
-      }
+      if (row < bs) va[kb][j] = *reinterpret_cast<const float4*>(pa);
+      if (row >= 32 * kb) vx[kb][j] = *reinterpret_cast<const float4*>(px);
     }
   }
   look_begin(ctl);
   // W_kk into S (the update is subtracted from it at the end)
-  diag_load(mi.W + (long long)o * ld + o, ld, bs, vec, S);
+  diag_load(mi.W + (long long)o * ld + o, ld, bs, S);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -839,13 +834,10 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
   const int bs = min(DB, mi.d - o);
   const int np = (bs + SB - 1) / SB;      // sub-blocks in use
   const long long ld = mi.ld;
-  const bool vec = ((reinterpret_cast<uintptr_t>(mi.W) |
-                     reinterpret_cast<uintptr_t>(mi.V) |
-                     reinterpret_cast<uintptr_t>(mi.X)) & 15) == 0;
   if (LOOK) {
-    if (!diag_lookahead(mi, o, bs, vec, sm.S, stage, ctl)) return;
+    if (!diag_lookahead(mi, o, bs, sm.S, stage, ctl)) return;
   } else {
-    diag_load(mi.W + (long long)o * ld + o, ld, bs, vec, sm.S);
+    diag_load(mi.W + (long long)o * ld + o, ld, bs, sm.S);
     diag_load_wait();
   }
   __syncthreads();
@@ -920,26 +912,6 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
   // 16-byte word per lane) into four contiguous row pieces.  The part above
   // the diagonal sub-blocks was zeroed when the plan was made.
   float* Xd = mi.X + (long long)o * ld + o;
-  if (!vec) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = 4 * warp + 64 * h, bi = r >> 5;
-      if (r >= bs) break;
-      for (int u = 0; u <= bi; ++u) {
-        const float4 v = *reinterpret_cast<const float4*>(
-            u == bi ? &sm.XD[u][lane * SLP + (r & (SB - 1))]
-                    : &sm.S[(SB * u + lane) * DLD + r]);
-        const int c = SB * u + lane;
-        if (c >= bs) continue;
-        float* dst = Xd + r * ld + c;
-        dst[0] = v.x;
-        if (r + 1 < bs) dst[ld] = v.y;
-        if (r + 2 < bs) dst[2 * ld] = v.z;
-        if (r + 3 < bs) dst[3 * ld] = v.w;
-      }
-    }
-    return;
-  }
   // (from X and d: two more pointers across the chain cost registers that it
   // does not have)
   const long long ptile =
@@ -1291,8 +1263,10 @@ static size_t chunk_bytes(int d) {
   return (size_t)((d + DB - 1) / DB) * chunk_tile_bytes(d);
 }
 
+// (the matrices begin at a multiple of 256 bytes, wherever the workspace does)
 extern "C" size_t kfac_inverse_workspace_bytes(int count, const int* dims) {
-  size_t total = 0;
+  if (count <= 0) return 0;
+  size_t total = 255;
   for (int i = 0; i < count; ++i) {
     if (dims[i] <= 0) return 0;
     total += 3 * matrix_bytes(dims[i]) +             // W, X, V
@@ -1332,12 +1306,13 @@ extern "C" int kfac_inverse_plan_create(
   // zeros by the wide tiles of the triangular-inverse products.
   KFAC_CUDA(cudaMemset(workspace, 0, need));
   const bool use_tc = engine() == 1;
-  // fp16 terms: every operand of the products has rows of 16-byte words
-  const int half =
-      use_tc && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 ? G_HALF : 0;
-  const int packed = half ? G_PACKED : 0;
+  // the tensor-core engine: operands in fp16 terms, in chunks where they are read
+  // more than once
+  const int half = use_tc ? G_HALF : 0;
+  const int packed = use_tc ? G_PACKED : 0;
   std::vector<MatInfo> mats(count);
-  char* ws = static_cast<char*>(workspace);
+  char* ws = reinterpret_cast<char*>(
+      (reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255);
   int dmax = 0;
   for (int i = 0; i < count; ++i) {
     MatInfo& m = mats[i];

@@ -742,6 +742,56 @@ def test_inverse_of_a_non_finite_factor_is_not_finite(ops, value, d, row, col):
     plan.close()
 
 
+def _inverse_in(ops, F, offset):
+    """Inverses by a plan whose workspace begins `offset` bytes behind a multiple
+    of 256."""
+    import ctypes
+    from chainerkfac_b200 import _lib
+    lib = _lib.load()
+    n, inv = len(F), [torch.zeros_like(f) for f in F]
+    dims = _lib.int_array([f.shape[0] for f in F])
+    need = lib.kfac_inverse_workspace_bytes(n, dims)
+    ws = torch.empty(need + 512, dtype=torch.uint8, device='cuda')
+    ptr = (ws.data_ptr() + 255) // 256 * 256 + offset
+    info = torch.zeros(n, dtype=torch.int32, device='cuda')
+    diag = torch.zeros(n, dtype=torch.float32, device='cuda')
+    plan = ctypes.c_void_p()
+    _lib.check(lib.kfac_inverse_plan_create(
+        n, dims, _lib.ptr_array([f.data_ptr() for f in F]),
+        _lib.ptr_array([f.data_ptr() for f in inv]), _lib.int_array([-1] * n),
+        _lib.int_array([2] * n), _lib.float_array([0.0] * n),
+        _lib.float_array([1.0] * n), ctypes.c_void_p(ptr), need,
+        ctypes.byref(plan)), 'kfac_inverse_plan_create')
+    try:
+        _lib.check(lib.kfac_inverse_plan_run(
+            plan, 1e-2, 0, ctypes.c_void_p(info.data_ptr()),
+            ctypes.c_void_p(diag.data_ptr()), ops._stream()), 'run')
+        torch.cuda.synchronize()
+    finally:
+        lib.kfac_inverse_plan_destroy(plan)
+    assert not info.any()
+    return inv
+
+
+def test_inverse_does_not_depend_on_where_its_workspace_begins(ops):
+    rng = np.random.default_rng(8)
+    F = [dev(spd(rng, d)) for d in (40, 130, 700, 1500)]
+    want = _inverse_in(ops, F, 0)
+    for offset in (4, 16, 252):
+        for a, b in zip(_inverse_in(ops, F, offset), want):
+            assert torch.equal(a, b)
+
+
+def test_inverse_without_look_ahead(ops, monkeypatch):
+    """The chain as one stream of launches, each waiting for the one before."""
+    monkeypatch.setenv('KFAC_INVERSE_LOOKAHEAD', '0')
+    rng = np.random.default_rng(9)
+    host_f = [spd(rng, d) for d in (40, 130, 700, 1500)]
+    for f, inv in zip(host_f, _inverse_in(ops, [dev(f) for f in host_f], 0)):
+        want = np.linalg.inv(f.astype(np.float64) + 1e-2 * np.eye(len(f)))
+        assert rel(host(inv), want) < INVERSE_TOL
+
+
 # ------------------------------------------------------------- precondition
 def precond_case(rng, dG, dW, bias):
     dA = dW + int(bias)
