@@ -121,11 +121,10 @@ __device__ __forceinline__ unsigned long long tc_smem_desc_mn(unsigned addr,
   return d;
 }
 
-// D = f32, A = B = f16, M = m (256: a pair of CTAs), N = n
-__device__ __forceinline__ unsigned tc_half_desc(int n, bool a_mn, bool b_mn,
-                                                 int m = TC_BM) {
+// D = f32, A = B = f16, M = 128, N = n
+__device__ __forceinline__ unsigned tc_half_desc(int n, bool a_mn, bool b_mn) {
   return (1u << 4) | ((unsigned)a_mn << 15) | ((unsigned)b_mn << 16) |
-         ((unsigned)(n >> 3) << 17) | ((unsigned)(m >> 4) << 24);
+         ((unsigned)(n >> 3) << 17) | ((unsigned)(TC_BM >> 4) << 24);
 }
 
 __device__ __forceinline__ void tc_mma_half(unsigned tmem_d,

@@ -1,6 +1,6 @@
 // Epilogue of the tile kernel (tc_tile.cu): 32 x 32 pieces of the accumulators
-// TMEM -> registers -> shared memory -> global rows, with the update of C,
-// mirrored rows, fp16 chunks of the result and the preconditioning update.
+// TMEM -> registers -> shared memory -> global rows (C = alpha A B), with mirrored
+// rows, fp16 chunks of the result and the preconditioning update.
 #pragma once
 
 #include "gemm_simt.cuh"
@@ -171,9 +171,7 @@ __device__ __forceinline__ void tile_epilogue(const GemmDesc& g,
   const int row0 = q * 32, rows = min(32, m_valid - row0);
   const bool lower = (flags & G_LOWER) != 0;
   const float alpha = g.alpha;
-  const float beta = (g.beta_until > 0 && m0 >= g.beta_until) ? 0.f : g.beta;
   float* C = g.C;
-  const float* un = g.unscale;
   const bool pack = g.pack_kind != PACK_NONE;
   const long long ldc = g.ldc;
   // rows of a piece as 16-byte words: lane -> row 4 i + lane / 8, word lane % 8
@@ -181,21 +179,11 @@ __device__ __forceinline__ void tile_epilogue(const GemmDesc& g,
                    (reinterpret_cast<uintptr_t>(C) & 15) == 0;
   const int sub = lane >> 3, wc = 4 * (lane & 7);
   // Pieces whose 32 rows and columns are all stored, in whole words, take a path
-  // without a test per row: eight loads, then eight stores, in flight together.
+  // without a test per row.
   auto whole = [&](int c0) {
     return vec && rows == 32 && c0 + 32 <= n_valid &&
            (!lower || n0 + c0 + 31 <= m0 + row0);
   };
-  float4 old[8];
-  auto prefetch = [&](int c0) {
-    if constexpr (PRE) return;
-    if (beta == 0.f || !whole(c0)) return;
-    const float* p = C + (long long)(m0 + row0 + sub) * ldc + n0 + c0 + wc;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      old[i] = *reinterpret_cast<const float4*>(p + 4 * i * ldc);
-  };
-  prefetch(32 * h);
   bool ok = true;
   if (!zero) {
     ok = wait();
@@ -211,32 +199,14 @@ __device__ __forceinline__ void tile_epilogue(const GemmDesc& g,
                      o.lr, o.momentum);
     } else if (whole(c0)) {
       const int gc = n0 + c0 + wc;
-      float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (un != nullptr) sc = *reinterpret_cast<const float4*>(&un[gc]);
 #pragma unroll
       for (int i0 = 0; i0 < 8; i0 += 4) {
         const int gr = m0 + row0 + sub + 4 * i0;
-        float* pp = &piece[(4 * i0 + sub) * TT_EP + wc];
+        const float* pp = &piece[(4 * i0 + sub) * TT_EP + wc];
         float4 x[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           x[i] = *reinterpret_cast<const float4*>(&pp[4 * i * TT_EP]);
-        if (un != nullptr) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float sr = un[gr + 4 * i];
-            x[i].x = x[i].x * sr * sc.x; x[i].y = x[i].y * sr * sc.y;
-            x[i].z = x[i].z * sr * sc.z; x[i].w = x[i].w * sr * sc.w;
-          }
-        }
-        if (beta != 0.f) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float4 y = old[i0 + i];
-            x[i].x += beta * y.x; x[i].y += beta * y.y;
-            x[i].z += beta * y.z; x[i].w += beta * y.w;
-          }
-        }
         if (pack) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) pack_store4(g, gr + 4 * i, gc, x[i]);
@@ -247,15 +217,8 @@ __device__ __forceinline__ void tile_epilogue(const GemmDesc& g,
           for (int i = 0; i < 4; ++i)
             *reinterpret_cast<float4*>(C + idx + 4 * i * ldc) = x[i];
         }
-        if ((flags & G_MIRROR) && (beta != 0.f || un != nullptr)) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<float4*>(&pp[4 * i * TT_EP]) = x[i];
-        }
       }
-      prefetch(c0 + 32 * G);
       if (flags & G_MIRROR) {
-        __syncwarp();
         // a row per lane, so that a column of the piece is a contiguous store
         float* dst = C + (long long)(n0 + c0) * ldc + m0 + row0 + lane;
 #pragma unroll
@@ -274,24 +237,9 @@ __device__ __forceinline__ void tile_epilogue(const GemmDesc& g,
         const int r = row0 + 4 * i + sub, c = c0 + wc;
         const int gr = m0 + r;
         const int cend = lower ? min(n_valid, gr - n0 + 1) : n_valid;
-        float4 x =
+        const float4 x =
             *reinterpret_cast<const float4*>(&piece[(4 * i + sub) * TT_EP + wc]);
-        if (un != nullptr) {
-          // (rows and words past the matrix: inside the vector's padding)
-          const float sr = un[gr];
-          const float4 sc = *reinterpret_cast<const float4*>(&un[n0 + c]);
-          x.x = x.x * sr * sc.x; x.y = x.y * sr * sc.y;
-          x.z = x.z * sr * sc.z; x.w = x.w * sr * sc.w;
-        }
         const long long idx = (long long)gr * ldc + n0 + c;
-        if (beta != 0.f && r < m_valid) {
-          if (c < n_valid) x.x += beta * C[idx];
-          if (c + 1 < n_valid) x.y += beta * C[idx + 1];
-          if (c + 2 < n_valid) x.z += beta * C[idx + 2];
-          if (c + 3 < n_valid) x.w += beta * C[idx + 3];
-        }
-        if ((beta != 0.f || un != nullptr) && (flags & G_MIRROR))
-          *reinterpret_cast<float4*>(&piece[(4 * i + sub) * TT_EP + wc]) = x;
         if (r >= m_valid || c >= cend) continue;
         // (packed results have whole words only)
         if (pack) pack_store4(g, gr, n0 + c, x);
@@ -305,11 +253,8 @@ __device__ __forceinline__ void tile_epilogue(const GemmDesc& g,
             if (c + e < cend) C[idx + e] = xs[e];
         }
       }
-      prefetch(c0 + 32 * G);
       if (flags & G_MIRROR) {
-        // the final values are in the piece; a row per lane, so that a
-        // column of the piece is a contiguous store
-        __syncwarp();
+        // a row per lane, so that a column of the piece is a contiguous store
         const int gr = m0 + row0 + lane;
         if (lane < rows) {
           float* dst = C + (long long)(n0 + c0) * ldc + gr;

@@ -110,7 +110,7 @@ __host__ __device__ __forceinline__ bool tile_operand_vec(const Operand& op) {
 // of the side (units past them stay idle: their rows are never stored).
 template <bool VEC>
 __device__ __forceinline__ void tile_unit_setup(const Operand& op, int r0,
-                                                int wu, int lane, int kbeg,
+                                                int wu, int lane,
                                                 int rows, unsigned side_off,
                                                 TileUnit& u) {
   const bool kf = op.kfast != 0;
@@ -123,7 +123,7 @@ __device__ __forceinline__ void tile_unit_setup(const Operand& op, int r0,
     u.flags |= U_EXTRA;
   if (!VEC) {
     const int row = kf ? first : first + lane;
-    u.k = kbeg + (kf ? lane : 16 * (wu & 1));
+    u.k = kf ? lane : 16 * (wu & 1);
     u.row = r0 + row;
     const int r = min(u.row, op.ncols - 1);
     u.last = op.ncols - 1 - r;
@@ -136,7 +136,7 @@ __device__ __forceinline__ void tile_unit_setup(const Operand& op, int r0,
   }
   if (kf) {
     const int chunk = lane & 7, row = first + (lane >> 3);
-    u.k = kbeg + 4 * chunk;
+    u.k = 4 * chunk;
     u.row = r0 + row;
     const int r = min(u.row, op.ncols - 1);
     u.last = op.ncols - 1 - r;
@@ -148,7 +148,7 @@ __device__ __forceinline__ void tile_unit_setup(const Operand& op, int r0,
   } else {
     const int kq = 4 * (wu & 1) + (lane & 3);
     const int row = first + 4 * (lane >> 2);
-    u.k = kbeg + 4 * kq;
+    u.k = 4 * kq;
     u.row = r0 + row;
     u.last = 0;
     // (whole words: the pitch covers the last one)
@@ -280,7 +280,7 @@ struct HalfUnit {
 
 // (a unit past the operand's last row reads that one again)
 __device__ __forceinline__ void half_unit_setup(const Operand& op, int r0,
-                                                int wu, int lane, int kbeg,
+                                                int wu, int lane,
                                                 int rows, unsigned side_off,
                                                 HalfUnit& u) {
   u.kf = op.kfast != 0;
@@ -288,7 +288,7 @@ __device__ __forceinline__ void half_unit_setup(const Operand& op, int r0,
   if (u.kf) {
     const int row = 16 * wu + 4 * (lane >> 3), chunk = lane & 7;
     u.live = 16 * wu < rows;
-    u.k = kbeg + 4 * chunk;
+    u.k = 4 * chunk;
     const int r = min(r0 + row, op.ncols - 1);
     u.p = op.base + (long long)r * ld + u.k;
 #pragma unroll
@@ -299,7 +299,7 @@ __device__ __forceinline__ void half_unit_setup(const Operand& op, int r0,
     const int group = wu >> 2, octet = wu & 3, kk = lane >> 4;
     const int row = 64 * group + 4 * (lane & 15);
     u.live = 64 * group < rows;
-    u.k = kbeg + 8 * octet + kk;
+    u.k = 8 * octet + kk;
     // (whole words: the pitch covers the last one)
     u.p = op.base + (long long)u.k * ld + min(r0 + row, (op.ncols - 1) & ~3);
 #pragma unroll
@@ -435,18 +435,12 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
   if (flags & G_LOWER) n_valid = min(n_valid, m0 + TC_BM - n0);
   const int n_inst = (n_valid + 15) & ~15;
   const int m_valid = min(TC_BM, g.M - m0);
-  int kbeg = 0, kend = (int)g.K;
-  if (flags & G_KBEG_N0) kbeg = max(kbeg, n0);
-  if (flags & G_KBEG_M0) kbeg = max(kbeg, m0 - g.kbeg_off);
+  int kend = (int)g.K;
   if (flags & G_KEND_M0) kend = min(kend, m0 + TC_BM);
   // a gated-off problem runs no k-blocks and stores nothing
   const bool gated_off = g.gate != nullptr && *g.gate == 0;
   const int nkb =
-      (kend > kbeg && !gated_off) ? (kend - kbeg + TT_BK - 1) / TT_BK : 0;
-  // X^T X on a diagonal tile: the tile's A rows are rows [m0 - n0, + 128) of
-  // its B rows, so only B is staged and the A descriptors point into it
-  const bool share_ab = (flags & G_SAME_AB) && (flags & G_LOWER) &&
-                        m0 >= n0 && m0 - n0 + TC_BM <= TN;
+      gated_off ? 0 : (kend + TT_BK - 1) / TT_BK;
 
   if (warp < Map::kWarps) {
     // ===================== producers =====================
@@ -460,23 +454,23 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
     const float scale1 = HALF ? g.sb : 1.f;
     {
       const int r0 = a0 ? m0 : n0, wu = a0 ? warp : warp - 8;
-      const int rows = a0 ? (share_ab ? 0 : m_valid) : n_valid;
+      const int rows = a0 ? m_valid : n_valid;
       const unsigned side = a0 ? 0 : Map::kABytes;
       if constexpr (HALF) {
-        half_unit_setup(op0, r0, wu, lane, kbeg, rows, side, u0);
+        half_unit_setup(op0, r0, wu, lane, rows, side, u0);
         if (Map::kTwo)
-          half_unit_setup(op1, n0, warp + Map::kWarps - 8, lane, kbeg, n_valid,
+          half_unit_setup(op1, n0, warp + Map::kWarps - 8, lane, n_valid,
                           Map::kABytes, u1);
       } else {
-        tile_unit_setup<VEC>(op0, r0, wu, lane, kbeg, rows, side, u0);
+        tile_unit_setup<VEC>(op0, r0, wu, lane, rows, side, u0);
         if (Map::kTwo)
-          tile_unit_setup<VEC>(op1, n0, warp + Map::kWarps - 8, lane, kbeg,
+          tile_unit_setup<VEC>(op1, n0, warp + Map::kWarps - 8, lane,
                                n_valid, Map::kABytes, u1);
       }
     }
     const unsigned base = smem_u32(smem);
     // blocks that end before kend (fp16 terms)
-    const int nfull = (kend - kbeg) / TT_BK;
+    const int nfull = kend / TT_BK;
     auto load = [&](int kb, float4* v) {
       if constexpr (HALF) {
         if (kb < nfull) {
@@ -569,8 +563,6 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
       // ===================== MMA issuer, fp16 terms =====================
       const bool ka = g.A.kfast != 0, kb_ = g.B.kfast != 0;
       const unsigned idesc = tc_half_desc(n_inst, !ka, !kb_);
-      const unsigned a_off =
-          share_ab ? (unsigned)(Map::kABytes + (m0 - n0) * 128) : 0u;
       // from the hi to the lo terms, and from 16 k to the next (16-byte units)
       const unsigned long long lo_a = (ka ? 64 : 4096) >> 4;
       const unsigned long long lo_b = (kb_ ? 64 : 4096) >> 4;
@@ -582,7 +574,7 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
                               &ctl->abort_flag, &g_tile_status))
           break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned sa = smem_u32(smem + s * Map::kStage) + a_off;
+        const unsigned sa = smem_u32(smem + s * Map::kStage);
         const unsigned sb = smem_u32(smem + s * Map::kStage) + Map::kABytes;
         unsigned long long a = ka ? tc_smem_desc(sa) : tc_smem_desc_mn(sa, 8192);
         unsigned long long b = kb_ ? tc_smem_desc(sb) : tc_smem_desc_mn(sb, 8192);
@@ -599,8 +591,6 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
     if (!HALF && elect_one()) {
       // ===================== MMA issuer =====================
       const unsigned idesc = tc_instr_desc(n_inst);
-      const unsigned a_off =
-          share_ab ? (unsigned)(Map::kABytes + (m0 - n0) * 128) : 0u;
       for (int kb = 0; kb < nkb; ++kb) {
         const int s = kb % Map::kStages;
         if (!mbar_wait_status(&ctl->full[s], (kb / Map::kStages) & 1,
@@ -608,9 +598,9 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
           break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const unsigned sa = smem_u32(smem + s * Map::kStage);
-        const unsigned long long a_hi = tc_smem_desc(sa + a_off);
+        const unsigned long long a_hi = tc_smem_desc(sa);
         const unsigned long long b_hi = tc_smem_desc(sa + Map::kABytes);
-        const unsigned long long a_lo = tc_smem_desc(sa + Map::kLo + a_off);
+        const unsigned long long a_lo = tc_smem_desc(sa + Map::kLo);
         const unsigned long long b_lo =
             tc_smem_desc(sa + Map::kLo + Map::kABytes);
 #pragma unroll
