@@ -679,16 +679,21 @@ def precondition(G_inv, A_inv, grad_W, grad_b, kf_W=None, kf_b=None,
     dG = _lib.int_array([g.shape[0] for g in G_inv])
     dW = _lib.int_array([w.numel() // w.shape[0] for w in grad_W])
     hb = _lib.int_array([0 if b is None else 1 for b in grad_b])
-    cols = []
+    cols, f32 = [], torch.float32
     for lst in (G_inv, A_inv, grad_W, grad_b, kf_W, kf_b, param_W, param_b,
                 mom_W, mom_b):
         if lst is None:
             cols.append(None)
             continue
+        ptrs = []
         for t in lst:
-            _chk(t, 'precondition argument')
-        cols.append(_lib.ptr_array([None if t is None else t.data_ptr()
-                                    for t in lst]))
+            if t is None:
+                ptrs.append(None)
+                continue
+            if not (t.is_cuda and t.dtype is f32 and t.is_contiguous()):
+                _chk(t, 'precondition argument')
+            ptrs.append(t.data_ptr())
+        cols.append(_lib.ptr_array(ptrs))
     nbytes = lib.kfac_precond_workspace_bytes(count, dG, dW, hb)
     # calls that may overlap on different streams pass different keys
     pool = _precond_ws.get(ws_key)
