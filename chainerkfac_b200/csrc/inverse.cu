@@ -1608,13 +1608,16 @@ extern "C" int kfac_inverse_plan_create(
   };
   // Whether a panel's steps also update the next one's first block column.  The
   // chain then goes on there without waiting for the near update, which only
-  // the second block needs (4608 rows beside 512: 1766 -> 1684 us); where the
-  // tiles fill the SMs anyway, the passes over that column only cost (108
-  // factors of ResNet-50, plans of 120, 309 and 225 row tiles: 4605 us without,
-  // 4650 in the first plan, 4690 in all).
+  // the second block needs.  us without and with, by row tiles, a plan by itself:
+  // 4608 rows (36) 1494 1420, 2 x 3400 (54) 1183 1088, 8 x 1024 (64) 414 405, 2 x 4608
+  // (72) 1835 1760, 4608 beside 6 x 1000 (84) 1554 1486, 5 x 2304 (90) 850 826, 6 x
+  // 2304 (108) 963 890, 16 x 1024 (128) 483 477.  Where plans run beside each
+  // other and fill the SMs, the passes over that column only cost (108 factors of
+  // ResNet-50, plans of 120, 309 and 225 row tiles: 4605 us without, 4650 in the
+  // first plan, 4690 in all); such plans are large.
   long long row_tiles = 0;
   for (int i = 0; i < count; ++i) row_tiles += (dims[i] + DB - 1) / DB;
-  const bool ahead = look && 2 * row_tiles <= sm_count();
+  const bool ahead = look && 4 * row_tiles <= 3 * sm_count();
   const int E = ahead ? DB : 0;
   int near_ev = -1;            // near updates of the panel before
   for (int co = 0; co < dmax; co += CW) {
