@@ -1,8 +1,8 @@
 // Preconditioning kf = G_inv * [grad_W, grad_b] * A_inv for all layers in two
 // grouped launches; the second launch's epilogue splits the result into the
 // weight and bias parts and can apply the momentum update in place.  Larger
-// calls go through fp16 chunks (tc_packed.cu): a launch that writes the three
-// operands' rows as chunks, U = grad * A_inv^T, kf = G_inv * U.
+// calls go through fp16 chunks (tc_packed.cu): sizes of the gradients' rows and
+// columns, operands' rows as chunks, U = grad * A_inv^T, kf = G_inv * U.
 #include <algorithm>
 #include <vector>
 

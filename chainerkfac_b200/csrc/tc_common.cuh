@@ -1,8 +1,8 @@
-// tcgen05 / mbarrier building blocks shared by the tile engine (tc_gemm.cu)
-// and the diagonal kernel of the inverse (inverse.cu): shared-memory and
-// instruction descriptors for K-major, 128-byte-swizzled fp32 (TF32) operand
-// tiles, MMA issue / commit, accumulator loads from tensor memory, bounded
-// barrier waits, and the splits of fp32 values into two TF32 or bf16 terms.
+// tcgen05 / mbarrier building blocks of the kernels on tensor cores: shared-memory
+// and instruction descriptors for 128-byte-swizzled operand tiles (TF32 K-major,
+// 16-bit values K- or MN-major), MMA issue / commit, accumulator loads from tensor
+// memory, bounded barrier waits, and the splits of fp32 values into two TF32, fp16
+// or bf16 terms.
 #pragma once
 
 #include <cuda_fp16.h>

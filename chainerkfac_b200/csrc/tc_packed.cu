@@ -373,10 +373,13 @@ __device__ __forceinline__ void pack_row(const PackRow& job, int row,
   // (what is left of a value under that is less than its terms hold): one
   // multiplication for the column and one for the row, and not the exponents
   // added up for every element.
+  // (a gradient row of zeros: any small factor of G_inv's column does)
   const unsigned unit = (unsigned)sign << 23;
   auto factor = [&](int e) {
+    if (INV) e = max(e, -126);
     return __uint_as_float(0x3f800000u + (unsigned)e * unit);
   };
+  auto width = [](int e) { return e == kNoExp ? 0u : (unsigned)abs(e); };
   unsigned widest = 0;
   float peak = 0.f;
   // (four loads in flight; zeros behind the end)
@@ -387,8 +390,8 @@ __device__ __forceinline__ void pack_row(const PackRow& job, int row,
     const float4 x = load(k);
     const short4 e = load_exp(k);
     if (INV)
-      widest = max(max(max(widest, (unsigned)abs(e.x)), (unsigned)abs(e.y)),
-                   max((unsigned)abs(e.z), (unsigned)abs(e.w)));
+      widest = max(max(max(widest, width(e.x)), width(e.y)),
+                   max(width(e.z), width(e.w)));
     peak = fmaxf(fmaxf(peak, fmaxf(fabsf(x.x * factor(e.x)),
                                    fabsf(x.y * factor(e.y)))),
                  fmaxf(fabsf(x.z * factor(e.z)), fabsf(x.w * factor(e.w))));

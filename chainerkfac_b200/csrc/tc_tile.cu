@@ -11,24 +11,21 @@
 //
 // One CTA owns a 128 x TN tile.  Producer warps load the operands from global
 // memory with 16-byte loads, one to three 32-k blocks ahead in registers, split them
-// and write the K-major, 128-byte-swizzled shared-memory layout that the MMA
-// descriptors expect; one more warp issues the MMAs.  The epilogue moves
-// 32 x 32 pieces of the accumulator TMEM -> registers -> shared memory ->
-// global rows (and, for symmetric outputs, mirrored rows straight from the
-// registers, where a column of a piece is contiguous).
+// and write the 128-byte-swizzled shared-memory layout that the MMA descriptors
+// expect (K-major; fp16 terms also MN-major, as they lie in memory); one more warp
+// issues the MMAs.  The epilogue (tc_epilogue.cuh) moves 32 x 32 pieces of the
+// accumulator TMEM -> registers -> shared memory -> global rows, mirrored rows or
+// fp16 chunks.
 //
-// Bound: long products by the loads and stores of their operands, not by the
-// MMAs (a 128 x 256 x 32 block 1600 ns with TF32 terms, the MMAs of it 810); the
-// many short ones (K = 128 inside a Cholesky panel) by latency: descriptor fetch, one trip to L2 per
-// register block, the epilogue's trip for C.  Hence the descriptors of small
-// launches travel as kernel arguments, C is prefetched before the accumulator
-// is waited for, and TN = 128 (half the work per CTA, twice the CTAs) is used
-// while 128 x 256 tiles would leave SMs idle.  One tile with K = 128: 20 us with
-// an update of C and 12.4 us without before, 13.5 and 11 us now; a 2304-row
-// inverse 888 -> 791 us, 14 pairs of odd sides 541 -> 447 us.  The 128-wide tile
-// has 16 producer warps of one unit and three blocks in flight: with eight warps
-// of two units and two blocks a k-block took the 1.3 us of a 256-wide one (144
-// tiles with K = 4608 190 -> 125 us; 2304-row inverse 796 -> 759 us).
+// Bound: the short products of the inverse (K <= 512) by latency: descriptor fetch,
+// one trip to L2 per register block, the epilogue; the preconditioning by the
+// loads and stores of its operands (a 128 x 256 x 32 block takes 1600 ns with TF32
+// terms, its MMAs 810), which is why longer layers go through chunks.  Hence the
+// descriptors of small launches travel as kernel arguments, and TN = 128 (half
+// the work per CTA, twice the CTAs) is used while 128 x 256 tiles would leave
+// SMs idle.  The 128-wide tile has 16 producer warps of one unit and three blocks
+// in flight: with eight warps of two units and two blocks a k-block took the
+// 1.3 us of a 256-wide one, 0.75 now.
 //
 // Every barrier wait is bounded; a wait that runs out raises a status word
 // instead of hanging.
@@ -703,14 +700,14 @@ int tc_number_tiles(GemmDesc* descs, int n, int narrow_max, int* tile_cols) {
   std::stable_partition(descs, descs + n, tile_desc_vec);
   // Narrow tiles (half the work per CTA, but the A rows are loaded, split and
   // read by the MMAs twice as often) up to `narrow_max` of them: as many as
-  // there are SMs for a launch that runs alone (512 x 4608 x 4608: 144 narrow
-  // tiles 125 us, 72 wide ones 190 us), three quarters where launches of other
-  // streams run beside it.  Measured with the line at 0, 20, 74, 111, 148 and
-  // 222 of 148 SMs: a 2304-row inverse 841, 819, 765, 763, 766, 769 us; a
-  // 4608-row one 2010, 1921, 1905, 1868, 1864, 1885; 14 pairs of odd sides 439,
-  // 425, 402, 390, 390, 390; the pair 4608 / 512 with its preconditioning 2225,
-  // 2138, 2119, 2081, 2048, 2072; 108 factors of ResNet-50 in three concurrent
-  // plans 6.10, 6.15, 6.17, 6.18, 6.19, 6.26 ms.
+  // there are SMs for a launch that runs alone, three quarters where launches of
+  // other streams run beside it.  us with the line at 0, 20, 74, 111, 148 and 222
+  // tiles on 148 SMs: inverses of 4608 beside 512 rows 1455, 1439, 1429, 1448,
+  // 1438, 1439; 2304 beside 256 699, 684, 669, 669, 668, 667; two of 1024 347, 338,
+  // 329, 330, 330, 331; 20 of 600 304, 304, 301, 290, 291, 290; 28 of odd sides 315,
+  // 312, 303, 303, 304, 304; 108 factors of ResNet-50 3381, 3386, 3370, 3377, 3383,
+  // 3366.  Preconditioning of short layers, wide and narrow: 54 narrow tiles 49 36,
+  // 72 49 36.5, 128 57 41, 176 109 109.
   long long narrow = 0;
   for (int i = 0; i < n; ++i) narrow += tile_count(descs[i], 128);
   const int tn = narrow <= narrow_max ? 128 : 256;
