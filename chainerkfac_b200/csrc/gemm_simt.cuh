@@ -377,8 +377,10 @@ int packed_status_read(int* out);
 // packed_takes_rows says that this pays.
 constexpr int kChunkExp = 14;    // scaled values of a row are below 2^15
 int launch_grad_sizes(const GradSizes* jobs_dev, const GradSizes* jobs_host,
-                      int njobs, int rows, int groups, bool wide,
+                      int njobs, int rows, int groups, int columns,
                       cudaStream_t stream);
+// Columns of a group in that launch (GradSizes::col_begin counts groups).
+int grad_group_columns(const int* cols, int n);
 int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,
                      int njobs, int rows, cudaStream_t stream);
 int launch_packed_precond(const GemmDesc* descs_dev, const GemmDesc* descs_host,

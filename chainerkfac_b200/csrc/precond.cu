@@ -104,9 +104,10 @@ static int precondition_chunks(
   char* const base = ws;
   const GemmDesc* descs_dev = reinterpret_cast<GemmDesc*>(base);
   ws += tables;
-  int rows = 0, rows_G = 0, groups = 0, wide_groups = 0;
-  for (int i = 0; i < count; ++i) wide_groups += (dW[i] + hb[i] + 31) / 32;
-  const bool wide = wide_groups >= sm_count() / 2;
+  int rows = 0, rows_G = 0, groups = 0;
+  std::vector<int> dA(count);
+  for (int i = 0; i < count; ++i) dA[i] = dW[i] + hb[i];
+  const int columns = grad_group_columns(dA.data(), count);
   auto at = [](char* base, size_t off) {
     return reinterpret_cast<unsigned char*>(base + off);
   };
@@ -132,7 +133,7 @@ static int precondition_chunks(
     z.row = exps(ws, c.row); z.col = exps(ws, c.col);
     z.rows = dg; z.cols = dw;
     z.row_begin = rows_G; z.col_begin = groups;
-    groups += wide ? (da + 31) / 32 : (da + 7) / 8;
+    groups += (da + columns - 1) / columns;
     auto job = [&](PackRows& j, const float* src, const float* extra,
                    size_t dst, const short* col, int sign, int cols, int nrows,
                    int& begin) {
@@ -193,7 +194,7 @@ static int precondition_chunks(
                               cudaMemcpyHostToDevice, st));
   const PackRows* jobs_dev = reinterpret_cast<PackRows*>(base + jobs_at);
   int rc = launch_grad_sizes(reinterpret_cast<GradSizes*>(base + sizes_at),
-                             sizes, count, rows_G, groups, wide, st);
+                             sizes, count, rows_G, groups, columns, st);
   if (rc == KFAC_OK) rc = launch_pack_rows(jobs_dev, jobs, 2 * count, rows, st);
   const bool beside = packed_takes_rows(tiles, rows_G);
   if (rc == KFAC_OK && !beside)

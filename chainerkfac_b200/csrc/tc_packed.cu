@@ -220,9 +220,8 @@ __device__ __forceinline__ void wait_for_launch_before() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Sizes of the rows of gradients (see GradSizes), WARPS warps per row.  A block per
-// row where there are few (the latency of a row counts), a warp per row elsewhere
-// (54 layers of ResNet-50: 60 us with blocks, 23 with warps).
+// Sizes of the rows of gradients (see GradSizes), WARPS warps per row: as many as
+// leave the launch one wave (54 layers of ResNet-50: 60 us with eight, 24 with one).
 template <int WARPS>
 __global__ void __launch_bounds__(256)
 grad_rows_kernel(const GradSizes* __restrict__ jobs, int njobs, int rows,
@@ -231,22 +230,21 @@ grad_rows_kernel(const GradSizes* __restrict__ jobs, int njobs, int rows,
   let_next_launch_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row_all = (8 / WARPS) * blockIdx.x + warp / WARPS;
-  if (row_all >= rows) return;           // (whole blocks where WARPS is 8)
+  const bool live = row_all < rows;
   const GradSizes* all = inl.n > 0 ? inl.j : jobs;
   int f = 0;
   for (int i = lane; i < njobs; i += 32)
     if (all[i].row_begin <= row_all) f = i;
   f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
   const GradSizes& job = all[f];
-  const int row = row_all - job.row_begin, cols = job.cols;
+  const int row = row_all - job.row_begin, cols = live ? job.cols : 0;
   const float* src = job.src + (long long)row * cols;
   const int at = 32 * (warp % WARPS) + lane;
   constexpr int S = 32 * WARPS;
   int top = kNoExp;
-  if (job.extra != nullptr && at == 0) top = exp_of(job.extra[row]);
+  if (live && job.extra != nullptr && at == 0) top = exp_of(job.extra[row]);
   // (eight loads in flight; past the end the last one again)
-  if (WARPS == 1 && (cols & 3) == 0 &&
-      (reinterpret_cast<uintptr_t>(job.src) & 15) == 0) {
+  if ((cols & 3) == 0 && (reinterpret_cast<uintptr_t>(job.src) & 15) == 0) {
     const float4* s4 = reinterpret_cast<const float4*>(src);
     const int n = cols >> 2;
     for (int k0 = at; k0 < n; k0 += 8 * S) {
@@ -272,14 +270,15 @@ grad_rows_kernel(const GradSizes* __restrict__ jobs, int njobs, int rows,
     if (lane == 0) part[warp] = top;
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 8; ++i) top = max(top, part[i]);
+    for (int i = 0; i < WARPS; ++i)
+      top = max(top, part[warp / WARPS * WARPS + i]);
   }
-  if (at == 0) job.row[row] = (short)top;
+  if (live && at == 0) job.row[row] = (short)top;
 }
 
-// Sizes of the columns behind it, W columns per block and 1024 / W rows at a time.
-// Narrow groups where wide ones would leave SMs idle (1000 x 1000: 5 us less), wide
-// ones elsewhere (512 x 4608: 6.5 us, 16 with narrow ones).
+// Sizes of the columns behind it, W columns per block and 1024 / W rows at a time:
+// as few as leave the launch one wave (W = 8 instead of 32 for 1000 x 1000: 5 us less;
+// in two waves, for 512 x 4608, 16 us instead of 6.5).
 template <int W>
 __global__ void __launch_bounds__(1024)
 grad_cols_kernel(const GradSizes* __restrict__ jobs, int njobs,
@@ -904,8 +903,17 @@ bool packed_takes_rows(int total_tiles, int rows) {
          rows <= free * (KP_THREADS / 32) + total_tiles * KP_EPI_WARPS;
 }
 
+int grad_group_columns(const int* cols, int n) {
+  for (int w = 8; w < 32; w *= 2) {
+    long long groups = 0;
+    for (int i = 0; i < n; ++i) groups += (cols[i] + w - 1) / w;
+    if (groups <= 2 * sm_count()) return w;      // (two blocks an SM)
+  }
+  return 32;
+}
+
 int launch_grad_sizes(const GradSizes* jobs_dev, const GradSizes* jobs_host,
-                      int njobs, int rows, int groups, bool wide,
+                      int njobs, int rows, int groups, int columns,
                       cudaStream_t stream) {
   if (njobs <= 0 || rows <= 0) return KFAC_OK;
   GradInline inl;
@@ -914,15 +922,22 @@ int launch_grad_sizes(const GradSizes* jobs_dev, const GradSizes* jobs_host,
     inl.n = njobs;
     std::copy(jobs_host, jobs_host + njobs, inl.j);
   }
-  const bool many = rows > 8 * sm_count();
-  const int rc = launch_behind(
-      "grad_rows_kernel", false, many ? grad_rows_kernel<1> : grad_rows_kernel<8>,
-      many ? (int)ceil_div(rows, 8) : rows, 256, 0, stream, jobs_dev, njobs, rows,
-      inl);
+  int warps = 8;                                 // (eight blocks an SM)
+  while (warps > 1 && ceil_div((int64_t)rows * warps, 8) > 8 * sm_count())
+    warps /= 2;
+  auto* by_rows = warps == 8   ? grad_rows_kernel<8>
+                  : warps == 4 ? grad_rows_kernel<4>
+                  : warps == 2 ? grad_rows_kernel<2>
+                               : grad_rows_kernel<1>;
+  const int rc = launch_behind("grad_rows_kernel", false, by_rows,
+                               ceil_div((int64_t)rows * warps, 8), 256, 0, stream,
+                               jobs_dev, njobs, rows, inl);
   if (rc != KFAC_OK) return rc;
-  return launch_behind("grad_cols_kernel", true,
-                       wide ? grad_cols_kernel<32> : grad_cols_kernel<8>, groups,
-                       1024, 0, stream, jobs_dev, njobs, inl);
+  auto* by_cols = columns == 8    ? grad_cols_kernel<8>
+                  : columns == 16 ? grad_cols_kernel<16>
+                                  : grad_cols_kernel<32>;
+  return launch_behind("grad_cols_kernel", true, by_cols, groups, 1024, 0, stream,
+                       jobs_dev, njobs, inl);
 }
 
 int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,

@@ -1010,6 +1010,41 @@ def test_precondition_of_features_of_any_scale(ops, dG, dW, bias, small):
     assert _worst(got, ref, 1) < 1e-5
 
 
+def test_precondition_of_long_layers_under_capture(ops, engine):
+    """The launches of a preconditioning in chunks begin before the one in front
+    has ended; captured and replayed on other gradients, call after call on one
+    workspace, they give what calls by themselves do."""
+    if engine == 0:
+        pytest.skip('chunks belong to the tensor-core engine')
+    rng = np.random.default_rng(41)
+    cases = [precond_case(rng, 512, 512, False), precond_case(rng, 300, 785, True)]
+    Gi, Ai, gW = ([dev(c[k]) for c in cases] for k in range(3))
+    gb = [None if c[3] is None else dev(c[3]) for c in cases]
+    kW = [torch.empty_like(t) for t in gW]
+    kb = [None if t is None else torch.empty_like(t) for t in gb]
+
+    def call():
+        ops.precondition(Gi, Ai, gW, gb, kW, kb)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        call()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            for _ in range(3):
+                call()
+        for scale in (1.0, 1e-6, 1e6):
+            for t in gW:
+                t.mul_(scale)
+            call()
+            want = [t.clone() for t in kW + kb if t is not None]
+            for t in kW:
+                t.zero_()
+            graph.replay()
+            for a, b in zip([t for t in kW + kb if t is not None], want):
+                assert torch.equal(a, b)
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize('value', [float('inf'), float('nan')])
 def test_precondition_of_a_non_finite_gradient_is_not_finite(ops, value):
     rng = np.random.default_rng(3)
