@@ -904,8 +904,9 @@ STAGE_KERNELS = {
                '(batched blocked Cholesky, '
                'triangular inverse and symmetric product of every factor, '
                'three size classes on three streams)',
-    'precondition': 'pack_rows_kernel + packed_tile_kernel (three grouped '
-                    'launches over all layers, update fused)'}
+    'precondition': 'grad_rows_kernel + grad_cols_kernel + pack_rows_kernel + '
+                    'packed_tile_kernel (six grouped launches over all '
+                    'layers, update fused)'}
 
 
 def run_ours(args):

@@ -267,8 +267,9 @@ int kfac_axpby_group(int n_arrays, const int64_t* counts, float a,
  *
  * The plan records device pointers, so the factor and inverse buffers must
  * stay where they are for the plan's lifetime.  `workspace` (device,
- * kfac_inverse_workspace_bytes bytes) is owned by the caller and must outlive
- * the plan; plans that run concurrently need distinct workspaces.
+ * kfac_inverse_workspace_bytes bytes, at any address) is owned by the caller
+ * and must outlive the plan; plans that run concurrently need distinct
+ * workspaces.
  */
 typedef struct kfac_inverse_plan kfac_inverse_plan;
 
@@ -334,7 +335,8 @@ int kfac_inverse_plan_destroy(kfac_inverse_plan* plan);
  * update_core (optimizers/kfac.py:87-116).
  *
  * All pointer arrays are host arrays of device pointers, read during the
- * call.  `workspace`: device, kfac_precond_workspace_bytes bytes.
+ * call.  `workspace`: device, kfac_precond_workspace_bytes bytes (which depend on
+ * the route that layers of these sizes take, so on all layers of the call).
  */
 size_t kfac_precond_workspace_bytes(int count, const int* dG, const int* dW,
                                     const int* has_bias);
