@@ -261,20 +261,7 @@ struct GemmDesc {
   int flags;
   int tile_begin;
   int tiles_m, tiles_n;
-  union {
-    struct {               // preconditioning, the product that gives kf
-      float *kfW, *kfb, *pW, *pb, *vW, *vb;
-    };
-    // the one before it, in chunks: rows of G_inv (M x M) packed beside it, from
-    // row inv_begin of the launch on
-    struct {
-      const float* inv;
-      unsigned char* inv_pack;
-      const short* inv_col;
-      short* inv_exp;
-      long long inv_begin;
-    };
-  };
+  float *kfW, *kfb, *pW, *pb, *vW, *vb;
   int dW;
   int splits;              // tensor-core engine: CTAs along the contraction
   int ntiles;              // tiles of one split (virtual tile = split * ntiles + tile)
@@ -303,26 +290,31 @@ struct GemmDesc {
   // and columns, exponents of the second's
   const float *rs, *cs;
   const short *re, *ce;
+  const short* wide;       // norms of the gradient's rows over their sizes
 };
 
 // Rows of a matrix (and an appended column) as K-major chunks, each scaled by a
-// power of two of its own, the columns before that by others.  A row of scale 2^s
-// whose values then have the 2-norm 2^n or less (n as small as a whole number
-// can be) leaves n - s, and 2^-n times `gain` as the factor that brings its
-// products with rows treated alike to at most `gain`; without `fit` it leaves -s.
-struct PackRow {
+// power of two 2^s of its own, the columns before that by others.  The scaled
+// values of a row have the 2-norm 2^n or less, n as small as a whole number can be.
+enum PackRole {
+  PACK_A,   // A_inv: leaves n - s and, as the factor of U's column, 2^-n `gain`
+  PACK_G,   // G_inv: leaves -s
+  PACK_GRAD // the gradient, rows of size 2^z: leaves n - s - z and 2^(-s - z)
+};
+struct PackRows {
   const float* src;
   const float* extra;      // appended column, NULL: none
   const short* col;        // exponents of the columns' factors
-  int col_sign;            // 1, or -1 where the columns are divided by them
+  const short* size;       // PACK_GRAD: z
   unsigned char* dst;
   short* exp;
   float* fit;
+  int col_sign;            // 1, or -1 where the columns are divided by them
+  int role;
   float gain;
   int cols;
-};
-struct PackRows : PackRow {
   int row_begin;           // first row in the launch
+  int pad_;
 };
 
 // Sizes of the columns of a gradient (and its bias column): exponents of the
@@ -373,8 +365,7 @@ int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
 int packed_status_read(int* out);
 // Preconditioning on chunks: sizes of the gradients, rows into chunks, then the
 // product whose result is chunks again and the one that gives the preconditioned
-// gradient.  Beside the first, `inv_rows` rows of G_inv are packed, where
-// packed_takes_rows says that this pays.
+// gradient (`last`).
 constexpr int kChunkExp = 14;    // scaled values of a row are below 2^15
 int launch_grad_sizes(const GradSizes* jobs_dev, const GradSizes* jobs_host,
                       int njobs, int rows, int groups, int columns,
@@ -384,9 +375,8 @@ int grad_group_columns(const int* cols, int n);
 int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,
                      int njobs, int rows, cudaStream_t stream);
 int launch_packed_precond(const GemmDesc* descs_dev, const GemmDesc* descs_host,
-                          int ndesc, int total_tiles, bool last, int inv_rows,
-                          float lr, float momentum, cudaStream_t stream);
-bool packed_takes_rows(int total_tiles, int rows);
+                          int ndesc, int total_tiles, bool last, float lr,
+                          float momentum, cudaStream_t stream);
 bool tc_desc_has_tails(const GemmDesc& g);
 size_t tc_factor_workspace_bytes(long long rows, int d, bool staged = true);
 size_t tc_lone_workspace_bytes(const Operand& X, long long rows, int d);

@@ -53,7 +53,7 @@ static __device__ int g_packed_status = 0;
 
 struct PackInline {
   int n;                       // 0: jobs in device memory
-  PackRows j[2 * TT_INLINE];   // two operands a layer
+  PackRows j[3 * TT_INLINE];   // three operands a layer
 };
 static_assert(sizeof(PackInline) <= 3800, "kernel argument space");
 
@@ -118,14 +118,15 @@ __device__ __forceinline__ void piece_each(int r, int c, int rows, int cols,
 // chunks, rows as k (zeros up to the end of the last k-block).  Rows and columns
 // are divided by bounds of the norms of what they are products of, so that an
 // entry is held relative to the most that its row and column could make it; the
-// rows' part is in G_inv's columns, the columns' comes out of kf.
+// rows' sizes are in G_inv's columns, the columns' part and `wide` (the most that
+// a row's norm exceeds its size) come out of kf.
 __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
-                                        int r, int c) {
+                                        int r, int c, float wide) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int gr = r + 8 * h;
     const bool in = gr < g.M;
-    const float s0 = g.rs[min(gr, g.M - 1)];
+    const float s0 = g.rs[min(gr, g.M - 1)] * wide;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       // (columns past the last one: any values, nobody stores their results)
@@ -143,12 +144,22 @@ __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
   }
 }
 
+// Exponent of the largest norm of a gradient row over its size, by a warp.
+__device__ __forceinline__ int widest_row(const GemmDesc& g, int lane) {
+  int m = kNoExp;
+#pragma unroll 4
+  for (int i = lane; i < g.M; i += 32) m = max(m, (int)g.wide[i]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  return m == kNoExp ? 0 : m;            // (a gradient of zeros)
+}
+
 // Second product: a 16 x 32 piece of kf to the weight and bias parts, and the
 // momentum update where the layer has it fused.
 __device__ __forceinline__ void store_kf(const GemmDesc& g, float v[16], int r,
-                                         int c, bool whole, float lr,
+                                         int c, bool whole, int wide, float lr,
                                          float momentum) {
-  const int e0 = g.re[min(r, g.M - 1)], e1 = g.re[min(r + 8, g.M - 1)];
+  const int e0 = g.re[min(r, g.M - 1)] + wide;
+  const int e1 = g.re[min(r + 8, g.M - 1)] + wide;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int e = g.ce[min(c + 8 * (j >> 1) + (j & 1), g.N - 1)];
@@ -329,9 +340,10 @@ grad_cols_kernel(const GradSizes* __restrict__ jobs, int njobs,
 
 // A row by a warp: its largest value, then (the row is in the L1 cache) the
 // scaled terms.  Bound by HBM: 4 bytes read and 4 written per element.
-// INV: exponents of any size (those of the gradient's columns are 126 at most).
+// INV (G_inv): exponents of any size (those of the gradient's columns are 126 at
+// most), no norm.
 template <bool INV>
-__device__ __forceinline__ void pack_row(const PackRow& job, int row,
+__device__ __forceinline__ void pack_row(const PackRows& job, int row,
                                          int lane) {
   const int cols = job.cols;
   const int total = cols + (job.extra != nullptr ? 1 : 0);
@@ -450,8 +462,10 @@ __device__ __forceinline__ void pack_row(const PackRow& job, int row,
     // sum < 2^(f + 1), its root at most 2^n (rounding of the sum: far inside
     // the factor of two that fp16 has left above 2^15)
     const int n = sum == 0.f ? 0 : (exp_of(sum) + 2) >> 1;
-    job.exp[row] = (short)(sum == 0.f ? kNoExp : n - s);
-    job.fit[row] = scale_exp(job.gain, -n);
+    const int z = job.role == PACK_GRAD && sum != 0.f ? job.size[row] : 0;
+    job.exp[row] = (short)(sum == 0.f ? kNoExp : n - s - z);
+    job.fit[row] = job.role == PACK_GRAD ? scale_exp(1.f, -s - z)
+                                         : scale_exp(job.gain, -n);
   }
 }
 
@@ -469,27 +483,10 @@ pack_rows_kernel(const PackRows* __restrict__ jobs, int njobs, int rows,
   f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
   const PackRows job = all[f];
   wait_for_launch_before();
-  if (job.fit != nullptr)
+  if (job.role != PACK_G)
     pack_row<false>(job, row_all - job.row_begin, lane);
   else
     pack_row<true>(job, row_all - job.row_begin, lane);
-}
-
-// A row of G_inv, of all layers' in a launch of the first product.
-__device__ __noinline__ void pack_inverse(const GemmDesc* all, int n,
-                                             int row_all, int lane) {
-  int f = 0;
-  for (int i = lane; i < n; i += 32)
-    if (all[i].inv_begin <= row_all) f = i;
-  f = (int)__reduce_max_sync(0xffffffffu, (unsigned)f);
-  const GemmDesc& g = all[f];
-  PackRow job;
-  job.src = g.inv; job.extra = nullptr;
-  job.col = g.inv_col; job.col_sign = 1;
-  job.dst = g.inv_pack;
-  job.exp = g.inv_exp; job.fit = nullptr; job.gain = 0.f;
-  job.cols = g.M;
-  pack_row<true>(job, row_all - (int)g.inv_begin, lane);
 }
 
 // MODE 0: the products of the inverse; 1, 2: first and second product of the
@@ -498,7 +495,7 @@ template <int MODE, int STAGES>
 __global__ void __launch_bounds__(KP_THREADS, STAGES == 3 ? 2 : 1)
 packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
                    const __grid_constant__ TileInline inl, float plr,
-                   float momentum, int inv_rows, int inv_ctas) {
+                   float momentum) {
   constexpr int kSegment = MODE == 0 ? KP_SEGMENT : 1 << 20;
   constexpr int TN = 128;
   extern __shared__ unsigned char kp_smem_raw[];
@@ -507,25 +504,7 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
   PackedControl* ctl =
       reinterpret_cast<PackedControl*>(smem + STAGES * KP_STAGE);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // First product: the rows of G_inv, which the next launch needs, may be packed by
-  // `inv_ctas` CTAs in front of the tiles (on SMs without one) and by the
-  // epilogue's warps while the MMAs run.  us in a launch of its own, in CTAs
-  // only, by the epilogues only: 512 x 512 +3.5, 40, 46; 1024 x 2048 +4, 87, 79.
-  const int tile = (int)blockIdx.x - inv_ctas;
-  auto pack_inverses = [&](int worker) {
-    const int workers = inv_ctas * (KP_THREADS / 32) +
-                        ((int)gridDim.x - inv_ctas) * KP_EPI_WARPS;
-    for (int i = worker; i < inv_rows; i += workers)
-      pack_inverse(inl.n > 0 ? inl.d : descs, ndesc, i, lane);
-  };
-  if constexpr (MODE == 1) {
-    if (tile < 0) {
-      let_next_launch_begin();
-      wait_for_launch_before();
-      pack_inverses(blockIdx.x * (KP_THREADS / 32) + warp);
-      return;
-    }
-  }
+  const int tile = blockIdx.x;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -668,9 +647,8 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
     const bool vec = (ldc & 1) == 0 &&
                      (reinterpret_cast<uintptr_t>(g.C) & 7) == 0;
     const int lr = lane >> 2, lc = 2 * (lane & 3);
-    if constexpr (MODE == 1)
-      pack_inverses(inv_ctas * (KP_THREADS / 32) + tile * KP_EPI_WARPS + warp -
-                    2);
+    // (while the MMAs run)
+    const int wide = MODE == 0 ? 0 : widest_row(g, lane);
     bool ok = true;
     const int nseg = nkb > 0 ? (kb0 + nkb - 1) / kSegment - seg0 + 1 : 1;
 #pragma unroll 1
@@ -732,11 +710,12 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
       }
       if (!live) continue;
       if constexpr (MODE == 1) {
-        store_u(g, v, r, c);
+        store_u(g, v, r, c, scale_exp(1.f, -wide));
         continue;
       }
       if constexpr (MODE == 2) {
-        store_kf(g, v, r, c, whole && c0 + 32 <= g.dW, plr, momentum);
+        store_kf(g, v, r, c, whole && c0 + 32 <= g.dW, wide, plr,
+                 momentum);
         continue;
       }
       if (un != nullptr) {
@@ -817,8 +796,7 @@ static int launch_behind(const char* name, bool early, void (*kernel)(P...),
 }
 
 struct PackedVariant {
-  void (*kernel)(const GemmDesc*, int, const TileInline, float, float, int,
-                 int);
+  void (*kernel)(const GemmDesc*, int, const TileInline, float, float);
   int stages;
 };
 // by mode; the preconditioning also with one CTA an SM
@@ -860,8 +838,7 @@ int packed_number_tiles(GemmDesc* descs, int n) {
 
 static int launch_mode(int mode, const GemmDesc* descs_dev,
                        const GemmDesc* descs_host, int ndesc, int total_tiles,
-                       int inv_rows, float lr, float momentum,
-                       cudaStream_t stream) {
+                       float lr, float momentum, cudaStream_t stream) {
   if (ndesc <= 0 || total_tiles <= 0) return KFAC_OK;
   const int rc = packed_prepare();
   if (rc != KFAC_OK) return rc;
@@ -873,34 +850,22 @@ static int launch_mode(int mode, const GemmDesc* descs_dev,
   }
   const bool one = mode > 0 && total_tiles <= sm_count();
   const PackedVariant& v = kPackedVariants[one ? mode + 2 : mode];
-  const int inv_ctas =
-      one ? std::min(sm_count() - total_tiles, (int)ceil_div(inv_rows, KP_THREADS / 32))
-          : 0;
-  return launch_behind("packed_tile_kernel", mode > 0, v.kernel,
-                       total_tiles + inv_ctas, KP_THREADS,
-                       packed_smem(v.stages), stream, descs_dev, ndesc, inl, lr,
-                       momentum, inv_rows, inv_ctas);
+  return launch_behind("packed_tile_kernel", mode > 0, v.kernel, total_tiles,
+                       KP_THREADS, packed_smem(v.stages), stream, descs_dev,
+                       ndesc, inl, lr, momentum);
 }
 
 int launch_packed(const GemmDesc* descs_dev, const GemmDesc* descs_host,
                   int ndesc, int total_tiles, cudaStream_t stream) {
-  return launch_mode(0, descs_dev, descs_host, ndesc, total_tiles, 0, 0.f, 0.f,
+  return launch_mode(0, descs_dev, descs_host, ndesc, total_tiles, 0.f, 0.f,
                      stream);
 }
 
 int launch_packed_precond(const GemmDesc* descs_dev, const GemmDesc* descs_host,
-                          int ndesc, int total_tiles, bool last, int inv_rows,
-                          float lr, float momentum, cudaStream_t stream) {
-  return launch_mode(last ? 2 : 1, descs_dev, descs_host, ndesc, total_tiles,
-                     inv_rows, lr, momentum, stream);
-}
-
-// One wave of tiles, and no warp with more than one row: else the rows hold up the
-// tiles (54 pairs of ResNet-50: 4413 us with a launch of their own, 4565 without).
-bool packed_takes_rows(int total_tiles, int rows) {
-  const int free = sm_count() - total_tiles;
-  return free >= 0 &&
-         rows <= free * (KP_THREADS / 32) + total_tiles * KP_EPI_WARPS;
+                          int ndesc, int total_tiles, bool last, float lr,
+                          float momentum, cudaStream_t stream) {
+  return launch_mode(last ? 2 : 1, descs_dev, descs_host, ndesc, total_tiles, lr,
+                     momentum, stream);
 }
 
 int grad_group_columns(const int* cols, int n) {
@@ -945,7 +910,7 @@ int launch_pack_rows(const PackRows* jobs_dev, const PackRows* jobs_host,
   if (njobs <= 0 || rows <= 0) return KFAC_OK;
   PackInline inl;
   inl.n = 0;
-  if (njobs <= 2 * TT_INLINE) {
+  if (njobs <= 3 * TT_INLINE) {
     inl.n = njobs;
     std::copy(jobs_host, jobs_host + njobs, inl.j);
   }
