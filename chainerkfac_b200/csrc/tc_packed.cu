@@ -121,12 +121,12 @@ __device__ __forceinline__ void piece_each(int r, int c, int rows, int cols,
 // rows' sizes are in G_inv's columns, the columns' part and `wide` (the most that
 // a row's norm exceeds its size) come out of kf.
 __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
-                                        int r, int c, float wide) {
+                                        int r, int c) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int gr = r + 8 * h;
     const bool in = gr < g.M;
-    const float s0 = g.rs[min(gr, g.M - 1)] * wide;
+    const float s0 = g.rs[min(gr, g.M - 1)];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       // (columns past the last one: any values, nobody stores their results)
@@ -144,22 +144,28 @@ __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
   }
 }
 
-// Exponent of the largest norm of a gradient row over its size, by a warp.
+// Exponent of the largest norm of a gradient row over its size, by a warp, eight
+// rows a load (the array begins at a multiple of 256 bytes).
 __device__ __forceinline__ int widest_row(const GemmDesc& g, int lane) {
-  int m = kNoExp;
-#pragma unroll 4
-  for (int i = lane; i < g.M; i += 32) m = max(m, (int)g.wide[i]);
+  unsigned pair = 0x80008000u;           // two shorts
+  const int n = g.M >> 3;
+#pragma unroll 8
+  for (int i = lane; i < n; i += 32) {
+    const uint4 w = reinterpret_cast<const uint4*>(g.wide)[i];
+    pair = __vmaxs2(__vmaxs2(__vmaxs2(pair, w.x), w.y), __vmaxs2(w.z, w.w));
+  }
+  int m = max((int)(short)pair, (int)(short)(pair >> 16));
+  if (8 * n + lane < g.M) m = max(m, (int)g.wide[8 * n + lane]);
   m = __reduce_max_sync(0xffffffffu, m);
-  return m == kNoExp ? 0 : m;            // (a gradient of zeros)
+  return m <= kNoExp ? 0 : m;            // (a gradient of zeros)
 }
 
 // Second product: a 16 x 32 piece of kf to the weight and bias parts, and the
 // momentum update where the layer has it fused.
 __device__ __forceinline__ void store_kf(const GemmDesc& g, float v[16], int r,
-                                         int c, bool whole, int wide, float lr,
+                                         int c, bool whole, float lr,
                                          float momentum) {
-  const int e0 = g.re[min(r, g.M - 1)] + wide;
-  const int e1 = g.re[min(r + 8, g.M - 1)] + wide;
+  const int e0 = g.re[min(r, g.M - 1)], e1 = g.re[min(r + 8, g.M - 1)];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int e = g.ce[min(c + 8 * (j >> 1) + (j & 1), g.N - 1)];
@@ -640,15 +646,18 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
     const int q = warp & 3, h = (warp - 2) >> 2;
     const int rows = g.M, cols = g.N;
     const bool lower = (flags & G_LOWER) != 0;
-    const float alpha = g.alpha;
+    // (preconditioning, while the MMAs run; a register of its own for it makes the
+    // second product spill: 54 layers of ResNet-50 267 us, 375 so)
+    const float alpha =
+        MODE == 0 ? g.alpha
+                  : scale_exp(g.alpha, MODE == 1 ? -widest_row(g, lane)
+                                                 : widest_row(g, lane));
     float beta = (g.beta_until > 0 && m0 >= g.beta_until) ? 0.f : g.beta;
     const float* un = g.unscale;
     const long long ldc = g.ldc;
     const bool vec = (ldc & 1) == 0 &&
                      (reinterpret_cast<uintptr_t>(g.C) & 7) == 0;
     const int lr = lane >> 2, lc = 2 * (lane & 3);
-    // (while the MMAs run)
-    const int wide = MODE == 0 ? 0 : widest_row(g, lane);
     bool ok = true;
     const int nseg = nkb > 0 ? (kb0 + nkb - 1) / kSegment - seg0 + 1 : 1;
 #pragma unroll 1
@@ -710,12 +719,11 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
       }
       if (!live) continue;
       if constexpr (MODE == 1) {
-        store_u(g, v, r, c, scale_exp(1.f, -wide));
+        store_u(g, v, r, c);
         continue;
       }
       if constexpr (MODE == 2) {
-        store_kf(g, v, r, c, whole && c0 + 32 <= g.dW, wide, plr,
-                 momentum);
+        store_kf(g, v, r, c, whole && c0 + 32 <= g.dW, plr, momentum);
         continue;
       }
       if (un != nullptr) {
