@@ -905,7 +905,7 @@ STAGE_KERNELS = {
                'triangular inverse and symmetric product of every factor, '
                'three size classes on three streams)',
     'precondition': 'grad_rows_kernel + grad_cols_kernel + pack_rows_kernel + '
-                    'packed_tile_kernel (six grouped launches over all '
+                    'packed_tile_kernel (five grouped launches over all '
                     'layers, update fused)'}
 
 
