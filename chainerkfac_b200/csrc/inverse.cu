@@ -212,52 +212,109 @@ constexpr int DLD = DB + 4;   // shared-memory row pitch of a 128 x 128 block
 constexpr int SB = 32;        // sub-block of the diagonal kernel
 constexpr int SLP = SB + 4;   // row pitch of a 32 x 32 sub-block
 constexpr int DT = 512;       // threads of the diagonal kernel
-constexpr int kLookTile = DB * 128;    // both fp16 terms of 128 rows x 32 k
-constexpr int kLookBytes = 8 * kLookTile;       // four k-blocks of A' and of X
-constexpr int kLookCols = 2 * DB;               // tensor-memory columns
+constexpr int kLookTile = DB * 128;    // one fp16 term of 128 rows x 64 k
+constexpr int kLookBytes = 8 * kLookTile;       // both of A' and of X_pp
+constexpr int kDiagCols = 2 * DB;               // tensor-memory columns
 
 static __device__ int g_diag_status = 0;
 
-struct LookControl {
-  unsigned long long full[4];  // a k-block of the first product is stored
+struct DiagControl {
+  // look-ahead
+  unsigned long long x_here;   // X_pp has arrived
   unsigned long long done[2];  // all MMAs of the first, second product
+  // elimination, one for each sub-block and step
+  unsigned long long step[4][4];  // eight columns of L_pp are in Ls
+  unsigned long long crit[4][4];  // eight columns of the next row-block in S
+  // a phase per sub-block
+  unsigned long long rows;     // all its columns are stored as operands
+  unsigned long long next;     // products with the next sub-block column,
+  unsigned long long beyond;   // with the columns beyond
   unsigned tmem_base;
   volatile int abort_flag;
+  volatile int grace;          // abort_flag of the wait at the very end
 };
 
-// Issue the three MMAs per product of one 32-k operand block: D(128 x n) += A B^T
-// with A, B given as tiles of 128-byte rows, hi terms then lo terms.  hi*hi goes
-// to columns [0, 128) of the tensor memory, the cross terms to [128, 256).
-__device__ __forceinline__ void look_mma_block(unsigned tmem, unsigned a,
-                                               unsigned b, int n, bool first) {
-  const unsigned idesc = tc_half_desc(n, false, false);
-  const unsigned long long da = tc_smem_desc(a), db = tc_smem_desc(b);
-  constexpr unsigned long long lo = 64 >> 4;
-#pragma unroll
-  for (int kk = 0; kk < 2; ++kk) {
-    const unsigned long long adv = (unsigned long long)(kk * 32 >> 4);
-    const unsigned acc = (first && kk == 0) ? 0u : 1u;
-    tc_mma_half(tmem + DB, da + lo + adv, db + adv, idesc, acc);
-    tc_mma_half(tmem + DB, da + adv, db + lo + adv, idesc, 1u);
-    tc_mma_half(tmem, da + adv, db + adv, idesc, acc);
+// Bounded wait on a phase of a barrier of this kernel; false if the limit ran out
+// here or elsewhere in the block (the status word is set at the end).  Shorter than
+// mbar_wait_status: see chol_diag_kernel on the size of its code.
+__device__ __forceinline__ bool diag_wait(unsigned long long* bar,
+                                          unsigned parity,
+                                          volatile int* abort_flag) {
+  const unsigned addr = smem_u32(bar);
+#pragma unroll 1
+  for (unsigned i = 0; i < TC_SPIN_LIMIT; ++i) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (*abort_flag) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
+
+// The same by a whole warp ahead of its use of tensor memory.
+__device__ __forceinline__ bool diag_wait_tmem(unsigned long long* bar,
+                                               unsigned parity,
+                                               volatile int* abort_flag) {
+  const bool ok = diag_wait(bar, parity, abort_flag);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  return __all_sync(0xffffffffu, ok);
+}
+
+// One product of the look-ahead, D(128 x 128) = A B^T over 128 k, 16 at a time:
+// operands as tiles of 64 k by term (hi, lo), then the next 64 k.  hi*hi goes to
+// columns [0, 128) of the tensor memory, the cross terms to [128, 256).  `lower`:
+// B's rows in front of the k of its columns are zeros, and not there.
+__device__ __forceinline__ void look_mma(unsigned tmem, unsigned a, unsigned b,
+                                         bool lower) {
+  constexpr unsigned long long lo = kLookTile >> 4;
+  unsigned long long da = tc_smem_desc(a), db = tc_smem_desc(b);
+#pragma unroll 1
+  for (int kk = 0; kk < 8; ++kk) {
+    const int n0 = lower ? 32 * (kk >> 1) : 0;
+    const unsigned long long bk = db + (unsigned long long)(n0 * 128 >> 4);
+    const unsigned idesc = tc_half_desc(DB - n0, false, false);
+    const unsigned d = tmem + n0;
+    tc_mma_half(d + DB, da + lo, bk, idesc, kk > 0);
+    tc_mma_half(d + DB, da, bk + lo, idesc, 1u);
+    tc_mma_half(d, da, bk, idesc, kk > 0);
+    const unsigned long long adv = kk == 3 ? (2 * kLookTile - 96) >> 4 : 32 >> 4;
+    da += adv;
+    db += adv;
   }
 }
 
-// Four scaled values of a row as fp16 terms into a tile (8-byte word `word` of
-// the row's hi and lo terms).
-__device__ __forceinline__ void look_store4(unsigned tile, int row, int word,
-                                            float4 x, float scale) {
-  const unsigned d = tile + sw128_chunk_off(row, word >> 1) + 8 * (word & 1);
-  unsigned h0, h1, l0, l1;
-  split_half2(scale * x.x, scale * x.y, h0, l0);
-  split_half2(scale * x.z, scale * x.w, h1, l1);
-  sts64(d, h0, h1);
-  sts64(d ^ 0x40u, l0, l1);
+// Sixteen scaled values, columns 16 c .. of 64 of a row, as fp16 terms into the
+// row of their tiles.
+__device__ __forceinline__ void look_store16(unsigned tile, int row, int c,
+                                             const float v[16], float scale) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    unsigned hi[4], lo[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      split_half2(scale * v[8 * i + 2 * e], scale * v[8 * i + 2 * e + 1], hi[e],
+                  lo[e]);
+    const unsigned d = tile + sw128_chunk_off(row, 2 * c + i);
+    sts128(d, make_float4(__uint_as_float(hi[0]), __uint_as_float(hi[1]),
+                          __uint_as_float(hi[2]), __uint_as_float(hi[3])));
+    sts128(d + kLookTile,
+           make_float4(__uint_as_float(lo[0]), __uint_as_float(lo[1]),
+                       __uint_as_float(lo[2]), __uint_as_float(lo[3])));
+  }
 }
 
-// 16 bytes global -> shared without a register in between.
-__device__ __forceinline__ void cp_async16(unsigned dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src)
+// 16 bytes global -> shared without a register in between; zeros if !there.
+__device__ __forceinline__ void cp_async16(unsigned dst, const float* src,
+                                           bool there = true) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst),
+               "l"(src), "r"(there ? 16 : 0)
                : "memory");
 }
 
@@ -267,6 +324,7 @@ __device__ __forceinline__ void cp_async16(unsigned dst, const float* src) {
 __device__ __forceinline__ void diag_load(const float* Wd, long long ld, int bs,
                                           float* S) {
   const int rows = (bs + SB - 1) / SB * SB;
+#pragma unroll 1
   for (int idx = threadIdx.x; idx < rows * (DB / 4); idx += DT) {
     const int r = idx >> 5, c = (idx & 31) * 4;
     float* dst = &S[r * DLD + c];
@@ -288,20 +346,28 @@ __device__ __forceinline__ void diag_load_wait() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// Barriers and tensor memory of the look-ahead; needs nothing of the matrix.
-__device__ __forceinline__ void look_begin(LookControl* ctl) {
-  if (threadIdx.x == 32) {
-#pragma unroll
-    for (int kb = 0; kb < 4; ++kb) mbar_init(&ctl->full[kb], DT / 32);
-    mbar_init(&ctl->done[0], 1);
-    mbar_init(&ctl->done[1], 1);
+// Barriers and tensor memory; needs nothing of the matrix but the number of
+// sub-blocks.
+__device__ __forceinline__ void diag_begin(DiagControl* ctl, int np) {
+  if (threadIdx.x >= 32 && threadIdx.x < 48) {
+    const int i = threadIdx.x - 32;
+    mbar_init(&ctl->step[i >> 2][i & 3], 1);
+    mbar_init(&ctl->crit[i >> 2][i & 3], 1);
+    if (i < 2) mbar_init(&ctl->done[i], 1);
+    if (i == 3) mbar_init(&ctl->x_here, 1);
+    // (a warp per row-block, X^T's new rows, and the warp that has taken the next
+    // diagonal sub-block's products out)
+    if (i == 0) mbar_init(&ctl->rows, np + 2);
+    if (i == 1) mbar_init(&ctl->next, 1);
+    if (i == 2) mbar_init(&ctl->beyond, 1);
     ctl->abort_flag = 0;
+    ctl->grace = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x < 32) {
     asm volatile(
         "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-        ::"r"(smem_u32(&ctl->tmem_base)), "r"(kLookCols)
+        ::"r"(smem_u32(&ctl->tmem_base)), "r"(kDiagCols)
         : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
                  ::: "memory");
@@ -315,113 +381,105 @@ __device__ __forceinline__ void look_begin(LookControl* ctl) {
 // leaves as it was) and X_pp (inverse of the previous diagonal block's factor),
 // so that this kernel does not have to wait for the panel solve and panel
 // update of step k - 1.  Both products run on the tensor cores (tcgen05,
-// operands in two fp16 terms, accumulators in tensor memory).  All global loads
-// are in flight at once (16 x 16 bytes per thread); the blocks of X_pp above its
-// diagonal are neither loaded nor multiplied.  Result: D in S.  Returns false if
-// a bounded wait ran out (the status word is set; the caller stores nothing).
-// With TF32 terms, twice the MMA time and shared memory for two k-blocks at a
-// time, the whole kernel took 31.7 us on average of a plan of 856 rows, now 29.6.
-__device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
+// operands in two fp16 terms, accumulators in tensor memory).  X_pp comes as the
+// chunks that the diagonal kernel of step k - 1 left, by bulk copies (rows of 64
+// columns, K-major here), those above its diagonal left out; A' and W_kk by
+// asynchronous copies, A' into the places of its own terms: piece i of 32 columns
+// into tile i.  Result: D in S.
+__device__ __forceinline__ void diag_lookahead(const MatInfo& mi, int o, int bs,
                                                float* S,
                                                unsigned char* stage,
-                                               LookControl* ctl) {
+                                               DiagControl* ctl) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long ld = mi.ld;
-  const float* Ap = mi.W + (long long)o * ld + (o - DB);
-  const float* Xp = mi.X + (long long)(o - DB) * ld + (o - DB);
-  // rows of a warp: eight; those of a half warp differ in the bit that moves the
-  // swizzle across the halves of a 128-byte row (8-byte stores)
-  const int row0 = 8 * warp + 4 * ((lane >> 3) & 1) + (lane >> 4);
-  const int word = lane & 7;
-  float4 va[4][2], vx[4][2];
-#pragma unroll
-  for (int kb = 0; kb < 4; ++kb) {
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int row = row0 + 2 * j, col = 32 * kb + 4 * word;
-      va[kb][j] = vx[kb][j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      const float* pa = &Ap[row * ld + col];
-      const float* px = &Xp[row * ld + col];
-      if (row < bs) va[kb][j] = *reinterpret_cast<const float4*>(pa);
-      if (row >= 32 * kb) vx[kb][j] = *reinterpret_cast<const float4*>(px);
+  const unsigned ta = smem_u32(stage), tx = ta + 4 * kLookTile;
+  diag_begin(ctl, (bs + SB - 1) / SB);
+  if (warp == 1) {
+    __syncwarp();
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                   ::"r"(smem_u32(&ctl->x_here)), "r"(12 * 4096)
+                   : "memory");
+    __syncwarp();
+    if (lane < 12) {
+      // 32 rows of one term of 64 columns
+      const int h = lane >> 3, term = lane & 1;
+      const int rc = h ? (lane - 4) >> 1 : lane >> 1;
+      const unsigned char* src =
+          mi.PX + (long long)(o / DB - 1) * mi.tile +
+          (long long)((o - DB) / 32 + rc) * kChunk + h * 8192 + term * 4096;
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
+          "[%0], [%1], 4096, [%2];"
+          ::"r"(tx + (2 * h + term) * kLookTile + rc * 4096), "l"(src),
+            "r"(smem_u32(&ctl->x_here))
+          : "memory");
     }
   }
-  look_begin(ctl);
-  // W_kk into S (the update is subtracted from it at the end)
+  {
+    const float* src = mi.W + (long long)o * ld + (o - DB) + 4 * lane;
+    const unsigned dst = ta + (lane >> 3) * kLookTile;
+#pragma unroll 2
+    for (int i = 0; i < 8; ++i) {
+      const int row = 8 * warp + i;
+      cp_async16(dst + sw128_chunk_off(row, lane & 7),
+                 row < bs ? src + row * ld : src, row < bs);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // (the update is subtracted from it at the end)
   diag_load(mi.W + (long long)o * ld + o, ld, bs, S);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+
+  // ---- A' into its terms, 64 columns at a time: a warp's own eight rows
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    __syncwarp();
+    const int row = 8 * warp + (lane & 7), c = lane >> 3;
+    const float4* src = reinterpret_cast<const float4*>(
+        stage + (2 * h + (c >> 1)) * kLookTile + row * 128);
+    float v[16];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 u = src[(4 * (c & 1) + e) ^ (row & 7)];
+      v[4 * e] = u.x; v[4 * e + 1] = u.y; v[4 * e + 2] = u.z; v[4 * e + 3] = u.w;
+    }
+    __syncwarp();
+    look_store16(ta + 2 * h * kLookTile, row, c, v, kScaleL);
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem = ctl->tmem_base;
-  const unsigned sbase = smem_u32(stage);
-  bool ok = true;
 
-  // ---- L' = A' X_pp^T: the MMAs of a block of 32 k as soon as all warps have
-  // stored it, issued between the first warp's own stores
-  auto issue = [&](int kb) {
-    const bool go = mbar_wait_status(&ctl->full[kb], 0, &ctl->abort_flag,
-                                     &g_diag_status);
+  // ---- L' = A' X_pp^T
+  if (warp == 0) {
+    const bool go = diag_wait(&ctl->x_here, 0, &ctl->abort_flag);
     if (__all_sync(0xffffffffu, go) && elect_one()) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const unsigned ta = sbase + 2 * kb * kLookTile;
-      // columns below 32 kb of L' get nothing from this block of k
-      look_mma_block(tmem + 32 * kb, ta,
-                     ta + kLookTile + (unsigned)(32 * kb) * 128, DB - 32 * kb,
-                     kb == 0);
-      if (kb == 3) tc_commit(&ctl->done[0]);
+      look_mma(tmem, ta, tx, true);
+      tc_commit(&ctl->done[0]);
     }
     __syncwarp();
-  };
-#pragma unroll
-  for (int kb = 0; kb < 4; ++kb) {
-    const unsigned ta = sbase + 2 * kb * kLookTile, tx = ta + kLookTile;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int row = row0 + 2 * j;
-      look_store4(ta, row, word, va[kb][j], kScaleL);
-      if (row >= 32 * kb) look_store4(tx, row, word, vx[kb][j], kScaleX);
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&ctl->full[kb]);
-    if (warp == 0 && kb > 0) issue(kb - 1);
   }
-  if (warp == 0) issue(3);
-  ok = mbar_wait_status(&ctl->done[0], 0, &ctl->abort_flag, &g_diag_status);
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  bool ok = diag_wait_tmem(&ctl->done[0], 0, &ctl->abort_flag);
 
-  // ---- L' out of tensor memory, split, into the operand blocks of the second
-  // product (A and B are the same matrix: four blocks of 32 k)
+  // ---- L' out of tensor memory, split, into the operand tiles of the second
+  // product (A and B are the same matrix)
   const int q = warp & 3, h = warp >> 2;
   const int row = 32 * q + lane;
-  ok = __all_sync(0xffffffffu, ok);     // the loads below are warp-wide
+  const unsigned acc = tmem + ((unsigned)(32 * q) << 16) + (unsigned)(32 * h);
   if (ok) {
-    const unsigned blk = sbase + (unsigned)h * kLookTile;
     // (the scale of A' X_pp^T is kScaleL kScaleX; L' keeps kScaleL of it)
-    constexpr float s = 1.f / kScaleX;
-#pragma unroll
+#pragma unroll 1
     for (int cc = 0; cc < 2; ++cc) {
-      const int c0 = 32 * h + 16 * cc;
       float v[16], w[16];
-      tc_ld16_pair(tmem + ((unsigned)(32 * q) << 16) + (unsigned)c0,
-                   tmem + ((unsigned)(32 * q) << 16) + (unsigned)(DB + c0), v,
-                   w);
+      tc_ld16_pair(acc + 16 * cc, acc + 16 * cc + DB, v, w);
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        unsigned hi[4], lo[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int c = 8 * i + 2 * e;
-          split_half2(s * (v[c] + w[c]), s * (v[c + 1] + w[c + 1]), hi[e],
-                      lo[e]);
-        }
-        const unsigned d = blk + sw128_chunk_off(row, 2 * cc + i);
-        sts128(d, make_float4(__uint_as_float(hi[0]), __uint_as_float(hi[1]),
-                              __uint_as_float(hi[2]), __uint_as_float(hi[3])));
-        sts128(d ^ 0x40u,
-               make_float4(__uint_as_float(lo[0]), __uint_as_float(lo[1]),
-                           __uint_as_float(lo[2]), __uint_as_float(lo[3])));
-      }
+      for (int e = 0; e < 16; ++e) v[e] += w[e];
+      look_store16(ta + 2 * (h >> 1) * kLookTile, row, 2 * (h & 1) + cc, v,
+                   1.f / kScaleX);
     }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -430,30 +488,22 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
   // ---- L' L'^T
   if (warp == 0 && !ctl->abort_flag && elect_one()) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-    for (int kb = 0; kb < 4; ++kb) {
-      const unsigned blk = sbase + (unsigned)kb * kLookTile;
-      look_mma_block(tmem, blk, blk, DB, kb == 0);
-    }
+    look_mma(tmem, ta, ta, false);
     tc_commit(&ctl->done[1]);
   }
   diag_load_wait();
-  ok = mbar_wait_status(&ctl->done[1], 0, &ctl->abort_flag, &g_diag_status) && ok;
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  ok = diag_wait_tmem(&ctl->done[1], 0, &ctl->abort_flag);
   __syncthreads();                      // every thread's part of W_kk is there
-  ok = __all_sync(0xffffffffu, ok);
   if (ok && h <= q) {                   // sub-blocks on and below the diagonal
     constexpr float s = -1.f / (kScaleL * kScaleL);
-#pragma unroll
+#pragma unroll 1
     for (int cc = 0; cc < 2; ++cc) {
-      const int c0 = 32 * h + 16 * cc;
       float v[16], w[16];
-      tc_ld16_pair(tmem + ((unsigned)(32 * q) << 16) + (unsigned)c0,
-                   tmem + ((unsigned)(32 * q) << 16) + (unsigned)(DB + c0), v,
-                   w);
+      tc_ld16_pair(acc + 16 * cc, acc + 16 * cc + DB, v, w);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float4* s4 = reinterpret_cast<float4*>(&S[row * DLD + c0 + 4 * i]);
+        float4* s4 = reinterpret_cast<float4*>(
+            &S[row * DLD + 32 * h + 16 * cc + 4 * i]);
         float4 d = *s4;
         d.x += s * (v[4 * i] + w[4 * i]);
         d.y += s * (v[4 * i + 1] + w[4 * i + 1]);
@@ -464,26 +514,27 @@ __device__ __forceinline__ bool diag_lookahead(const MatInfo& mi, int o, int bs,
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
-                 ::"r"(tmem), "r"(kLookCols)
-                 : "memory");
-  }
-  return ctl->abort_flag == 0;
 }
 
 // ------------------------------------------------ one 128 x 128 diagonal block
 // Shared memory of the diagonal kernel, in floats.
-constexpr int LSP = SB + 16;   // row pitch of Ls (reads run past the last column)
+constexpr int LSP = SB + 4;    // row pitch of Ls
+constexpr int kDiagTile = DB * 128;            // 128 rows x 32 k of two bf16 terms
 struct DiagSmem {
   float S[DB * DLD];          // D / L in the sub-blocks on and below the
                               // diagonal, X^T in those above it
   float XD[4][SB * SLP];      // X_pp^T: inverse of sub-block p of the diagonal
-  float Ls[SB][LSP];          // L_pp by columns
-  float rl[SB];               // 1 / l_cc
+  float Ls[2][SB][LSP];       // L_pp by columns (p & 1: followers that the chain
+  float rl[2][SB];            // does not wait for may be behind it), 1 / l_cc
   float pv[SB][8];            // the running step's eight columns
 };
+
+// What lies behind S: the rest of DiagSmem, then (at a multiple of 1024 bytes from
+// the look-ahead's stages on) the operand tiles of the elimination.
+constexpr int kDiagStage =
+    (int)((sizeof(DiagSmem) - DB * DLD * sizeof(float) + 1023) / 1024 * 1024) +
+    2 * kDiagTile;
+static_assert(kDiagStage <= kLookBytes, "diagonal kernel shared memory");
 
 __device__ __forceinline__ void bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -494,11 +545,37 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) {
 }
 
 // Named barriers of the diagonal kernel.
-constexpr int kBarStep = 1;    // + step: eight columns of L_pp are in Ls
-constexpr int kRestWarps = 4; // warps of diag_base_rest
-constexpr int kBarNext = 4;    // + step (1, 2): the columns after the next are
-constexpr int kBarDiag = 7;    // the next diagonal sub-block is up to date
-constexpr int kBarRows = 8;    // so are the rows that follow it
+constexpr int kRestWarps = 4;  // warps of diag_base_rest
+constexpr int kBarNext = 0;    // + step (1, 2): the columns after the next are
+                               // up to date
+constexpr int kBarDiag = 3;    // the next diagonal sub-block is up to date
+constexpr int kBarStore = 4;   // + p: rows SB p .. of X are in shared memory
+constexpr int kBarPre = 8;     // earlier products are out of the next sub-block
+
+// Two multiply-adds an instruction; a pair is a register pair.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float x, float y) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpair(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// Four floats of shared memory as two pairs.
+__device__ __forceinline__ ulonglong2 load_pairs(const float* p) {
+  return *reinterpret_cast<const ulonglong2*>(p);
+}
+__device__ __forceinline__ void store_pairs(float* p, f32x2 a, f32x2 b) {
+  *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(a, b);
+}
 
 // Pivot k of an 8 x 8 block: r = 1 / sqrt(q) by the approximation and one
 // Newton step; `next`, if given, becomes p / sqrt(q) without waiting for r.  The
@@ -531,13 +608,16 @@ __global__ void pivots_selftest_kernel(int count, const float* q, const float* p
 }
 
 // Cholesky factor of the 8 x 8 block p (lower part, in place), r = reciprocal
-// square roots of the pivots.
+// square roots of the pivots.  The row x goes through the triangle on the way: its
+// multiply-adds fill the wait for the next pivot.
 template <bool CHECK>
-__device__ __forceinline__ void diag_chol8(float p[8][8], float r[8]) {
+__device__ __forceinline__ void diag_chol8(float p[8][8], float r[8],
+                                           float x[8]) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     float l = k < 7 ? p[k + 1][k] : 0.f;
     r[k] = diag_pivot<CHECK>(p[k][k], k < 7 ? &l : nullptr);
+    x[k] *= r[k];
     if (k == 7) break;
     p[k + 1][k] = CHECK ? p[k + 1][k] * r[k] : l;
 #pragma unroll
@@ -546,19 +626,8 @@ __device__ __forceinline__ void diag_chol8(float p[8][8], float r[8]) {
     for (int j = k + 1; j < 8; ++j)
 #pragma unroll
       for (int i = j; i < 8; ++i) p[i][j] = fmaf(-p[i][k], p[j][k], p[i][j]);
-  }
-}
-
-// Row (a0 .. a7) of the step's eight columns through the 8 x 8 triangle:
-// l(i, k) gives L[i][k].
-template <typename F>
-__device__ __forceinline__ void diag_solve8(float x[8], const float r[8], F l) {
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    float v = x[k];
-#pragma unroll
-    for (int m = 0; m < k; ++m) v = fmaf(-x[m], l(k, m), v);
-    x[k] = v * r[k];
+    for (int i = k + 1; i < 8; ++i) x[i] = fmaf(-x[k], p[i][k], x[i]);
   }
 }
 
@@ -583,98 +652,142 @@ __device__ __forceinline__ void diag_load8(const DiagSmem& sm, int j,
 // the columns to the other rows comes once in eight columns.  Of a step's
 // rank-8 update this warp applies only the part on the next eight columns; the
 // columns after those are updated by other warps (diag_base_rest) meanwhile.
-__device__ __forceinline__ void diag_base(DiagSmem& sm, int p, int lane, int id,
-                                          int col0, int followers, int* info) {
-  const float4* row = reinterpret_cast<const float4*>(
-      &sm.S[(SB * p + lane) * DLD + SB * p]);
-  float x[8];
-  float4 u = row[0], v = row[1];
+__device__ __forceinline__ void diag_base(DiagSmem& sm, DiagControl* ctl, int p,
+                                          int lane, int id, int col0, int* info) {
+  const float* row = &sm.S[(SB * p + lane) * DLD + SB * p];
+  float* const rl = sm.rl[p & 1];
+  f32x2 y[4];                  // this lane's row, eight columns
+  {
+    const ulonglong2 u = load_pairs(row), v = load_pairs(row + 4);
+    y[0] = u.x; y[1] = u.y; y[2] = v.x; y[3] = v.y;
+  }
 #pragma unroll 1
   for (int s = 0; s < 4; ++s) {
     const int j = 8 * s;
-    float blk[8][8], r[8];
-    float4* pv = reinterpret_cast<float4*>(sm.pv[lane]);
-    pv[0] = u;
-    pv[1] = v;
+    float blk[8][8], r[8], x[8];
+    store_pairs(&sm.pv[lane][0], y[0], y[1]);
+    store_pairs(&sm.pv[lane][4], y[2], y[3]);
     __syncwarp();
     diag_load8(sm, j, blk);
-    diag_chol8<false>(blk, r);
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      const float2 v = unpair(y[k / 2]);
+      x[k] = v.x; x[k + 1] = v.y;
+    }
+    // (rows above the pivot: unused)
+    diag_chol8<false>(blk, r, x);
     if (!(r[7] == r[7])) {
       // some pivot is not positive (every later one is NaN then): report the
       // first, carry on with ones in their place
       diag_load8(sm, j, blk);
-      diag_chol8<true>(blk, r);
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        const float2 v = unpair(y[k / 2]);
+        x[k] = v.x; x[k + 1] = v.y;
+      }
+      diag_chol8<true>(blk, r, x);
       int first = 0;
 #pragma unroll
       for (int k = 7; k >= 0; --k)
         if (!(blk[k][k] >= 1.17549435e-38f)) first = j + k + 1;
       if (lane == 0 && first != 0) atomicCAS(&info[id], 0, col0 + first);
     }
-    // this lane's row (rows above the pivot: unused)
-    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
-    x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
-    diag_solve8(x, r, [&](int i, int k) { return blk[i][k]; });
-    float (*L)[LSP] = &sm.Ls[j];
+    float (*L)[LSP] = &sm.Ls[p & 1][j];
 #pragma unroll
     for (int k = 0; k < 8; ++k) L[k][lane] = x[k];
     // (every lane stores the same)
-    *reinterpret_cast<float4*>(&sm.rl[j]) = make_float4(r[0], r[1], r[2], r[3]);
-    *reinterpret_cast<float4*>(&sm.rl[j + 4]) = make_float4(r[4], r[5], r[6], r[7]);
+    *reinterpret_cast<float4*>(&rl[j]) = make_float4(r[0], r[1], r[2], r[3]);
+    *reinterpret_cast<float4*>(&rl[j + 4]) = make_float4(r[4], r[5], r[6], r[7]);
     __syncwarp();
-    bar_arrive(kBarStep + s, followers + (s < 2 ? 32 * kRestWarps : 0));
+    if (lane == 0) mbar_arrive(&ctl->step[p][s]);
     if (s == 3) break;
     if (s > 0) bar_sync(kBarNext + s, 32 + 32 * kRestWarps);
-    u = row[2 * s + 2];
-    v = row[2 * s + 3];
+    {
+      const ulonglong2 u = load_pairs(row + j + 8), v = load_pairs(row + j + 12);
+      y[0] = u.x; y[1] = u.y; y[2] = v.x; y[3] = v.y;
+    }
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const float4 l = *reinterpret_cast<const float4*>(&L[k][j + 8]);
-      const float4 m = *reinterpret_cast<const float4*>(&L[k][j + 12]);
-      u.x = fmaf(-x[k], l.x, u.x); u.y = fmaf(-x[k], l.y, u.y);
-      u.z = fmaf(-x[k], l.z, u.z); u.w = fmaf(-x[k], l.w, u.w);
-      v.x = fmaf(-x[k], m.x, v.x); v.y = fmaf(-x[k], m.y, v.y);
-      v.z = fmaf(-x[k], m.z, v.z); v.w = fmaf(-x[k], m.w, v.w);
+      const ulonglong2 l = load_pairs(&L[k][j + 8]);
+      const ulonglong2 m = load_pairs(&L[k][j + 12]);
+      const f32x2 nx = pair(-x[k], -x[k]);
+      y[0] = fma2(nx, l.x, y[0]); y[1] = fma2(nx, l.y, y[1]);
+      y[2] = fma2(nx, m.x, y[2]); y[3] = fma2(nx, m.y, y[3]);
     }
   }
 }
 
 // The part of diag_base's updates that its own warp leaves: step s on columns
 // 8 s + 16 .. 31 of the sub-block, in shared memory, four columns per warp.
-__device__ __forceinline__ void diag_base_rest(DiagSmem& sm, int p, int lane,
-                                               int h, int followers) {
+__device__ __forceinline__ void diag_base_rest(DiagSmem& sm, DiagControl* ctl,
+                                               int p, int lane, int h) {
 #pragma unroll 1
   for (int s = 0; s < 2; ++s) {
-    bar_sync(kBarStep + s, followers + 32 * kRestWarps);
+    diag_wait(&ctl->step[p][s], 0, &ctl->abort_flag);
     const int c = 8 * s + 16 + 4 * h;
     if (c < SB) {
-      const float (*L)[LSP] = &sm.Ls[8 * s];
-      float4* row = reinterpret_cast<float4*>(
-          &sm.S[(SB * p + lane) * DLD + SB * p + c]);
-      float4 u = *row;
+      const float (*L)[LSP] = &sm.Ls[p & 1][8 * s];
+      float* row = &sm.S[(SB * p + lane) * DLD + SB * p + c];
+      ulonglong2 u = load_pairs(row);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const float x = L[k][lane];
-        const float4 l = *reinterpret_cast<const float4*>(&L[k][c]);
-        u.x = fmaf(-x, l.x, u.x); u.y = fmaf(-x, l.y, u.y);
-        u.z = fmaf(-x, l.z, u.z); u.w = fmaf(-x, l.w, u.w);
+        const ulonglong2 l = load_pairs(&L[k][c]);
+        const f32x2 nx = pair(-x, -x);
+        u.x = fma2(nx, l.x, u.x); u.y = fma2(nx, l.y, u.y);
       }
-      *row = u;
+      store_pairs(row, u.x, u.y);
       __syncwarp();
     }
     bar_arrive(kBarNext + s + 1, 32 + 32 * kRestWarps);
   }
 }
 
-template <int NC>
-__device__ __forceinline__ void diag_follow_step(const DiagSmem& sm, int s,
-                                                 float a[2][SB], float* row0,
-                                                 float* row1) {
+// Eight columns (step s) of a row as three bf16 terms, 24 significant bits, into the
+// operand tiles: hi and mid in the halves of a row of the first, lo in the second.
+// (lo is cut off, not rounded, which keeps a NaN.)
+__device__ __forceinline__ void diag_store_terms(unsigned tile, int row, int s,
+                                                 const float x[8]) {
+  unsigned hi[4], mid[4], lo[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float x0 = x[2 * i], x1 = x[2 * i + 1];
+    const unsigned a0 = __float_as_uint(x0) + 0x8000u;
+    const unsigned a1 = __float_as_uint(x1) + 0x8000u;
+    hi[i] = __byte_perm(a0, a1, 0x7632);
+    const float y0 = x0 - __uint_as_float(a0 & 0xffff0000u);
+    const float y1 = x1 - __uint_as_float(a1 & 0xffff0000u);
+    const unsigned b0 = __float_as_uint(y0) + 0x8000u;
+    const unsigned b1 = __float_as_uint(y1) + 0x8000u;
+    mid[i] = __byte_perm(b0, b1, 0x7632);
+    lo[i] = __byte_perm(__float_as_uint(y0 - __uint_as_float(b0 & 0xffff0000u)),
+                        __float_as_uint(y1 - __uint_as_float(b1 & 0xffff0000u)),
+                        0x7632);
+  }
+  auto put = [&](unsigned t, int chunk, const unsigned v[4]) {
+    sts128(t + sw128_chunk_off(row, chunk),
+           make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]),
+                       __uint_as_float(v[2]), __uint_as_float(v[3])));
+  };
+  put(tile, s, hi);
+  put(tile, 4 + s, mid);
+  put(tile + kDiagTile, s, lo);
+}
+
+// Step s of a row per lane.  `out` gets the finished values (NULL: a row of L that
+// nothing reads but as an operand), `tile` its terms (0: none; row `tile_row`);
+// `crit`, if given, is told when they are in `out`.
+__device__ __forceinline__ void diag_follow_step(const DiagSmem& sm, int p, int s,
+                                                 f32x2 a[SB / 2], float* out,
+                                                 unsigned tile, int tile_row,
+                                                 int lane,
+                                                 unsigned long long* crit) {
   const int j = 8 * s;
-  const float (*L)[LSP] = &sm.Ls[j];
-  float r[8], l[8][8], x[2][8];
+  const float (*L)[LSP] = &sm.Ls[p & 1][j];
+  float r[8], l[8][8], x[8];
 #pragma unroll
   for (int k = 0; k < 8; k += 4) {
-    const float4 v = *reinterpret_cast<const float4*>(&sm.rl[j + k]);
+    const float4 v = *reinterpret_cast<const float4*>(&sm.rl[p & 1][j + k]);
     r[k] = v.x; r[k + 1] = v.y; r[k + 2] = v.z; r[k + 3] = v.w;
   }
 #pragma unroll
@@ -686,120 +799,222 @@ __device__ __forceinline__ void diag_follow_step(const DiagSmem& sm, int s,
       l[i][k] = v.x; l[i + 1][k] = v.y; l[i + 2][k] = v.z; l[i + 3][k] = v.w;
     }
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) x[q][k] = a[q][k];
-    diag_solve8(x[q], r, [&](int i, int k) { return l[i][k]; });
-    float4* row = reinterpret_cast<float4*>(&(q ? row1 : row0)[j]);
-    row[0] = make_float4(x[q][0], x[q][1], x[q][2], x[q][3]);
-    row[1] = make_float4(x[q][4], x[q][5], x[q][6], x[q][7]);
+  for (int k = 0; k < 8; k += 2) {
+    const float2 v = unpair(a[k / 2]);
+    x[k] = v.x; x[k + 1] = v.y;
   }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    x[k] *= r[k];
+#pragma unroll
+    for (int i = k + 1; i < 8; ++i) x[i] = fmaf(-x[k], l[i][k], x[i]);
+  }
+  if (out != nullptr) {
+    float4* row = reinterpret_cast<float4*>(&out[j]);
+    row[0] = make_float4(x[0], x[1], x[2], x[3]);
+    row[1] = make_float4(x[4], x[5], x[6], x[7]);
+  }
+  if (crit != nullptr) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&crit[s]);
+  }
+  if (tile != 0) diag_store_terms(tile, tile_row, s, x);
   // the registers move down by eight columns
+  f32x2 nx[8];
 #pragma unroll
-  for (int c = 0; c < NC; c += 4) {
-    float4 u = make_float4(a[0][c + 8], a[0][c + 9], a[0][c + 10], a[0][c + 11]);
-    float4 v = make_float4(a[1][c + 8], a[1][c + 9], a[1][c + 10], a[1][c + 11]);
+  for (int k = 0; k < 8; ++k) nx[k] = pair(-x[k], -x[k]);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float4 w = *reinterpret_cast<const float4*>(&L[k][j + 8 + c]);
-      u.x = fmaf(-x[0][k], w.x, u.x); v.x = fmaf(-x[1][k], w.x, v.x);
-      u.y = fmaf(-x[0][k], w.y, u.y); v.y = fmaf(-x[1][k], w.y, v.y);
-      u.z = fmaf(-x[0][k], w.z, u.z); v.z = fmaf(-x[1][k], w.z, v.z);
-      u.w = fmaf(-x[0][k], w.w, u.w); v.w = fmaf(-x[1][k], w.w, v.w);
+  for (int c = 0; c < 24; c += 8) {
+    if (c >= 24 - j) break;
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+      const int d = (c + h) / 2;
+      f32x2 u = a[d + 4], v = a[d + 5];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const ulonglong2 w = load_pairs(&L[k][j + 8 + c + h]);
+        u = fma2(nx[k], w.x, u);
+        v = fma2(nx[k], w.y, v);
+      }
+      a[d] = u; a[d + 1] = v;
     }
-    a[0][c] = u.x; a[0][c + 1] = u.y; a[0][c + 2] = u.z; a[0][c + 3] = u.w;
-    a[1][c] = v.x; a[1][c + 1] = v.y; a[1][c + 2] = v.z; a[1][c + 3] = v.w;
   }
 }
 
-// row <- row L_pp^-T for two rows per lane, step by step behind diag_base.
-// `unit0` / `unit1`: the row starts as the unit vector e_lane and ends as row
+// D(128 x 32 nc) += rows of the operand tiles times rows 32 c .. of them, in six
+// terms (all but mid lo, lo mid and lo lo): columns 32 c .. of the accumulators for
+// hi hi, those 128 columns on for the others.  The tensor core adds with
+// truncation; products of 8-bit terms leave it little to cut off, and what it cuts
+// off the others is below their 2^-8.
+__device__ __forceinline__ void diag_mma(unsigned tmem, unsigned tile, int c,
+                                         int nc, bool first) {
+  constexpr unsigned long long mid = 64 >> 4, lo = kDiagTile >> 4;
+  const unsigned idesc = tc_bf16_desc(SB * nc);
+  const unsigned d = tmem + SB * c;
+  unsigned long long a = tc_smem_desc(tile);
+  unsigned long long b = tc_smem_desc(tile + c * SB * 128);
+#pragma unroll 1
+  for (int kk = 0; kk < 2; ++kk) {
+    const unsigned acc = !first || kk > 0;
+    tc_mma_half(d + DB, a + lo, b, idesc, acc);
+    tc_mma_half(d + DB, a, b + lo, idesc, 1u);
+    tc_mma_half(d + DB, a + mid, b + mid, idesc, 1u);
+    tc_mma_half(d + DB, a + mid, b, idesc, 1u);
+    tc_mma_half(d + DB, a, b + mid, idesc, 1u);
+    tc_mma_half(d, a, b, idesc, acc);
+    a += 32 >> 4;
+    b += 32 >> 4;
+  }
+}
+
+// Zeros into a warp's lanes of 32 columns of tensor memory.
+__device__ __forceinline__ void diag_clear(unsigned taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+      "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};"
+      ::"r"(taddr), "r"(0)
+      : "memory");
+}
+
+// 32 columns of a warp's lanes of tensor memory: the hi hi and cross accumulators.
+__device__ __forceinline__ void diag_fetch(unsigned t, f32x2 v[SB / 2]) {
+#pragma unroll
+  for (int cc = 0; cc < SB; cc += 16) {
+    float m[16], x[16];
+    tc_ld16_pair(t + cc, t + DB + cc, m, x);
+#pragma unroll
+    for (int i = 0; i < 16; i += 2)
+      v[(cc + i) / 2] = pair(m[i] + x[i], m[i + 1] + x[i + 1]);
+  }
+}
+
+// row <- row L_pp^-T for a row per lane, step by step behind diag_base: row `lane`
+// of row-block r, columns of sub-block p.  A row of D (r > p) comes from S less the
+// products collected in tensor memory, one of X^T (r < p) is minus them; that of
+// X^T's new row-block (r == p) starts as the unit vector e_lane and ends as row
 // `lane` of X_pp^T.
-__device__ __forceinline__ void diag_follow(const DiagSmem& sm, int lane,
-                                            int followers, float* row0,
-                                            float* row1, bool unit0,
-                                            bool unit1) {
-  float a[2][SB];
+__device__ __forceinline__ void diag_follow(DiagSmem& sm, DiagControl* ctl,
+                                            unsigned tmem, int p, int np, int r,
+                                            int lane, unsigned tile) {
+  f32x2 a[SB / 2];
+  float* src = &sm.S[(SB * r + lane) * DLD + SB * p];
+  float* out = r == p ? &sm.XD[p][lane * SLP] : r <= p + 1 ? src : nullptr;
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
-#pragma unroll
-    for (int j = 0; j < SB; j += 4) {
-      float4 v = make_float4(j == lane ? 1.f : 0.f, j + 1 == lane ? 1.f : 0.f,
-                             j + 2 == lane ? 1.f : 0.f, j + 3 == lane ? 1.f : 0.f);
-      if (!(q ? unit1 : unit0))
-        v = *reinterpret_cast<const float4*>(&(q ? row1 : row0)[j]);
-      a[q][j] = v.x; a[q][j + 1] = v.y; a[q][j + 2] = v.z; a[q][j + 3] = v.w;
-    }
-#pragma unroll 1
-  for (int s = 0; s < 2; ++s) {
-    bar_sync(kBarStep + s, followers + 32 * kRestWarps);
-    diag_follow_step<24>(sm, s, a, row0, row1);
+  for (int j = 0; j < SB; j += 4) {
+    ulonglong2 v = make_ulonglong2(0, 0);
+    if (r > p) v = load_pairs(&src[j]);
+    if (r == p && (lane & ~3) == j)
+      v = make_ulonglong2(pair(j == lane ? 1.f : 0.f, j + 1 == lane ? 1.f : 0.f),
+                          pair(j + 2 == lane ? 1.f : 0.f, j + 3 == lane ? 1.f : 0.f));
+    a[j / 2] = v.x; a[j / 2 + 1] = v.y;
   }
+  if (p > 0) {
+    if (r != p) {
+      if (diag_wait_tmem(&ctl->next, (p - 1) & 1, &ctl->abort_flag)) {
+        f32x2 t[SB / 2];
+        diag_fetch(tmem + ((unsigned)(SB * r) << 16) + (unsigned)(SB * p), t);
+        const f32x2 minus = pair(-1.f, -1.f);
+#pragma unroll
+        for (int j = 0; j < SB / 2; ++j) a[j] = fma2(t[j], minus, a[j]);
+      }
+    }
+    // the products of the sub-block before have read the tiles
+    diag_wait(&ctl->beyond, (p - 1) & 1, &ctl->abort_flag);
+  }
+  unsigned long long* crit = r == p + 1 ? ctl->crit[p] : nullptr;
 #pragma unroll 1
-  for (int s = 2; s < 4; ++s) {
-    bar_sync(kBarStep + s, followers);
-    diag_follow_step<8>(sm, s, a, row0, row1);
+  for (int s = 0; s < 4; ++s) {
+    diag_wait(&ctl->step[p][s], 0, &ctl->abort_flag);
+    diag_follow_step(sm, p, s, a, out, tile, SB * r + lane, lane, crit);
   }
 }
 
-// C(8 RI x ..) -= A B^T over 32 k by one warp: lane (rg, cg) holds rows
-// rg + RG i, columns cg + CG j (RG CG = 32); A and B are contiguous along k.
-// The 16-byte loads of a quarter warp fall into different banks.  `fresh`: C
-// starts from zero.
-template <int RG, int RI, int CJ>
-__device__ __forceinline__ void diag_mac(float* C, const float* A, int pa,
-                                         const float* B, int lane, bool fresh) {
-  constexpr int CG = 32 / RG;
-  const int rg = lane / CG, cg = lane % CG;
-  const float* ar = A + rg * pa;
-  const float* br = B + cg * DLD;
-  float acc[RI][CJ];
+// The next diagonal sub-block loses its row-block's product with itself, eight
+// columns as soon as they are there: 16 rows from r0 on, 16 columns from c0 on.
+// Lane (rg, cg) holds rows rg + 8 i, columns cg + 4 j, sums over even and odd k.
+__device__ __forceinline__ void diag_next(DiagSmem& sm, DiagControl* ctl, int p,
+                                          int r0, int c0, int lane) {
+  constexpr int CJ = 4;
+  const int rg = lane >> 2, cg = lane & 3;
+  float* C = &sm.S[(SB * (p + 1) + r0 + rg) * DLD + SB * (p + 1) + c0 + cg];
+  const float* A = &sm.S[(SB * (p + 1) + r0 + rg) * DLD + SB * p];
+  const float* B = &sm.S[(SB * (p + 1) + c0 + cg) * DLD + SB * p];
+  float d[2][CJ];
+  f32x2 acc[2][CJ];
 #pragma unroll
-  for (int i = 0; i < RI; ++i)
-#pragma unroll
-    for (int j = 0; j < CJ; ++j) acc[i][j] = 0.f;
-#pragma unroll 2
-  for (int k = 0; k < SB; k += 4) {
-    float av[RI][4], bv[CJ][4];
-#pragma unroll
-    for (int i = 0; i < RI; ++i) {
-      const float4 v = *reinterpret_cast<const float4*>(&ar[RG * i * pa + k]);
-      av[i][0] = v.x; av[i][1] = v.y; av[i][2] = v.z; av[i][3] = v.w;
-    }
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < CJ; ++j) {
-      const float4 v = *reinterpret_cast<const float4*>(&br[CG * j * DLD + k]);
-      bv[j][0] = v.x; bv[j][1] = v.y; bv[j][2] = v.z; bv[j][3] = v.w;
+      d[i][j] = C[8 * i * DLD + 4 * j];
+      acc[i][j] = 0;
     }
-    // (consecutive multiply-adds go to different accumulators)
+#pragma unroll 1
+  for (int s = 0; s < 4; ++s) {
+    diag_wait(&ctl->crit[p][s], 0, &ctl->abort_flag);
+#pragma unroll 1
+    for (int k = 8 * s; k < 8 * s + 8; k += 4) {
+      ulonglong2 a[2];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
+      for (int i = 0; i < 2; ++i) a[i] = load_pairs(&A[8 * i * DLD + k]);
 #pragma unroll
-      for (int j = 0; j < CJ; ++j)
+      for (int j = 0; j < CJ; ++j) {
+        const ulonglong2 b = load_pairs(&B[4 * j * DLD + k]);
 #pragma unroll
-        for (int i = 0; i < RI; ++i)
-          acc[i][j] = fmaf(av[i][e], bv[j][e], acc[i][j]);
+        for (int i = 0; i < 2; ++i) {
+          acc[i][j] = fma2(a[i].x, b.x, acc[i][j]);
+          acc[i][j] = fma2(a[i].y, b.y, acc[i][j]);
+        }
+      }
+    }
   }
-  float* dst = C + rg * DLD + cg;
 #pragma unroll
-  for (int i = 0; i < RI; ++i)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < CJ; ++j) {
-      const float v = fresh ? 0.f : dst[RG * i * DLD + CG * j];
-      dst[RG * i * DLD + CG * j] = v - acc[i][j];
+      const float2 v = unpair(acc[i][j]);
+      C[8 * i * DLD + 4 * j] = d[i][j] - (v.x + v.y);
     }
 }
 
-// Row-block r of column c of the working matrix loses its product with row c
-// of column p: r > c are rows of the block, r < c (r <= p) rows of X^T.
-// `half`: its upper or lower 16 rows.
-__device__ __forceinline__ void diag_update_block(DiagSmem& sm, int r, int half,
-                                                  int c, int p, int lane) {
-  const float* A = r == p ? &sm.XD[p][16 * half * SLP]
-                          : &sm.S[(SB * r + 16 * half) * DLD + SB * p];
-  diag_mac<8, 2, 8>(&sm.S[(SB * r + 16 * half) * DLD + SB * c], A,
-                    r == p ? SLP : DLD, &sm.S[SB * c * DLD + SB * p], lane,
-                    r == p);
+// Sub-block (p, u) of X, or its upper or lower half, to global memory: a lane
+// takes a 4 x 4 block, four words along the rows of X^T, turned by naming
+// registers, so that X and its fp16 terms are stored in words of four columns.
+// Lanes are laid out so that a quarter warp's loads fall into different banks.
+__device__ __forceinline__ void diag_store(const DiagSmem& sm, const MatInfo& mi,
+                                           int o, int bs, int p, int u, int half,
+                                           int lane, int pack) {
+  const long long ld = mi.ld;
+  float* Xd = mi.X + (long long)o * ld + o;
+  unsigned char* const px = mi.PX + (long long)(o / DB) * mi.tile;
+  const int c = 4 * (lane >> 2), r = 16 * half + 4 * (lane & 3);
+  float x[4][4];              // [column][row]
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float4 v = *reinterpret_cast<const float4*>(
+        u == p ? &sm.XD[u][(c + e) * SLP + r]
+               : &sm.S[(SB * u + c + e) * DLD + SB * p + r]);
+    x[e][0] = v.x; x[e][1] = v.y; x[e][2] = v.z; x[e][3] = v.w;
+  }
+  const int gc = SB * u + c;
+  const int gr0 = SB * p + r;
+  float* dst = Xd + gr0 * ld + gc;
+  unsigned char* q = px + (long long)((o + gr0) >> 5) * kChunk + (gc >> 6) * 8192 +
+                     8 * ((gc >> 2) & 1);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if (gr0 + e >= bs) break;
+    // (columns past bs are zeros above the diagonal, inside the row pitch)
+    *reinterpret_cast<float4*>(dst + e * ld) =
+        make_float4(x[0][e], x[1][e], x[2][e], x[3][e]);
+    if (!pack) continue;
+    unsigned h0, h1, l0, l1;
+    split_half2(kScaleX * x[0][e], kScaleX * x[1][e], h0, l0);
+    split_half2(kScaleX * x[2][e], kScaleX * x[3][e], h1, l1);
+    unsigned char* w = q + sw128_chunk_off((gr0 + e) & 31, (gc & 63) >> 3);
+    *reinterpret_cast<uint2*>(w) = make_uint2(h0, h1);
+    *reinterpret_cast<uint2*>(w + 4096) = make_uint2(l0, l1);
+  }
 }
 
 // Factor one diagonal block (<= 128 x 128) of W and invert the resulting
@@ -809,13 +1024,32 @@ __device__ __forceinline__ void diag_update_block(DiagSmem& sm, int r, int half,
 // Elimination of [D; I] by four sub-blocks of 32 columns: row-blocks in play at
 // sub-block p are p .. 3 of D and 0 .. p of X^T (which starts as I).  Bound:
 // the serial chain of 128 pivots.  So per sub-block one warp runs the pivot
-// chain alone (diag_base), two warps carry the other four row-blocks behind
-// it, two rows per lane (diag_follow), and the product of the finished column
-// with the next one is split: its diagonal sub-block first (six warps, then
-// the chain goes on), the rows that follow it (six warps, then the followers
-// go on), and the columns beyond next to the next chain.  128 rows: 61 us with
-// 8 x 8 register blocks per thread and a barrier per block column, 20 us now with
-// the launch, 29 us with the look-ahead's two products in front.
+// chain alone (diag_base), four apply what it leaves of its own updates, a warp per
+// row-block carries the others behind it (diag_follow), and three take the next
+// row-block's products out of the next diagonal sub-block, where the chain goes on
+// (diag_next).
+//
+// All other products of the finished columns with the later ones run on the tensor
+// cores (tcgen05): the followers leave their rows as bf16 terms, and D(r, c) and
+// X^T(r, c) lose rows r times rows c, for all r at once, collected in tensor
+// memory over the sub-blocks; first the next column, which the followers fetch,
+// then those beyond.  Row-block r takes D's products with columns it does not have
+// until X^T's row r begins: its warp clears those accumulators before.
+//
+// What bounds the work beside the chain, measured in cycles of the block at 128
+// rows: these products on the CUDA cores, six warps with 2 x 8 values a lane, took
+// 12 800 cycles of shared-memory loads, more than the chain itself takes, and
+// delayed its own loads; in two TF32 terms they were as fast as now but left
+// inverses of 128 rows 1.24 times the error, in three bf16 terms 0.92 times.
+// Followers on mma.sync take 1400 cycles a step, with multiply-adds 550 to 1150.
+// And the instruction cache of an SM holds about 2000 instructions: code that does
+// not fit, or runs once, costs three cycles an instruction and more, so loops that
+// are not the chain's are left rolled (8200 instructions with the look-ahead,
+// 46 900 cycles; 3400 now, 42 000; 56 000 before all of this).
+//
+// 128 rows: 16 us with the launch, 22 us with the look-ahead in front (20.5 and 30
+// before); a row panel of X is stored when its sub-block is through, beside the
+// next.
 template <bool LOOK>
 __global__ void __launch_bounds__(DT, 1)
 chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
@@ -827,134 +1061,136 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
   // written only after its last barrier
   unsigned char* stage = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(dsm + DB * DLD) + 1023) & ~(uintptr_t)1023);
-  LookControl* ctl = reinterpret_cast<LookControl*>(stage + kLookBytes);
+  DiagControl* ctl = reinterpret_cast<DiagControl*>(
+      stage + (LOOK ? kLookBytes : kDiagStage));
   const MatInfo mi = mats[blockIdx.x];
   const int id = mi.id;
   const int o = step * DB;
   const int bs = min(DB, mi.d - o);
   const int np = (bs + SB - 1) / SB;      // sub-blocks in use
-  const long long ld = mi.ld;
   if (LOOK) {
-    if (!diag_lookahead(mi, o, bs, sm.S, stage, ctl)) return;
+    diag_lookahead(mi, o, bs, sm.S, stage, ctl);
   } else {
-    diag_load(mi.W + (long long)o * ld + o, ld, bs, sm.S);
+    diag_load(mi.W + (long long)o * mi.ld + o, mi.ld, bs, sm.S);
+    diag_begin(ctl, np);
     diag_load_wait();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
   __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem = ctl->tmem_base;
+  const unsigned tile = smem_u32(stage + kDiagStage - 2 * kDiagTile);
 
-  const int followers = 32 * (1 + (np + 1) / 2);   // threads of a step barrier
-  // roles: 0 chain; 3, 4, 8, 12 the rest of its updates (on 3, 13 .. 15, which
-  // keeps them from the chain's scheduler: 0.4 % slower at 2304 and 4608 rows);
-  // 1, 2 followers; 5 6 7 9 10 11 rows and columns behind them; 3, 12 .. 15 the
-  // diagonal sub-block, with 0
-  const bool diag_warp = warp == 0 || warp == 3 || warp >= 12;
-  const bool work_warp = warp >= 5 && warp <= 11 && warp != 8;
-  const int worker = warp < 8 ? warp - 5 : warp - 6;            // 0 .. 5
-  for (int p = 0; p < np; ++p) {
-    if (p > 0) {
-      // product of sub-block column p - 1 with column p (this panel) ...
-      if (diag_warp) {
-        // lower 16 x 16 quadrants (0,0) (1,0) (1,1), 8 rows per warp
-        const int u = warp == 0 ? 0 : warp == 3 ? 1 : warp - 10;
-        const int r = (u < 2 ? 0 : 16) + 8 * (u & 1), c = u < 4 ? 0 : 16;
-        const int base = SB * p * DLD + SB * (p - 1);
-        diag_mac<4, 2, 2>(&sm.S[(SB * p + r) * DLD + SB * p + c],
-                          &sm.S[base + r * DLD], DLD, &sm.S[base + c * DLD],
-                          lane, false);
-        bar_sync(kBarDiag, 6 * 32);
-      } else if (work_warp || warp == 1 || warp == 2) {
-        if (work_warp && worker < 2 * (np - 1)) {
-          const int q = worker >> 1;         // rows below, then rows of X^T
-          const int r = q < np - 1 - p ? p + 1 + q : q - (np - 1 - p);
-          diag_update_block(sm, r, worker & 1, p, p - 1, lane);
-        }
-        bar_sync(kBarRows, 8 * 32);
-      }
+  // A row panel of X is stored by two warps beside the next sub-block, the last
+  // one by all that have nothing else to do then.
+  constexpr int kStore = 2, kStoreLast = 9;
+  int slot = -1, first = np - 1;           // of a storing warp, its first panel
+  if (warp == 0) {
+#pragma unroll 1
+    for (int p = 0; p < np; ++p) {
+      if (p > 0) bar_sync(kBarDiag, 128);
+      diag_base(sm, ctl, p, lane, id, o + SB * p, info);
     }
-    if (warp == 0) {
-      diag_base(sm, p, lane, id, o + SB * p, followers, info);
-    } else if (warp == 3 || (warp & 3) == 0) {
-      diag_base_rest(sm, p, lane, warp == 3 ? 3 : (warp >> 2) - 1, followers);
-    } else if (warp <= 2) {
-      const int q = 2 * (warp - 1);
-      if (q < np) {
-        float* row[2];
-        bool unit[2];
+  } else if (warp == 1 || (warp >= 4 && warp < 4 + np)) {
+    // row-block warp - 4 (its lanes of tensor memory), warp 1: X^T's new rows
+#pragma unroll 1
+    for (int p = 0; p < np; ++p) {
+      const int r = warp == 1 ? p : warp - 4;
+      const bool last = p == np - 1;
+      if (warp == 1 || r != p) {
+        diag_follow(sm, ctl, tmem, p, np, r, lane, last ? 0u : tile);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      } else if (p > 0 && !last) {
+        // from here on row-block r collects rows of X^T
+        const bool ok = diag_wait_tmem(&ctl->beyond, (p - 1) & 1, &ctl->abort_flag);
+#pragma unroll 1
+        for (int c = 2 * (p + 1); ok && c < 2 * np; ++c)
+          diag_clear(tmem + ((unsigned)(SB * r) << 16) +
+                     (unsigned)(SB * (c >> 1) + DB * (c & 1)));
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      }
+      bar_arrive(kBarStore + p, 32 * (np + 1 + (last ? kStoreLast : kStore)));
+      if (last) break;
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->rows);
+    }
+  } else if (warp == 3) {
+#pragma unroll 1
+    for (int p = 0; p < np - 1; ++p) {
+      const bool go = diag_wait_tmem(&ctl->rows, p & 1, &ctl->abort_flag);
+      if (go && elect_one()) {
+#pragma unroll 1
+        for (int part = 0; part < 2; ++part) {
+          const int c = p + 1 + part, nc = part ? np - 2 - p : 1;
+          if (nc > 0) diag_mma(tmem, tile, c, nc, p == 0);
+          tc_commit(part ? &ctl->beyond : &ctl->next);
+        }
+      }
+      __syncwarp();
+    }
+  } else if (warp == 9 || warp == 10 || warp == 11 || warp == 13) {
+    const int h = warp == 13 ? 3 : warp - 9;
+#pragma unroll 1
+    for (int p = 0; p < np; ++p) diag_base_rest(sm, ctl, p, lane, h);
+    slot = h + 5;
+  } else if (warp == 2 || warp >= 14) {
+    const int u = warp == 2 ? 0 : warp - 13, r = warp - 12;
+#pragma unroll 1
+    for (int p = 0; p < np - 1; ++p) {
+      if (p == 0) {
+        if (u == 0 && lane == 0) mbar_arrive(&ctl->rows);
+      } else {
+        if (r == p + 1) {
+          // what earlier sub-blocks have collected for the next diagonal one
+          if (diag_wait_tmem(&ctl->beyond, (p - 1) & 1, &ctl->abort_flag)) {
+            f32x2 t[SB / 2];
+            diag_fetch(tmem + ((unsigned)(SB * r) << 16) + (unsigned)(SB * r), t);
+            float* row = &sm.S[(SB * r + lane) * DLD + SB * r];
+            const f32x2 minus = pair(-1.f, -1.f);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          // rows below, then rows 0 .. p of X^T (an odd last one twice)
-          const int f = min(q + e, np - 1);
-          const int r = f < np - 1 - p ? p + 1 + f : f - (np - 1 - p);
-          unit[e] = r == p;
-          row[e] = unit[e] ? &sm.XD[p][lane * SLP]
-                           : &sm.S[(SB * r + lane) * DLD + SB * p];
+            for (int j = 0; j < SB; j += 4) {
+              const ulonglong2 v = load_pairs(&row[j]);
+              store_pairs(&row[j], fma2(t[j / 2], minus, v.x),
+                          fma2(t[j / 2 + 1], minus, v.y));
+            }
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl->rows);
         }
-        diag_follow(sm, lane, followers, row[0], row[1], unit[0], unit[1]);
+        bar_sync(kBarPre, 96);
       }
-    } else if (p > 0 && work_warp) {
-      // ... and with the columns beyond it, next to this panel's chain: rows
-      // c .. np - 1 of the block and rows 0 .. p - 1 of X^T
-      int first = 0;
-      for (int c = p + 1; c < np; ++c) {
-        const int n = 2 * (np - c + p);
-        for (int u = (worker + 12 - first) % 6; u < n; u += 6) {
-          const int q = u >> 1;
-          diag_update_block(sm, q < np - c ? c + q : q - (np - c), u & 1, c,
-                            p - 1, lane);
-        }
-        first = (first + n) % 6;
-      }
+      diag_next(sm, ctl, p, u ? 16 : 0, u == 2 ? 16 : 0, lane);
+      bar_arrive(kBarDiag, 128);
     }
-    __syncthreads();
+    slot = u + 2;
+  } else if (warp == 8 || warp == 12) {
+    slot = warp == 8 ? 0 : 1;
+    first = 0;
   }
-
-  // ---- X to global memory: a warp turns 32 columns x 4 rows of X^T (one
-  // 16-byte word per lane) into four contiguous row pieces.  The part above
-  // the diagonal sub-blocks was zeroed when the plan was made.
-  float* Xd = mi.X + (long long)o * ld + o;
-  // (from X and d: two more pointers across the chain cost registers that it
-  // does not have)
-  const long long ptile =
-      (long long)((mi.d + DB - 1) / DB) * (DB / 32) * kChunk;
-  unsigned char* const px = reinterpret_cast<unsigned char*>(mi.X) +
-                            matrix_bytes(mi.d) + step * ptile;
-  // a warp takes 16 rows x 32 columns, a lane a 4 x 4 block: four words along the
-  // rows of X^T, turned by naming registers, so that X and its fp16 terms are
-  // stored in words of four columns.  Lanes are laid out so that a quarter
-  // warp's loads fall into different banks.  (2.2 us with a column of four rows
-  // a lane, 2.0 us now; the rest is what one SM can store.)
-  const int nb = (bs + SB - 1) / SB;
-  for (int item = warp; item < nb * (nb + 1); item += DT / 32) {
-    int bi = 0, u = item >> 1;
-    while (u > bi) u -= ++bi;
-    const int c = 4 * (lane >> 2), r = 16 * (item & 1) + 4 * (lane & 3);
-    float x[4][4];              // [column][row]
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float4 v = *reinterpret_cast<const float4*>(
-          u == bi ? &sm.XD[u][(c + e) * SLP + r]
-                  : &sm.S[(SB * u + c + e) * DLD + SB * bi + r]);
-      x[e][0] = v.x; x[e][1] = v.y; x[e][2] = v.z; x[e][3] = v.w;
+  if (slot >= 0) {
+#pragma unroll 1
+    for (int p = first; p < np; ++p) {
+      const int warps = p == np - 1 ? kStoreLast : kStore;
+      bar_sync(kBarStore + p, 32 * (np + 1 + warps));
+      if (ctl->abort_flag != 0) continue;
+#pragma unroll 1
+      for (int u = slot; u < 2 * (p + 1); u += warps)
+        diag_store(sm, mi, o, bs, p, u >> 1, u & 1, lane, pack);
     }
-    const int gc = SB * u + c;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int gr = SB * bi + r + e;
-      if (gr >= bs) continue;
-      // (columns past bs are zeros above the diagonal, inside the row pitch)
-      *reinterpret_cast<float4*>(Xd + gr * ld + gc) =
-          make_float4(x[0][e], x[1][e], x[2][e], x[3][e]);
-      if (!pack) continue;
-      unsigned h0, h1, l0, l1;
-      split_half2(kScaleX * x[0][e], kScaleX * x[1][e], h0, l0);
-      split_half2(kScaleX * x[2][e], kScaleX * x[3][e], h1, l1);
-      unsigned char* q = px + (long long)((o + gr) >> 5) * kChunk +
-                         (gc >> 6) * 8192 +
-                         sw128_chunk_off(gr & 31, (gc & 63) >> 3) +
-                         8 * ((gc >> 2) & 1);
-      *reinterpret_cast<uint2*>(q) = make_uint2(h0, h1);
-      *reinterpret_cast<uint2*>(q + 4096) = make_uint2(l0, l1);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    if (ctl->abort_flag != 0) {
+      // (its own copies have to be over before the block is)
+      if (LOOK) mbar_wait_status(&ctl->x_here, 0, &ctl->grace, &g_diag_status);
+      if (lane == 0) atomicExch(&g_diag_status, 1);
     }
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+                 ::"r"(tmem), "r"(kDiagCols)
+                 : "memory");
   }
 }
 
@@ -1170,11 +1406,13 @@ refine_apply_kernel(const MatInfo* __restrict__ mats,
       mi.inv[(long long)r * it.d + c] += mi.V[(long long)r * mi.ld + c];
 }
 
-constexpr size_t kDiagSmemBytes = sizeof(DiagSmem);
+constexpr int kDiagControl = 512;
+constexpr size_t kDiagSmemBytes =
+    DB * DLD * sizeof(float) + 1024 + kDiagStage + kDiagControl;
 constexpr size_t kDiagLookSmemBytes =
-    DB * DLD * sizeof(float) + 1024 + kLookBytes + 256;
+    DB * DLD * sizeof(float) + 1024 + kLookBytes + kDiagControl;
 static_assert(kDiagLookSmemBytes >= kDiagSmemBytes &&
-                  kDiagLookSmemBytes <= 227 * 1024,
+                  kDiagLookSmemBytes <= 227 * 1024 && sizeof(DiagControl) <= kDiagControl,
               "diagonal kernel shared memory");
 
 // Streams of one run: the chain of diagonal kernels, panel solves and updates
@@ -1332,7 +1570,6 @@ extern "C" int kfac_inverse_plan_create(
     m.id = i;
     if (half) {
       m.tile = chunk_tile_bytes(dims[i]);
-      // (the diagonal kernel takes PX to lie right behind X)
       m.PX = reinterpret_cast<unsigned char*>(ws); ws += chunk_bytes(dims[i]);
       m.PL = reinterpret_cast<unsigned char*>(ws); ws += chunk_bytes(dims[i]);
     } else {

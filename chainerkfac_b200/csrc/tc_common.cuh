@@ -127,6 +127,12 @@ __device__ __forceinline__ unsigned tc_half_desc(int n, bool a_mn, bool b_mn) {
          ((unsigned)(n >> 3) << 17) | ((unsigned)(TC_BM >> 4) << 24);
 }
 
+// D = f32, A = B = bf16, both K-major, M = 128, N = n
+__device__ __forceinline__ unsigned tc_bf16_desc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) |
+         ((unsigned)(TC_BM >> 4) << 24);
+}
+
 __device__ __forceinline__ void tc_mma_half(unsigned tmem_d,
                                             unsigned long long da,
                                             unsigned long long db,
@@ -188,6 +194,23 @@ __device__ __forceinline__ void tc_ld16_pair(unsigned ta, unsigned tb,
     v[i] = __uint_as_float(r[i]);
     w[i] = __uint_as_float(s[i]);
   }
+}
+
+// 32 columns of 16 accumulator rows of a warp's quarter: v[4 j + 2 h + e] is row
+// lane / 4 + 8 h, column 8 j + 2 (lane % 4) + e.  The caller waits
+// (tcgen05.wait::ld).
+__device__ __forceinline__ void tc_ld_16x32(unsigned taddr, float v[16]) {
+  unsigned r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+        "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 // Byte offset of element (row, k) inside a K-major SW128 tile (k < 32).

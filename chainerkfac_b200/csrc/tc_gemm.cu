@@ -162,12 +162,6 @@ __device__ __forceinline__ void tc_tri_tile(int t, int& bi, int& bj) {
 // products hi*hi + hi*lo + lo*hi are exact in the fp32 accumulator.  Halves
 // the shared-memory bytes per k of the split-TF32 scheme (stores and tensor
 // core operand reads), which is what bounds the tile kernels.
-__device__ __forceinline__ unsigned tc_instr_desc_bf16(int n) {
-  // D = f32, A = B = bf16, both K-major, M = 128, N = n
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) |
-         ((unsigned)(TC_BM >> 4) << 24);
-}
-
 __device__ __forceinline__ void tc_mma_bf16(unsigned tmem_d,
                                             unsigned long long da,
                                             unsigned long long db,
@@ -588,7 +582,7 @@ tc_pair_kernel(const GemmDesc* __restrict__ descs, int ndesc,
   } else {
     // ===================== MMA issuer =====================
     if (elect_one()) {
-      const unsigned idesc = tc_instr_desc_bf16(n_inst);
+      const unsigned idesc = tc_bf16_desc(n_inst);
       const unsigned a_off = share ? (unsigned)PK_TILE_BYTES : 0u;
       for (int kb = 0; kb < nkb; ++kb) {
         const int s = kb % PK_STAGES;

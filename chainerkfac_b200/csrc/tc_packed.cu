@@ -82,22 +82,6 @@ __device__ __forceinline__ void bulk_load(unsigned dst, const void* src,
       : "memory");
 }
 
-// 32 columns of 16 accumulator rows of a warp's quarter: v[4 j + 2 h + e] is row
-// lane / 4 + 8 h, column 8 j + 2 (lane % 4) + e.
-__device__ __forceinline__ void tc_ld_16x32(unsigned taddr, float v[16]) {
-  unsigned r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-        "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
 // Elements of a 16 x 32 piece of C in that order, this lane's first at row r,
 // column c: f(i, row offset, column offset) for those stored, which are all
 // (WHOLE), or the ones in front of `rows` and `cols` and (lower) not above the

@@ -1061,6 +1061,37 @@ def test_inverse_around_block_sizes(ops, d):
     run_pairs(ops, [d], [max(1, d // 3)], 1e-3, seed=d)
 
 
+@pytest.mark.parametrize('blocks', [0, 1, 4])
+@pytest.mark.parametrize('rows', [1, 31, 32, 33, 64, 65, 95, 96, 97, 127, 128])
+def test_inverse_sub_blocks_of_the_diagonal_kernel(ops, blocks, rows):
+    """A last diagonal block of `rows` rows, on its own and behind others: its
+    sub-blocks of 32 columns and their remainders, with and without the update of
+    the block before it.  Error of entry (i, j) against sqrt(inv_ii inv_jj), which
+    a Cholesky factorisation bounds by the condition of the scaled factor (here at
+    most 35) times the rounding of sums of at most d terms, d 2^-24."""
+    d = 128 * blocks + rows
+    rng = np.random.default_rng(d)
+    x = rng.standard_normal((2 * d + 64, d)) * np.exp(rng.uniform(-3, 3, d))
+    f = (x.T @ x / len(x)).astype(np.float32)
+    f = (f + f.T) / 2
+    F = [dev(f)] * 3
+    inv = [torch.empty_like(F[0]) for _ in F]
+    plan = ops.InversePlan(F, inv, [-1] * 3, [2] * 3, scale=[1.0] * 3)
+    plan.set_refine(0)
+    plan.run(1e-7)
+    torch.cuda.synchronize()
+    assert host(plan.info).tolist() == [0] * 3
+    truth = np.linalg.inv(f.astype(np.float64) + 1e-7 * np.eye(d))
+    s = np.sqrt(np.diag(truth))
+    for i in inv:
+        got = host(i)
+        assert np.array_equal(got, got.T)
+        assert (np.abs(got - truth) / s[:, None] / s[None, :]).max() < \
+            35 * d * 2.0 ** -24
+    assert torch.equal(inv[0], inv[2])
+    plan.close()
+
+
 def test_precondition_matches_oracle(ops):
     rng = np.random.default_rng(11)
     shapes = [(10, 1000, True), (64, 147, True), (300, 129, False),
