@@ -1061,6 +1061,33 @@ def test_inverse_around_block_sizes(ops, d):
     run_pairs(ops, [d], [max(1, d // 3)], 1e-3, seed=d)
 
 
+@pytest.mark.parametrize('dims', [[129], [300, 10, 257], [640, 1100, 96],
+                                  [520] * 20])
+def test_inverse_by_graph_and_by_plain_launches(ops, monkeypatch, dims):
+    """The same launches in the same order: bit for bit, three runs over inputs
+    that change (the graph's kernels begin before the ones in front have ended)."""
+    rng = np.random.default_rng(len(dims))
+    F = [torch.empty((d, d), device='cuda') for d in dims]
+    plans, outs = [], []
+    for graph in ('1', '0'):
+        monkeypatch.setenv('KFAC_INVERSE_GRAPH', graph)
+        outs.append([torch.empty_like(f) for f in F])
+        plans.append(ops.InversePlan(F, outs[-1], [-1] * len(dims),
+                                     [2] * len(dims), scale=[1.0] * len(dims)))
+    for _ in range(3):
+        for f in F:
+            x = dev(rng.standard_normal((f.shape[0] + 50, f.shape[0])))
+            f.copy_(x.t() @ x / len(x))
+            f.copy_((f + f.t()) / 2)
+        for plan in plans:
+            plan.run(1e-2)
+        torch.cuda.synchronize()
+        for a, b in zip(*outs):
+            assert torch.isfinite(a).all() and torch.equal(a, b)
+    for plan in plans:
+        plan.close()
+
+
 @pytest.mark.parametrize('blocks', [0, 1, 4])
 @pytest.mark.parametrize('rows', [1, 31, 32, 33, 64, 65, 95, 96, 97, 127, 128])
 def test_inverse_sub_blocks_of_the_diagonal_kernel(ops, blocks, rows):
