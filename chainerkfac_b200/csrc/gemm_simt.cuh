@@ -249,7 +249,6 @@ enum GemmFlags {
 // hi terms of 32 k, 128 bytes each, then lo terms), both 128-byte swizzled.
 // Consecutive k-blocks of a 128-row tile follow each other.
 constexpr int kChunk = 16384;
-enum PackKind { PACK_NONE, PACK_K, PACK_MN };
 
 struct GemmDesc {
   Operand A, B;
@@ -279,12 +278,11 @@ struct GemmDesc {
   float sa, sb;            // G_HALF: powers of two that scale the operands
   const unsigned char *ca, *cb;  // G_PACKED: chunk of the first tile and k
   long long ca_tile, cb_tile;    // bytes from one 128-row tile to the next
-  // the result is also stored in chunks, as an operand of later products: rows
-  // of C are the chunks' rows (PACK_K) or their k (PACK_MN)
+  // if set, the result is also stored in chunks, as an operand of later products:
+  // rows of C are the chunks' k (MN-major)
   unsigned char* pack;     // chunk of C's first row and column
   long long pack_tile;
   float pack_scale;
-  int pack_kind;
   const float* unscale;    // if set, C(m, n) = .. + unscale[m] unscale[n] A B
   // preconditioning in chunks, see PackRows: factors of the first product's rows
   // and columns, exponents of the second's

@@ -213,7 +213,8 @@ constexpr int SB = 32;        // sub-block of the diagonal kernel
 constexpr int SLP = SB + 4;   // row pitch of a 32 x 32 sub-block
 constexpr int DT = 512;       // threads of the diagonal kernel
 constexpr int kLookTile = DB * 128;    // one fp16 term of 128 rows x 64 k
-constexpr int kLookBytes = 8 * kLookTile;       // both of A' and of X_pp
+constexpr int kLookX = 3 * kLookTile;           // X_pp, see look_load_x
+constexpr int kLookBytes = 4 * kLookTile + kLookX;
 constexpr int kDiagCols = 2 * DB;               // tensor-memory columns
 
 static __device__ int g_diag_status = 0;
@@ -267,14 +268,14 @@ __device__ __forceinline__ bool diag_wait_tmem(unsigned long long* bar,
   return __all_sync(0xffffffffu, ok);
 }
 
-// One product of the look-ahead, D(128 x 128) = A B^T over 128 k, 16 at a time:
-// operands as tiles of 64 k by term (hi, lo), then the next 64 k.  hi*hi goes to
-// columns [0, 128) of the tensor memory, the cross terms to [128, 256).  `lower`:
-// B's rows in front of the k of its columns are zeros, and not there.
+// D(128 x 128) = A B^T over 128 k, 16 at a time: operands as tiles of 64 k by term
+// (hi, lo), then the next 64 k.  hi*hi goes to columns [0, 128) of the tensor
+// memory, the cross terms to [128, 256).  `lower`: B is X_pp as look_load_x leaves
+// it.
 __device__ __forceinline__ void look_mma(unsigned tmem, unsigned a, unsigned b,
                                          bool lower) {
   constexpr unsigned long long lo = kLookTile >> 4;
-  unsigned long long da = tc_smem_desc(a), db = tc_smem_desc(b);
+  unsigned long long da = tc_smem_desc(a), db = tc_smem_desc(b), lo_b = lo;
 #pragma unroll 1
   for (int kk = 0; kk < 8; ++kk) {
     const int n0 = lower ? 32 * (kk >> 1) : 0;
@@ -282,12 +283,37 @@ __device__ __forceinline__ void look_mma(unsigned tmem, unsigned a, unsigned b,
     const unsigned idesc = tc_half_desc(DB - n0, false, false);
     const unsigned d = tmem + n0;
     tc_mma_half(d + DB, da + lo, bk, idesc, kk > 0);
-    tc_mma_half(d + DB, da, bk + lo, idesc, 1u);
+    tc_mma_half(d + DB, da, bk + lo_b, idesc, 1u);
     tc_mma_half(d, da, bk, idesc, kk > 0);
-    const unsigned long long adv = kk == 3 ? (2 * kLookTile - 96) >> 4 : 32 >> 4;
-    da += adv;
-    db += adv;
+    da += (kk == 3 ? 2 * kLookTile - 96 : 32) >> 4;
+    if (kk == 3 && lower) lo_b = lo / 2;
+    db += (kk != 3 ? 32 : lower ? 3 * kLookTile / 2 - 96 : 2 * kLookTile - 96) >> 4;
   }
+}
+
+// X_pp (columns and rows from xo on) from its chunks to tx, by twelve lanes: rows of
+// 64 columns, K-major as a B operand: columns 0 .. 63 hi, then lo, and columns 64
+// .. hi and lo of rows 64 .. only (those above are zeros, and not read).
+__device__ __forceinline__ void look_load_x(const MatInfo& mi, int xo, unsigned tx,
+                                            unsigned long long* bar, int lane) {
+  if (lane == 0)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                 ::"r"(smem_u32(bar)), "r"(kLookX)
+                 : "memory");
+  __syncwarp();
+  if (lane >= kLookX / 4096) return;
+  // 32 rows of one term of 64 columns
+  const int h = lane >> 3, term = lane & 1, rc = (h ? lane - 4 : lane) >> 1;
+  const unsigned char* src = mi.PX + (long long)(xo / DB) * mi.tile +
+                             (long long)(xo / 32 + rc) * kChunk + h * 8192 +
+                             term * 4096;
+  const unsigned dst =
+      tx + (h ? (3 + term) * (kLookTile / 2) : term * kLookTile) + rc * 4096;
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1], 4096, [%2];"
+      ::"r"(dst), "l"(src), "r"(smem_u32(bar))
+      : "memory");
 }
 
 // Sixteen scaled values, columns 16 c .. of 64 of a row, as fp16 terms into the
@@ -316,6 +342,40 @@ __device__ __forceinline__ void cp_async16(unsigned dst, const float* src,
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst),
                "l"(src), "r"(there ? 16 : 0)
                : "memory");
+}
+
+// Eight rows of a 128 x 128 block of fp32 values to ta by a warp, asynchronously, into
+// the places of their own terms: piece i of 32 columns in tile i.  Zeros for rows
+// from `valid` on.
+__device__ __forceinline__ void look_load_a(unsigned ta, const float* block,
+                                            long long ld, int row0, int valid,
+                                            int lane) {
+  const float* src = block + 4 * lane;
+  const unsigned dst = ta + (lane >> 3) * kLookTile;
+#pragma unroll 2
+  for (int row = row0; row < row0 + 8; ++row)
+    cp_async16(dst + sw128_chunk_off(row, lane & 7),
+               row < valid ? src + row * ld : src, row < valid);
+}
+
+// Those rows, once they are there, into their terms, 64 columns at a time.
+__device__ __forceinline__ void look_split_a(unsigned char* stage, int row0,
+                                             int lane) {
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    __syncwarp();
+    const int row = row0 + (lane & 7), c = lane >> 3;
+    const float4* src = reinterpret_cast<const float4*>(
+        stage + (2 * h + (c >> 1)) * kLookTile + row * 128);
+    float v[16];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 u = src[(4 * (c & 1) + e) ^ (row & 7)];
+      v[4 * e] = u.x; v[4 * e + 1] = u.y; v[4 * e + 2] = u.z; v[4 * e + 3] = u.w;
+    }
+    __syncwarp();
+    look_store16(smem_u32(stage) + 2 * h * kLookTile, row, c, v, kScaleL);
+  }
 }
 
 // W_kk (bs x bs) into S; beyond bs the identity, so that the sweeps below run
@@ -382,10 +442,7 @@ __device__ __forceinline__ void diag_begin(DiagControl* ctl, int np) {
 // so that this kernel does not have to wait for the panel solve and panel
 // update of step k - 1.  Both products run on the tensor cores (tcgen05,
 // operands in two fp16 terms, accumulators in tensor memory).  X_pp comes as the
-// chunks that the diagonal kernel of step k - 1 left, by bulk copies (rows of 64
-// columns, K-major here), those above its diagonal left out; A' and W_kk by
-// asynchronous copies, A' into the places of its own terms: piece i of 32 columns
-// into tile i.  Result: D in S.
+// chunks that the diagonal kernel of step k - 1 left.  Result: D in S.
 __device__ __forceinline__ void diag_lookahead(const MatInfo& mi, int o, int bs,
                                                float* S,
                                                unsigned char* stage,
@@ -394,63 +451,20 @@ __device__ __forceinline__ void diag_lookahead(const MatInfo& mi, int o, int bs,
   const long long ld = mi.ld;
   const unsigned ta = smem_u32(stage), tx = ta + 4 * kLookTile;
   diag_begin(ctl, (bs + SB - 1) / SB);
-  if (warp == 1) {
-    __syncwarp();
-    // all of the above and the copies of A' and W_kk may run beside the diagonal
-    // kernel of step k - 1; X_pp, and whatever this kernel writes, comes after it
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (lane == 0)
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                   ::"r"(smem_u32(&ctl->x_here)), "r"(12 * 4096)
-                   : "memory");
-    __syncwarp();
-    if (lane < 12) {
-      // 32 rows of one term of 64 columns
-      const int h = lane >> 3, term = lane & 1;
-      const int rc = h ? (lane - 4) >> 1 : lane >> 1;
-      const unsigned char* src =
-          mi.PX + (long long)(o / DB - 1) * mi.tile +
-          (long long)((o - DB) / 32 + rc) * kChunk + h * 8192 + term * 4096;
-      asm volatile(
-          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
-          "[%0], [%1], 4096, [%2];"
-          ::"r"(tx + (2 * h + term) * kLookTile + rc * 4096), "l"(src),
-            "r"(smem_u32(&ctl->x_here))
-          : "memory");
-    }
-  }
-  {
-    const float* src = mi.W + (long long)o * ld + (o - DB) + 4 * lane;
-    const unsigned dst = ta + (lane >> 3) * kLookTile;
-#pragma unroll 2
-    for (int i = 0; i < 8; ++i) {
-      const int row = 8 * warp + i;
-      cp_async16(dst + sw128_chunk_off(row, lane & 7),
-                 row < bs ? src + row * ld : src, row < bs);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
+  look_load_a(ta, mi.W + (long long)o * ld + (o - DB), ld, 8 * warp, bs, lane);
+  asm volatile("cp.async.commit_group;" ::: "memory");
   // (the update is subtracted from it at the end)
   diag_load(mi.W + (long long)o * ld + o, ld, bs, S);
   asm volatile("cp.async.commit_group;" ::: "memory");
-
-  // ---- A' into its terms, 64 columns at a time: a warp's own eight rows
-  asm volatile("cp.async.wait_group 1;" ::: "memory");
-#pragma unroll 1
-  for (int h = 0; h < 2; ++h) {
+  if (warp == 1) {
     __syncwarp();
-    const int row = 8 * warp + (lane & 7), c = lane >> 3;
-    const float4* src = reinterpret_cast<const float4*>(
-        stage + (2 * h + (c >> 1)) * kLookTile + row * 128);
-    float v[16];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float4 u = src[(4 * (c & 1) + e) ^ (row & 7)];
-      v[4 * e] = u.x; v[4 * e + 1] = u.y; v[4 * e + 2] = u.z; v[4 * e + 3] = u.w;
-    }
-    __syncwarp();
-    look_store16(ta + 2 * h * kLookTile, row, c, v, kScaleL);
+    // all of the above and the terms of A' may run beside the diagonal kernel of
+    // step k - 1; X_pp, and whatever this kernel writes, comes after it
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    look_load_x(mi, o - DB, tx, &ctl->x_here, lane);
   }
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  look_split_a(stage, 8 * warp, lane);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1198,6 +1212,128 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
   }
 }
 
+// ------------------------------------------------------------ panel solve
+// L = A' X_kk^T for the rows below diagonal block `step`: a CTA per 128 rows
+// (blockIdx.x) of a matrix (blockIdx.y), the look-ahead's first product.  W stays as
+// it is; L goes to its chunks.  Two CTAs an SM.  One product of 128^3 takes a
+// microsecond; the rest is 64 KB of A', 48 KB of X_kk and 64 KB of L for each CTA,
+// one after the other, of which A' and its terms come before the wait for the
+// diagonal kernel.  (By the tile kernel, which reads X_kk as fp32 and splits it in
+// every CTA, 7.5 to 9.5 us a launch.)
+constexpr int kSolveThreads = 256;
+struct SolveControl {
+  unsigned long long x_here, done;
+  unsigned tmem_base;
+  volatile int abort_flag, grace;
+};
+constexpr int kSolveSmemBytes = kLookBytes + 64;
+static_assert(sizeof(SolveControl) <= 64 && 2 * (kSolveSmemBytes + 1024) <= 227 * 1024,
+              "panel solve shared memory");
+
+__global__ void __launch_bounds__(kSolveThreads, 2)
+panel_solve_kernel(const MatInfo* __restrict__ mats, int step) {
+  extern __shared__ __align__(1024) unsigned char stage[];
+  SolveControl* ctl = reinterpret_cast<SolveControl*>(stage + kLookBytes);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const MatInfo mi = mats[blockIdx.y];
+  const int o = step * DB, r0 = o + DB * (1 + (int)blockIdx.x);
+  const int rows = mi.d - r0;
+  if (rows <= 0) return;
+  const unsigned ta = smem_u32(stage), tx = ta + 4 * kLookTile;
+  const float* block = mi.W + (long long)r0 * mi.ld + o;
+  look_load_a(ta, block, mi.ld, 8 * warp, rows, lane);
+  look_load_a(ta, block, mi.ld, 8 * warp + 64, rows, lane);
+  if (warp == 0) {
+    asm volatile(
+        "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+        ::"r"(smem_u32(&ctl->tmem_base)), "r"(kDiagCols)
+        : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
+                 ::: "memory");
+  } else if (warp == 1) {
+    if (lane == 0) {
+      mbar_init(&ctl->x_here, 1);
+      mbar_init(&ctl->done, 1);
+      ctl->abort_flag = 0;
+      ctl->grace = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+  }
+  diag_load_wait();
+  look_split_a(stage, 8 * warp, lane);
+  look_split_a(stage, 8 * warp + 64, lane);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (warp == 1) look_load_x(mi, o, tx, &ctl->x_here, lane);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem = ctl->tmem_base;
+  if (warp == 0) {
+    const bool go = diag_wait(&ctl->x_here, 0, &ctl->abort_flag);
+    if (__all_sync(0xffffffffu, go) && elect_one()) {
+      look_mma(tmem, ta, tx, true);
+      tc_commit(&ctl->done);
+    }
+    __syncwarp();
+  }
+  const bool ok = diag_wait_tmem(&ctl->done, 0, &ctl->abort_flag);
+  if (ok) {
+    // a warp: 32 rows, 64 columns; A' has been read
+    const int q = warp & 3, h = warp >> 2, row = 32 * q + lane;
+    const unsigned acc = tmem + ((unsigned)(32 * q) << 16) + (unsigned)(64 * h);
+#pragma unroll 1
+    for (int cc = 0; cc < 4; ++cc) {
+      float v[16], w[16];
+      tc_ld16_pair(acc + 16 * cc, acc + 16 * cc + DB, v, w);
+      const unsigned chunk = ta + (2 * h + (cc >> 1)) * kChunk;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        unsigned hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          // (the scale of A' X_kk^T is kScaleL kScaleX; L keeps kScaleL of it)
+          constexpr float s = 1.f / kScaleX;
+          const int c = 8 * i + 2 * e;
+          split_half2(s * (v[c] + w[c]), s * (v[c + 1] + w[c + 1]), hi[e], lo[e]);
+        }
+        const unsigned d = chunk + sw128_chunk_off(row, 2 * (cc & 1) + i);
+        sts128(d, make_float4(__uint_as_float(hi[0]), __uint_as_float(hi[1]),
+                              __uint_as_float(hi[2]), __uint_as_float(hi[3])));
+        sts128(d ^ 0x40u,
+               make_float4(__uint_as_float(lo[0]), __uint_as_float(lo[1]),
+                           __uint_as_float(lo[2]), __uint_as_float(lo[3])));
+      }
+    }
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1 && lane == 0 && ctl->abort_flag == 0) {
+    // (rows past the matrix: zeros, as the chunks' rows there are)
+    unsigned char* dst =
+        mi.PL + (long long)(r0 / DB) * mi.tile + (long long)(o / 32) * kChunk;
+    asm volatile(
+        "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+        ::"l"(dst), "r"(ta), "r"(4 * kChunk)
+        : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
+  if (warp == 0) {
+    if (ctl->abort_flag != 0) {
+      // (its own copies have to be over before the block is)
+      mbar_wait_status(&ctl->x_here, 0, &ctl->grace, &g_diag_status);
+      if (lane == 0) atomicExch(&g_diag_status, 1);
+    }
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+                 ::"r"(tmem), "r"(kDiagCols)
+                 : "memory");
+  }
+}
+
 // ---------------------------------------------------------------- refinement
 // One step of iterative refinement for factors whose fp32 inverse is visibly
 // off (ill-conditioned factors: the error of any fp32 inverse grows with the
@@ -1426,11 +1562,11 @@ enum PlanStream { S_CHAIN, S_BULK, S_FAR, S_ROWS, S_PROD, S_COUNT };
 
 struct Launch {
   int tile_cols; // grouped gemm: tile width
-  int kind;      // 0 diag kernel, 1 grouped gemm
+  int kind;      // 0 diag kernel, 1 grouped gemm, 2 panel solve
   int off;       // grouped gemm: offset into descs
   int n;         // number of matrices / descs
-  int tiles;     // grouped gemm: total tiles
-  int step;      // diag kernel: panel index
+  int tiles;     // grouped gemm: total tiles; panel solve: of the largest matrix
+  int step;      // diag kernel, panel solve: index of the diagonal block
   int stream;    // PlanStream
   // events (indices into the plan's events, -1: none) to wait for first and to
   // record afterwards
@@ -1438,6 +1574,8 @@ struct Launch {
   int rec_ev;
   bool look;     // diag kernel: with the look-ahead prologue
   bool packed;   // grouped gemm: operands in fp16 chunks
+  bool behind;   // follows the launch before it on its stream and nothing else
+                 // that may still run
 
   void wait(int ev) {
     if (ev < 0) return;
@@ -1744,7 +1882,7 @@ extern "C" int kfac_inverse_plan_create(
           h.sa = kScaleX; h.sb = kScaleT;
           if (packed) {
             h.pack = chunk_x(m, s + b, s); h.pack_tile = m.tile;
-            h.pack_scale = kScaleX; h.pack_kind = PACK_MN;
+            h.pack_scale = kScaleX;
           }
           second.push_back(h);
         }
@@ -1776,7 +1914,7 @@ extern "C" int kfac_inverse_plan_create(
         if (packed) {              // nothing reads these rows but as chunks
           g.C = nullptr;
           g.pack = chunk_x(m, po, 0); g.pack_tile = m.tile;
-          g.pack_scale = kScaleX; g.pack_kind = PACK_MN;
+          g.pack_scale = kScaleX;
         }
         push_desc(rows, g);
       }
@@ -1881,24 +2019,26 @@ extern "C" int kfac_inverse_plan_create(
       diag_ev[o / DB] = end_gemm(dl, look);
 
       Launch trsm = begin_gemm(s_bulk);
+      if (packed) {
+        trsm.kind = 2;
+        trsm.step = o / DB;
+      }
       for (int i : order) {
         const int d = dims[i];
         const int M = d - o - DB;
         if (M <= 0) continue;
         const MatInfo& m = mats[i];
         const long long ld = m.ld;
+        if (packed) {              // (the largest matrix comes first)
+          if (trsm.n++ == 0) trsm.tiles = (M + DB - 1) / DB;
+          continue;
+        }
         GemmDesc g = {};
         float* panel = m.W + (o + DB) * ld + o;
         g.A = strided_operand(panel, 1, ld, M);
         g.B = strided_operand(m.X + o * ld + o, 1, ld, DB);
         g.C = panel; g.ldc = ld; g.M = M; g.N = DB; g.K = DB;
-        g.alpha = 1.f; g.beta = 0.f; g.flags = half;
-        g.sa = kScaleL; g.sb = kScaleX;
-        if (packed) {              // L is read as chunks only
-          g.C = nullptr;
-          g.pack = chunk_l(m, o + DB, o); g.pack_tile = m.tile;
-          g.pack_scale = kScaleL; g.pack_kind = PACK_K;
-        }
+        g.alpha = 1.f; g.beta = 0.f; g.flags = 0;
         push_desc(trsm, g);
       }
       trsm.wait(diag_ev[o / DB]);
@@ -1911,6 +2051,7 @@ extern "C" int kfac_inverse_plan_create(
       // diagonal kernel.
       const int skip = look && (ahead || o + DB < co + inner) ? DB : 0;
       Launch upd = begin_gemm(s_bulk);
+      upd.behind = packed != 0;
       for (int i : order) {
         const int d = dims[i];
         const int M = d - o - DB - skip;
@@ -2105,6 +2246,10 @@ extern "C" int kfac_inverse_plan_create(
     e = cudaFuncSetAttribute(chol_diag_kernel<true>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kDiagLookSmemBytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(panel_solve_kernel,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kSolveSmemBytes);
   if (e != cudaSuccess) {
     kfac_inverse_plan_destroy(p);
     return fail(KFAC_ERR_CUDA, "inverse_plan_create: %s", cudaGetErrorString(e));
@@ -2182,7 +2327,7 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
         diag_dev, p->use_tc ? 1 : 0);
     KFAC_LAUNCH_CHECK("damp_copy_kernel");
   }
-  cudaGraphNode_t last_diag = nullptr;
+  cudaGraphNode_t last_diag = nullptr, last_solve = nullptr;
   for (const Launch& l : p->launches) {
     st = sts[l.stream];
     for (int ev : l.wait_ev)
@@ -2201,7 +2346,15 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
             p->sorted_dev, l.step, info, p->packed);
       KFAC_LAUNCH_CHECK("chol_diag_kernel");
       if (graph) last_diag = captured_node(st);
+    } else if (l.kind == 2) {
+      if (last_diag != nullptr) KFAC_CUDA(begin_before_end_of(st, last_diag));
+      panel_solve_kernel<<<dim3(l.tiles, l.n), kSolveThreads, kSolveSmemBytes,
+                           st>>>(p->sorted_dev, l.step);
+      KFAC_LAUNCH_CHECK("panel_solve_kernel");
+      if (graph) last_solve = captured_node(st);
     } else {
+      if (l.behind && last_solve != nullptr)
+        KFAC_CUDA(begin_before_end_of(st, last_solve));
       int rc = l.packed
                    ? launch_packed(p->descs_dev + l.off, &p->descs[l.off], l.n,
                                    l.tiles, st)

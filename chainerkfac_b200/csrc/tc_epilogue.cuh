@@ -138,19 +138,10 @@ __device__ __forceinline__ void pack_store4(const GemmDesc& g, int gr, int gc,
   split_half2(s * x.x, s * x.y, h0, l0);
   split_half2(s * x.z, s * x.w, h1, l1);
   unsigned char* p = g.pack + 8 * ((gc >> 2) & 1);
-  if (g.pack_kind == PACK_K) {
-    p += (long long)(gr >> 7) * g.pack_tile + (long long)(gc >> 5) * kChunk +
-         sw128_chunk_off(gr & 127, (gc & 31) >> 3);
-    *reinterpret_cast<uint2*>(p) = make_uint2(h0, h1);
-    // (the lo terms: the other half of the 128-byte row)
-    p = reinterpret_cast<unsigned char*>(reinterpret_cast<uintptr_t>(p) ^ 0x40);
-    *reinterpret_cast<uint2*>(p) = make_uint2(l0, l1);
-  } else {
-    p += (long long)(gc >> 7) * g.pack_tile + (long long)(gr >> 5) * kChunk +
-         ((gc >> 6) & 1) * 8192 + sw128_chunk_off(gr & 31, (gc & 63) >> 3);
-    *reinterpret_cast<uint2*>(p) = make_uint2(h0, h1);
-    *reinterpret_cast<uint2*>(p + 4096) = make_uint2(l0, l1);
-  }
+  p += (long long)(gc >> 7) * g.pack_tile + (long long)(gr >> 5) * kChunk +
+       ((gc >> 6) & 1) * 8192 + sw128_chunk_off(gr & 31, (gc & 63) >> 3);
+  *reinterpret_cast<uint2*>(p) = make_uint2(h0, h1);
+  *reinterpret_cast<uint2*>(p + 4096) = make_uint2(l0, l1);
 }
 
 struct TileOut {
@@ -172,7 +163,7 @@ __device__ __forceinline__ void tile_epilogue(const GemmDesc& g,
   const bool lower = (flags & G_LOWER) != 0;
   const float alpha = g.alpha;
   float* C = g.C;
-  const bool pack = g.pack_kind != PACK_NONE;
+  const bool pack = g.pack != nullptr;
   const long long ldc = g.ldc;
   // rows of a piece as 16-byte words: lane -> row 4 i + lane / 8, word lane % 8
   const bool vec = (ldc & 3) == 0 &&
