@@ -86,6 +86,7 @@ __global__ void set_run_params_kernel(RunParams* prm, float damping,
 // Also keeps the diagonal (the scales are made of it).
 __global__ void trace_kernel(const MatInfo* __restrict__ mats,
                              float* __restrict__ trace, int* __restrict__ info) {
+  let_next_launch_begin();
   const MatInfo mi = mats[blockIdx.x];
   float s = 0.f;
   for (int i = threadIdx.x; i < mi.d; i += blockDim.x) {
@@ -150,7 +151,9 @@ __global__ void damp_copy_kernel(const MatInfo* __restrict__ mats,
                                  float* __restrict__ add,
                                  float* __restrict__ add2,
                                  float* __restrict__ add_out, int equil) {
+  let_next_launch_begin();
   const MatInfo mi = mats[blockIdx.y];
+  wait_for_launch_before();
   const float2 ad = damping_of(mats, blockIdx.y, mi, trace, prm);
   const float a_first = ad.x, a_second = ad.y;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -431,6 +434,7 @@ __device__ __forceinline__ void diag_begin(DiagControl* ctl, int np) {
         : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
                  ::: "memory");
+    let_next_launch_begin();
   }
 }
 
@@ -460,7 +464,7 @@ __device__ __forceinline__ void diag_lookahead(const MatInfo& mi, int o, int bs,
     __syncwarp();
     // all of the above and the terms of A' may run beside the diagonal kernel of
     // step k - 1; X_pp, and whatever this kernel writes, comes after it
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    wait_for_launch_before();
     look_load_x(mi, o - DB, tx, &ctl->x_here, lane);
   }
   asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -1080,7 +1084,6 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
       (reinterpret_cast<uintptr_t>(dsm + DB * DLD) + 1023) & ~(uintptr_t)1023);
   DiagControl* ctl = reinterpret_cast<DiagControl*>(
       stage + (LOOK ? kLookBytes : kDiagStage));
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const MatInfo mi = mats[blockIdx.x];
   const int id = mi.id;
   const int o = step * DB;
@@ -1234,7 +1237,6 @@ __global__ void __launch_bounds__(kSolveThreads, 2)
 panel_solve_kernel(const MatInfo* __restrict__ mats, int step) {
   extern __shared__ __align__(1024) unsigned char stage[];
   SolveControl* ctl = reinterpret_cast<SolveControl*>(stage + kLookBytes);
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const MatInfo mi = mats[blockIdx.y];
   const int o = step * DB, r0 = o + DB * (1 + (int)blockIdx.x);
@@ -1251,6 +1253,7 @@ panel_solve_kernel(const MatInfo* __restrict__ mats, int step) {
         : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;"
                  ::: "memory");
+    let_next_launch_begin();
   } else if (warp == 1) {
     if (lane == 0) {
       mbar_init(&ctl->x_here, 1);
@@ -1265,7 +1268,7 @@ panel_solve_kernel(const MatInfo* __restrict__ mats, int step) {
   look_split_a(stage, 8 * warp, lane);
   look_split_a(stage, 8 * warp + 64, lane);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  wait_for_launch_before();
   if (warp == 1) look_load_x(mi, o, tx, &ctl->x_here, lane);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1373,6 +1376,8 @@ refine_probe_kernel(const MatInfo* __restrict__ mats,
                     const float* __restrict__ add,
                     const float* __restrict__ add2, double* __restrict__ sums,
                     const RunParams* __restrict__ prm, int stage) {
+  let_next_launch_begin();
+  wait_for_launch_before();
   if (prm->refine_max_dim <= 0) return;
   const RefineItem it = items[blockIdx.y];
   const MatInfo mi = mats[it.mat];
@@ -1436,6 +1441,8 @@ __global__ void refine_gate_kernel(const RefineItem* __restrict__ items, int n,
                                    const RunParams* __restrict__ prm,
                                    int* __restrict__ gate,
                                    int* __restrict__ refined_count) {
+  let_next_launch_begin();
+  wait_for_launch_before();
   const int max_dim = prm->refine_max_dim;
   const float threshold = prm->refine_threshold;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1470,6 +1477,8 @@ refine_residual_kernel(const MatInfo* __restrict__ mats,
     }
     s_item = lo;
   }
+  let_next_launch_begin();
+  wait_for_launch_before();
   __syncthreads();
   const int item = s_item;
   if (gate[item] == 0) return;
@@ -1538,6 +1547,7 @@ __global__ void __launch_bounds__(256)
 refine_apply_kernel(const MatInfo* __restrict__ mats,
                     const RefineItem* __restrict__ items,
                     const int* __restrict__ gate) {
+  wait_for_launch_before();
   if (gate[blockIdx.y] == 0) return;
   const RefineItem it = items[blockIdx.y];
   const MatInfo mi = mats[it.mat];
@@ -1574,8 +1584,6 @@ struct Launch {
   int rec_ev;
   bool look;     // diag kernel: with the look-ahead prologue
   bool packed;   // grouped gemm: operands in fp16 chunks
-  bool behind;   // follows the launch before it on its stream and nothing else
-                 // that may still run
 
   void wait(int ev) {
     if (ev < 0) return;
@@ -2051,7 +2059,6 @@ extern "C" int kfac_inverse_plan_create(
       // diagonal kernel.
       const int skip = look && (ahead || o + DB < co + inner) ? DB : 0;
       Launch upd = begin_gemm(s_bulk);
-      upd.behind = packed != 0;
       for (int i : order) {
         const int d = dims[i];
         const int M = d - o - DB - skip;
@@ -2266,15 +2273,18 @@ extern "C" int kfac_inverse_plan_create(
   return KFAC_OK;
 }
 
-// The node that the next launch on a capturing stream follows, if it is one.
-static cudaGraphNode_t captured_node(cudaStream_t st) {
+// The kernel that the next launch on a capturing stream follows, if it follows
+// nothing else.
+static cudaGraphNode_t captured_kernel(cudaStream_t st) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   const cudaGraphNode_t* deps = nullptr;
   const cudaGraphEdgeData* edges = nullptr;
+  cudaGraphNodeType type = cudaGraphNodeTypeEmpty;
   size_t n = 0;
   if (cudaStreamGetCaptureInfo_v3(st, &cs, nullptr, nullptr, &deps, &edges, &n) !=
           cudaSuccess ||
-      n != 1) {
+      n != 1 || cudaGraphNodeGetType(deps[0], &type) != cudaSuccess ||
+      type != cudaGraphNodeTypeKernel) {
     cudaGetLastError();
     return nullptr;
   }
@@ -2317,8 +2327,16 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
     sts[k] = side_st[k];
     KFAC_CUDA(cudaStreamWaitEvent(sts[k], p->fork_ev, 0));
   }
+  // A launch that follows one kernel only may begin before that has ended.  (The
+  // other engine's kernels do not wait for it themselves.)
+  graph = graph && p->use_tc;
+  auto early = [&](bool when) -> cudaError_t {
+    const cudaGraphNode_t before = graph && when ? captured_kernel(st) : nullptr;
+    return before != nullptr ? begin_before_end_of(st, before) : cudaSuccess;
+  };
   trace_kernel<<<p->count, 256, 0, st>>>(p->mats_dev, p->trace_dev, info);
   KFAC_LAUNCH_CHECK("trace_kernel");
+  KFAC_CUDA(early(true));
   {
     // a block copies about four rows of the largest matrix
     dim3 grid(std::max(1, std::min(512, p->dmax / 4)), p->count);
@@ -2327,15 +2345,16 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
         diag_dev, p->use_tc ? 1 : 0);
     KFAC_LAUNCH_CHECK("damp_copy_kernel");
   }
-  cudaGraphNode_t last_diag = nullptr, last_solve = nullptr;
+  cudaGraphNode_t last_diag = nullptr;
   for (const Launch& l : p->launches) {
     st = sts[l.stream];
     for (int ev : l.wait_ev)
       if (ev >= 0) KFAC_CUDA(cudaStreamWaitEvent(st, p->events[ev], 0));
     if (l.kind == 0) {
-      // what it reads before the wait comes from launches that it follows wholly, or
-      // that the diagonal kernel before it has followed (a layer of 334 x 53, three
-      // diagonal blocks in a row: 222.6 us, 217.7 so; one of 4608 x 512 1304, 1294)
+      // What it reads before the wait comes from launches that it follows wholly, or
+      // that the diagonal kernel before it has followed wholly: one without the
+      // look-ahead does not begin early itself.  (A layer of 334 x 53, three
+      // diagonal blocks in a row: 222.6 us, 217.7 so; one of 4608 x 512 1304, 1294.)
       if (l.look && last_diag != nullptr)
         KFAC_CUDA(begin_before_end_of(st, last_diag));
       if (l.look)
@@ -2345,16 +2364,14 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
         chol_diag_kernel<false><<<l.n, DT, kDiagSmemBytes, st>>>(
             p->sorted_dev, l.step, info, p->packed);
       KFAC_LAUNCH_CHECK("chol_diag_kernel");
-      if (graph) last_diag = captured_node(st);
+      if (graph) last_diag = captured_kernel(st);
     } else if (l.kind == 2) {
       if (last_diag != nullptr) KFAC_CUDA(begin_before_end_of(st, last_diag));
       panel_solve_kernel<<<dim3(l.tiles, l.n), kSolveThreads, kSolveSmemBytes,
                            st>>>(p->sorted_dev, l.step);
       KFAC_LAUNCH_CHECK("panel_solve_kernel");
-      if (graph) last_solve = captured_node(st);
     } else {
-      if (l.behind && last_solve != nullptr)
-        KFAC_CUDA(begin_before_end_of(st, last_solve));
+      KFAC_CUDA(early(l.tiles <= sm_count()));
       int rc = l.packed
                    ? launch_packed(p->descs_dev + l.off, &p->descs[l.off], l.n,
                                    l.tiles, st)
@@ -2376,19 +2393,23 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
   if (p->n_refine > 0) {
     const dim3 pgrid(ceil_div(p->refine_dmax, 8), p->n_refine);
     for (int stage = 0; stage < 3; ++stage) {
+      KFAC_CUDA(early(true));
       refine_probe_kernel<<<pgrid, 256, 0, st>>>(
           p->mats_dev, p->refine_items_dev, p->add_dev, p->add2_dev,
           p->refine_sums_dev, p->params_dev, stage);
       KFAC_LAUNCH_CHECK("refine_probe_kernel");
     }
+    KFAC_CUDA(early(true));
     refine_gate_kernel<<<ceil_div(p->n_refine, 256), 256, 0, st>>>(
         p->refine_items_dev, p->n_refine, p->refine_sums_dev, p->params_dev,
         p->refine_gate_dev, p->refine_count_dev);
     KFAC_LAUNCH_CHECK("refine_gate_kernel");
+    KFAC_CUDA(early(true));
     refine_residual_kernel<<<p->refine_tiles, 256, 0, st>>>(
         p->mats_dev, p->refine_items_dev, p->n_refine, p->add_dev,
         p->add2_dev, p->refine_gate_dev);
     KFAC_LAUNCH_CHECK("refine_residual_kernel");
+    KFAC_CUDA(early(true));
     const Launch& l = p->refine_prod;
     int rc = p->use_tc
                  ? launch_tc_grouped(p->descs_dev + l.off, &p->descs[l.off],
@@ -2397,6 +2418,7 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
                  : launch_grouped_gemm(p->descs_dev + l.off, l.n, l.tiles, 0.f,
                                        0.f, st);
     if (rc != KFAC_OK) return rc;
+    KFAC_CUDA(early(true));
     const dim3 agrid(64, p->n_refine);
     refine_apply_kernel<<<agrid, 256, 0, st>>>(p->mats_dev, p->refine_items_dev,
                                                p->refine_gate_dev);

@@ -18,6 +18,18 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) {
   return (unsigned)__cvta_generic_to_shared(p);
 }
 
+// Launches that may begin while the one before still runs (programmatic dependent
+// launch): they read nothing that it writes, and write nothing, before
+// wait_for_launch_before, which returns when it is complete.  A kernel lets the next
+// one begin once it has its tensor memory: the next one's CTAs keep theirs while
+// they wait.
+__device__ __forceinline__ void let_next_launch_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_launch_before() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // True in one lane of a converged warp.  MMAs are issued behind this, not behind
 // a comparison of the lane number: the compiler then knows that one thread
 // issues them (measured per 128 x 64 x 16 bf16 MMA: 110 cycles against 237).

@@ -211,16 +211,6 @@ __device__ __forceinline__ void store_kf(const GemmDesc& g, float v[16], int r,
   });
 }
 
-// The launches of a preconditioning, and an inverse's updates behind a panel solve,
-// may begin while the one before still runs (programmatic dependent launch); they read nothing that it writes, and write
-// nothing, before wait_for_launch_before, which returns when it is complete.
-__device__ __forceinline__ void let_next_launch_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void wait_for_launch_before() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // Sizes of the rows of gradients (see GradSizes), WARPS warps per row: as many as
 // leave the launch one wave (54 layers of ResNet-50: 60 us with eight, 24 with one).
 template <int WARPS>
@@ -539,8 +529,7 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if constexpr (MODE > 0)
-    let_next_launch_begin();     // (its CTAs cannot take this one's tensor memory)
+  let_next_launch_begin();
   wait_for_launch_before();
 
   const GemmDesc& g = ctl->desc;

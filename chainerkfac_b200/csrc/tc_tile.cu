@@ -415,6 +415,8 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  let_next_launch_begin();
+  wait_for_launch_before();
 
   const GemmDesc& g = ctl->desc;
   const unsigned tmem = ctl->tmem_base;
