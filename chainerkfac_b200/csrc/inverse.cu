@@ -83,16 +83,28 @@ __global__ void set_run_params_kernel(RunParams* prm, float damping,
   prm->refine_threshold = refine_threshold;
 }
 
-// Also keeps the diagonal (the scales are made of it).
-__global__ void trace_kernel(const MatInfo* __restrict__ mats,
+// Also keeps the diagonal (the scales are made of it).  Bound by the latency of
+// its loads, so as many threads as a block has and four loads of each in flight
+// (4608 and 512 rows: 15 us with 256 threads and a load at a time, 6 so).
+constexpr int kTraceThreads = 1024;
+__global__ void __launch_bounds__(kTraceThreads) trace_kernel(const MatInfo* __restrict__ mats,
                              float* __restrict__ trace, int* __restrict__ info) {
   let_next_launch_begin();
   const MatInfo mi = mats[blockIdx.x];
   float s = 0.f;
-  for (int i = threadIdx.x; i < mi.d; i += blockDim.x) {
-    const float v = mi.F[(long long)i * mi.d + i];
-    mi.diag[i] = v;
-    s += v;
+  for (int i0 = threadIdx.x; i0 < mi.d; i0 += 4 * kTraceThreads) {
+    float v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = i0 + k * kTraceThreads;
+      v[k] = i < mi.d ? mi.F[(long long)i * (mi.d + 1)] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = i0 + k * kTraceThreads;
+      if (i < mi.d) mi.diag[i] = v[k];
+      s += v[k];
+    }
   }
   __shared__ float sh[32];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
@@ -141,18 +153,23 @@ __device__ __forceinline__ float equil_scale(float x) {
   return __uint_as_float((unsigned)(127 - (e >> 1)) << 23);
 }
 
-// W = S (F + add * I) S, blockIdx.y = matrix, blockIdx.x strides over rows.
-// Only the lower triangle and the rest of each diagonal 128-block (which the
-// trailing updates read-modify-write) is ever used, so only that is copied.
-// `equil` off: S = I.
-__global__ void damp_copy_kernel(const MatInfo* __restrict__ mats,
-                                 const float* __restrict__ trace,
-                                 const RunParams* __restrict__ prm,
-                                 float* __restrict__ add,
-                                 float* __restrict__ add2,
-                                 float* __restrict__ add_out, int equil) {
+// W = S (F + add * I) S, blockIdx.y = matrix, blockIdx.x strides over groups of four
+// rows, which share the columns' scales and are in flight together.  Only the lower
+// triangle and the rest of each diagonal 128-block (which the trailing updates
+// read-modify-write) is ever used, so only that is copied.  `equil` off: S = I.
+// (Row by row: 28 matrices of up to 856 rows 13.7 us, 4608 and 512 rows 23.5; a warp
+// a row 16.6 and 28.9; so 11.9 and 17.3.)
+constexpr int kDampRows = 4;
+__global__ void __launch_bounds__(256, 4)
+damp_copy_kernel(const MatInfo* __restrict__ mats,
+                 const float* __restrict__ trace,
+                 const RunParams* __restrict__ prm, float* __restrict__ add,
+                 float* __restrict__ add2, float* __restrict__ add_out,
+                 int equil) {
   let_next_launch_begin();
   const MatInfo mi = mats[blockIdx.y];
+  const int d = mi.d;
+  if (kDampRows * (int)blockIdx.x >= d) return;
   wait_for_launch_before();
   const float2 ad = damping_of(mats, blockIdx.y, mi, trace, prm);
   const float a_first = ad.x, a_second = ad.y;
@@ -161,7 +178,6 @@ __global__ void damp_copy_kernel(const MatInfo* __restrict__ mats,
     add2[blockIdx.y] = a_second;
     if (add_out) add_out[blockIdx.y] = a_first;
   }
-  const int d = mi.d;
   auto damp = [&](int r) {
     return (mi.role == 2 && 2 * r >= d) ? a_second : a_first;
   };
@@ -171,39 +187,56 @@ __global__ void damp_copy_kernel(const MatInfo* __restrict__ mats,
   const bool vec = (d & 3) == 0 &&
                    ((reinterpret_cast<uintptr_t>(mi.F) |
                      reinterpret_cast<uintptr_t>(mi.W)) & 15) == 0;
-  for (int r = blockIdx.x; r < d; r += gridDim.x) {
-    const float a = damp(r), sr = scale(r, mi.diag[r]);
-    if (threadIdx.x == 0) mi.S[r] = sr;
-    const int cend = min(d, (r | (DB - 1)) + 1);
-    const float* src = mi.F + (long long)r * d;
-    float* dst = mi.W + (long long)r * mi.ld;
+  for (int r0 = kDampRows * blockIdx.x; r0 < d; r0 += kDampRows * gridDim.x) {
+    float sr[kDampRows], a[kDampRows];
+    const float *src[kDampRows];
+    float* dst[kDampRows];
+#pragma unroll
+    for (int i = 0; i < kDampRows; ++i) {
+      const int r = min(r0 + i, d - 1);    // (past the end: the last row again)
+      a[i] = damp(r);
+      sr[i] = scale(r, mi.diag[r]);
+      src[i] = mi.F + (long long)r * d;
+      dst[i] = mi.W + (long long)r * mi.ld;
+      if (threadIdx.x == 0) mi.S[r] = sr[i];
+    }
+    const int cend = min(d, (r0 | (DB - 1)) + 1);
     if (vec) {
       // cend is a multiple of 128 or equals d, itself a multiple of 4 here
-      const float4* s4 = reinterpret_cast<const float4*>(src);
       const float4* g4 = reinterpret_cast<const float4*>(mi.diag);
-      float4* d4 = reinterpret_cast<float4*>(dst);
-#pragma unroll 4
-      for (int c4 = threadIdx.x; c4 < (cend >> 2); c4 += blockDim.x) {
-        float4 v = s4[c4];
+#pragma unroll 1
+      for (int c4 = threadIdx.x; c4 < (cend >> 2); c4 += 256) {
+        float4 v[kDampRows];
+#pragma unroll
+        for (int i = 0; i < kDampRows; ++i)
+          v[i] = reinterpret_cast<const float4*>(src[i])[c4];
         const float4 g = g4[c4];
-        if ((r >> 2) == c4) {
-          if ((r & 3) == 0) v.x += a;
-          else if ((r & 3) == 1) v.y += a;
-          else if ((r & 3) == 2) v.z += a;
-          else v.w += a;
+        const float sx = scale(4 * c4, g.x), sy = scale(4 * c4 + 1, g.y);
+        const float sz = scale(4 * c4 + 2, g.z), sw = scale(4 * c4 + 3, g.w);
+        if ((r0 >> 2) == c4) {             // (the rows' four diagonal entries)
+          v[0].x += a[0];
+          v[1].y += a[1];
+          v[2].z += a[2];
+          v[3].w += a[3];
         }
-        v.x = v.x * sr * scale(4 * c4, g.x);
-        v.y = v.y * sr * scale(4 * c4 + 1, g.y);
-        v.z = v.z * sr * scale(4 * c4 + 2, g.z);
-        v.w = v.w * sr * scale(4 * c4 + 3, g.w);
-        d4[c4] = v;
+#pragma unroll
+        for (int i = 0; i < kDampRows; ++i)
+          reinterpret_cast<float4*>(dst[i])[c4] =
+              make_float4(v[i].x * sr[i] * sx, v[i].y * sr[i] * sy,
+                          v[i].z * sr[i] * sz, v[i].w * sr[i] * sw);
       }
     } else {
-      for (int c = threadIdx.x; c < cend; c += blockDim.x) {
-        float v = src[c];
-        if (r == c) v += a;
-        v = v * sr * scale(c, mi.diag[c]);
-        dst[c] = v;
+#pragma unroll 2
+      for (int c = threadIdx.x; c < cend; c += 256) {
+        float v[kDampRows];
+#pragma unroll
+        for (int i = 0; i < kDampRows; ++i) v[i] = src[i][c];
+        const float sc = scale(c, mi.diag[c]);
+#pragma unroll
+        for (int i = 0; i < kDampRows; ++i) {
+          if (min(r0 + i, d - 1) == c) v[i] += a[i];
+          dst[i][c] = v[i] * sr[i] * sc;
+        }
       }
     }
   }
@@ -2334,12 +2367,11 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
     const cudaGraphNode_t before = graph && when ? captured_kernel(st) : nullptr;
     return before != nullptr ? begin_before_end_of(st, before) : cudaSuccess;
   };
-  trace_kernel<<<p->count, 256, 0, st>>>(p->mats_dev, p->trace_dev, info);
+  trace_kernel<<<p->count, kTraceThreads, 0, st>>>(p->mats_dev, p->trace_dev, info);
   KFAC_LAUNCH_CHECK("trace_kernel");
   KFAC_CUDA(early(true));
   {
-    // a block copies about four rows of the largest matrix
-    dim3 grid(std::max(1, std::min(512, p->dmax / 4)), p->count);
+    const dim3 grid(std::min(1024, ceil_div(p->dmax, kDampRows)), p->count);
     damp_copy_kernel<<<grid, 256, 0, st>>>(
         p->mats_dev, p->trace_dev, p->params_dev, p->add_dev, p->add2_dev,
         diag_dev, p->use_tc ? 1 : 0);
