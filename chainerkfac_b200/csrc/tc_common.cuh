@@ -315,4 +315,24 @@ __device__ __forceinline__ void split_bf16x2(float x0, float x1, unsigned& hi,
                    __float_as_uint(l1) + 0x8000u, 0x7632);
 }
 
+// `early`: the launch may begin before the one in front of it has ended.
+template <typename... P, typename... A>
+static int launch_behind(const char* name, bool early, void (*kernel)(P...),
+                         int blocks, int threads, int smem, cudaStream_t stream,
+                         A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
+  KFAC_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  KFAC_LAUNCH_CHECK(name);
+  return KFAC_OK;
+}
+
 }  // namespace kfac

@@ -108,24 +108,39 @@ __device__ __forceinline__ void tile_precond(const GemmDesc& g,
   float* ovel = w ? g.vW : g.vb;
   const long long step = w ? dW : 1;
   long long idx = gr0 * step + (w ? gc0 + lane : 0);
+  // (values, then stores, each under one condition: with branches between them a
+  // row takes 250 cycles)
+#pragma unroll 1
   for (int r0 = 0; r0 < rows; r0 += 8, idx += 8 * step) {
-    float ov[8], op[8];
+    const int n = rows - r0;
+    float ov[8], op[8], kf[8];
+    if (opar != nullptr) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (opar != nullptr && r0 + i < rows) {
-        ov[i] = ovel[idx + i * step];
-        op[i] = opar[idx + i * step];
-      }
+      for (int i = 0; i < 8; ++i)
+        if (i < n) {
+          ov[i] = ovel[idx + i * step];
+          op[i] = opar[idx + i * step];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) kf[i] = piece[(r0 + i) * TT_EP + lane];
+    if (okf != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < n) okf[idx + i * step] = kf[i];
+    }
+    if (opar == nullptr) continue;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      if (r0 + i >= rows) continue;
-      const float kf = piece[(r0 + i) * TT_EP + lane];
-      if (okf != nullptr) okf[idx + i * step] = kf;
-      if (opar == nullptr) continue;
-      const float nv = momentum * ov[i] - lr * kf;
-      ovel[idx + i * step] = nv;
-      opar[idx + i * step] = op[i] + nv;
+      kf[i] = momentum * ov[i] - lr * kf[i];
+      op[i] += kf[i];
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i < n) ovel[idx + i * step] = kf[i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i < n) opar[idx + i * step] = op[i];
   }
 }
 

@@ -104,24 +104,37 @@ __device__ __forceinline__ void piece_each(int r, int c, int rows, int cols,
 // entry is held relative to the most that its row and column could make it; the
 // rows' sizes are in G_inv's columns, the columns' part and `wide` (the most that
 // a row's norm exceeds its size) come out of kf.
+// `rs`, `cs`: the lane's two rows' and eight columns' factors.
+__device__ __forceinline__ void load_u(const GemmDesc& g, int r, float rs[2]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    rs[h] = r + 8 * h < g.M ? g.rs[r + 8 * h] : 0.f;
+}
+__device__ __forceinline__ void load_u_columns(const GemmDesc& g, int c,
+                                               float cs[8]) {
+  // (columns past the last one: any values, nobody stores their results)
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    cs[j] = g.cs[min(c + 8 * (j >> 1) + (j & 1), g.N - 1)];
+}
 __device__ __forceinline__ void store_u(const GemmDesc& g, const float v[16],
-                                        int r, int c) {
+                                        int r, int c, const float rs[2],
+                                        const float cs[8]) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int gr = r + 8 * h;
     const bool in = gr < g.M;
-    const float s0 = g.rs[min(gr, g.M - 1)];
+    unsigned char* const row = g.pack + (long long)(gr >> 5) * kChunk +
+                               (long long)(c >> 7) * g.pack_tile +
+                               ((c >> 6) & 1) * 8192;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      // (columns past the last one: any values, nobody stores their results)
-      const int gc = c + 8 * j, k0 = min(gc, g.N - 1), k1 = min(gc + 1, g.N - 1);
       unsigned hi, lo;
-      split_half2(in ? v[4 * j + 2 * h] * s0 * g.cs[k0] : 0.f,
-                  in ? v[4 * j + 2 * h + 1] * s0 * g.cs[k1] : 0.f, hi, lo);
-      unsigned char* p = g.pack + (long long)(gc >> 7) * g.pack_tile +
-                         (long long)(gr >> 5) * kChunk +
-                         ((gc >> 6) & 1) * 8192 +
-                         sw128_chunk_off(gr & 31, (gc & 63) >> 3) + 2 * (gc & 7);
+      split_half2(in ? v[4 * j + 2 * h] * rs[h] * cs[2 * j] : 0.f,
+                  in ? v[4 * j + 2 * h + 1] * rs[h] * cs[2 * j + 1] : 0.f, hi, lo);
+      const int gc = c + 8 * j;              // (in the piece's half of a tile)
+      unsigned char* p =
+          row + sw128_chunk_off(gr & 31, (gc & 63) >> 3) + 2 * (gc & 7);
       *reinterpret_cast<unsigned*>(p) = hi;
       *reinterpret_cast<unsigned*>(p + 4096) = lo;
     }
@@ -144,71 +157,90 @@ __device__ __forceinline__ int widest_row(const GemmDesc& g, int lane) {
   return m <= kNoExp ? 0 : m;            // (a gradient of zeros)
 }
 
-// Second product: a 16 x 32 piece of kf to the weight and bias parts, and the
-// momentum update where the layer has it fused.
-__device__ __forceinline__ void store_kf(const GemmDesc& g, float v[16], int r,
-                                         int c, bool whole, float lr,
-                                         float momentum) {
-  const int e0 = g.re[min(r, g.M - 1)], e1 = g.re[min(r + 8, g.M - 1)];
+// The second product's epilogue takes a 16 x 32 piece of kf through shared memory and
+// has a column a lane: rows of weights, velocities and kf are read and written 128
+// bytes at a time, wherever they begin, without a branch between the rows, and the
+// next piece's loads come before this one's stores where a CTA has the registers.
+// (A lane's values straight from the accumulators, with branches past the edges: 62
+// tiles of odd sizes 25.5 us, so 16; 144 tiles of 512 x 4608 20 us either way, 47 MB
+// of weights, velocities and kf.)  Bound: 32 bytes a cycle that an SM can store.
+constexpr int KF_PITCH = 36;                 // floats
+struct KfOld {
+  float v[16], p[16];                        // velocities, weights
+  int er, ec;                                // exponents: row `lane`, the column
+};
+
+// Of a lane's column, weight or bias: first row's place, and from a row to the next.
+struct KfColumn {
+  long long at, step;
+  bool weight, live;
+};
+__device__ __forceinline__ KfColumn kf_column(const GemmDesc& g, int r0, int c) {
+  KfColumn k;
+  k.weight = c < g.dW;
+  k.live = c < g.N;
+  k.step = k.weight ? g.dW : 1;
+  k.at = (long long)r0 * k.step + (k.weight ? c : 0);
+  return k;
+}
+
+__device__ __forceinline__ void load_kf(const GemmDesc& g, int r0, int c0,
+                                        int lane, KfOld& o) {
+  o.er = g.re[min(r0 + (lane & 15), g.M - 1)];
+  o.ec = g.ce[min(c0 + lane, g.N - 1)];
+  const KfColumn k = kf_column(g, r0, c0 + lane);
+  const float* v = k.weight ? g.vW : g.vb;
+  const float* p = k.weight ? g.pW : g.pb;
+  const bool on = g.pW != nullptr && k.live;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int e = g.ce[min(c + 8 * (j >> 1) + (j & 1), g.N - 1)];
-    const int i = 4 * (j >> 1) + (j & 1);
-    v[i] = scale_exp(v[i], e0 + e);
-    v[i + 2] = scale_exp(v[i + 2], e1 + e);
+  for (int i = 0; i < 16; ++i) {
+    const bool in = on && r0 + i < g.M;
+    o.v[i] = in ? v[k.at + i * k.step] : 0.f;
+    o.p[i] = in ? p[k.at + i * k.step] : 0.f;
   }
-  const int dW = g.dW;
+}
+
+// kf to the weight and bias parts, and the momentum update where the layer has it
+// fused.  `piece`: 16 x KF_PITCH floats of this warp's own.
+__device__ __forceinline__ void store_kf(const GemmDesc& g, const float v[16],
+                                         float* piece, int r0, int c0, int lane,
+                                         float lr, float momentum,
+                                         const KfOld& o) {
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 16; i += 2)
+    *reinterpret_cast<float2*>(&piece[((lane >> 2) + 8 * ((i >> 1) & 1)) * KF_PITCH +
+                                      2 * (lane & 3) + 8 * (i >> 2)]) =
+        make_float2(v[i], v[i + 1]);
+  __syncwarp();
+  const KfColumn k = kf_column(g, r0, c0 + lane);
+  float* const okf = k.weight ? g.kfW : g.kfb;
+  float* const ov = k.weight ? g.vW : g.vb;
+  float* const op = k.weight ? g.pW : g.pb;
   const bool fused = g.pW != nullptr;
-  if (whole && (dW & 1) == 0 &&
-      ((reinterpret_cast<uintptr_t>(g.kfW) | reinterpret_cast<uintptr_t>(g.pW) |
-        reinterpret_cast<uintptr_t>(g.vW)) & 7) == 0) {
-    const long long at = (long long)r * dW + c;
-    if (g.kfW != nullptr) {
+  // (values, then stores, each under one condition: with branches between them a
+  // row took 250 cycles)
+  float kf[16];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        *reinterpret_cast<float2*>(g.kfW + at + 8 * (i >> 1) +
-                                   8LL * (i & 1) * dW) =
-            make_float2(v[2 * i], v[2 * i + 1]);
-    }
-    if (!fused) return;
-    float2 ov[8], op[8];
+  for (int i = 0; i < 16; ++i)
+    kf[i] = scale_exp(piece[i * KF_PITCH + lane],
+                      __shfl_sync(0xffffffffu, o.er, i) + o.ec);
+  const int rows = k.live ? g.M - r0 : 0;
+  auto put = [&](float* base, const float (&x)[16], int n) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const long long d = at + 8 * (i >> 1) + 8LL * (i & 1) * dW;
-      ov[i] = *reinterpret_cast<const float2*>(g.vW + d);
-      op[i] = *reinterpret_cast<const float2*>(g.pW + d);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const long long d = at + 8 * (i >> 1) + 8LL * (i & 1) * dW;
-      const float n0 = momentum * ov[i].x - lr * v[2 * i];
-      const float n1 = momentum * ov[i].y - lr * v[2 * i + 1];
-      *reinterpret_cast<float2*>(g.vW + d) = make_float2(n0, n1);
-      *reinterpret_cast<float2*>(g.pW + d) =
-          make_float2(op[i].x + n0, op[i].y + n1);
-    }
-    return;
-  }
-  float ov[16], op[16];
-  auto part = [&](int dr, int dc, float* w, float* b) {
-    return c + dc < dW ? w + (long long)(r + dr) * dW + c + dc : b + r + dr;
+    for (int i = 0; i < 16; ++i)
+      if (i < n) base[k.at + i * k.step] = x[i];
   };
-  if (fused)
-    // (past the edges the last row or column: no branch, all in flight)
-    piece_each<true>(r, c, g.M, g.N, false, [&](int i, int dr, int dc) {
-      const int y = min(r + dr, g.M - 1), x = min(c + dc, g.N - 1);
-      const long long at = x < dW ? (long long)y * dW + x : y;
-      ov[i] = (x < dW ? g.vW : g.vb)[at];
-      op[i] = (x < dW ? g.pW : g.pb)[at];
-    });
-  piece_each<false>(r, c, g.M, g.N, false, [&](int i, int dr, int dc) {
-    if ((c + dc < dW ? g.kfW : g.kfb) != nullptr)
-      *part(dr, dc, g.kfW, g.kfb) = v[i];
-    if (!fused) return;
-    const float n = momentum * ov[i] - lr * v[i];
-    *part(dr, dc, g.vW, g.vb) = n;
-    *part(dr, dc, g.pW, g.pb) = op[i] + n;
-  });
+  put(okf, kf, okf != nullptr ? rows : 0);
+  if (!fused) return;
+  float w[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    kf[i] = momentum * o.v[i] - lr * kf[i];
+    w[i] = o.p[i] + kf[i];
+  }
+  put(ov, kf, rows);
+  put(op, w, rows);
 }
 
 // Sizes of the rows of gradients (see GradSizes), WARPS warps per row: as many as
@@ -632,6 +664,27 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
     const int lr = lane >> 2, lc = 2 * (lane & 3);
     bool ok = true;
     const int nseg = nkb > 0 ? (kb0 + nkb - 1) / kSegment - seg0 + 1 : 1;
+    // The second product of a preconditioning, where a CTA has the registers: what a
+    // piece reads is loaded while the piece before it (or the MMAs) runs.  The piece
+    // itself goes through the stages, which the MMAs have read by then.
+    constexpr bool kAhead = MODE == 2 && STAGES > 3;
+    KfOld ahead;
+    float* const piece =
+        reinterpret_cast<float*>(smem) + (warp - 2) * 16 * KF_PITCH;
+    auto load_piece = [&](int u, KfOld& o) {
+      const int r0 = m0 + 32 * q + 16 * (u & 1);
+      const int c0 = n0 + 32 * h + 64 * (u >> 1);
+      if (r0 < rows && c0 < cols) load_kf(g, r0, c0, lane, o);
+    };
+    if constexpr (kAhead) load_piece(0, ahead);
+    float u_rows[2][2], u_cols[2][8];
+    if constexpr (MODE == 1) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        load_u(g, m0 + 32 * q + 16 * k + lr, u_rows[k]);
+        load_u_columns(g, n0 + 32 * h + 64 * k + lc, u_cols[k]);
+      }
+    }
 #pragma unroll 1
     for (int it = 0; it < 4 * nseg; ++it) {
       const int u = it & 3, seg = it >> 2;
@@ -663,6 +716,11 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
           });
         }
       }
+      KfOld kf_old;
+      if constexpr (kAhead) {
+        kf_old = ahead;
+        if (u < 3) load_piece(u + 1, ahead);
+      }
       if (u == 0 && nkb > 0) {
         ok = mbar_wait_status(&ctl->accum, seg & 1, &ctl->abort_flag,
                               &g_packed_status);
@@ -691,11 +749,17 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
       }
       if (!live) continue;
       if constexpr (MODE == 1) {
-        store_u(g, v, r, c);
+        float rs[2], cs[8];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) rs[k] = u & 1 ? u_rows[1][k] : u_rows[0][k];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) cs[k] = u > 1 ? u_cols[1][k] : u_cols[0][k];
+        store_u(g, v, r, c, rs, cs);
         continue;
       }
       if constexpr (MODE == 2) {
-        store_kf(g, v, r, c, whole && c0 + 32 <= g.dW, plr, momentum);
+        if constexpr (!kAhead) load_piece(u, kf_old);
+        store_kf(g, v, piece, r0, c0, lane, plr, momentum, kf_old);
         continue;
       }
       if (un != nullptr) {
@@ -755,26 +819,6 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
 }
 
 // ------------------------------------------------------------------ host side
-// `early`: the launch may begin before the one in front of it has ended.
-template <typename... P, typename... A>
-static int launch_behind(const char* name, bool early, void (*kernel)(P...),
-                         int blocks, int threads, int smem, cudaStream_t stream,
-                         A... args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = early ? 1 : 0;
-  KFAC_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
-  KFAC_LAUNCH_CHECK(name);
-  return KFAC_OK;
-}
-
 struct PackedVariant {
   void (*kernel)(const GemmDesc*, int, const TileInline, float, float);
   int stages;

@@ -761,9 +761,11 @@ int launch_tc_grouped(const GemmDesc* descs_dev, const GemmDesc* descs_host,
     const TileVariant& v =
         half ? kHalfVariants[tile_cols == 128]
              : kTileVariants[tile_cols == 128][precond][k == 0];
-    v.kernel<<<end - tile0, v.threads, v.smem, stream>>>(
-        descs_dev + first, n, tile0, inl, lr, momentum);
-    KFAC_LAUNCH_CHECK("tc_tile_kernel");
+    // (a preconditioning's second product begins behind its first)
+    const int rc = launch_behind("tc_tile_kernel", precond, v.kernel, end - tile0,
+                                 v.threads, v.smem, stream, descs_dev + first, n,
+                                 tile0, inl, lr, momentum);
+    if (rc != KFAC_OK) return rc;
   }
   return KFAC_OK;
 }
