@@ -685,9 +685,45 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
         load_u_columns(g, n0 + 32 * h + 64 * k + lc, u_cols[k]);
       }
     }
+    // C of an inverse's product, a piece ahead: with the loads of a piece behind the
+    // stores of the one before, an SM had 32 KB under way and a tile's epilogue took
+    // as long as the MMAs of 512 k.
+    float old_ahead[16];
+    auto load_old = [&](int it) {
+      const int u = it & 3;
+      const int r0 = m0 + 32 * q + 16 * (u & 1);
+      const int c0 = n0 + 32 * h + 64 * (u >> 1);
+      if ((it < 4 ? beta : 1.f) == 0.f || r0 >= rows || c0 >= cols ||
+          (lower && c0 > r0 + 15))
+        return;
+      const int r = r0 + lr, c = c0 + lc;
+      if (vec && r0 + 16 <= rows && c0 + 32 <= cols && (!lower || c0 + 31 <= r0)) {
+        const float* p = g.C + (long long)r * ldc + c;
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          const float2 x = *reinterpret_cast<const float2*>(
+              p + 8 * ((i >> 1) & 1) * ldc + 8 * (i >> 2));
+          old_ahead[i] = x.x;
+          old_ahead[i + 1] = x.y;
+        }
+      } else {
+        // (past the edges the last row or column: no branch, all in flight)
+        piece_each<true>(r, c, rows, cols, lower, [&](int i, int dr, int dc) {
+          old_ahead[i] = g.C[(long long)min(r + dr, rows - 1) * ldc +
+                             min(c + dc, cols - 1)];
+        });
+      }
+    };
 #pragma unroll 1
-    for (int it = 0; it < 4 * nseg; ++it) {
+    for (int it = MODE == 0 ? -1 : 0; it < 4 * nseg; ++it) {
       const int u = it & 3, seg = it >> 2;
+      float old[16];
+      if constexpr (MODE == 0) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) old[i] = old_ahead[i];
+        if (it + 1 < 4 * nseg) load_old(it + 1);
+        if (it < 0) continue;
+      }
       if (it == 4) beta = 1.f;             // onto the segments before
       const int r0 = m0 + 32 * q + 16 * (u & 1);
       const int c0 = n0 + 32 * h + 64 * (u >> 1);
@@ -698,24 +734,6 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
           r0 + 16 <= rows && c0 + 32 <= cols && (!lower || c0 + 31 <= r0);
       const int r = r0 + lr, c = c0 + lc;
       float* p = g.C + (long long)r * ldc + c;
-      float old[16];
-      if (MODE == 0 && beta != 0.f && live) {
-        if (whole && vec) {
-#pragma unroll
-          for (int i = 0; i < 16; i += 2) {
-            const float2 x = *reinterpret_cast<const float2*>(
-                p + 8 * ((i >> 1) & 1) * ldc + 8 * (i >> 2));
-            old[i] = x.x;
-            old[i + 1] = x.y;
-          }
-        } else {
-          // (past the edges the last row or column: no branch, all in flight)
-          piece_each<true>(r, c, rows, cols, lower, [&](int i, int dr, int dc) {
-            old[i] = g.C[(long long)min(r + dr, rows - 1) * ldc +
-                         min(c + dc, cols - 1)];
-          });
-        }
-      }
       KfOld kf_old;
       if constexpr (kAhead) {
         kf_old = ahead;
