@@ -1853,8 +1853,8 @@ extern "C" int kfac_inverse_plan_create(
   // Width of the chain's panels.  Between two panels the chain waits for the
   // last solve and the near part of the trailing update, so matrices of up to
   // two panels are one where the longer panel updates of a step still fit the
-  // SMs (1024 rows 380 -> 360 us; 68 such matrices at once, or 4608 rows, whose
-  // panel updates are what the chain waits for, gain nothing from it).
+  // SMs (1024 rows 232 us in two, 228 in one, 5 x 1001 274 and 264; 20 x 1024, or 4608
+  // rows, whose panel updates are what the chain waits for, gain nothing from it).
   long long step_tiles = 0;
   for (int i = 0; i < count; ++i)
     if (dims[i] > PW)
@@ -2028,16 +2028,18 @@ extern "C" int kfac_inverse_plan_create(
   };
   // Whether a panel's steps also update the next one's first block column.  The
   // chain then goes on there without waiting for the near update, which only
-  // the second block needs.  us without and with, by row tiles, a plan by itself:
-  // 4608 rows (36) 1494 1420, 2 x 3400 (54) 1183 1088, 8 x 1024 (64) 414 405, 2 x 4608
-  // (72) 1835 1760, 4608 beside 6 x 1000 (84) 1554 1486, 5 x 2304 (90) 850 826, 6 x
-  // 2304 (108) 963 890, 16 x 1024 (128) 483 477.  Where plans run beside each
-  // other and fill the SMs, the passes over that column only cost (108 factors of
-  // ResNet-50, plans of 120, 309 and 225 row tiles: 4605 us without, 4650 in the
-  // first plan, 4690 in all); such plans are large.
+  // the second block needs.  It pays for matrices of two panels, where the one near
+  // update between them is a good part of the chain; longer ones wait for their
+  // panel updates anyway, which the further column makes longer.  us without and
+  // with, by row tiles, a plan by itself: 8 x 1024 (64) 323 312, 16 x 1024 (128) 388
+  // 377; 4608 rows (36) 1069 1081, 2 x 3400 (54) 872 875, 2 x 4608 (72) 1384 1411,
+  // 4608 beside 6 x 1000 (84) 1133 1158, 5 x 2304 (90) 651 649, 6 x 2304 (108) 713
+  // 724.  Where plans run beside each other and fill the SMs, the passes over that
+  // column only cost (108 factors of ResNet-50, plans of 120, 309 and 225 row tiles);
+  // such plans are large.
   long long row_tiles = 0;
   for (int i = 0; i < count; ++i) row_tiles += (dims[i] + DB - 1) / DB;
-  const bool ahead = look && 4 * row_tiles <= 3 * sm_count();
+  const bool ahead = look && dmax <= 2 * PW && row_tiles <= sm_count();
   const int E = ahead ? DB : 0;
   int near_ev = -1;            // near updates of the panel before
   for (int co = 0; co < dmax; co += CW) {
@@ -2403,6 +2405,9 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
                            st>>>(p->sorted_dev, l.step);
       KFAC_LAUNCH_CHECK("panel_solve_kernel");
     } else {
+      // (more tiles than SMs: the next launch's waiting CTAs only take room; 54 pairs
+      // of ResNet-50 with a limit of half the SMs 3966 us, all of them 3931; of twice
+      // as many, beside others in another run, 4094, without a limit 4083, 3993 so)
       KFAC_CUDA(early(l.tiles <= sm_count()));
       int rc = l.packed
                    ? launch_packed(p->descs_dev + l.off, &p->descs[l.off], l.n,
