@@ -772,14 +772,16 @@ __device__ __forceinline__ void diag_base(DiagSmem& sm, DiagControl* ctl, int p,
 }
 
 // The part of diag_base's updates that its own warp leaves: step s on columns
-// 8 s + 16 .. 31 of the sub-block, in shared memory, four columns per warp.
+// 8 s + 16 .. 31 of the sub-block, in shared memory, four columns per warp.  Each has
+// the same columns in both steps: nothing orders one warp's first step before
+// another's second.
 __device__ __forceinline__ void diag_base_rest(DiagSmem& sm, DiagControl* ctl,
                                                int p, int lane, int h) {
 #pragma unroll 1
   for (int s = 0; s < 2; ++s) {
     diag_wait(&ctl->step[p][s], 0, &ctl->abort_flag);
-    const int c = 8 * s + 16 + 4 * h;
-    if (c < SB) {
+    const int c = 16 + 4 * h;
+    if (c >= 8 * s + 16) {
       const float (*L)[LSP] = &sm.Ls[p & 1][8 * s];
       float* row = &sm.S[(SB * p + lane) * DLD + SB * p + c];
       ulonglong2 u = load_pairs(row);

@@ -1088,6 +1088,31 @@ def test_inverse_by_graph_and_by_plain_launches(ops, monkeypatch, dims):
         plan.close()
 
 
+def test_inverses_repeat_bit_for_bit_beside_each_other(ops):
+    """Sums are in a fixed order, so nothing changes from run to run, also where
+    three plans fill the SMs and warps of a block wait for each other longer (a
+    warp's columns of a diagonal sub-block were touched by another one too soon in
+    one of ten runs of such a set)."""
+    from bench_workloads import layer_dims, resnet50_layers
+    dims = [d for l in resnet50_layers() for d in layer_dims(l)[:2]]
+    g = torch.Generator(device='cuda')
+    g.manual_seed(5)
+    F = []
+    for d in dims:
+        x = torch.randn((2 * d, d), device='cuda', generator=g)
+        f = x.t() @ x / (2 * d)
+        F.append((f + f.t()) / 2)
+    inv = [torch.empty_like(f) for f in F]
+    plan = ops.InversePlanSet(F, inv, [i ^ 1 for i in range(len(F))],
+                              [0, 1] * (len(F) // 2))
+    plan.run(1e-3)
+    first = [v.clone() for v in inv]
+    for _ in range(100):
+        plan.run(1e-3)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(first, inv))
+
+
 @pytest.mark.parametrize('blocks', [0, 1, 4])
 @pytest.mark.parametrize('rows', [1, 31, 32, 33, 64, 65, 95, 96, 97, 127, 128])
 def test_inverse_sub_blocks_of_the_diagonal_kernel(ops, blocks, rows):
