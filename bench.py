@@ -900,7 +900,8 @@ def time_alone(torch, fn, reps):
 STAGE_KERNELS = {
     'factor': 'gram_kernel + direct_kernel + tc_pair_kernel (grouped launches '
               'over all factors, plus staging and the split reductions)',
-    'inverse': 'packed_tile_kernel + tc_tile_kernel + chol_diag_kernel '
+    'inverse': 'packed_tile_kernel + tc_tile_kernel + chol_diag_kernel + '
+               'panel_solve_kernel '
                '(batched blocked Cholesky, '
                'triangular inverse and symmetric product of every factor, '
                'three size classes on three streams)',

@@ -1104,7 +1104,7 @@ __device__ __forceinline__ void diag_store(const DiagSmem& sm, const MatInfo& mi
 // 46 900 cycles; 3400 now, 42 000; 56 000 before all of this).
 //
 // 128 rows: 16 us with the launch, 22 us with the look-ahead in front (20.5 and 30
-// before); a row panel of X is stored when its sub-block is through, beside the
+// before), 18 of them behind the end of the kernel in front; a row panel of X is stored when its sub-block is through, beside the
 // next.
 template <bool LOOK>
 __global__ void __launch_bounds__(DT, 1)
@@ -1257,7 +1257,8 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
 // microsecond; the rest is 64 KB of A', 48 KB of X_kk and 64 KB of L for each CTA,
 // one after the other, of which A' and its terms come before the wait for the
 // diagonal kernel.  (By the tile kernel, which reads X_kk as fp32 and splits it in
-// every CTA, 7.5 to 9.5 us a launch.)
+// every CTA, 7.5 to 9.5 us a launch; solve and update behind a diagonal kernel 18.5
+// us then, 11.5 now.)
 constexpr int kSolveThreads = 256;
 struct SolveControl {
   unsigned long long x_here, done;
