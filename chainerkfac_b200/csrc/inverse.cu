@@ -2044,6 +2044,48 @@ extern "C" int kfac_inverse_plan_create(
   for (int i = 0; i < count; ++i) row_tiles += (dims[i] + DB - 1) / DB;
   const bool ahead = look && dmax <= 2 * PW && row_tiles <= sm_count();
   const int E = ahead ? DB : 0;
+  // Update of the window of columns from s on with columns k .. k + K of L.
+  auto window = [&](const MatInfo& m, int d, int s, int k, int K,
+                    std::vector<GemmDesc>& out) {
+    const int M = d - s, N = std::min(CW, M);
+    if (M <= 0) return;
+    const long long ld = m.ld;
+    const float* rows = m.W + s * ld + k;
+    GemmDesc g = {};     // square block on the diagonal: lower tiles
+    g.A = strided_operand(rows, 1, ld, N);
+    g.B = g.A;
+    g.C = m.W + s * ld + s;
+    g.ldc = ld; g.M = N; g.N = N; g.K = K;
+    g.alpha = -1.f; g.beta = 1.f; g.flags = G_LOWER | G_SAME_AB | packed;
+    set_l(g, m, s, s, k);
+    out.push_back(g);
+    if (M == N) return;
+    GemmDesc h = {};     // rectangle below it
+    h.A = strided_operand(rows + N * ld, 1, ld, M - N);
+    h.B = strided_operand(rows, 1, ld, N);
+    h.C = m.W + (long long)(s + N) * ld + s;
+    h.ldc = ld; h.M = M - N; h.N = N; h.K = K;
+    h.alpha = -1.f; h.beta = 1.f; h.flags = packed;
+    set_l(h, m, s + N, s, k);
+    out.push_back(h);
+  };
+  // Whether the near update takes the columns of the panel's last block by
+  // themselves, so that the others' part runs beside the last diagonal kernel and
+  // the chain waits for 128 k instead of 512.  It costs another pass over the window,
+  // behind the far update of the panel before: not where plans fill the SMs (the
+  // three of ResNet-50 4092 us without, 4141 with), nor where that update takes as
+  // long as a panel, which goes by the squares of the sides.  us without and with, by
+  // squares in tiles: 8 x 1024 (512) 311 304, 16 x 1024 (1024) 374 367, 4608 rows
+  // (1296) 1066 1055, 2 x 3400 (1458) 868 854, 5 x 2304 (1620) 647 621, 3 x 3000
+  // (1728) 820 789, 6 x 2304 (1944) 709 684, 2 x 4000 (2048) 1081 1066, 3 x 3400
+  // (2187) 1026 1011, 6000 rows (2209) 1716 1685; 2 x 4608 (2592) 1364 1376.
+  long long squares = 0;
+  for (int i = 0; i < count; ++i) {
+    const long long t = (dims[i] + DB - 1) / DB;
+    squares += t * t;
+  }
+  const bool split_near =
+      look && row_tiles <= sm_count() && squares <= 16 * sm_count();
   int near_ev = -1;            // near updates of the panel before
   for (int co = 0; co < dmax; co += CW) {
     const int inner = std::min(CW, dmax - co);
@@ -2117,6 +2159,15 @@ extern "C" int kfac_inverse_plan_create(
       }
       upd_ev[o / DB] = end_gemm(upd, look);
       if (upd_ev[o / DB] >= 0) bulk_ev = upd_ev[o / DB];
+      if (split_near && inner > DB && o + 2 * DB == co + inner) {
+        std::vector<GemmDesc> pre_descs;
+        for (int i : order)
+          window(mats[i], dims[i], co + CW + E, co, inner - DB, pre_descs);
+        Launch pre = begin_gemm(S_FAR);
+        for (auto& g : pre_descs) push_desc(pre, g);
+        pre.wait(solve_ev);      // (and, on this stream, the far update before)
+        if (pre.n > 0) prev_far_ev = end_gemm(pre, true);
+      }
       // (the last rows of a chain panel come behind its trailing update)
       if ((o + DB) % PW == 0 && o + DB < co + inner) row_panel(o + DB - PW);
     }
@@ -2127,33 +2178,10 @@ extern "C" int kfac_inverse_plan_create(
     // ordered by events (near of a panel after far of the one before).
     Launch near = begin_gemm(s_bulk);
     std::vector<GemmDesc> far_descs;
-    auto window = [&](const MatInfo& m, int d, int s, int k, int K,
-                      std::vector<GemmDesc>& out) {
-      const int M = d - s, N = std::min(CW, M);
-      if (M <= 0) return;
-      const long long ld = m.ld;
-      const float* rows = m.W + s * ld + k;
-      GemmDesc g = {};     // square block on the diagonal: lower tiles
-      g.A = strided_operand(rows, 1, ld, N);
-      g.B = g.A;
-      g.C = m.W + s * ld + s;
-      g.ldc = ld; g.M = N; g.N = N; g.K = K;
-      g.alpha = -1.f; g.beta = 1.f; g.flags = G_LOWER | G_SAME_AB | packed;
-      set_l(g, m, s, s, k);
-      out.push_back(g);
-      if (M == N) return;
-      GemmDesc h = {};     // rectangle below it
-      h.A = strided_operand(rows + N * ld, 1, ld, M - N);
-      h.B = strided_operand(rows, 1, ld, N);
-      h.C = m.W + (long long)(s + N) * ld + s;
-      h.ldc = ld; h.M = M - N; h.N = N; h.K = K;
-      h.alpha = -1.f; h.beta = 1.f; h.flags = packed;
-      set_l(h, m, s + N, s, k);
-      out.push_back(h);
-    };
     std::vector<GemmDesc> near_descs;
     for (int i : order) {
-      window(mats[i], dims[i], co + CW + E, co, CW, near_descs);
+      const int done = split_near ? inner - DB : 0;
+      window(mats[i], dims[i], co + CW + E, co + done, CW - done, near_descs);
       window(mats[i], dims[i], co + 2 * CW + E, 0, co + CW, far_descs);
     }
     for (auto& g : near_descs) push_desc(near, g);

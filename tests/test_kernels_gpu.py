@@ -1088,6 +1088,14 @@ def test_inverse_by_graph_and_by_plain_launches(ops, monkeypatch, dims):
         plan.close()
 
 
+@pytest.mark.parametrize('dims', [[513, 512, 30], [641, 640, 513], [1153, 700, 300],
+                                  [1537, 1025, 512], [2305, 1664, 129]])
+def test_inverse_windows_behind_a_panel(ops, dims):
+    """The updates of the columns behind a panel of 512, in two parts: windows of
+    one row and more, and matrices that end before, at and behind the panel."""
+    run_pairs(ops, dims, [max(1, d // 5) for d in dims], 1e-3, seed=dims[0])
+
+
 def test_inverses_repeat_bit_for_bit_beside_each_other(ops):
     """Sums are in a fixed order, so nothing changes from run to run, also where
     three plans fill the SMs and warps of a block wait for each other longer (a
