@@ -2034,9 +2034,9 @@ extern "C" int kfac_inverse_plan_create(
   // the second block needs.  It pays for matrices of two panels, where the one near
   // update between them is a good part of the chain; longer ones wait for their
   // panel updates anyway, which the further column makes longer.  us without and
-  // with, by row tiles, a plan by itself: 8 x 1024 (64) 323 312, 16 x 1024 (128) 388
-  // 377; 4608 rows (36) 1069 1081, 2 x 3400 (54) 872 875, 2 x 4608 (72) 1384 1411,
-  // 4608 beside 6 x 1000 (84) 1133 1158, 5 x 2304 (90) 651 649, 6 x 2304 (108) 713
+  // with, by row tiles, a plan by itself: 8 x 1024 (64) 314 307, 16 x 1024 (128) 378
+  // 368; 4608 rows (36) 1057 1063, 2 x 3400 (54) 853 863, 2 x 4608 (72) 1381 1414,
+  // 4608 beside 6 x 1000 (84) 1118 1139, 5 x 2304 (90) 625 638, 6 x 2304 (108) 690
   // 724.  Where plans run beside each other and fill the SMs, the passes over that
   // column only cost (108 factors of ResNet-50, plans of 120, 309 and 225 row tiles);
   // such plans are large.
