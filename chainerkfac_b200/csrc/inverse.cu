@@ -162,10 +162,8 @@ __device__ __forceinline__ float equil_scale(float x) {
 constexpr int kDampRows = 4;
 __global__ void __launch_bounds__(256, 4)
 damp_copy_kernel(const MatInfo* __restrict__ mats,
-                 const float* __restrict__ trace,
-                 const RunParams* __restrict__ prm, float* __restrict__ add,
-                 float* __restrict__ add2, float* __restrict__ add_out,
-                 int equil) {
+                 const float* trace, const RunParams* __restrict__ prm,
+                 float* add, float* add2, float* add_out, int equil) {
   let_next_launch_begin();
   const MatInfo mi = mats[blockIdx.y];
   const int d = mi.d;
@@ -1109,7 +1107,7 @@ __device__ __forceinline__ void diag_store(const DiagSmem& sm, const MatInfo& mi
 template <bool LOOK>
 __global__ void __launch_bounds__(DT, 1)
 chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
-                 int* __restrict__ info, int pack) {
+                 int* info, int pack) {
   extern __shared__ __align__(16) float dsm[];
   DiagSmem& sm = *reinterpret_cast<DiagSmem*>(dsm);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1409,8 +1407,7 @@ __device__ __forceinline__ float damp_of_row(const MatInfo& mi, float add,
 __global__ void __launch_bounds__(256)
 refine_probe_kernel(const MatInfo* __restrict__ mats,
                     const RefineItem* __restrict__ items,
-                    const float* __restrict__ add,
-                    const float* __restrict__ add2, double* __restrict__ sums,
+                    const float* add, const float* add2, double* sums,
                     const RunParams* __restrict__ prm, int stage) {
   let_next_launch_begin();
   wait_for_launch_before();
@@ -1473,10 +1470,9 @@ refine_probe_kernel(const MatInfo* __restrict__ mats,
 }
 
 __global__ void refine_gate_kernel(const RefineItem* __restrict__ items, int n,
-                                   const double* __restrict__ sums,
+                                   const double* sums,
                                    const RunParams* __restrict__ prm,
-                                   int* __restrict__ gate,
-                                   int* __restrict__ refined_count) {
+                                   int* gate, int* refined_count) {
   let_next_launch_begin();
   wait_for_launch_before();
   const int max_dim = prm->refine_max_dim;
@@ -1498,9 +1494,7 @@ __global__ void refine_gate_kernel(const RefineItem* __restrict__ items, int n,
 __global__ void __launch_bounds__(256)
 refine_residual_kernel(const MatInfo* __restrict__ mats,
                        const RefineItem* __restrict__ items, int nitems,
-                       const float* __restrict__ add,
-                       const float* __restrict__ add2,
-                       const int* __restrict__ gate) {
+                       const float* add, const float* add2, const int* gate) {
   __shared__ double As[16][64 + 2];   // As[k][i] = A[i0 + i][k0 + k]
   __shared__ double Bs[16][64 + 2];   // Bs[k][j] = X[k0 + k][j0 + j]
   __shared__ int s_item;
@@ -1582,7 +1576,7 @@ refine_residual_kernel(const MatInfo* __restrict__ mats,
 __global__ void __launch_bounds__(256)
 refine_apply_kernel(const MatInfo* __restrict__ mats,
                     const RefineItem* __restrict__ items,
-                    const int* __restrict__ gate) {
+                    const int* gate) {
   wait_for_launch_before();
   if (gate[blockIdx.y] == 0) return;
   const RefineItem it = items[blockIdx.y];

@@ -23,6 +23,10 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) {
 // wait_for_launch_before, which returns when it is complete.  A kernel lets the next
 // one begin once it has its tensor memory: the next one's CTAs keep theirs while
 // they wait.
+// So what any launch of such a row writes is changed while the kernel runs, and a
+// parameter that points there is not `__restrict__` (nor read by __ldg): the compiler
+// may move reads through one ahead of the wait.  That is for tables written before
+// the first of the row.
 __device__ __forceinline__ void let_next_launch_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
