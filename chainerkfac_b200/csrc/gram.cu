@@ -345,17 +345,9 @@ gram_kernel(const GramGroup* __restrict__ groups, int ngroups) {
                     0, cend, 32);
     }
   }
-  if (tid == 0 && ctl->abort_flag != 0) {
-    // a wait ran out: give the copies already issued time to land before
-    // the shared memory is handed back (bounded: 64 us)
-    for (int i = 0; i < 64; ++i) __nanosleep(1000);
-  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
-                 ::"r"(tmem), "r"(512)
-                 : "memory");
+  if (warp == 1) tc_release(tmem, 512, ctl->abort_flag != 0);
 }
 
 // ---------------------------------------------------- products without planes
@@ -646,15 +638,9 @@ direct_kernel(const DirectGroup* __restrict__ groups, int ngroups) {
                     32 * (warp >> 3), cend, 64);
     }
   }
-  if (tid == 0 && ctl->abort_flag != 0) {
-    for (int i = 0; i < 64; ++i) __nanosleep(1000);
-  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == DR_SPLIT + 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
-                 ::"r"(tmem), "r"(512)
-                 : "memory");
+  if (warp == DR_SPLIT + 1) tc_release(tmem, 512, ctl->abort_flag != 0);
 }
 
 // ------------------------------------------------------------------- staging

@@ -1242,9 +1242,7 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
       if (LOOK) mbar_wait_status(&ctl->x_here, 0, &ctl->grace, &g_diag_status);
       if (lane == 0) atomicExch(&g_diag_status, 1);
     }
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
-                 ::"r"(tmem), "r"(kDiagCols)
-                 : "memory");
+    tc_release(tmem, kDiagCols, ctl->abort_flag != 0);
   }
 }
 
@@ -1365,9 +1363,7 @@ panel_solve_kernel(const MatInfo* __restrict__ mats, int step) {
       mbar_wait_status(&ctl->x_here, 0, &ctl->grace, &g_diag_status);
       if (lane == 0) atomicExch(&g_diag_status, 1);
     }
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
-                 ::"r"(tmem), "r"(kDiagCols)
-                 : "memory");
+    tc_release(tmem, kDiagCols, ctl->abort_flag != 0);
   }
 }
 

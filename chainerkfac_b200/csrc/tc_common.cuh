@@ -229,6 +229,23 @@ __device__ __forceinline__ void tc_ld_16x32(unsigned taddr, float v[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Hands a block's tensor memory back, by the warp that took it, behind the block's
+// last barrier.  `aborted`: a wait of the block ran out, and the copies and MMAs
+// already issued get time to end before the tensor memory, and with the block its
+// shared memory, are another's (bounded: 64 us).  Not ahead of that barrier: a warp
+// that is done before the others wait would find no flag.
+__device__ __forceinline__ void tc_release(unsigned tmem, unsigned columns,
+                                           bool aborted) {
+  if (aborted) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    __syncwarp();
+  }
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+               ::"r"(tmem), "r"(columns)
+               : "memory");
+}
+
 // Byte offset of element (row, k) inside a K-major SW128 tile (k < 32).
 __device__ __forceinline__ int sw128_chunk_off(int row, int chunk) {
   return row * 128 + ((chunk ^ (row & 7)) << 4);

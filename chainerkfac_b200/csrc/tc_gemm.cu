@@ -692,18 +692,9 @@ tc_pair_kernel(const GemmDesc* __restrict__ descs, int ndesc,
       asm volatile("bar.sync 1, %0;" ::"r"(PK_PRODUCERS) : "memory");
     }
   }
-  if (STAGED && tid == 0 && ctl->abort_flag != 0) {
-    // a wait ran out: give the copies already issued time to land before
-    // the shared memory is handed back (bounded: 64 us)
-    for (int i = 0; i < 64; ++i) __nanosleep(1000);
-  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == PK_PWARPS) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
-                 ::"r"(tmem), "r"(TC_TMEM_COLS)
-                 : "memory");
-  }
+  if (warp == PK_PWARPS) tc_release(tmem, TC_TMEM_COLS, ctl->abort_flag != 0);
 }
 
 

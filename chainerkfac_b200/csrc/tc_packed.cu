@@ -822,18 +822,7 @@ packed_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc,
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 1 && ctl->abort_flag != 0) {
-    // a wait ran out: give the copies and MMAs already issued time to end before
-    // the shared and the tensor memory are handed back (bounded: 64 us).  Behind
-    // the barrier: the warp that issues the copies is done before the others wait
-    // for them, and would find no flag.
-    for (int i = 0; i < 64; ++i) __nanosleep(1000);
-    __syncwarp();
-  }
-  if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
-                 ::"r"(tmem), "r"(2 * TN)
-                 : "memory");
+  if (warp == 1) tc_release(tmem, 2 * TN, ctl->abort_flag != 0);
 }
 
 // ------------------------------------------------------------------ host side

@@ -633,11 +633,7 @@ tc_tile_kernel(const GemmDesc* __restrict__ descs, int ndesc, int tile0,
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == Map::kWarps) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
-                 ::"r"(tmem), "r"(Map::kTmem)
-                 : "memory");
-  }
+  if (warp == Map::kWarps) tc_release(ctl->tmem_base, Map::kTmem, ctl->abort_flag != 0);
 }
 
 // ------------------------------------------------------------------ host side

@@ -85,3 +85,26 @@ def test_early_kernels_promise_nothing_of_what_others_write(early):
                 m = re.match(r'\s*const\s+(\w+)\s*\*\s*__restrict__\s+\w+\s*$', p)
                 assert m and m.group(1) in STATIC, (name, p.strip())
         assert not re.search(r'__ldg\s*\(|ld\.global\.nc', body), name
+
+
+def test_tensor_memory_goes_back_behind_what_is_under_way():
+    """Where a bounded wait has run out, copies and MMAs may still be under way:
+    only tc_release hands tensor memory back, which gives them time, and only
+    behind the block's last barrier, where the flag is everybody's."""
+    text = source()
+    assert text.count('tcgen05.dealloc') == 1
+    fns = functions(text)
+    assert 'tcgen05.dealloc' in fns['tc_release'][2]
+    assert '__nanosleep' in fns['tc_release'][2]
+    users = 0
+    for name, (kernel, _, body) in fns.items():
+        if 'tc_release(' not in body:
+            continue
+        users += 1
+        assert kernel, name
+        last = body[body.rindex('__syncthreads()'):]
+        assert re.search(r'tc_release\([^;]*abort_flag != 0\)', last), name
+        assert 'tcgen05.mma' not in last and 'complete_tx' not in last, name
+    # (the allocation of the diagonal kernel is in a function of its own)
+    assert users == len([b for _, _, b in fns.values()
+                         if 'tcgen05.alloc' in b])
