@@ -1465,24 +1465,30 @@ refine_probe_kernel(const MatInfo* __restrict__ mats,
   }
 }
 
-__global__ void refine_gate_kernel(const RefineItem* __restrict__ items, int n,
-                                   const double* sums,
-                                   const RunParams* __restrict__ prm,
-                                   int* gate, int* refined_count) {
+// Which matrices the step refines, and how many: one block, as the count has to be
+// whole when it is stored.
+constexpr int kGateThreads = 256;
+__global__ void __launch_bounds__(kGateThreads)
+refine_gate_kernel(const RefineItem* __restrict__ items, int n, const double* sums,
+                   const RunParams* __restrict__ prm, int* gate,
+                   int* refined_count) {
   let_next_launch_begin();
   wait_for_launch_before();
   const int max_dim = prm->refine_max_dim;
-  const float threshold = prm->refine_threshold;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) *refined_count = 0;
-  __syncthreads();
-  if (i >= n) return;
-  const double e2 = sums[2 * i], t2 = sums[2 * i + 1];
-  const double thr = (double)threshold;
-  // a NaN estimate (broken factorisation) is left alone: info reports it
-  const int on = items[i].d <= max_dim && e2 > thr * thr * t2;
-  gate[i] = on;
-  if (on) atomicAdd(refined_count, 1);
+  const double thr = (double)prm->refine_threshold;
+  int refined = 0;
+  for (int i0 = 0; i0 < n; i0 += kGateThreads) {
+    const int i = i0 + (int)threadIdx.x;
+    int on = 0;
+    if (i < n) {
+      const double e2 = sums[2 * i], t2 = sums[2 * i + 1];
+      // a NaN estimate (broken factorisation) is left alone: info reports it
+      on = items[i].d <= max_dim && e2 > thr * thr * t2;
+      gate[i] = on;
+    }
+    refined += __syncthreads_count(on);
+  }
+  if (threadIdx.x == 0) *refined_count = refined;
 }
 
 // R = I - (F + add I) X for a 64 x 64 tile, fp64 accumulation, R stored as
@@ -2458,7 +2464,7 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
       KFAC_LAUNCH_CHECK("refine_probe_kernel");
     }
     KFAC_CUDA(early(true));
-    refine_gate_kernel<<<ceil_div(p->n_refine, 256), 256, 0, st>>>(
+    refine_gate_kernel<<<1, kGateThreads, 0, st>>>(
         p->refine_items_dev, p->n_refine, p->refine_sums_dev, p->params_dev,
         p->refine_gate_dev, p->refine_count_dev);
     KFAC_LAUNCH_CHECK("refine_gate_kernel");

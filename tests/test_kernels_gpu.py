@@ -688,6 +688,30 @@ def test_inverse_reports_non_spd(ops):
     plan.close()
 
 
+@pytest.mark.parametrize('count', [255, 256, 257, 900])
+def test_refined_factors_are_all_counted(ops, count):
+    """Plans of more factors than a block has threads: the count is whole, and of
+    the factors whose estimate exceeds the threshold."""
+    rng = np.random.default_rng(count)
+    F = [dev(spd(rng, 3 + i % 7)) for i in range(count)]
+    inv = [torch.empty_like(f) for f in F]
+    plan = ops.InversePlan(F, inv, [-1] * count, [2] * count)
+    plan.run(1e-3)
+    est = np.sort(plan.error_estimates())
+    assert est[0] >= 0
+    above = list(est[1:]) + [2 * est[-1] + 1e-6]
+    for at in (0, count // 2, count - 1):
+        line = float(np.float32(0.5 * (est[at] + above[at])))
+        plan.set_refine(1024, line)
+        for _ in range(5):
+            plan.run(1e-3)
+            assert plan.refined() == int((est > line).sum())
+    plan.set_refine(0)
+    plan.run(1e-3)
+    assert plan.refined() == 0
+    plan.close()
+
+
 @pytest.mark.parametrize('d', [97, 130, 640, 1100, 2200])
 def test_inverse_of_badly_scaled_factors(ops, d):
     """Columns whose scales span six orders of magnitude: the error of entry
