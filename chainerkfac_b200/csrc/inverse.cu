@@ -1672,6 +1672,8 @@ struct kfac_inverse_plan {
   int* graph_info;
   float* graph_diag;
   long long graph_launches;
+  int graph_early;                   // of them, those that begin early
+  int run_early;                     // of the last run, -1: plain launches
   bool graph_ok;
 };
 
@@ -2244,6 +2246,8 @@ extern "C" int kfac_inverse_plan_create(
   p->graph_info = nullptr;
   p->graph_diag = nullptr;
   p->graph_launches = 0;
+  p->graph_early = 0;
+  p->run_early = -1;
   {
     const char* env = getenv("KFAC_INVERSE_GRAPH");
     p->graph_ok = !(env && env[0] == '0');
@@ -2355,8 +2359,9 @@ static cudaGraphNode_t captured_kernel(cudaStream_t st) {
 
 // The next launch on a capturing stream may begin before `node` has ended
 // (programmatic dependency: it waits for the rest of it itself), but not before
-// anything else that it follows.
-static cudaError_t begin_before_end_of(cudaStream_t st, cudaGraphNode_t node) {
+// anything else that it follows.  `count` goes up if it does.
+static cudaError_t begin_before_end_of(cudaStream_t st, cudaGraphNode_t node,
+                                       int* count) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   const cudaGraphNode_t* deps = nullptr;
   const cudaGraphEdgeData* edges = nullptr;
@@ -2373,8 +2378,11 @@ static cudaError_t begin_before_end_of(cudaStream_t st, cudaGraphNode_t node) {
       data[i].type = cudaGraphDependencyTypeProgrammatic;
     }
   }
-  return cudaStreamUpdateCaptureDependencies_v2(
+  e = cudaStreamUpdateCaptureDependencies_v2(
       st, nodes.data(), data.data(), n, cudaStreamSetCaptureDependencies);
+  if (e == cudaSuccess)
+    *count += (int)std::count(nodes.begin(), nodes.end(), node);
+  return e;
 }
 
 // Issue every launch of one run into `st` (a real stream, or one that is
@@ -2394,7 +2402,8 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
   graph = graph && p->use_tc;
   auto early = [&](bool when) -> cudaError_t {
     const cudaGraphNode_t before = graph && when ? captured_kernel(st) : nullptr;
-    return before != nullptr ? begin_before_end_of(st, before) : cudaSuccess;
+    return before != nullptr ? begin_before_end_of(st, before, &p->graph_early)
+                             : cudaSuccess;
   };
   trace_kernel<<<p->count, kTraceThreads, 0, st>>>(p->mats_dev, p->trace_dev, info);
   KFAC_LAUNCH_CHECK("trace_kernel");
@@ -2417,7 +2426,7 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
       // look-ahead does not begin early itself.  (A layer of 334 x 53, three
       // diagonal blocks in a row: 222.6 us, 217.7 so; one of 4608 x 512 1304, 1294.)
       if (l.look && last_diag != nullptr)
-        KFAC_CUDA(begin_before_end_of(st, last_diag));
+        KFAC_CUDA(begin_before_end_of(st, last_diag, &p->graph_early));
       if (l.look)
         chol_diag_kernel<true><<<l.n, DT, kDiagLookSmemBytes, st>>>(
             p->sorted_dev, l.step, info, p->packed);
@@ -2427,7 +2436,8 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
       KFAC_LAUNCH_CHECK("chol_diag_kernel");
       if (graph) last_diag = captured_kernel(st);
     } else if (l.kind == 2) {
-      if (last_diag != nullptr) KFAC_CUDA(begin_before_end_of(st, last_diag));
+      if (last_diag != nullptr)
+        KFAC_CUDA(begin_before_end_of(st, last_diag, &p->graph_early));
       panel_solve_kernel<<<dim3(l.tiles, l.n), kSolveThreads, kSolveSmemBytes,
                            st>>>(p->sorted_dev, l.step);
       KFAC_LAUNCH_CHECK("panel_solve_kernel");
@@ -2536,6 +2546,7 @@ static void plan_capture(kfac_inverse_plan* p, int* info, float* diag_dev) {
     p->graph_ok = false;
     return;
   }
+  p->graph_early = 0;
   const int rc = plan_enqueue(p, info, diag_dev, c.chain, c.side, true);
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(c.chain, &graph);
@@ -2579,10 +2590,12 @@ extern "C" int kfac_inverse_plan_run(kfac_inverse_plan* p, float damping,
       if (p->graph_exec != nullptr) {
         KFAC_CUDA(cudaGraphLaunch(p->graph_exec, st));
         count_launches(p->graph_launches);
+        p->run_early = p->graph_early;
         return KFAC_OK;
       }
     }
   }
+  p->run_early = -1;
   KFAC_CUDA(make_side_streams(p->side_stream));
   return plan_enqueue(p, info, diag_dev, st, p->side_stream, false);
 }
@@ -2595,6 +2608,14 @@ extern "C" int kfac_inverse_plan_set_refine(kfac_inverse_plan* p, int max_dim,
                (double)threshold);
   p->refine_max_dim = max_dim < kRefineDimCap ? max_dim : kRefineDimCap;
   p->refine_threshold = threshold;
+  return KFAC_OK;
+}
+
+extern "C" int kfac_inverse_plan_early_launches(kfac_inverse_plan* p,
+                                                int* early_out) {
+  KFAC_REQUIRE(p != nullptr && early_out != nullptr,
+               "inverse_plan_early_launches: null argument");
+  *early_out = p->run_early;
   return KFAC_OK;
 }
 

@@ -467,6 +467,14 @@ class InversePlan(object):
             self._handle, out), 'kfac_inverse_plan_error_estimates')
         return list(out)
 
+    def early_launches(self):
+        """Launches of the last run that could begin before the one in front had
+        ended (-1: plain launches, no replayed graph)."""
+        n = ctypes.c_int(0)
+        _lib.check(self._lib.kfac_inverse_plan_early_launches(
+            self._handle, ctypes.byref(n)), 'kfac_inverse_plan_early_launches')
+        return n.value
+
     def refined(self):
         """Number of factors the last run refined (synchronises)."""
         n = ctypes.c_int(0)

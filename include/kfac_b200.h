@@ -301,6 +301,12 @@ int kfac_inverse_plan_run(kfac_inverse_plan* plan, float damping, int use_pi,
  * next run. */
 int kfac_inverse_plan_set_refine(kfac_inverse_plan* plan, int max_dim,
                                  float threshold);
+/* *early_out = number of launches of the plan's last run that could begin before
+ * the launch in front of them had ended, or -1 if the run was plain launches one
+ * behind the other (no replayed CUDA graph: KFAC_INVERSE_GRAPH=0, a capturing
+ * caller, a graph that could not be made) or there was none. */
+int kfac_inverse_plan_early_launches(kfac_inverse_plan* plan, int* early_out);
+
 /* Synchronises the device; *refined_out = number of factors the last run
  * refined. */
 int kfac_inverse_plan_refined(kfac_inverse_plan* plan, int* refined_out);

@@ -1087,7 +1087,7 @@ def test_inverse_around_block_sizes(ops, d):
 
 @pytest.mark.parametrize('dims', [[129], [300, 10, 257], [640, 1100, 96],
                                   [520] * 20])
-def test_inverse_by_graph_and_by_plain_launches(ops, monkeypatch, dims):
+def test_inverse_by_graph_and_by_plain_launches(ops, engine, monkeypatch, dims):
     """The same launches in the same order: bit for bit, three runs over inputs
     that change (the graph's kernels begin before the ones in front have ended)."""
     rng = np.random.default_rng(len(dims))
@@ -1105,6 +1105,10 @@ def test_inverse_by_graph_and_by_plain_launches(ops, monkeypatch, dims):
             f.copy_((f + f.t()) / 2)
         for plan in plans:
             plan.run(1e-2)
+        # (what they were: a diagonal kernel and a solve per block but the first;
+        # nothing begins early on the other engine)
+        assert plans[0].early_launches() >= 2 * ((max(dims) - 1) // 128) * engine
+        assert plans[1].early_launches() == -1
         torch.cuda.synchronize()
         for a, b in zip(*outs):
             assert torch.isfinite(a).all() and torch.equal(a, b)
@@ -1120,7 +1124,7 @@ def test_inverse_windows_behind_a_panel(ops, dims):
     run_pairs(ops, dims, [max(1, d // 5) for d in dims], 1e-3, seed=dims[0])
 
 
-def test_inverses_repeat_bit_for_bit_beside_each_other(ops):
+def test_inverses_repeat_bit_for_bit_beside_each_other(ops, engine):
     """Sums are in a fixed order, so nothing changes from run to run, also where
     three plans fill the SMs and warps of a block wait for each other longer (a
     warp's columns of a diagonal sub-block were touched by another one too soon in
@@ -1143,6 +1147,8 @@ def test_inverses_repeat_bit_for_bit_beside_each_other(ops):
         plan.run(1e-3)
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(first, inv))
+        for p in plan.plans:
+            assert p.early_launches() > 0 if engine else p.early_launches() == 0
 
 
 @pytest.mark.parametrize('blocks', [0, 1, 4])
