@@ -1037,7 +1037,7 @@ __device__ __forceinline__ void diag_next(DiagSmem& sm, DiagControl* ctl, int p,
 // Lanes are laid out so that a quarter warp's loads fall into different banks.
 __device__ __forceinline__ void diag_store(const DiagSmem& sm, const MatInfo& mi,
                                            int o, int bs, int p, int u, int half,
-                                           int lane, int pack) {
+                                           int lane) {
   const long long ld = mi.ld;
   float* Xd = mi.X + (long long)o * ld + o;
   unsigned char* const px = mi.PX + (long long)(o / DB) * mi.tile;
@@ -1061,7 +1061,6 @@ __device__ __forceinline__ void diag_store(const DiagSmem& sm, const MatInfo& mi
     // (columns past bs are zeros above the diagonal, inside the row pitch)
     *reinterpret_cast<float4*>(dst + e * ld) =
         make_float4(x[0][e], x[1][e], x[2][e], x[3][e]);
-    if (!pack) continue;
     unsigned h0, h1, l0, l1;
     split_half2(kScaleX * x[0][e], kScaleX * x[1][e], h0, l0);
     split_half2(kScaleX * x[2][e], kScaleX * x[3][e], h1, l1);
@@ -1106,8 +1105,7 @@ __device__ __forceinline__ void diag_store(const DiagSmem& sm, const MatInfo& mi
 // next.
 template <bool LOOK>
 __global__ void __launch_bounds__(DT, 1)
-chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
-                 int* info, int pack) {
+chol_diag_kernel(const MatInfo* __restrict__ mats, int step, int* info) {
   extern __shared__ __align__(16) float dsm[];
   DiagSmem& sm = *reinterpret_cast<DiagSmem*>(dsm);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1231,7 +1229,7 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
       if (ctl->abort_flag != 0) continue;
 #pragma unroll 1
       for (int u = slot; u < 2 * (p + 1); u += warps)
-        diag_store(sm, mi, o, bs, p, u >> 1, u & 1, lane, pack);
+        diag_store(sm, mi, o, bs, p, u >> 1, u & 1, lane);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1244,6 +1242,75 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step,
     }
     tc_release(tmem, kDiagCols, ctl->abort_flag != 0);
   }
+}
+
+// The same on engine 0: fp32 multiply-adds and nothing of the kernel above, as the
+// tests hold that one against this.  A column of [D; I] at a time, all of it in one
+// square of registers: row i is D's until column i is through, then X^T's, which
+// begins on the diagonal.  A thread has rows warp + 16 a, columns lane + 32 b.
+// Bound by the chain of its 128 steps, a root, a quotient and a barrier each: 56 us
+// for 128 rows with the launch (16 by the kernel above; 159 with the square in shared
+// memory and two barriers a step).
+__global__ void __launch_bounds__(DT, 1)
+chol_diag_ffma_kernel(const MatInfo* __restrict__ mats, int step, int* info) {
+  constexpr int RA = DB / (DT / 32), CB = DB / 32;
+  __shared__ float cols[2][DB];           // the step's column (twice: one barrier)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const MatInfo mi = mats[blockIdx.x];
+  const int o = step * DB;
+  const int bs = min(DB, mi.d - o);
+  const long long ld = mi.ld, at = (long long)o * ld + o;
+  float m[RA][CB];
+#pragma unroll
+  for (int a = 0; a < RA; ++a)
+#pragma unroll
+    for (int b = 0; b < CB; ++b) {
+      const int i = warp + DT / 32 * a, c = lane + 32 * b;
+      m[a][b] = i < bs && c <= i ? mi.W[at + i * ld + c] : 0.f;
+    }
+#pragma unroll
+  for (int b0 = 0; b0 < CB; ++b0) {
+#pragma unroll 1
+    for (int j = 32 * b0; j < min(bs, 32 * b0 + 32); ++j) {
+      float* const col = cols[j & 1];
+      if (lane == j - 32 * b0) {
+#pragma unroll
+        for (int a = 0; a < RA; ++a) col[warp + DT / 32 * a] = m[a][b0];
+      }
+      __syncthreads();
+      const float q = col[j];
+      const bool positive = q >= 1.17549435e-38f;
+      const float r = positive ? 1.f / sqrtf(q) : 1.f;
+      if (threadIdx.x == 0 && !positive) atomicCAS(&info[mi.id], 0, o + j + 1);
+      float x[RA], y[CB];
+#pragma unroll
+      for (int a = 0; a < RA; ++a) x[a] = col[warp + DT / 32 * a] * r;
+#pragma unroll
+      for (int b = b0; b < CB; ++b) y[b] = col[lane + 32 * b] * r;
+#pragma unroll
+      for (int a = 0; a < RA; ++a) {
+        // row-block a / 2: of X^T in front of this one, of D behind it, where what
+        // is above the diagonal does not count until the row begins again
+        const bool begins = a / 2 == b0 && warp + DT / 32 * a == j;
+        if (begins) x[a] = r;
+#pragma unroll
+        for (int b = b0; b < (a / 2 > b0 ? a / 2 + 1 : CB); ++b) {
+          if (b > b0 || lane > j - 32 * b0)
+            m[a][b] = fmaf(-x[a], y[b], begins ? 0.f : m[a][b]);
+          else if (lane == j - 32 * b0)
+            m[a][b] = x[a];
+        }
+      }
+    }
+  }
+  // (above the diagonal X is zeros from the start)
+#pragma unroll
+  for (int a = 0; a < RA; ++a)
+#pragma unroll
+    for (int b = 0; b < CB; ++b) {
+      const int i = warp + DT / 32 * a, c = lane + 32 * b;
+      if (c >= i && c < bs) mi.X[at + c * ld + i] = m[a][b];
+    }
 }
 
 // ------------------------------------------------------------ panel solve
@@ -1646,7 +1713,7 @@ struct kfac_inverse_plan {
   GemmDesc* descs_dev;
   std::vector<GemmDesc> descs;       // the same on the host
   std::vector<Launch> launches;
-  bool use_tc, packed;
+  bool use_tc;
   // refinement (see refine_* kernels)
   float* add2_dev;
   int n_refine;
@@ -2225,7 +2292,6 @@ extern "C" int kfac_inverse_plan_create(
   p->count = count;
   p->launches = launches;
   p->use_tc = use_tc;
-  p->packed = packed != 0;
   p->mats_dev = nullptr; p->trace_dev = nullptr; p->add_dev = nullptr;
   p->info_dev = nullptr; p->sorted_dev = nullptr; p->descs_dev = nullptr;
   p->add2_dev = nullptr; p->refine_items_dev = nullptr;
@@ -2427,12 +2493,14 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
       // diagonal blocks in a row: 222.6 us, 217.7 so; one of 4608 x 512 1304, 1294.)
       if (l.look && last_diag != nullptr)
         KFAC_CUDA(begin_before_end_of(st, last_diag, &p->graph_early));
-      if (l.look)
+      if (!p->use_tc)
+        chol_diag_ffma_kernel<<<l.n, DT, 0, st>>>(p->sorted_dev, l.step, info);
+      else if (l.look)
         chol_diag_kernel<true><<<l.n, DT, kDiagLookSmemBytes, st>>>(
-            p->sorted_dev, l.step, info, p->packed);
+            p->sorted_dev, l.step, info);
       else
         chol_diag_kernel<false><<<l.n, DT, kDiagSmemBytes, st>>>(
-            p->sorted_dev, l.step, info, p->packed);
+            p->sorted_dev, l.step, info);
       KFAC_LAUNCH_CHECK("chol_diag_kernel");
       if (graph) last_diag = captured_kernel(st);
     } else if (l.kind == 2) {

@@ -27,9 +27,9 @@ def ops():
 
 @pytest.fixture(autouse=True, params=[1, 0], ids=['tcgen05', 'fp32'])
 def engine(request):
-    """Every test runs on both arithmetic engines: tcgen05 split-TF32 tensor
-    cores (the default) and the fp32 FFMA tiles.  After a tensor-core run the
-    engine's status word must be clean (no barrier wait ran out)."""
+    """Every test runs on both arithmetic engines: tcgen05 tensor cores with
+    operands in terms (the default) and the fp32 FFMA tiles.  After a run the
+    status word must be clean (no barrier wait ran out)."""
     import ctypes
     from chainerkfac_b200 import _lib
     lib = _lib.load()
@@ -1179,6 +1179,46 @@ def test_inverse_sub_blocks_of_the_diagonal_kernel(ops, blocks, rows):
         assert (np.abs(got - truth) / s[:, None] / s[None, :]).max() < \
             35 * d * 2.0 ** -24
     assert torch.equal(inv[0], inv[2])
+    plan.close()
+
+
+def _multiply_adds(W):
+    """X = L^-1 of a Cholesky factor, a column of [W; I] at a time in fp32, every
+    product added with one rounding."""
+    f32, n = np.float32, len(W)
+    M = np.tril(W)
+    for j in range(n):
+        r = f32(1) / np.sqrt(M[j, j])
+        col = M[:, j] * r
+        col[j] = r
+        # (a product of two fp32 numbers is exact in fp64)
+        to = (M - np.outer(col.astype(np.float64), col)).astype(f32)
+        for i in range(n):
+            end = n if i <= j else i + 1
+            M[i, j + 1:end] = to[i, j + 1:end]
+        M[:j + 1, j] = col[:j + 1]
+    return np.triu(M).T
+
+
+@pytest.mark.parametrize('d', [1, 2, 31, 33, 100, 128])
+def test_yardstick_engine_eliminates_in_fp32(ops, engine, d):
+    """Engine 0 is what the tensor-core engine is measured against: its diagonal
+    blocks are multiply-adds in fp32 to the bit, none of the other's terms."""
+    if engine == 1:
+        pytest.skip('the tensor-core engine eliminates in bf16 terms')
+    rng = np.random.default_rng(d)
+    f = spd(rng, d)
+    F = dev(f)
+    plan = ops.InversePlan([F], [torch.empty_like(F)], [-1], [2])
+    plan.run(1e-3)
+    W = f.copy()
+    W[np.arange(d), np.arange(d)] += host(plan.diag)[0]
+    # the workspace: W, V and X, rows of a multiple of 32, from 256 bytes on
+    pitch = (d + 31) // 32 * 32
+    each = (4 * d * pitch + 255) // 256 * 256
+    at = -plan.workspace.data_ptr() % 256 + 2 * each
+    X = host(plan.workspace)[at:at + 4 * d * pitch].view(np.float32)
+    assert np.array_equal(X.reshape(d, pitch)[:, :d], _multiply_adds(W))
     plan.close()
 
 
