@@ -949,8 +949,8 @@ __device__ __forceinline__ void diag_fetch(unsigned t, f32x2 v[SB / 2]) {
 // X^T's new row-block (r == p) starts as the unit vector e_lane and ends as row
 // `lane` of X_pp^T.
 __device__ __forceinline__ void diag_follow(DiagSmem& sm, DiagControl* ctl,
-                                            unsigned tmem, int p, int np, int r,
-                                            int lane, unsigned tile) {
+                                            unsigned tmem, int p, int r, int lane,
+                                            unsigned tile) {
   f32x2 a[SB / 2];
   float* src = &sm.S[(SB * r + lane) * DLD + SB * p];
   float* out = r == p ? &sm.XD[p][lane * SLP] : r <= p + 1 ? src : nullptr;
@@ -1150,10 +1150,12 @@ chol_diag_kernel(const MatInfo* __restrict__ mats, int step, int* info) {
       const int r = warp == 1 ? p : warp - 4;
       const bool last = p == np - 1;
       if (warp == 1 || r != p) {
-        diag_follow(sm, ctl, tmem, p, np, r, lane, last ? 0u : tile);
+        diag_follow(sm, ctl, tmem, p, r, lane, last ? 0u : tile);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       } else if (p > 0 && !last) {
-        // from here on row-block r collects rows of X^T
+        // from here on row-block r collects rows of X^T.  (Nothing of `next` is read
+        // here, but its next phase is waited for by parity: this one has to be over.)
+        diag_wait(&ctl->next, (p - 1) & 1, &ctl->abort_flag);
         const bool ok = diag_wait_tmem(&ctl->beyond, (p - 1) & 1, &ctl->abort_flag);
 #pragma unroll 1
         for (int c = 2 * (p + 1); ok && c < 2 * np; ++c)
