@@ -1100,9 +1100,10 @@ __device__ __forceinline__ void diag_store(const DiagSmem& sm, const MatInfo& mi
 // are not the chain's are left rolled (8200 instructions with the look-ahead,
 // 46 900 cycles; 3400 now, 42 000; 56 000 before all of this).
 //
+// A row panel of X is stored when its sub-block is through, beside the next.
+//
 // 128 rows: 16 us with the launch, 22 us with the look-ahead in front (20.5 and 30
-// before), 18 of them behind the end of the kernel in front; a row panel of X is stored when its sub-block is through, beside the
-// next.
+// before), 18 of them behind the end of the kernel in front.
 template <bool LOOK>
 __global__ void __launch_bounds__(DT, 1)
 chol_diag_kernel(const MatInfo* __restrict__ mats, int step, int* info) {
@@ -1923,8 +1924,8 @@ extern "C" int kfac_inverse_plan_create(
   // Width of the chain's panels.  Between two panels the chain waits for the
   // last solve and the near part of the trailing update, so matrices of up to
   // two panels are one where the longer panel updates of a step still fit the
-  // SMs (1024 rows 232 us in two, 228 in one, 5 x 1001 274 and 264; 20 x 1024, or 4608
-  // rows, whose panel updates are what the chain waits for, gain nothing from it).
+  // SMs (5 x 1001 rows 274 us in two, 264 in one).  Where they do not (20 x 1024), or
+  // the chain waits for its panel updates anyway (4608 rows), nothing is gained.
   long long step_tiles = 0;
   for (int i = 0; i < count; ++i)
     if (dims[i] > PW)
@@ -1944,8 +1945,9 @@ extern "C" int kfac_inverse_plan_create(
   // The chain carries the diagonal kernels; the diagonal kernel of step k applies
   // step k-1's update to its own block itself (diag_lookahead), so it only waits
   // for the panel update of step k-2.  The panel solves, panel updates and near
-  // updates run on the bulk stream behind the chain.  A panel solve leaves W as it is (the look-ahead reads it) and
-  // stores L as fp16 chunks, which is how every product reads it.
+  // updates run on the bulk stream behind the chain.  A panel solve leaves W as it
+  // is (the look-ahead reads it) and stores L as fp16 chunks, which is how every
+  // product reads it.
   //
   // The inverse grows with the factor, a row panel at a time: with X = L^-1,
   //   T = L_p X_<p,  X_p = -X_pp T  (X_pp by doubling from the 128-blocks),
@@ -2099,14 +2101,11 @@ extern "C" int kfac_inverse_plan_create(
   // Whether a panel's steps also update the next one's first block column.  The
   // chain then goes on there without waiting for the near update, which only
   // the second block needs.  It pays for matrices of two panels, where the one near
-  // update between them is a good part of the chain; longer ones wait for their
-  // panel updates anyway, which the further column makes longer.  us without and
-  // with, by row tiles, a plan by itself: 8 x 1024 (64) 314 307, 16 x 1024 (128) 378
-  // 368; 4608 rows (36) 1057 1063, 2 x 3400 (54) 853 863, 2 x 4608 (72) 1381 1414,
-  // 4608 beside 6 x 1000 (84) 1118 1139, 5 x 2304 (90) 625 638, 6 x 2304 (108) 690
-  // 724.  Where plans run beside each other and fill the SMs, the passes over that
-  // column only cost (108 factors of ResNet-50, plans of 120, 309 and 225 row tiles);
-  // such plans are large.
+  // update between them is a good part of the chain (16 x 1024 rows 378 us without,
+  // 368 with); longer ones wait for their panel updates anyway, which the further
+  // column makes longer (2 x 4608 rows 1381 without, 1414 with).  Nor in plans of more
+  // row tiles than SMs: beside others, which such plans run, the passes over that
+  // column only cost.
   long long row_tiles = 0;
   for (int i = 0; i < count; ++i) row_tiles += (dims[i] + DB - 1) / DB;
   const bool ahead = look && dmax <= 2 * PW && row_tiles <= sm_count();
@@ -2141,11 +2140,8 @@ extern "C" int kfac_inverse_plan_create(
   // the chain waits for 128 k instead of 512.  It costs another pass over the window,
   // behind the far update of the panel before: not where plans fill the SMs (the
   // three of ResNet-50 4092 us without, 4141 with), nor where that update takes as
-  // long as a panel, which goes by the squares of the sides.  us without and with, by
-  // squares in tiles: 8 x 1024 (512) 311 304, 16 x 1024 (1024) 374 367, 4608 rows
-  // (1296) 1066 1055, 2 x 3400 (1458) 868 854, 5 x 2304 (1620) 647 621, 3 x 3000
-  // (1728) 820 789, 6 x 2304 (1944) 709 684, 2 x 4000 (2048) 1081 1066, 3 x 3400
-  // (2187) 1026 1011, 6000 rows (2209) 1716 1685; 2 x 4608 (2592) 1364 1376.
+  // long as a panel, which goes by the squares of the sides: between 6000 rows (2209
+  // squares of tiles: 1716 us without, 1685 with) and 2 x 4608 (2592: 1364, 1376).
   long long squares = 0;
   for (int i = 0; i < count; ++i) {
     const long long t = (dims[i] + DB - 1) / DB;
@@ -2240,9 +2236,10 @@ extern "C" int kfac_inverse_plan_create(
     }
 
     // Updates behind the finished panel, for windows of columns that begin with a
-    // panel (`ahead`: one block later): the next window with this panel, the window after it with all panels so
-    // far, next to the next panel's chain.  What touches the same tiles is
-    // ordered by events (near of a panel after far of the one before).
+    // panel (`ahead`: one block later): the next window with this panel, the window
+    // after it with all panels so far, next to the next panel's chain.  What touches
+    // the same tiles is ordered by events (near of a panel after far of the one
+    // before).
     Launch near = begin_gemm(s_bulk);
     std::vector<GemmDesc> far_descs;
     std::vector<GemmDesc> near_descs;
@@ -2513,8 +2510,7 @@ static int plan_enqueue(kfac_inverse_plan* p, int* info, float* diag_dev,
       KFAC_LAUNCH_CHECK("panel_solve_kernel");
     } else {
       // (more tiles than SMs: the next launch's waiting CTAs only take room; 54 pairs
-      // of ResNet-50 with a limit of half the SMs 3966 us, all of them 3931; of twice
-      // as many, beside others in another run, 4094, without a limit 4083, 3993 so)
+      // of ResNet-50 3993 us so, 4083 without a limit)
       KFAC_CUDA(early(l.tiles <= sm_count()));
       int rc = l.packed
                    ? launch_packed(p->descs_dev + l.off, &p->descs[l.off], l.n,
